@@ -186,6 +186,23 @@ def load():
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native host path (``_host.so``: torch tensors in, launches out), loaded with the library on first use."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _host as mod
+        except ImportError as e:
+            raise RuntimeError(f"the native host path _host.so is missing or does not load ({e}): "
+                               "run `python -m late_interaction_kernels_b200._build`.") from e
+        _host = mod
+    return _host
+
+
 def check(rc: int, what: str):
     if rc != 0:
         msg = load().lik_last_error().decode(errors="replace")

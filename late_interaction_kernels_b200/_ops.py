@@ -3,7 +3,8 @@
 Everything here takes torch CUDA tensors, allocates outputs / workspaces with
 torch (so the caching allocator and CUDA-graph capture keep working), fills the
 argument structs of ``include/lik_b200.h`` and calls the library on the current
-stream.  No arithmetic happens in Python.
+stream.  No arithmetic happens in Python.  The scoring operators' own calls take
+the native host path (``_lib.host()``) instead; it does the same in C++.
 """
 
 from __future__ import annotations
@@ -14,11 +15,22 @@ from dataclasses import dataclass
 import torch
 
 from . import _lib
-from ._lib import BwdArgs, FwdArgs, HiddenFwdArgs, PlaidIndex, Seqs, TopkSpec
+from ._lib import FwdArgs, HiddenFwdArgs, PlaidIndex, Seqs, TopkSpec
 
 # The launchers hand raw pointers to a C library: keep torch.compile from tracing into them (it
 # breaks the graph around the call instead).
 _no_trace = getattr(getattr(torch, "compiler", None), "disable", None) or (lambda f: f)
+
+
+@_no_trace
+def _untraced(fn, *args):
+    return fn(*args)
+
+
+def native_call(fn, *args):
+    """A call into the native host path: direct, or outside the graph when torch.compile is tracing (the wrapper that
+    keeps it from tracing costs microseconds per call, so it is only used there)."""
+    return _untraced(fn, *args) if torch.compiler.is_compiling() else fn(*args)
 
 
 @dataclass
@@ -33,7 +45,10 @@ class SeqSpec:
     lens: torch.Tensor | None = None  # int32 [n_seq]
     mask: torch.Tensor | None = None  # uint8 [n_rows]
     scale: torch.Tensor | None = None  # fp32 [n_rows]
-    scale_scalar: float = 1.0
+
+    def native(self):
+        """The fields as the native host path takes them."""
+        return self.data, self.n_seq, self.max_len, self.seq_stride, self.cu, self.lens, self.mask, self.scale
 
     def c_struct(self) -> Seqs:
         d = self.data
@@ -48,7 +63,7 @@ class SeqSpec:
             lens=_lib.ptr(self.lens),
             mask=_lib.ptr(self.mask),
             scale=_lib.ptr(self.scale),
-            scale_scalar=float(self.scale_scalar),
+            scale_scalar=1.0,
             reserved=0,
         )
 
@@ -64,7 +79,7 @@ def _as_u8_mask(mask: torch.Tensor | None) -> torch.Tensor | None:
     return (m != 0).view(torch.uint8)
 
 
-def padded_spec(x: torch.Tensor, mask=None, lens=None, scale=None, scale_scalar=1.0) -> SeqSpec:
+def padded_spec(x: torch.Tensor, mask=None, lens=None, scale=None) -> SeqSpec:
     """[N, L, d] tensor -> padded SeqSpec (copies only if not contiguous)."""
     x = x.contiguous()
     N, L, d = x.shape
@@ -75,27 +90,20 @@ def padded_spec(x: torch.Tensor, mask=None, lens=None, scale=None, scale_scalar=
         lens = lens.to(device=x.device, dtype=torch.int32).contiguous()
     if scale is not None:
         scale = scale.to(device=x.device, dtype=torch.float32).contiguous().reshape(-1)
-    return SeqSpec(x.view(N * L, d), N, L, L, None, lens, m, scale, scale_scalar)
+    return SeqSpec(x.view(N * L, d), N, L, L, None, lens, m, scale)
 
 
 def packed_spec(x: torch.Tensor, cu: torch.Tensor, max_len: int, scale=None) -> SeqSpec:
     """[sum L, d] tensor + int32 cumulative offsets -> packed SeqSpec."""
     x = x.contiguous()
     cu = cu.to(device=x.device, dtype=torch.int32).contiguous()
-    return SeqSpec(x, cu.numel() - 1, int(max_len), 0, cu, None, None, scale, 1.0)
-
-
-_status = {}
+    return SeqSpec(x, cu.numel() - 1, int(max_len), 0, cu, None, None, scale)
 
 
 def status_word(device) -> torch.Tensor:
     """Per-device int32 word the kernels OR their LIK_DEV_* bits into."""
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
-    t = _status.get(key)
-    if t is None:
-        t = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", key))
-        _status[key] = t
-    return t
+    index = torch.device(device).index
+    return _lib.host().status_word(torch.cuda.current_device() if index is None else index)
 
 
 def check_device_status(device=None, *, reset=True):
@@ -112,45 +120,15 @@ def check_device_status(device=None, *, reset=True):
         raise RuntimeError("late-interaction kernels reported: " + "; ".join(reasons))
 
 
-def n_scores(pairing, q: SeqSpec, d: SeqSpec, n_pairs) -> int:
-    if pairing == _lib.PAIR_CROSS:
-        return q.n_seq * d.n_seq
-    if pairing == _lib.PAIR_GROUPED:
-        return d.n_seq
-    return n_pairs
-
-
 @_no_trace
 def forward(q: SeqSpec, d: SeqSpec, *, pairing=_lib.PAIR_CROSS, group=0, pair_q=None, pair_d=None,
             normalize=0, save_argmax=False, argmax_stride=None, engine=0):
     """Launch ``lik_maxsim_fwd``.  Returns (scores fp32 [n_scores], argmax int32 [n_scores, stride] | None)."""
-    lib = _lib.load()
-    dev = q.data.device
     _lib.require_cuda(q.data, d.data, op="maxsim forward")
     if q.data.dtype != d.data.dtype:
         raise ValueError(f"Q and D must share a dtype on the kernel path; got {q.data.dtype} vs {d.data.dtype}")
-    dim = q.data.shape[1]
-    n_pairs = 0 if pair_q is None else pair_q.numel()
-    ns = n_scores(pairing, q, d, n_pairs)
-    scores = torch.empty(ns, dtype=torch.float32, device=dev)
     stride = q.max_len if argmax_stride is None else int(argmax_stride)
-    argmax = torch.empty((ns, stride), dtype=torch.int32, device=dev) if save_argmax else None
-    if ns == 0:
-        return scores, argmax
-    a = FwdArgs(
-        q=q.c_struct(), d=d.c_struct(), dtype=_lib.lik_dtype(q.data.dtype), dim=dim, pairing=pairing, group=group,
-        pair_q=_lib.ptr(pair_q), pair_d=_lib.ptr(pair_d), n_pairs=n_pairs, normalize=int(normalize), engine=engine,
-        scores=scores.data_ptr(), argmax=_lib.ptr(argmax) if (argmax is not None and argmax.numel()) else None,
-        argmax_stride=stride, reserved=0, workspace=None, workspace_bytes=0, status=status_word(dev).data_ptr(),
-    )
-    nbytes = lib.lik_maxsim_fwd_workspace(C.byref(a))
-    ws = None
-    if nbytes:
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-        a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
-    with torch.cuda.device(dev):
-        _lib.check(lib.lik_maxsim_fwd(C.byref(a), _lib.stream_ptr(dev)), "lik_maxsim_fwd")
-    return scores, argmax
+    return _lib.host().forward(q.native(), d.native(), pairing, group, pair_q, pair_d, int(normalize), save_argmax, stride, engine)
 
 
 @_no_trace
@@ -302,39 +280,9 @@ def backward(q: SeqSpec, d: SeqSpec, grad_scores: torch.Tensor, argmax: torch.Te
              group=0, pair_q=None, pair_d=None, normalize=0, deterministic=True, grad_dtype=None,
              need_q=True, need_d=True):
     """Launch ``lik_maxsim_bwd``.  Returns (grad_q [n_rows_q, dim] | None, grad_d [n_rows_d, dim] | None)."""
-    lib = _lib.load()
-    dev = q.data.device
     _lib.require_cuda(q.data, d.data, grad_scores, argmax, op="maxsim backward")
-    dim = q.data.shape[1]
-    gdt = q.data.dtype if grad_dtype is None else grad_dtype
-    gq = torch.empty((q.data.shape[0], dim), dtype=gdt, device=dev) if need_q else None
-    gd = torch.empty((d.data.shape[0], dim), dtype=gdt, device=dev) if need_d else None
-    n_pairs = 0 if pair_q is None else pair_q.numel()
-    ns = n_scores(pairing, q, d, n_pairs)
-    if ns == 0 or argmax.numel() == 0:
-        if gq is not None:
-            gq.zero_()
-        if gd is not None:
-            gd.zero_()
-        return gq, gd
-    g = grad_scores.contiguous().to(torch.float32).reshape(-1)
-    a = BwdArgs(
-        q=q.c_struct(), d=d.c_struct(), dtype=_lib.lik_dtype(q.data.dtype), dim=dim, pairing=pairing, group=group,
-        pair_q=_lib.ptr(pair_q), pair_d=_lib.ptr(pair_d), n_pairs=n_pairs, normalize=int(normalize),
-        deterministic=int(bool(deterministic)), grad_scores=g.data_ptr(), argmax=argmax.data_ptr(),
-        argmax_stride=argmax.shape[-1], grad_dtype=_lib.lik_dtype(gdt),
-        grad_q=_lib.ptr(gq) if (gq is not None and gq.numel()) else None,
-        grad_d=_lib.ptr(gd) if (gd is not None and gd.numel()) else None,
-        workspace=None, workspace_bytes=0, status=status_word(dev).data_ptr(),
-    )
-    nbytes = lib.lik_maxsim_bwd_workspace(C.byref(a))
-    ws = None
-    if nbytes:
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-        a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
-    with torch.cuda.device(dev):
-        _lib.check(lib.lik_maxsim_bwd(C.byref(a), _lib.stream_ptr(dev)), "lik_maxsim_bwd")
-    return gq, gd
+    return _lib.host().backward(q.native(), d.native(), grad_scores, argmax, pairing, group, pair_q, pair_d, int(normalize),
+                                bool(deterministic), grad_dtype, need_q, need_d)
 
 
 def _topk_rows_sorted(scores, k, largest, index_offset, out):

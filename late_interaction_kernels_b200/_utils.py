@@ -46,10 +46,3 @@ def common_dtype(Q: torch.Tensor, D: torch.Tensor) -> torch.dtype:
     if torch.bfloat16 in (Q.dtype, D.dtype):
         return torch.bfloat16
     return torch.float16
-
-
-def max_seqlen_from_cu(cu: torch.Tensor) -> int:
-    """Longest sequence in a cumulative-offset vector (one device->host sync)."""
-    if cu.numel() <= 1:
-        return 0
-    return int((cu[1:] - cu[:-1]).max().item())

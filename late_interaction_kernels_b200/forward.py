@@ -1,8 +1,8 @@
 """Fused MaxSim forward on padded ``[N, L, d]`` inputs.
 
 Host-side twin of the reference's ``forward.py``: same two entry points
-(``_run_forward`` for the autograd layer, ``maxsim_forward`` for callers that
-want scores and the optional argmax), same shapes and return conventions
+(``_run_forward`` and ``maxsim_forward``, for callers that want scores and the optional
+argmax outside autograd), same shapes and return conventions
 (forward.py:228-398).  The work is done by ``lik_maxsim_fwd``.
 """
 

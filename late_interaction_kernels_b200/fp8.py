@@ -100,10 +100,7 @@ def maxsim_inference_fp8(Q, D, *, scale_Q, scale_D, q_mask=None, d_mask=None):
             sd_tok = sd_tok * mult
         else:
             sq_tok = mult.expand(Nq, Lq).contiguous()
-    q = _ops.padded_spec(Q, q_mask, scale=sq_tok)
-    dd = _ops.padded_spec(D3, dm, scale=sd_tok)
-    scores, _ = _ops.forward(q, dd, pairing=_lib.PAIR_GROUPED if kd else _lib.PAIR_CROSS, group=nd_eff if kd else 0)
-    scores = scores.view(Nq, nd_eff)
+    scores = _ops.native_call(_lib.host().maxsim_fp8, Q, D3, sq_tok, sd_tok, q_mask, dm, nd_eff if kd else 0)
     if kd:
         return scores
     if q2 and d2:

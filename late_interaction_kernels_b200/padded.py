@@ -13,7 +13,6 @@ from dataclasses import dataclass
 import torch
 
 from . import _lib, _ops
-from ._utils import common_dtype
 
 
 @dataclass(frozen=True)
@@ -95,33 +94,6 @@ def pack_padded(queries, documents, query_lengths, doc_lengths, *, validate=Fals
     return PackedBatch(Q_packed, cu_q, D_packed, cu_d, pair_q.contiguous(), flat.contiguous(), int(max_q), int(max_d))
 
 
-class _MaxSimPaddedFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, queries, documents, qlen, dlen):
-        B, Lq, d = queries.shape
-        _, C, Ld, _ = documents.shape
-        dt = common_dtype(queries, documents)
-        q = _ops.padded_spec(queries.to(dt), lens=qlen)
-        dd = _ops.padded_spec(documents.to(dt).view(B * C, Ld, d), lens=dlen)
-        scores, argmax = _ops.forward(q, dd, pairing=_lib.PAIR_GROUPED, group=C, save_argmax=True, argmax_stride=Lq)
-        ctx.save_for_backward(queries, documents, qlen, dlen, argmax)
-        return scores.view(B, C)
-
-    @staticmethod
-    def backward(ctx, grad):
-        queries, documents, qlen, dlen, argmax = ctx.saved_tensors
-        B, Lq, d = queries.shape
-        _, C, Ld, _ = documents.shape
-        dt = common_dtype(queries, documents)
-        q = _ops.padded_spec(queries.to(dt), lens=qlen)
-        dd = _ops.padded_spec(documents.to(dt).view(B * C, Ld, d), lens=dlen)
-        gq, gd = _ops.backward(q, dd, grad, argmax, pairing=_lib.PAIR_GROUPED, group=C, deterministic=True, grad_dtype=dt,
-                               need_q=ctx.needs_input_grad[0], need_d=ctx.needs_input_grad[1])
-        gq = None if gq is None else gq.view(B, Lq, d).to(queries.dtype)
-        gd = None if gd is None else gd.view(B, C, Ld, d).to(documents.dtype)
-        return gq, gd, None, None
-
-
 def maxsim_padded(queries, documents, query_lengths, doc_lengths, *, validate=False):
     """Score ``C`` candidates per query from padded inputs -> fp32 ``[B, C]``; autograd-aware
     (padded.py:216-268).  Only the first ``query_lengths[b]`` / ``doc_lengths[b, c]`` tokens count;
@@ -138,14 +110,7 @@ def maxsim_padded(queries, documents, query_lengths, doc_lengths, *, validate=Fa
     dlen = doc_lengths.to(device=dev, dtype=torch.int32).contiguous().reshape(-1)
     if validate:
         _validate_lengths(qlen, dlen, Lq, Ld)
-    queries, documents = queries.contiguous(), documents.contiguous()
-    if torch.is_grad_enabled() and (queries.requires_grad or documents.requires_grad):
-        return _MaxSimPaddedFn.apply(queries, documents, qlen, dlen)
-    dt = common_dtype(queries, documents)
-    q = _ops.padded_spec(queries.to(dt), lens=qlen)
-    dd = _ops.padded_spec(documents.to(dt).view(B * C, Ld, d), lens=dlen)
-    scores, _ = _ops.forward(q, dd, pairing=_lib.PAIR_GROUPED, group=C)
-    return scores.view(B, C)
+    return _ops.native_call(_lib.host().maxsim_padded, queries, documents, qlen, dlen)
 
 
 __all__ = ["PackedBatch", "pack_padded", "maxsim_padded"]

@@ -9,10 +9,8 @@ device status word (``check_device_status()``) instead of a device-side assert, 
 
 from __future__ import annotations
 
-import torch
-
 from . import _lib, _ops
-from ._utils import common_dtype, max_seqlen_from_cu
+from ._utils import common_dtype
 
 
 def _check_packed(Q_packed, D_packed):
@@ -34,49 +32,17 @@ def _check_packed(Q_packed, D_packed):
 
 
 def _varlen_forward(Q_packed, D_packed, cu_seqlens_q, cu_seqlens_d, max_seqlen_q, max_seqlen_d, save_argmax):
-    """Returns ``(scores [Nq, Nd], argmax [Nq, Nd, max_q] | None, max_q, max_d)`` (varlen.py:271-364)."""
+    """Scores and winners outside autograd: ``(scores [Nq, Nd], argmax [Nq, Nd, max_q] | None, max_q, max_d)``
+    (varlen.py:271-364)."""
     _check_packed(Q_packed, D_packed)
     _lib.require_cuda(Q_packed, D_packed, cu_seqlens_q, cu_seqlens_d, op="maxsim_varlen")
-    cu_q = cu_seqlens_q.to(torch.int32).contiguous()
-    cu_d = cu_seqlens_d.to(torch.int32).contiguous()
-    Nq, Nd = cu_q.numel() - 1, cu_d.numel() - 1
-    # the longest query sizes the query tiles (and the saved argmax); like the reference it costs one
-    # device->host sync when the caller does not pass it.  The longest document is only needed by the backward.
-    max_q = max_seqlen_from_cu(cu_q) if max_seqlen_q is None else int(max_seqlen_q)
-    if save_argmax:
-        max_d = max_seqlen_from_cu(cu_d) if max_seqlen_d is None else int(max_seqlen_d)
-    else:
-        max_d = 0 if max_seqlen_d is None else int(max_seqlen_d)
     dt = common_dtype(Q_packed, D_packed)
-    q = _ops.packed_spec(Q_packed.to(dt), cu_q, max_q)
-    d = _ops.packed_spec(D_packed.to(dt), cu_d, max_d)
-    scores, argmax = _ops.forward(q, d, pairing=_lib.PAIR_CROSS, save_argmax=save_argmax, argmax_stride=max_q)
+    q = _ops.packed_spec(Q_packed.to(dt), cu_seqlens_q, max_seqlen_q)
+    d = _ops.packed_spec(D_packed.to(dt), cu_seqlens_d, max_seqlen_d)
+    scores, argmax = _ops.forward(q, d, pairing=_lib.PAIR_CROSS, save_argmax=save_argmax, argmax_stride=q.max_len)
     if argmax is not None:
-        argmax = argmax.view(Nq, Nd, max_q)
-    return scores.view(Nq, Nd), argmax, max_q, max_d
-
-
-class _MaxSimVarlenFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, Q, D, cu_q, cu_d, max_q, max_d):
-        scores, argmax, max_q, max_d = _varlen_forward(Q, D, cu_q, cu_d, max_q, max_d, save_argmax=True)
-        ctx.save_for_backward(Q, D, cu_q, cu_d, argmax)
-        ctx.max_q, ctx.max_d = max_q, max_d
-        return scores
-
-    @staticmethod
-    def backward(ctx, grad_scores):
-        Q, D, cu_q, cu_d, argmax = ctx.saved_tensors
-        dt = common_dtype(Q, D)
-        q = _ops.packed_spec(Q.to(dt), cu_q, ctx.max_q)
-        d = _ops.packed_spec(D.to(dt), cu_d, ctx.max_d)
-        gq, gd = _ops.backward(
-            q, d, grad_scores, argmax.view(-1, argmax.shape[-1]), pairing=_lib.PAIR_CROSS, deterministic=True,
-            grad_dtype=dt, need_q=ctx.needs_input_grad[0], need_d=ctx.needs_input_grad[1],
-        )
-        gq = None if gq is None else gq.to(Q.dtype)
-        gd = None if gd is None else gd.to(D.dtype)
-        return gq, gd, None, None, None, None
+        argmax = argmax.view(q.n_seq, d.n_seq, q.max_len)
+    return scores.view(q.n_seq, d.n_seq), argmax, q.max_len, d.max_len
 
 
 def maxsim_varlen(Q_packed, D_packed, cu_seqlens_q, cu_seqlens_d, max_seqlen_q=None, max_seqlen_d=None):
@@ -85,11 +51,7 @@ def maxsim_varlen(Q_packed, D_packed, cu_seqlens_q, cu_seqlens_d, max_seqlen_q=N
     Empty sequences score 0.  ``max_seqlen_q`` sizes the query tiles and the saved argmax, ``max_seqlen_d``
     the backward grid; when omitted they are read from ``cu_seqlens`` with one device->host sync (pass them
     to stay sync-free, e.g. under CUDA-graph capture)."""
-    if torch.is_grad_enabled() and (Q_packed.requires_grad or D_packed.requires_grad):
-        _check_packed(Q_packed, D_packed)
-        return _MaxSimVarlenFn.apply(
-            Q_packed.contiguous(), D_packed.contiguous(), cu_seqlens_q.to(torch.int32).contiguous(),
-            cu_seqlens_d.to(torch.int32).contiguous(), max_seqlen_q, max_seqlen_d,
-        )
-    scores, _, _, _ = _varlen_forward(Q_packed, D_packed, cu_seqlens_q, cu_seqlens_d, max_seqlen_q, max_seqlen_d, False)
-    return scores
+    _check_packed(Q_packed, D_packed)
+    _lib.require_cuda(Q_packed, D_packed, cu_seqlens_q, cu_seqlens_d, op="maxsim_varlen")
+    return _ops.native_call(_lib.host().maxsim_packed, Q_packed, D_packed, cu_seqlens_q, cu_seqlens_d, None, None,
+                            None if max_seqlen_q is None else int(max_seqlen_q), None if max_seqlen_d is None else int(max_seqlen_d))
