@@ -375,6 +375,7 @@ Tensor maxsim_fp8(const Tensor& Q, const Tensor& D, const OptTensor& q_scale, co
 }
 
 // ---- the launch helpers themselves, for the Python modules that describe their sides one by one ----
+}  // namespace
 Side side_of(const pybind11::tuple& t) {
   auto tensor = [&](int i) { return t[i].is_none() ? Tensor() : t[i].cast<Tensor>(); };
   Side s;
@@ -388,6 +389,7 @@ Side side_of(const pybind11::tuple& t) {
   s.scale = tensor(7);
   return s;
 }
+namespace {
 Pairing pairing_of(int kind, int64_t group, const OptTensor& pq, const OptTensor& pd) {
   Pairing p;
   p.kind = kind;
@@ -425,5 +427,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("maxsim_fp8", torch::wrap_pybind_function_no_gil(&maxsim_fp8));
   m.def("forward", torch::wrap_pybind_function(&forward_py));
   m.def("backward", torch::wrap_pybind_function(&backward_py));
+  bind_head(m);
+  bind_search(m);
   m.def("status_word", torch::wrap_pybind_function_no_gil(&status_tensor));
 }

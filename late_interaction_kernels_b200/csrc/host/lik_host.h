@@ -52,4 +52,10 @@ std::tuple<Tensor, Tensor> forward(const Side& q, const Side& d, const Pairing& 
 std::tuple<Tensor, Tensor> backward(const Side& q, const Side& d, const Pairing& p, const Tensor& grad_scores, const Tensor& argmax, int normalize,
                                     bool deterministic, at::ScalarType grad_dtype, bool need_q, bool need_d);
 
+// a side as the Python modules hand it over: (data, n_seq, max_len, seq_stride, cu, lens, mask, scale)
+Side side_of(const pybind11::tuple& t);
+
+void bind_head(pybind11::module_& m);
+void bind_search(pybind11::module_& m);
+
 }  // namespace lik_host

@@ -13,7 +13,7 @@ The backward works on the winning tokens alone: ``lik_hidden_winners`` turns the
 into a short "compact" document, those rows of ``H_d`` are gathered and projected again, the deterministic
 argmax-driven kernels (with the normalise Jacobian of the document side) produce the gradient of the projected rows,
 the three GEMMs of the linear layer run on those rows, and ``lik_hidden_scatter_rows`` writes ``grad_H`` in one pass
-(a winner's row or zeros).
+(a winner's row or zeros).  The chained path and the backward are native: ``csrc/host/lik_host_head.cpp``.
 """
 
 from __future__ import annotations
@@ -77,50 +77,9 @@ class _MaxSimFromHiddenFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_scores):
-        # Only winning tokens carry gradient (fused_head.py:332-456 gathers H_d at the winners too): the distinct winners
-        # of every document, in token order, form a short "compact" document of at most Nq * Lq tokens
-        # (lik_hidden_winners).  Those rows of H_d are gathered and projected again, the deterministic backward kernels
-        # run on the compact documents (with the document-side normalise Jacobian), the three GEMMs of the linear layer
-        # see the winner rows alone, and one pass writes grad_H: a winner's row or zeros (lik_hidden_scatter_rows).
-        # No host synchronisation; cost follows the winners, apart from that one pass over grad_H.
         Q, H_d, W, b, d_mask, argmax = ctx.saved_tensors
-        Nq, Lq, d_out = Q.shape
-        Nd, Ld, d_model = H_d.shape
-        dev = Q.device
-        dt = common_dtype(Q, H_d)
-        need_q, need_h, need_w, need_b = ctx.needs_input_grad[:4]
-        need_b = need_b and b is not None
-        need_d = need_h or need_w or need_b
-        g = grad_scores.contiguous().to(torch.float32)
-        S = max(1, min(Nq * Lq, Ld))  # slots of a compact document
-        am_c, rows, counts, bitmap, prefix = _ops.hidden_winners(argmax, Nq, Nd, Lq, Ld, S)
-        H_rows = H_d.reshape(Nd * Ld, d_model).index_select(0, rows)  # [Nd * S, d_model]
-        P_rows = _project(H_rows, W, b, dt)
-        q = _ops.padded_spec(Q.to(dt))
-        dd = _ops.padded_spec(P_rows.view(Nd, S, d_out), lens=counts)
-        norm = _lib.NORM_D if ctx.normalize else _lib.NORM_NONE
-        gq, gp = _ops.backward(q, dd, g, am_c.view(Nq * Nd, Lq), normalize=norm, deterministic=True, grad_dtype=torch.float32,
-                               need_q=need_q, need_d=need_d)  # gp: gradient w.r.t. the projected winner rows before normalisation
-        gQ = gq.view(Nq, Lq, d_out).to(Q.dtype) if need_q else None
-        gH = gW = gb = None
-        if need_d:
-            # 16-bit models: the linear layer's gradient GEMMs take 16-bit operands with fp32 accumulation, as its forward does
-            low = dt in (torch.bfloat16, torch.float16)
-            gpl = gp.to(dt) if low else gp
-            if need_h:
-                g_rows = (gpl @ (W.to(dt) if low else W.float())).to(H_d.dtype)
-                gH = torch.empty_like(H_d)
-                if (d_model * gH.element_size()) % 16 == 0:
-                    _ops.hidden_scatter_rows(g_rows, bitmap, prefix, gH.view(Nd * Ld, d_model), Nd, Ld, S)  # one pass, every row written once
-                else:
-                    gH.zero_()
-                    live = (torch.arange(S, device=dev).unsqueeze(0) < counts.unsqueeze(1)).reshape(-1)
-                    gH.view(Nd * Ld, d_model).index_copy_(0, rows[live], g_rows[live])
-            if need_w:
-                gW = (gpl.t() @ (H_rows.to(dt) if low else H_rows.float())).to(W.dtype)
-            if need_b:
-                gb = gp.sum(0).to(b.dtype)
-        return gQ, gH, gW, gb, None, None
+        gq, gh, gw, gb = _lib.host().hidden_backward(grad_scores, Q, H_d, W, b, argmax, ctx.normalize, *ctx.needs_input_grad[:4])
+        return gq, gh, gw, gb, None, None
 
 
 def maxsim_from_hidden(Q, H_d, W, b=None, d_mask=None, normalize=True):
@@ -146,15 +105,16 @@ def maxsim_from_hidden(Q, H_d, W, b=None, d_mask=None, normalize=True):
     if b is not None and (b.dim() != 1 or b.shape[0] != Q.shape[-1]):
         raise ValueError(f"b must be [d_out={Q.shape[-1]}]; got {tuple(b.shape)}")
     _lib.require_cuda(Q, H_d, W, op="maxsim_from_hidden")
-    Qc, Hc, Wc = Q.contiguous(), H_d.contiguous(), W.contiguous()
-    bc = None if b is None else b.contiguous()
-    mc = None if d_mask is None else d_mask.contiguous()
-    needs_grad = torch.is_grad_enabled() and (Qc.requires_grad or Hc.requires_grad or Wc.requires_grad or (bc is not None and bc.requires_grad))
-    if needs_grad:
-        scores = _MaxSimFromHiddenFn.apply(Qc, Hc, Wc, bc, mc, normalize)
-    else:
-        with torch.no_grad():
-            scores, _ = _forward(Qc, Hc, Wc, bc, mc, normalize, False)
+    scores = _ops.native_call(_lib.host().maxsim_from_hidden, Q, H_d, W, b, d_mask, normalize) if _CHAINED else None
+    if scores is None:  # not a problem of the chained kernel: project with a GEMM, piece by piece
+        Qc, Hc, Wc = Q.contiguous(), H_d.contiguous(), W.contiguous()
+        bc = None if b is None else b.contiguous()
+        mc = None if d_mask is None else d_mask.contiguous()
+        if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (Qc, Hc, Wc, bc)):
+            scores = _MaxSimFromHiddenFn.apply(Qc, Hc, Wc, bc, mc, normalize)
+        else:
+            with torch.no_grad():
+                scores, _ = _forward(Qc, Hc, Wc, bc, mc, normalize, False)
     return scores.squeeze(0) if q2 else scores
 
 

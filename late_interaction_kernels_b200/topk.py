@@ -14,7 +14,6 @@ from __future__ import annotations
 import torch
 
 from . import _lib, _ops
-from ._utils import common_dtype, ensure_contiguous_last
 from .forward import maxsim_forward
 
 
@@ -39,10 +38,7 @@ def maxsim_topk(Q, D, k, q_mask=None, d_mask=None, *, normalize=False, chunk_siz
     out = None
     with torch.no_grad():
         if Nd > 0 and Q.shape[0] > 0 and k <= _lib.TOPK_FUSED_MAX and Q.shape[-1] == D.shape[-1]:
-            dt = common_dtype(Q, D)
-            q = _ops.padded_spec(ensure_contiguous_last(Q).to(dt), q_mask)
-            dd = _ops.padded_spec(ensure_contiguous_last(D).to(dt), d_mask)
-            out = _ops.forward_fused(q, dd, normalize=_lib.NORM_BOTH if normalize else _lib.NORM_NONE, topk=k, largest=largest)
+            out = _ops.native_call(_lib.host().topk, Q, D, k, q_mask, d_mask, bool(normalize), bool(largest))
         for start in range(0, Nd if out is None else 0, max(step, 1)):
             end = min(start + step, Nd)
             dm = d_mask[start:end] if d_mask is not None else None
