@@ -174,6 +174,10 @@ __device__ __forceinline__ bool wait_bar(unsigned long long* bar, uint32_t parit
   if (mbar_try_wait(b, parity)) return true;
   return wait_bar_slow(b, parity, ctl, status);
 }
+// The same for all lanes of a warp: they leave together, with one answer.
+__device__ __forceinline__ bool wait_bar_warp(unsigned long long* bar, uint32_t parity, SharedCtl* ctl, int* status) {
+  return __all_sync(0xffffffffu, wait_bar(bar, parity, ctl, status));
+}
 // Bounded wait until the producer has published unit `uc` of this CTA in the unit ring.
 // Returns 1 when the unit is there, 2 when the stream has ended before it, 0 when the CTA is aborting.
 __device__ __noinline__ int wait_posted_slow(SharedCtl* ctl, int uc, int* status) {
@@ -638,89 +642,70 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
     }
   } else if (warp == 1) {
     // =========================== MMA issuer ===========================
-    // Driven by the stage words alone: between two MMA groups it runs a few dozen instructions, so the
-    // tensor pipe's queue never drains while work is available.
-    if (lane == 0) {
-      uint32_t st = 0, ph = 0, q_ph = 0, acc_ph = 0;  // acc_ph: one phase bit per accumulator
-      bool ok = true;
-      const uint32_t q_tile_desc = (uint32_t)(q_tile_bytes >> 4);
-      const uint32_t desc_hi = (uint32_t)(smem_desc_sw128(0) >> 32);
-      const uint32_t a_desc0 = (uint32_t)smem_desc_sw128(smem_u32(q_smem));
-      const uint32_t b_desc0 = (uint32_t)smem_desc_sw128(smem_u32(d_smem));
-      const uint32_t stage_desc = (uint32_t)(d_stage_bytes >> 4);
-      const uint32_t idesc0 = instr_desc(P.ab_format, 0);
-      const int k_steps = P.k_steps, n_slabs = P.n_slabs;
-      const uint32_t a_tile1 = P.mt == 2 ? q_tile_desc : 0u;  // descriptor offset of the second resident tile
-      uint32_t a_lo0[8], a_lo1[8];  // the eight K steps of either resident tile never move
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        a_lo0[k] = a_desc0 + (uint32_t)((k & 3) * 2 + (k >> 2) * ((TILE_M * SLAB_BYTES_ROW) >> 4));
-        a_lo1[k] = a_lo0[k] + a_tile1;
-      }
-      while (ok) {
-        ok = wait_bar(&ctl->d_full[st], ph, ctl, P.status);
+    // Driven by the stage words alone.  The whole warp runs the loop on warp-uniform values (the stage word is broadcast from
+    // lane 0, which also tells the compiler that it is uniform) and one elected lane issues: tcgen05.mma takes its
+    // descriptors from uniform registers, and with the loop under `lane == 0` every MMA paid about 100 cycles for moving
+    // them there, whatever its width.
+    uint32_t st = 0, ph = 0, q_ph = 0, acc_ph = 0;  // acc_ph: one phase bit per accumulator
+    bool ok = true;
+    const bool issue = elect_one();
+    const uint32_t desc_hi = (uint32_t)(smem_desc_sw128(0) >> 32);
+    const uint32_t a_desc0 = (uint32_t)smem_desc_sw128(smem_u32(q_smem));
+    const uint32_t b_desc0 = (uint32_t)smem_desc_sw128(smem_u32(d_smem));
+    const uint32_t stage_desc = (uint32_t)(d_stage_bytes >> 4);
+    const uint32_t a_tile1 = P.mt == 2 ? (uint32_t)(q_tile_bytes >> 4) : 0u;  // descriptor offset of the second resident tile
+    const uint32_t idesc0 = instr_desc(P.ab_format, 0);
+    const int k_steps = P.k_steps;
+    constexpr uint32_t A_SLAB = (TILE_M * SLAB_BYTES_ROW) >> 4, B_SLAB = (TILE_N * SLAB_BYTES_ROW) >> 4;
+    while (ok) {
+      ok = wait_bar_warp(&ctl->d_full[st], ph, ctl, P.status);
+      if (!ok) break;
+      const uint32_t info = __shfl_sync(0xffffffffu, ctl->stage_info[st], 0);
+      if (info & STAGE_END) break;
+      if (info & STAGE_FIRST) {
+        ok = wait_bar_warp(&ctl->q_full, q_ph, ctl, P.status);
         if (!ok) break;
-        const uint32_t info = ctl->stage_info[st];
-        if (info & STAGE_END) break;
-        if (info & STAGE_FIRST) {
-          ok = wait_bar(&ctl->q_full, q_ph, ctl, P.status);
-          if (!ok) break;
-          q_ph ^= 1;
-        }
-        const uint32_t ncols = info & STAGE_COLS_MASK;
-        {
-          const uint32_t idesc = idesc0 | (((ncols + 15) >> 4) << 18);  // N / 8 in bits 17..22
-          const uint32_t b_stage = b_desc0 + st * stage_desc;
-          uint32_t b_lo[8];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) b_lo[k] = b_stage + (uint32_t)((k & 3) * 2 + (k >> 2) * ((TILE_N * SLAB_BYTES_ROW) >> 4));
-#pragma unroll
-          for (int a = 0; a < 2; ++a) {
-            if (!(info & (STAGE_ACC0 << a))) continue;
-            ok = wait_bar(&ctl->acc_empty[a], ((acc_ph >> a) & 1u) ^ 1u, ctl, P.status);
-            if (!ok) break;
-            acc_ph ^= 1u << a;
-            tc_fence_after();
-            const uint32_t d_tmem = tmem_base + (uint32_t)(a * ACC_COLS);
-            // descriptors differ only in the 16-byte-unit start address: add offsets to a base descriptor
-            uint32_t a_desc = a_desc0 + a * a_tile1;
-            uint32_t b_desc = b_stage;
-            if (ncols == 0) {
-              // empty document: the accumulator still changes hands so that both sides keep their phase
-            } else if (k_steps == 8) {
-              // the common width (128 two-byte or 256 one-byte elements): straight-line issue from
-              // descriptor words prepared ahead of the accumulator wait
-              const uint32_t* al = a ? a_lo1 : a_lo0;
-              tc_mma<FP8>(d_tmem, al[0], b_lo[0], desc_hi, idesc, 0u);
-              tc_mma<FP8>(d_tmem, al[1], b_lo[1], desc_hi, idesc, 1u);
-              tc_mma<FP8>(d_tmem, al[2], b_lo[2], desc_hi, idesc, 1u);
-              tc_mma<FP8>(d_tmem, al[3], b_lo[3], desc_hi, idesc, 1u);
-              tc_mma<FP8>(d_tmem, al[4], b_lo[4], desc_hi, idesc, 1u);
-              tc_mma<FP8>(d_tmem, al[5], b_lo[5], desc_hi, idesc, 1u);
-              tc_mma<FP8>(d_tmem, al[6], b_lo[6], desc_hi, idesc, 1u);
-              tc_mma<FP8>(d_tmem, al[7], b_lo[7], desc_hi, idesc, 1u);
-            } else {
-              int left = k_steps;
-              uint32_t accum = 0;
-              for (int sl = 0; sl < n_slabs; ++sl) {
-                tc_mma<FP8>(d_tmem, a_desc, b_desc, desc_hi, idesc, accum);
-                accum = 1;
-                if (left > 1) tc_mma<FP8>(d_tmem, a_desc + 2, b_desc + 2, desc_hi, idesc, 1u);
-                if (left > 2) tc_mma<FP8>(d_tmem, a_desc + 4, b_desc + 4, desc_hi, idesc, 1u);
-                if (left > 3) tc_mma<FP8>(d_tmem, a_desc + 6, b_desc + 6, desc_hi, idesc, 1u);
-                left -= 4;
-                a_desc += (uint32_t)((TILE_M * SLAB_BYTES_ROW) >> 4);
-                b_desc += (uint32_t)((TILE_N * SLAB_BYTES_ROW) >> 4);
-              }
-            }
-            tc_commit(smem_u32(&ctl->acc_full[a]));
-          }
-          if (!ok) break;
-        }
-        tc_commit(smem_u32(&ctl->d_empty[st]));  // ring slot reusable once these MMAs retire
-        if (info & STAGE_LAST) tc_commit(smem_u32(&ctl->q_empty));  // and so are the query tiles
-        if (++st == (uint32_t)P.stages) { st = 0; ph ^= 1; }
+        q_ph ^= 1;
       }
+      const uint32_t ncols = info & STAGE_COLS_MASK;
+      const uint32_t idesc = idesc0 | (((ncols + 15) >> 4) << 18);  // N / 8 in bits 17..22
+      const uint32_t b_stage = b_desc0 + st * stage_desc;
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        if (!ok || !(info & (STAGE_ACC0 << a))) continue;
+        ok = wait_bar_warp(&ctl->acc_empty[a], ((acc_ph >> a) & 1u) ^ 1u, ctl, P.status);
+        if (!ok) continue;
+        acc_ph ^= 1u << a;
+        tc_fence_after();
+        if (issue) {
+          if (ncols) {  // (an empty document: the accumulator still changes hands so that both sides keep their phase)
+            const uint32_t d_tmem = tmem_base + (uint32_t)(a * ACC_COLS);
+            const uint32_t a_desc = a_desc0 + (a ? a_tile1 : 0u);
+            // descriptors differ only in the start address, in units of 16 bytes
+            if (k_steps == 8) {  // the common width (128 two-byte or 256 one-byte elements): straight-line issue
+#pragma unroll
+              for (int k = 0; k < 8; ++k)
+                tc_mma<FP8>(d_tmem, a_desc + (uint32_t)((k & 3) * 2) + (k >> 2) * A_SLAB, b_stage + (uint32_t)((k & 3) * 2) + (k >> 2) * B_SLAB, desc_hi,
+                            idesc, k ? 1u : 0u);
+            } else {
+#pragma unroll
+              for (int k = 0; k < 8; ++k)
+                if (k < k_steps)
+                  tc_mma<FP8>(d_tmem, a_desc + (uint32_t)((k & 3) * 2) + (k >> 2) * A_SLAB, b_stage + (uint32_t)((k & 3) * 2) + (k >> 2) * B_SLAB,
+                              desc_hi, idesc, k ? 1u : 0u);
+            }
+          }
+          tc_commit(smem_u32(&ctl->acc_full[a]));
+        }
+        __syncwarp();
+      }
+      if (!ok) break;
+      if (issue) {
+        tc_commit(smem_u32(&ctl->d_empty[st]));                     // ring slot reusable once these MMAs retire
+        if (info & STAGE_LAST) tc_commit(smem_u32(&ctl->q_empty));  // and so are the query tiles
+      }
+      __syncwarp();
+      if (++st == (uint32_t)P.stages) { st = 0; ph ^= 1; }
     }
   } else if (warp < 2 + 2 * GROUP_WARPS) {
     // =========================== epilogue groups ===========================
@@ -1125,6 +1110,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
   }
 
   // ---- teardown (also reached when aborting: every wait above is bounded) ----
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
