@@ -2,11 +2,10 @@
 #include <mutex>
 
 #include "lik_common.cuh"
+#include "lik_prep.cuh"
 #include "lik_tc.cuh"
 
 namespace lik {
-int launch_row_inv_norm(const void* data, int dtype, long long n_rows, int dim, long long stride, float eps, float* out,
-                        cudaStream_t st);
 int launch_row_normalize(const void* data, int dtype, long long n_rows, int dim, long long stride, float eps, void* out,
                          cudaStream_t st);
 int launch_fwd_generic(const lik_fwd_args& a, const float* qn, const float* dn, cudaStream_t st);
@@ -103,6 +102,7 @@ int run_fwd(const lik_fwd_args& a, const FwdPlan& pl, cudaStream_t st, const TcE
   int rc;
   lik_fwd_args b = a;
   const float *qn = nullptr, *dn = nullptr;
+  PrepJobs prep;
   if (a.normalize & LIK_NORM_Q) {
     if (pl.copies) {
       rc = launch_row_normalize(a.q.data, a.dtype, a.q.n_rows, a.dim, a.q.row_stride, kFwdNormEps, ws + pl.qcopy_off, st);
@@ -111,8 +111,7 @@ int run_fwd(const lik_fwd_args& a, const FwdPlan& pl, cudaStream_t st, const TcE
       b.q.row_stride = a.dim;
     } else {
       float* w = (float*)(ws + pl.qn_off);
-      rc = launch_row_inv_norm(a.q.data, a.dtype, a.q.n_rows, a.dim, a.q.row_stride, kFwdNormEps, w, st);
-      if (rc) return rc;
+      prep.norm[0] = norm_job(a.q, a.dtype, a.dim, kFwdNormEps, w, false);
       qn = w;
     }
   }
@@ -124,17 +123,18 @@ int run_fwd(const lik_fwd_args& a, const FwdPlan& pl, cudaStream_t st, const TcE
       b.d.row_stride = a.dim;
     } else {
       float* w = (float*)(ws + pl.dn_off);
-      rc = launch_row_inv_norm(a.d.data, a.dtype, a.d.n_rows, a.dim, a.d.row_stride, kFwdNormEps, w, st);
-      if (rc) return rc;
+      prep.norm[1] = norm_job(a.d, a.dtype, a.dim, kFwdNormEps, w, false);
       dn = w;
     }
   }
   b.normalize = pl.copies ? 0 : (a.normalize & LIK_NORM_BOTH);
-  if (pl.use_tc) return launch_fwd_tc(b, qn, dn, ws + pl.tc_off, fwd_tc_workspace(b, x), st, x);
+  if (pl.use_tc) return launch_fwd_tc(b, qn, dn, prep, ws + pl.tc_off, fwd_tc_workspace(b, x), st, x);
   if (x.plaid || x.topk_k > 0) {
     set_error("this problem is outside what the fused tensor-core path takes");
     return LIK_ERR_UNSUPPORTED;
   }
+  rc = launch_prep(prep, st);
+  if (rc) return rc;
   return launch_fwd_generic(b, qn, dn, st);
 }
 }  // namespace
@@ -322,7 +322,13 @@ extern "C" int lik_row_inv_norm(const void* data, int32_t dtype, int64_t n_rows,
   using namespace lik;
   LIK_REQUIRE(n_rows >= 0 && dim > 0 && row_stride >= dim, "bad shape");
   LIK_REQUIRE((data && out) || n_rows == 0, "NULL pointer");
-  return launch_row_inv_norm(data, dtype, n_rows, dim, row_stride, eps, out, (cudaStream_t)stream);
+  lik_seqs s{};
+  s.data = data;
+  s.n_rows = n_rows;
+  s.row_stride = row_stride;
+  PrepJobs prep;
+  prep.norm[0] = norm_job(s, dtype, dim, eps, out, true);
+  return launch_prep(prep, (cudaStream_t)stream);
 }
 
 extern "C" const char* lik_last_error(void) { return lik::get_error(); }

@@ -11,6 +11,7 @@
 #include <mutex>
 
 #include "lik_common.cuh"
+#include "lik_prep.cuh"
 #include "lik_sort.cuh"
 
 namespace lik {
@@ -851,7 +852,7 @@ constexpr int DD_UNROLL = LIK_DD_UNROLL;  // independent list entries in flight 
 struct DdSortOut {
   int2* pairs;            // [n_scores * lq] (query row, weight bits), grouped by document then token
   long long* tok_begin;   // [d.n_rows] first list entry of every document row
-  int* tok_cnt;           // [d.n_rows] list length (zero-initialised by the launcher)
+  int* tok_cnt;           // [d.n_rows] list length (cleared before the sort)
 };
 
 // Offsets of the winner sort.  In: hist[w][t] = winners of token t counted by warp w (n_hist of the CTA's n_warps warps
@@ -1369,9 +1370,6 @@ __global__ void __launch_bounds__(256) bwd_finalize_kernel(const float* __restri
   }
 }
 
-int launch_row_inv_norm(const void* data, int dtype, long long n_rows, int dim, long long stride, float eps, float* out,
-                        cudaStream_t st);
-
 // Sort keys of a pair list: the query and the document of every pair (a pair with an index out of range gets the key
 // one past the last sequence on both sides, so it sorts behind every run and no gradient kernel visits it), and the
 // pair index as the value that travels with them.
@@ -1617,7 +1615,6 @@ int run_bwd(const lik_bwd_args& a, BwdParams& P, const BwdPlan& pl, cudaStream_t
       O.pairs = (int2*)(ws + pl.pairs_off);
       O.tok_begin = (long long*)(ws + pl.begin_off);
       O.tok_cnt = (int*)(ws + pl.cnt_off);
-      LIK_CUDA_OK(cudaMemsetAsync(O.tok_cnt, 0, (size_t)a.d.n_rows * sizeof(int), st));
       const bool quads = a.argmax_stride % 4 == 0 && ((uintptr_t)a.argmax % 16) == 0;
       if (quads) {
         LIK_CUDA_OK(cudaFuncSetAttribute(bwd_dd_sort4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.sort_smem));
@@ -1726,17 +1723,21 @@ extern "C" int lik_maxsim_bwd(const lik_bwd_args* a, lik_stream_t stream) {
     return LIK_ERR_WORKSPACE;
   }
   const float *qn = nullptr, *dn = nullptr;
+  PrepJobs prep;
   if (a->normalize & LIK_NORM_Q) {
     float* w = (float*)((char*)a->workspace + pl.qn_off);
-    int rc = launch_row_inv_norm(a->q.data, a->dtype, a->q.n_rows, a->dim, a->q.row_stride, kBwdNormEps, w, st);
-    if (rc) return rc;
+    prep.norm[0] = norm_job(a->q, a->dtype, a->dim, kBwdNormEps, w, false);
     qn = w;
   }
   if (a->normalize & LIK_NORM_D) {
     float* w = (float*)((char*)a->workspace + pl.dn_off);
-    int rc = launch_row_inv_norm(a->d.data, a->dtype, a->d.n_rows, a->dim, a->d.row_stride, kBwdNormEps, w, st);
-    if (rc) return rc;
+    prep.norm[1] = norm_job(a->d, a->dtype, a->dim, kBwdNormEps, w, false);
     dn = w;
+  }
+  if (pl.sorted) prep.fill[0] = FillJob{(char*)a->workspace + pl.cnt_off, (size_t)a->d.n_rows * sizeof(int), 0};  // no winners yet
+  {
+    const int rc = launch_prep(prep, st);
+    if (rc) return rc;
   }
   BwdParams P;
   P.q = make_view(a->q, qn);

@@ -1162,30 +1162,6 @@ __global__ void list_units_kernel(SeqView q, SeqView d, const int* __restrict__ 
   tab[p] = t;
 }
 
-// Effective length of every padded document under its token mask: 1 + index of the last valid
-// token, tagged with LEN_FLAG_MASKED when the valid tokens are not exactly the prefix [0, length).
-__global__ void mask_lens_kernel(const unsigned char* __restrict__ mask, const int* __restrict__ lens, int n_seq, int max_len,
-                                 long long seq_stride, int* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (j >= n_seq) return;
-  int len0 = max_len;
-  if (lens) len0 = min(max(lens[j], 0), max_len);
-  const unsigned char* m = mask + (long long)j * seq_stride;
-  int last = -1, cnt = 0;
-  for (int t = lane; t < len0; t += 32)
-    if (m[t]) {
-      last = t;
-      ++cnt;
-    }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
-    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-  }
-  if (lane == 0) out[j] = (last + 1) | (cnt != last + 1 ? LEN_FLAG_MASKED : 0);
-}
-
 constexpr int PACK_MAX_QUERIES = 8192;  // offsets are staged in shared memory; larger batches use fixed groups
 
 // Greedy packing of ragged queries into 128-row tiles: a tile takes whole consecutive queries until the next
@@ -1404,14 +1380,6 @@ int make_tmap_rows(CUtensorMap* map, const void* data, int dtype, long long inne
   return make_map(map, s, dtype, (int)inner, box_rows);
 }
 bool tmap_available() { return get_encode_fn() != nullptr; }
-int launch_mask_lens(const unsigned char* mask, const int* lens, int n_seq, int max_len, long long seq_stride, int* out,
-                     cudaStream_t st) {
-  if (n_seq <= 0) return LIK_OK;
-  mask_lens_kernel<<<(unsigned)ceil_div(n_seq, 8), 256, 0, st>>>(mask, lens, n_seq, max_len, seq_stride, out), ::lik::count_launch();
-  LIK_CUDA_OK(cudaGetLastError());
-  return LIK_OK;
-}
-
 // The fused top-k needs fixed query slots (padded queries of at most 128 tokens) and k within the list size.
 bool fwd_tc_topk_supported(const lik_fwd_args& a, const TcExtra& x) {
   if (!tc_problem_ok(a, x.plaid != nullptr)) return false;
@@ -1482,7 +1450,7 @@ static cudaError_t allow_smem(size_t bytes) {
   return e;
 }
 
-int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, void* ws, size_t ws_bytes, cudaStream_t st,
+int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, PrepJobs prep, void* ws, size_t ws_bytes, cudaStream_t st,
                   const TcExtra& x) {
   TcPlan pl = plan_tc(a, x);
   if (pl.stages < 1) {
@@ -1569,8 +1537,7 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, void*
   if (a.d.mask && !a.d.cu) {
     // trim every document to its last valid token; only documents with holes pay for per-column masking
     int* eff = (int*)((char*)ws + w.lens);
-    mask_lens_kernel<<<(unsigned)ceil_div(a.d.n_seq, 8), 256, 0, st>>>(a.d.mask, a.d.lens, a.d.n_seq, a.d.max_len, a.d.seq_stride, eff), ::lik::count_launch();
-    LIK_CUDA_OK(cudaGetLastError());
+    prep.mask_lens = MaskLensJob{a.d.mask, a.d.lens, a.d.n_seq, a.d.max_len, a.d.seq_stride, eff};
     P.d.lens = eff;
     P.d_len_flagged = 1;
   }
@@ -1593,12 +1560,17 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, void*
     P.topk.doc_base = x.topk_doc_base;
     P.topk.n_lists = (int)w.n_lists;
     if (!(x.topk_flags & LIK_TOPK_CONTINUE))
-      LIK_CUDA_OK(cudaMemsetAsync(P.topk.hdr, 0, (size_t)w.n_lists * sizeof(int2), st));  // empty lists, no threshold
+      prep.fill[0] = FillJob{P.topk.hdr, (size_t)w.n_lists * sizeof(int2), 0};  // empty lists, no threshold
   }
   // positions of the saved argmax that no accumulator row covers (queries shorter than the stride)
   if (a.argmax && (a.q.cu || a.q.lens || a.argmax_stride > a.q.max_len))
-    LIK_CUDA_OK(cudaMemsetAsync(a.argmax, 0xFF,
-                                (size_t)n_scores_of(a.pairing, a.q.n_seq, a.d.n_seq, a.n_pairs) * a.argmax_stride * sizeof(int), st));
+    if ((uintptr_t)a.argmax & 15)
+      LIK_CUDA_OK(cudaMemsetAsync(a.argmax, 0xFF,
+                                  (size_t)n_scores_of(a.pairing, a.q.n_seq, a.d.n_seq, a.n_pairs) * a.argmax_stride * sizeof(int), st));
+    else
+      prep.fill[1] = FillJob{a.argmax, (size_t)n_scores_of(a.pairing, a.q.n_seq, a.d.n_seq, a.n_pairs) * a.argmax_stride * sizeof(int), -1};
+  rc = launch_prep(prep, st);
+  if (rc) return rc;
 
   const bool fp8 = a.dtype == LIK_E4M3;
   const bool argmax = a.argmax != nullptr;

@@ -661,7 +661,9 @@ extern "C" int lik_maxsim_hidden_fwd(const lik_hidden_fwd_args* args, lik_stream
   P.mask = a.h.mask;
   if (a.h.mask) {
     int* eff = (int*)a.workspace;
-    rc = launch_mask_lens(a.h.mask, a.h.lens, a.h.n_seq, a.h.max_len, a.h.seq_stride, eff, st);
+    PrepJobs prep;
+    prep.mask_lens = MaskLensJob{a.h.mask, a.h.lens, a.h.n_seq, a.h.max_len, a.h.seq_stride, eff};
+    rc = launch_prep(prep, st);
     if (rc) return rc;
     P.lens = eff;
     P.lens_flagged = 1;
