@@ -14,7 +14,7 @@ namespace {
 constexpr float kFwdNormEps = 1e-12f;
 
 struct FwdPlan {
-  size_t qn_off, dn_off, qcopy_off, dcopy_off, tc_off, total;
+  size_t qn_off, dn_off, qcopy_off, dcopy_off, tc_off, lens_off, total;
   bool use_tc;
   bool copies;  // fused normalisation through normalised operand copies instead of per-row multipliers
 };
@@ -63,7 +63,7 @@ FwdPlan plan_fwd(const lik_fwd_args& a, const TcExtra& x = TcExtra()) {
     off = align_up(off + bytes, 256);
     return o;
   };
-  pl.qn_off = pl.dn_off = pl.qcopy_off = pl.dcopy_off = pl.tc_off = (size_t)-1;
+  pl.qn_off = pl.dn_off = pl.qcopy_off = pl.dcopy_off = pl.tc_off = pl.lens_off = (size_t)-1;
   pl.copies = (a.normalize & LIK_NORM_ROUNDED) && (a.normalize & LIK_NORM_BOTH) && (a.dtype == LIK_BF16 || a.dtype == LIK_F16) &&
               !x.plaid;
   const size_t eb = dtype_size(a.dtype);
@@ -93,6 +93,8 @@ FwdPlan plan_fwd(const lik_fwd_args& a, const TcExtra& x = TcExtra()) {
     if (pl.copies) pl.dcopy_off = take((size_t)a.d.n_rows * a.dim * eb);
     else pl.dn_off = take((size_t)a.d.n_rows * 4);
   }
+  // the portable kernel trims masked documents too
+  if (!pl.use_tc && a.d.mask && !a.d.cu) pl.lens_off = take((size_t)a.d.n_seq * 4);
   pl.total = off;
   return pl;
 }
@@ -132,6 +134,11 @@ int run_fwd(const lik_fwd_args& a, const FwdPlan& pl, cudaStream_t st, const TcE
   if (x.plaid || x.topk_k > 0) {
     set_error("this problem is outside what the fused tensor-core path takes");
     return LIK_ERR_UNSUPPORTED;
+  }
+  if (pl.lens_off != (size_t)-1) {
+    int* eff = (int*)(ws + pl.lens_off);
+    prep.mask_lens = MaskLensJob{a.d.mask, a.d.lens, a.d.n_seq, a.d.max_len, a.d.seq_stride, eff, 0};
+    b.d.lens = eff;
   }
   rc = launch_prep(prep, st);
   if (rc) return rc;

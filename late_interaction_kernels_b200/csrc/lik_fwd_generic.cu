@@ -86,18 +86,18 @@ int launch_row_normalize(const void* data, int dtype, long long n_rows, int dim,
 // ---------------------------------------------------------------------------------
 // Exact forward: fp32 FMA in a fixed order.
 //
-// A CTA scores one document against QB queries (QB = 2 for the cross product, where both share the staged document; 1
-// otherwise).  Tile: 32 query tokens x 128 document tokens per query, four warps of 32 document tokens each; a thread owns
-// 4 query tokens x 8 document tokens and walks the width four features at a time: twelve 16-byte shared-memory loads feed
-// 64 two-wide FMAs (a feature pair of a row is a register pair as it is loaded, so nothing is packed; an accumulator holds
-// the sums over even and odd features, added at the end).  Rows are staged row-major with a pitch of KC + 4 floats: the
-// rows a warp's load touches lie four banks apart, no conflicts.  Warps whose tokens lie behind the document's end skip the
-// arithmetic.  Bound by the fp32 pipe: 32 queries x 32 documents of 36..180 tokens 91 -> 25 us (a thread per query token
-// and scalar FMAs fed by one 16-byte load per four of them before).
+// A CTA of four warps scores one document against QB queries (QB = 2 for the cross product, where both share the staged
+// document; 1 otherwise).  Tile: 32 query tokens of every query x up to 128 document tokens, a quarter per warp; a thread owns
+// 4 QB query tokens x up to 8 document tokens and walks the width four features at a time: with QB = 2, sixteen 16-byte
+// shared-memory loads feed 256 FMAs, the ratio at which both pipes are busy.  Rows are staged row-major with a pitch of
+// KC + 4 floats: the rows that a quarter-warp's load touches lie four banks apart.  Documents are trimmed to their last valid
+// token.  32 queries x 32 documents of 36..180 tokens: 91 -> 58 us (a thread per query token before, one 16-byte load per
+// four FMAs, padding multiplied); what is left beside the FMAs (23 us of issue) is the uneven documents: the slowest SM is a
+// third behind the mean.
 // ---------------------------------------------------------------------------------
 constexpr int G_QC = 32;   // query tokens per tile
 constexpr int G_DC = 128;  // document tokens per tile
-constexpr int G_KC = 128;  // features staged at once
+constexpr int G_KC = 64;   // features staged at once: 52 KB per CTA
 constexpr int G_PITCH = G_KC + 4;
 
 struct GenericFwdParams {
@@ -118,36 +118,61 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // rows [0, n) of a matrix, features [k0, k0 + kw) -> dst rows of G_PITCH floats; rows past `n` up to `rows` become zeros
 template <typename T>
-__device__ __forceinline__ void stage_rows(float* dst, const T* src, long long pitch, int rows, int n, int k0, int kw, bool vec16, int tid, int nt) {
-  if (sizeof(T) == 4 && vec16) {
-    const int per = kw >> 2;
-    for (int x = tid; x < rows * per; x += nt) {
-      const int r = x / per, c = (x - r * per) * 4;
+__device__ __forceinline__ void stage_rows(float* dst, const T* src, long long pitch, int rows, int n, int k0, int kw, bool vec16, int tid) {
+  const int lane = tid & 31;
+  if (sizeof(T) == 4 && vec16) {  // a warp per row, sixteen bytes per lane
+    const bool col = lane * 4 < kw;
+    const float* p = reinterpret_cast<const float*>(src) + k0 + lane * 4;
+    for (int r = tid >> 5; r < rows; r += 4) {
       const bool on = r < n;
-      cp_async16_zfill(dst + r * G_PITCH + c, reinterpret_cast<const float*>(src + (on ? r : 0) * pitch + k0 + c), on);
+      if (col) cp_async16_zfill(dst + r * G_PITCH + lane * 4, p + (on ? r : 0) * pitch, on);
     }
   } else {
     const int kp = (kw + 3) & ~3;
-    for (int x = tid; x < rows * kp; x += nt) {
-      const int r = x / kp, c = x - r * kp;
-      dst[r * G_PITCH + c] = (r < n && c < kw) ? to_f32(src[r * pitch + k0 + c]) : 0.f;
+    for (int r = tid >> 5; r < rows; r += 4)
+      for (int c = lane; c < kp; c += 32) dst[r * G_PITCH + c] = (r < n && c < kw) ? to_f32(src[r * pitch + k0 + c]) : 0.f;
+  }
+}
+
+// acc[i][t] += <query token i, document token t> over k_end staged features
+template <int QI, int TN>
+__device__ __forceinline__ void generic_tile(float (&acc)[QI][8], const float* qp, const float* dp, int k_end) {
+#pragma unroll 1
+  for (int k = 0; k < k_end; k += 4) {
+    float4 q4[QI];
+#pragma unroll
+    for (int i = 0; i < QI; ++i) q4[i] = *reinterpret_cast<const float4*>(qp + i * 8 * G_PITCH + k);
+#pragma unroll
+    for (int t = 0; t < TN; t += 2) {
+      float4 d4[2];
+      d4[0] = *reinterpret_cast<const float4*>(dp + t * 4 * G_PITCH + k);
+      d4[1] = *reinterpret_cast<const float4*>(dp + (t + 1) * 4 * G_PITCH + k);
+      // feature by feature, so that the FMAs of one accumulator stand apart
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int i = 0; i < QI; ++i)
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const float q = c == 0 ? q4[i].x : (c == 1 ? q4[i].y : (c == 2 ? q4[i].z : q4[i].w));
+            const float d = c == 0 ? d4[u].x : (c == 1 ? d4[u].y : (c == 2 ? d4[u].z : d4[u].w));
+            acc[i][t + u] = fmaf(q, d, acc[i][t + u]);
+          }
     }
   }
 }
 
-__device__ __forceinline__ void ffma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
-
 template <typename T, int QB>
-__global__ void __launch_bounds__(128 * QB, 2) fwd_generic_kernel(GenericFwdParams P) {
+__global__ void __launch_bounds__(128, 3) fwd_generic_kernel(GenericFwdParams P) {
   extern __shared__ __align__(16) float smem[];
   float* Qs = smem;                            // [QB][32 rows]
   float* Ds = smem + QB * G_QC * G_PITCH;      // [128 rows]
   __shared__ float red_m[QB][4][G_QC];
   __shared__ int red_i[QB][4][G_QC];
+  __shared__ float col_f[G_DC];  // multiplier of every document token of the tile; NaN: the token does not count
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) & 3, qb = tid >> 7;
+  constexpr int QI = 4 * QB;  // query tokens per thread: qg + 8 i of the staged 32 QB
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int qg = lane & 7, dg = lane >> 3;
   const T* __restrict__ Qg = (const T*)P.q.data;
   const T* __restrict__ Dg = (const T*)P.d.data;
@@ -187,78 +212,70 @@ __global__ void __launch_bounds__(128 * QB, 2) fwd_generic_kernel(GenericFwdPara
     }
     qmax = max(qmax, qlen[b]);
   }
-  const int my_qlen = QB == 1 ? qlen[0] : (qb ? qlen[QB - 1] : qlen[0]);
-  const long long my_qrow0 = QB == 1 ? qrow0[0] : (qb ? qrow0[QB - 1] : qrow0[0]);
-  const long long my_slot = QB == 1 ? slot[0] : (qb ? slot[QB - 1] : slot[0]);
-  const bool my_ok = QB == 1 || (qb ? ok[QB - 1] : ok[0]);
+  // the query that this warp sums at the end of a tile (warps 0 .. QB - 1)
+  const int mq = warp < QB ? warp : 0;
+  const int my_qlen = QB == 1 || mq == 0 ? qlen[0] : qlen[QB - 1];
+  const long long my_qrow0 = QB == 1 || mq == 0 ? qrow0[0] : qrow0[QB - 1];
+  const long long my_slot = QB == 1 || mq == 0 ? slot[0] : slot[QB - 1];
+  const bool my_ok = QB == 1 || mq == 0 ? ok[0] : ok[QB - 1];
 
-  float score = 0.f;  // meaningful in the query block's warp 0
+  float score = 0.f;  // meaningful in warps 0 .. QB - 1
   for (int qc = 0; qc < qmax; qc += G_QC) {
-    float m[4];
-    int mi[4];
+    float m[QI];
+    int mi[QI];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < QI; ++i) {
       m[i] = -INFINITY;
       mi[i] = -1;
     }
-    for (int dc = 0; dc < dlen; dc += G_DC) {
-      unsigned long long acc[4][8];
+    // the document in chunks of equal size, four warps with an equal part of a chunk each
+    const int n_chunk = (dlen + G_DC - 1) / G_DC;
+    const int per = n_chunk ? ((dlen + n_chunk - 1) / n_chunk + 31) & ~31 : 0;
+    const int T_n = per >> 4;  // document tokens per thread: 2, 4, 6 or 8
+    for (int dc = 0; dc < dlen; dc += per) {
+      float acc[QI][8];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < QI; ++i)
 #pragma unroll
-        for (int t = 0; t < 8; ++t) acc[i][t] = 0ull;
-      const int ncols = min(G_DC, dlen - dc);
-      const bool busy = warp * 32 < ncols && qc < my_qlen;
+        for (int t = 0; t < 8; ++t) acc[i][t] = 0.f;
+      const int ncols = min(per, dlen - dc);
       for (int kc = 0; kc < k_chunks; ++kc) {
         const int k0 = kc * G_KC, kw = min(G_KC, P.dim - k0);
         __syncthreads();
         if (dc == 0 || k_chunks > 1) {
 #pragma unroll
           for (int b = 0; b < QB; ++b)
-            stage_rows<T>(Qs + b * G_QC * G_PITCH, Qg + (qrow0[b] + qc) * P.q.row_stride, P.q.row_stride, G_QC, min(G_QC, qlen[b] - qc), k0, kw,
-                          P.vec16, tid, 128 * QB);
+            stage_rows<T>(Qs + b * G_QC * G_PITCH, Qg + (qrow0[b] + qc) * P.q.row_stride, P.q.row_stride, G_QC, min(G_QC, qlen[b] - qc), k0, kw, P.vec16, tid);
         }
-        stage_rows<T>(Ds, Dg + (drow0 + dc) * P.d.row_stride, P.d.row_stride, (ncols + 31) & ~31, ncols, k0, kw, P.vec16, tid, 128 * QB);
+        stage_rows<T>(Ds, Dg + (drow0 + dc) * P.d.row_stride, P.d.row_stride, per, ncols, k0, kw, P.vec16, tid);
+        if (kc == 0) {  // (one token per thread, in flight with the rows: read token by token behind the FMAs they cost more than those)
+          float f = __int_as_float(0x7fffffff);
+          if (tid < ncols && row_valid(P.d, drow0 + dc + tid)) f = row_factor(P.d, drow0 + dc + tid);
+          col_f[tid] = f;
+        }
         cp_async_wait_all();
         __syncthreads();
-        if (busy) {
-          const float* qp = Qs + qb * G_QC * G_PITCH + qg * G_PITCH;           // query tokens qg, qg + 8, ...
-          const float* dp = Ds + (warp * 32 + dg) * G_PITCH;                   // document tokens dg, dg + 4, ...
-          const int k_end = (kw + 3) & ~3;
-#pragma unroll 1
-          for (int k = 0; k < k_end; k += 4) {
-            ulonglong2 q4[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) q4[i] = *reinterpret_cast<const ulonglong2*>(qp + i * 8 * G_PITCH + k);
-#pragma unroll
-            for (int t = 0; t < 8; ++t) {
-              const ulonglong2 d4 = *reinterpret_cast<const ulonglong2*>(dp + t * 4 * G_PITCH + k);
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                ffma2(acc[i][t], q4[i].x, d4.x);
-                ffma2(acc[i][t], q4[i].y, d4.y);
-              }
-            }
-          }
-        }
+        const float* qp = Qs + qg * G_PITCH;                      // query tokens qg, qg + 8, ...
+        const float* dp = Ds + (warp * 4 * T_n + dg) * G_PITCH;   // document tokens dg, dg + 4, ...
+        const int k_end = (kw + 3) & ~3;
+        // straight-line code for every even count of document tokens: a test inside the loop keeps the FMAs of its two sides apart
+        if (T_n <= 2) generic_tile<QI, 2>(acc, qp, dp, k_end);
+        else if (T_n <= 4) generic_tile<QI, 4>(acc, qp, dp, k_end);
+        else if (T_n <= 6) generic_tile<QI, 6>(acc, qp, dp, k_end);
+        else generic_tile<QI, 8>(acc, qp, dp, k_end);
       }
-      if (busy) {
+      {
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
-          const int tok = dc + warp * 32 + dg + 4 * t;
-          if (tok < dlen) {
-            const long long row = drow0 + tok;
-            if (row_valid(P.d, row)) {
-              const float f = row_factor(P.d, row);
+          if (t >= T_n) break;
+          const int tok = dc + warp * 4 * T_n + dg + 4 * t;
+          const float f = col_f[warp * 4 * T_n + dg + 4 * t];
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const float2 a = *reinterpret_cast<const float2*>(&acc[i][t]);
-                const float v = (a.x + a.y) * f;
-                if (v > m[i]) {
-                  m[i] = v;
-                  mi[i] = tok;
-                }
-              }
+          for (int i = 0; i < QI; ++i) {
+            const float v = acc[i][t] * f;  // (a NaN beats nothing)
+            if (v > m[i]) {
+              m[i] = v;
+              mi[i] = tok;
             }
           }
         }
@@ -267,7 +284,7 @@ __global__ void __launch_bounds__(128 * QB, 2) fwd_generic_kernel(GenericFwdPara
     // combine the lanes that hold the same query tokens, then the warps (each saw other document tokens; ties: lower token)
     auto better = [](float wm, int wi, float bm, int bi) { return wi >= 0 && (bi < 0 || wm > bm || (wm == bm && wi < bi)); };
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < QI; ++i) {
 #pragma unroll
       for (int o = 8; o <= 16; o <<= 1) {
         const float wm = __shfl_xor_sync(0xffffffffu, m[i], o);
@@ -278,19 +295,19 @@ __global__ void __launch_bounds__(128 * QB, 2) fwd_generic_kernel(GenericFwdPara
         }
       }
       if (dg == 0) {
-        red_m[qb][warp][qg + 8 * i] = m[i];
-        red_i[qb][warp][qg + 8 * i] = mi[i];
+        red_m[i >> 2][warp][qg + 8 * (i & 3)] = m[i];
+        red_i[i >> 2][warp][qg + 8 * (i & 3)] = mi[i];
       }
     }
     __syncthreads();
-    if (warp == 0) {
-      float bm = red_m[qb][0][lane];
-      int bi = red_i[qb][0][lane];
+    if (warp < QB) {
+      float bm = red_m[mq][0][lane];
+      int bi = red_i[mq][0][lane];
 #pragma unroll
       for (int w = 1; w < 4; ++w)
-        if (better(red_m[qb][w][lane], red_i[qb][w][lane], bm, bi)) {
-          bm = red_m[qb][w][lane];
-          bi = red_i[qb][w][lane];
+        if (better(red_m[mq][w][lane], red_i[mq][w][lane], bm, bi)) {
+          bm = red_m[mq][w][lane];
+          bi = red_i[mq][w][lane];
         }
       const int s = qc + lane;
       float val = 0.f;
@@ -303,7 +320,7 @@ __global__ void __launch_bounds__(128 * QB, 2) fwd_generic_kernel(GenericFwdPara
     }
     __syncthreads();  // the next query tokens reuse the hand-over arrays
   }
-  if (warp == 0 && my_ok) {
+  if (warp < QB && my_ok) {
     if (lane == 0) P.scores[my_slot] = score;
     if (P.argmax)
       for (int s = max(my_qlen, 0) + lane; s < P.argmax_stride; s += 32) P.argmax[my_slot * P.argmax_stride + s] = -1;
@@ -326,7 +343,7 @@ static int launch_generic(const GenericFwdParams& P, cudaStream_t st) {
 #define LIK_LAUNCH_GENERIC(QB)                                                                                            \
   do {                                                                                                                    \
     LIK_CUDA_OK(cudaFuncSetAttribute(fwd_generic_kernel<T, QB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    fwd_generic_kernel<T, QB><<<(unsigned)grid, 128 * QB, smem, st>>>(P), ::lik::count_launch();                          \
+    fwd_generic_kernel<T, QB><<<(unsigned)grid, 128, smem, st>>>(P), ::lik::count_launch();                          \
   } while (0)
   if (cross) LIK_LAUNCH_GENERIC(2);
   else LIK_LAUNCH_GENERIC(1);

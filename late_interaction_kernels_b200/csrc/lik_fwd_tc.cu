@@ -1537,7 +1537,7 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, PrepJ
   if (a.d.mask && !a.d.cu) {
     // trim every document to its last valid token; only documents with holes pay for per-column masking
     int* eff = (int*)((char*)ws + w.lens);
-    prep.mask_lens = MaskLensJob{a.d.mask, a.d.lens, a.d.n_seq, a.d.max_len, a.d.seq_stride, eff};
+    prep.mask_lens = MaskLensJob{a.d.mask, a.d.lens, a.d.n_seq, a.d.max_len, a.d.seq_stride, eff, LEN_FLAG_MASKED};
     P.d.lens = eff;
     P.d_len_flagged = 1;
   }

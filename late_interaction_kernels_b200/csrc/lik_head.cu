@@ -662,7 +662,7 @@ extern "C" int lik_maxsim_hidden_fwd(const lik_hidden_fwd_args* args, lik_stream
   if (a.h.mask) {
     int* eff = (int*)a.workspace;
     PrepJobs prep;
-    prep.mask_lens = MaskLensJob{a.h.mask, a.h.lens, a.h.n_seq, a.h.max_len, a.h.seq_stride, eff};
+    prep.mask_lens = MaskLensJob{a.h.mask, a.h.lens, a.h.n_seq, a.h.max_len, a.h.seq_stride, eff, LEN_FLAG_MASKED};
     rc = launch_prep(prep, st);
     if (rc) return rc;
     P.lens = eff;

@@ -6,7 +6,6 @@
 // and load, every row.)  Small problems are launch-bound, hence everything in one grid: the jobs take consecutive ranges
 // of blocks.
 #include "lik_prep.cuh"
-#include "lik_tc.cuh"
 
 namespace lik {
 
@@ -185,7 +184,7 @@ __device__ __forceinline__ void mask_lens_block(const MaskLensJob& J, int block)
     last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
     cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
   }
-  if (lane == 0) J.out[j] = (last + 1) | (cnt != last + 1 ? LEN_FLAG_MASKED : 0);
+  if (lane == 0) J.out[j] = (last + 1) | (cnt != last + 1 ? J.flag : 0);
 }
 
 __device__ __forceinline__ void fill_block(const FillJob& J, int block) {

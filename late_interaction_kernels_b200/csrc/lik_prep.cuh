@@ -17,12 +17,13 @@ struct NormJob {  // out[r] = 1 / max(||x_r||, eps); rows that no valid token si
   float* out = nullptr;
 };
 
-struct MaskLensJob {  // out[j] = (1 + last valid token) | LEN_FLAG_MASKED when the valid tokens are not a prefix
+struct MaskLensJob {  // out[j] = 1 + last valid token, tagged with `flag` when the valid tokens are not a prefix
   const unsigned char* mask = nullptr;  // nullptr: no job
   const int* lens = nullptr;
   int n_seq = 0, max_len = 0;
   long long seq_stride = 0;
   int* out = nullptr;
+  int flag = 0;  // or-ed into out[j] when the mask has holes
 };
 
 struct FillJob {  // whole 32-bit words, 16-byte aligned
