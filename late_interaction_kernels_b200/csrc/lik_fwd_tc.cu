@@ -1393,7 +1393,7 @@ bool fwd_tc_plaid_supported(const lik_fwd_args& a, const TcExtra& x) {
   return plaid_row16_ok(*x.plaid);
 }
 
-int topk_merge_parts(int n_ctas, int n_groups);
+int topk_merge_parts(int n_ctas, int n_groups, int mt);
 
 namespace {
 struct TcWs {
@@ -1418,8 +1418,8 @@ TcWs tc_ws_layout(const TcPlan& pl, const lik_fwd_args& a, const TcExtra& x) {
     w.keys = take((size_t)w.n_lists * TOPK_CAP * sizeof(float));
     w.idx = take((size_t)w.n_lists * TOPK_CAP * sizeof(int));
     // few tile groups: a query has lists from many CTAs, which are merged in parts by as many CTAs first
-    w.merge_parts = topk_merge_parts(pl.grid, pl.n_groups);
-    w.merge = take(w.merge_parts > 1 ? (size_t)w.merge_parts * a.q.n_seq * x.topk_k * (sizeof(float) + sizeof(long long)) + 8 : 0);
+    w.merge_parts = topk_merge_parts(pl.grid, pl.n_groups, pl.mt);
+    w.merge = take(w.merge_parts > 1 ? (size_t)w.merge_parts * a.q.n_seq * x.topk_k * sizeof(long long) : 0);
   }
   w.partial = take(pl.q_chunks > 1 ? (size_t)pl.n_tiles * a.d.n_seq * sizeof(float) : 0);
   w.lens = take((a.d.mask && !a.d.cu) ? (size_t)a.d.n_seq * sizeof(int) : 0);

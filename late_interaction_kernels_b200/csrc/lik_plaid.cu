@@ -90,11 +90,11 @@ __global__ void __launch_bounds__(256) plaid_decompress_kernel(PlaidView v, long
 // 16-byte centroid loads, one load for a lane's eight bucket codes, 16-byte stores.
 constexpr int PD_RUN = 64;  // consecutive tokens per half-warp
 
-template <typename O, bool CF32>
+template <typename O, bool CF32, bool CBF16, int NBITS>
 __global__ void __launch_bounds__(256) plaid_decompress16_kernel(PlaidSrc S, long long tok0, long long count, O* __restrict__ out,
                                                                int* status) {
-  __shared__ float bw[256];
-  for (int b = threadIdx.x; b < (1 << S.nbits); b += blockDim.x) bw[b] = S.bucket_weights[b];
+  __shared__ __align__(16) float tab[PlaidTable<NBITS>::WORDS];
+  PlaidTable<NBITS>::fill(tab, S.bucket_weights, threadIdx.x, blockDim.x);
   __syncthreads();
   const int lane = threadIdx.x & 31, hl = lane & 15;
   const long long first = ((long long)blockIdx.x * 16 + (threadIdx.x >> 4)) * PD_RUN;  // first token of this half-warp's run
@@ -111,7 +111,22 @@ __global__ void __launch_bounds__(256) plaid_decompress16_kernel(PlaidSrc S, lon
       *reinterpret_cast<uint4*>(p) = plaid_pack16(e, dtype_of<O>::value == LIK_F16);
     }
   };
-  plaid_decode_range<CF32, CF32 ? 4 : 8>(S, bw, tok0 + first, n, PD_RUN, lane, hl * 8 < dim, status, sink);
+  plaid_decode_run<CF32, CBF16, NBITS>(S, tab, tok0 + first, n, tok0 + count - 1, PD_RUN, lane, hl * 8 < dim, status, sink);
+}
+
+template <typename O>
+static void launch_decompress16(const PlaidSrc& S, long long tok0, long long count, O* out, int* status, cudaStream_t st) {
+  const unsigned blocks = (unsigned)ceil_div(count, 16 * PD_RUN);
+#define LIK_DEC16(CF, CB)                                                                                                                  \
+  do {                                                                                                                                     \
+    if (S.nbits == 2) plaid_decompress16_kernel<O, CF, CB, 2><<<blocks, 256, 0, st>>>(S, tok0, count, out, status), ::lik::count_launch(); \
+    else if (S.nbits == 4) plaid_decompress16_kernel<O, CF, CB, 4><<<blocks, 256, 0, st>>>(S, tok0, count, out, status), ::lik::count_launch(); \
+    else plaid_decompress16_kernel<O, CF, CB, 8><<<blocks, 256, 0, st>>>(S, tok0, count, out, status), ::lik::count_launch();              \
+  } while (0)
+  if (S.centroid_dtype == LIK_F32) LIK_DEC16(true, false);
+  else if (S.centroid_dtype == LIK_BF16) LIK_DEC16(false, true);
+  else LIK_DEC16(false, false);
+#undef LIK_DEC16
 }
 
 // Approximate score: one warp per document, lane = query token (chunks of 32).  The document's codes are read 32
@@ -256,22 +271,9 @@ extern "C" int lik_plaid_decompress(const lik_plaid_index* index, int64_t token_
     PlaidSrc S{index->codes, index->residuals, index->centroids, index->bucket_weights, index->centroid_dtype, index->n_centroids,
                index->nbits, v.packed_dim, index->dim, normalize ? 1 : 0};
     if (plaid_row16_ok(S) && ((uintptr_t)out % 16) == 0 && (out_dtype == LIK_F32 || out_dtype == LIK_F16 || out_dtype == LIK_BF16)) {
-      const unsigned blocks = (unsigned)ceil_div(token_count, 16 * PD_RUN);
-      const bool cf32 = index->centroid_dtype == LIK_F32;
-#define LIK_DEC16(O)                                                                                                  \
-  do {                                                                                                                \
-    if (cf32)                                                                                                         \
-      plaid_decompress16_kernel<O, true><<<blocks, 256, 0, st>>>(S, token_begin, token_count, (O*)out, status), ::lik::count_launch(); \
-    else                                                                                                              \
-      plaid_decompress16_kernel<O, false><<<blocks, 256, 0, st>>>(S, token_begin, token_count, (O*)out, status), ::lik::count_launch(); \
-  } while (0)
-      if (out_dtype == LIK_F32)
-        LIK_DEC16(float);
-      else if (out_dtype == LIK_F16)
-        LIK_DEC16(__half);
-      else
-        LIK_DEC16(__nv_bfloat16);
-#undef LIK_DEC16
+      if (out_dtype == LIK_F32) launch_decompress16<float>(S, token_begin, token_count, (float*)out, status, st);
+      else if (out_dtype == LIK_F16) launch_decompress16<__half>(S, token_begin, token_count, (__half*)out, status, st);
+      else launch_decompress16<__nv_bfloat16>(S, token_begin, token_count, (__nv_bfloat16*)out, status, st);
       LIK_CUDA_OK(cudaGetLastError());
       return LIK_OK;
     }

@@ -147,6 +147,151 @@ __device__ __forceinline__ void plaid_decode_range(const PlaidSrc& S, const floa
   }
 }
 
+// The same arithmetic (bit for bit) with everything that varies between indexes known at compile time, for the stand-alone
+// decompress kernel.  What the form above spends its instructions on - 64-bit shifts by a run-time width per feature, a
+// table look-up per feature, a square root and a division on all sixteen lanes for every token, a branch per load - goes:
+// two-bit codes are looked up in pairs (a sixteen-entry table of two floats: one shared-memory bank per word, so no lookup
+// conflicts), the norms of four tokens are reduced together (each lane ends with one token's sum and takes one root), and
+// loads behind the run's end are clamped to its last token instead of branched around.
+template <int NBITS>
+struct PlaidTable {
+  static constexpr int WORDS = NBITS == 2 ? 32 : (1 << NBITS);  // floats in shared memory
+  // bw: the 2^NBITS weights
+  static __device__ __forceinline__ void fill(float* tab, const float* bw, int tid, int nt) {
+    if (NBITS == 2) {
+      for (int x = tid; x < 32; x += nt) tab[x] = bw[(x & 1) ? (x >> 3) & 3 : (x >> 1) & 3];  // entry x / 2 = code | next code << 2
+    } else {
+      for (int x = tid; x < (1 << NBITS); x += nt) tab[x] = bw[x];
+    }
+  }
+};
+
+template <bool CF32, int NBITS>
+struct PlaidPiece {  // one lane's part of a token as it is loaded
+  uint4 c0, c1;      // centroid (c1: fp32 centroids only)
+  unsigned w0, w1;   // residual codes (w1: eight-bit codes only)
+};
+
+template <bool CF32, int NBITS>
+__device__ __forceinline__ PlaidPiece<CF32, NBITS> plaid_piece(const PlaidSrc& S, long long tok, int code, int hl) {
+  PlaidPiece<CF32, NBITS> r;
+  const long long off = (long long)code * S.dim + hl * 8;
+  if constexpr (CF32) {
+    const uint4* p = reinterpret_cast<const uint4*>(static_cast<const float*>(S.centroids) + off);
+    r.c0 = __ldg(p);
+    r.c1 = __ldg(p + 1);
+  } else {
+    r.c0 = __ldg(reinterpret_cast<const uint4*>(static_cast<const unsigned short*>(S.centroids) + off));
+  }
+  const unsigned char* rp = S.residuals + tok * S.packed_dim + hl * NBITS;
+  if constexpr (NBITS == 2) r.w0 = __ldg(reinterpret_cast<const unsigned short*>(rp));
+  else if constexpr (NBITS == 4) r.w0 = __ldg(reinterpret_cast<const unsigned*>(rp));
+  else {
+    const uint2 w = __ldg(reinterpret_cast<const uint2*>(rp));
+    r.w0 = w.x;
+    r.w1 = w.y;
+  }
+  return r;
+}
+
+template <bool CF32, bool CBF16, int NBITS>
+__device__ __forceinline__ void plaid_values(const PlaidPiece<CF32, NBITS>& r, const float* tab, float (&e)[8]) {
+  if constexpr (CF32) {
+    e[0] = __uint_as_float(r.c0.x); e[1] = __uint_as_float(r.c0.y); e[2] = __uint_as_float(r.c0.z); e[3] = __uint_as_float(r.c0.w);
+    e[4] = __uint_as_float(r.c1.x); e[5] = __uint_as_float(r.c1.y); e[6] = __uint_as_float(r.c1.z); e[7] = __uint_as_float(r.c1.w);
+  } else {
+    const unsigned w[4] = {r.c0.x, r.c0.y, r.c0.z, r.c0.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if constexpr (CBF16) {
+        e[2 * i] = __uint_as_float(w[i] << 16);
+        e[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+      } else {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+        e[2 * i] = v.x;
+        e[2 * i + 1] = v.y;
+      }
+    }
+  }
+  if constexpr (NBITS == 2) {
+    const char* t = reinterpret_cast<const char*>(tab);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const unsigned at = i == 0 ? (r.w0 << 3) & 0x78u : (r.w0 >> (4 * i - 3)) & 0x78u;  // eight bytes per entry
+      const float2 v = *reinterpret_cast<const float2*>(t + at);
+      e[2 * i] += v.x;
+      e[2 * i + 1] += v.y;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const unsigned c = NBITS == 4 ? (r.w0 >> (4 * i)) & 15u : ((i < 4 ? r.w0 : r.w1) >> (8 * (i & 3))) & 255u;
+      e[i] += tab[c];
+    }
+  }
+}
+
+// `n` >= 0 consecutive tokens from tok0 for each of the two half-warps of a warp (their own tok0 and n); `last` is a token
+// that may be read when a half-warp has none.  n_uniform: at least either n, a multiple of 4.
+template <bool CF32, bool CBF16, int NBITS, typename Sink>
+__device__ __forceinline__ void plaid_decode_run(const PlaidSrc& S, const float* tab, long long tok0, int n, long long last, int n_uniform, int lane,
+                                                 bool lane_on, int* status, Sink sink) {
+  constexpr int U = 4;
+  const int hl = lane & 15, ll = lane_on ? hl : 0;
+  const long long end = n > 0 ? tok0 + n - 1 : last;
+  auto at = [&](int t) -> long long { return t < n ? tok0 + t : end; };
+  int code_next = plaid_code(S, at(hl), status);
+  PlaidPiece<CF32, NBITS> nx[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) nx[u] = plaid_piece<CF32, NBITS>(S, at(u), __shfl_sync(0xffffffffu, code_next, (lane & 16) | u), ll);
+  for (int c0 = 0; c0 < n_uniform; c0 += 16) {
+    const int code_cur = code_next;
+    code_next = plaid_code(S, at(c0 + 16 + hl), status);
+#pragma unroll 1
+    for (int b = 0; b < 16; b += U) {
+      PlaidPiece<CF32, NBITS> cur[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) cur[u] = nx[u];
+      // the next four tokens' rows are on their way while these four are finished
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int code = b + U < 16 ? __shfl_sync(0xffffffffu, code_cur, (lane & 16) | ((b + U + u) & 15)) : __shfl_sync(0xffffffffu, code_next, (lane & 16) | u);
+        nx[u] = plaid_piece<CF32, NBITS>(S, at(c0 + b + U + u), code, ll);
+      }
+      float e[U][8], ss[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        plaid_values<CF32, CBF16, NBITS>(cur[u], tab, e[u]);
+        ss[u] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ss[u] = fmaf(e[u][i], e[u][i], ss[u]);
+        if (!lane_on) ss[u] = 0.f;
+      }
+      float inv[U];
+      if (S.normalize) {
+        // (the sums pair lanes 8, 4, 2 and 1 apart, in that order, as the one-token reduction does)
+        const bool h8 = hl & 8, h4 = hl & 4;
+        const float a0 = (h8 ? ss[2] : ss[0]) + __shfl_xor_sync(0xffffffffu, h8 ? ss[0] : ss[2], 8);
+        const float a1 = (h8 ? ss[3] : ss[1]) + __shfl_xor_sync(0xffffffffu, h8 ? ss[1] : ss[3], 8);
+        float t = (h4 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, h4 ? a0 : a1, 4);
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        t += __shfl_xor_sync(0xffffffffu, t, 1);
+        const float mine = 1.f / fmaxf(sqrtf(t), 1e-12f);  // of token 2 * (bit 3) + (bit 2)
+#pragma unroll
+        for (int u = 0; u < U; ++u) inv[u] = __shfl_sync(0xffffffffu, mine, (lane & 16) | ((u >> 1) << 3) | ((u & 1) << 2));
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (S.normalize) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) e[u][i] *= inv[u];
+        }
+        if (c0 + b + u < n && lane_on) sink(c0 + b + u, e[u]);
+      }
+    }
+  }
+}
+
 // eight fp32 values -> eight 16-bit operand values (bf16 or fp16), round to nearest even
 __device__ __forceinline__ uint4 plaid_pack16(const float (&v)[8], bool f16) {
   uint4 o;

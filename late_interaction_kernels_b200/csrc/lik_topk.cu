@@ -161,151 +161,207 @@ __global__ void __launch_bounds__(NT, MIN_CTAS) topk_kernel(TopkParams P) {
 }
 
 // Merge of the candidate lists the fused scoring kernel leaves (lik_fwd_tc.cu): list slot of (CTA c, tile
-// group g) is c + g, each slot holds 2 * qpt lists of up to `cap` entries (unsorted), and CTA c of n_ctas can
+// group g) is c + g, each slot holds 2 * qpt lists of up to 256 entries (unsorted), and CTA c of n_ctas can
 // only have worked on the groups [n_groups * c / n_ctas, n_groups * (c + 1) / n_ctas] (a superset of the ones
 // it really met; lists it never touched are empty).  A group is `mt` query tiles of `qpt` queries; with two
 // tiles a query has one list per slot (tile * qpt + position), with one tile it has two (the kernel's two
-// epilogue groups take alternate documents).  One CTA per (query, part): with few tile groups a query has lists
-// from many CTAs, which would make one CTA walk hundreds of lists one after the other, so the CTAs' range is cut
-// in `parts` parts merged side by side into [parts, n_q, k] lists, and the plain list merge (topk_kernel) makes
-// the answer from those.
+// epilogue groups take alternate documents).
+//
+// An entry becomes one 64-bit number, larger = better: the score's ordered key above the complement of the document
+// index, so that ties need no second look.  A CTA holds the entries of up to 32 lists in registers (sixteen per thread),
+// finds the k-th largest by bisection on the bits with a block-wide count per bit - neighbouring scores share their upper
+// bits, on which a radix histogram's counters collide - and sorts the k survivors.  A query with more lists (few tile
+// groups: lists from every CTA) is cut in parts, whose winners go through the same selection once more.  One query over
+// 25 000 documents, 296 lists: 91 -> 15 us (list after list through bitonic merges before).
+typedef unsigned long long u64;
+constexpr int SLOT_CAP = 256;     // entries of a candidate list
+constexpr int SLOT_LISTS = 32;    // lists per CTA
+constexpr int SLOT_T = 512;
+constexpr int SLOT_PER = SLOT_LISTS * SLOT_CAP / SLOT_T;
+constexpr int SLOT_K = 128;       // largest k of the fused path
+
 struct SlotParams {
   const float* keys;
   const int* idx;
   const int2* hdr;
-  int cap, n_ctas, n_groups, mt, qpt;
+  int n_ctas, n_groups, mt, qpt;
   long long n_q, index_offset, n_lists;
-  int k, KP, largest;
+  int k, largest;
   float* out_scores;
   long long* out_index;
-  int parts;  // > 1: blockIdx.y is the part, the outputs are [parts, n_q, k] and carry keys' signs undone
+  int parts;   // lists of a query are merged in this many parts first ...
+  u64* part;   // ... into [parts, n_q, k] entries (0: none)
 };
 
-constexpr int SLOT_W = 256;  // merge width: the capacity of a candidate list, and the block size
+__device__ __forceinline__ unsigned slot_order(float f) {
+  const unsigned u = __float_as_uint(f);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float slot_unorder(unsigned k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k); }
 
-// The kept list (SLOT_W entries, best first; the first k are the answer so far) absorbs the pending block.
-__device__ void slots_flush(float* top_k, long long* top_i, float* blk_k, long long* blk_i, int n_pend, int tid) {
-  if (tid >= n_pend) {
-    blk_k[tid] = -INFINITY;
-    blk_i[tid] = kPadIdx;
-  }
-  bitonic_sort(blk_k, blk_i, SLOT_W, tid, SLOT_W);
-  {
-    Cand a{top_k[tid], top_i[tid]}, c{blk_k[SLOT_W - 1 - tid], blk_i[SLOT_W - 1 - tid]};
-    if (before(c, a)) {
-      top_k[tid] = c.key;
-      top_i[tid] = c.idx;
+// The k largest of the block's entries (0: none), written to out[0 .. n) in shared memory, best first; returns n.
+__device__ int slot_select(const u64 (&e)[SLOT_PER], int k, u64* out, int* cnt) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int WARPS = SLOT_T / 32;
+  // block-wide count of the entries at or above a bound (cnt: two rows of WARPS words, used in turn)
+  int turn = 0;
+  auto count_ge = [&](u64 bound) {
+    int c = 0;
+#pragma unroll
+    for (int j = 0; j < SLOT_PER; ++j) c += e[j] >= bound ? 1 : 0;
+    c = __reduce_add_sync(0xffffffffu, c);
+    int* row = cnt + (turn & 1) * WARPS;
+    ++turn;
+    if (lane == 0) row[warp] = c;
+    __syncthreads();
+    return __reduce_add_sync(0xffffffffu, lane < WARPS ? row[lane] : 0);
+  };
+  u64 kth = 1;
+  const int total = count_ge(1);
+  if (total > k) {
+    kth = 0;
+    for (int bit = 63; bit >= 0; --bit) {
+      const u64 cand = kth | (1ull << bit);
+      const int c = count_ge(cand);
+      if (c >= k) kth = cand;
+      if (c == k) break;  // exactly the k best lie at or above it
     }
   }
-  bitonic_merge(top_k, top_i, SLOT_W, tid, SLOT_W);
+  const int n = total < k ? total : k;
+  int* fill = cnt + 2 * WARPS;
+  if (tid == 0) *fill = 0;
+  for (int t = tid; t < SLOT_K; t += SLOT_T) out[t] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < SLOT_PER; ++j)
+    if (e[j] >= kth && e[j] != 0) {
+      const int pos = atomicAdd(fill, 1);
+      if (pos < SLOT_K) out[pos] = e[j];
+    }
+  int KP = 2;
+  while (KP < n) KP <<= 1;
+  for (int size = 2; size <= KP; size <<= 1)
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      __syncthreads();
+      if (tid < (KP >> 1)) {
+        const int i = 2 * tid - (tid & (stride - 1)), j = i + stride;
+        const bool up = (i & size) == 0;
+        const u64 a = out[i], b = out[j];
+        if (up ? b > a : a > b) {
+          out[i] = b;
+          out[j] = a;
+        }
+      }
+    }
+  __syncthreads();
+  return n;
 }
 
-// One CTA of SLOT_W threads per query.  Every list of the query is read once (one entry per thread); only
-// entries that beat the current k-th best are collected, and the collected block is sorted and merged when it
-// would overflow.  After the first list few entries survive the filter, so the sorts are rare.
-__global__ void __launch_bounds__(SLOT_W) topk_slots_kernel(SlotParams P) {
-  __shared__ long long top_i[SLOT_W], blk_i[SLOT_W];
-  __shared__ float top_k[SLOT_W], blk_k[SLOT_W];
-  __shared__ int n_pend_s;
-  const int tid = threadIdx.x, lane = tid & 31;
+__device__ __forceinline__ void slot_write(const SlotParams& P, long long q, const u64* top, int n) {
+  const float sgn = P.largest ? 1.f : -1.f;
+  for (int t = threadIdx.x; t < P.k; t += SLOT_T) {
+    const u64 v = t < n ? top[t] : 0;
+    P.out_scores[q * P.k + t] = v ? sgn * slot_unorder((unsigned)(v >> 32)) : -sgn * INFINITY;
+    P.out_index[q * P.k + t] = v ? (long long)(unsigned)~(unsigned)v + P.index_offset : -1;
+  }
+}
+
+// grid (n_q, parts)
+__global__ void __launch_bounds__(SLOT_T) topk_slots_kernel(SlotParams P) {
+  __shared__ u64 top[SLOT_K];
+  __shared__ int cnt[2 * SLOT_T / 32 + 1];
+  __shared__ int slots[256];  // list slots of this query, in CTA order
+  __shared__ int n_slots_s;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long q = blockIdx.x;
   const int tile = (int)(q / P.qpt), et = (int)(q - (long long)tile * P.qpt);
   const int g = tile / P.mt, m = tile - g * P.mt;
   const int n_sub = P.mt == 2 ? 1 : 2;
-  top_k[tid] = -INFINITY;
-  top_i[tid] = kPadIdx;
-  if (tid == 0) n_pend_s = 0;
+  if (warp == 0) {  // the CTAs that can have met this group
+    int n = 0;
+    for (int c0 = 0; c0 < P.n_ctas; c0 += 32) {
+      const int c = c0 + lane;
+      const bool hit = c < P.n_ctas && g >= (long long)P.n_groups * c / P.n_ctas && g <= (long long)P.n_groups * (c + 1) / P.n_ctas;
+      const unsigned mask = __ballot_sync(0xffffffffu, hit);
+      const int pos = n + __popc(mask & ((1u << lane) - 1u));
+      if (hit && pos < 256) slots[pos] = c + g;
+      n += __popc(mask);
+    }
+    if (lane == 0) n_slots_s = n < 256 ? n : 256;
+  }
   __syncthreads();
-  const int c_lo = (int)((long long)P.n_ctas * blockIdx.y / P.parts), c_hi = (int)((long long)P.n_ctas * (blockIdx.y + 1) / P.parts);
-  for (int c = c_lo; c < c_hi; ++c) {
-    const long long g_lo = (long long)P.n_groups * c / P.n_ctas, g_hi = (long long)P.n_groups * (c + 1) / P.n_ctas;
-    if (g < g_lo || g > g_hi) continue;
-    for (int sub = 0; sub < n_sub; ++sub) {
-      const long long list = (long long)(c + g) * (2 * P.qpt) + (P.mt == 2 ? m : sub) * P.qpt + et;
-      if (list >= P.n_lists) continue;
-      int cnt = P.hdr[list].x;
-      if (cnt > P.cap) cnt = P.cap;
-      if (cnt <= 0) continue;
-      int n_pend = n_pend_s;
-      __syncthreads();  // every thread has read the count before this list's survivors are added to it
-      if (n_pend + cnt > SLOT_W) {  // the pending block could overflow: absorb it first
-        slots_flush(top_k, top_i, blk_k, blk_i, n_pend, tid);
-        if (tid == 0) n_pend_s = 0;
-        __syncthreads();
-        n_pend = 0;
+  const int n_lists = n_slots_s * n_sub;
+  const int lo = (int)((long long)n_lists * blockIdx.y / P.parts), hi = (int)((long long)n_lists * (blockIdx.y + 1) / P.parts);
+  u64 e[SLOT_PER];
+#pragma unroll
+  for (int j = 0; j < SLOT_PER; ++j) e[j] = 0;
+  constexpr int PER_LIST = SLOT_CAP / 32;
+#pragma unroll
+  for (int u = 0; u < SLOT_LISTS / (SLOT_T / 32); ++u) {  // a warp per list
+    const int li = lo + u * (SLOT_T / 32) + warp;
+    if (li < hi) {
+      const int sub = li % n_sub;
+      const long long list = (long long)slots[li / n_sub] * (2 * P.qpt) + (P.mt == 2 ? m : sub) * P.qpt + et;
+      const int c = list < P.n_lists ? min(P.hdr[list].x, SLOT_CAP) : 0;
+#pragma unroll
+      for (int x = 0; x < PER_LIST; ++x) {
+        const int t = x * 32 + lane;
+        if (t < c)
+          e[u * PER_LIST + x] = ((u64)slot_order(P.keys[list * SLOT_CAP + t]) << 32) | (unsigned)~(unsigned)P.idx[list * SLOT_CAP + t];
       }
-      Cand mine{-INFINITY, kPadIdx};
-      if (tid < cnt) mine = Cand{P.keys[list * P.cap + tid], (long long)P.idx[list * P.cap + tid]};
-      const Cand kth{top_k[P.k - 1], top_i[P.k - 1]};
-      const bool pass = tid < cnt && before(mine, kth);
-      const unsigned mask = __ballot_sync(0xffffffffu, pass);
-      int base = 0;
-      if (lane == 0 && mask) base = atomicAdd(&n_pend_s, __popc(mask));
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (pass) {
-        const int pos = base + __popc(mask & ((1u << lane) - 1u));
-        blk_k[pos] = mine.key;
-        blk_i[pos] = mine.idx;
-      }
-      __syncthreads();
     }
   }
-  {
-    const int n_pend = n_pend_s;
-    __syncthreads();
-    if (n_pend > 0) slots_flush(top_k, top_i, blk_k, blk_i, n_pend, tid);
+  const int n = slot_select(e, P.k, top, cnt);
+  if (P.parts == 1) {
+    slot_write(P, q, top, n);
+  } else {
+    u64* out = P.part + ((long long)blockIdx.y * P.n_q + q) * P.k;
+    for (int t = tid; t < P.k; t += SLOT_T) out[t] = t < n ? top[t] : 0;
   }
-  const float sgn = P.largest ? 1.f : -1.f;
-  if (tid < P.k) {
-    const bool pad = top_i[tid] == kPadIdx;
-    const long long o = ((long long)blockIdx.y * P.n_q + q) * P.k + tid;
-    P.out_scores[o] = pad ? -sgn * INFINITY : sgn * top_k[tid];
-    P.out_index[o] = pad ? -1 : top_i[tid] + P.index_offset;
+}
+
+// the parts' winners: at most SLOT_PER * SLOT_T entries
+__global__ void __launch_bounds__(SLOT_T) topk_parts_kernel(SlotParams P) {
+  __shared__ u64 top[SLOT_K];
+  __shared__ int cnt[2 * SLOT_T / 32 + 1];
+  const long long q = blockIdx.x;
+  const int n_ent = P.parts * P.k;
+  u64 e[SLOT_PER];
+#pragma unroll
+  for (int j = 0; j < SLOT_PER; ++j) {
+    const int x = j * SLOT_T + threadIdx.x;
+    const int p = x / P.k;
+    e[j] = x < n_ent ? P.part[((long long)p * P.n_q + q) * P.k + (x - p * P.k)] : 0;
   }
+  const int n = slot_select(e, P.k, top, cnt);
+  slot_write(P, q, top, n);
 }
 
 static int launch_topk(TopkParams& P, cudaStream_t st);
 
-// In how many parts the lists of a query are merged first: a part should not walk more than about 24 CTAs' lists.
-int topk_merge_parts(int n_ctas, int n_groups) {
+// In how many parts the lists of a query are merged first: a CTA holds those of one part.  (The CTAs whose share of the
+// units can touch one tile group are at most n_ctas / n_groups + 2.)
+int topk_merge_parts(int n_ctas, int n_groups, int mt) {
   if (n_ctas <= 0 || n_groups <= 0) return 1;
-  const int ctas_per_group = n_ctas / n_groups + 2;  // CTAs whose share of the units can touch one tile group
-  if (ctas_per_group <= 32) return 1;
-  const int parts = (ctas_per_group + 15) / 16;
-  return parts > 16 ? 16 : parts;
+  return (int)ceil_div((int64_t)(n_ctas / n_groups + 2) * (mt == 2 ? 1 : 2), SLOT_LISTS);
 }
 
 int launch_topk_slots(const float* keys, const int* idx, const int2* hdr, long long n_lists, int cap, int n_ctas, int n_groups,
                       int mt, int qpt, long long n_q, int k, int largest, long long index_offset, float* out_scores,
                       long long* out_index, int parts, void* part_buf, cudaStream_t st) {
   if (n_q <= 0 || k <= 0) return LIK_OK;
-  if (cap > SLOT_W || k > SLOT_W) {
-    set_error("candidate lists of %d entries / k = %d exceed the merge width %d", cap, k, SLOT_W);
+  if (cap != SLOT_CAP || k > SLOT_K || n_ctas > 256 || parts * k > SLOT_PER * SLOT_T || (parts > 1 && !part_buf)) {
+    set_error("candidate lists of %d entries from %d CTAs, k = %d: outside what the merge takes", cap, n_ctas, k);
     return LIK_ERR_UNSUPPORTED;
   }
-  if (parts <= 1 || !part_buf) {
-    SlotParams P{keys, idx, hdr, cap, n_ctas, n_groups, mt, qpt, n_q, index_offset, n_lists, k, 2, largest, out_scores, out_index, 1};
-    topk_slots_kernel<<<(unsigned)n_q, SLOT_W, 0, st>>>(P), ::lik::count_launch();
-    LIK_CUDA_OK(cudaGetLastError());
-    return LIK_OK;
-  }
-  float* part_scores = (float*)part_buf;
-  long long* part_index = (long long*)((char*)part_buf + align_up((size_t)parts * n_q * k * sizeof(float), 8));
-  SlotParams P{keys, idx, hdr, cap, n_ctas, n_groups, mt, qpt, n_q, index_offset, n_lists, k, 2, largest, part_scores, part_index, parts};
-  topk_slots_kernel<<<dim3((unsigned)n_q, (unsigned)parts), SLOT_W, 0, st>>>(P), ::lik::count_launch();
+  SlotParams P{keys, idx, hdr, n_ctas, n_groups, mt, qpt, n_q, index_offset, n_lists, k, largest, out_scores, out_index, parts, (u64*)part_buf};
+  topk_slots_kernel<<<dim3((unsigned)n_q, (unsigned)parts), SLOT_T, 0, st>>>(P), ::lik::count_launch();
   LIK_CUDA_OK(cudaGetLastError());
-  TopkParams M{};
-  M.mode = 1;
-  M.cand_scores = part_scores;
-  M.cand_index = part_index;
-  M.n_lists = parts;
-  M.n_rows = n_q;
-  M.k = k;
-  M.largest = largest;
-  M.merge = 0;
-  M.out_scores = out_scores;
-  M.out_index = out_index;
-  return launch_topk(M, st);
+  if (parts > 1) {
+    topk_parts_kernel<<<(unsigned)n_q, SLOT_T, 0, st>>>(P), ::lik::count_launch();
+    LIK_CUDA_OK(cudaGetLastError());
+  }
+  return LIK_OK;
 }
 
 
