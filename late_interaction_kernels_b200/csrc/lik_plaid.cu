@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(256) plaid_decompress_kernel(PlaidView v, long
 constexpr int PD_RUN = 64;  // consecutive tokens per half-warp
 
 template <typename O, bool CF32, bool CBF16, int NBITS>
-__global__ void __launch_bounds__(256) plaid_decompress16_kernel(PlaidSrc S, long long tok0, long long count, O* __restrict__ out,
+__global__ void __launch_bounds__(256, CF32 ? 2 : 3) plaid_decompress16_kernel(PlaidSrc S, long long tok0, long long count, O* __restrict__ out,
                                                                int* status) {
   __shared__ __align__(16) float tab[PlaidTable<NBITS>::WORDS];
   PlaidTable<NBITS>::fill(tab, S.bucket_weights, threadIdx.x, blockDim.x);

@@ -172,18 +172,14 @@ struct PlaidPiece {  // one lane's part of a token as it is loaded
   unsigned w0, w1;   // residual codes (w1: eight-bit codes only)
 };
 
+// cen / res: the lane's bytes of centroid 0 and of the run's first token; addresses are one 32 x 32 + 64-bit multiply-add each
 template <bool CF32, int NBITS>
-__device__ __forceinline__ PlaidPiece<CF32, NBITS> plaid_piece(const PlaidSrc& S, long long tok, int code, int hl) {
+__device__ __forceinline__ PlaidPiece<CF32, NBITS> plaid_piece(const char* cen, unsigned cen_pitch, unsigned code, const char* res, unsigned res_pitch, unsigned t) {
   PlaidPiece<CF32, NBITS> r;
-  const long long off = (long long)code * S.dim + hl * 8;
-  if constexpr (CF32) {
-    const uint4* p = reinterpret_cast<const uint4*>(static_cast<const float*>(S.centroids) + off);
-    r.c0 = __ldg(p);
-    r.c1 = __ldg(p + 1);
-  } else {
-    r.c0 = __ldg(reinterpret_cast<const uint4*>(static_cast<const unsigned short*>(S.centroids) + off));
-  }
-  const unsigned char* rp = S.residuals + tok * S.packed_dim + hl * NBITS;
+  const uint4* p = reinterpret_cast<const uint4*>(cen + (unsigned long long)code * cen_pitch);
+  r.c0 = __ldg(p);
+  if constexpr (CF32) r.c1 = __ldg(p + 1);
+  const char* rp = res + (unsigned long long)t * res_pitch;
   if constexpr (NBITS == 2) r.w0 = __ldg(reinterpret_cast<const unsigned short*>(rp));
   else if constexpr (NBITS == 4) r.w0 = __ldg(reinterpret_cast<const unsigned*>(rp));
   else {
@@ -192,6 +188,14 @@ __device__ __forceinline__ PlaidPiece<CF32, NBITS> plaid_piece(const PlaidSrc& S
     r.w1 = w.y;
   }
   return r;
+}
+
+// two-wide forms of the same IEEE operations
+__device__ __forceinline__ void plaid_add2(float& a, float& b, float x, float y) {
+  asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%0, %1};\n\tmov.b64 q, {%2, %3};\n\tadd.rn.f32x2 p, p, q;\n\tmov.b64 {%0, %1}, p;\n\t}" : "+f"(a), "+f"(b) : "f"(x), "f"(y));
+}
+__device__ __forceinline__ void plaid_mul2(float& a, float& b, float m) {
+  asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%0, %1};\n\tmov.b64 q, {%2, %2};\n\tmul.rn.f32x2 p, p, q;\n\tmov.b64 {%0, %1}, p;\n\t}" : "+f"(a), "+f"(b) : "f"(m));
 }
 
 template <bool CF32, bool CBF16, int NBITS>
@@ -219,8 +223,7 @@ __device__ __forceinline__ void plaid_values(const PlaidPiece<CF32, NBITS>& r, c
     for (int i = 0; i < 4; ++i) {
       const unsigned at = i == 0 ? (r.w0 << 3) & 0x78u : (r.w0 >> (4 * i - 3)) & 0x78u;  // eight bytes per entry
       const float2 v = *reinterpret_cast<const float2*>(t + at);
-      e[2 * i] += v.x;
-      e[2 * i + 1] += v.y;
+      plaid_add2(e[2 * i], e[2 * i + 1], v.x, v.y);
     }
   } else {
 #pragma unroll
@@ -238,16 +241,20 @@ __device__ __forceinline__ void plaid_decode_run(const PlaidSrc& S, const float*
                                                  bool lane_on, int* status, Sink sink) {
   constexpr int U = 4;
   const int hl = lane & 15, ll = lane_on ? hl : 0;
-  const long long end = n > 0 ? tok0 + n - 1 : last;
-  auto at = [&](int t) -> long long { return t < n ? tok0 + t : end; };
-  int code_next = plaid_code(S, at(hl), status);
+  const long long first = n > 0 ? tok0 : last;
+  const int t_max = n > 0 ? n - 1 : 0;
+  const char* cen = static_cast<const char*>(S.centroids) + ll * (CF32 ? 32 : 16);
+  const char* res = reinterpret_cast<const char*>(S.residuals) + first * S.packed_dim + ll * NBITS;
+  const unsigned cen_pitch = (unsigned)S.dim * (CF32 ? 4u : 2u), res_pitch = (unsigned)S.packed_dim;
+  int code_next = plaid_code(S, first + min(hl, t_max), status);
   PlaidPiece<CF32, NBITS> nx[U];
 #pragma unroll
-  for (int u = 0; u < U; ++u) nx[u] = plaid_piece<CF32, NBITS>(S, at(u), __shfl_sync(0xffffffffu, code_next, (lane & 16) | u), ll);
+  for (int u = 0; u < U; ++u)
+    nx[u] = plaid_piece<CF32, NBITS>(cen, cen_pitch, __shfl_sync(0xffffffffu, code_next, (lane & 16) | u), res, res_pitch, min(u, t_max));
   for (int c0 = 0; c0 < n_uniform; c0 += 16) {
     const int code_cur = code_next;
-    code_next = plaid_code(S, at(c0 + 16 + hl), status);
-#pragma unroll 1
+    code_next = plaid_code(S, first + min(c0 + 16 + hl, t_max), status);
+#pragma unroll
     for (int b = 0; b < 16; b += U) {
       PlaidPiece<CF32, NBITS> cur[U];
 #pragma unroll
@@ -256,7 +263,7 @@ __device__ __forceinline__ void plaid_decode_run(const PlaidSrc& S, const float*
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int code = b + U < 16 ? __shfl_sync(0xffffffffu, code_cur, (lane & 16) | ((b + U + u) & 15)) : __shfl_sync(0xffffffffu, code_next, (lane & 16) | u);
-        nx[u] = plaid_piece<CF32, NBITS>(S, at(c0 + b + U + u), code, ll);
+        nx[u] = plaid_piece<CF32, NBITS>(cen, cen_pitch, code, res, res_pitch, min(c0 + b + U + u, t_max));
       }
       float e[U][8], ss[U];
 #pragma unroll
@@ -284,7 +291,7 @@ __device__ __forceinline__ void plaid_decode_run(const PlaidSrc& S, const float*
       for (int u = 0; u < U; ++u) {
         if (S.normalize) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) e[u][i] *= inv[u];
+          for (int i = 0; i < 8; i += 2) plaid_mul2(e[u][i], e[u][i + 1], inv[u]);
         }
         if (c0 + b + u < n && lane_on) sink(c0 + b + u, e[u]);
       }
