@@ -212,6 +212,9 @@ __device__ __forceinline__ unsigned warp_peers(int v, int nbits) {
   return peers;
 }
 
+// Waits until the kernels in front of a programmatically serialised launch have finished and their writes are visible.
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

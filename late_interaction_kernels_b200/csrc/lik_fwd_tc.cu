@@ -47,7 +47,8 @@ namespace {
 constexpr int TILE_N = LIK_TILE_N;     // document tokens per TMA stage = columns of one accumulator
 constexpr int ACC_COLS = 256;          // TMEM columns reserved per accumulator
 static_assert(TILE_N <= ACC_COLS && TILE_N % 32 == 0, "a stage must fit one accumulator");
-constexpr int BOX_ROWS = 64;        // granule of the document TMA boxes (64, 128, 192 or 256 rows)
+constexpr int BOX_ROWS = 32;        // granule of the document TMA boxes: 32, 64, ... 256 rows (64 read a sixth more rows than ragged documents have)
+constexpr int N_BOXES = TILE_N / BOX_ROWS;
 constexpr int SLAB_BYTES_ROW = 128; // one swizzle span: 64 two-byte or 128 one-byte elements
 constexpr int MAX_SLABS = 2;
 constexpr int NUM_THREADS = 640;
@@ -256,12 +257,19 @@ __device__ __forceinline__ bool iter_enter(const TcParams& P, int n_groups, Unit
       it.doc_hi = P.n_d;
       units = P.n_flat;
     }
-    const long long u = units * c / G, u_end = units * (c + 1) / G;
+    long long u, u_end;
+    if (units < (1ll << 32) / 256) {  // (a 64-bit division is a hundred dependent instructions in front of the first load; grids have at most 256 CTAs)
+      u = (unsigned)units * (unsigned)c / (unsigned)G;
+      u_end = (unsigned)units * (unsigned)(c + 1) / (unsigned)G;
+    } else {
+      u = units * c / G;
+      u_end = units * (c + 1) / G;
+    }
     if (u < u_end) {
       it.left = (int)(u_end - u);
       if (P.pairing == LIK_PAIR_CROSS) {
         const int nd_b = it.doc_hi - it.doc_lo;
-        it.grp = (int)(u / nd_b);
+        it.grp = u < (1ll << 32) ? (int)((unsigned)u / (unsigned)nd_b) : (int)(u / nd_b);
         it.doc = it.doc_lo + (int)(u - (long long)it.grp * nd_b);
         it.in_grp = 0;
       } else if (P.pairing == LIK_PAIR_GROUPED) {
@@ -349,7 +357,7 @@ __device__ __forceinline__ void unit_resolve(const TcParams& P, int doc, const U
 }
 
 struct DocMaps {
-  CUtensorMap m[4];  // document boxes of 64, 128, 192 and 256 rows: one copy per K slab whatever the tile height
+  CUtensorMap m[N_BOXES];  // document boxes of 32, 64, ... rows: one copy per K slab whatever the tile height
 };
 
 // Word the producer leaves beside every ring stage for the MMA issuer.
@@ -433,9 +441,6 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  // greedy-packed query tiles are counted on the device (the count sits in front of the table)
-  const int n_tiles = P.tile_q0 ? P.tile_q0[-1] : P.n_tiles;
-  const int n_groups = (n_tiles + P.mt - 1) / P.mt;
   const bool list = P.pairing == LIK_PAIR_LIST;
   const bool topk = !ARGMAX && P.topk.cand_key != nullptr;  // the fused top-k never saves winners
 
@@ -457,18 +462,23 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
     fence_barrier_init();
     prefetch_tmap(&q_map);
     if (!PLAID)
-      for (int i = 0; i < 4; ++i) prefetch_tmap(&d_maps.m[i]);
+      for (int i = 0; i < N_BOXES; ++i) prefetch_tmap(&d_maps.m[i]);
   }
-  if (PLAID)
-    for (int b = tid; b < (1 << P.plaid.nbits); b += NUM_THREADS) ctl->plaid_bw[b] = P.plaid.bucket_weights[b];
   if (warp == 1) {
     tmem_alloc(smem_u32(&ctl->tmem_base), 512);
     tmem_relinquish();
   }
+  // Launched with programmatic stream serialisation: the set-up above overlaps the kernel in front, nothing below may.
+  griddep_wait();
+  if (PLAID)
+    for (int b = tid; b < (1 << P.plaid.nbits); b += NUM_THREADS) ctl->plaid_bw[b] = P.plaid.bucket_weights[b];
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
+  // greedy-packed query tiles are counted on the device (the count sits in front of the table)
+  const int n_tiles = P.tile_q0 ? P.tile_q0[-1] : P.n_tiles;
+  const int n_groups = (n_tiles + P.mt - 1) / P.mt;
 
   const bool producer_warp = warp == 0 || (PLAID && warp >= 2 + 2 * GROUP_WARPS);
   if (producer_warp) {
@@ -1470,7 +1480,7 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, PrepJ
   int rc = make_map(&q_map, a.q, a.dtype, a.dim, TILE_M);
   if (rc) return rc;
   if (!plaid) {
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < N_BOXES; ++i) {
       rc = make_map(&d_maps.m[i], a.d, a.dtype, a.dim, (i + 1) * BOX_ROWS);
       if (rc) return rc;
     }
@@ -1575,11 +1585,21 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, PrepJ
   const bool fp8 = a.dtype == LIK_E4M3;
   const bool argmax = a.argmax != nullptr;
   const bool affine = a.d.scale || dn;  // a per-column multiplier for every document
-  dim3 grid((unsigned)pl.grid), block(NUM_THREADS);
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)pl.grid);
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = pl.smem_bytes;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
 #define LIK_TC_LAUNCH(F, A, X, PL)                                                                                     \
   do {                                                                                                                 \
     LIK_CUDA_OK((allow_smem<F, A, X, PL>(pl.smem_bytes)));                                                             \
-    fwd_tc_kernel<F, A, X, PL><<<grid, block, pl.smem_bytes, st>>>(q_map, d_maps, P), ::lik::count_launch();           \
+    LIK_CUDA_OK(cudaLaunchKernelEx(&cfg, fwd_tc_kernel<F, A, X, PL>, q_map, d_maps, P));                               \
+    ::lik::count_launch();                                                                                             \
   } while (0)
   // LIK_LONG_DOC_TOKENS overrides the length from which the lazy winner scan is used (a tuning knob)
   static int long_doc_tokens = 0;
