@@ -265,7 +265,8 @@ Tensor scored(const Tensor& Q, const Tensor& D, const Problem& pr, at::IntArrayR
   {
     at::AutoDispatchBelowADInplaceOrView below;
     auto [sq, sd] = sides(Q, D, pr, common_dtype(Q, D));
-    std::tie(scores, argmax) = forward(sq, sd, pr.pairing, pr.normalize, grad, sq.max_len, 0);
+    // (saved winners in rows of whole 16-byte groups: the backward reads four at a time)
+    std::tie(scores, argmax) = forward(sq, sd, pr.pairing, pr.normalize, grad, (sq.max_len + 3) & ~int64_t(3), 0);
     scores = scores.view(shape);
   }
   if (grad) {

@@ -855,18 +855,69 @@ struct DdSortOut {
   int* tok_cnt;           // [d.n_rows] list length (cleared before the sort)
 };
 
+// A cluster of CTAs shares one document when the documents are fewer than the SMs: each takes a slice of the entries.
+struct SortCluster {
+  int rank, size;
+};
+__device__ __forceinline__ SortCluster sort_cluster() {
+  SortCluster c;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(c.rank));
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(c.size));
+  return c;
+}
+__device__ __forceinline__ void sort_cluster_sync(const SortCluster& c) {
+  if (c.size > 1)
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  else
+    __syncthreads();
+}
+__device__ __forceinline__ int load_cluster_int(const int* p, int rank) {  // the word at p's place in the shared memory of another CTA
+  unsigned a;
+  int v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// Words of shared memory beside the histograms: per token its count in this CTA, in the cluster and in the CTAs before
+// this one, then the offsets and block totals of the scan.
+__host__ __device__ inline size_t dds_scratch_words(int ld_pad) { return (size_t)4 * ld_pad + 1 + (ld_pad + 31) / 32 + 1; }
+
 // Offsets of the winner sort.  In: hist[w][t] = winners of token t counted by warp w (n_hist of the CTA's n_warps warps
 // count).  Out: the token's first list entry and count (global), and hist[w][t] = first write position of warp w for token
 // t.  All warps work: each takes whole blocks of 32 tokens (totals, prefix inside the block), warp 0 scans the block
-// totals, then every warp finishes its blocks.  tok_off [ld_pad] and blk [ceil(ld_pad / 32) + 1] are scratch in shared memory.
-__device__ __forceinline__ void dds_offsets(int* hist, int* tok_off, int* blk, int n_warps, int n_hist, int ld_pad, int dlen,
+// totals, then every warp finishes its blocks.  The order inside a token's list is (CTA, warp, entry).  All CTAs of a
+// cluster call it with the same dlen.
+__device__ __forceinline__ void dds_offsets(int* hist, int* scratch, const SortCluster& cl, int n_warps, int n_hist, int ld_pad, int dlen,
                                             long long base, long long drow0, const DdSortOut& O, int warp, int lane) {
+  int* mine = scratch;               // [ld_pad] this CTA's winners of a token
+  int* all = mine + ld_pad;          // [ld_pad] the cluster's
+  int* before = all + ld_pad;        // [ld_pad] those of the CTAs before this one
+  int* tok_off = before + ld_pad;    // [ld_pad + 1]
+  int* blk = tok_off + ld_pad + 1;   // [ceil(ld_pad / 32) + 1]
+  for (int t = warp * 32 + lane; t < dlen; t += n_warps * 32) {
+    int tot = 0;
+    for (int w = 0; w < n_hist; ++w) tot += hist[w * ld_pad + t];
+    mine[t] = tot;
+  }
+  sort_cluster_sync(cl);
   const int n_blk = (dlen + 31) >> 5;
   for (int b = warp; b < n_blk; b += n_warps) {
     const int t = b * 32 + lane;
-    int tot = 0;
-    if (t < dlen)
-      for (int w = 0; w < n_hist; ++w) tot += hist[w * ld_pad + t];
+    int tot = 0, bef = 0;
+    if (t < dlen) {
+      if (cl.size == 1) {
+        tot = mine[t];
+      } else {
+        for (int r = 0; r < cl.size; ++r) {
+          const int v = load_cluster_int(mine + t, r);
+          tot += v;
+          if (r < cl.rank) bef += v;
+        }
+      }
+      all[t] = tot;
+      before[t] = bef;
+    }
     int incl = tot;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -876,7 +927,7 @@ __device__ __forceinline__ void dds_offsets(int* hist, int* tok_off, int* blk, i
     if (t < dlen) tok_off[t] = incl - tot;
     if (lane == 31) blk[b] = incl;
   }
-  __syncthreads();
+  sort_cluster_sync(cl);  // (the other CTAs have read `mine` too: it may go away with this CTA)
   if (warp == 0) {
     int running = 0;
     for (int b0 = 0; b0 < n_blk; b0 += 32) {
@@ -897,14 +948,16 @@ __device__ __forceinline__ void dds_offsets(int* hist, int* tok_off, int* blk, i
     const int t = b * 32 + lane;
     if (t < dlen) {
       const int excl = blk[b] + tok_off[t];
-      int pos = excl;
+      int pos = excl + before[t];
       for (int w = 0; w < n_hist; ++w) {
         const int c = hist[w * ld_pad + t];
         hist[w * ld_pad + t] = pos;
         pos += c;
       }
-      O.tok_begin[drow0 + t] = base + excl;
-      O.tok_cnt[drow0 + t] = pos - excl;
+      if (cl.rank == 0) {
+        O.tok_begin[drow0 + t] = base + excl;
+        O.tok_cnt[drow0 + t] = all[t];
+      }
     }
   }
   __syncthreads();
@@ -916,7 +969,8 @@ __global__ void __launch_bounds__(DDS_WARPS * 32) bwd_dd_sort_kernel(BwdParams P
   const int n_warps = blockDim.x >> 5;
   extern __shared__ int dds_raw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int j = blockIdx.x;
+  const SortCluster cl = sort_cluster();
+  const int j = blockIdx.x / cl.size;  // (all CTAs of a cluster leave together: what decides is the document's)
   long long drow0;
   int dlen;
   seq_bounds(P.d, j, drow0, dlen, nullptr);
@@ -932,9 +986,8 @@ __global__ void __launch_bounds__(DDS_WARPS * 32) bwd_dd_sort_kernel(BwdParams P
   const int n_ent = ds.n_qr * lq;
   const long long base = list ? ds.first * lq : (long long)j * n_ent;  // first entry of the document's slice of the list
   int* hist = dds_raw;                          // [n_hist][ld_pad]
-  int* tok_off = hist + n_hist * ld_pad;      // [ld_pad + 1]
-  int* blk = tok_off + ld_pad + 1;            // [ceil(ld_pad / 32) + 1]
-  float* gcol = reinterpret_cast<float*>(blk + (ld_pad + 31) / 32 + 1);  // [n_qr] (not for pair lists)
+  int* scratch = hist + n_hist * ld_pad;
+  float* gcol = reinterpret_cast<float*>(scratch + dds_scratch_words(ld_pad));  // [n_qr] (not for pair lists)
 
   for (int x = tid; x < n_hist * ld_pad; x += blockDim.x) hist[x] = 0;
   if (!list)
@@ -942,8 +995,9 @@ __global__ void __launch_bounds__(DDS_WARPS * 32) bwd_dd_sort_kernel(BwdParams P
   __syncthreads();
 
   // entry e = ii * lq + s ; slice of this warp (multiple of 32 so rounds stay aligned)
-  const int per_warp = ((n_ent + n_hist - 1) / n_hist + 31) & ~31;  // (warps beyond n_hist get an empty slice)
-  const int e_lo = warp * per_warp, e_hi = min(n_ent, e_lo + per_warp);
+  const int n_slices = n_hist * cl.size;
+  const int per_warp = ((n_ent + n_slices - 1) / n_slices + 31) & ~31;
+  const int e_lo = min(n_ent, (cl.rank * n_hist + warp) * per_warp), e_hi = warp < n_hist ? min(n_ent, e_lo + per_warp) : e_lo;
 
   // raw saved winner of entry e (no validation): a plain load that can be issued ahead of its use
   auto raw_winner = [&](int e) -> int {
@@ -979,7 +1033,7 @@ __global__ void __launch_bounds__(DDS_WARPS * 32) bwd_dd_sort_kernel(BwdParams P
   }
   __syncthreads();
   // offsets: warp 0 scans the tokens; hist[w][t] becomes the first write position of warp w for token t
-  dds_offsets(hist, tok_off, blk, n_warps, n_hist, ld_pad, dlen, base, drow0, O, warp, lane);
+  dds_offsets(hist, scratch, cl, n_warps, n_hist, ld_pad, dlen, base, drow0, O, warp, lane);
   // stable placement
   int t_next = raw_winner(e_lo + lane);
   for (int eb = e_lo; eb < e_hi; eb += 32) {
@@ -1089,7 +1143,8 @@ __global__ void __launch_bounds__(DDS_WARPS * 32) bwd_dd_sort4_kernel(BwdParams 
   const int n_warps = blockDim.x >> 5;
   extern __shared__ int dds_raw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int j = blockIdx.x;
+  const SortCluster cl = sort_cluster();
+  const int j = blockIdx.x / cl.size;  // (all CTAs of a cluster leave together: what decides is the document's)
   long long drow0;
   int dlen;
   seq_bounds(P.d, j, drow0, dlen, nullptr);
@@ -1107,9 +1162,8 @@ __global__ void __launch_bounds__(DDS_WARPS * 32) bwd_dd_sort4_kernel(BwdParams 
   const int n_ent = n_quad * 4;
   const long long base = list ? ds.first * lq : (long long)j * n_ent;
   int* hist = dds_raw;                          // [n_hist][ld_pad]
-  int* tok_off = hist + n_hist * ld_pad;      // [ld_pad + 1]
-  int* blk = tok_off + ld_pad + 1;            // [ceil(ld_pad / 32) + 1]
-  float* gcol = reinterpret_cast<float*>(blk + (ld_pad + 31) / 32 + 1);  // [n_qr] (not for pair lists)
+  int* scratch = hist + n_hist * ld_pad;
+  float* gcol = reinterpret_cast<float*>(scratch + dds_scratch_words(ld_pad));  // [n_qr] (not for pair lists)
   int* q_first = reinterpret_cast<int*>(gcol + ds.n_qr);  // [n_qr] first row and length of every score's query (not for pair lists)
   int* q_len = q_first + ds.n_qr;
 
@@ -1128,8 +1182,9 @@ __global__ void __launch_bounds__(DDS_WARPS * 32) bwd_dd_sort4_kernel(BwdParams 
 
   // slice of this warp in 16-byte groups (whole warp loads); a round is DDS_LOADS loads per lane
   const int round_quads = 32 * DDS_LOADS;
-  const int per_warp = ((n_quad + n_hist - 1) / n_hist + 31) & ~31;  // (warps beyond n_hist get an empty slice)
-  const int m_lo = warp * per_warp, m_hi = min(n_quad, m_lo + per_warp);
+  const int n_slices = n_hist * cl.size;
+  const int per_warp = ((n_quad + n_slices - 1) / n_slices + 31) & ~31;
+  const int m_lo = min(n_quad, (cl.rank * n_hist + warp) * per_warp), m_hi = warp < n_hist ? min(n_quad, m_lo + per_warp) : m_lo;
   const int4 none = make_int4(-1, -1, -1, -1);
 
   auto load_quad = [&](int m) -> int4 {
@@ -1175,7 +1230,7 @@ __global__ void __launch_bounds__(DDS_WARPS * 32) bwd_dd_sort4_kernel(BwdParams 
   }
   __syncthreads();
   // ---- offsets: warp 0 scans the per-token totals ----
-  dds_offsets(hist, tok_off, blk, n_warps, n_hist, ld_pad, dlen, base, drow0, O, warp, lane);
+  dds_offsets(hist, scratch, cl, n_warps, n_hist, ld_pad, dlen, base, drow0, O, warp, lane);
   // ---- pass 2: placement (the winners come from L2 this time) ----
   for (int mb = m_lo; mb < m_hi; mb += round_quads) {
     int4 w[DDS_LOADS];
@@ -1395,6 +1450,7 @@ struct BwdPlan {
   bool fast, sorted;
   bool list_sorted;  // pair list on the deterministic kernels
   int sort_warps;    // warps of the winner sort that take entries (a histogram each): at least 256 entries of a document per warp
+  int sort_cluster;  // CTAs per document
   int sort_threads;  // threads of its CTAs: more warps than that when the documents are long (clearing and offsets go with the length)
   bool row16;  // 16-byte gathers: rows 16-byte aligned, width a multiple of 16 bytes, at most 1024 bytes
   int dq_split;    // grad_q: document ranges per query (1: one CTA walks all the documents of its query tokens)
@@ -1437,7 +1493,7 @@ BwdPlan plan_bwd(const lik_bwd_args& a) {
   pl.list_sorted = list && a.deterministic && pl.fast && a.n_pairs > 0 && a.n_pairs < (1ll << 31) && a.d.max_len > 0 &&
                    a.q.max_len > 0 && a.q.n_seq > 0 && a.d.n_seq > 0;
   if (pl.list_sorted) {
-    const size_t ws_sort = ((size_t)(a.d.max_len + 1) + a.d.max_len + 2) * 4;  // with one warp per CTA
+    const size_t ws_sort = ((size_t)(a.d.max_len + 1) + dds_scratch_words(a.d.max_len + 1)) * 4;  // with one warp per CTA
     if (ws_sort > 200 * 1024) pl.list_sorted = false;
   }
   if (pl.list_sorted) {
@@ -1474,10 +1530,13 @@ BwdPlan plan_bwd(const lik_bwd_args& a) {
     const long long ent = a.pairing == LIK_PAIR_CROSS ? (long long)a.q.n_seq * a.argmax_stride
                           : a.pairing == LIK_PAIR_GROUPED ? (long long)a.argmax_stride
                                                           : ceil_div(a.n_pairs, a.d.n_seq) * a.argmax_stride;
-    long long nw = ceil_div(ent, 256);  // a warp per 256 entries: few, long documents still fill their CTAs
+    // fewer documents than SMs: as many CTAs per document as leave each two thousand entries, so that the GPU fills up
+    pl.sort_cluster = 1;
+    while (pl.sort_cluster < 8 && (long long)a.d.n_seq * pl.sort_cluster * 2 <= 2 * sm_count() && ent >= 4096ll * pl.sort_cluster) pl.sort_cluster *= 2;
+    long long nw = ceil_div(ceil_div(ent, pl.sort_cluster), 256);  // a warp per 256 entries: few, long documents still fill their CTAs
     pl.sort_warps = (int)(nw < 1 ? 1 : (nw > DDS_WARPS ? DDS_WARPS : nw));
     auto smem_for = [&](int w) {
-      return ((size_t)w * pl.ld_pad + pl.ld_pad + 1 + (size_t)(pl.ld_pad + 31) / 32 + 1 + 3 * (size_t)n_qrange) * 4;
+      return ((size_t)w * pl.ld_pad + dds_scratch_words(pl.ld_pad) + 3 * (size_t)n_qrange) * 4;
     };
     while (pl.sort_warps > 1 && smem_for(pl.sort_warps) > 200 * 1024) pl.sort_warps >>= 1;  // long documents: fewer histograms
     pl.sort_smem = smem_for(pl.sort_warps);
@@ -1616,14 +1675,21 @@ int run_bwd(const lik_bwd_args& a, BwdParams& P, const BwdPlan& pl, cudaStream_t
       O.tok_begin = (long long*)(ws + pl.begin_off);
       O.tok_cnt = (int*)(ws + pl.cnt_off);
       const bool quads = a.argmax_stride % 4 == 0 && ((uintptr_t)a.argmax % 16) == 0;
-      if (quads) {
-        LIK_CUDA_OK(cudaFuncSetAttribute(bwd_dd_sort4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.sort_smem));
-        bwd_dd_sort4_kernel<<<(unsigned)a.d.n_seq, pl.sort_threads, pl.sort_smem, st>>>(P, O, pl.ld_pad, pl.sort_warps), ::lik::count_launch();
-      } else {
-        LIK_CUDA_OK(cudaFuncSetAttribute(bwd_dd_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.sort_smem));
-        bwd_dd_sort_kernel<<<(unsigned)a.d.n_seq, pl.sort_threads, pl.sort_smem, st>>>(P, O, pl.ld_pad, pl.sort_warps), ::lik::count_launch();
-      }
-      LIK_CUDA_OK(cudaGetLastError());
+      auto kernel = quads ? bwd_dd_sort4_kernel : bwd_dd_sort_kernel;
+      if (pl.sort_smem > 48 * 1024) LIK_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.sort_smem));
+      cudaLaunchAttribute attr{};
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = (unsigned)pl.sort_cluster;
+      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3((unsigned)a.d.n_seq * (unsigned)pl.sort_cluster);
+      cfg.blockDim = dim3((unsigned)pl.sort_threads);
+      cfg.dynamicSmemBytes = pl.sort_smem;
+      cfg.stream = st;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      LIK_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, P, O, pl.ld_pad, pl.sort_warps));
+      ::lik::count_launch();
       if (pl.row16) {
         // one CTA per 16 tokens, except for very many tokens (long documents): there a capped grid walks them
         const long long rg = ceil_div(a.d.n_rows, 16);

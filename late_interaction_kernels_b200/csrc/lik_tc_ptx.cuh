@@ -175,11 +175,9 @@ __device__ __forceinline__ void fold32(const float (&v)[32], int col0, float& ru
 __device__ __forceinline__ void scale32(float (&v)[32], const float* scale) {
 #pragma unroll
   for (int i = 0; i < 32; i += 4) {
-    const float4 sc = *reinterpret_cast<const float4*>(scale + i);
-    v[i + 0] *= sc.x;
-    v[i + 1] *= sc.y;
-    v[i + 2] *= sc.z;
-    v[i + 3] *= sc.w;
+    const ulonglong2 sc = *reinterpret_cast<const ulonglong2*>(scale + i);
+    asm("{\n\t.reg .b64 p;\n\tmov.b64 p, {%0, %1};\n\tmul.rn.f32x2 p, p, %2;\n\tmov.b64 {%0, %1}, p;\n\t}" : "+f"(v[i]), "+f"(v[i + 1]) : "l"(sc.x));
+    asm("{\n\t.reg .b64 p;\n\tmov.b64 p, {%0, %1};\n\tmul.rn.f32x2 p, p, %2;\n\tmov.b64 {%0, %1}, p;\n\t}" : "+f"(v[i + 2]), "+f"(v[i + 3]) : "l"(sc.y));
   }
 }
 // v[i] = v[i] * scale[i] for the first `lim` columns, -inf for the others (whatever scale holds there)
