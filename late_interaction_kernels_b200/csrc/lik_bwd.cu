@@ -695,14 +695,12 @@ __device__ __forceinline__ void dq16_finish_row(const BwdParams& P, float (&acc)
   store_row16<T, G, CH>((G*)P.grad_q + qrow * P.dim, acc, P.dim, hl);
 }
 
-template <typename T, typename G, int CH>
-__global__ void __launch_bounds__(256) bwd_dq16_kernel(BwdParams P) {
+// One block of 16 * TOK threads: query tokens [s0, s0 + TOK) of query i, document range z.
+template <typename T, typename G, int CH, int TOK>
+__device__ __forceinline__ void dq16_block(const BwdParams& P, int i, int s0, int z, int2 (*s_e)[TOK]) {
   constexpr int N = Vec16<T>::N;
   constexpr int U = 8 / CH;  // rows in flight per half-warp
-  __shared__ int2 s_e[DQ_JC][DQ16_TOK];
   const int tid = threadIdx.x, hl = tid & 15, hw = tid >> 4;
-  const int i = blockIdx.x;
-  const int s0 = blockIdx.y * DQ16_TOK;
   const int s = s0 + hw;
   long long qrow0;
   int qlen;
@@ -727,19 +725,19 @@ __global__ void __launch_bounds__(256) bwd_dq16_kernel(BwdParams P) {
 #pragma unroll
   for (int c = 0; c < CH; ++c) lane_on[c] = elt16<T>(c, hl) < P.dim;
   const bool d_factor = P.d.inv_norm || P.d.scale || P.d.scale_scalar != 1.f;
-  // this CTA's range of the query's documents (all of them unless the documents are split over blockIdx.z)
+  // this CTA's range of the query's documents (all of them unless the documents are split over blocks)
   int jb_lo = 0, jb_hi = count;
   if (P.dq_split > 1) {
     const int chunk = ((count + DQ_JC - 1) / DQ_JC + P.dq_split - 1) / P.dq_split * DQ_JC;
-    jb_lo = min(count, (int)blockIdx.z * chunk);
+    jb_lo = min(count, z * chunk);
     jb_hi = min(count, jb_lo + chunk);
   }
   for (int jb = jb_lo; jb < jb_hi; jb += DQ_JC) {
     __syncthreads();
 #pragma unroll
-    for (int x = tid; x < DQ_JC * DQ16_TOK; x += 256) {
+    for (int x = tid; x < DQ_JC * TOK; x += 16 * TOK) {
       // entry (jj, r): winner of document jb + jj for query token s0 + r
-      const int jj = x >> 4, r = x & 15;
+      const int jj = x / TOK, r = x % TOK;
       int2 e = make_int2(-1, 0);
       if (jb + jj < jb_hi && s0 + r < lq) {
         long long slot;
@@ -786,10 +784,16 @@ __global__ void __launch_bounds__(256) bwd_dq16_kernel(BwdParams P) {
   }
   if (!owns) return;
   if (P.dq_split > 1) {  // the partial sum of this range; bwd_dq16_sum_kernel finishes the row
-    store_row16<T, float, CH>(P.dq_partial + ((long long)blockIdx.z * P.q.n_rows + qrow) * P.dim, acc, P.dim, hl);
+    store_row16<T, float, CH>(P.dq_partial + ((long long)z * P.q.n_rows + qrow) * P.dim, acc, P.dim, hl);
     return;
   }
   dq16_finish_row<T, G, CH>(P, acc, qrow, active, hl);
+}
+
+template <typename T, typename G, int CH>
+__global__ void __launch_bounds__(256) bwd_dq16_kernel(BwdParams P) {
+  __shared__ int2 s_e[DQ_JC][DQ16_TOK];
+  dq16_block<T, G, CH, DQ16_TOK>(P, blockIdx.x, blockIdx.y * DQ16_TOK, blockIdx.z, s_e);
 }
 
 // Second half of the split grad_q: the partial rows of the document ranges, summed in range order.
@@ -1266,7 +1270,7 @@ __global__ void __launch_bounds__(DDS_WARPS * 32) bwd_dd_sort4_kernel(BwdParams 
 
 // grad_d reduce with 16-byte gathers: one half-warp per document token, 16 tokens per CTA.
 template <typename T, typename G, int CH>
-__device__ __forceinline__ void dd_reduce16_row(const BwdParams& P, const DdSortOut& O, long long drow, int hl) {
+__device__ __forceinline__ void dd_reduce16_list(const BwdParams& P, const int2* __restrict__ list, int cnt, long long drow, int hl) {
   constexpr int N = Vec16<T>::N;
   constexpr int U = 8 / CH;
   float acc[CH][N];
@@ -1274,10 +1278,7 @@ __device__ __forceinline__ void dd_reduce16_row(const BwdParams& P, const DdSort
   for (int c = 0; c < CH; ++c)
 #pragma unroll
     for (int e = 0; e < N; ++e) acc[c][e] = 0.f;
-  const int cnt = __ldg(O.tok_cnt + drow);
-  const long long begin = __ldg(O.tok_begin + drow);
   if (cnt > 0) {
-    const int2* __restrict__ list = O.pairs + begin;
     const long long pitch = P.q.row_stride;
     const T* __restrict__ Qlane = (const T*)P.q.data + hl * N;
     bool lane_on[CH];
@@ -1287,7 +1288,7 @@ __device__ __forceinline__ void dd_reduce16_row(const BwdParams& P, const DdSort
     for (; k + U <= cnt; k += U) {
       int2 e[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) e[u] = __ldg(list + k + u);
+      for (int u = 0; u < U; ++u) e[u] = list[k + u];
       uint4 v[U][CH];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -1303,7 +1304,7 @@ __device__ __forceinline__ void dd_reduce16_row(const BwdParams& P, const DdSort
       }
     }
     for (; k < cnt; ++k) {
-      const int2 e = __ldg(list + k);
+      const int2 e = list[k];
       const float w = __int_as_float(e.y);
       const T* src = Qlane + e.x * pitch;
 #pragma unroll
@@ -1323,6 +1324,13 @@ __device__ __forceinline__ void dd_reduce16_row(const BwdParams& P, const DdSort
     }
   }
   store_row16<T, G, CH>((G*)P.grad_d + drow * P.dim, acc, P.dim, hl);
+}
+
+template <typename T, typename G, int CH>
+__device__ __forceinline__ void dd_reduce16_row(const BwdParams& P, const DdSortOut& O, long long drow, int hl) {
+  const int cnt = __ldg(O.tok_cnt + drow);
+  const long long begin = __ldg(O.tok_begin + drow);
+  dd_reduce16_list<T, G, CH>(P, O.pairs + begin, cnt, drow, hl);
 }
 
 template <typename T, typename G, int CH>
@@ -1349,6 +1357,158 @@ __global__ void __launch_bounds__(256) bwd_dd_reduce16_walk_kernel(BwdParams P, 
       store_row16<T, G, CH>((G*)P.grad_d + drow * P.dim, zero, P.dim, hl);
     } else {
       dd_reduce16_row<T, G, CH>(P, O, drow, hl);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------
+// Both gradients in one launch, for problems whose documents have few winners each (small batches, candidate lists):
+// the first dq_blocks blocks are grad_q blocks, the others take a document each - the counting sort of its winners stays in
+// shared memory and the same block reduces and stores the document's rows.  Such problems are bound by launches and by the
+// zero rows of grad_d, not by gathers: against sort and reduce kernels this saves two launches, the list's round trip
+// and a scheduling pass over 16-row blocks.  64 x 32 candidate lists of 300 tokens: 75 -> 45 us; a 16 x 16 batch 26 -> 14 us.
+// The order inside a token's list is (warp, round, lane): fixed by the data alone.
+// ---------------------------------------------------------------------------------
+constexpr int FUSED_ENT = 4096;  // most winners of a document
+constexpr int FUSED_SMEM = 112 * 1024;  // two blocks per SM
+struct FusedShape {
+  int dq_blocks, dq_per_query;  // grad_q blocks, and how many a query has
+  int ld_pad, n_hist;
+  int parts;                    // blocks per document: each sorts all of its winners and stores every parts-th run of rows
+};
+inline size_t fused_smem(int n_ent, int ld_pad, int n_hist) { return (size_t)n_ent * sizeof(int2) + ((size_t)n_hist + 2) * ld_pad * 4 + 64 * 4; }
+
+template <typename T, typename G, int CH, int NT>
+__global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape F) {
+  constexpr int TOK = NT / 16;
+  extern __shared__ __align__(16) unsigned char fused_raw[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, hl = tid & 15, hw = tid >> 4;
+  if ((int)blockIdx.x < F.dq_blocks) {
+    const int i = blockIdx.x / F.dq_per_query;
+    dq16_block<T, G, CH, TOK>(P, i, (blockIdx.x - i * F.dq_per_query) * TOK, 0, reinterpret_cast<int2(*)[TOK]>(fused_raw));
+    return;
+  }
+  const int j = (blockIdx.x - F.dq_blocks) / F.parts, part = (blockIdx.x - F.dq_blocks) - j * F.parts;
+  long long drow0;
+  int dlen;
+  seq_bounds(P.d, j, drow0, dlen, nullptr);
+  const int d_rows = P.d.cu ? dlen : P.d.max_len;
+  if (P.d.cu && part == 0 && (j == 0 || j == P.d.n_seq - 1)) {
+    // packed rows that no document owns (in front of the first, behind the last)
+    float zero[CH][Vec16<T>::N];
+#pragma unroll
+    for (int c = 0; c < CH; ++c)
+#pragma unroll
+      for (int e = 0; e < Vec16<T>::N; ++e) zero[c][e] = 0.f;
+    const long long lo = 0, hi = j == 0 ? min((long long)P.d.cu[0], P.d.n_rows) : 0;
+    for (long long r = lo + hw; r < hi; r += TOK) store_row16<T, G, CH>((G*)P.grad_d + r * P.dim, zero, P.dim, hl);
+    if (j == P.d.n_seq - 1)
+      for (long long r = (long long)P.d.cu[j + 1] + hw; r < P.d.n_rows; r += TOK) store_row16<T, G, CH>((G*)P.grad_d + r * P.dim, zero, P.dim, hl);
+  }
+  if (d_rows <= 0) return;
+  const bool fits = dlen < F.ld_pad;  // (otherwise max_len understated the longest document: reported, its rows are zero)
+  if (!fits && tid == 0 && P.status) atomicOr(P.status, LIK_DEV_LEN_RANGE);
+  const DocScores ds = doc_scores(P, j);
+  const int lq = P.argmax_stride, n_ent = ds.n_qr * lq;
+  int2* list = reinterpret_cast<int2*>(fused_raw);            // [n_ent] (query row, weight)
+  int* hist = reinterpret_cast<int*>(list + n_ent);           // [n_hist][ld_pad]
+  int* begin = hist + F.n_hist * F.ld_pad;                    // [ld_pad]
+  int* cnt = begin + F.ld_pad;                                // [ld_pad]
+  int* wsum = cnt + F.ld_pad;                                 // [NT / 32]
+  if (fits) {
+    for (int x = tid; x < F.n_hist * F.ld_pad; x += NT) hist[x] = 0;
+    // the winners of this thread: round k is entry k * NT + tid
+    constexpr int ROUNDS = FUSED_ENT / NT;
+    int t_r[ROUNDS];
+#pragma unroll
+    for (int k = 0; k < ROUNDS; ++k) {
+      const int e = k * NT + tid;
+      t_r[k] = -1;
+      if (e < n_ent) {
+        const int ii = e / lq, s = e - ii * lq;
+        t_r[k] = __ldg(P.argmax + doc_slot(P, ds, j, ii) * lq + s);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < ROUNDS; ++k) {
+      if (k * NT >= n_ent) break;
+      const int e = k * NT + tid;
+      int t = t_r[k];
+      if (t >= dlen) t = -1;
+      if (t >= 0) {
+        const int ii = e / lq, s = e - ii * lq;
+        long long qrow0;
+        int qlen;
+        seq_bounds(P.q, ds.i_begin + ii, qrow0, qlen, nullptr);
+        if (s >= qlen || !row_valid(P.q, qrow0 + s)) t = -1;
+      }
+      t_r[k] = t;
+      if (t >= 0) atomicAdd(&hist[warp * F.ld_pad + t], 1);
+    }
+    __syncthreads();
+    // offsets: a run of tokens per thread, scanned over the block
+    const int per = (dlen + NT - 1) / NT;
+    const int t0 = min(dlen, tid * per), t1 = min(dlen, t0 + per);
+    int sum = 0;
+    for (int t = t0; t < t1; ++t) {
+      int c = 0;
+      for (int w = 0; w < F.n_hist; ++w) c += hist[w * F.ld_pad + t];
+      cnt[t] = c;
+      sum += c;
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    int pos = incl - sum;
+    for (int w = 0; w < warp; ++w) pos += wsum[w];
+    for (int t = t0; t < t1; ++t) {
+      begin[t] = pos;
+      for (int w = 0; w < F.n_hist; ++w) {
+        const int c = hist[w * F.ld_pad + t];
+        hist[w * F.ld_pad + t] = pos;
+        pos += c;
+      }
+    }
+    __syncthreads();
+    const int t_bits = 32 - __clz(F.ld_pad);  // winners are below ld_pad
+#pragma unroll
+    for (int k = 0; k < ROUNDS; ++k) {
+      if (k * NT >= n_ent) break;
+      const int t = t_r[k];
+      const unsigned peers = warp_peers(t, t_bits);
+      if (t >= 0) {
+        const int e = k * NT + tid, ii = e / lq, s = e - ii * lq;
+        const int i = ds.i_begin + ii;
+        long long qrow0;
+        int qlen;
+        seq_bounds(P.q, i, qrow0, qlen, nullptr);
+        const long long qrow = qrow0 + s;
+        const float w = P.g[doc_slot(P, ds, j, ii)] * row_factor(P.q, qrow);
+        list[hist[warp * F.ld_pad + t] + __popc(peers & ((1u << lane) - 1u))] = make_int2((int)qrow, __float_as_int(w));
+      }
+      __syncwarp();
+      if (t >= 0 && (peers & ((1u << lane) - 1u)) == 0) hist[warp * F.ld_pad + t] += __popc(peers);
+      __syncwarp();
+    }
+    __syncthreads();
+  }
+  for (int t = part * TOK + hw; t < d_rows; t += TOK * F.parts) {
+    const int c = fits && t < dlen ? cnt[t] : 0;
+    if (c == 0) {
+      float zero[CH][Vec16<T>::N];
+#pragma unroll
+      for (int cc = 0; cc < CH; ++cc)
+#pragma unroll
+        for (int e = 0; e < Vec16<T>::N; ++e) zero[cc][e] = 0.f;
+      store_row16<T, G, CH>((G*)P.grad_d + (drow0 + t) * P.dim, zero, P.dim, hl);
+    } else {
+      dd_reduce16_list<T, G, CH>(P, list + begin[t], c, drow0 + t, hl);
     }
   }
 }
@@ -1453,6 +1613,9 @@ struct BwdPlan {
   int sort_cluster;  // CTAs per document
   int sort_threads;  // threads of its CTAs: more warps than that when the documents are long (clearing and offsets go with the length)
   bool row16;  // 16-byte gathers: rows 16-byte aligned, width a multiple of 16 bytes, at most 1024 bytes
+  bool fused;      // both gradients in one launch (bwd_fused16_kernel)
+  int fused_threads, fused_hist, fused_parts;
+  size_t fused_bytes;
   int dq_split;    // grad_q: document ranges per query (1: one CTA walks all the documents of its query tokens)
   size_t dqp_off;  // their partial rows
   int ld_pad;
@@ -1485,6 +1648,7 @@ BwdPlan plan_bwd(const lik_bwd_args& a) {
   pl.fast = bwd_fast_ok(a);
   pl.row16 = bwd_row16_ok(a);
   pl.sorted = false;
+  pl.fused = false;
   if (a.normalize & LIK_NORM_Q) pl.qn_off = take((size_t)a.q.n_rows * 4);
   if (a.normalize & LIK_NORM_D) pl.dn_off = take((size_t)a.d.n_rows * 4);
   const bool list = a.pairing == LIK_PAIR_LIST;
@@ -1519,10 +1683,29 @@ BwdPlan plan_bwd(const lik_bwd_args& a) {
       pl.dqp_off = take((size_t)z * a.q.n_rows * a.dim * 4);
     }
   }
+  // Few winners per document, and documents that one block can store: everything in one launch.  (With many winners per
+  // document and few documents the sort and reduce kernels spread a document over the GPU; long documents too.)
+  {
+    const long long ent = a.pairing == LIK_PAIR_CROSS ? (long long)a.q.n_seq * a.argmax_stride : (long long)a.argmax_stride;
+    const bool rows_owned = a.d.cu || (a.d.seq_stride == a.d.max_len && a.d.n_rows == (int64_t)a.d.n_seq * a.d.seq_stride);
+    if (!list && a.deterministic && pl.row16 && a.grad_d && a.d.n_seq > 0 && a.d.max_len > 0 && a.d.max_len <= 1536 && a.q.n_seq > 0 &&
+        a.q.max_len > 0 && ent > 0 && ent <= FUSED_ENT && (ent <= 1024 || a.d.n_seq >= 96) && rows_owned) {
+      pl.fused_threads = ent > 512 ? 512 : 256;
+      const int warps = pl.fused_threads / 32;
+      pl.fused_hist = (int)(ceil_div(ent, 32) < warps ? ceil_div(ent, 32) : warps);
+      pl.fused_bytes = fused_smem((int)ent, a.d.max_len + 1, pl.fused_hist);
+      const size_t dq_bytes = (size_t)DQ_JC * (pl.fused_threads / 16) * sizeof(int2);
+      if (pl.fused_bytes < dq_bytes) pl.fused_bytes = dq_bytes;
+      pl.fused = pl.fused_bytes <= FUSED_SMEM;
+      // few documents: several blocks each, with at least two rows per half-warp
+      const long long parts = 2ll * sm_count() / a.d.n_seq, most = ceil_div(a.d.max_len, pl.fused_threads / 16 * 2);
+      pl.fused_parts = (int)(parts < 1 ? 1 : (parts > most ? most : parts));
+    }
+  }
   const bool scatter = list && !pl.list_sorted;
   if (a.grad_q && scatter) pl.gq32_off = take((size_t)a.q.n_rows * a.dim * 4);
   if (a.grad_d && (scatter || !a.deterministic)) pl.gd32_off = take((size_t)a.d.n_rows * a.dim * 4);
-  if (a.grad_d && !scatter && a.deterministic && pl.fast && a.d.n_seq > 0 && a.d.max_len > 0 && a.d.n_rows < (1ll << 31) &&
+  if (!pl.fused && a.grad_d && !scatter && a.deterministic && pl.fast && a.d.n_seq > 0 && a.d.max_len > 0 && a.d.n_rows < (1ll << 31) &&
       a.q.n_rows < (1ll << 31)) {
     const long long n_qrange = a.pairing == LIK_PAIR_CROSS ? a.q.n_seq : (list ? 0 : 1);
     pl.ld_pad = a.d.max_len + 1;
@@ -1639,7 +1822,8 @@ int run_bwd(const lik_bwd_args& a, BwdParams& P, const BwdPlan& pl, cudaStream_t
   } while (0)
 
   const bool fast = pl.fast;
-  if (a.grad_q && !list && a.q.n_seq > 0 && a.q.max_len > 0) {
+  const bool dq_fused = pl.fused && a.grad_q && pl.dq_split == 1;
+  if (a.grad_q && !dq_fused && !list && a.q.n_seq > 0 && a.q.max_len > 0) {
     dim3 grid((unsigned)a.q.n_seq, (unsigned)ceil_div(a.q.max_len, 8));
     if (pl.row16) {
       const dim3 grid16((unsigned)a.q.n_seq, (unsigned)ceil_div(a.q.max_len, DQ16_TOK), (unsigned)pl.dq_split);
@@ -1668,7 +1852,33 @@ int run_bwd(const lik_bwd_args& a, BwdParams& P, const BwdPlan& pl, cudaStream_t
     LIK_CUDA_OK(cudaEventRecord(fj->join, fj->aux));
     st = st_main;
   }
-  if (a.grad_d && !list && a.deterministic && a.d.n_seq > 0 && a.d.max_len > 0) {
+  if (pl.fused) {
+    FusedShape F;
+    F.ld_pad = a.d.max_len + 1;
+    F.n_hist = pl.fused_hist;
+    F.dq_per_query = (int)ceil_div(a.q.max_len, pl.fused_threads / 16);
+    F.dq_blocks = dq_fused ? a.q.n_seq * F.dq_per_query : 0;
+    F.parts = pl.fused_parts;
+    const unsigned grid = (unsigned)(F.dq_blocks + a.d.n_seq * F.parts);
+    const size_t row_bytes = (size_t)a.dim * sizeof(T);
+#define LIK_FUSED(CH_, NT_)                                                                                                          \
+  do {                                                                                                                               \
+    if (pl.fused_bytes > 48 * 1024)                                                                                                  \
+      LIK_CUDA_OK(cudaFuncSetAttribute(bwd_fused16_kernel<T, G, CH_, NT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM)); \
+    bwd_fused16_kernel<T, G, CH_, NT_><<<grid, NT_, pl.fused_bytes, st>>>(P, F), ::lik::count_launch();                              \
+  } while (0)
+#define LIK_FUSED_NT(CH_)                               \
+  do {                                                  \
+    if (pl.fused_threads == 256) LIK_FUSED(CH_, 256);   \
+    else LIK_FUSED(CH_, 512);                           \
+  } while (0)
+    if (row_bytes <= 256) LIK_FUSED_NT(1);
+    else if (row_bytes <= 512) LIK_FUSED_NT(2);
+    else LIK_FUSED_NT(4);
+#undef LIK_FUSED_NT
+#undef LIK_FUSED
+    LIK_CUDA_OK(cudaGetLastError());
+  } else if (a.grad_d && !list && a.deterministic && a.d.n_seq > 0 && a.d.max_len > 0) {
     if (pl.sorted) {
       DdSortOut O;
       O.pairs = (int2*)(ws + pl.pairs_off);
@@ -1687,7 +1897,7 @@ int run_bwd(const lik_bwd_args& a, BwdParams& P, const BwdPlan& pl, cudaStream_t
       cfg.dynamicSmemBytes = pl.sort_smem;
       cfg.stream = st;
       cfg.attrs = &attr;
-      cfg.numAttrs = 1;
+      cfg.numAttrs = pl.sort_cluster > 1 ? 1 : 0;  // (a launch with clusters of one took 14 us more over 2048 documents)
       LIK_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, P, O, pl.ld_pad, pl.sort_warps));
       ::lik::count_launch();
       if (pl.row16) {
