@@ -1376,7 +1376,7 @@ struct FusedShape {
   int ld_pad, n_hist;
   int parts;                    // blocks per document: each sorts all of its winners and stores every parts-th run of rows
 };
-inline size_t fused_smem(int n_ent, int ld_pad, int n_hist) { return (size_t)n_ent * sizeof(int2) + ((size_t)n_hist + 2) * ld_pad * 4 + 64 * 4; }
+inline size_t fused_smem(int n_ent, int ld_pad, int n_hist) { return (size_t)n_ent * sizeof(int2) + ((size_t)n_hist + 3) * ld_pad * 4 + 64 * 4; }
 
 template <typename T, typename G, int CH, int NT>
 __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape F) {
@@ -1414,7 +1414,16 @@ __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape
   int* hist = reinterpret_cast<int*>(list + n_ent);           // [n_hist][ld_pad]
   int* begin = hist + F.n_hist * F.ld_pad;                    // [ld_pad]
   int* cnt = begin + F.ld_pad;                                // [ld_pad]
-  int* wsum = cnt + F.ld_pad;                                 // [NT / 32]
+  int* live = cnt + F.ld_pad;                                 // [ld_pad] this block's tokens with a winner
+  int* wsum = live + F.ld_pad;                                // [NT / 32 + 1]
+  float zero[CH][Vec16<T>::N];
+#pragma unroll
+  for (int c = 0; c < CH; ++c)
+#pragma unroll
+    for (int e = 0; e < Vec16<T>::N; ++e) zero[c][e] = 0.f;
+  // Mostly rows without a winner: all are cleared while the winners are on their way, and the few others, listed by the
+  // scan below so that every half-warp has its share of them, are written again.
+  const bool prefill = n_ent * 2 < d_rows;
   if (fits) {
     for (int x = tid; x < F.n_hist * F.ld_pad; x += NT) hist[x] = 0;
     // the winners of this thread: round k is entry k * NT + tid
@@ -1429,6 +1438,8 @@ __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape
         t_r[k] = __ldg(P.argmax + doc_slot(P, ds, j, ii) * lq + s);
       }
     }
+    if (prefill)
+      for (int t = part * TOK + hw; t < d_rows; t += TOK * F.parts) store_row16<T, G, CH>((G*)P.grad_d + (drow0 + t) * P.dim, zero, P.dim, hl);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < ROUNDS; ++k) {
@@ -1456,6 +1467,7 @@ __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape
       for (int w = 0; w < F.n_hist; ++w) c += hist[w * F.ld_pad + t];
       cnt[t] = c;
       sum += c;
+      if (c && (t / TOK) % F.parts == part) sum += 1 << 16;  // (at most 4096 winners and 1536 tokens: one scan for both counts)
     }
     int incl = sum;
 #pragma unroll
@@ -1465,9 +1477,12 @@ __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape
     }
     if (lane == 31) wsum[warp] = incl;
     __syncthreads();
-    int pos = incl - sum;
-    for (int w = 0; w < warp; ++w) pos += wsum[w];
+    int at = incl - sum;
+    for (int w = 0; w < warp; ++w) at += wsum[w];
+    if (tid == NT - 1) wsum[NT / 32] = (at + sum) >> 16;
+    int pos = at & 0xFFFF, n_live = at >> 16;
     for (int t = t0; t < t1; ++t) {
+      if (cnt[t] && (t / TOK) % F.parts == part) live[n_live++] = t;
       begin[t] = pos;
       for (int w = 0; w < F.n_hist; ++w) {
         const int c = hist[w * F.ld_pad + t];
@@ -1498,14 +1513,17 @@ __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape
     }
     __syncthreads();
   }
+  if (prefill && fits) {
+    const int n_live = wsum[NT / 32];
+    for (int u = hw; u < n_live; u += TOK) {
+      const int t = live[u];
+      dd_reduce16_list<T, G, CH>(P, list + begin[t], cnt[t], drow0 + t, hl);
+    }
+    return;
+  }
   for (int t = part * TOK + hw; t < d_rows; t += TOK * F.parts) {
     const int c = fits && t < dlen ? cnt[t] : 0;
     if (c == 0) {
-      float zero[CH][Vec16<T>::N];
-#pragma unroll
-      for (int cc = 0; cc < CH; ++cc)
-#pragma unroll
-        for (int e = 0; e < Vec16<T>::N; ++e) zero[cc][e] = 0.f;
       store_row16<T, G, CH>((G*)P.grad_d + (drow0 + t) * P.dim, zero, P.dim, hl);
     } else {
       dd_reduce16_list<T, G, CH>(P, list + begin[t], c, drow0 + t, hl);
