@@ -44,6 +44,8 @@ constexpr int HD_TOK = 128;          // document tokens per tile
 constexpr int HD_SLAB_ROW = 128;     // bytes of one K slab per row (one swizzle span)
 constexpr int HD_SLAB = HD_TOK * HD_SLAB_ROW;  // bytes of a 128-row slab
 constexpr int HD_THREADS = 448;
+// Up to this many ragged documents are dealt to the CTAs by length (see the kernel); more even out by themselves.
+constexpr int HD_DEAL_MAX = 1024;
 constexpr int HD_EPI_WARP0 = 6;  // warps 2..5 convert, warps 6.. score
 constexpr int HD_MAX_STAGES = 6;
 constexpr long long HD_WAIT_LIMIT = 4000000000ll;  // about 2 s at 2 GHz
@@ -58,6 +60,7 @@ struct HeadParams {
   int n_k;                     // 128-byte K slabs of the projection
   int n_s2;                    // 128-byte K slabs of the scoring MMA (d_out)
   int stages;
+  int deal;                    // documents are dealt by length instead of in contiguous ranges
   int mt;                      // resident query tiles (1 or 2)
   int n_q, lq, q_per_tile;
   int q_last_rows;             // rows held of the last query tile (a multiple of 8): the rows behind them are never looked at
@@ -83,6 +86,7 @@ struct HeadCtl {
   alignas(16) float col_scale[2][HD_TOK];
   alignas(16) float col_bias[2][HD_TOK];
   float emit[2][2][TILE_M];
+  int docs[HD_DEAL_MAX / 64];  // dealt documents: this CTA's, longest first
 };
 
 __device__ __noinline__ bool hd_wait_slow(uint32_t b, uint32_t parity, HeadCtl* ctl, int* status) {
@@ -101,6 +105,11 @@ __device__ __forceinline__ bool hd_wait(unsigned long long* bar, uint32_t parity
   const uint32_t b = smem_u32(bar);
   if (mbar_try_wait(b, parity)) return true;
   return hd_wait_slow(b, parity, ctl, status);
+}
+
+// the same for all lanes of a warp, with one answer
+__device__ __forceinline__ bool hd_wait_warp(unsigned long long* bar, uint32_t parity, HeadCtl* ctl, int* status) {
+  return __all_sync(0xffffffffu, hd_wait(bar, parity, ctl, status));
 }
 
 // Tokens of document `doc` that take part (its tiles cover [0, len)).
@@ -214,14 +223,39 @@ head_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
     tmem_alloc(smem_u32(&ctl->tmem_base), 512);
     tmem_relinquish();
   }
+  // This CTA's documents: a contiguous range, or, when a few ragged documents per CTA would leave some CTAs twice the
+  // others' tokens, every CTA's turn in a deal from the longest to the shortest, there and back (c, 2 G - 1 - c, 2 G + c,
+  // ...).  Every CTA ranks all documents for itself; the ring is still free to hold the lengths.  256 documents of 200 to
+  // 1 024 tokens: the fullest CTA goes from 1.9 to 1.04 times the mean.
+  int doc_lo = 0, n_my = 0;
+  if (P.deal) {
+    const int G = gridDim.x, c = blockIdx.x, nd4 = (P.n_d + 3) & ~3;
+    int* len = reinterpret_cast<int*>(ring);
+    for (int j = tid; j < nd4; j += HD_THREADS) len[j] = j < P.n_d ? hd_doc_len(P, j) : -1;
+    __syncthreads();
+    for (int j = tid; j < P.n_d; j += HD_THREADS) {
+      const int l = len[j];
+      int rank = 0;
+      for (int k = 0; k < nd4; k += 4) {
+        const int4 v = *reinterpret_cast<const int4*>(len + k);
+        rank += (v.x > l || (v.x == l && k < j)) + (v.y > l || (v.y == l && k + 1 < j)) + (v.z > l || (v.z == l && k + 2 < j)) +
+                (v.w > l || (v.w == l && k + 3 < j));
+      }
+      const int turn = rank / G, pos = rank - turn * G;
+      if (((turn & 1) ? G - 1 - pos : pos) == c) ctl->docs[turn] = j;
+    }
+    for (; n_my * G < P.n_d; ++n_my)
+      if (n_my * G + ((n_my & 1) ? G - 1 - c : c) >= P.n_d) break;
+  } else {
+    doc_lo = (int)((long long)P.n_d * blockIdx.x / gridDim.x);
+    n_my = (int)((long long)P.n_d * (blockIdx.x + 1) / gridDim.x) - doc_lo;
+  }
+  if (P.deal) fence_proxy_async();  // (the lengths were written where copies will land)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
-
-  // this CTA's documents
-  const int doc_lo = (int)((long long)P.n_d * blockIdx.x / gridDim.x);
-  const int doc_hi = (int)((long long)P.n_d * (blockIdx.x + 1) / gridDim.x);
+  auto my_doc = [&](int x) { return P.deal ? ctl->docs[x] : doc_lo + x; };
   const int ab_format = P.f16 ? 0 : 1;
 
   if (warp == 0) {
@@ -239,7 +273,8 @@ head_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
                         smem_u32(&ctl->q_full));
       }
       const uint32_t stage_tx = (uint32_t)(HD_SLAB + P.d_out * HD_SLAB_ROW);
-      for (int doc = doc_lo; doc < doc_hi && ok; ++doc) {
+      for (int x = 0; x < n_my && ok; ++x) {
+        const int doc = my_doc(x);
         const int len = hd_doc_len(P, doc);
         const long long row0 = (long long)doc * P.seq_stride;
         for (int t0 = 0; t0 < len && ok; t0 += HD_TOK) {
@@ -274,7 +309,10 @@ head_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
     }
   } else if (warp == 1) {
     // =========================== MMA issuer ===========================
-    if (lane == 0) {
+    // (the whole warp runs the loop and one elected lane issues: the descriptors then sit in uniform registers, where
+    // tcgen05.mma takes them from)
+    {
+      const bool issue = elect_one();
       uint32_t st = 0, ph = 0, n1 = 0, n2 = 0;
       bool ok = true, have_pend = false;
       int pend_cols = 0;
@@ -285,19 +323,19 @@ head_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
       const uint32_t idesc1 = instr_desc(ab_format, P.d_out);
       const uint32_t idesc2_0 = instr_desc(ab_format, 0);
       const int k2_steps = P.d_out / 16;
-      const uint32_t full0 = smem_u32(&ctl->ring_full[0]), empty0 = smem_u32(&ctl->ring_empty[0]);
       const uint32_t last_q_slab = (uint32_t)((P.q_last_rows * HD_SLAB_ROW) >> 4);  // slab pitch of the last (trimmed) query tile
       // scoring MMA of the tile converted last: every resident query tile against the tile's tokens
       auto score_tile = [&](int ncols) -> bool {
-        if (n2 == 0 && !hd_wait(&ctl->q_full, 0, ctl, P.status)) return false;
-        if (!hd_wait(&ctl->p_full, n2 & 1, ctl, P.status)) return false;
+        if (n2 == 0 && !hd_wait_warp(&ctl->q_full, 0, ctl, P.status)) return false;
+        if (!hd_wait_warp(&ctl->p_full, n2 & 1, ctl, P.status)) return false;
         const uint32_t idesc2 = idesc2_0 | ((uint32_t)((ncols + 31) >> 5) << 19);  // N / 8 in bits 17..22, N a multiple of 32
         for (int m = 0; m < P.mt; ++m) {
-          if (!hd_wait(&ctl->acc2_empty[m], (n2 & 1) ^ 1, ctl, P.status)) return false;
+          if (!hd_wait_warp(&ctl->acc2_empty[m], (n2 & 1) ^ 1, ctl, P.status)) return false;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + 256u + (uint32_t)(m * HD_TOK);
           const uint32_t a0 = q_desc0 + (uint32_t)((m * q_tile_bytes) >> 4);
           const uint32_t a_slab = m == P.mt - 1 ? last_q_slab : (uint32_t)(HD_SLAB >> 4);
+          if (!issue) continue;
           if (k2_steps == 8) {
             tc_mma_slab_f16(d_tmem, a0, p_desc0, desc_hi, idesc2, 0u);
             tc_mma_slab_f16(d_tmem, a0 + a_slab, p_desc0 + (uint32_t)(HD_SLAB >> 4), desc_hi, idesc2, 1u);
@@ -308,31 +346,35 @@ head_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
           }
           tc_commit(smem_u32(&ctl->acc2_full[m]));
         }
-        tc_commit(smem_u32(&ctl->p_empty));
+        __syncwarp();
+        if (issue) tc_commit(smem_u32(&ctl->p_empty));
         ++n2;
         return true;
       };
-      for (int doc = doc_lo; doc < doc_hi && ok; ++doc) {
+      for (int x = 0; x < n_my && ok; ++x) {
+        const int doc = my_doc(x);
         const int len = hd_doc_len(P, doc);
         for (int t0 = 0; t0 < len && ok; t0 += HD_TOK) {
           const uint32_t a = n1 & 1;
-          ok = hd_wait(&ctl->acc1_empty[a], ((n1 >> 1) & 1) ^ 1, ctl, P.status);
+          ok = hd_wait_warp(&ctl->acc1_empty[a], ((n1 >> 1) & 1) ^ 1, ctl, P.status);
           if (!ok) break;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + a * (uint32_t)HD_TOK;
           for (int ks = 0; ks < P.n_k; ++ks) {
             // (data landed by TMA and consumed by the MMA: the barrier alone orders the two)
-            if (!mbar_try_wait(full0 + 8u * st, ph)) {
-              ok = hd_wait_slow(full0 + 8u * st, ph, ctl, P.status);
-              if (!ok) break;
-            }
+            ok = hd_wait_warp(&ctl->ring_full[st], ph, ctl, P.status);
+            if (!ok) break;
             const uint32_t h_desc = ring_desc0 + st * (uint32_t)(STAGE_BYTES >> 4);
-            tc_mma_slab_f16(d_tmem, h_desc, h_desc + (uint32_t)(HD_SLAB >> 4), desc_hi, idesc1, (uint32_t)ks);
-            tc_commit(empty0 + 8u * st);
+            if (issue) {
+              tc_mma_slab_f16(d_tmem, h_desc, h_desc + (uint32_t)(HD_SLAB >> 4), desc_hi, idesc1, (uint32_t)ks);
+              tc_commit(smem_u32(&ctl->ring_empty[st]));
+            }
+            __syncwarp();
             if (++st == (uint32_t)P.stages) { st = 0; ph ^= 1; }
           }
           if (!ok) break;
-          tc_commit(smem_u32(&ctl->acc1_full[a]));
+          if (issue) tc_commit(smem_u32(&ctl->acc1_full[a]));
+          __syncwarp();
           ++n1;
           if (have_pend) ok = score_tile(pend_cols);
           pend_cols = min(HD_TOK, len - t0);
@@ -349,7 +391,8 @@ head_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
     unsigned char* row_base = p_smem + row * HD_SLAB_ROW;
     uint32_t n1 = 0;
     bool ok = true;
-    for (int doc = doc_lo; doc < doc_hi && ok; ++doc) {
+    for (int x = 0; x < n_my && ok; ++x) {
+        const int doc = my_doc(x);
       const int len = hd_doc_len(P, doc);
       const long long row0 = (long long)doc * P.seq_stride;
       for (int t0 = 0; t0 < len; t0 += HD_TOK) {
@@ -400,7 +443,8 @@ head_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
       const bool in_q = row < q_here * P.lq;
       uint32_t n = 0, n_doc = 0;
       bool ok = true;
-      for (int doc = doc_lo; doc < doc_hi && ok; ++doc) {
+      for (int x = 0; x < n_my && ok; ++x) {
+        const int doc = my_doc(x);
         const int len = hd_doc_len(P, doc);
         float run_m = -INFINITY;
         int run_i = -1;
@@ -454,6 +498,7 @@ head_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
   }
 
   // ---- teardown (also reached when aborting: every wait above is bounded) ----
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -668,6 +713,7 @@ extern "C" int lik_maxsim_hidden_fwd(const lik_hidden_fwd_args* args, lik_stream
     P.lens = eff;
     P.lens_flagged = 1;
   }
+  P.deal = P.lens && a.h.n_seq > pl.grid && a.h.n_seq <= HD_DEAL_MAX && ceil_div(a.h.n_seq, pl.grid) <= HD_DEAL_MAX / 64;
   P.d_model = a.d_model;
   P.d_out = a.d_out;
   P.n_k = pl.n_k;
