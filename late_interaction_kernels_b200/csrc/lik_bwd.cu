@@ -1366,7 +1366,7 @@ __global__ void __launch_bounds__(256) bwd_dd_reduce16_walk_kernel(BwdParams P, 
 // the first dq_blocks blocks are grad_q blocks, the others take a document each - the counting sort of its winners stays in
 // shared memory and the same block reduces and stores the document's rows.  Such problems are bound by launches and by the
 // zero rows of grad_d, not by gathers: against sort and reduce kernels this saves two launches, the list's round trip
-// and a scheduling pass over 16-row blocks.  64 x 32 candidate lists of 300 tokens: 75 -> 45 us; a 16 x 16 batch 26 -> 14 us.
+// and a scheduling pass over 16-row blocks.  64 x 32 candidate lists of 300 tokens: 75 -> 45 us; a 16 x 16 batch 26 -> 12 us.
 // The order inside a token's list is (warp, round, lane): fixed by the data alone.
 // ---------------------------------------------------------------------------------
 constexpr int FUSED_ENT = 4096;  // most winners of a document

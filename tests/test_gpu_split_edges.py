@@ -1,0 +1,158 @@
+"""Kernels and launch rules at the sizes where a split or a tile changes: one parametrised test each.
+
+Integer-valued inputs make sums exact in fp32 (every partial sum is far below 2**24), whatever their order: scores and
+winners are compared with ``==``, and a gradient is the exact sum rounded once to the output type."""
+
+import numpy as np
+import pytest
+import torch
+
+import cases
+from oracle import maxsim_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def dev(x, dtype=None):
+    if x is None:
+        return None
+    t = torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    return t.to(dtype) if dtype is not None else t
+
+
+def f32(t):
+    return t.detach().float().cpu().numpy()
+
+
+def ints(rng, *shape):
+    return rng.integers(-2, 3, size=shape).astype(np.float32)
+
+
+def once_rounded(x, dtype):
+    return torch.from_numpy(np.ascontiguousarray(x, dtype=np.float32)).to(dtype)
+
+
+# entries of a document = queries x query tokens.  One launch for both gradients up to 4096 entries and 1536 document
+# tokens (from 1025 entries on only with 96 documents or more); sorted by a cluster of CTAs per document from 4096 entries
+# with few documents; one CTA per document otherwise.
+@pytest.mark.parametrize("Nq,Lq,Nd,Ld,dtype", [
+    (1, 1, 1, 1, torch.bfloat16),         # one entry, one row
+    (3, 5, 2, 1536, torch.float16),       # the longest document of one launch, several blocks per document
+    (3, 5, 2, 1537, torch.bfloat16),      # one token more: sorted and reduced separately
+    (16, 32, 7, 180, torch.bfloat16),     # 512 entries: 256 threads
+    (3, 171, 7, 33, torch.bfloat16),      # 513 entries, rows of 171 winners (not a multiple of four): 512 threads
+    (32, 32, 95, 17, torch.float16),      # 1024 entries: the last with few documents
+    (25, 41, 95, 17, torch.bfloat16),     # 1025 entries and 95 documents: separate
+    (25, 41, 96, 17, torch.bfloat16),     # ... and 96: one launch
+    (32, 128, 97, 40, torch.bfloat16),    # 4096 entries
+    (241, 17, 97, 40, torch.bfloat16),    # 4097
+    (64, 130, 3, 50, torch.bfloat16),     # cluster of four, rows of 130 winners
+    (300, 128, 1, 2000, torch.float16),   # cluster of eight, one document, query rows split over blocks
+])
+def test_backward_splits(Nq, Lq, Nd, Ld, dtype):
+    import late_interaction_kernels_b200 as lik
+    from late_interaction_kernels_b200.forward import maxsim_forward
+
+    rng = np.random.default_rng(Nq * 131 + Nd)
+    Q, D, g = ints(rng, Nq, Lq, 64), ints(rng, Nd, Ld, 64), ints(rng, Nq, Nd)
+    dm = cases.prefix_mask(rng.integers(0, Ld + 1, size=Nd), Ld)
+    dm[0] = True
+    tQ, tD = dev(Q, dtype).requires_grad_(True), dev(D, dtype).requires_grad_(True)
+    (lik.maxsim(tQ, tD, None, dev(dm)) * dev(g)).sum().backward()
+    _, am = maxsim_forward(tQ.detach(), tD.detach(), None, dev(dm), save_argmax=True)
+    wq, wd = O.backward_from_argmax(g, Q, D, am.cpu().numpy().reshape(Nq, Nd, Lq))
+    assert torch.equal(tQ.grad.cpu(), once_rounded(wq, dtype))
+    assert torch.equal(tD.grad.cpu(), once_rounded(wd, dtype))
+
+
+@pytest.mark.parametrize("Nq,K,Lq,Ld", [(1, 1, 4, 9), (5, 7, 30, 129), (40, 5, 33, 64)])
+def test_backward_of_candidate_lists_and_packed_rows_without_owner(Nq, K, Lq, Ld):
+    import late_interaction_kernels_b200 as lik
+    from late_interaction_kernels_b200.forward import maxsim_forward
+
+    rng = np.random.default_rng(Nq + K)
+    Q, D, g = ints(rng, Nq, Lq, 128), ints(rng, Nq, K, Ld, 128), ints(rng, Nq, K)
+    tQ, tD = dev(Q, torch.bfloat16).requires_grad_(True), dev(D, torch.bfloat16).requires_grad_(True)
+    (lik.maxsim(tQ, tD) * dev(g)).sum().backward()
+    wq, wd = np.zeros_like(Q), np.zeros_like(D)
+    for i in range(Nq):
+        _, am = O.maxsim(Q[i : i + 1], D[i], None, None, return_argmax=True)  # ties to the lower column, as the kernel
+        wq[i : i + 1], wd[i] = O.backward_from_argmax(g[i : i + 1], Q[i : i + 1], D[i], am)
+    assert torch.equal(tQ.grad.cpu(), once_rounded(wq, torch.bfloat16))
+    assert torch.equal(tD.grad.cpu(), once_rounded(wd, torch.bfloat16))
+    # packed: rows in front of the first and behind the last document belong to none, their gradient is zero
+    dl = rng.integers(0, Ld + 1, size=K)
+    dl[-1] = Ld
+    cu_d = (3 + np.concatenate([[0], np.cumsum(dl)])).astype(np.int32)
+    cu_q = (np.arange(Nq + 1) * Lq).astype(np.int32)
+    Dp = ints(rng, int(cu_d[-1]) + 13, 128)
+    tQ, tD = dev(Q.reshape(-1, 128), torch.bfloat16).requires_grad_(True), dev(Dp, torch.bfloat16).requires_grad_(True)
+    (lik.maxsim_varlen(tQ, tD, dev(cu_q), dev(cu_d), Lq, Ld) * dev(g)).sum().backward()
+    wq, wd = O.varlen_grads(g, Q.reshape(-1, 128), Dp, cu_q, cu_d)
+    assert torch.equal(tQ.grad.cpu(), once_rounded(wq, torch.bfloat16))
+    assert torch.equal(tD.grad.cpu(), once_rounded(wd, torch.bfloat16))
+
+
+# fp32 tiles: 32 query tokens of one or two queries x 128 document tokens, slabs of 64 features
+@pytest.mark.parametrize("Nq,Lq,Nd,Ld,d", [(1, 1, 1, 1, 1), (2, 31, 3, 127, 63), (2, 32, 2, 128, 64), (3, 33, 5, 129, 65), (5, 7, 4, 257, 132)])
+def test_exact_fp32_tiles(Nq, Lq, Nd, Ld, d):
+    from late_interaction_kernels_b200.forward import maxsim_forward
+
+    rng = np.random.default_rng(Ld)
+    Q, D = ints(rng, Nq, Lq, d), ints(rng, Nd, Ld, d)
+    dm = cases.prefix_mask(rng.integers(1, Ld + 1, size=Nd), Ld)
+    holes = rng.random((Nd, Ld)) < 0.6
+    for m in (None, dm, holes):
+        want, am = O.maxsim(Q, D, None, m, return_argmax=True)
+        s, got = maxsim_forward(dev(Q), dev(D), None, dev(m), save_argmax=True)
+        assert np.array_equal(f32(s), want) and np.array_equal(got.cpu().numpy().reshape(am.shape), am)
+
+
+# candidate lists of every CTA merged at once (many queries) or in parts (few), lists shorter and longer than k, ties
+@pytest.mark.parametrize("Nq,Nd,k", [(1, 1, 1), (1, 149, 149), (1, 20000, 100), (2, 30000, 128), (9, 9000, 127), (40, 3000, 33)])
+def test_candidate_lists_are_merged_in_order(Nq, Nd, k):
+    from late_interaction_kernels_b200.topk import maxsim_topk
+
+    rng = np.random.default_rng(Nd)
+    Q, D = ints(rng, Nq, 8, 32), ints(rng, Nd, 3, 32)
+    for largest in (True, False):
+        s, i = maxsim_topk(dev(Q, torch.bfloat16), dev(D, torch.bfloat16), k, largest=largest)
+        full = torch.from_numpy(O.maxsim(Q, D))
+        order = torch.sort(full, dim=-1, descending=largest, stable=True).indices[:, :k]
+        assert torch.equal(i.cpu(), order) and torch.equal(s.cpu().double(), torch.gather(full, 1, order).double())
+
+
+# norm groups of 8, 16 and 32 lanes with 16-byte loads; rows that do not start on 16 bytes element by element.  Rows are
+# one-hot times a power of two: the norm is a power of two, the normalised row and so the scores are exact.
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("d", [1, 8, 33, 64, 136, 264, 520])
+def test_row_norms_by_width(dtype, d):
+    import late_interaction_kernels_b200 as lik
+
+    rng = np.random.default_rng(d)
+    def rows(n, length):
+        x = np.zeros((n, length, d), np.float32)
+        at = rng.integers(0, d, size=(n, length))
+        np.put_along_axis(x, at[..., None], (2.0 ** rng.integers(-3, 4, size=(n, length)) * rng.choice([-1, 1], size=(n, length)))[..., None].astype(np.float32), -1)
+        return x
+    Q, D = rows(3, 5), rows(37, 21)
+    dm = cases.prefix_mask(rng.integers(1, 22, size=37), 21)
+    want = O.maxsim(np.sign(Q), np.sign(D), None, dm)
+    big = torch.zeros(D.size + 1, device="cuda", dtype=dtype)
+    shifted = big[1:].view(D.shape)  # starts 2 or 4 bytes behind a 16-byte boundary
+    shifted.copy_(dev(D))
+    for t in (dev(D, dtype), shifted):
+        assert np.array_equal(f32(lik.maxsim(dev(Q, dtype), t, None, dev(dm), normalize=True)), want)
+
+
+# documents of a masked batch are dealt to the CTAs by length up to 1024 of them, in ranges beyond
+@pytest.mark.parametrize("Nd,Ld,lens", [(149, 130, "empty"), (300, 70, "ragged"), (297, 140, "same"), (1024, 9, "ragged"), (1025, 9, "ragged")])
+def test_document_head_deals_ragged_documents(Nd, Ld, lens):
+    from late_interaction_kernels_b200.fused_head import maxsim_from_hidden
+
+    rng = np.random.default_rng(Nd)
+    n = {"empty": np.where(np.arange(Nd) % 3, 0, Ld), "ragged": rng.integers(0, Ld + 1, size=Nd), "same": np.full(Nd, Ld - 1)}[lens]
+    Q, H, W = ints(rng, 2, 9, 32), ints(rng, Nd, Ld, 64), np.eye(32, 64, dtype=np.float32)  # projected rows are integers too
+    dm = cases.prefix_mask(n, Ld)
+    got = maxsim_from_hidden(*(dev(x, torch.bfloat16) for x in (Q, H, W)), None, dev(dm), normalize=False)
+    assert np.array_equal(f32(got), O.maxsim(Q, H[..., :32], None, dm))
