@@ -32,7 +32,8 @@ __device__ __forceinline__ int load_u8_if(const unsigned char* p, bool on) {
 __device__ __forceinline__ bool norm_row_live(const NormJob& J, long long row) {
   if (row >= J.n_rows) return false;
   if (J.lens) {
-    const long long j = row / J.seq_stride;
+    // (64-bit divisions are a hundred instructions: only where 32 bits do not hold the row)
+    const long long j = J.n_rows < (1ll << 31) ? (long long)((unsigned)row / (unsigned)J.seq_stride) : row / J.seq_stride;
     if (row - j * J.seq_stride >= J.lens[j]) return false;
   }
   return true;
@@ -84,42 +85,52 @@ __device__ __forceinline__ float sum_sq16<e4m3_t>(const uint4& r) {
 // lanes that cover a row: as many as it has 16-byte pieces, at most a warp
 __host__ __device__ inline int norm_lanes(long long row_bytes) { return row_bytes <= 128 ? 8 : (row_bytes <= 256 ? 16 : 32); }
 
-template <typename T>
+template <typename T, int L>
 __device__ __forceinline__ void norm_rows_vec(const NormJob& J, int block) {
   const int row_bytes = J.dim * (int)sizeof(T);
-  const int L = norm_lanes(row_bytes);
-  const int gl = threadIdx.x & (L - 1), g = threadIdx.x / L, groups = PREP_THREADS / L;
+  constexpr int groups = PREP_THREADS / L;
+  const int gl = threadIdx.x & (L - 1), g = threadIdx.x / L;
   const long long row0 = (long long)block * groups * NORM_ROWS + g;
-  const char* base = static_cast<const char*>(J.data);
   float ss[NORM_ROWS];
   bool live[NORM_ROWS];
 #pragma unroll
   for (int u = 0; u < NORM_ROWS; ++u) {
     ss[u] = 0.f;
-    const long long row = row0 + (long long)u * groups;
-    live[u] = norm_row_live(J, row);
+    live[u] = norm_row_live(J, row0 + u * groups);
   }
   if (J.mask) {
     int mb[NORM_ROWS];
+    const unsigned char* m = J.mask + row0;
 #pragma unroll
-    for (int u = 0; u < NORM_ROWS; ++u) mb[u] = load_u8_if(J.mask + row0 + (long long)u * groups, live[u]);
+    for (int u = 0; u < NORM_ROWS; ++u) mb[u] = load_u8_if(m + u * groups, live[u]);
 #pragma unroll
     for (int u = 0; u < NORM_ROWS; ++u) live[u] = mb[u] != 0;
   }
-  const long long pitch = J.stride * (long long)sizeof(T);
-  for (int b = gl * 16; b < row_bytes; b += L * 16) {
-    uint4 r[NORM_ROWS];
+  const long long pitch = J.stride * (long long)sizeof(T), step = pitch * groups;
+  const char* p = static_cast<const char*>(J.data) + row0 * pitch + gl * 16;
+  if (__any_sync(0xffffffffu, live[0] | live[1] | live[2] | live[3])) {
+    for (int b = gl * 16; b < row_bytes; b += L * 16, p += L * 16) {
+      uint4 r[NORM_ROWS];
 #pragma unroll
-    for (int u = 0; u < NORM_ROWS; ++u) r[u] = load16_if(base + (row0 + (long long)u * groups) * pitch + b, live[u]);
+      for (int u = 0; u < NORM_ROWS; ++u) r[u] = load16_if(p + u * step, live[u]);
 #pragma unroll
-    for (int u = 0; u < NORM_ROWS; ++u) ss[u] += sum_sq16<T>(r[u]);
+      for (int u = 0; u < NORM_ROWS; ++u) ss[u] += sum_sq16<T>(r[u]);
+    }
   }
+  // The sums of the four rows in one butterfly: at the first two steps a lane hands over the rows that it will not finish,
+  // so that every quarter of the group ends up with one row (a fifth of the shuffles, a quarter of the roots and divisions).
+  const bool up2 = gl & (L / 2), up1 = gl & (L / 4);
+  float a0 = up2 ? ss[2] : ss[0], a1 = up2 ? ss[3] : ss[1];
+  a0 += __shfl_xor_sync(0xffffffffu, up2 ? ss[0] : ss[2], L / 2);
+  a1 += __shfl_xor_sync(0xffffffffu, up2 ? ss[1] : ss[3], L / 2);
+  float v = up1 ? a1 : a0;
+  v += __shfl_xor_sync(0xffffffffu, up1 ? a0 : a1, L / 4);
 #pragma unroll
-  for (int u = 0; u < NORM_ROWS; ++u) {
-    for (int o = L >> 1; o > 0; o >>= 1) ss[u] += __shfl_xor_sync(0xffffffffu, ss[u], o);
-    const long long row = row0 + (long long)u * groups;
-    if (gl == 0 && row < J.n_rows) J.out[row] = live[u] ? 1.0f / fmaxf(sqrtf(ss[u]), J.eps) : 0.f;
-  }
+  for (int o = L / 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  const int u = (up2 ? 2 : 0) + (up1 ? 1 : 0);
+  const bool on = up2 ? (up1 ? live[3] : live[2]) : (up1 ? live[1] : live[0]);
+  const long long row = row0 + u * groups;
+  if ((gl & (L / 4 - 1)) == 0 && row < J.n_rows) J.out[row] = on ? 1.0f / fmaxf(sqrtf(v), J.eps) : 0.f;
 }
 
 // any width and alignment: a warp per row
@@ -148,8 +159,14 @@ __host__ __device__ inline bool norm_vec_ok(const NormJob& J) {
 
 template <typename T>
 __device__ __forceinline__ void norm_block(const NormJob& J, int block) {
-  if (norm_vec_ok(J)) norm_rows_vec<T>(J, block);
-  else norm_rows_any<T>(J, block);
+  if (!norm_vec_ok(J)) {
+    norm_rows_any<T>(J, block);
+    return;
+  }
+  const int L = norm_lanes((long long)J.dim * (int)sizeof(T));
+  if (L == 8) norm_rows_vec<T, 8>(J, block);
+  else if (L == 16) norm_rows_vec<T, 16>(J, block);
+  else norm_rows_vec<T, 32>(J, block);
 }
 
 // a warp per document
