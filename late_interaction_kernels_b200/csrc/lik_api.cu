@@ -91,7 +91,7 @@ FwdPlan plan_fwd(const lik_fwd_args& a, const TcExtra& x = TcExtra()) {
   }
   if (norm_d) {
     if (pl.copies) pl.dcopy_off = take((size_t)a.d.n_rows * a.dim * eb);
-    else pl.dn_off = take((size_t)a.d.n_rows * 4);
+    else pl.dn_off = take((size_t)a.d.n_rows * 4);  // (also where the kernel takes the norms itself: a caller's buffer fits by size alone)
   }
   // the portable kernel trims masked documents too
   if (!pl.use_tc && a.d.mask && !a.d.cu) pl.lens_off = take((size_t)a.d.n_seq * 4);
@@ -104,6 +104,7 @@ int run_fwd(const lik_fwd_args& a, const FwdPlan& pl, cudaStream_t st, const TcE
   int rc;
   lik_fwd_args b = a;
   const float *qn = nullptr, *dn = nullptr;
+  float norm_d_eps = 0.f;  // > 0: the scoring kernel takes the documents' norms itself
   PrepJobs prep;
   if (a.normalize & LIK_NORM_Q) {
     if (pl.copies) {
@@ -123,6 +124,8 @@ int run_fwd(const lik_fwd_args& a, const FwdPlan& pl, cudaStream_t st, const TcE
       if (rc) return rc;
       b.d.data = ws + pl.dcopy_off;
       b.d.row_stride = a.dim;
+    } else if (pl.use_tc && fwd_tc_norms_in_kernel(a, x)) {
+      norm_d_eps = kFwdNormEps;
     } else {
       float* w = (float*)(ws + pl.dn_off);
       prep.norm[1] = norm_job(a.d, a.dtype, a.dim, kFwdNormEps, w, false);
@@ -130,7 +133,7 @@ int run_fwd(const lik_fwd_args& a, const FwdPlan& pl, cudaStream_t st, const TcE
     }
   }
   b.normalize = pl.copies ? 0 : (a.normalize & LIK_NORM_BOTH);
-  if (pl.use_tc) return launch_fwd_tc(b, qn, dn, prep, ws + pl.tc_off, fwd_tc_workspace(b, x), st, x);
+  if (pl.use_tc) return launch_fwd_tc(b, qn, dn, norm_d_eps, prep, ws + pl.tc_off, fwd_tc_workspace(b, x), st, x);
   if (x.plaid || x.topk_k > 0) {
     set_error("this problem is outside what the fused tensor-core path takes");
     return LIK_ERR_UNSUPPORTED;

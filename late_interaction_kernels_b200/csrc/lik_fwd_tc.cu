@@ -120,12 +120,16 @@ struct TcParams {
   // back from every earlier tile - and an epilogue gives it back only after its last read of the multipliers.
   int sc_per;
   int sc_slots;          // 2 * sc_per, or 0
+  float norm_eps;     // > 0: the kernel takes the documents' inverse norms from the tiles themselves (NORM_WARPS)
   int d_full_count;   // arrivals that complete a ring stage: 1 (TMA) or the number of decompress warps
   TopkOut topk;       // cand_key == nullptr: scores are written instead
   PlaidSrc plaid;     // PLAID kernels: the compressed documents
   int plaid_f16;      // PLAID kernels: operand type fp16 instead of bf16
 };
 
+// Warps 18 and 19 take the rows' inverse norms from the tiles in shared memory when the launch asks for it: the documents
+// are then read once instead of twice, and no norms go through device memory.
+constexpr int NORM_WARPS = 2;
 constexpr int PLAID_WARPS = 3;  // warps 0, 18 and 19 decode compressed tokens in the PLAID kernels
 
 struct SharedCtl {
@@ -356,6 +360,42 @@ __device__ __forceinline__ void unit_resolve(const TcParams& P, int doc, const U
   }
 }
 
+// Sum of squares of one row of a stage (lane = row: eight consecutive rows of a swizzled slab lie in different banks).  The
+// pieces of 16 bytes are summed and combined in the order of prep_kernel's butterfly, so that the norms of a row are the
+// same number wherever they are taken.
+template <bool BF16>
+__device__ __forceinline__ float stage_row_sum_sq(const unsigned char* row, int r, bool two_slabs) {
+  auto piece = [&](int p) {  // pieces p and p + 8 side by side
+    const unsigned char* a = row + ((p ^ (r & 7)) << 4);
+    const uint4 x = *reinterpret_cast<const uint4*>(a);
+    uint4 y = make_uint4(0, 0, 0, 0);
+    if (two_slabs) y = *reinterpret_cast<const uint4*>(a + TILE_N * SLAB_BYTES_ROW);
+    const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float2 u, w;
+      if (BF16) {
+        u = make_float2(__uint_as_float(xs[i] << 16), __uint_as_float(xs[i] & 0xffff0000u));
+        w = make_float2(__uint_as_float(ys[i] << 16), __uint_as_float(ys[i] & 0xffff0000u));
+      } else {
+        u = __half22float2(*reinterpret_cast<const __half2*>(&xs[i]));
+        w = __half22float2(*reinterpret_cast<const __half2*>(&ys[i]));
+      }
+      fma_sq2(u.y, w.y, s0, s1);
+      fma_sq2(u.x, w.x, s0, s1);
+    }
+    return s0 + s1;
+  };
+  float u[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float a = piece(i);
+    u[i] = a + piece(i + 4);
+  }
+  return (u[0] + u[2]) + (u[1] + u[3]);
+}
+
 struct DocMaps {
   CUtensorMap m[N_BOXES];  // document boxes of 32, 64, ... rows: one copy per K slab whatever the tile height
 };
@@ -444,15 +484,16 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
   const bool list = P.pairing == LIK_PAIR_LIST;
   const bool topk = !ARGMAX && P.topk.cand_key != nullptr;  // the fused top-k never saves winners
 
+  const bool norm_warps = SCALED && !FP8 && !PLAID && P.norm_eps > 0.f;  // (a member of every pipeline barrier then)
   if (tid == 0) {
     mbar_init(smem_u32(&ctl->q_full), 1);
     mbar_init(smem_u32(&ctl->q_empty), 1);
     for (int s = 0; s < P.stages; ++s) {
       mbar_init(smem_u32(&ctl->d_full[s]), (uint32_t)P.d_full_count);
-      mbar_init(smem_u32(&ctl->d_empty[s]), 1);
+      mbar_init(smem_u32(&ctl->d_empty[s]), norm_warps ? 1 + NORM_WARPS : 1);
     }
     for (int a = 0; a < 2; ++a) {
-      mbar_init(smem_u32(&ctl->acc_full[a]), 1);
+      mbar_init(smem_u32(&ctl->acc_full[a]), norm_warps ? 1 + NORM_WARPS : 1);
       mbar_init(smem_u32(&ctl->acc_empty[a]), GROUP_WARPS);
     }
     ctl->abort_flag = 0;
@@ -737,7 +778,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
     int uc = 0;
     bool ok = true;
     // per-row / per-warp state for the resident query tile
-    bool have_tile = false, in_seg = false, row_ok = false, aligned = false;
+    bool have_tile = false, warp_rows = false, in_seg = false, row_ok = false, aligned = false;
     float my_qf = 1.f;
     int tile_id = 0;
     long long arg_off = -1;   // ARGMAX: offset of this row's slot for document 0 (-1: row stores nothing)
@@ -805,7 +846,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
   } while (0)
 
     const bool cross = P.pairing == LIK_PAIR_CROSS;
-    const bool bulk = SCALED && P.col_src != nullptr;  // the multipliers of a tile arrive with it
+    const bool bulk = SCALED && P.sc_slots != 0;  // the multipliers of a tile arrive with it, or are made from it
     const bool every_group_full = P.mt == 1 || (n_tiles & 1) == 0;
     for (;; ++uc) {
       // with one resident tile the two groups take alternate units
@@ -912,6 +953,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
             if (ARGMAX && my_s < P.argmax_stride)
               arg_off = (cross ? (long long)my_q * P.n_d : 0ll) * P.argmax_stride + my_s;
           }
+          warp_rows = __any_sync(0xffffffffu, in_seg);
           const int sg0 = ctl->row_seg[wg][quad * 32];
           if (aligned && sg0 >= 0) {
             warp_seg = sg0;
@@ -949,7 +991,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
       float sc = 1.f, bi = -INFINITY;                                                                     \
       if (c < ncols) {                                                                                    \
         const long long drow = drow0 + c0 + c;                                                            \
-        sc = row_factor(P.d, drow);                                                                       \
+        sc = norm_warps ? sc_ring[sc_slot * TILE_N + c] : row_factor(P.d, drow);                          \
         bi = row_valid(P.d, drow) ? 0.f : -INFINITY;                                                      \
       }                                                                                                   \
       ctl->col_scale[wg][c] = sc;                                                                         \
@@ -958,14 +1000,14 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
   } while (0)
         // before the accumulator wait: overlaps the MMAs; the wait's rendezvous also publishes the columns
         // (not needed when the multipliers came with the tile and the mask has no holes)
-        const bool staged = SCALED && (general || !bulk);
+        const bool staged = SCALED && (general || !bulk) && !norm_warps;
         if (staged) LIK_STAGE_COLUMNS(c0 > 0);
         if (SCALED || c0 > 0) {
           LIK_GROUP_WAIT_ACC();
           if (!ok) break;
         }
         ++n_acc;
-        if (!SCALED && use_cols) {  // a document whose mask has holes: known only now
+        if (general && (!SCALED || norm_warps)) {  // a document whose mask has holes: known only now, or its multipliers are
           LIK_STAGE_COLUMNS(true);
           LIK_GRP_SYNC();
         }
@@ -979,7 +1021,8 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
     if (lane == 0) mbar_arrive(acc_empty_bar);                     \
   } while (0)
         // chunks of this half: cc, cc + 64, ...; only the tile's last chunk can be partial
-        int cc = sub * 32;
+        // (a warp without a query row, as most have under a single short query, only hands the accumulator on)
+        int cc = warp_rows ? sub * 32 : ncols;
         if (cc >= ncols) LIK_RELEASE_ACC();
         if (use_cols && general) {
           // a mask with holes: every chunk takes multiplier and additive mask
@@ -1117,6 +1160,42 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
 #undef LIK_GRP_SYNC
 #undef LIK_GRP_SYNC_COUNT
 #undef LIK_SUB_SYNC
+  } else if (SCALED && !FP8 && !PLAID && norm_warps) {
+    // =========================== inverse norms of the tiles ===========================
+    // The multipliers of a tile go into its ring slot, and the arrival that announces them belongs to the phase of the
+    // accumulator(s) that the tile feeds: the epilogue waits for both with one wait.  An arrival must not fall into the
+    // phase before, hence the wait for that one; it also says that the epilogue is done with the slots three tiles back.
+    const int nw = warp - (2 + 2 * GROUP_WARPS);
+    uint32_t st = 0, ph = 0, n_acc[2] = {0, 0};
+    int sc_cnt[2] = {0, 0};
+    bool ok = true;
+    const bool bf16 = P.ab_format == 1, two_slabs = P.n_slabs == 2;
+    while (ok) {
+      ok = wait_bar_warp(&ctl->d_full[st], ph, ctl, P.status);
+      if (!ok) break;
+      const uint32_t info = __shfl_sync(0xffffffffu, ctl->stage_info[st], 0);
+      if (info & STAGE_END) break;
+      const int ncols = (int)(info & STAGE_COLS_MASK);
+      const int ring = (info & STAGE_ACC0) ? 0 : 1;
+      float* slot = sc_ring + (ring * P.sc_per + sc_cnt[ring]) * TILE_N;
+      const unsigned char* stage = d_smem + (size_t)st * d_stage_bytes;
+      for (int r = nw * 32 + lane; r < ncols; r += NORM_WARPS * 32) {
+        const float ss = bf16 ? stage_row_sum_sq<true>(stage + r * SLAB_BYTES_ROW, r, two_slabs)
+                              : stage_row_sum_sq<false>(stage + r * SLAB_BYTES_ROW, r, two_slabs);
+        slot[r] = 1.0f / fmaxf(sqrtf(ss), P.norm_eps);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&ctl->d_empty[st]));
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        if (!ok || !(info & (STAGE_ACC0 << a))) continue;
+        if (n_acc[a]) ok = wait_bar_warp(&ctl->acc_full[a], (n_acc[a] - 1) & 1, ctl, P.status);
+        if (ok && lane == 0) mbar_arrive(smem_u32(&ctl->acc_full[a]));
+        ++n_acc[a];
+      }
+      if (++sc_cnt[ring] >= P.sc_per) sc_cnt[ring] = 0;
+      if (++st == (uint32_t)P.stages) { st = 0; ph ^= 1; }
+    }
   }
 
   // ---- teardown (also reached when aborting: every wait above is bounded) ----
@@ -1460,8 +1539,16 @@ static cudaError_t allow_smem(size_t bytes) {
   return e;
 }
 
-int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, PrepJobs prep, void* ws, size_t ws_bytes, cudaStream_t st,
-                  const TcExtra& x) {
+// A launch that reads every document once takes the documents' norms from its tiles.  (With several query-tile groups the
+// norms would be taken once per group by two warps: there they come from one pass of prep_kernel in front.)
+bool fwd_tc_norms_in_kernel(const lik_fwd_args& a, const TcExtra& x) {
+  if (!(a.normalize & LIK_NORM_D) || x.plaid || (a.dtype != LIK_BF16 && a.dtype != LIK_F16) || a.d.scale || a.d.scale_scalar != 1.0f) return false;
+  const TcPlan pl = plan_tc(a, x);
+  return pl.stages >= 2 && (a.pairing == LIK_PAIR_GROUPED || (a.pairing == LIK_PAIR_CROSS && pl.n_groups == 1));
+}
+
+int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float norm_d_eps, PrepJobs prep, void* ws, size_t ws_bytes,
+                  cudaStream_t st, const TcExtra& x) {
   TcPlan pl = plan_tc(a, x);
   if (pl.stages < 1) {
     set_error("not enough shared memory for the document ring");
@@ -1516,9 +1603,10 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, PrepJ
   // stay inside the array: padded documents whose stride and row count are multiples of four.
   P.col_src = nullptr;
   P.sc_per = P.sc_slots = 0;
-  if (!plaid && !a.d.cu && a.d.scale_scalar == 1.0f && ((a.d.scale != nullptr) != (dn != nullptr))) {
+  P.norm_eps = norm_d_eps;
+  if (norm_d_eps > 0.f || (!plaid && !a.d.cu && a.d.scale_scalar == 1.0f && ((a.d.scale != nullptr) != (dn != nullptr)))) {
     const float* arr = a.d.scale ? a.d.scale : dn;
-    if (((uintptr_t)arr & 15) == 0 && a.d.seq_stride % 4 == 0 && a.d.n_rows % 4 == 0) {
+    if (norm_d_eps > 0.f || (((uintptr_t)arr & 15) == 0 && a.d.seq_stride % 4 == 0 && a.d.n_rows % 4 == 0)) {
       const size_t stage = (size_t)pl.n_slabs * TILE_N * SLAB_BYTES_ROW;
       const size_t fixed = pl.smem_bytes - (size_t)pl.stages * stage;
       auto need = [&](int stages) { return fixed + (size_t)stages * stage + (size_t)2 * (stages + 1) * TILE_N * sizeof(float); };
@@ -1532,6 +1620,11 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, PrepJ
         P.sc_per = stages + 1;
         P.sc_slots = 2 * P.sc_per;
       }
+    }
+    if (norm_d_eps > 0.f) P.col_src = nullptr;
+    if (norm_d_eps > 0.f && P.sc_per < 3) {
+      set_error("not enough shared memory for the documents' norms");
+      return LIK_ERR_UNSUPPORTED;
     }
   }
   if (plaid) {
@@ -1584,7 +1677,7 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, PrepJ
 
   const bool fp8 = a.dtype == LIK_E4M3;
   const bool argmax = a.argmax != nullptr;
-  const bool affine = a.d.scale || dn;  // a per-column multiplier for every document
+  const bool affine = a.d.scale || dn || norm_d_eps > 0.f;  // a per-column multiplier for every document
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;

@@ -27,8 +27,10 @@ bool fwd_tc_topk_supported(const lik_fwd_args& a, const TcExtra& x);
 bool fwd_tc_plaid_supported(const lik_fwd_args& a, const TcExtra& x);
 size_t fwd_tc_workspace(const lik_fwd_args& a, const TcExtra& x);
 // `prep`: what still has to be written before the kernel runs; the launch adds its own jobs and sends them in one go
-int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, PrepJobs prep, void* ws, size_t ws_bytes, cudaStream_t st,
-                  const TcExtra& x);
+// `norm_d_eps` > 0 (where fwd_tc_norms_in_kernel says so, dn == nullptr): the kernel takes the documents' norms itself
+bool fwd_tc_norms_in_kernel(const lik_fwd_args& a, const TcExtra& x);
+int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float norm_d_eps, PrepJobs prep, void* ws, size_t ws_bytes,
+                  cudaStream_t st, const TcExtra& x);
 
 
 // Shared with the document-head kernel (lik_head.cu).

@@ -156,3 +156,37 @@ def test_document_head_deals_ragged_documents(Nd, Ld, lens):
     dm = cases.prefix_mask(n, Ld)
     got = maxsim_from_hidden(*(dev(x, torch.bfloat16) for x in (Q, H, W)), None, dev(dm), normalize=False)
     assert np.array_equal(f32(got), O.maxsim(Q, H[..., :32], None, dm))
+
+
+# one group of query tiles: norms taken inside the scoring kernel; several groups: by a pass in front.  The two sum a row in
+# the same order, so a query scores the same bits alone and in a large batch.
+@pytest.mark.parametrize("Lq,Nd,Ld,d,dtype,mask", [
+    (32, 1, 1, 128, torch.bfloat16, "none"),
+    (32, 301, 300, 128, torch.float16, "prefix"),
+    (8, 150, 257, 96, torch.bfloat16, "holes"),   # two tiles, the second of one row
+    (128, 40, 1030, 64, torch.float16, "holes"),  # many tiles per document, one K slab
+    (17, 299, 33, 40, torch.bfloat16, "prefix"),  # rows of 80 bytes
+    (31, 7, 2049, 16, torch.float16, "none"),
+])
+def test_norms_in_the_scoring_kernel(Lq, Nd, Ld, d, dtype, mask):
+    from late_interaction_kernels_b200.forward import maxsim_forward
+    import late_interaction_kernels_b200 as lik
+
+    rng = np.random.default_rng(Nd + d)
+    D = dev(rng.standard_normal((Nd, Ld, d)).astype(np.float32) * rng.uniform(0.01, 30, size=(Nd, Ld, 1)).astype(np.float32), dtype)
+    Q = dev(rng.standard_normal((300 // Lq + 2, Lq, d)).astype(np.float32), dtype)  # more rows than two query tiles hold
+    dm = {"none": None, "prefix": cases.prefix_mask(rng.integers(0, Ld + 1, size=Nd), Ld), "holes": rng.random((Nd, Ld)) < 0.6}[mask]
+    many, many_am = maxsim_forward(Q, D, None, dev(dm), save_argmax=True, normalize=True)
+    for q in (Q[:1], Q[1 : 1 + max(1, 256 // Lq)]):  # one tile; two full ones
+        lo = 0 if q.shape[0] == 1 else 1
+        s, am = maxsim_forward(q, D, None, dev(dm), save_argmax=True, normalize=True)
+        assert torch.equal(s, many[lo : lo + q.shape[0]])
+        assert torch.equal(am.view(q.shape[0], Nd, Lq), many_am.view(-1, Nd, Lq)[lo : lo + q.shape[0]])
+        assert torch.equal(lik.maxsim(q, D, d_mask=dev(dm), normalize=True), s)
+    # candidate lists: documents belong to one query each
+    K = min(Nd, 5)
+    n = min(Q.shape[0], Nd // K)
+    D4, m4 = D[: n * K].view(n, K, Ld, d), None if dm is None else dev(dm)[: n * K].view(n, K, Ld)
+    kd = lik.maxsim(Q[:n], D4, d_mask=m4, normalize=True)
+    assert torch.equal(kd, torch.stack([many[i, i * K : (i + 1) * K] for i in range(n)]))
+    lik.check_device_status()
