@@ -9,6 +9,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <type_traits>
 
 #include "lik_b200.h"
 
@@ -215,6 +216,18 @@ __device__ __forceinline__ unsigned warp_peers(int v, int nbits) {
 // Waits until the kernels in front of a programmatically serialised launch have finished and their writes are visible.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// 1 / max(sqrt(ss), eps), the root's reciprocal rounded once.  (A root and a division, each with its own iteration and its
+// own rounding, took a quarter of the time of a kernel that does little else.)
+__device__ __forceinline__ float inv_norm(float ss, float eps) { return fminf(__frsqrt_rn(ss), 1.0f / eps); }
+// s += x * x for both 16-bit halves of a word, the upper one first: products exact, sums in fp32, no conversions in between
+template <typename T>
+__device__ __forceinline__ void fma_sq_pair(uint32_t w, float& s) {
+  static_assert(std::is_same<T, __half>::value || std::is_same<T, __nv_bfloat16>::value, "a 16-bit float");
+  if (std::is_same<T, __half>::value)
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tfma.rn.f32.f16 %0, h, h, %0;\n\tfma.rn.f32.f16 %0, l, l, %0;\n\t}" : "+f"(s) : "r"(w));
+  else
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tfma.rn.f32.bf16 %0, h, h, %0;\n\tfma.rn.f32.bf16 %0, l, l, %0;\n\t}" : "+f"(s) : "r"(w));
+}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -53,7 +53,7 @@ __global__ void row_normalize_kernel(const T* __restrict__ x, long long n_rows, 
     ss = fmaf(w, w, ss);
   }
   ss = warp_sum(ss);
-  const float inv = 1.0f / fmaxf(sqrtf(ss), eps);
+  const float inv = inv_norm(ss, eps);
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
     const int k = c * 32 + lane;

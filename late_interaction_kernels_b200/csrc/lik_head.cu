@@ -418,7 +418,7 @@ head_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&ctl->acc1_empty[a]));
-        const float inv = P.normalize ? 1.0f / fmaxf(sqrtf(ss), 1e-12f) : 1.0f;
+        const float inv = P.normalize ? inv_norm(ss, 1e-12f) : 1.0f;
         ctl->col_scale[n1 & 1][row] = in_doc ? inv : 0.f;
         ctl->col_bias[n1 & 1][row] = valid ? 0.f : -INFINITY;
         fence_proxy_async();  // the operand stores above are read by the tensor core

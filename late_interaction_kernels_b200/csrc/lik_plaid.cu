@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(256) plaid_decompress_kernel(PlaidView v, long
     ss = fmaf(e[c], e[c], ss);
   }
   float inv = 1.f;
-  if (normalize) inv = 1.f / fmaxf(sqrtf(warp_sum(ss)), 1e-12f);
+  if (normalize) inv = inv_norm(warp_sum(ss), 1e-12f);
 #pragma unroll
   for (int c = 0; c < FMAX; ++c) {
     int f = c * 32 + lane;
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(256) plaid_bwd_dq_kernel(PlaidView v, int max_
       ss = fmaf(e[c], e[c], ss);
     }
     float f = g[(long long)i * n_docs + j];
-    if (normalize) f *= 1.f / fmaxf(sqrtf(warp_sum(ss)), 1e-12f);
+    if (normalize) f *= inv_norm(warp_sum(ss), 1e-12f);
 #pragma unroll
     for (int c = 0; c < FMAX; ++c) acc[c] = fmaf(f, e[c], acc[c]);
   }
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(256) plaid_bwd_dq_kernel(PlaidView v, int max_
       qv[c] = f < v.dim ? to_f32(qrow[f]) : 0.f;
       ss = fmaf(qv[c], qv[c], ss);
     }
-    const float inv = 1.f / fmaxf(sqrtf(warp_sum(ss)), 1e-6f);
+    const float inv = inv_norm(warp_sum(ss), 1e-6f);
     float dot = 0.f;
 #pragma unroll
     for (int c = 0; c < FMAX; ++c) {

@@ -104,7 +104,7 @@ __device__ __forceinline__ float plaid_inv_norm(const PlaidSrc& S, const float (
   for (int i = 0; i < 8; ++i) ss = fmaf(e[i], e[i], ss);
 #pragma unroll
   for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  return 1.f / fmaxf(sqrtf(ss), 1e-12f);
+  return inv_norm(ss, 1e-12f);
 }
 
 // A half-warp decodes the `n` consecutive tokens [tok0, tok0 + n) and hands the lane's eight finished values of
@@ -283,7 +283,7 @@ __device__ __forceinline__ void plaid_decode_run(const PlaidSrc& S, const float*
         float t = (h4 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, h4 ? a0 : a1, 4);
         t += __shfl_xor_sync(0xffffffffu, t, 2);
         t += __shfl_xor_sync(0xffffffffu, t, 1);
-        const float mine = 1.f / fmaxf(sqrtf(t), 1e-12f);  // of token 2 * (bit 3) + (bit 2)
+        const float mine = inv_norm(t, 1e-12f);  // of token 2 * (bit 3) + (bit 2)
 #pragma unroll
         for (int u = 0; u < U; ++u) inv[u] = __shfl_sync(0xffffffffu, mine, (lane & 16) | ((u >> 1) << 3) | ((u & 1) << 2));
       }

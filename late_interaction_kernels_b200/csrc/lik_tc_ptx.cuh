@@ -150,11 +150,6 @@ __device__ __forceinline__ int first_match32(const float (&v)[32], float cmax) {
   return (int)fminf(min3(b0, b1, b2), b3);
 }
 
-// s0 += a * a, s1 += b * b in one instruction
-__device__ __forceinline__ void fma_sq2(float a, float b, float& s0, float& s1) {
-  asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%0, %1};\n\tfma.rn.f32x2 q, p, p, q;\n\tmov.b64 {%0, %1}, q;\n\t}"
-      : "+f"(s0), "+f"(s1) : "f"(a), "f"(b));
-}
 // Fold the maximum of one 32-column chunk into the running (max, argmax) of a row.  The column scan
 // only runs when the chunk beats the running maximum (strict: an equal value in a later chunk never
 // displaces an earlier winner) and returns the lowest matching column.
