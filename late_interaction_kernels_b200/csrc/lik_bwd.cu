@@ -856,7 +856,8 @@ constexpr int DD_UNROLL = LIK_DD_UNROLL;  // independent list entries in flight 
 struct DdSortOut {
   int2* pairs;            // [n_scores * lq] (query row, weight bits), grouped by document then token
   long long* tok_begin;   // [d.n_rows] first list entry of every document row
-  int* tok_cnt;           // [d.n_rows] list length (cleared before the sort)
+  int* tok_cnt;           // [d.n_rows] list length
+  int clear_rest;         // the sort also clears the counts behind a document's end (else they were cleared before)
 };
 
 // A cluster of CTAs shares one document when the documents are fewer than the SMs: each takes a slice of the entries.
@@ -978,6 +979,8 @@ __global__ void __launch_bounds__(DDS_WARPS * 32) bwd_dd_sort_kernel(BwdParams P
   long long drow0;
   int dlen;
   seq_bounds(P.d, j, drow0, dlen, nullptr);
+  if (O.clear_rest && cl.rank == 0)
+    for (int t = (dlen > 0 && dlen < ld_pad ? dlen : 0) + tid; t < P.d.max_len; t += blockDim.x) O.tok_cnt[drow0 + t] = 0;
   if (dlen <= 0) return;
   if (dlen >= ld_pad) {  // max_len understated the longest document: report instead of overrunning shared memory
     if (tid == 0 && P.status) atomicOr(P.status, LIK_DEV_LEN_RANGE);
@@ -1152,6 +1155,8 @@ __global__ void __launch_bounds__(DDS_WARPS * 32) bwd_dd_sort4_kernel(BwdParams 
   long long drow0;
   int dlen;
   seq_bounds(P.d, j, drow0, dlen, nullptr);
+  if (O.clear_rest && cl.rank == 0)
+    for (int t = (dlen > 0 && dlen < ld_pad ? dlen : 0) + tid; t < P.d.max_len; t += blockDim.x) O.tok_cnt[drow0 + t] = 0;
   if (dlen <= 0) return;
   if (dlen >= ld_pad) {  // max_len understated the longest document: report instead of overrunning shared memory
     if (tid == 0 && P.status) atomicOr(P.status, LIK_DEV_LEN_RANGE);
@@ -1634,6 +1639,7 @@ struct BwdPlan {
   bool list_sorted;  // pair list on the deterministic kernels
   int sort_warps;    // warps of the winner sort that take entries (a histogram each): at least 256 entries of a document per warp
   int sort_cluster;  // CTAs per document
+  bool sort_clears;  // every row belongs to a document: the sort writes all the counts, nothing is cleared in front of it
   int sort_threads;  // threads of its CTAs: more warps than that when the documents are long (clearing and offsets go with the length)
   bool row16;  // 16-byte gathers: rows 16-byte aligned, width a multiple of 16 bytes, at most 1024 bytes
   bool fused;      // both gradients in one launch (bwd_fused16_kernel)
@@ -1753,6 +1759,7 @@ BwdPlan plan_bwd(const lik_bwd_args& a) {
     }
     if (pl.sort_smem <= 200 * 1024) {
       pl.sorted = true;
+      pl.sort_clears = !a.d.cu && a.d.seq_stride == a.d.max_len && a.d.n_rows == (int64_t)a.d.n_seq * a.d.seq_stride;
       const long long n_ent = n_scores_of(a.pairing, a.q.n_seq, a.d.n_seq, a.n_pairs) * (long long)a.argmax_stride;
       pl.pairs_off = take((size_t)n_ent * sizeof(int2));
       pl.begin_off = take((size_t)a.d.n_rows * sizeof(long long));
@@ -1910,6 +1917,7 @@ int run_bwd(const lik_bwd_args& a, BwdParams& P, const BwdPlan& pl, cudaStream_t
       O.pairs = (int2*)(ws + pl.pairs_off);
       O.tok_begin = (long long*)(ws + pl.begin_off);
       O.tok_cnt = (int*)(ws + pl.cnt_off);
+      O.clear_rest = pl.sort_clears;
       const bool quads = a.argmax_stride % 4 == 0 && ((uintptr_t)a.argmax % 16) == 0;
       auto kernel = quads ? bwd_dd_sort4_kernel : bwd_dd_sort_kernel;
       if (pl.sort_smem > 48 * 1024) LIK_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.sort_smem));
@@ -2036,7 +2044,7 @@ extern "C" int lik_maxsim_bwd(const lik_bwd_args* a, lik_stream_t stream) {
     prep.norm[1] = norm_job(a->d, a->dtype, a->dim, kBwdNormEps, w, false);
     dn = w;
   }
-  if (pl.sorted) prep.fill[0] = FillJob{(char*)a->workspace + pl.cnt_off, (size_t)a->d.n_rows * sizeof(int), 0};  // no winners yet
+  if (pl.sorted && !pl.sort_clears) prep.fill[0] = FillJob{(char*)a->workspace + pl.cnt_off, (size_t)a->d.n_rows * sizeof(int), 0};  // no winners yet
   {
     const int rc = launch_prep(prep, st);
     if (rc) return rc;
