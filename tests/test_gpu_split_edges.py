@@ -93,8 +93,9 @@ def test_backward_of_candidate_lists_and_packed_rows_without_owner(Nq, K, Lq, Ld
     assert torch.equal(tD.grad.cpu(), once_rounded(wd, torch.bfloat16))
 
 
-# fp32 tiles: 32 query tokens of one or two queries x 128 document tokens, slabs of 64 features
-@pytest.mark.parametrize("Nq,Lq,Nd,Ld,d", [(1, 1, 1, 1, 1), (2, 31, 3, 127, 63), (2, 32, 2, 128, 64), (3, 33, 5, 129, 65), (5, 7, 4, 257, 132)])
+# fp32 tiles: 32 query tokens of one query, or of two (from two blocks per SM on), x 128 document tokens, slabs of 64 features
+@pytest.mark.parametrize("Nq,Lq,Nd,Ld,d", [(1, 1, 1, 1, 1), (2, 31, 3, 127, 63), (2, 32, 2, 128, 64), (3, 33, 5, 129, 65), (5, 7, 4, 257, 132),
+                                              (34, 31, 19, 127, 64), (35, 33, 19, 129, 65)])
 def test_exact_fp32_tiles(Nq, Lq, Nd, Ld, d):
     from late_interaction_kernels_b200.forward import maxsim_forward
 
