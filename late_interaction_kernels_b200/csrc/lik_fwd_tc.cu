@@ -1535,13 +1535,13 @@ static cudaError_t allow_smem(size_t bytes) {
   return e;
 }
 
-// A launch that reads every document once or twice takes the documents' norms from its tiles: twelve queries of 32 tokens
-// against 8000 documents of 300 516 -> 433 us, 4 x 128 against 8000 of 1030 1970 -> 1420.  With more groups of
+// A launch that reads every document up to four times takes the documents' norms from its tiles: twelve queries of 32 tokens
+// against 8000 documents of 300 516 -> 433 us, 4 x 128 against 8000 of 1030 1970 -> 1520, four groups (8 x 128 against 4000 of 500) 732 -> 667.  With more groups of
 // query tiles the two warps would take every norm once per group; there one pass of prep_kernel in front takes them.
 bool fwd_tc_norms_in_kernel(const lik_fwd_args& a, const TcExtra& x) {
   if (!(a.normalize & LIK_NORM_D) || x.plaid || (a.dtype != LIK_BF16 && a.dtype != LIK_F16) || a.d.scale || a.d.scale_scalar != 1.0f) return false;
   const TcPlan pl = plan_tc(a, x);
-  return pl.stages >= 2 && (a.pairing == LIK_PAIR_GROUPED || (a.pairing == LIK_PAIR_CROSS && pl.n_groups <= 2));
+  return pl.stages >= 2 && (a.pairing == LIK_PAIR_GROUPED || (a.pairing == LIK_PAIR_CROSS && pl.n_groups <= 4));
 }
 
 int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float norm_d_eps, PrepJobs prep, void* ws, size_t ws_bytes,

@@ -159,7 +159,7 @@ def test_document_head_deals_ragged_documents(Nd, Ld, lens):
     assert np.array_equal(f32(got), O.maxsim(Q, H[..., :32], None, dm))
 
 
-# one or two groups of query tiles: norms taken inside the scoring kernel; more groups: by a pass in front.  The two sum a row in
+# up to four groups of query tiles: norms taken inside the scoring kernel; more groups: by a pass in front.  The two sum a row in
 # the same order, so a query scores the same bits alone and in a large batch.
 @pytest.mark.parametrize("Lq,Nd,Ld,d,dtype,mask", [
     (32, 1, 1, 128, torch.bfloat16, "none"),
@@ -175,10 +175,10 @@ def test_norms_in_the_scoring_kernel(Lq, Nd, Ld, d, dtype, mask):
 
     rng = np.random.default_rng(Nd + d)
     D = dev(rng.standard_normal((Nd, Ld, d)).astype(np.float32) * rng.uniform(0.01, 30, size=(Nd, Ld, 1)).astype(np.float32), dtype)
-    Q = dev(rng.standard_normal((520 // Lq + 2, Lq, d)).astype(np.float32), dtype)  # more rows than four query tiles hold
+    Q = dev(rng.standard_normal((1040 // Lq + 9, Lq, d)).astype(np.float32), dtype)  # more rows than eight query tiles hold
     dm = {"none": None, "prefix": cases.prefix_mask(rng.integers(0, Ld + 1, size=Nd), Ld), "holes": rng.random((Nd, Ld)) < 0.6}[mask]
     many, many_am = maxsim_forward(Q, D, None, dev(dm), save_argmax=True, normalize=True)
-    for lo, n in ((0, 1), (1, 128 // Lq * 2), (1, 128 // Lq * 3), (0, 128 // Lq * 4)):  # one tile, two, three (the last alone), four
+    for lo, n in ((0, 1), (1, 128 // Lq * 2), (1, 128 // Lq * 3), (0, 128 // Lq * 8)):  # one tile, two, three (the last alone), eight
         q = Q[lo : lo + n]
         s, am = maxsim_forward(q, D, None, dev(dm), save_argmax=True, normalize=True)
         assert torch.equal(s, many[lo : lo + q.shape[0]])
