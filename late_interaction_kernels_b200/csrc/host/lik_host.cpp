@@ -231,6 +231,7 @@ struct MaxSimBackward : public torch::autograd::Node {
 
   std::string name() const override { return "MaxSimBackward"; }
   void release_variables() override {
+    const std::lock_guard<std::mutex> lock(mutex_);
     for (SavedVariable* v : {&q, &d, &q_mask, &d_mask, &q_lens, &d_lens, &cu_q, &cu_d, &pair_q, &pair_d, &argmax}) v->reset_data();
   }
   torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
@@ -238,20 +239,28 @@ struct MaxSimBackward : public torch::autograd::Node {
     if (!grads[0].defined()) return out;
     const bool need_q = task_should_compute_output(0), need_d = task_should_compute_output(1);
     if (!need_q && !need_d) return out;
-    at::AutoDispatchBelowADInplaceOrView below;
-    const Tensor Q = q.unpack(), D = d.unpack();
+    Tensor Q, D, winners;
     Problem pr = scalars;
-    pr.q_mask = q_mask.unpack();
-    pr.d_mask = d_mask.unpack();
-    pr.q_lens = q_lens.unpack();
-    pr.d_lens = d_lens.unpack();
-    pr.cu_q = cu_q.unpack();
-    pr.cu_d = cu_d.unpack();
-    pr.pairing.pair_q = pair_q.unpack();
-    pr.pairing.pair_d = pair_d.unpack();
+    {
+      // Unpacking may run the caller's hooks (activation checkpointing computes the forward again in one), so it comes
+      // before the autograd keys are switched off.
+      const std::lock_guard<std::mutex> lock(mutex_);
+      Q = q.unpack();
+      D = d.unpack();
+      winners = argmax.unpack();
+      pr.q_mask = q_mask.unpack();
+      pr.d_mask = d_mask.unpack();
+      pr.q_lens = q_lens.unpack();
+      pr.d_lens = d_lens.unpack();
+      pr.cu_q = cu_q.unpack();
+      pr.cu_d = cu_d.unpack();
+      pr.pairing.pair_q = pair_q.unpack();
+      pr.pairing.pair_d = pair_d.unpack();
+    }
+    at::AutoDispatchBelowADInplaceOrView below;
     const auto dt = common_dtype(Q, D);
     auto [sq, sd] = sides(Q, D, pr, dt);
-    auto [gq, gd] = backward(sq, sd, pr.pairing, grads[0], argmax.unpack(), pr.normalize, pr.deterministic, dt, need_q, need_d);
+    auto [gq, gd] = backward(sq, sd, pr.pairing, grads[0], winners, pr.normalize, pr.deterministic, dt, need_q, need_d);
     if (need_q) out[0] = gq.view(Q.sizes()).to(Q.scalar_type());
     if (need_d) out[1] = gd.view(D.sizes()).to(D.scalar_type());
     return out;

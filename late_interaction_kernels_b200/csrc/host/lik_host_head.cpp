@@ -6,6 +6,8 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <mutex>
+
 namespace lik_host {
 
 namespace {
@@ -125,15 +127,25 @@ struct MaxSimFromHiddenBackward : public torch::autograd::Node {
 
   std::string name() const override { return "MaxSimFromHiddenBackward"; }
   void release_variables() override {
+    const std::lock_guard<std::mutex> lock(mutex_);
     for (SavedVariable* v : {&q, &h, &w, &b, &argmax}) v->reset_data();
   }
   torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
     torch::autograd::variable_list out(4);
     if (!grads[0].defined()) return out;
+    Tensor Q, H, W, B, winners;
+    {
+      // (before the autograd keys are switched off: unpacking may run the caller's hooks)
+      const std::lock_guard<std::mutex> lock(mutex_);
+      Q = q.unpack();
+      H = h.unpack();
+      W = w.unpack();
+      B = b.unpack();
+      winners = argmax.unpack();
+    }
     at::AutoDispatchBelowADInplaceOrView below;
-    std::tie(out[0], out[1], out[2], out[3]) =
-        head_backward(grads[0], q.unpack(), h.unpack(), w.unpack(), b.unpack(), argmax.unpack(), normalize, task_should_compute_output(0),
-                      task_should_compute_output(1), task_should_compute_output(2), task_should_compute_output(3));
+    std::tie(out[0], out[1], out[2], out[3]) = head_backward(grads[0], Q, H, W, B, winners, normalize, task_should_compute_output(0),
+                                                             task_should_compute_output(1), task_should_compute_output(2), task_should_compute_output(3));
     return out;
   }
 };

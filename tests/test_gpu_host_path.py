@@ -1,0 +1,75 @@
+"""The native host path under what a training program puts around a call: activation checkpointing and saved-tensor
+hooks."""
+
+import numpy as np
+import pytest
+import torch
+from torch.utils.checkpoint import checkpoint
+
+import cases
+
+pytestmark = pytest.mark.gpu
+
+
+def dev(x, dtype=None):
+    t = torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    return t.to(dtype) if dtype is not None else t
+
+
+def scoring_calls():
+    """name -> (function of its differentiable inputs, those inputs)"""
+    import late_interaction_kernels_b200 as lik
+    from late_interaction_kernels_b200.fused_head import maxsim_from_hidden
+    from late_interaction_kernels_b200.padded import maxsim_padded
+    from late_interaction_kernels_b200.score_pairs import score_pairs_packed
+
+    rng = np.random.default_rng(3)
+    half = torch.bfloat16
+    Q, D = dev(rng.standard_normal((4, 8, 64)), half), dev(rng.standard_normal((5, 24, 64)), half)
+    dm = dev(cases.prefix_mask(np.array([24, 3, 17, 1, 9]), 24))
+    cu_q, cu_d = dev(np.arange(0, 33, 8, dtype=np.int32)), dev(np.arange(0, 121, 24, dtype=np.int32))
+    pq, pd = dev(np.array([0, 0, 3], np.int32)), dev(np.array([4, 1, 2], np.int32))
+    W, b = dev(rng.standard_normal((64, 128)) / 12, half), dev(rng.standard_normal(64), half)
+    H = dev(rng.standard_normal((5, 24, 128)), half)
+    flat = lambda x: x.reshape(-1, x.shape[-1])
+    return {
+        "maxsim": (lambda q, d: lik.maxsim(q, d, d_mask=dm), (Q, D)),
+        "normalised": (lambda q, d: lik.maxsim(q, d, d_mask=dm, normalize=True), (Q, D)),
+        "varlen": (lambda q, d: lik.maxsim_varlen(q, d, cu_q, cu_d), (flat(Q), flat(D))),
+        "pairs": (lambda q, d: score_pairs_packed(q, d, cu_q, cu_d, pq, pd), (flat(Q), flat(D))),
+        "padded": (lambda q, d: maxsim_padded(q, d.unsqueeze(1), torch.full((5,), 8), torch.full((5, 1), 20)), (Q[[0, 1, 2, 3, 0]], D)),
+        "head": (lambda q, h, w, c: maxsim_from_hidden(q, h, w, c, dm), (Q, H, W, b)),
+        "head fp32": (lambda q, h, w, c: maxsim_from_hidden(q, h, w, c, dm), (Q.float(), H.float(), W.float(), b.float())),
+    }
+
+
+NAMES = ["maxsim", "normalised", "varlen", "pairs", "padded", "head", "head fp32"]
+
+
+def gradients(fn, inputs):
+    leaves = [x.detach().clone().requires_grad_() for x in inputs]
+    out = fn(*leaves)
+    (out * torch.arange(1, out.numel() + 1, device="cuda").view(out.shape)).sum().backward()
+    return [out.detach()] + [x.grad for x in leaves]
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_checkpointed_call_has_the_gradients_of_the_plain_one(name):
+    """Non-reentrant checkpointing computes the forward again inside the hook that unpacks a saved tensor."""
+    fn, inputs = scoring_calls()[name]
+    plain = gradients(fn, inputs)
+    again = gradients(lambda *x: checkpoint(fn, *x, use_reentrant=False), inputs)
+    # (work in front of the call: what the checkpoint saves then includes tensors of other operators)
+    chained = gradients(lambda *x: checkpoint(lambda *y: fn(*[t * 1 for t in y]), *x, use_reentrant=False), inputs)
+    for a, b, c in zip(plain, again, chained):
+        assert torch.equal(a, b) and torch.equal(a, c)
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_saved_tensors_may_travel(name):
+    fn, inputs = scoring_calls()[name]
+    plain = gradients(fn, inputs)
+    with torch.autograd.graph.save_on_cpu():
+        kept = gradients(fn, inputs)
+    for a, b in zip(plain, kept):
+        assert torch.equal(a, b)
