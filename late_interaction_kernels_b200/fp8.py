@@ -40,13 +40,13 @@ def dequantize_fp8_per_token(X_fp8: torch.Tensor, scale: torch.Tensor) -> torch.
     return X_fp8.to(torch.float32) * scale.unsqueeze(-1)
 
 
-def _scale_args(scale, token_shape, name):
-    """-> (per-token fp32 tensor | None, scalar multiplier tensor | None)."""
+def _scale_args(scale, token_shape, name, device):
+    """-> (per-token fp32 tensor on ``device`` | None, scalar multiplier tensor | None)."""
     if scale.dim() == 0:
         return None, scale.to(torch.float32)
     if tuple(scale.shape) != tuple(token_shape):
         raise ValueError(f"{name} must be a scalar or have shape {tuple(token_shape)}; got {tuple(scale.shape)}.")
-    return scale.to(torch.float32).contiguous(), None
+    return scale.to(device=device, dtype=torch.float32).contiguous(), None
 
 
 def maxsim_inference_fp8(Q, D, *, scale_Q, scale_D, q_mask=None, d_mask=None):
@@ -80,15 +80,15 @@ def maxsim_inference_fp8(Q, D, *, scale_Q, scale_D, q_mask=None, d_mask=None):
         K, Ld = D.shape[1], D.shape[2]
         D3 = D.contiguous().view(Nq * K, Ld, d)
         dm = d_mask.contiguous().view(Nq * K, Ld) if d_mask is not None else None
-        sd_tok, sd_sc = _scale_args(scale_D, (Nq, K, Ld), "scale_D")
+        sd_tok, sd_sc = _scale_args(scale_D, (Nq, K, Ld), "scale_D", Q.device)
         nd_eff = K
     else:
         D3, dm = D.contiguous(), d_mask
-        sd_tok, sd_sc = _scale_args(scale_D, D3.shape[:2], "scale_D")
+        sd_tok, sd_sc = _scale_args(scale_D, D3.shape[:2], "scale_D", Q.device)
         nd_eff = D3.shape[0]
-    sq_tok, sq_sc = _scale_args(scale_Q, (Nq, Lq), "scale_Q")
-    # per-tensor multipliers stay on the device: fold them into a per-token vector of the other
-    # side when there is one, otherwise into a one-element-per-token expansion of the query side.
+    sq_tok, sq_sc = _scale_args(scale_Q, (Nq, Lq), "scale_Q", Q.device)
+    # per-tensor multipliers stay where they are: fold them into a per-token vector of the other side when there is one,
+    # otherwise into a one-element-per-token expansion of the query side, on the queries' device.
     mult = None
     for s in (sq_sc, sd_sc):
         if s is not None:
@@ -99,7 +99,7 @@ def maxsim_inference_fp8(Q, D, *, scale_Q, scale_D, q_mask=None, d_mask=None):
         elif sd_tok is not None:
             sd_tok = sd_tok * mult
         else:
-            sq_tok = mult.expand(Nq, Lq).contiguous()
+            sq_tok = mult.expand(Nq, Lq).contiguous().to(Q.device)
     scores = _ops.native_call(_lib.host().maxsim_fp8, Q, D3, sq_tok, sd_tok, q_mask, dm, nd_eff if kd else 0)
     if kd:
         return scores

@@ -185,3 +185,29 @@ def test_reference_package_name_resolves_to_this_build():
     assert importlib.import_module("late_interaction_kernels.plaid").maxsim_residual is impl.plaid.maxsim_residual
     assert importlib.import_module("late_interaction_kernels.retrieve").retrieve is impl.retrieve
     from late_interaction_kernels.backward.lowmem import maxsim_backward_lowmem  # noqa: F401
+
+
+@pytest.mark.parametrize("per_token_q,per_token_d,kd", [(False, False, False), (True, False, False), (False, True, True), (True, True, True)])
+def test_fp8_scales_reach_the_kernel_on_the_inputs_device(monkeypatch, per_token_q, per_token_d, kd):
+    """Scales read from a checkpoint are host tensors; what the native call gets must sit where the embeddings are."""
+    from late_interaction_kernels_b200 import _lib, fp8
+
+    got = {}
+
+    class Host:
+        @staticmethod
+        def maxsim_fp8(Q, D, scale_Q, scale_D, q_mask, d_mask, group):
+            got.update(q=scale_Q, d=scale_D)
+            return torch.empty((Q.shape[0], group or D.shape[0]), device=Q.device)
+
+    monkeypatch.setattr(_lib, "host", lambda: Host)
+    monkeypatch.setattr(_lib, "require_cuda", lambda *a, **k: None)
+    e4m3 = torch.float8_e4m3fn
+    Q = torch.empty((2, 3, 16), dtype=e4m3, device="meta")  # stands in for a GPU: any device that is not the host
+    D = torch.empty((2, 5, 4, 16) if kd else (5, 4, 16), dtype=e4m3, device="meta")
+    sq = torch.ones((2, 3), dtype=torch.float64) if per_token_q else torch.tensor(0.5)
+    sd = torch.ones(D.shape[:-1], dtype=torch.float64) if per_token_d else torch.tensor(0.25)
+    fp8.maxsim_inference_fp8(Q, D, scale_Q=sq, scale_D=sd)
+    for t in got.values():
+        assert t is None or (t.device == Q.device and t.dtype == torch.float32)
+    assert any(t is not None for t in got.values())

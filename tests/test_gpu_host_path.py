@@ -1,5 +1,5 @@
-"""The native host path under what a training program puts around a call: activation checkpointing and saved-tensor
-hooks."""
+"""The native host path under what a program puts around a call: activation checkpointing, saved-tensor hooks, arguments
+on the host."""
 
 import numpy as np
 import pytest
@@ -73,3 +73,16 @@ def test_saved_tensors_may_travel(name):
         kept = gradients(fn, inputs)
     for a, b in zip(plain, kept):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("per_token_q,per_token_d", [(False, False), (True, False), (False, True), (True, True)])
+def test_fp8_scales_on_the_host(per_token_q, per_token_d):
+    from late_interaction_kernels_b200.fp8 import maxsim_inference_fp8
+
+    rng = np.random.default_rng(5)
+    e4m3 = torch.float8_e4m3fn
+    Q, D = dev(rng.standard_normal((3, 8, 64)), e4m3), dev(rng.standard_normal((6, 20, 64)), e4m3)
+    sq = torch.rand((3, 8)) if per_token_q else torch.tensor(0.5)
+    sd = torch.rand((6, 20)) if per_token_d else torch.tensor(0.02)
+    want = maxsim_inference_fp8(Q, D, scale_Q=sq.cuda(), scale_D=sd.cuda())
+    assert torch.equal(maxsim_inference_fp8(Q, D, scale_Q=sq, scale_D=sd), want)
