@@ -63,6 +63,12 @@ void check(int rc, const char* what) {
   if (rc != 0) throw std::runtime_error(std::string(what) + " failed (status " + std::to_string(rc) + "): " + lik_last_error());
 }
 
+void require_device(const at::Device& dev, std::initializer_list<std::pair<const char*, const Tensor*>> tensors) {
+  for (const auto& [name, t] : tensors)
+    if (t->defined() && t->device() != dev)
+      value_error(std::string(name) + " must be on the same device as the queries; got " + t->device().str() + " vs " + dev.str() + ".");
+}
+
 // One status word per device for the life of the process (never freed: the CUDA context may be gone before statics are).
 Tensor status_tensor(int64_t index) {
   static std::mutex mutex;
@@ -338,6 +344,7 @@ std::optional<Tensor> maxsim(const Tensor& Q, const Tensor& D, const OptTensor& 
 
 // candidate lists with length vectors: queries [B, Lq, d], documents [B, C, Ld, d], int32 lengths
 Tensor maxsim_padded(const Tensor& Q, const Tensor& D, const Tensor& q_lens, const Tensor& d_lens) {
+  require_device(Q.device(), {{"documents", &D}, {"query_lengths", &q_lens}, {"doc_lengths", &d_lens}});
   Problem pr;
   pr.q_lens = q_lens;
   pr.d_lens = d_lens;
@@ -346,7 +353,8 @@ Tensor maxsim_padded(const Tensor& Q, const Tensor& D, const Tensor& q_lens, con
   return scored(Q, D, pr, {D.size(0), D.size(1)});
 }
 
-Tensor as_int(const Tensor& t) { return t.to(at::kInt).contiguous(); }
+// offsets and pair indices as the kernels take them: int32 beside the embeddings
+Tensor as_int(const Tensor& t, const at::Device& dev) { return t.to(dev, at::kInt).contiguous(); }
 
 int64_t longest(const Tensor& cu) {  // one device-to-host copy
   return cu.numel() <= 1 ? 0 : (cu.slice(0, 1) - cu.slice(0, 0, -1)).max().item<int64_t>();
@@ -355,17 +363,19 @@ int64_t longest(const Tensor& cu) {  // one device-to-host copy
 // packed batches: every query against every document, or a pair list
 Tensor maxsim_packed(const Tensor& Q, const Tensor& D, const Tensor& cu_q, const Tensor& cu_d, const OptTensor& pair_q, const OptTensor& pair_d,
                      std::optional<int64_t> max_q, std::optional<int64_t> max_d) {
+  const auto dev = Q.device();
+  require_device(dev, {{"D_packed", &D}});
   Problem pr;
-  pr.cu_q = as_int(cu_q);
-  pr.cu_d = as_int(cu_d);
+  pr.cu_q = as_int(cu_q, dev);
+  pr.cu_d = as_int(cu_d, dev);
   const bool grad = at::GradMode::is_enabled() && (Q.requires_grad() || D.requires_grad());
   // the longest query sizes the query tiles (and the saved winners); the longest document is only needed by the backward
   pr.max_q = max_q ? *max_q : longest(pr.cu_q);
   pr.max_d = max_d ? *max_d : (grad ? longest(pr.cu_d) : 0);
   if (pair_q) {
     pr.pairing.kind = LIK_PAIR_LIST;
-    pr.pairing.pair_q = as_int(*pair_q);
-    pr.pairing.pair_d = as_int(*pair_d);
+    pr.pairing.pair_q = as_int(*pair_q, dev);
+    pr.pairing.pair_d = as_int(*pair_d, dev);
     return scored(Q, D, pr, {pr.pairing.pair_q.numel()});
   }
   return scored(Q, D, pr, {pr.cu_q.numel() - 1, pr.cu_d.numel() - 1});
@@ -374,12 +384,14 @@ Tensor maxsim_packed(const Tensor& Q, const Tensor& D, const Tensor& cu_q, const
 // e4m3 inputs: D [.., Ld, d] with one (kd) or no leading candidate dimension folded in; fp32 scales per token or absent
 Tensor maxsim_fp8(const Tensor& Q, const Tensor& D, const OptTensor& q_scale, const OptTensor& d_scale, const OptTensor& q_mask, const OptTensor& d_mask,
                   int64_t group) {
+  const Tensor qm = opt(q_mask), dm = opt(d_mask), qs = opt(q_scale), ds = opt(d_scale);
+  require_device(Q.device(), {{"D", &D}, {"scale_Q", &qs}, {"scale_D", &ds}, {"q_mask", &qm}, {"d_mask", &dm}});
   at::AutoDispatchBelowADInplaceOrView below;
   Pairing p;
   p.kind = group > 0 ? LIK_PAIR_GROUPED : LIK_PAIR_CROSS;
   p.group = group;
-  const Side q = padded_side(Q, Q.scalar_type(), opt(q_mask), Tensor(), opt(q_scale));
-  const Side d = padded_side(D, D.scalar_type(), opt(d_mask), Tensor(), opt(d_scale));
+  const Side q = padded_side(Q, Q.scalar_type(), qm, Tensor(), qs);
+  const Side d = padded_side(D, D.scalar_type(), dm, Tensor(), ds);
   const int64_t cols = group > 0 ? group : d.n_seq;
   return std::get<0>(forward(q, d, p, LIK_NORM_NONE, false, q.max_len, 0)).view({q.n_seq, cols});
 }

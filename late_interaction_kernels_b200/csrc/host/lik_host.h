@@ -6,9 +6,11 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
 
+#include <initializer_list>
 #include <optional>
 #include <string>
 #include <tuple>
+#include <utility>
 
 #include "lik_b200.h"
 
@@ -29,6 +31,8 @@ struct Side {
 int dtype_code(at::ScalarType t);  // lik_dtype; raises ValueError for a type without a kernel
 at::ScalarType common_dtype(const Tensor& a, const Tensor& b);
 void check(int rc, const char* what);
+// every tensor's address goes to a kernel on `dev`: raises ValueError for a (defined) one that is somewhere else
+void require_device(const at::Device& dev, std::initializer_list<std::pair<const char*, const Tensor*>> tensors);
 int32_t* status_ptr(const at::Device& dev);
 Tensor status_tensor(int64_t index);
 

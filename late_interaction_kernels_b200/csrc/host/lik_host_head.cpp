@@ -152,14 +152,15 @@ struct MaxSimFromHiddenBackward : public torch::autograd::Node {
 
 // maxsim_from_hidden on the chained kernel, autograd-aware; None when the kernel does not take the problem
 OptTensor maxsim_from_hidden(const Tensor& Q, const Tensor& H, const Tensor& W, const OptTensor& b_, const OptTensor& mask, bool normalize) {
-  const Tensor b = b_ ? *b_ : Tensor();
+  const Tensor b = b_ ? *b_ : Tensor(), dm = mask ? *mask : Tensor();
+  require_device(Q.device(), {{"H_d", &H}, {"W", &W}, {"b", &b}, {"d_mask", &dm}});
   const bool grad = at::GradMode::is_enabled() && (Q.requires_grad() || H.requires_grad() || W.requires_grad() || (b.defined() && b.requires_grad()));
   const auto dt = common_dtype(Q, H);
   if (!half_type(dt)) return std::nullopt;
   Tensor scores, argmax;
   {
     at::AutoDispatchBelowADInplaceOrView below;
-    auto got = head_forward(padded_side(Q, dt, Tensor(), Tensor(), Tensor()), padded_side(H, dt, mask ? *mask : Tensor(), Tensor(), Tensor()),
+    auto got = head_forward(padded_side(Q, dt, Tensor(), Tensor(), Tensor()), padded_side(H, dt, dm, Tensor(), Tensor()),
                             W.to(dt).contiguous(), b.defined() ? b.to(dt).contiguous() : b, normalize, grad);
     if (!got) return std::nullopt;
     std::tie(scores, argmax) = *got;

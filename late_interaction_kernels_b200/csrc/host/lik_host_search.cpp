@@ -13,12 +13,14 @@ using OptTensor = std::optional<Tensor>;
 // Q [Nq, Lq, d], D [Nd, Ld, d], masks [Nq, Lq] / [Nd, Ld].
 std::optional<std::tuple<Tensor, Tensor>> topk(const Tensor& Q, const Tensor& D, int64_t k, const OptTensor& q_mask, const OptTensor& d_mask,
                                                bool normalize, bool largest) {
-  at::AutoDispatchBelowADInplaceOrView below;
   const auto dev = Q.device();
+  const Tensor qm = q_mask ? *q_mask : Tensor(), dm = d_mask ? *d_mask : Tensor();
+  require_device(dev, {{"D", &D}, {"q_mask", &qm}, {"d_mask", &dm}});
+  at::AutoDispatchBelowADInplaceOrView below;
   const c10::cuda::CUDAGuard guard(dev);
   const auto dt = common_dtype(Q, D);
-  const Side q = padded_side(Q, dt, q_mask ? *q_mask : Tensor(), Tensor(), Tensor());
-  const Side d = padded_side(D, dt, d_mask ? *d_mask : Tensor(), Tensor(), Tensor());
+  const Side q = padded_side(Q, dt, qm, Tensor(), Tensor());
+  const Side d = padded_side(D, dt, dm, Tensor(), Tensor());
   lik_fwd_args a{};
   a.q = q.c_struct();
   a.d = d.c_struct();

@@ -211,3 +211,32 @@ def test_fp8_scales_reach_the_kernel_on_the_inputs_device(monkeypatch, per_token
     for t in got.values():
         assert t is None or (t.device == Q.device and t.dtype == torch.float32)
     assert any(t is not None for t in got.values())
+
+
+def test_native_entries_refuse_tensors_of_another_device(lib):
+    """Addresses go to a kernel as they are: a tensor that is not where the queries are is refused on the host, before
+    anything touches a GPU."""
+    from late_interaction_kernels_b200 import _lib
+
+    host = _lib.host()
+    here, there = torch.device("meta"), torch.device("cpu")  # two devices that a machine without a GPU has
+    e = lambda *shape, dev=here, dtype=torch.bfloat16: torch.zeros(shape, dtype=dtype, device=dev)
+    Q, D, qm, dm = e(2, 3, 16), e(4, 5, 16), e(2, 3, dtype=torch.bool), e(4, 5, dtype=torch.bool)
+    Qp, Dp, cu = e(6, 16), e(8, 16), torch.tensor([0, 3, 6], dtype=torch.int32)
+    ql, dl = e(2, dtype=torch.int32), e(4, dtype=torch.int32)
+    Q8, D8 = e(2, 3, 16, dtype=torch.float8_e4m3fn), e(4, 5, 16, dtype=torch.float8_e4m3fn)
+    sq, sd = e(2, 3, dtype=torch.float32), e(4, 5, dtype=torch.float32)
+    H, W, b = e(4, 5, 32), e(16, 32), e(16)
+    calls = [
+        (host.maxsim_padded, [Q, e(2, 2, 5, 16), ql, dl], [1, 2, 3]),
+        (host.maxsim_packed, [Qp, Dp, cu, cu, None, None, 3, 3], [1]),
+        (host.maxsim_fp8, [Q8, D8, sq, sd, qm, dm, 0], [1, 2, 3, 4, 5]),
+        (host.topk, [Q, D, 2, qm, dm, False, True], [1, 3, 4]),
+        (host.maxsim_from_hidden, [Q, H, W, b, dm, True], [1, 2, 3, 4]),
+    ]
+    for fn, args, movable in calls:
+        for i in movable:
+            bad = list(args)
+            bad[i] = torch.zeros(args[i].shape, dtype=args[i].dtype, device=there)
+            with pytest.raises(ValueError, match="same device"):
+                fn(*bad)
