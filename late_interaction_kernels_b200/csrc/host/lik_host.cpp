@@ -273,8 +273,13 @@ struct MaxSimBackward : public torch::autograd::Node {
   }
 };
 
-// Scores of a problem, reshaped to `shape`, attached to the graph when a gradient is wanted.
-Tensor scored(const Tensor& Q, const Tensor& D, const Problem& pr, at::IntArrayRef shape) {
+// Scores of a problem, reshaped to `shape`, attached to the graph when a gradient is wanted.  What the backward needs is
+// kept in the layout the kernels read: strided inputs and masks of wider types are copied once, outside the node, and the
+// caller may overwrite what they were copied from.
+Tensor scored(const Tensor& Q_, const Tensor& D_, Problem pr, at::IntArrayRef shape) {
+  const Tensor Q = Q_.contiguous(), D = D_.contiguous();
+  pr.q_mask = byte_mask(pr.q_mask);
+  pr.d_mask = byte_mask(pr.d_mask);
   const bool grad = at::GradMode::is_enabled() && (Q.requires_grad() || D.requires_grad());
   Tensor scores, argmax;
   {

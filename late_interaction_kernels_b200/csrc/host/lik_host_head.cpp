@@ -151,8 +151,9 @@ struct MaxSimFromHiddenBackward : public torch::autograd::Node {
 };
 
 // maxsim_from_hidden on the chained kernel, autograd-aware; None when the kernel does not take the problem
-OptTensor maxsim_from_hidden(const Tensor& Q, const Tensor& H, const Tensor& W, const OptTensor& b_, const OptTensor& mask, bool normalize) {
-  const Tensor b = b_ ? *b_ : Tensor(), dm = mask ? *mask : Tensor();
+OptTensor maxsim_from_hidden(const Tensor& Q_, const Tensor& H_, const Tensor& W_, const OptTensor& b_, const OptTensor& mask, bool normalize) {
+  // (strided inputs are copied once, outside the node: the backward reads the same copies)
+  const Tensor Q = Q_.contiguous(), H = H_.contiguous(), W = W_.contiguous(), b = b_ ? b_->contiguous() : Tensor(), dm = mask ? *mask : Tensor();
   require_device(Q.device(), {{"H_d", &H}, {"W", &W}, {"b", &b}, {"d_mask", &dm}});
   const bool grad = at::GradMode::is_enabled() && (Q.requires_grad() || H.requires_grad() || W.requires_grad() || (b.defined() && b.requires_grad()));
   const auto dt = common_dtype(Q, H);

@@ -86,3 +86,26 @@ def test_fp8_scales_on_the_host(per_token_q, per_token_d):
     sd = torch.rand((6, 20)) if per_token_d else torch.tensor(0.02)
     want = maxsim_inference_fp8(Q, D, scale_Q=sq.cuda(), scale_D=sd.cuda())
     assert torch.equal(maxsim_inference_fp8(Q, D, scale_Q=sq, scale_D=sd), want)
+
+
+def test_what_was_copied_for_the_kernel_may_be_overwritten():
+    """A mask of integers and strided embeddings are brought to the kernels' layout by a copy; a program that reuses their
+    memory before the backward (a mask buffer filled for the next batch) gets the gradients of the values it passed."""
+    import late_interaction_kernels_b200 as lik
+
+    rng = np.random.default_rng(9)
+    Q, D = dev(rng.standard_normal((3, 16, 8)), torch.bfloat16), dev(rng.standard_normal((20, 4, 16)), torch.bfloat16)  # [., d, Lq], [Ld, Nd, d]
+    qm, dm = dev(rng.integers(0, 2, (3, 8))), dev(rng.integers(0, 2, (4, 20)))
+
+    def step(touch):
+        bq, bd = Q.clone().requires_grad_(), D.clone().requires_grad_()
+        q, d, m, n = bq * 1, bd * 1, qm.clone(), dm.clone()
+        out = lik.maxsim(q.transpose(1, 2), d.transpose(0, 1), q_mask=m, d_mask=n)
+        if touch:
+            for t in (q, d, m, n):
+                t.detach().zero_() if t.is_floating_point() else t.zero_()
+        out.sum().backward()
+        return out.detach(), bq.grad, bd.grad
+
+    for a, b in zip(step(False), step(True)):
+        assert torch.equal(a, b)
