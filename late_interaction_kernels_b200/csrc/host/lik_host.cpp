@@ -69,6 +69,11 @@ void require_device(const at::Device& dev, std::initializer_list<std::pair<const
       value_error(std::string(name) + " must be on the same device as the queries; got " + t->device().str() + " vs " + dev.str() + ".");
 }
 
+void require_no_tangent(std::initializer_list<const Tensor*> tensors) {
+  for (const Tensor* t : tensors)
+    TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(0).defined(), "MaxSim scores have no forward-mode derivative.");
+}
+
 // One status word per device for the life of the process (never freed: the CUDA context may be gone before statics are).
 Tensor status_tensor(int64_t index) {
   static std::mutex mutex;
@@ -281,6 +286,7 @@ Tensor scored(const Tensor& Q_, const Tensor& D_, Problem pr, at::IntArrayRef sh
   pr.q_mask = byte_mask(pr.q_mask);
   pr.d_mask = byte_mask(pr.d_mask);
   const bool grad = at::GradMode::is_enabled() && (Q.requires_grad() || D.requires_grad());
+  if (grad) require_no_tangent({&Q, &D});
   Tensor scores, argmax;
   {
     at::AutoDispatchBelowADInplaceOrView below;

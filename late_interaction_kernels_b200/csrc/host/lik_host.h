@@ -33,6 +33,8 @@ at::ScalarType common_dtype(const Tensor& a, const Tensor& b);
 void check(int rc, const char* what);
 // every tensor's address goes to a kernel on `dev`: raises ValueError for a (defined) one that is somewhere else
 void require_device(const at::Device& dev, std::initializer_list<std::pair<const char*, const Tensor*>> tensors);
+// differentiable calls have no forward mode: raises NotImplementedError for an input that carries a tangent
+void require_no_tangent(std::initializer_list<const Tensor*> tensors);
 int32_t* status_ptr(const at::Device& dev);
 Tensor status_tensor(int64_t index);
 

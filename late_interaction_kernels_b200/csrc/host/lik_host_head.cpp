@@ -158,6 +158,7 @@ OptTensor maxsim_from_hidden(const Tensor& Q_, const Tensor& H_, const Tensor& W
   const bool grad = at::GradMode::is_enabled() && (Q.requires_grad() || H.requires_grad() || W.requires_grad() || (b.defined() && b.requires_grad()));
   const auto dt = common_dtype(Q, H);
   if (!half_type(dt)) return std::nullopt;
+  if (grad) require_no_tangent({&Q, &H, &W, &b});
   Tensor scores, argmax;
   {
     at::AutoDispatchBelowADInplaceOrView below;

@@ -109,3 +109,15 @@ def test_what_was_copied_for_the_kernel_may_be_overwritten():
 
     for a, b in zip(step(False), step(True)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_forward_mode_is_refused(name):
+    """There is no forward-mode rule; a tangent must not get lost on the way."""
+    fn, inputs = scoring_calls()[name]
+    with torch.autograd.forward_ad.dual_level():
+        for i in range(len(inputs)):
+            x = [t.clone() for t in inputs]
+            x[i] = torch.autograd.forward_ad.make_dual(x[i].requires_grad_(), torch.ones_like(x[i]))
+            with pytest.raises(NotImplementedError):
+                fn(*x)
