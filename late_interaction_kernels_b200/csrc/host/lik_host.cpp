@@ -381,8 +381,9 @@ Tensor maxsim_packed(const Tensor& Q, const Tensor& D, const Tensor& cu_q, const
   pr.cu_d = as_int(cu_d, dev);
   const bool grad = at::GradMode::is_enabled() && (Q.requires_grad() || D.requires_grad());
   // the longest query sizes the query tiles (and the saved winners); the longest document is only needed by the backward
-  pr.max_q = max_q ? *max_q : longest(pr.cu_q);
-  pr.max_d = max_d ? *max_d : (grad ? longest(pr.cu_d) : 0);
+  const bool none = pair_q && pair_q->numel() == 0;  // nothing to score, nothing to wait for
+  pr.max_q = max_q ? *max_q : (none ? 0 : longest(pr.cu_q));
+  pr.max_d = max_d ? *max_d : (grad && !none ? longest(pr.cu_d) : 0);
   if (pair_q) {
     pr.pairing.kind = LIK_PAIR_LIST;
     pr.pairing.pair_q = as_int(*pair_q, dev);

@@ -121,3 +121,20 @@ def test_forward_mode_is_refused(name):
             x[i] = torch.autograd.forward_ad.make_dual(x[i].requires_grad_(), torch.ones_like(x[i]))
             with pytest.raises(NotImplementedError):
                 fn(*x)
+
+
+def test_an_empty_pair_list_does_not_wait_for_the_gpu():
+    """A cascade stage without survivors: no offsets need to be read back (a captured graph could not)."""
+    from late_interaction_kernels_b200.score_pairs import score_pairs_packed
+
+    Q, D = torch.randn((6, 64), device="cuda", dtype=torch.bfloat16), torch.randn((9, 64), device="cuda", dtype=torch.bfloat16)
+    cu_q, cu_d, none = dev(np.array([0, 2, 6], np.int32)), dev(np.array([0, 9], np.int32)), torch.empty(0, dtype=torch.int32, device="cuda")
+    torch.cuda.set_sync_debug_mode("error")
+    try:
+        scores = score_pairs_packed(Q, D, cu_q, cu_d, none, none)
+        grad = score_pairs_packed(Q.requires_grad_(), D, cu_q, cu_d, none, none)
+    finally:
+        torch.cuda.set_sync_debug_mode("default")
+    assert scores.shape == grad.shape == (0,)
+    (gq,) = torch.autograd.grad(grad.sum(), Q)
+    assert not gq.any()
