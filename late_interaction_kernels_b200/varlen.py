@@ -31,12 +31,20 @@ def _check_packed(Q_packed, D_packed):
         )
 
 
+def _longest(cu):
+    return int((cu[1:] - cu[:-1]).max()) if cu.numel() > 1 else 0
+
+
 def _varlen_forward(Q_packed, D_packed, cu_seqlens_q, cu_seqlens_d, max_seqlen_q, max_seqlen_d, save_argmax):
     """Scores and winners outside autograd: ``(scores [Nq, Nd], argmax [Nq, Nd, max_q] | None, max_q, max_d)``
-    (varlen.py:271-364)."""
+    (varlen.py:271-364).  A longest length that is not given is read from the offsets, the documents' only for winners."""
     _check_packed(Q_packed, D_packed)
     _lib.require_cuda(Q_packed, D_packed, cu_seqlens_q, cu_seqlens_d, op="maxsim_varlen")
     dt = common_dtype(Q_packed, D_packed)
+    if max_seqlen_q is None:
+        max_seqlen_q = _longest(cu_seqlens_q)
+    if max_seqlen_d is None:
+        max_seqlen_d = _longest(cu_seqlens_d) if save_argmax else 0
     q = _ops.packed_spec(Q_packed.to(dt), cu_seqlens_q, max_seqlen_q)
     d = _ops.packed_spec(D_packed.to(dt), cu_seqlens_d, max_seqlen_d)
     scores, argmax = _ops.forward(q, d, pairing=_lib.PAIR_CROSS, save_argmax=save_argmax, argmax_stride=q.max_len)

@@ -240,3 +240,14 @@ def test_native_entries_refuse_tensors_of_another_device(lib):
             bad[i] = torch.zeros(args[i].shape, dtype=args[i].dtype, device=there)
             with pytest.raises(ValueError, match="same device"):
                 fn(*bad)
+
+
+@pytest.mark.parametrize("save_argmax", [False, True])
+def test_varlen_forward_finds_the_longest_lengths(monkeypatch, save_argmax):
+    from late_interaction_kernels_b200 import _lib, _ops, varlen
+
+    monkeypatch.setattr(_lib, "require_cuda", lambda *a, **k: None)
+    monkeypatch.setattr(_ops, "forward", lambda q, d, **k: (torch.zeros(q.n_seq * d.n_seq), None))
+    cu_q, cu_d = torch.tensor([0, 2, 6], dtype=torch.int32), torch.tensor([0, 1, 1, 9], dtype=torch.int32)
+    s, _, max_q, max_d = varlen._varlen_forward(torch.zeros(6, 8), torch.zeros(9, 8), cu_q, cu_d, None, None, save_argmax)
+    assert s.shape == (2, 3) and max_q == 4 and max_d == (8 if save_argmax else 0)
