@@ -884,9 +884,12 @@ __device__ __forceinline__ int load_cluster_int(const int* p, int rank) {  // th
   return v;
 }
 
-// Words of shared memory beside the histograms: per token its count in this CTA, in the cluster and in the CTAs before
-// this one, then the offsets and block totals of the scan.
-__host__ __device__ inline size_t dds_scratch_words(int ld_pad) { return (size_t)4 * ld_pad + 1 + (ld_pad + 31) / 32 + 1; }
+// Words of shared memory beside the histograms: the offsets and block totals of the scan and, where a cluster shares the
+// document, per token its count in this CTA, in the cluster and in the CTAs before this one.  (One CTA has no use for the
+// latter; with them a document's limit is 10 240 tokens instead of 25 000.)
+__host__ __device__ inline size_t dds_scratch_words(int ld_pad, int cluster) {
+  return (size_t)ld_pad + 1 + (ld_pad + 31) / 32 + 1 + (cluster > 1 ? (size_t)3 * ld_pad : 0);
+}
 
 // Offsets of the winner sort.  In: hist[w][t] = winners of token t counted by warp w (n_hist of the CTA's n_warps warps
 // count).  Out: the token's first list entry and count (global), and hist[w][t] = first write position of warp w for token
@@ -895,33 +898,38 @@ __host__ __device__ inline size_t dds_scratch_words(int ld_pad) { return (size_t
 // cluster call it with the same dlen.
 __device__ __forceinline__ void dds_offsets(int* hist, int* scratch, const SortCluster& cl, int n_warps, int n_hist, int ld_pad, int dlen,
                                             long long base, long long drow0, const DdSortOut& O, int warp, int lane) {
-  int* mine = scratch;               // [ld_pad] this CTA's winners of a token
-  int* all = mine + ld_pad;          // [ld_pad] the cluster's
-  int* before = all + ld_pad;        // [ld_pad] those of the CTAs before this one
-  int* tok_off = before + ld_pad;    // [ld_pad + 1]
-  int* blk = tok_off + ld_pad + 1;   // [ceil(ld_pad / 32) + 1]
-  for (int t = warp * 32 + lane; t < dlen; t += n_warps * 32) {
+  int* tok_off = scratch;                    // [ld_pad + 1]
+  int* blk = tok_off + ld_pad + 1;           // [ceil(ld_pad / 32) + 1]
+  int* mine = blk + (ld_pad + 31) / 32 + 1;  // clusters: [ld_pad] this CTA's winners of a token
+  int* all = mine + ld_pad;                  // [ld_pad] the cluster's
+  int* before = all + ld_pad;                // [ld_pad] those of the CTAs before this one
+  auto own = [&](int t) {
     int tot = 0;
     for (int w = 0; w < n_hist; ++w) tot += hist[w * ld_pad + t];
-    mine[t] = tot;
+    return tot;
+  };
+  const bool shared = cl.size > 1;
+  if (shared) {
+    for (int t = warp * 32 + lane; t < dlen; t += n_warps * 32) mine[t] = own(t);
+    sort_cluster_sync(cl);
   }
-  sort_cluster_sync(cl);
   const int n_blk = (dlen + 31) >> 5;
   for (int b = warp; b < n_blk; b += n_warps) {
     const int t = b * 32 + lane;
-    int tot = 0, bef = 0;
+    int tot = 0;
     if (t < dlen) {
-      if (cl.size == 1) {
-        tot = mine[t];
-      } else {
+      if (shared) {
+        int bef = 0;
         for (int r = 0; r < cl.size; ++r) {
           const int v = load_cluster_int(mine + t, r);
           tot += v;
           if (r < cl.rank) bef += v;
         }
+        all[t] = tot;
+        before[t] = bef;
+      } else {
+        tot = own(t);
       }
-      all[t] = tot;
-      before[t] = bef;
     }
     int incl = tot;
 #pragma unroll
@@ -953,7 +961,7 @@ __device__ __forceinline__ void dds_offsets(int* hist, int* scratch, const SortC
     const int t = b * 32 + lane;
     if (t < dlen) {
       const int excl = blk[b] + tok_off[t];
-      int pos = excl + before[t];
+      int pos = excl + (shared ? before[t] : 0);
       for (int w = 0; w < n_hist; ++w) {
         const int c = hist[w * ld_pad + t];
         hist[w * ld_pad + t] = pos;
@@ -961,7 +969,7 @@ __device__ __forceinline__ void dds_offsets(int* hist, int* scratch, const SortC
       }
       if (cl.rank == 0) {
         O.tok_begin[drow0 + t] = base + excl;
-        O.tok_cnt[drow0 + t] = all[t];
+        O.tok_cnt[drow0 + t] = shared ? all[t] : pos - excl;
       }
     }
   }
@@ -994,7 +1002,7 @@ __global__ void __launch_bounds__(DDS_WARPS * 32) bwd_dd_sort_kernel(BwdParams P
   const long long base = list ? ds.first * lq : (long long)j * n_ent;  // first entry of the document's slice of the list
   int* hist = dds_raw;                          // [n_hist][ld_pad]
   int* scratch = hist + n_hist * ld_pad;
-  float* gcol = reinterpret_cast<float*>(scratch + dds_scratch_words(ld_pad));  // [n_qr] (not for pair lists)
+  float* gcol = reinterpret_cast<float*>(scratch + dds_scratch_words(ld_pad, cl.size));  // [n_qr] (not for pair lists)
 
   for (int x = tid; x < n_hist * ld_pad; x += blockDim.x) hist[x] = 0;
   if (!list)
@@ -1172,7 +1180,7 @@ __global__ void __launch_bounds__(DDS_WARPS * 32) bwd_dd_sort4_kernel(BwdParams 
   const long long base = list ? ds.first * lq : (long long)j * n_ent;
   int* hist = dds_raw;                          // [n_hist][ld_pad]
   int* scratch = hist + n_hist * ld_pad;
-  float* gcol = reinterpret_cast<float*>(scratch + dds_scratch_words(ld_pad));  // [n_qr] (not for pair lists)
+  float* gcol = reinterpret_cast<float*>(scratch + dds_scratch_words(ld_pad, cl.size));  // [n_qr] (not for pair lists)
   int* q_first = reinterpret_cast<int*>(gcol + ds.n_qr);  // [n_qr] first row and length of every score's query (not for pair lists)
   int* q_len = q_first + ds.n_qr;
 
@@ -1686,7 +1694,7 @@ BwdPlan plan_bwd(const lik_bwd_args& a) {
   pl.list_sorted = list && a.deterministic && pl.fast && a.n_pairs > 0 && a.n_pairs < (1ll << 31) && a.d.max_len > 0 &&
                    a.q.max_len > 0 && a.q.n_seq > 0 && a.d.n_seq > 0;
   if (pl.list_sorted) {
-    const size_t ws_sort = ((size_t)(a.d.max_len + 1) + dds_scratch_words(a.d.max_len + 1)) * 4;  // with one warp per CTA
+    const size_t ws_sort = ((size_t)(a.d.max_len + 1) + a.d.max_len + 2) * 4;  // one CTA per document, one warp counts
     if (ws_sort > 200 * 1024) pl.list_sorted = false;
   }
   if (pl.list_sorted) {
@@ -1745,11 +1753,12 @@ BwdPlan plan_bwd(const lik_bwd_args& a) {
     // fewer documents than SMs: as many CTAs per document as leave each two thousand entries, so that the GPU fills up
     pl.sort_cluster = 1;
     while (pl.sort_cluster < 8 && (long long)a.d.n_seq * pl.sort_cluster * 2 <= 2 * sm_count() && ent >= 4096ll * pl.sort_cluster) pl.sort_cluster *= 2;
+    auto smem_for = [&](int w) {
+      return ((size_t)w * pl.ld_pad + dds_scratch_words(pl.ld_pad, pl.sort_cluster) + 3 * (size_t)n_qrange) * 4;
+    };
+    if (pl.sort_cluster > 1 && smem_for(1) > 200 * 1024) pl.sort_cluster = 1;  // a document too long for the cluster's counts
     long long nw = ceil_div(ceil_div(ent, pl.sort_cluster), 256);  // a warp per 256 entries: few, long documents still fill their CTAs
     pl.sort_warps = (int)(nw < 1 ? 1 : (nw > DDS_WARPS ? DDS_WARPS : nw));
-    auto smem_for = [&](int w) {
-      return ((size_t)w * pl.ld_pad + dds_scratch_words(pl.ld_pad) + 3 * (size_t)n_qrange) * 4;
-    };
     while (pl.sort_warps > 1 && smem_for(pl.sort_warps) > 200 * 1024) pl.sort_warps >>= 1;  // long documents: fewer histograms
     pl.sort_smem = smem_for(pl.sort_warps);
     {

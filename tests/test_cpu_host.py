@@ -251,3 +251,32 @@ def test_varlen_forward_finds_the_longest_lengths(monkeypatch, save_argmax):
     cu_q, cu_d = torch.tensor([0, 2, 6], dtype=torch.int32), torch.tensor([0, 1, 1, 9], dtype=torch.int32)
     s, _, max_q, max_d = varlen._varlen_forward(torch.zeros(6, 8), torch.zeros(9, 8), cu_q, cu_d, None, None, save_argmax)
     assert s.shape == (2, 3) and max_q == 4 and max_d == (8 if save_argmax else 0)
+
+
+@pytest.mark.parametrize("max_len", [300, 10_239, 10_241, 24_000])
+@pytest.mark.parametrize("pairing,n_q,n_d", [("cross", 4, 64), ("cross", 64, 8), ("cross", 600, 2), ("list", 8, 10)])
+def test_long_documents_keep_the_sorted_backward(lib, pairing, n_q, n_d, max_len):
+    """The winners of a document are sorted in shared memory up to about 25 000 tokens.  Beyond that a pair list scatters with
+    atomics, in no fixed order, into fp32 buffers of the gradients' size; the sort's lists grow with the winners alone."""
+    import ctypes as C
+
+    from late_interaction_kernels_b200 import _lib
+
+    def workspace(dim):
+        a = _lib.BwdArgs()
+        for side, n in ((a.q, n_q), (a.d, n_d)):
+            side.n_seq, side.row_stride = n, dim
+        a.q.max_len = a.q.seq_stride = 32
+        a.d.max_len = a.d.seq_stride = max_len
+        a.q.n_rows, a.d.n_rows = n_q * 32, n_d * max_len
+        a.dtype = a.grad_dtype = _lib.LIK_BF16
+        a.dim, a.argmax_stride, a.deterministic = dim, 32, 1
+        a.grad_d = 1 << 20  # (an address that is never read: the plan looks at its alignment)
+        a.pairing = _lib.PAIR_LIST if pairing == "list" else _lib.PAIR_CROSS
+        a.n_pairs = 30 if pairing == "list" else 0
+        return lib.lik_maxsim_bwd_workspace(C.byref(a))
+
+    entries = (30 if pairing == "list" else n_q * n_d) * 32
+    assert workspace(64) == workspace(128)
+    if n_q * 32 > 4096 or max_len > 1536 or pairing == "list":  # (smaller problems sort in the one-launch kernel)
+        assert workspace(64) >= entries * 8 + n_d * max_len * 12

@@ -191,3 +191,33 @@ def test_norms_in_the_scoring_kernel(Lq, Nd, Ld, d, dtype, mask):
     kd = lik.maxsim(Q[:n], D4, d_mask=m4, normalize=True)
     assert torch.equal(kd, torch.stack([many[i, i * K : (i + 1) * K] for i in range(n)]))
     lik.check_device_status()
+
+
+# documents behind 10 240 tokens, where a cluster's counts would no longer fit in shared memory: a CTA per document, and one
+# histogram from 12 800 tokens on
+@pytest.mark.parametrize("Nq,Lq,Nd,Ld", [(4, 32, 3, 10_240), (64, 130, 2, 10_241), (40, 128, 2, 25_000)])
+@pytest.mark.parametrize("as_list", [False, True])
+def test_backward_of_very_long_documents(Nq, Lq, Nd, Ld, as_list):
+    import late_interaction_kernels_b200 as lik
+    from late_interaction_kernels_b200.forward import maxsim_forward
+    from late_interaction_kernels_b200.score_pairs import score_pairs_packed
+
+    rng = np.random.default_rng(Ld)
+    Q, D, g = ints(rng, Nq, Lq, 64), ints(rng, Nd, Ld, 64), ints(rng, Nq, Nd)
+    tQ, tD = dev(Q, torch.bfloat16).requires_grad_(True), dev(D, torch.bfloat16).requires_grad_(True)
+    _, am = maxsim_forward(tQ.detach(), tD.detach(), save_argmax=True)
+    if as_list:
+        at = lambda n, step: dev(np.arange(0, (n + 1) * step, step, dtype=np.int32))
+        i, j = np.divmod(np.arange(Nq * Nd, dtype=np.int32), Nd)
+        s = score_pairs_packed(tQ.view(-1, 64), tD.view(-1, 64), at(Nq, Lq), at(Nd, Ld), dev(i), dev(j), max_seqlen_q=Lq, max_seqlen_d=Ld)
+        s.backward(dev(g).view(-1))
+    else:
+        lik.maxsim(tQ, tD).backward(dev(g))
+    win = am.view(Nq, Nd, Lq).cpu().numpy()
+    wq, wd = np.zeros_like(Q), np.zeros_like(D)
+    for i in range(Nq):
+        for j in range(Nd):
+            wq[i] += g[i, j] * D[j, win[i, j]]
+            np.add.at(wd[j], win[i, j], g[i, j] * Q[i])
+    assert torch.equal(tQ.grad.cpu(), once_rounded(wq, torch.bfloat16))
+    assert torch.equal(tD.grad.cpu(), once_rounded(wd, torch.bfloat16))
