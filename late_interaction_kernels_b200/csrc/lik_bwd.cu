@@ -1385,13 +1385,14 @@ __global__ void __launch_bounds__(256) bwd_dd_reduce16_walk_kernel(BwdParams P, 
 // shared memory and the same block reduces and stores the document's rows.  Such problems are bound by launches and by the
 // zero rows of grad_d, not by gathers: against sort and reduce kernels this saves two launches, the list's round trip
 // and a scheduling pass over 16-row blocks.  64 x 32 candidate lists of 300 tokens: 75 -> 45 us; a 16 x 16 batch 26 -> 12 us.
-// The order inside a token's list is (warp, round, lane): fixed by the data alone.
+// The order inside a token's list is the sort kernels': the gradients have the same bits whichever launch makes them.
 // ---------------------------------------------------------------------------------
 constexpr int FUSED_ENT = 4096;  // most winners of a document
 constexpr int FUSED_SMEM = 112 * 1024;  // two blocks per SM
 struct FusedShape {
   int dq_blocks, dq_per_query;  // grad_q blocks, and how many a query has
   int ld_pad, n_hist;
+  int rounds, quads;            // rows of 32 entries per warp; their order (see the kernel)
   int parts;                    // blocks per document: each sorts all of its winners and stores every parts-th run of rows
 };
 inline size_t fused_smem(int n_ent, int ld_pad, int n_hist) { return (size_t)n_ent * sizeof(int2) + ((size_t)n_hist + 3) * ld_pad * 4 + 64 * 4; }
@@ -1444,13 +1445,19 @@ __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape
   const bool prefill = n_ent * 2 < d_rows;
   if (fits) {
     for (int x = tid; x < F.n_hist * F.ld_pad; x += NT) hist[x] = 0;
-    // the winners of this thread: round k is entry k * NT + tid
+    // The winners of this thread, one of every row of its warp.  A row is 32 entries; bwd_dd_sort4_kernel reads four winners
+    // at a time and places first, second, third and fourth words of 32 such loads in turn, so there four rows share 128.
     constexpr int ROUNDS = FUSED_ENT / NT;
+    auto entry_of = [&](int k) {
+      const int r = warp * F.rounds + k;
+      return F.quads ? (r >> 2) * 128 + lane * 4 + (r & 3) : r * 32 + lane;
+    };
     int t_r[ROUNDS];
 #pragma unroll
     for (int k = 0; k < ROUNDS; ++k) {
-      const int e = k * NT + tid;
       t_r[k] = -1;
+      if (k >= F.rounds) continue;
+      const int e = entry_of(k);
       if (e < n_ent) {
         const int ii = e / lq, s = e - ii * lq;
         t_r[k] = __ldg(P.argmax + doc_slot(P, ds, j, ii) * lq + s);
@@ -1461,8 +1468,8 @@ __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < ROUNDS; ++k) {
-      if (k * NT >= n_ent) break;
-      const int e = k * NT + tid;
+      if (k >= F.rounds) break;
+      const int e = entry_of(k);
       int t = t_r[k];
       if (t >= dlen) t = -1;
       if (t >= 0) {
@@ -1512,11 +1519,11 @@ __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape
     const int t_bits = 32 - __clz(F.ld_pad);  // winners are below ld_pad
 #pragma unroll
     for (int k = 0; k < ROUNDS; ++k) {
-      if (k * NT >= n_ent) break;
+      if (k >= F.rounds) break;
       const int t = t_r[k];
       const unsigned peers = warp_peers(t, t_bits);
       if (t >= 0) {
-        const int e = k * NT + tid, ii = e / lq, s = e - ii * lq;
+        const int e = entry_of(k), ii = e / lq, s = e - ii * lq;
         const int i = ds.i_begin + ii;
         long long qrow0;
         int qlen;
@@ -1651,7 +1658,8 @@ struct BwdPlan {
   int sort_threads;  // threads of its CTAs: more warps than that when the documents are long (clearing and offsets go with the length)
   bool row16;  // 16-byte gathers: rows 16-byte aligned, width a multiple of 16 bytes, at most 1024 bytes
   bool fused;      // both gradients in one launch (bwd_fused16_kernel)
-  int fused_threads, fused_hist, fused_parts;
+  bool fused_quads;
+  int fused_threads, fused_rounds, fused_hist, fused_parts;
   size_t fused_bytes;
   int dq_split;    // grad_q: document ranges per query (1: one CTA walks all the documents of its query tokens)
   size_t dqp_off;  // their partial rows
@@ -1672,6 +1680,9 @@ bool bwd_row16_ok(const lik_bwd_args& a) {
   return bwd_fast_ok(a) && (a.dim * eb) % 16 == 0 && a.dim * eb <= 1024 && (a.q.row_stride * eb) % 16 == 0 &&
          (a.d.row_stride * eb) % 16 == 0 && ((uintptr_t)a.q.data % 16) == 0 && ((uintptr_t)a.d.data % 16) == 0;
 }
+
+// saved winners that are read (and sorted) four at a time
+bool winners_in_quads(const lik_bwd_args& a) { return a.argmax_stride % 4 == 0 && ((uintptr_t)a.argmax % 16) == 0; }
 
 BwdPlan plan_bwd(const lik_bwd_args& a) {
   BwdPlan pl{};
@@ -1729,7 +1740,10 @@ BwdPlan plan_bwd(const lik_bwd_args& a) {
         a.q.max_len > 0 && ent > 0 && ent <= FUSED_ENT && (ent <= 1024 || a.d.n_seq >= 96) && rows_owned) {
       pl.fused_threads = ent > 512 ? 512 : 256;
       const int warps = pl.fused_threads / 32;
-      pl.fused_hist = (int)(ceil_div(ent, 32) < warps ? ceil_div(ent, 32) : warps);
+      pl.fused_quads = winners_in_quads(a);
+      const long long rows = pl.fused_quads ? ceil_div(ent, 128) * 4 : ceil_div(ent, 32);
+      pl.fused_rounds = (int)ceil_div(rows, warps);
+      pl.fused_hist = (int)ceil_div(rows, pl.fused_rounds);
       pl.fused_bytes = fused_smem((int)ent, a.d.max_len + 1, pl.fused_hist);
       const size_t dq_bytes = (size_t)DQ_JC * (pl.fused_threads / 16) * sizeof(int2);
       if (pl.fused_bytes < dq_bytes) pl.fused_bytes = dq_bytes;
@@ -1900,6 +1914,8 @@ int run_bwd(const lik_bwd_args& a, BwdParams& P, const BwdPlan& pl, cudaStream_t
     F.n_hist = pl.fused_hist;
     F.dq_per_query = (int)ceil_div(a.q.max_len, pl.fused_threads / 16);
     F.dq_blocks = dq_fused ? a.q.n_seq * F.dq_per_query : 0;
+    F.rounds = pl.fused_rounds;
+    F.quads = pl.fused_quads;
     F.parts = pl.fused_parts;
     const unsigned grid = (unsigned)(F.dq_blocks + a.d.n_seq * F.parts);
     const size_t row_bytes = (size_t)a.dim * sizeof(T);
@@ -1927,8 +1943,7 @@ int run_bwd(const lik_bwd_args& a, BwdParams& P, const BwdPlan& pl, cudaStream_t
       O.tok_begin = (long long*)(ws + pl.begin_off);
       O.tok_cnt = (int*)(ws + pl.cnt_off);
       O.clear_rest = pl.sort_clears;
-      const bool quads = a.argmax_stride % 4 == 0 && ((uintptr_t)a.argmax % 16) == 0;
-      auto kernel = quads ? bwd_dd_sort4_kernel : bwd_dd_sort_kernel;
+      auto kernel = winners_in_quads(a) ? bwd_dd_sort4_kernel : bwd_dd_sort_kernel;
       if (pl.sort_smem > 48 * 1024) LIK_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.sort_smem));
       cudaLaunchAttribute attr{};
       attr.id = cudaLaunchAttributeClusterDimension;

@@ -221,3 +221,31 @@ def test_backward_of_very_long_documents(Nq, Lq, Nd, Ld, as_list):
             np.add.at(wd[j], win[i, j], g[i, j] * Q[i])
     assert torch.equal(tQ.grad.cpu(), once_rounded(wq, torch.bfloat16))
     assert torch.equal(tD.grad.cpu(), once_rounded(wd, torch.bfloat16))
+
+
+# the one-launch backward (documents without gaps) against the sort and reduction kernels (a row between the documents)
+@pytest.mark.parametrize("Nq,Lq,Nd,Ld,stride,grouped", [
+    (1, 32, 3, 40, 32, False),
+    (5, 7, 9, 33, 7, False),       # winners read one at a time
+    (16, 32, 16, 60, 32, False),   # 512 entries
+    (3, 171, 7, 33, 172, False),   # padded winner rows
+    (25, 41, 97, 17, 44, False),   # 1100 entries
+    (32, 128, 97, 40, 128, False),  # 4096
+    (6, 24, 24, 50, 24, True),     # candidate lists
+])
+def test_gradients_do_not_depend_on_the_route(Nq, Lq, Nd, Ld, stride, grouped):
+    from late_interaction_kernels_b200 import _lib, _ops
+
+    gen = torch.Generator(device="cuda").manual_seed(Nd * 64 + Ld)
+    rand = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+    Q, D, dmask = rand(Nq * Lq, 64).bfloat16(), rand(Nd, Ld + 1, 64).bfloat16(), torch.rand((Nd, Ld + 1), generator=gen, device="cuda") < 0.8
+    g = rand(Nd if grouped else Nq * Nd)
+    how = dict(pairing=_lib.PAIR_GROUPED if grouped else _lib.PAIR_CROSS, group=Nd // Nq if grouped else 0)
+    q = _ops.SeqSpec(Q, Nq, Lq, Lq)
+    apart = _ops.SeqSpec(D.view(-1, 64), Nd, Ld, Ld + 1, mask=dmask.view(torch.uint8).view(-1))
+    packed = _ops.SeqSpec(D[:, :Ld].reshape(-1, 64), Nd, Ld, Ld, mask=dmask[:, :Ld].contiguous().view(torch.uint8).view(-1))
+    _, am = _ops.forward(q, packed, save_argmax=True, argmax_stride=stride, **how)
+    for norm in (_lib.NORM_NONE, _lib.NORM_BOTH):
+        a, b = (_ops.backward(q, d, g, am, normalize=norm, **how) for d in (apart, packed))
+        assert torch.equal(a[0], b[0])
+        assert torch.equal(a[1].view(Nd, Ld + 1, 64)[:, :Ld], b[1].view(Nd, Ld, 64))
