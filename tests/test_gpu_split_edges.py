@@ -249,3 +249,26 @@ def test_gradients_do_not_depend_on_the_route(Nq, Lq, Nd, Ld, stride, grouped):
         a, b = (_ops.backward(q, d, g, am, normalize=norm, **how) for d in (apart, packed))
         assert torch.equal(a[0], b[0])
         assert torch.equal(a[1].view(Nd, Ld + 1, 64)[:, :Ld], b[1].view(Nd, Ld, 64))
+
+
+# the portable forward stages four elements at a time where rows allow it and one by one otherwise: the same scores
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16, torch.float8_e4m3fn])
+@pytest.mark.parametrize("d", [4, 60, 64, 68, 196])
+def test_staging_of_the_portable_forward(dtype, d):
+    from late_interaction_kernels_b200 import _ops
+
+    gen = torch.Generator(device="cuda").manual_seed(d)
+
+    def sides(shift):  # the same rows, `shift` elements behind a boundary and at a pitch that is a multiple of four or not
+        out = []
+        for i, (n, length) in enumerate([(3, 35), (4, 130)]):
+            rows = torch.randn((n * length, d), generator=gen.manual_seed(i), device="cuda").to(dtype)
+            buf = torch.zeros((n * length, d + 4 + shift), dtype=torch.float32, device="cuda").to(dtype)
+            buf[:, shift:shift + d] = rows
+            out.append(_ops.SeqSpec(buf[:, shift:shift + d], n, length, length))
+        return out
+
+    want = _ops.forward(*sides(1), engine=1, save_argmax=True)
+    for shift in (0, 4):
+        got = _ops.forward(*sides(shift), engine=1, save_argmax=True)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
