@@ -109,6 +109,7 @@ struct GenericFwdParams {
   int* argmax;
   int argmax_stride;
   int* status;
+  long long first;  // number of the launch's first block: a grid holds fewer than 2^31
 };
 
 __device__ __forceinline__ void cp_async16_zfill(float* dst, const float* src, bool on) {
@@ -213,13 +214,14 @@ __global__ void __launch_bounds__(128, 3) fwd_generic_kernel(GenericFwdParams P)
   long long slot[QB];
   int qi[QB], dj = 0;
   bool ok[QB];
+  const long long block = P.first + blockIdx.x;
   if (QB == 1) {
-    slot[0] = blockIdx.x;
+    slot[0] = block;
     ok[0] = decode_pair(P.pm, slot[0], qi[0], dj, tid == 0 ? P.status : nullptr);
   } else {
     const int n_qb = (P.pm.n_q + QB - 1) / QB;
-    dj = (int)(blockIdx.x / n_qb);
-    const int q0 = (int)(blockIdx.x - (long long)dj * n_qb) * QB;
+    dj = (int)(block / n_qb);
+    const int q0 = (int)(block - (long long)dj * n_qb) * QB;
 #pragma unroll
     for (int b = 0; b < QB; ++b) {
       qi[b] = q0 + b;
@@ -363,21 +365,21 @@ __global__ void __launch_bounds__(128, 3) fwd_generic_kernel(GenericFwdParams P)
 }
 
 template <typename T>
-static int launch_generic(const GenericFwdParams& P, cudaStream_t st) {
+static int launch_generic(GenericFwdParams P, cudaStream_t st) {
   // Two queries share a staged document where that still leaves every SM two blocks; fewer pairs spread better one by one
   // (8 x 32 documents of up to 300 tokens 57.6 -> 47.3 us, 4 x 100 of 512 96.7 -> 74.2; at 32 x 32 sharing is ahead, 64.1 to 67.3)
   const long long shared = (long long)((P.pm.n_q + 1) / 2) * P.pm.n_d;
   const bool cross = P.pm.pairing == LIK_PAIR_CROSS && P.pm.n_q > 1 && shared >= 2 * sm_count();
-  const long long grid = cross ? shared : P.pm.n_scores;
-  if (grid >= (1ll << 31)) {
-    set_error("too many (query, document) pairs for one launch");
-    return LIK_ERR_UNSUPPORTED;
-  }
+  const long long blocks = cross ? shared : P.pm.n_scores;
+  constexpr long long kMaxGrid = 1ll << 30;
   const size_t smem = (size_t)((cross ? 2 : 1) * G_QC + G_DC) * G_PITCH * sizeof(float);
 #define LIK_LAUNCH_GENERIC(QB)                                                                                            \
   do {                                                                                                                    \
     LIK_CUDA_OK(cudaFuncSetAttribute(fwd_generic_kernel<T, QB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    fwd_generic_kernel<T, QB><<<(unsigned)grid, 128, smem, st>>>(P), ::lik::count_launch();                          \
+    for (P.first = 0; P.first < blocks; P.first += kMaxGrid) {                                                            \
+      const long long n = blocks - P.first < kMaxGrid ? blocks - P.first : kMaxGrid;                                      \
+      fwd_generic_kernel<T, QB><<<(unsigned)n, 128, smem, st>>>(P), ::lik::count_launch();                                \
+    }                                                                                                                     \
   } while (0)
   if (cross) LIK_LAUNCH_GENERIC(2);
   else LIK_LAUNCH_GENERIC(1);
@@ -394,6 +396,7 @@ int launch_fwd_generic(const lik_fwd_args& a, const float* qn, const float* dn, 
                  n_scores_of(a.pairing, a.q.n_seq, a.d.n_seq, a.n_pairs)};
   P.dim = a.dim;
   const uintptr_t four = 4 * dtype_size(a.dtype) - 1;
+  P.first = 0;
   P.vec4 = a.dim % 4 == 0 && a.q.row_stride % 4 == 0 && a.d.row_stride % 4 == 0 && ((uintptr_t)a.q.data & four) == 0 && ((uintptr_t)a.d.data & four) == 0;
   P.scores = a.scores;
   P.argmax = a.argmax;

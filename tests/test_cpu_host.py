@@ -280,3 +280,19 @@ def test_long_documents_keep_the_sorted_backward(lib, pairing, n_q, n_d, max_len
     assert workspace(64) == workspace(128)
     if n_q * 32 > 4096 or max_len > 1536 or pairing == "list":  # (smaller problems sort in the one-launch kernel)
         assert workspace(64) >= entries * 8 + n_d * max_len * 12
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="looks at what happens before the first launch")
+def test_more_pairs_than_a_grid_has_blocks_are_not_refused(lib):
+    """The portable forward launches 2**30 blocks at a time.  (On the GPU 65 536 x 65 537 one-token pairs, 17 GB of scores
+    in three launches, take half a minute: too long for the suite.)  Without a GPU it is the launch that fails."""
+    import ctypes as C
+
+    from late_interaction_kernels_b200 import _lib
+
+    a = _lib.FwdArgs()
+    for side, n in ((a.q, 65536), (a.d, 65537)):
+        side.data, side.row_stride, side.n_rows, side.n_seq, side.max_len, side.seq_stride = 1 << 20, 4, n, n, 1, 1
+    a.dtype, a.dim, a.engine, a.scores = _lib.LIK_F32, 4, 1, 1 << 20
+    assert lib.lik_maxsim_fwd(C.byref(a), None) != 0
+    assert b"too many" not in lib.lik_last_error(), lib.lik_last_error()
