@@ -140,7 +140,7 @@ int run_fwd(const lik_fwd_args& a, const FwdPlan& pl, cudaStream_t st, const TcE
   }
   if (pl.lens_off != (size_t)-1) {
     int* eff = (int*)(ws + pl.lens_off);
-    prep.mask_lens = MaskLensJob{a.d.mask, a.d.lens, a.d.n_seq, a.d.max_len, a.d.seq_stride, eff, 0};
+    prep.mask_lens = MaskLensJob{a.d.mask, a.d.lens, a.d.n_seq, a.d.max_len, a.d.seq_stride, eff, 0, a.status};
     b.d.lens = eff;
   }
   rc = launch_prep(prep, st);

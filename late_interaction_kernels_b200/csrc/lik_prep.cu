@@ -171,7 +171,11 @@ __device__ __forceinline__ void mask_lens_block(const MaskLensJob& J, int block)
   const int j = block * (PREP_THREADS / 32) + (threadIdx.x >> 5);
   if (j >= J.n_seq) return;
   int len0 = J.max_len;
-  if (J.lens) len0 = min(max(J.lens[j], 0), J.max_len);
+  if (J.lens) {
+    const int l = J.lens[j];
+    len0 = min(max(l, 0), J.max_len);
+    if (l != len0 && lane == 0 && J.status) atomicOr(J.status, LIK_DEV_LEN_RANGE);
+  }
   const unsigned char* m = J.mask + (long long)j * J.seq_stride;
   int last = -1, cnt = 0;
   if (((uintptr_t)J.mask | (uintptr_t)J.seq_stride) % 4 == 0) {  // four tokens per load

@@ -24,6 +24,7 @@ struct MaskLensJob {  // out[j] = 1 + last valid token, tagged with `flag` when 
   long long seq_stride = 0;
   int* out = nullptr;
   int flag = 0;  // or-ed into out[j] when the mask has holes
+  int* status = nullptr;  // lengths outside [0, max_len] are reported here (they are clamped either way)
 };
 
 struct FillJob {  // whole 32-bit words, 16-byte aligned

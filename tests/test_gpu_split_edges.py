@@ -272,3 +272,19 @@ def test_staging_of_the_portable_forward(dtype, d):
     for shift in (0, 4):
         got = _ops.forward(*sides(shift), engine=1, save_argmax=True)
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("bad", [-1, 9])
+def test_portable_forward_reports_lengths_out_of_range_under_a_mask(bad):
+    """Masked documents are trimmed before the kernel sees their lengths; what is wrong with them is reported all the same."""
+    import late_interaction_kernels_b200 as lik
+    from late_interaction_kernels_b200 import _ops
+
+    q = _ops.SeqSpec(torch.ones((4, 8), device="cuda"), 2, 2, 2)
+    lens = torch.tensor([3, bad, 8], dtype=torch.int32, device="cuda")
+    d = _ops.SeqSpec(torch.ones((24, 8), device="cuda"), 3, 8, 8, lens=lens, mask=torch.ones(24, dtype=torch.uint8, device="cuda"))
+    lik.check_device_status()
+    scores, _ = _ops.forward(q, d)
+    with pytest.raises(RuntimeError):
+        lik.check_device_status()
+    assert scores.tolist() == [16.0, 16.0 if bad > 0 else 0.0, 16.0] * 2
