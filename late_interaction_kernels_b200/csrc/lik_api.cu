@@ -14,7 +14,8 @@ namespace {
 constexpr float kFwdNormEps = 1e-12f;
 
 struct FwdPlan {
-  size_t qn_off, dn_off, qcopy_off, dcopy_off, tc_off, lens_off, total;
+  size_t qn_off, dn_off, qcopy_off, dcopy_off, tc_off, lens_off;
+  size_t need, total;  // without and with the trimmed lengths of the portable kernel, which it can do without
   bool use_tc;
   bool copies;  // fused normalisation through normalised operand copies instead of per-row multipliers
 };
@@ -93,7 +94,9 @@ FwdPlan plan_fwd(const lik_fwd_args& a, const TcExtra& x = TcExtra()) {
     if (pl.copies) pl.dcopy_off = take((size_t)a.d.n_rows * a.dim * eb);
     else pl.dn_off = take((size_t)a.d.n_rows * 4);  // (also where the kernel takes the norms itself: a caller's buffer fits by size alone)
   }
-  // the portable kernel trims masked documents too
+  pl.need = off;
+  // the portable kernel trims masked documents too, where the workspace has room for the lengths: calls that never had to
+  // bring room for them (a fixed scratch array, a buffer sized long ago) read the padding instead
   if (!pl.use_tc && a.d.mask && !a.d.cu) pl.lens_off = take((size_t)a.d.n_seq * 4);
   pl.total = off;
   return pl;
@@ -138,7 +141,7 @@ int run_fwd(const lik_fwd_args& a, const FwdPlan& pl, cudaStream_t st, const TcE
     set_error("this problem is outside what the fused tensor-core path takes");
     return LIK_ERR_UNSUPPORTED;
   }
-  if (pl.lens_off != (size_t)-1) {
+  if (pl.lens_off != (size_t)-1 && ws && a.workspace_bytes >= pl.total) {
     int* eff = (int*)(ws + pl.lens_off);
     prep.mask_lens = MaskLensJob{a.d.mask, a.d.lens, a.d.n_seq, a.d.max_len, a.d.seq_stride, eff, 0, a.status};
     b.d.lens = eff;
@@ -166,7 +169,7 @@ int fwd_entry(const lik_fwd_args* a, lik_stream_t stream) {
     set_error("tcgen05 engine requested but this problem is outside what it takes");
     return LIK_ERR_UNSUPPORTED;
   }
-  if (pl.total > a->workspace_bytes || (pl.total && !a->workspace)) {
+  if (pl.need > a->workspace_bytes || (pl.need && !a->workspace)) {
     set_error("workspace too small: need %zu bytes, got %zu", pl.total, a->workspace_bytes);
     return LIK_ERR_WORKSPACE;
   }
@@ -312,7 +315,7 @@ extern "C" int lik_maxsim_fwd_static(const lik_fwd_args* a, lik_stream_t stream)
   LIK_REQUIRE(a != nullptr, "args is NULL");
   int rc = validate_fwd(*a);
   if (rc) return rc;
-  const size_t need = plan_fwd(*a).total;
+  const size_t need = plan_fwd(*a).need;
   if (need > (size_t)LIK_STATIC_SCRATCH_BYTES) {
     set_error("lik_maxsim_fwd_static: this problem needs %zu bytes of scratch, the built-in buffer holds %zu; "
               "use lik_maxsim_fwd with a caller workspace", need, (size_t)LIK_STATIC_SCRATCH_BYTES);

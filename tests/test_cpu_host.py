@@ -296,3 +296,22 @@ def test_more_pairs_than_a_grid_has_blocks_are_not_refused(lib):
     a.dtype, a.dim, a.engine, a.scores = _lib.LIK_F32, 4, 1, 1 << 20
     assert lib.lik_maxsim_fwd(C.byref(a), None) != 0
     assert b"too many" not in lib.lik_last_error(), lib.lik_last_error()
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="looks at what happens before the first launch")
+@pytest.mark.parametrize("entry", ["lik_maxsim_fwd", "lik_maxsim_fwd_static"])
+def test_trimmed_lengths_are_not_demanded_of_a_workspace(lib, entry):
+    """Five million masked one-token documents need no scratch at all; room for their trimmed lengths (20 MB) is asked for
+    but not insisted on.  Without a GPU it is the launch that fails."""
+    import ctypes as C
+
+    from late_interaction_kernels_b200 import _lib
+
+    a = _lib.FwdArgs()
+    for side, n in ((a.q, 1), (a.d, 5_000_000)):
+        side.data, side.row_stride, side.n_rows, side.n_seq, side.max_len, side.seq_stride = 1 << 20, 4, n, n, 1, 1
+    a.d.mask = 1 << 20
+    a.dtype, a.dim, a.engine, a.scores = _lib.LIK_F32, 4, 1, 1 << 20
+    assert lib.lik_maxsim_fwd_workspace(C.byref(a)) >= 20_000_000
+    assert getattr(lib, entry)(C.byref(a), None) != 0
+    assert b"workspace" not in lib.lik_last_error() and b"scratch" not in lib.lik_last_error(), lib.lik_last_error()

@@ -288,3 +288,22 @@ def test_portable_forward_reports_lengths_out_of_range_under_a_mask(bad):
     with pytest.raises(RuntimeError):
         lik.check_device_status()
     assert scores.tolist() == [16.0, 16.0 if bad > 0 else 0.0, 16.0] * 2
+
+
+def test_portable_forward_without_room_for_trimmed_lengths():
+    """The scores of masked documents whether their padding is trimmed or read."""
+    import ctypes as C
+
+    from late_interaction_kernels_b200 import _lib, _ops
+
+    rng = np.random.default_rng(0)
+    mask = dev(rng.integers(0, 2, (5, 40)).astype(np.uint8))
+    q = _ops.SeqSpec(dev(ints(rng, 21, 20)), 3, 7, 7)
+    d = _ops.SeqSpec(dev(ints(rng, 200, 20)), 5, 40, 40, mask=mask.view(-1))
+    want, _ = _ops.forward(q, d, engine=1)
+    got = torch.full((15,), -7.0, device="cuda")
+    a = _lib.FwdArgs(q=q.c_struct(), d=d.c_struct(), dtype=_lib.LIK_F32, dim=20, pairing=_lib.PAIR_CROSS, engine=1, scores=got.data_ptr(),
+                     status=_ops.status_word(got.device).data_ptr())
+    assert _lib.load().lik_maxsim_fwd_workspace(C.byref(a)) > 0
+    _lib.check(_lib.load().lik_maxsim_fwd(C.byref(a), _lib.stream_ptr(got.device)), "lik_maxsim_fwd")
+    assert torch.equal(got, want)
