@@ -1664,11 +1664,7 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
   }
   // positions of the saved argmax that no accumulator row covers (queries shorter than the stride)
   if (a.argmax && (a.q.cu || a.q.lens || a.argmax_stride > a.q.max_len))
-    if ((uintptr_t)a.argmax & 15)
-      LIK_CUDA_OK(cudaMemsetAsync(a.argmax, 0xFF,
-                                  (size_t)n_scores_of(a.pairing, a.q.n_seq, a.d.n_seq, a.n_pairs) * a.argmax_stride * sizeof(int), st));
-    else
-      prep.fill[1] = FillJob{a.argmax, (size_t)n_scores_of(a.pairing, a.q.n_seq, a.d.n_seq, a.n_pairs) * a.argmax_stride * sizeof(int), -1};
+    prep.fill[1] = FillJob{a.argmax, (size_t)n_scores_of(a.pairing, a.q.n_seq, a.d.n_seq, a.n_pairs) * a.argmax_stride * sizeof(int), -1};
   rc = launch_prep(prep, st);
   if (rc) return rc;
 

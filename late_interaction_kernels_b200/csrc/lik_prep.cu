@@ -208,6 +208,10 @@ __device__ __forceinline__ void fill_block(const FillJob& J, int block) {
   const size_t lo = (size_t)block * FILL_PER_BLOCK, hi = lo + FILL_PER_BLOCK < J.bytes ? lo + FILL_PER_BLOCK : J.bytes;
   const int4 v = make_int4(J.word, J.word, J.word, J.word);
   char* p = static_cast<char*>(J.ptr);
+  if ((uintptr_t)p & 15) {  // a caller's buffer may sit anywhere
+    for (size_t w = lo + (size_t)threadIdx.x * 4; w + 4 <= hi; w += PREP_THREADS * 4) *reinterpret_cast<int*>(p + w) = J.word;
+    return;
+  }
   size_t b = lo + (size_t)threadIdx.x * 16;
   for (; b + 16 <= hi; b += PREP_THREADS * 16) *reinterpret_cast<int4*>(p + b) = v;
   if (b < hi)  // the last whole words
@@ -269,10 +273,6 @@ int launch_prep(const PrepJobs& jobs, cudaStream_t st) {
     G.end[1 + i] = (int)n;
   }
   for (int i = 0; i < 2; ++i) {
-    if (jobs.fill[i].ptr && jobs.fill[i].bytes && ((uintptr_t)jobs.fill[i].ptr & 15)) {  // a caller's buffer may sit anywhere
-      set_error("fill target is not 16-byte aligned");
-      return LIK_ERR_INVALID;
-    }
     if (jobs.fill[i].ptr && jobs.fill[i].bytes) n += ceil_div((int64_t)jobs.fill[i].bytes, FILL_PER_BLOCK);
     G.end[3 + i] = (int)n;
   }

@@ -27,7 +27,7 @@ struct MaskLensJob {  // out[j] = 1 + last valid token, tagged with `flag` when 
   int* status = nullptr;  // lengths outside [0, max_len] are reported here (they are clamped either way)
 };
 
-struct FillJob {  // whole 32-bit words, 16-byte aligned
+struct FillJob {  // whole 32-bit words (sixteen bytes at a time where they lie on such a boundary)
   void* ptr = nullptr;  // nullptr: no job
   size_t bytes = 0;
   int word = 0;

@@ -307,3 +307,59 @@ def test_portable_forward_without_room_for_trimmed_lengths():
     assert _lib.load().lik_maxsim_fwd_workspace(C.byref(a)) > 0
     _lib.check(_lib.load().lik_maxsim_fwd(C.byref(a), _lib.stream_ptr(got.device)), "lik_maxsim_fwd")
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("shift", [0, 8, 16])
+def test_workspaces_and_winners_off_a_16_byte_boundary(shift):
+    """A caller's workspace of the C interface may start on any multiple of eight bytes, its array of winners anywhere:
+    fused top-k, a packed backward with clustered sorting, and winners of queries shorter than their rows."""
+    import ctypes as C
+
+    import late_interaction_kernels_b200 as lik
+    from late_interaction_kernels_b200 import _lib, _ops
+
+    lib, cuda = _lib.load(), torch.device("cuda")
+    rng = np.random.default_rng(1)
+    status, st = _ops.status_word(torch.device("cuda", 0)), _lib.stream_ptr(torch.device("cuda", 0))
+    room = lambda n: torch.empty(n + 64, dtype=torch.uint8, device=cuda)
+
+    # top-k
+    Q, D = dev(ints(rng, 3, 8, 64), torch.bfloat16), dev(ints(rng, 300, 9, 64), torch.bfloat16)
+    want = lik.retrieve(Q, D, 5, normalize=False)
+    q, d = _ops.padded_spec(Q), _ops.padded_spec(D)
+    s, i = torch.empty((3, 5), device=cuda), torch.empty((3, 5), dtype=torch.int64, device=cuda)
+    a = _lib.FwdArgs(q=q.c_struct(), d=d.c_struct(), dtype=_lib.LIK_BF16, dim=64, pairing=_lib.PAIR_CROSS, argmax_stride=8, status=status.data_ptr())
+    t = _lib.TopkSpec(k=5, largest=1, index_offset=0, out_scores=s.data_ptr(), out_index=i.data_ptr(), flags=0, doc_base=0)
+    n = lib.lik_maxsim_fwd_topk_workspace(C.byref(a), C.byref(t))
+    ws = room(n)
+    a.workspace, a.workspace_bytes = ws.data_ptr() + shift, n
+    _lib.check(lib.lik_maxsim_fwd_topk(C.byref(a), C.byref(t), st), "lik_maxsim_fwd_topk")
+    assert torch.equal(s, want[0]) and torch.equal(i, want[1])
+
+    # packed queries of 90 to 130 tokens, so that the winners' rows are partly behind their query, and their backward
+    ql, dl = rng.integers(90, 131, 60), rng.integers(20, 41, 5)
+    cu = lambda x: dev(np.concatenate([[0], np.cumsum(x)]).astype(np.int32))
+    Qp, Dp = dev(ints(rng, int(ql.sum()), 64), torch.bfloat16), dev(ints(rng, int(dl.sum()), 64), torch.bfloat16)
+    q, d = _ops.packed_spec(Qp, cu(ql), 130), _ops.packed_spec(Dp, cu(dl), 40)
+    want_s, want_am = _ops.forward(q, d, save_argmax=True, argmax_stride=132)
+    am = torch.zeros(300 * 132 + 16, dtype=torch.int32, device=cuda)[shift // 8:][:300 * 132].view(300, 132)
+    got_s = torch.empty(300, device=cuda)
+    a = _lib.FwdArgs(q=q.c_struct(), d=d.c_struct(), dtype=_lib.LIK_BF16, dim=64, pairing=_lib.PAIR_CROSS, scores=got_s.data_ptr(),
+                     argmax=am.data_ptr(), argmax_stride=132, status=status.data_ptr())
+    n = lib.lik_maxsim_fwd_workspace(C.byref(a))
+    ws = room(n)
+    a.workspace, a.workspace_bytes = ws.data_ptr(), n
+    _lib.check(lib.lik_maxsim_fwd(C.byref(a), st), "lik_maxsim_fwd")
+    assert torch.equal(got_s, want_s) and torch.equal(am, want_am)
+    g = dev(ints(rng, 300))
+    want_q, want_d = _ops.backward(q, d, g, want_am)
+    gq, gd = torch.empty_like(Qp), torch.empty_like(Dp)
+    b = _lib.BwdArgs(q=q.c_struct(), d=d.c_struct(), dtype=_lib.LIK_BF16, dim=64, pairing=_lib.PAIR_CROSS, deterministic=1, grad_scores=g.data_ptr(),
+                     argmax=am.data_ptr(), argmax_stride=132, grad_dtype=_lib.LIK_BF16, grad_q=gq.data_ptr(), grad_d=gd.data_ptr(),
+                     status=status.data_ptr())
+    n = lib.lik_maxsim_bwd_workspace(C.byref(b))
+    ws = room(n)
+    b.workspace, b.workspace_bytes = ws.data_ptr() + shift, n
+    _lib.check(lib.lik_maxsim_bwd(C.byref(b), st), "lik_maxsim_bwd")
+    assert torch.equal(gq, want_q) and torch.equal(gd, want_d)
+    lik.check_device_status()
