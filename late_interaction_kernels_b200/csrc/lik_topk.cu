@@ -306,8 +306,11 @@ __global__ void __launch_bounds__(SLOT_T) topk_slots_kernel(SlotParams P) {
 #pragma unroll
       for (int x = 0; x < PER_LIST; ++x) {
         const int t = x * 32 + lane;
-        if (t < c)
-          e[u * PER_LIST + x] = ((u64)slot_order(P.keys[list * SLOT_CAP + t]) << 32) | (unsigned)~(unsigned)P.idx[list * SLOT_CAP + t];
+        if (t < c) {
+          const float key = P.keys[list * SLOT_CAP + t];
+          if (key == key)  // (a score that is no number beats nothing)
+            e[u * PER_LIST + x] = ((u64)slot_order(key) << 32) | (unsigned)~(unsigned)P.idx[list * SLOT_CAP + t];
+        }
       }
     }
   }

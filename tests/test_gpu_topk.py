@@ -124,3 +124,25 @@ def test_maxsim_topk_with_k_above_1024():
     full = lik.maxsim(Q, D)
     ws, wi = _want(full, 2000)
     assert torch.equal(s, ws) and torch.equal(i, wi)
+
+
+@pytest.mark.parametrize("largest", [True, False])
+@pytest.mark.parametrize("k", [10, 30])
+def test_scores_that_are_no_numbers_are_not_retrieved(k, largest):
+    """An infinite query embedding has norm infinity: its products with half of the documents are inf * 0.  They take no
+    place among the k."""
+    import late_interaction_kernels_b200 as lik
+
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    Q = torch.randn((2, 8, 64), generator=gen, device="cuda", dtype=torch.bfloat16)
+    D = torch.randn((40, 12, 64), generator=gen, device="cuda", dtype=torch.bfloat16)
+    D[..., 0] = D[..., 0].abs() + 0.1
+    D[::2, :, 0] *= -1
+    Q[0, 3, 0] = float("inf")
+    s = lik.maxsim(Q, D, normalize=True)
+    assert s[0].isnan().sum() == 20 and not s[1].isnan().any()
+    worst = float("-inf") if largest else float("inf")
+    want = torch.where(s.isnan(), worst, s).topk(k, dim=1, largest=largest)
+    index = torch.where(want.values == worst, -1, want.indices)
+    got = lik.retrieve(Q, D, k, largest=largest)
+    assert torch.equal(got[0], want.values) and torch.equal(got[1], index)
