@@ -613,9 +613,11 @@ __device__ __forceinline__ void fma16_raw<__nv_bfloat16>(float (&acc)[8], float 
     asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[2 * i]), "=f"(acc[2 * i + 1]) : "l"(a));
   }
 }
+// (names its own half alone: the other may be in another row, in a branch without a sum, or done)
 __device__ __forceinline__ float half_warp_sum(float v) {
+  const unsigned half = 0xffffu << (threadIdx.x & 16);
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(half, v, o);
   return v;
 }
 // element offset of chunk c for lane hl of the half-warp
