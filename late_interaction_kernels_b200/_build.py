@@ -63,6 +63,20 @@ def _stale(target, inputs) -> bool:
     return any(os.path.getmtime(p) > t for p in inputs)
 
 
+def _host_abi() -> str:
+    """What a built host path is bound to besides its sources: torch's class layouts and the interpreter."""
+    import sysconfig
+    from importlib.metadata import version
+
+    return f"host path for torch {version('torch')}, {sysconfig.get_config_var('SOABI')}"
+
+
+def _host_fits(path) -> bool:
+    """Whether the extension at ``path`` was built for this torch and this interpreter (it carries their names)."""
+    with open(path, "rb") as f:
+        return _host_abi().encode() + b"\0" in f.read()
+
+
 def _run(cmd, what):
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
@@ -76,14 +90,15 @@ def _host_flags():
     from torch.utils import cpp_extension
 
     inc = [INCLUDE, HOST_SRC, sysconfig.get_paths()["include"], *cpp_extension.include_paths("cuda")]
-    flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_host", "-DTORCH_API_INCLUDE_EXTENSION_H"]
+    flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_host", "-DTORCH_API_INCLUDE_EXTENSION_H", f'-DLIK_HOST_ABI="{_host_abi()}"']
     return flags + [x for p in inc for x in ("-isystem" if p not in (INCLUDE, HOST_SRC) else "-I", p)]
 
 
 def build(force: bool = False, verbose: bool = False, extra_flags=()) -> str:
     """Compile what is stale and return the path of the kernel library."""
     want_lib = force or _stale(LIB_PATH, _sources() + _headers())
-    want_host = force or _stale(HOST_PATH, _host_sources() + _host_headers())
+    other_host = os.path.exists(HOST_PATH) and not _host_fits(HOST_PATH)  # torch or the interpreter was replaced
+    want_host = force or other_host or _stale(HOST_PATH, _host_sources() + _host_headers())
     if not (want_lib or want_host):
         return LIB_PATH
     os.makedirs(OBJ_DIR, exist_ok=True)
@@ -93,7 +108,7 @@ def build(force: bool = False, verbose: bool = False, extra_flags=()) -> str:
     def compile_one(src):
         host = src.endswith(".cpp")
         obj = os.path.join(OBJ_DIR, os.path.splitext(os.path.basename(src))[0] + ".o")
-        if not force and not _stale(obj, [src] + (_host_headers() if host else _headers())):
+        if not (force or (host and other_host)) and not _stale(obj, [src] + (_host_headers() if host else _headers())):
             return obj, ""
         cmd = ["g++", *host_flags, "-c", src, "-o", obj] if host else [nvcc, *NVCC_FLAGS, *extra_flags, "-c", src, "-o", obj]
         return obj, _run(cmd, f"compiling {src}")

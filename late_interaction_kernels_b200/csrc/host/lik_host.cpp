@@ -455,6 +455,7 @@ std::tuple<OptTensor, OptTensor> backward_py(const pybind11::tuple& q, const pyb
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   using namespace lik_host;
   m.doc() = "Native host path of the MaxSim operators (torch tensors in, launches of liblik_b200.so out).";
+  m.attr("abi") = LIK_HOST_ABI;  // looked for in the file when the build decides whether it is up to date
   m.def("maxsim", torch::wrap_pybind_function_no_gil(&maxsim));
   m.def("maxsim_padded", torch::wrap_pybind_function_no_gil(&maxsim_padded));
   m.def("maxsim_packed", torch::wrap_pybind_function_no_gil(&maxsim_packed));

@@ -315,3 +315,17 @@ def test_trimmed_lengths_are_not_demanded_of_a_workspace(lib, entry):
     assert lib.lik_maxsim_fwd_workspace(C.byref(a)) >= 20_000_000
     assert getattr(lib, entry)(C.byref(a), None) != 0
     assert b"workspace" not in lib.lik_last_error() and b"scratch" not in lib.lik_last_error(), lib.lik_last_error()
+
+
+def test_host_path_of_another_torch_is_stale(lib, monkeypatch):
+    """The native host path is bound to torch's class layouts: after an upgrade in place it is rebuilt, sources unchanged."""
+    from late_interaction_kernels_b200 import _build, _lib
+
+    assert _lib.host().abi == _build._host_abi() and _build._host_fits(_build.HOST_PATH)
+    monkeypatch.setattr(_build, "_host_abi", lambda: "host path for torch 99.0, cpython-99")
+    assert not _build._host_fits(_build.HOST_PATH)
+    ran = []
+    monkeypatch.setattr(_build, "_run", lambda cmd, what: ran.append(what) or "")
+    monkeypatch.setattr(_build.os, "replace", lambda a, b: None)
+    _build.build()
+    assert sorted(w.split()[0] for w in ran) == ["compiling"] * len(_build._host_sources()) + ["linking"]
