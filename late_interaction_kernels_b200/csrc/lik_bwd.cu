@@ -1384,7 +1384,9 @@ __global__ void __launch_bounds__(256) bwd_dd_reduce16_walk_kernel(BwdParams P, 
 // ---------------------------------------------------------------------------------
 // Both gradients in one launch, for problems whose documents have few winners each (small batches, candidate lists):
 // the first dq_blocks blocks are grad_q blocks, the others take a document each - the counting sort of its winners stays in
-// shared memory and the same block reduces and stores the document's rows.  Such problems are bound by launches and by the
+// shared memory and the same block reduces and stores the document's rows (a grad_q whose documents are split into ranges
+// brings its partial rows in the same launch: as a launch in front, 64 x 512 documents took 126 us, now 103).  Such problems are
+// bound by launches and by the
 // zero rows of grad_d, not by gathers: against sort and reduce kernels this saves two launches, the list's round trip
 // and a scheduling pass over 16-row blocks.  64 x 32 candidate lists of 300 tokens: 75 -> 45 us; a 16 x 16 batch 26 -> 12 us.
 // The order inside a token's list is the sort kernels': the gradients have the same bits whichever launch makes them.
@@ -1392,7 +1394,8 @@ __global__ void __launch_bounds__(256) bwd_dd_reduce16_walk_kernel(BwdParams P, 
 constexpr int FUSED_ENT = 4096;  // most winners of a document
 constexpr int FUSED_SMEM = 112 * 1024;  // two blocks per SM
 struct FusedShape {
-  int dq_blocks, dq_per_query;  // grad_q blocks, and how many a query has
+  int dq_blocks, dq_per_query;  // grad_q blocks of one document range, and how many a query has
+  int dq_split;                 // document ranges (0: no grad_q in this launch)
   int ld_pad, n_hist;
   int rounds, quads;            // rows of 32 entries per warp; their order (see the kernel)
   int parts;                    // blocks per document: each sorts all of its winners and stores every parts-th run of rows
@@ -1404,12 +1407,13 @@ __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape
   constexpr int TOK = NT / 16;
   extern __shared__ __align__(16) unsigned char fused_raw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, hl = tid & 15, hw = tid >> 4;
-  if ((int)blockIdx.x < F.dq_blocks) {
-    const int i = blockIdx.x / F.dq_per_query;
-    dq16_block<T, G, CH, TOK>(P, i, (blockIdx.x - i * F.dq_per_query) * TOK, 0, reinterpret_cast<int2(*)[TOK]>(fused_raw));
+  const int first_doc = F.dq_blocks * F.dq_split;
+  if ((int)blockIdx.x < first_doc) {
+    const int z = blockIdx.x / F.dq_blocks, b = blockIdx.x - z * F.dq_blocks, i = b / F.dq_per_query;
+    dq16_block<T, G, CH, TOK>(P, i, (b - i * F.dq_per_query) * TOK, z, reinterpret_cast<int2(*)[TOK]>(fused_raw));
     return;
   }
-  const int j = (blockIdx.x - F.dq_blocks) / F.parts, part = (blockIdx.x - F.dq_blocks) - j * F.parts;
+  const int j = (blockIdx.x - first_doc) / F.parts, part = (blockIdx.x - first_doc) - j * F.parts;
   long long drow0;
   int dlen;
   seq_bounds(P.d, j, drow0, dlen, nullptr);
@@ -1683,6 +1687,9 @@ bool bwd_row16_ok(const lik_bwd_args& a) {
          (a.d.row_stride * eb) % 16 == 0 && ((uintptr_t)a.q.data % 16) == 0 && ((uintptr_t)a.d.data % 16) == 0;
 }
 
+// winners of a problem from which grad_Q runs on a second stream beside the sort and reduce kernels of grad_D
+constexpr long long kForkEntries = 1ll << 20;
+
 // saved winners that are read (and sorted) four at a time
 bool winners_in_quads(const lik_bwd_args& a) { return a.argmax_stride % 4 == 0 && ((uintptr_t)a.argmax % 16) == 0; }
 
@@ -1733,13 +1740,22 @@ BwdPlan plan_bwd(const lik_bwd_args& a) {
       pl.dqp_off = take((size_t)z * a.q.n_rows * a.dim * 4);
     }
   }
-  // Few winners per document, and documents that one block can store: everything in one launch.  (With many winners per
-  // document and few documents the sort and reduce kernels spread a document over the GPU; long documents too.)
+  // Few winners per document, and documents whose histograms fit beside each other: everything in one launch, where the sort
+  // and reduce kernels do not run beside the grad_Q kernel on a second stream (kForkEntries).  Backward of bf16 rows of 128,
+  // sort route to one launch, queries of 32 tokens against documents of up to 300 unless stated: 8 x 32 34 -> 14 us, 32 x 96
+  // 46 -> 28, 128 x 128 84 -> 64, 16 x 1024 108 -> 89, 48 x 512 107 -> 91 (up to 1030 tokens 167 -> 140); a candidate list each for
+  // 32 queries, 1024 documents 56 -> 29.  From kForkEntries on the two streams win, 32 x 1024 110 to 132, 32 x 2000 205 to 235,
+  // 64 x 512 of 1030 137 to 161, except where a document's rows have many winners each and grad_Q is not split: 128 x 2000 670
+  // to 592, 96 x 1024 320 to 293, 128 x 2000 of 100 620 to 533; but 128 x 512 of 1030 211 to 246, hence eight per token.
+  // (The limits of 1536 tokens and, for more than 1024 winners, 96 documents are the tested range, not crossings: 64 x 95 would
+  // go from 52 to 39, 8 x 32 of 1800 tokens from 38 to 28.)
   {
     const long long ent = a.pairing == LIK_PAIR_CROSS ? (long long)a.q.n_seq * a.argmax_stride : (long long)a.argmax_stride;
     const bool rows_owned = a.d.cu || (a.d.seq_stride == a.d.max_len && a.d.n_rows == (int64_t)a.d.n_seq * a.d.seq_stride);
     if (!list && a.deterministic && pl.row16 && a.grad_d && a.d.n_seq > 0 && a.d.max_len > 0 && a.d.max_len <= 1536 && a.q.n_seq > 0 &&
-        a.q.max_len > 0 && ent > 0 && ent <= FUSED_ENT && (ent <= 1024 || a.d.n_seq >= 96) && rows_owned) {
+        a.q.max_len > 0 && ent > 0 && ent <= FUSED_ENT && (ent <= 1024 || a.d.n_seq >= 96) && rows_owned &&
+        (n_scores_of(a.pairing, a.q.n_seq, a.d.n_seq, a.n_pairs) * a.argmax_stride < kForkEntries ||
+         (pl.dq_split == 1 && ent >= 8ll * a.d.max_len))) {
       pl.fused_threads = ent > 512 ? 512 : 256;
       const int warps = pl.fused_threads / 32;
       pl.fused_quads = winners_in_quads(a);
@@ -1848,7 +1864,7 @@ int run_bwd(const lik_bwd_args& a, BwdParams& P, const BwdPlan& pl, cudaStream_t
   }
   // fork only when both gradients run the gather kernels and the problem is large enough to matter
   const bool want_fork = a.grad_q && a.grad_d && !list && a.deterministic && pl.fast && pl.sorted &&
-                         P.pm.n_scores * (long long)a.argmax_stride >= (1ll << 20);
+                         P.pm.n_scores * (long long)a.argmax_stride >= kForkEntries;
   std::unique_lock<std::mutex> fork_lock(g_fork_mutex, std::defer_lock);
   ForkJoin* fj = nullptr;
   if (want_fork) {
@@ -1880,7 +1896,7 @@ int run_bwd(const lik_bwd_args& a, BwdParams& P, const BwdPlan& pl, cudaStream_t
   } while (0)
 
   const bool fast = pl.fast;
-  const bool dq_fused = pl.fused && a.grad_q && pl.dq_split == 1;
+  const bool dq_fused = pl.fused && a.grad_q;
   if (a.grad_q && !dq_fused && !list && a.q.n_seq > 0 && a.q.max_len > 0) {
     dim3 grid((unsigned)a.q.n_seq, (unsigned)ceil_div(a.q.max_len, 8));
     if (pl.row16) {
@@ -1915,17 +1931,20 @@ int run_bwd(const lik_bwd_args& a, BwdParams& P, const BwdPlan& pl, cudaStream_t
     F.ld_pad = a.d.max_len + 1;
     F.n_hist = pl.fused_hist;
     F.dq_per_query = (int)ceil_div(a.q.max_len, pl.fused_threads / 16);
-    F.dq_blocks = dq_fused ? a.q.n_seq * F.dq_per_query : 0;
+    F.dq_blocks = a.q.n_seq * F.dq_per_query;
+    F.dq_split = dq_fused ? pl.dq_split : 0;
     F.rounds = pl.fused_rounds;
     F.quads = pl.fused_quads;
     F.parts = pl.fused_parts;
-    const unsigned grid = (unsigned)(F.dq_blocks + a.d.n_seq * F.parts);
+    const unsigned grid = (unsigned)(F.dq_blocks * F.dq_split + a.d.n_seq * F.parts);
+    const dim3 grid_sum((unsigned)a.q.n_seq, (unsigned)ceil_div(a.q.max_len, DQ16_TOK));
     const size_t row_bytes = (size_t)a.dim * sizeof(T);
 #define LIK_FUSED(CH_, NT_)                                                                                                          \
   do {                                                                                                                               \
     if (pl.fused_bytes > 48 * 1024)                                                                                                  \
       LIK_CUDA_OK(cudaFuncSetAttribute(bwd_fused16_kernel<T, G, CH_, NT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM)); \
     bwd_fused16_kernel<T, G, CH_, NT_><<<grid, NT_, pl.fused_bytes, st>>>(P, F), ::lik::count_launch();                              \
+    if (F.dq_split > 1) bwd_dq16_sum_kernel<T, G, CH_><<<grid_sum, 256, 0, st>>>(P), ::lik::count_launch();                          \
   } while (0)
 #define LIK_FUSED_NT(CH_)                               \
   do {                                                  \

@@ -48,6 +48,10 @@ def once_rounded(x, dtype):
     (241, 17, 97, 40, torch.bfloat16),    # 4097
     (64, 130, 3, 50, torch.bfloat16),     # cluster of four, rows of 130 winners
     (300, 128, 1, 2000, torch.float16),   # cluster of eight, one document, query rows split over blocks
+    (2, 5, 200, 17, torch.bfloat16),      # one launch with grad_q split over document ranges
+    (8, 128, 1023, 20, torch.bfloat16),   # ... the last of these before 2**20 winners
+    (8, 128, 1024, 20, torch.bfloat16),   # 2**20: two streams
+    (128, 32, 256, 20, torch.float16),    # 2**20, many winners per token, grad_q not split: one launch
 ])
 def test_backward_splits(Nq, Lq, Nd, Ld, dtype):
     import late_interaction_kernels_b200 as lik
