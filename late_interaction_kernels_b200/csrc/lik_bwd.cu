@@ -1391,13 +1391,15 @@ __global__ void __launch_bounds__(256) bwd_dd_reduce16_walk_kernel(BwdParams P, 
 // and a scheduling pass over 16-row blocks.  64 x 32 candidate lists of 300 tokens: 75 -> 45 us; a 16 x 16 batch 26 -> 12 us.
 // The order inside a token's list is the sort kernels': the gradients have the same bits whichever launch makes them.
 // ---------------------------------------------------------------------------------
-constexpr int FUSED_ENT = 4096;  // most winners of a document
+constexpr int FUSED_ENT = 4096;     // most winners of a document
+constexpr int FUSED_ENT_256 = 512;  // ... of one that a block of 256 threads takes
 constexpr int FUSED_SMEM = 112 * 1024;  // two blocks per SM
 struct FusedShape {
   int dq_blocks, dq_per_query;  // grad_q blocks of one document range, and how many a query has
   int dq_split;                 // document ranges (0: no grad_q in this launch)
   int ld_pad, n_hist;
-  int rounds, quads;            // rows of 32 entries per warp; their order (see the kernel)
+  int rounds, quads;            // rows of 32 entries per warp; their order (see the kernel):
+  int full_rows, tail;          // ... rows in whole groups of four, and the loads of the last, partial group (256 threads)
   int parts;                    // blocks per document: each sorts all of its winners and stores every parts-th run of rows
 };
 inline size_t fused_smem(int n_ent, int ld_pad, int n_hist) { return (size_t)n_ent * sizeof(int2) + ((size_t)n_hist + 3) * ld_pad * 4 + 64 * 4; }
@@ -1452,15 +1454,38 @@ __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape
   if (fits) {
     for (int x = tid; x < F.n_hist * F.ld_pad; x += NT) hist[x] = 0;
     // The winners of this thread, one of every row of its warp.  A row is 32 entries; bwd_dd_sort4_kernel reads four winners
-    // at a time and places first, second, third and fourth words of 32 such loads in turn, so there four rows share 128.
-    constexpr int ROUNDS = FUSED_ENT / NT;
+    // at a time and places first, second, third and fourth words of 32 such loads in turn, so there four rows share 128.  (In
+    // small documents the words of the last few loads follow one another without gaps; the division costs more than the empty
+    // places of a row where there are many.)
+    constexpr int ROUNDS = (NT == 256 ? FUSED_ENT_256 : FUSED_ENT) / NT;
     auto entry_of = [&](int k) {
       const int r = warp * F.rounds + k;
-      return F.quads ? (r >> 2) * 128 + lane * 4 + (r & 3) : r * 32 + lane;
+      if (!F.quads) return r * 32 + lane;
+      if (NT > 256 || r < F.full_rows) return (r >> 2) * 128 + lane * 4 + (r & 3);
+      const int p = (r - F.full_rows) * 32 + lane, loads = max(F.tail, 1), word = p / loads;
+      return word < 4 ? F.full_rows * 32 + (p - word * loads) * 4 + word : n_ent;
     };
     int t_r[ROUNDS];
+    // (where a thread has whole groups of four rows, the four words of a load are its own)
+    const bool by_four = ROUNDS >= 4 && F.quads && (F.rounds & 3) == 0;
+    if constexpr (ROUNDS >= 4) {
+#pragma unroll
+      for (int k = 0; k < ROUNDS; k += 4) {
+        int4 w = make_int4(-1, -1, -1, -1);
+        const int e = entry_of(k);
+        if (by_four && k < F.rounds && e < n_ent) {
+          const int ii = e / lq, s = e - ii * lq;
+          w = __ldg(reinterpret_cast<const int4*>(P.argmax + doc_slot(P, ds, j, ii) * lq + s));
+        }
+        t_r[k] = w.x;
+        t_r[k + 1] = w.y;
+        t_r[k + 2] = w.z;
+        t_r[k + 3] = w.w;
+      }
+    }
 #pragma unroll
     for (int k = 0; k < ROUNDS; ++k) {
+      if (by_four) continue;
       t_r[k] = -1;
       if (k >= F.rounds) continue;
       const int e = entry_of(k);
@@ -1756,10 +1781,10 @@ BwdPlan plan_bwd(const lik_bwd_args& a) {
         a.q.max_len > 0 && ent > 0 && ent <= FUSED_ENT && (ent <= 1024 || a.d.n_seq >= 96) && rows_owned &&
         (n_scores_of(a.pairing, a.q.n_seq, a.d.n_seq, a.n_pairs) * a.argmax_stride < kForkEntries ||
          (pl.dq_split == 1 && ent >= 8ll * a.d.max_len))) {
-      pl.fused_threads = ent > 512 ? 512 : 256;
+      pl.fused_threads = ent > FUSED_ENT_256 ? 512 : 256;
       const int warps = pl.fused_threads / 32;
       pl.fused_quads = winners_in_quads(a);
-      const long long rows = pl.fused_quads ? ceil_div(ent, 128) * 4 : ceil_div(ent, 32);
+      const long long rows = pl.fused_quads && pl.fused_threads > 256 ? ceil_div(ent, 128) * 4 : ceil_div(ent, 32);
       pl.fused_rounds = (int)ceil_div(rows, warps);
       pl.fused_hist = (int)ceil_div(rows, pl.fused_rounds);
       pl.fused_bytes = fused_smem((int)ent, a.d.max_len + 1, pl.fused_hist);
@@ -1935,6 +1960,11 @@ int run_bwd(const lik_bwd_args& a, BwdParams& P, const BwdPlan& pl, cudaStream_t
     F.dq_split = dq_fused ? pl.dq_split : 0;
     F.rounds = pl.fused_rounds;
     F.quads = pl.fused_quads;
+    {
+      const long long ent = a.pairing == LIK_PAIR_CROSS ? (long long)a.q.n_seq * a.argmax_stride : (long long)a.argmax_stride;
+      F.full_rows = (int)(ent / 128 * 4);
+      F.tail = (int)(ent % 128 / 4);
+    }
     F.parts = pl.fused_parts;
     const unsigned grid = (unsigned)(F.dq_blocks * F.dq_split + a.d.n_seq * F.parts);
     const dim3 grid_sum((unsigned)a.q.n_seq, (unsigned)ceil_div(a.q.max_len, DQ16_TOK));
