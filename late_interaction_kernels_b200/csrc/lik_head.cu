@@ -44,8 +44,17 @@ constexpr int HD_TOK = 128;          // document tokens per tile
 constexpr int HD_SLAB_ROW = 128;     // bytes of one K slab per row (one swizzle span)
 constexpr int HD_SLAB = HD_TOK * HD_SLAB_ROW;  // bytes of a 128-row slab
 constexpr int HD_THREADS = 448;
-// Up to this many ragged documents are dealt to the CTAs by length (see the kernel); more even out by themselves.
+// Most documents that are dealt to the CTAs by length (see the kernel): sixteen numbers per CTA are kept for them.
 constexpr int HD_DEAL_MAX = 1024;
+// Whether dealing pays.  Every CTA ranks all documents, n^2 steps over the launch (2 us for 150, 11 for 512, 43 for 1024),
+// and what is won grows with the work of a document's tokens behind its first tile.  Forward, lengths spread from a fifth of
+// the longest to the longest, contiguous ranges to dealt: 256 documents of up to 1024 tokens, d_model 768, 79 -> 63 us, 740 of
+// them 163 -> 159, 1024 of them 228 -> 226; 400 of up to 512 63 -> 63, 740 of them 97 -> 106; 200 of up to 256 30 -> 28, 300 of them
+// 34 -> 36; 512 of up to 128 32 -> 44, 1024 of them 48 -> 91.  d_model 384: 600 of up to 1024 116 -> 101, 880 of them 140 -> 151.
+// d_model 1536: 740 of up to 1024 306 -> 277; 400 of up to 256 65 -> 67.
+static bool deal_pays(long long n, long long ld, long long d_model) {
+  return n <= HD_DEAL_MAX && ld > HD_TOK && n * n * n <= (ld - HD_TOK) * (ld - HD_TOK) * d_model;
+}
 constexpr int HD_EPI_WARP0 = 6;  // warps 2..5 convert, warps 6.. score
 constexpr int HD_MAX_STAGES = 6;
 constexpr long long HD_WAIT_LIMIT = 4000000000ll;  // about 2 s at 2 GHz
@@ -713,7 +722,7 @@ extern "C" int lik_maxsim_hidden_fwd(const lik_hidden_fwd_args* args, lik_stream
     P.lens = eff;
     P.lens_flagged = 1;
   }
-  P.deal = P.lens && a.h.n_seq > pl.grid && a.h.n_seq <= HD_DEAL_MAX && ceil_div(a.h.n_seq, pl.grid) <= HD_DEAL_MAX / 64;
+  P.deal = P.lens && a.h.n_seq > pl.grid && deal_pays(a.h.n_seq, a.h.max_len, a.d_model) && ceil_div(a.h.n_seq, pl.grid) <= HD_DEAL_MAX / 64;
   P.d_model = a.d_model;
   P.d_out = a.d_out;
   P.n_k = pl.n_k;

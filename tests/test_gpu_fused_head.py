@@ -287,3 +287,17 @@ def test_hidden_winners_and_scatter_rows_against_numpy():
     for j in range(Nd):
         want[torch.from_numpy(rows[j, :counts[j]]).cuda()] = compact[j * S:j * S + counts[j]]
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("Nd,Ld", [(149, 200), (230, 256), (300, 256), (200, 128)])
+def test_dealt_documents_have_the_scores_of_single_calls(Nd, Ld):
+    """Few long ragged documents are dealt to the CTAs by length, others taken in order: a document's score is the same."""
+    from late_interaction_kernels_b200.fused_head import maxsim_from_hidden
+
+    gen = torch.Generator(device="cuda").manual_seed(Nd)
+    rand = lambda *shape: torch.randn(shape, generator=gen, device="cuda").bfloat16()
+    Q, H, W, b = rand(2, 8, 64), rand(Nd, Ld, 768), rand(64, 768), rand(64)
+    dm = torch.arange(Ld, device="cuda") < torch.randint(0, Ld + 1, (Nd, 1), generator=gen, device="cuda")
+    got = maxsim_from_hidden(Q, H, W, b, dm)
+    for j in range(0, Nd, 7):
+        assert torch.equal(got[:, j:j + 1], maxsim_from_hidden(Q, H[j:j + 1], W, b, dm[j:j + 1]))
