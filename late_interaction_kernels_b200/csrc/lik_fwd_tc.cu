@@ -129,7 +129,7 @@ struct TcParams {
 
 // Warps 18 and 19 take the rows' inverse norms from the tiles in shared memory when the launch asks for it: the documents
 // are then read once instead of twice, and no norms go through device memory.  Two queries of 128 tokens against 4000
-// documents of up to 1030: 444 -> 228 us (158 without normalisation; the two warps' arithmetic is what remains of the gap).
+// documents of up to 1030: 484 -> 232 us (146 without normalisation; the two warps' arithmetic is what remains of the gap).
 constexpr int NORM_WARPS = 2;
 constexpr int PLAID_WARPS = 3;  // warps 0, 18 and 19 decode compressed tokens in the PLAID kernels
 
@@ -1535,9 +1535,11 @@ static cudaError_t allow_smem(size_t bytes) {
   return e;
 }
 
-// A launch that reads every document up to four times takes the documents' norms from its tiles: twelve queries of 32 tokens
-// against 8000 documents of 300 516 -> 433 us, 4 x 128 against 8000 of 1030 1970 -> 1520, four groups (8 x 128 against 4000 of 500) 732 -> 667.  With more groups of
-// query tiles the two warps would take every norm once per group; there one pass of prep_kernel in front takes them.
+// A launch that reads every document up to four times takes the documents' norms from its tiles instead of one pass of
+// prep_kernel in front.  A query of 32 tokens against 1000 documents of up to 300 40 -> 30 us; two groups of query tiles (12 x 32
+// against 8000 of 300) 407 -> 308, (4 x 128 against 8000 of 1030) 1498 -> 953; 128-token queries against 4000 documents of up
+// to 500: three groups 458 -> 394, four 540 -> 484, five 646 -> 611, six 740 -> 724, eight 921 -> 930: the two warps take every
+// norm once per group.
 bool fwd_tc_norms_in_kernel(const lik_fwd_args& a, const TcExtra& x) {
   if (!(a.normalize & LIK_NORM_D) || x.plaid || (a.dtype != LIK_BF16 && a.dtype != LIK_F16) || a.d.scale || a.d.scale_scalar != 1.0f) return false;
   const TcPlan pl = plan_tc(a, x);

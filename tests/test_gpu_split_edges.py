@@ -33,7 +33,7 @@ def once_rounded(x, dtype):
 
 
 # entries of a document = queries x query tokens.  One launch for both gradients up to 4096 entries and 1536 document
-# tokens (from 1025 entries on only with 96 documents or more); sorted by a cluster of CTAs per document from 4096 entries
+# tokens (from 1025 entries on only with 96 documents or more; from 2**20 winners in all on only with many per token); sorted by a cluster of CTAs per document from 4096 entries
 # with few documents; one CTA per document otherwise.
 @pytest.mark.parametrize("Nq,Lq,Nd,Ld,dtype", [
     (1, 1, 1, 1, torch.bfloat16),         # one entry, one row
