@@ -126,50 +126,45 @@ __device__ __forceinline__ float max32(const float (&v)[32]) {
   return fmaxf(max3(b0, b1, b2), b3);
 }
 
-__device__ __forceinline__ float min3(float a, float b, float c) {
-  float d;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-// Position (0..31) of the first element of v that equals cmax, where cmax is the maximum of v.
-// Compare / select / logic instructions share one half-rate pipe, which a per-element equality scan
-// would saturate, so the scan is arithmetic instead: key_i = (cmax - v_i) * 2^154 + i is exactly i
-// for a match and at least 32 (or +inf) otherwise, because two different floats never differ by
-// less than 2^-149; the scaling is split in two exact powers of two that cannot overflow for
-// |cmax| < 2^64.  The minimum key is the answer.
-__device__ __forceinline__ int first_match32(const float (&v)[32], float cmax) {
-  const float c2 = cmax * 0x1p64f;
-  float k[32];
-#pragma unroll
-  for (int i = 0; i < 32; ++i) k[i] = fmaf(fmaf(v[i], -0x1p64f, c2), 0x1p90f, (float)i);
-  float a0 = min3(k[0], k[1], k[2]), a1 = min3(k[3], k[4], k[5]), a2 = min3(k[6], k[7], k[8]);
-  float a3 = min3(k[9], k[10], k[11]), a4 = min3(k[12], k[13], k[14]), a5 = min3(k[15], k[16], k[17]);
-  float a6 = min3(k[18], k[19], k[20]), a7 = min3(k[21], k[22], k[23]), a8 = min3(k[24], k[25], k[26]);
-  float a9 = min3(k[27], k[28], k[29]);
-  float b0 = min3(a0, a1, a2), b1 = min3(a3, a4, a5), b2 = min3(a6, a7, a8), b3 = min3(a9, k[30], k[31]);
-  return (int)fminf(min3(b0, b1, b2), b3);
-}
-
-// Fold the maximum of one 32-column chunk into the running (max, argmax) of a row.  The column scan
-// only runs when the chunk beats the running maximum (strict: an equal value in a later chunk never
-// displaces an earlier winner) and returns the lowest matching column.
-// LAZY: the scan is skipped when no row of the warp has a new maximum in this chunk - worth its branch only deep
+// Fold the maximum of one 32-column chunk into the running (max, argmax) of a row: an equal value in a later chunk never
+// displaces an earlier winner, and of equal values in a chunk the lowest column wins.
+// The column is found by descent: of two halves the lower one is taken when its maximum is the chunk's, and what was taken
+// is halved again.  The maxima of the groups of eight fall out of the maximum itself, so a chunk costs 55 instructions where
+// a key per column ((cmax - v) * 2^154 + column, reduced by minima) took 103: 100 cycles against 122 per chunk and warp with
+// four warps on a scheduler, and there is no arithmetic on the values, so infinities and the largest floats are like any other.
+// LAZY: the search is skipped when no row of the warp has a new maximum in this chunk - worth its branch only deep
 // into a long document, where most chunks bring none.
 template <bool ARGMAX, bool LAZY = false>
 __device__ __forceinline__ void fold32(const float (&v)[32], int col0, float& run_m, int& run_i) {
-  const float cmax = max32(v);
-  if (ARGMAX) {
-    // (unconditional by default: with 32 rows per warp some row nearly always has a new maximum in a document of a few
-    // chunks, and a branch costs more than the scan)
-    const bool better = cmax > run_m;
-    if (!LAZY || __any_sync(0xffffffffu, better)) {
-      const int p = first_match32(v, cmax);
-      run_i = better ? col0 + p : run_i;
-    }
-    run_m = better ? cmax : run_m;
-  } else {
-    run_m = fmaxf(run_m, cmax);
+  if (!ARGMAX) {
+    run_m = fmaxf(run_m, max32(v));
+    return;
   }
+  float g[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) g[j] = max3(max3(v[8 * j], v[8 * j + 1], v[8 * j + 2]), max3(v[8 * j + 3], v[8 * j + 4], v[8 * j + 5]), fmaxf(v[8 * j + 6], v[8 * j + 7]));
+  const float g01 = fmaxf(g[0], g[1]);
+  const float cmax = max3(g01, g[2], g[3]);
+  // (unconditional by default: with 32 rows per warp some row nearly always has a new maximum in a document of a few
+  // chunks, and a branch costs more than the search)
+  const bool better = cmax > run_m;
+  if (!LAZY || __any_sync(0xffffffffu, better)) {
+    float s[16], t[8], u[4];
+    const bool in16 = g01 == cmax;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) s[i] = in16 ? v[i] : v[16 + i];
+    const bool in8 = (in16 ? g[0] : g[2]) == cmax;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t[i] = in8 ? s[i] : s[8 + i];
+    const bool in4 = fmaxf(max3(t[0], t[1], t[2]), t[3]) == cmax;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) u[i] = in4 ? t[i] : t[4 + i];
+    const bool in2 = fmaxf(u[0], u[1]) == cmax;
+    const bool in1 = (in2 ? u[0] : u[2]) == cmax;
+    const int p = (in16 ? 0 : 16) + (in8 ? 0 : 8) + (in4 ? 0 : 4) + (in2 ? 0 : 2) + (in1 ? 0 : 1);
+    run_i = better ? col0 + p : run_i;
+  }
+  run_m = better ? cmax : run_m;
 }
 // v[i] *= scale[i]: per-column multiplier staged in shared memory
 __device__ __forceinline__ void scale32(float (&v)[32], const float* scale) {
@@ -202,37 +197,6 @@ __device__ __forceinline__ void affine32(float (&v)[32], const float* scale, con
     v[i + 2] = fmaf(v[i + 2], sc.z, bi.z);
     v[i + 3] = fmaf(v[i + 3], sc.w, bi.w);
   }
-}
-
-// Partial chunk of `lim` (1..31) columns: loaded as pieces of 16, 8, 4, 2 and 1 columns according to
-// the bits of lim into v[0..15], v[16..23], v[24..27], v[28..29], v[30]; pieces that are absent keep
-// the value the caller put there.  Piece n starts at column (lim with the bits below 2n cleared).
-__device__ __forceinline__ void tmem_ld_tail(uint32_t taddr, int lim, float (&v)[32]) {
-  if (lim & 16) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]), "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15]) : "r"(taddr + (uint32_t)(lim & 0)) : "memory");
-  }
-  if (lim & 8) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];" : "+f"(v[16]), "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]), "+f"(v[22]), "+f"(v[23]) : "r"(taddr + (uint32_t)(lim & 16)) : "memory");
-  }
-  if (lim & 4) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]) : "r"(taddr + (uint32_t)(lim & 24)) : "memory");
-  }
-  if (lim & 2) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "+f"(v[28]), "+f"(v[29]) : "r"(taddr + (uint32_t)(lim & 28)) : "memory");
-  }
-  if (lim & 1) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "+f"(v[30]) : "r"(taddr + (uint32_t)(lim & 30)) : "memory");
-  }
-  asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]), "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15]), "+f"(v[16]), "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]), "+f"(v[22]), "+f"(v[23]), "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]), "+f"(v[29]), "+f"(v[30]) : : "memory");
-}
-// Column (relative to the chunk) of the first element of a tmem_ld_tail() array that equals cmax.
-__device__ __forceinline__ int tail_first_match(const float (&v)[32], float cmax, int lim) {
-  const int p = first_match32(v, cmax);  // array position; pieces are stored in ascending column order
-  if (p < 16) return p;
-  if (p < 24) return (lim & 16) + (p - 16);
-  if (p < 28) return (lim & 24) + (p - 24);
-  if (p < 30) return (lim & 28) + (p - 28);
-  return lim & 30;
 }
 
 // Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row groups 1024 bytes apart.

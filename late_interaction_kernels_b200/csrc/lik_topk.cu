@@ -161,11 +161,10 @@ __global__ void __launch_bounds__(NT, MIN_CTAS) topk_kernel(TopkParams P) {
 }
 
 // Merge of the candidate lists the fused scoring kernel leaves (lik_fwd_tc.cu): list slot of (CTA c, tile
-// group g) is c + g, each slot holds 2 * qpt lists of up to 256 entries (unsorted), and CTA c of n_ctas can
+// group g) is c + g, each slot holds 4 * qpt lists of up to 256 entries (unsorted), and CTA c of n_ctas can
 // only have worked on the groups [n_groups * c / n_ctas, n_groups * (c + 1) / n_ctas] (a superset of the ones
-// it really met; lists it never touched are empty).  A group is `mt` query tiles of `qpt` queries; with two
-// tiles a query has one list per slot (tile * qpt + position), with one tile it has two (the kernel's two
-// epilogue groups take alternate documents).
+// it really met; lists it never touched are empty).  A group is `mt` query tiles of `qpt` queries.  The kernel has
+// 4 / mt documents in flight per CTA, each with lists of its own: a query has that many per slot.
 //
 // An entry becomes one 64-bit number, larger = better: the score's ordered key above the complement of the document
 // index, so that ties need no second look.  A CTA holds the entries of up to 32 lists in registers (sixteen per thread),
@@ -276,7 +275,7 @@ __global__ void __launch_bounds__(SLOT_T) topk_slots_kernel(SlotParams P) {
   const long long q = blockIdx.x;
   const int tile = (int)(q / P.qpt), et = (int)(q - (long long)tile * P.qpt);
   const int g = tile / P.mt, m = tile - g * P.mt;
-  const int n_sub = P.mt == 2 ? 1 : 2;
+  const int n_sub = 4 / P.mt;
   if (warp == 0) {  // the CTAs that can have met this group
     int n = 0;
     for (int c0 = 0; c0 < P.n_ctas; c0 += 32) {
@@ -301,7 +300,7 @@ __global__ void __launch_bounds__(SLOT_T) topk_slots_kernel(SlotParams P) {
     const int li = lo + u * (SLOT_T / 32) + warp;
     if (li < hi) {
       const int sub = li % n_sub;
-      const long long list = (long long)slots[li / n_sub] * (2 * P.qpt) + (P.mt == 2 ? m : sub) * P.qpt + et;
+      const long long list = (long long)slots[li / n_sub] * (4 * P.qpt) + (sub * P.mt + m) * P.qpt + et;
       const int c = list < P.n_lists ? min(P.hdr[list].x, SLOT_CAP) : 0;
 #pragma unroll
       for (int x = 0; x < PER_LIST; ++x) {
@@ -346,7 +345,7 @@ static int launch_topk(TopkParams& P, cudaStream_t st);
 // units can touch one tile group are at most n_ctas / n_groups + 2.)
 int topk_merge_parts(int n_ctas, int n_groups, int mt) {
   if (n_ctas <= 0 || n_groups <= 0) return 1;
-  return (int)ceil_div((int64_t)(n_ctas / n_groups + 2) * (mt == 2 ? 1 : 2), SLOT_LISTS);
+  return (int)ceil_div((int64_t)(n_ctas / n_groups + 2) * (4 / mt), SLOT_LISTS);
 }
 
 int launch_topk_slots(const float* keys, const int* idx, const int2* hdr, long long n_lists, int cap, int n_ctas, int n_groups,
