@@ -41,11 +41,16 @@ namespace lik {
 
 namespace {
 
-constexpr int TILE_N = 128;         // document tokens per piece: rows of a TMA stage, columns of an accumulator
-constexpr int SETS = 4;             // accumulators of 128 columns fill the 512 of tensor memory; each has its own set of epilogue warps
+constexpr int TILE_N = 96;          // document tokens per piece: rows of a TMA stage, columns of an accumulator
+constexpr int SETS = 4;             // accumulators, each with its own set of epilogue warps
 constexpr int SET_WARPS = 4;        // one per quadrant of 32 TMEM lanes
 constexpr int ACC_COLS = TILE_N;
-constexpr int BOX_ROWS = 32;        // granule of the document TMA boxes: 32, 64, 96 and 128 rows
+// The query tiles sit in tensor memory behind the accumulators, 64 columns each: an MMA that reads A from shared memory moves
+// 4 KB of it for every 16 features, more than the 3 KB of 96 document rows, and took 56 cycles instead of 48 for that.
+constexpr int A_COL0 = SETS * ACC_COLS;
+constexpr int A_COLS = 64;
+static_assert(A_COL0 + 2 * A_COLS == 512, "accumulators and query tiles fill the tensor memory");
+constexpr int BOX_ROWS = 32;        // granule of the document TMA boxes: 32, 64 and 96 rows
 constexpr int N_BOXES = TILE_N / BOX_ROWS;
 constexpr int SLAB_BYTES_ROW = 128; // one swizzle span: 64 two-byte or 128 one-byte elements
 constexpr int MAX_SLABS = 2;
@@ -118,6 +123,7 @@ struct TcParams {
   int sc_per;
   int sc_slots;          // lanes * sc_per, or 0
   float norm_eps;     // > 0: the kernel takes the documents' inverse norms from the tiles themselves (NORM_WARPS)
+  int d_deep;         // the documents' rows fill their slabs: one copy brings all slabs of a piece
   int d_full_count;   // arrivals that complete a ring stage: 1 (TMA) or the number of decompress warps
   TopkOut topk;       // cand_key == nullptr: scores are written instead
   PlaidSrc plaid;     // PLAID kernels: the compressed documents
@@ -131,7 +137,8 @@ constexpr int NORM_WARPS = 2;
 constexpr int PLAID_WARPS = 3;  // warps 0, 18 and 19 decode compressed tokens in the PLAID kernels
 
 struct SharedCtl {
-  unsigned long long q_full[2], q_empty[2];  // by place of the query tile (two resident tiles use the first)
+  unsigned long long q_full, q_empty;
+  unsigned long long a_idle[2];       // an issuer's MMAs on the query tiles in tensor memory are done
   unsigned long long d_full[8], d_empty[8];
   unsigned long long acc_full[SETS], acc_empty[SETS];
   unsigned long long set_sync[SETS];  // rendezvous of an epilogue set
@@ -298,8 +305,6 @@ __device__ __forceinline__ UnitRaw unit_fetch(const TcParams& P, const UnitWalk&
   }
   return r;
 }
-// Tokens per piece of a document: it is cut where an accumulator is full, one that fits two in two halves of about the same size.
-__device__ __forceinline__ int piece_of(int dlen) { return dlen > TILE_N && dlen <= 2 * TILE_N ? (((dlen + 1) >> 1) + 31) & ~31 : TILE_N; }
 // First row and column count of the fetched document; `masked` tells whether its mask has holes.
 // Lengths come from the caller-validated views, clamped to the padded extent.
 // (the tensor-core path takes fewer than 2^31 rows)
@@ -329,11 +334,11 @@ __device__ __forceinline__ void unit_resolve(const TcParams& P, const UnitRaw& r
   row = (int)row0;
 }
 
-// Sum of squares of one row of a stage (lane = row: eight consecutive rows of a swizzled slab lie in different banks).  The
+// Sum of squares of one row of a stage whose second slab, if any, lies `slab_rows` rows behind the first (lane = row: eight consecutive rows of a swizzled slab lie in different banks).  The
 // pieces of 16 bytes are summed and combined in the order of prep_kernel's butterfly, so that the norms of a row are the
 // same number wherever they are taken.
 template <typename T>
-__device__ __forceinline__ float stage_row_sum_sq(const unsigned char* row, int r, bool two_slabs) {
+__device__ __forceinline__ float stage_row_sum_sq(const unsigned char* row, int r, int slab_rows) {
   float half[2];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {  // pieces h, h + 2, h + 4, h + 6, each beside its partner eight further: their loads in flight together
@@ -343,7 +348,7 @@ __device__ __forceinline__ float stage_row_sum_sq(const unsigned char* row, int 
       const unsigned char* a = row + (((2 * i + h) ^ (r & 7)) << 4);
       x[i] = *reinterpret_cast<const uint4*>(a);
       y[i] = make_uint4(0, 0, 0, 0);
-      if (two_slabs) y[i] = *reinterpret_cast<const uint4*>(a + TILE_N * SLAB_BYTES_ROW);
+      if (slab_rows) y[i] = *reinterpret_cast<const uint4*>(a + slab_rows * SLAB_BYTES_ROW);
     }
     float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -359,17 +364,17 @@ __device__ __forceinline__ float stage_row_sum_sq(const unsigned char* row, int 
 }
 
 struct DocMaps {
-  CUtensorMap m[N_BOXES];  // document boxes of 32, 64, ... rows: one copy per K slab whatever the tile height
+  CUtensorMap flat[N_BOXES];  // document boxes of 32, 64, 96 rows, one 128-byte slab wide
+  CUtensorMap deep[N_BOXES];  // the same with all slabs of the rows, slab behind slab (rows that fill their slabs)
 };
 
 // Word the producer leaves beside every ring stage for the MMA issuer.
-constexpr uint32_t STAGE_COLS_MASK = 0x1FFu;   // valid document rows in the stage
+constexpr uint32_t STAGE_COLS_MASK = 0x7Fu;    // rows of the stage that are multiplied: a multiple of 32
 constexpr int STAGE_LANE_SHIFT = 16;           // the lane whose accumulator(s) the piece feeds
-constexpr uint32_t STAGE_FIRST = 1u << 18;     // first stage of a query-tile group: wait for the tiles
-constexpr uint32_t STAGE_LAST = 1u << 19;      // last stage of the group: hand the tiles back afterwards
+constexpr uint32_t STAGE_FIRST = 1u << 18;     // first stage of a query-tile group: take the tiles over first
 constexpr uint32_t STAGE_END = 1u << 20;       // no more work
 constexpr uint32_t STAGE_LONE = 1u << 21;      // the second accumulator has no query tile: it changes hands, nothing is multiplied into it
-constexpr uint32_t STAGE_QSLOT = 1u << 22;     // the query tile lies in the second place
+constexpr uint32_t STAGE_WIDE = 1u << 22;      // the slabs lie a full stage apart instead of right behind each other
 
 // Monotone map float -> unsigned (larger float, larger key); 0 is below every float.
 __device__ __forceinline__ unsigned ordered_key(float f) {
@@ -441,8 +446,8 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int q_tile_bytes = P.n_slabs * TILE_M * SLAB_BYTES_ROW;
   const int d_stage_bytes = P.n_slabs * TILE_N * SLAB_BYTES_ROW;
-  unsigned char* q_smem = smem;                              // [2][n_slabs][128 rows][128 B]
-  unsigned char* d_smem = smem + 2 * q_tile_bytes;           // [stages][n_slabs][128 rows][128 B]
+  unsigned char* q_smem = smem;                              // [mt][n_slabs][128 rows][128 B], on their way to tensor memory
+  unsigned char* d_smem = smem + P.mt * q_tile_bytes;        // [stages][n_slabs][rows][128 B]
   float* sc_ring = reinterpret_cast<float*>(d_smem + (size_t)P.stages * d_stage_bytes);  // [lanes][sc_per][TILE_N] (kernels with multipliers)
   SharedCtl* ctl = reinterpret_cast<SharedCtl*>(d_smem + (size_t)P.stages * d_stage_bytes + (size_t)P.sc_slots * TILE_N * sizeof(float));
 
@@ -454,10 +459,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
   const bool norm_warps = SCALED && !FP8 && !PLAID && P.norm_eps > 0.f;  // (a member of every pipeline barrier then)
   const int n_issuers = PLAID || norm_warps ? 1 : 2;
   if (tid == 0) {
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&ctl->q_full[i]), 1);
-      mbar_init(smem_u32(&ctl->q_empty[i]), (uint32_t)n_issuers);
-    }
+    mbar_init(smem_u32(&ctl->q_full), 1);
+    mbar_init(smem_u32(&ctl->q_empty), (uint32_t)n_issuers);
+    for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&ctl->a_idle[i]), 1);
     for (int s = 0; s < P.stages; ++s) {
       mbar_init(smem_u32(&ctl->d_full[s]), (uint32_t)P.d_full_count);
       mbar_init(smem_u32(&ctl->d_empty[s]), (uint32_t)(norm_warps ? n_issuers + NORM_WARPS : n_issuers));
@@ -473,7 +477,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
     fence_barrier_init();
     prefetch_tmap(&q_map);
     if (!PLAID)
-      for (int i = 0; i < N_BOXES; ++i) prefetch_tmap(&d_maps.m[i]);
+      for (int i = 0; i < N_BOXES; ++i) prefetch_tmap(P.d_deep ? &d_maps.deep[i] : &d_maps.flat[i]);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(&ctl->tmem_base), 512);
@@ -503,17 +507,17 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
     {
       const int pw = warp == 0 ? 0 : warp - (2 + SETS * SET_WARPS) + 1;  // decoder warp number 0..2
       const bool elect = warp == 0 && elect_one();
-      int cur_grp = -1, q_slot = 1;
+      int cur_grp = -1;
       uint32_t n_qload = 0, st = 0, ph = 0, n_dload = 0;
       const int x_per_slab = SLAB_BYTES_ROW / P.elt_bytes;
       bool ok = true;
       uint32_t lone = 0, first = 0;
       // the documents in flight, one per lane: what is left of each
-      int l_len[SETS], l_c0[SETS], l_piece[SETS], l_uc[SETS], l_sc[SETS], l_row[SETS];
+      int l_len[SETS], l_c0[SETS], l_uc[SETS], l_sc[SETS], l_row[SETS];
 #pragma unroll
       for (int l = 0; l < SETS; ++l) {
         l_len[l] = -1;  // none
-        l_c0[l] = l_piece[l] = l_uc[l] = l_sc[l] = l_row[l] = 0;
+        l_c0[l] = l_uc[l] = l_sc[l] = l_row[l] = 0;
       }
       int open = 0;  // lanes with a document
       // 32 units at a time, a lane of the warp each: a batch that is dealt out, and one whose length words are on their way
@@ -569,18 +573,16 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
               first = STAGE_FIRST;
               const int t0 = grp * P.mt, t1 = min(t0 + P.mt, n_tiles);
               lone = P.mt == 2 && t1 - t0 < 2 ? STAGE_LONE : 0u;
-              q_slot = P.mt == 2 ? 0 : q_slot ^ 1;  // a lone tile has two places, so that the next one need not wait for the last to be done with
               if (warp == 0) {
-                // wait until the MMAs that read the previous query tiles in this place are done
-                const uint32_t use = P.mt == 2 ? n_qload : n_qload >> 1;
-                ok = wait_bar_warp(&ctl->q_empty[q_slot], (use & 1) ^ 1, ctl, P.status);
+                // wait until the issuers have copied the previous query tiles to tensor memory
+                ok = wait_bar_warp(&ctl->q_empty, (n_qload & 1) ^ 1, ctl, P.status);
                 if (ok && elect) {
-                  mbar_arrive_expect_tx(smem_u32(&ctl->q_full[q_slot]), (uint32_t)((t1 - t0) * q_tile_bytes));
+                  mbar_arrive_expect_tx(smem_u32(&ctl->q_full), (uint32_t)((t1 - t0) * q_tile_bytes));
                   for (int t = t0; t < t1; ++t) {
                     TileInfo ti = tile_info(P, t);
                     for (int sl = 0; sl < P.n_slabs; ++sl)
-                      tma_load_2d(smem_u32(q_smem + (q_slot + t - t0) * q_tile_bytes + sl * TILE_M * SLAB_BYTES_ROW), &q_map, sl * x_per_slab,
-                                  (int)ti.row0, smem_u32(&ctl->q_full[q_slot]));
+                      tma_load_2d(smem_u32(q_smem + (t - t0) * q_tile_bytes + sl * TILE_M * SLAB_BYTES_ROW), &q_map, sl * x_per_slab, (int)ti.row0,
+                                  smem_u32(&ctl->q_full));
                   }
                 }
                 __syncwarp();
@@ -592,27 +594,31 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
             // unit passes through the same hand-shakes
             if (elect) {
               ctl->unit_info[l][l_uc[l] & (UNIT_RING - 1)] = make_int4(dlen | (SCALED ? l_sc[l] << UNIT_SLOT_SHIFT : 0) | dmasked, drow0, grp, doc);
-              __threadfence_block();
-              ctl->units_posted[l] = l_uc[l] + 1;
+              if (SCALED) {  // (the others learn of it from a full accumulator)
+                __threadfence_block();
+                ctl->units_posted[l] = l_uc[l] + 1;
+              }
             }
             ++l_uc[l];
             ++open;
             l_len[l] = dlen;
             l_c0[l] = 0;
             l_row[l] = drow0;
-            l_piece[l] = piece_of(dlen);
           }
           // the lane's next piece
           const int c0 = l_c0[l], dlen = l_len[l], drow0 = l_row[l];
-          const int ncols = min(l_piece[l], dlen - c0);
-          const bool ends = c0 + l_piece[l] >= dlen;
+          const int ncols = min(TILE_N, dlen - c0);
+          const bool ends = c0 + TILE_N >= dlen;
+          const int rows = __shfl_sync(0xffffffffu, (ncols + BOX_ROWS - 1) & ~(BOX_ROWS - 1), 0);
+          // A short document that is no multiple of 32 tokens takes two boxes, the second moved back to end where the document
+          // ends; a longer one's last piece is moved back as a whole.
+          const bool split = SHIFT && dlen < rows && dlen > BOX_ROWS;
           ok = wait_bar_warp(&ctl->d_empty[st], ph ^ 1, ctl, P.status);
           if (!ok) continue;
           const uint32_t full = smem_u32(&ctl->d_full[st]);
           if (ends) --open;
-          uint32_t info = (uint32_t)ncols | ((uint32_t)l << STAGE_LANE_SHIFT) | (q_slot ? STAGE_QSLOT : 0u) | first | lone;
-          if (ends && !open && !(have && nx_grp == cur_grp)) info |= STAGE_LAST;
-          if (elect) ctl->stage_info[st] = info;
+          if (elect)
+            ctl->stage_info[st] = (uint32_t)rows | ((uint32_t)l << STAGE_LANE_SHIFT) | first | lone | (split || PLAID ? STAGE_WIDE : 0u);
           first = 0;
           if (PLAID) {
             // the piece's tokens in six equal runs, one per half-warp of the three decoder warps
@@ -634,23 +640,23 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
             __syncwarp();
             if (lane == 0) mbar_arrive(full);
           } else {
-            const int boxes = (ncols + BOX_ROWS - 1) / BOX_ROWS;
-            const bool moved = SHIFT && (ncols & (BOX_ROWS - 1)) != 0 && dlen >= BOX_ROWS;
-            const int straight = __shfl_sync(0xffffffffu, moved ? boxes - 1 : boxes, 0);  // boxes that lie one behind the other
-            const int row = __shfl_sync(0xffffffffu, drow0 + c0, 0);
+            const int row = __shfl_sync(0xffffffffu, drow0 + (SHIFT ? max(min(c0, dlen - rows), 0) : c0), 0);
             // the piece's multipliers ride on the same barrier: whole groups of four floats, never past the array's end
             uint32_t sc_bytes = 0;
-            if (SCALED && P.col_src && boxes > 0) sc_bytes = (uint32_t)min((long long)((ncols + 3) & ~3), P.d.n_rows - row) * 4u;
+            if (SCALED && P.col_src && rows > 0) sc_bytes = (uint32_t)min((long long)((ncols + 3) & ~3), P.d.n_rows - row) * 4u;
             if (elect) {
               const uint32_t dst = smem_u32(d_smem) + st * (uint32_t)d_stage_bytes;
-              if (boxes > 0) {
-                mbar_arrive_expect_tx(full, (uint32_t)(boxes * BOX_ROWS * SLAB_BYTES_ROW * P.n_slabs) + sc_bytes);
-#pragma unroll
-                for (int sl = 0; sl < MAX_SLABS; ++sl) {
-                  if (sl >= P.n_slabs) continue;
-                  const uint32_t to = dst + sl * TILE_N * SLAB_BYTES_ROW;
-                  if (!SHIFT || straight) tma_load_2d(to, &d_maps.m[straight - 1], sl * x_per_slab, row, full);
-                  if (moved) tma_load_2d(to + straight * BOX_ROWS * SLAB_BYTES_ROW, &d_maps.m[0], sl * x_per_slab, row + ncols - BOX_ROWS, full);
+              if (rows > 0) {
+                mbar_arrive_expect_tx(full, (uint32_t)(rows * SLAB_BYTES_ROW * P.n_slabs) + sc_bytes);
+                const int box = rows / BOX_ROWS - 1;
+                if (!split && P.d_deep) {
+                  tma_load_3d(dst, &d_maps.deep[box], 0, row, 0, full);
+                } else {
+                  const uint32_t slab = (uint32_t)((split ? TILE_N : rows) * SLAB_BYTES_ROW);
+                  for (int sl = 0; sl < P.n_slabs; ++sl) {
+                    tma_load_2d(dst + sl * slab, &d_maps.flat[split ? box - 1 : box], sl * x_per_slab, row, full);
+                    if (split) tma_load_2d(dst + sl * slab + box * BOX_ROWS * SLAB_BYTES_ROW, &d_maps.flat[0], sl * x_per_slab, row + dlen - BOX_ROWS, full);
+                  }
                 }
                 if (sc_bytes) bulk_load_1d(smem_u32(sc_ring + (l * P.sc_per + l_sc[l]) * TILE_N), P.col_src + row, sc_bytes, full);
               } else {
@@ -662,7 +668,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
           ++n_dload;
           if (++st == (uint32_t)P.stages) { st = 0; ph ^= 1; }
           if (SCALED && ++l_sc[l] >= P.sc_per) l_sc[l] = 0;
-          l_c0[l] = c0 + l_piece[l];
+          l_c0[l] = c0 + TILE_N;
           if (ends) l_len[l] = -1;
         }
       }
@@ -695,10 +701,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
             }
           }
         }
-        for (uint32_t i = 1; i <= (P.mt == 2 ? 1u : 2u) && i <= n_qload; ++i) {
-          const uint32_t load = n_qload - i, slot = P.mt == 2 ? 0u : load & 1, use = P.mt == 2 ? load : load >> 1;
-          const uint32_t bar = smem_u32(&ctl->q_full[slot]);
-          for (int spin = 0; spin < (1 << 16) && !mbar_try_wait(bar, use & 1); ++spin) {
+        if (n_qload) {
+          const uint32_t bar = smem_u32(&ctl->q_full);
+          for (int spin = 0; spin < (1 << 16) && !mbar_try_wait(bar, (n_qload - 1) & 1); ++spin) {
           }
         }
       }
@@ -713,7 +718,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
     // tensor pipe holds about four MMAs ahead, some 250 cycles, and the waits and words of a piece take a warp longer than
     // that; each of the two has the other's MMAs to hide behind.
     const uint32_t me = warp == 1 ? 0u : 1u;
-    uint32_t st = 0, ph = 0, q_ph = 0, acc_ph = 0;  // q_ph, acc_ph: one phase bit per place / accumulator
+    uint32_t st = 0, ph = 0, n_q = 0, acc_ph = 0;  // acc_ph: one phase bit per accumulator
     bool ok = true;
     const bool issue = elect_one();
     const uint32_t desc_hi = (uint32_t)(smem_desc_sw128(0) >> 32);
@@ -740,15 +745,32 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
         }
         break;
       }
-      const uint32_t q_slot = info & STAGE_QSLOT ? 1u : 0u;
       if (info & STAGE_FIRST) {
-        ok = wait_bar_warp(&ctl->q_full[q_slot], (q_ph >> q_slot) & 1u, ctl, P.status);
+        // New query tiles: this warp copies the ones it multiplies with to its place(s) in tensor memory, once its MMAs on the
+        // old ones are done.  (A copy and an MMA that follows it run in order.)  With one tile and two issuers either has its own.
+        ok = wait_bar_warp(&ctl->q_full, n_q & 1u, ctl, P.status);
+        if (ok && n_q) {
+          if (issue) tc_commit(smem_u32(&ctl->a_idle[me]));
+          __syncwarp();
+          ok = wait_bar_warp(&ctl->a_idle[me], (n_q - 1) & 1u, ctl, P.status);
+        }
         if (!ok) break;
-        q_ph ^= 1u << q_slot;
+        ++n_q;
+        tc_fence_after();
+        if (issue) {
+          for (uint32_t t = 0; t < mt; ++t) {
+            if (mt == 2 && step == 2 && t != me) continue;
+            const uint32_t to = tmem_base + A_COL0 + (mt == 2 ? t : me) * A_COLS;
+            for (int k = 0; k < k_steps; ++k) tc_copy_128x256b(to + 8 * k, a_desc0 + t * q_desc + (uint32_t)((k & 3) * 2) + (k >> 2) * A_SLAB, desc_hi);
+          }
+          tc_commit(smem_u32(&ctl->q_empty));
+        }
+        __syncwarp();
       }
-      const uint32_t ncols = info & STAGE_COLS_MASK;
-      const uint32_t idesc = idesc0 | (SHIFT ? ((ncols + 31) >> 5) << 19 : ((ncols + 15) >> 4) << 18);  // N / 8 in bits 17..22
+      const uint32_t rows = info & STAGE_COLS_MASK;
+      const uint32_t idesc = idesc0 | (rows << 14);  // N / 8 in bits 17..22
       const uint32_t b_stage = b_desc0 + st * stage_desc;
+      const uint32_t b_slab = info & STAGE_WIDE ? B_SLAB : rows * (SLAB_BYTES_ROW >> 4);
       const uint32_t set0 = ((info >> STAGE_LANE_SHIFT) & (SETS - 1)) * mt;
       uint32_t a = set0;
       if (step == 2 && ((a ^ me) & 1u)) ++a;
@@ -761,21 +783,18 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
         const uint32_t t = a - set0;
         tc_fence_after();
         if (issue) {
-          if (ncols && !(t == 1 && (info & STAGE_LONE))) {  // (the accumulator always changes hands, so that both sides keep their phase)
+          if (rows && !(t == 1 && (info & STAGE_LONE))) {  // (the accumulator always changes hands, so that both sides keep their phase)
             const uint32_t d_tmem = tmem_base + a * ACC_COLS;
-            const uint32_t a_desc = a_desc0 + (t + q_slot) * q_desc;
+            const uint32_t a_tmem = tmem_base + A_COL0 + (mt == 2 ? t : me) * A_COLS;
             // descriptors differ only in the start address, in units of 16 bytes
             if (k_steps == 8) {  // the common width (128 two-byte or 256 one-byte elements): straight-line issue
 #pragma unroll
               for (int k = 0; k < 8; ++k)
-                tc_mma<FP8>(d_tmem, a_desc + (uint32_t)((k & 3) * 2) + (k >> 2) * A_SLAB, b_stage + (uint32_t)((k & 3) * 2) + (k >> 2) * B_SLAB, desc_hi,
-                            idesc, k ? 1u : 0u);
+                tc_mma_ts<FP8>(d_tmem, a_tmem + 8 * k, b_stage + (uint32_t)((k & 3) * 2) + (k >> 2) * b_slab, desc_hi, idesc, k ? 1u : 0u);
             } else {
 #pragma unroll
               for (int k = 0; k < 8; ++k)
-                if (k < k_steps)
-                  tc_mma<FP8>(d_tmem, a_desc + (uint32_t)((k & 3) * 2) + (k >> 2) * A_SLAB, b_stage + (uint32_t)((k & 3) * 2) + (k >> 2) * B_SLAB,
-                              desc_hi, idesc, k ? 1u : 0u);
+                if (k < k_steps) tc_mma_ts<FP8>(d_tmem, a_tmem + 8 * k, b_stage + (uint32_t)((k & 3) * 2) + (k >> 2) * b_slab, desc_hi, idesc, k ? 1u : 0u);
             }
           }
           tc_commit(smem_u32(&ctl->acc_full[a]));
@@ -784,9 +803,8 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
       }
       if (!ok) break;
       if (issue) {
-        if (mine) tc_commit(smem_u32(&ctl->d_empty[st]));                   // ring slot reusable once these MMAs retire
+        if (mine) tc_commit(smem_u32(&ctl->d_empty[st]));  // ring slot reusable once these MMAs retire
         else mbar_arrive(smem_u32(&ctl->d_empty[st]));
-        if (info & STAGE_LAST) tc_commit(smem_u32(&ctl->q_empty[q_slot]));  // and so are the query tiles
       }
       __syncwarp();
       if (++st == (uint32_t)P.stages) { st = 0; ph ^= 1; }
@@ -964,7 +982,6 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
         }
       }
       const int dlen = uinfo.x & UNIT_LEN_MASK;
-      const int piece = piece_of(dlen);
       int sc_slot = SCALED ? (uinfo.x >> UNIT_SLOT_SHIFT) & 15 : 0;  // multiplier slot of the unit's first piece, in its lane's ring
       const long long drow0 = uinfo.y;
       const bool holes = (uinfo.x & LEN_FLAG_MASKED) != 0;  // the document's mask is not a plain prefix
@@ -981,7 +998,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
       constexpr bool lazy = decltype(lazy_)::value;        // long document: winner scan only when some row of the warp needs it
       constexpr bool use_cols = SCALED || general;          // per-column multiplier / additive mask needed
       do {
-        const int ncols = max(0, min(piece, dlen - c0));
+        const int ncols = max(0, min(TILE_N, dlen - c0));
+        // SHIFT: the token of the piece's first column; a chunk of 32 columns never reaches behind the document's end
+        const int base = SHIFT ? max(min(c0, dlen - ((ncols + 31) & ~31)), 0) : c0;
         // Per-column arrays of this piece, staged by the whole set.  There are two of them, so that the one rendezvous
         // behind the writes also says that everyone is done with the one that the piece after the next will overwrite.
         float* const col_scale = ctl->col_scale[set][n_col & 1];
@@ -990,13 +1009,12 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
         const float* const sc_arr = SCALED && bulk ? sc_ring + (ln * P.sc_per + sc_slot) * TILE_N : col_scale;
         auto stage_columns = [&]() {
           ++n_col;
-          const int whole = ncols & ~31;
           const int c = et;  // a thread per column
           if (c < ((ncols + 31) & ~31)) {
             float sc = 1.f, bi = -INFINITY;
-            const int t = SHIFT && c >= whole && dlen >= BOX_ROWS ? ncols - ((ncols + 31) & ~31) + c : c;  // the token that column c stands for
-            if (t < ncols) {
-              const long long drow = drow0 + c0 + t;
+            const int tok = SHIFT && dlen >= BOX_ROWS ? min(base + (c & ~31), dlen - BOX_ROWS) + (c & 31) : base + c;  // the token that column c stands for
+            if (tok < dlen) {
+              const long long drow = drow0 + tok;
               sc = norm_warps ? sc_arr[c] : row_factor(P.d, drow);
               bi = row_valid(P.d, drow) ? 0.f : -INFINITY;
             }
@@ -1038,7 +1056,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
             tmem_ld_wait(v);
             affine32(v, col_scale + cc, col_bias + cc);  // bias is -inf past ncols and in holes
             if (cc + 32 >= ncols) LIK_RELEASE_ACC();
-            fold32<ARGMAX, lazy>(v, c0 + (SHIFT && dlen >= BOX_ROWS ? min(cc, ncols - 32) : cc), run_m, run_i);
+            fold32<ARGMAX, lazy>(v, SHIFT && dlen >= BOX_ROWS ? min(base + cc, dlen - BOX_ROWS) : base + cc, run_m, run_i);
           }
         } else if (use_cols) {
           // whole chunks are valid: multiplier only; the partial last chunk also takes the mask (-inf past ncols).
@@ -1061,13 +1079,13 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
             tmem_ld32_issue(lane_addr + (uint32_t)cc, v);
             tmem_ld_wait(v);
             if (cc + 32 >= ncols) LIK_RELEASE_ACC();
-            int at = min(cc, ncols - 32);  // (below 0 where a long document's last piece is shorter than a box)
+            int at = min(base + cc, dlen - BOX_ROWS);
             if (dlen < BOX_ROWS) {  // a document of fewer than 32 tokens is all that still needs a mask
 #pragma unroll
               for (int i = 0; i < 32; ++i) v[i] = i < ncols ? v[i] : -INFINITY;
               at = 0;
             }
-            fold32<ARGMAX, lazy>(v, c0 + at, run_m, run_i);
+            fold32<ARGMAX, lazy>(v, at, run_m, run_i);
           }
         } else {
           for (; cc < ncols; cc += 32) {
@@ -1083,7 +1101,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
           }
         }
 #undef LIK_RELEASE_ACC
-        c0 += piece;
+        c0 += TILE_N;
         if (SCALED && ++sc_slot >= P.sc_per) sc_slot = 0;
       } while (c0 < dlen);
       };
@@ -1157,7 +1175,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
         for (uint32_t a = 0; a < SETS; ++a) announce(a);
         break;
       }
-      const int ncols = (int)(info & STAGE_COLS_MASK);
+      const int rows = (int)(info & STAGE_COLS_MASK);
       const uint32_t ln = (info >> STAGE_LANE_SHIFT) & (SETS - 1);
       int at = 0;
 #pragma unroll
@@ -1168,9 +1186,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
         }
       float* slot = sc_ring + (ln * P.sc_per + at) * TILE_N;
       const unsigned char* stage = d_smem + (size_t)st * d_stage_bytes;
-      for (int r = nw * 32 + lane; r < ncols; r += NORM_WARPS * 32) {
-        const float ss = bf16 ? stage_row_sum_sq<__nv_bfloat16>(stage + r * SLAB_BYTES_ROW, r, two_slabs)
-                              : stage_row_sum_sq<__half>(stage + r * SLAB_BYTES_ROW, r, two_slabs);
+      for (int r = nw * 32 + lane; r < rows; r += NORM_WARPS * 32) {
+        const float ss = bf16 ? stage_row_sum_sq<__nv_bfloat16>(stage + r * SLAB_BYTES_ROW, r, two_slabs ? rows : 0)
+                              : stage_row_sum_sq<__half>(stage + r * SLAB_BYTES_ROW, r, two_slabs ? rows : 0);
         slot[r] = inv_norm(ss, P.norm_eps);
       }
       __syncwarp();
@@ -1197,7 +1215,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
 __global__ void wait_probe_kernel(long long limit, int* status, int* result) {
   __shared__ SharedCtl ctl;
   if (threadIdx.x == 0) {
-    mbar_init(smem_u32(&ctl.q_full[0]), 1);
+    mbar_init(smem_u32(&ctl.q_full), 1);
     ctl.abort_flag = 0;
     ctl.wait_limit = limit;
     fence_barrier_init();
@@ -1205,7 +1223,7 @@ __global__ void wait_probe_kernel(long long limit, int* status, int* result) {
   __syncthreads();
   if (threadIdx.x == 0) {
     const long long t0 = clock64();
-    const bool got = wait_bar(&ctl.q_full[0], 0, &ctl, status);
+    const bool got = wait_bar(&ctl.q_full, 0, &ctl, status);
     const long long dt = clock64() - t0;
     result[0] = got ? 1 : 0;
     result[1] = ctl.abort_flag;
@@ -1302,7 +1320,8 @@ EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-int make_map(CUtensorMap* map, const lik_seqs& s, int dtype, int dim, int box_rows) {
+// `slabs` 0: a map over the rows, one slab wide; otherwise rows x slabs, whose boxes hold all slabs of their rows
+int make_map(CUtensorMap* map, const lik_seqs& s, int dtype, int dim, int box_rows, int slabs = 0) {
   EncodeTiledFn enc = get_encode_fn();
   if (!enc) {
     set_error("cuTensorMapEncodeTiled is not available from this driver");
@@ -1312,11 +1331,12 @@ int make_map(CUtensorMap* map, const lik_seqs& s, int dtype, int dim, int box_ro
   CUtensorMapDataType dt = dtype == LIK_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                            : dtype == LIK_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                               : CU_TENSOR_MAP_DATA_TYPE_UINT8;
-  cuuint64_t gdim[2] = {(cuuint64_t)dim, (cuuint64_t)(s.n_rows > 0 ? s.n_rows : 1)};
-  cuuint64_t gstride[1] = {(cuuint64_t)s.row_stride * eb};
-  cuuint32_t box[2] = {(cuuint32_t)(SLAB_BYTES_ROW / eb), (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(map, dt, 2, const_cast<void*>(s.data), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  const cuuint32_t slab_elems = (cuuint32_t)(SLAB_BYTES_ROW / eb);
+  cuuint64_t gdim[3] = {slabs ? (cuuint64_t)slab_elems : (cuuint64_t)dim, (cuuint64_t)(s.n_rows > 0 ? s.n_rows : 1), (cuuint64_t)slabs};
+  cuuint64_t gstride[2] = {(cuuint64_t)s.row_stride * eb, (cuuint64_t)SLAB_BYTES_ROW};
+  cuuint32_t box[3] = {slab_elems, (cuuint32_t)box_rows, (cuuint32_t)slabs};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(map, dt, slabs ? 3 : 2, const_cast<void*>(s.data), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     set_error("cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
@@ -1395,7 +1415,7 @@ TcPlan plan_tc(const lik_fwd_args& a, const TcExtra& x) {
   pl.grid = (int)(g < 0 ? 0 : g);
   // the fused top-k numbers its candidate lists by CTA: the same grid whatever the piece of the corpus
   if (x.topk_k > 0 && pl.grid > 0) pl.grid = sm_count();
-  const size_t q_bytes = 2 * (size_t)pl.n_slabs * TILE_M * SLAB_BYTES_ROW;
+  const size_t q_bytes = (size_t)pl.mt * pl.n_slabs * TILE_M * SLAB_BYTES_ROW;
   const size_t stage = (size_t)pl.n_slabs * TILE_N * SLAB_BYTES_ROW;
   const size_t fixed = q_bytes + sizeof(SharedCtl) + 1024;
   const size_t budget = 227 * 1024;
@@ -1551,9 +1571,11 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
   memset(&d_maps, 0, sizeof(d_maps));
   int rc = make_map(&q_map, a.q, a.dtype, a.dim, TILE_M);
   if (rc) return rc;
+  const bool deep = a.dim * (int)dtype_size(a.dtype) == pl.n_slabs * SLAB_BYTES_ROW;
   if (!plaid) {
     for (int i = 0; i < N_BOXES; ++i) {
-      rc = make_map(&d_maps.m[i], a.d, a.dtype, a.dim, (i + 1) * BOX_ROWS);
+      rc = make_map(&d_maps.flat[i], a.d, a.dtype, a.dim, (i + 1) * BOX_ROWS);
+      if (!rc && deep) rc = make_map(&d_maps.deep[i], a.d, a.dtype, a.dim, (i + 1) * BOX_ROWS, pl.n_slabs);
       if (rc) return rc;
     }
   }
@@ -1582,6 +1604,7 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
   P.d_len_flagged = 0;
   P.tile_q0 = nullptr;
   P.list_tab = nullptr;
+  P.d_deep = deep;
   P.d_full_count = plaid ? PLAID_WARPS : 1;
   // Per-column multipliers that are exactly one fp32 array over the document rows (inverse norms or per-token scales,
   // not both) travel with the tiles when every tile's run of them starts on a 16-byte boundary and whole groups of four
