@@ -1,4 +1,6 @@
-// Blackwell tensor-core MaxSim forward (sm_100a: TMA + tcgen05.mma + TMEM).
+// Blackwell tensor-core MaxSim forward (sm_100a: TMA + tcgen05.mma + TMEM): the kernel for smaller problems, for norms taken
+// from the document tiles and for documents decoded from a PLAID index, and the host side of both tensor-core kernels.
+// Larger problems run in lik_fwd_streams.cu (plan_tc has the rule).
 //
 // GEMM view: rows = query tokens (A operand, K-major, 128 per tile), columns = document tokens (B
 // operand, K-major, up to 256 per tile), K = embedding width.  A CTA is persistent: it keeps one or
@@ -32,103 +34,29 @@
 #include <cstring>
 #include <type_traits>
 
-#include "lik_common.cuh"
-#include "lik_plaid_row.cuh"
-#include "lik_tc.cuh"
-#include "lik_tc_ptx.cuh"
+#include "lik_fwd_tc.cuh"
 
 namespace lik {
 
 namespace {
 
-constexpr int TILE_N = 96;          // document tokens per piece: rows of a TMA stage, columns of an accumulator
-constexpr int SETS = 4;             // accumulators, each with its own set of epilogue warps
-constexpr int SET_WARPS = 4;        // one per quadrant of 32 TMEM lanes
-constexpr int ACC_COLS = TILE_N;
-// The query tiles sit in tensor memory behind the accumulators, 64 columns each: an MMA that reads A from shared memory moves
-// 4 KB of it for every 16 features, more than the 3 KB of 96 document rows, and took 56 cycles instead of 48 for that.
-constexpr int A_COL0 = SETS * ACC_COLS;
-constexpr int A_COLS = 64;
-static_assert(A_COL0 + 2 * A_COLS == 512, "accumulators and query tiles fill the tensor memory");
-constexpr int BOX_ROWS = 32;        // granule of the document TMA boxes: 32, 64 and 96 rows
+#ifndef LIK_TILE_N
+#define LIK_TILE_N 256
+#endif
+constexpr int TILE_N = LIK_TILE_N;     // document tokens per TMA stage = columns of one accumulator
+constexpr int ACC_COLS = 256;          // TMEM columns reserved per accumulator
+static_assert(TILE_N <= ACC_COLS && TILE_N % 32 == 0, "a stage must fit one accumulator");
 constexpr int N_BOXES = TILE_N / BOX_ROWS;
-constexpr int SLAB_BYTES_ROW = 128; // one swizzle span: 64 two-byte or 128 one-byte elements
-constexpr int MAX_SLABS = 2;
 constexpr int NUM_THREADS = 640;
-constexpr long long WAIT_LIMIT_CYCLES = 4000000000ll;  // default limit of a wait: about 2 s at 2 GHz
-constexpr int UNIT_RING = 16;                 // slots of a lane's producer -> epilogue unit ring: more than ring stages + 2
+constexpr int EPI_THREADS = 128;     // threads per half of an epilogue group (one per accumulator row)
+constexpr int GROUP_WARPS = 8;
+constexpr int UNIT_RING = 8;                  // slots of the producer -> epilogue unit ring
 constexpr int LONG_DOC_TOKENS = 2048;         // problems whose documents can be this long run the kernel with the lazy winner scan
-constexpr int UNIT_LEN_MASK = 0xFFFFFF;       // unit_info.x: document length in the low 24 bits,
-constexpr int UNIT_SLOT_SHIFT = 24;           // the multiplier slot of its first piece in bits 24..27, LEN_FLAG_MASKED above,
-constexpr int UNIT_END = 1 << 31;             // the sign bit in the entries behind the last unit
 
-// ---------------------------------------------------------------------------------------------
-// Kernel parameters
-// ---------------------------------------------------------------------------------------------
-// Fused top-k (retrieve).  Instead of a score matrix the epilogue keeps candidate lists: one list per
-// (CTA, query) for every query of the tile groups the CTA works on.  A CTA meets the documents of a
-// group in ascending order, so a list is append-only in document order; a score enters when it beats the
-// list's threshold (strictly: an equal score that arrives later has a higher index and loses the tie).
-// A full list (TOPK_CAP entries) is cut back to its k best by the warp that owns it, which also raises
-// the threshold to the k-th best.  The lists of a query are merged by lik::launch_topk_slots afterwards.
-// List slot of (CTA c, group g) is c + g: a CTA works on a contiguous range of groups and the ranges of
-// consecutive CTAs are ordered, so c + g is unique among the pairs that occur.
-constexpr int TOPK_CAP = 256;  // entries per list: eight per lane of the owning warp
-struct TopkOut {
-  float* cand_key;  // [n_slots * qpg][TOPK_CAP]: score (negated when the smallest are wanted)
-  int* cand_idx;    // same shape: document index
-  int2* hdr;        // [n_slots * qpg]: x = entries in the list, y = threshold as an ordered key (0: none yet)
-  int k;
-  int qpg;          // lists per slot: one per accumulator and query of its tile
-  int largest;
-  int doc_base;     // added to the document index stored with a candidate
-  int n_lists;      // lists allocated (the kernel checks every list number against it)
-};
-
-// One row of the pair-list table (LIK_PAIR_LIST): written by list_units_kernel, read by the producer.
-//   x = query (0 for a pair that is out of range), y = first document row, z = document length, w = unused
-struct TcParams {
-  SeqView q, d;
-  int pairing;       // CROSS, GROUPED or LIST
-  int group;         // GROUPED: documents per query
-  int n_q, n_d;
-  int elt_bytes;     // 1 or 2
-  int ab_format;     // instruction-descriptor operand format
-  int n_slabs;       // 128-byte K slabs per row
-  int k_steps;       // MMA K steps (32 bytes each)
-  int stages;        // document ring depth
-  int q_per_tile;    // whole queries per 128-row tile (when q_chunks == 1)
-  int q_chunks;      // 128-row chunks per query (> 1: one query chunk per tile)
-  int n_tiles;       // query tiles
-  int mt;            // query tiles resident per CTA (1 or 2)
-  int n_sb;          // CROSS: the documents are walked in n_sb super-blocks of sb_docs documents (L2-sized)
-  int sb_docs;
-  long long n_flat;  // GROUPED / LIST: number of units
-  const int4* list_tab;  // LIST: one row per pair
-  float* scores;
-  float* partial;    // [n_tiles * 4, n_d] when q_chunks > 1: sums of 32 rows
-  int* argmax;
-  int argmax_stride;
-  int* status;
-  const int* tile_q0;  // packed queries: tile m holds queries [tile_q0[m], tile_q0[m+1]); tile_q0[-1] is the tile count
-  int d_len_flagged;  // d.lens carries LEN_FLAG_MASKED on documents whose mask is not a plain prefix
-  // Per-column multipliers that are one fp32 per document row (inverse norms, or per-token scales) and whose layout
-  // allows it travel with the tile: the producer copies the tile's run of them into a slot of a small ring in shared
-  // memory (bulk copy on the stage's barrier) instead of the epilogue fetching them from device memory per tile.
-  const float* col_src;  // nullptr: the epilogue stages the multipliers itself
-  // A ring of sc_per = stages + 1 slots per lane.  The slot of a lane's piece n is refilled for its piece n + sc_per: by
-  // then the MMAs of the lane's piece n + 1 have completed (the producer is at most `stages` pieces ahead of the tensor
-  // pipe), which needed the lane's accumulators back from piece n - and an epilogue gives an accumulator back only
-  // after its last read of the multipliers.
-  int sc_per;
-  int sc_slots;          // lanes * sc_per, or 0
-  float norm_eps;     // > 0: the kernel takes the documents' inverse norms from the tiles themselves (NORM_WARPS)
-  int d_deep;         // the documents' rows fill their slabs: one copy brings all slabs of a piece
-  int d_full_count;   // arrivals that complete a ring stage: 1 (TMA) or the number of decompress warps
-  TopkOut topk;       // cand_key == nullptr: scores are written instead
-  PlaidSrc plaid;     // PLAID kernels: the compressed documents
-  int plaid_f16;      // PLAID kernels: operand type fp16 instead of bf16
-};
+// Rings of multiplier slots: two of sc_per = stages + 1 slots, one per accumulator (tiles that feed both use the first).  Slot n
+// of an accumulator's ring is refilled for its tile n + sc_per: by then the MMAs of one of the sc_per - 1 tiles between them have
+// completed (the producer is at most `stages` tiles ahead of the tensor pipe), which needed the accumulator back from every
+// earlier tile - and an epilogue gives it back only after its last read of the multipliers.
 
 // Warps 18 and 19 take the rows' inverse norms from the tiles in shared memory when the launch asks for it: the documents
 // are then read once instead of twice, and no norms go through device memory.  Two queries of 128 tokens against 4000
@@ -138,27 +66,28 @@ constexpr int PLAID_WARPS = 3;  // warps 0, 18 and 19 decode compressed tokens i
 
 struct SharedCtl {
   unsigned long long q_full, q_empty;
-  unsigned long long a_idle[2];       // an issuer's MMAs on the query tiles in tensor memory are done
   unsigned long long d_full[8], d_empty[8];
-  unsigned long long acc_full[SETS], acc_empty[SETS];
-  unsigned long long set_sync[SETS];  // rendezvous of an epilogue set
+  unsigned long long acc_full[2], acc_empty[2];
   uint32_t stage_info[8];
-  int4 unit_info[SETS][UNIT_RING];    // by lane; per work unit: x = document length | flags, y = its first row, z = tile group, w = document
-  volatile int units_posted[SETS];    // entries published in a lane's ring so far
+  int4 unit_info[UNIT_RING];    // per work unit: x = document length | LEN_FLAG_MASKED, y = its first row, z = tile group, w = document
+  volatile int units_posted;    // units published in unit_info so far
+  volatile int units_total;     // all units of this CTA once the producer has walked them (INT_MAX until then)
   uint32_t tmem_base;
   volatile int abort_flag;
   long long wait_limit;         // cycles after which a wait gives up
-  short seg_off[SETS][TILE_M], seg_len[SETS][TILE_M], row_seg[SETS][TILE_M];
-  int seg_q[SETS][TILE_M];
-  int n_seg[SETS];
-  int warp_aligned[SETS];  // every query of the tile sits inside one warp's 32 rows, starting at its first row
-  float emit[SETS][2][TILE_M];
-  alignas(16) float col_scale[SETS][2][TILE_N];  // by set and parity of the piece; read as float4
-  alignas(16) float col_bias[SETS][2][TILE_N];
+  int seg_off[2][TILE_M], seg_len[2][TILE_M], seg_q[2][TILE_M];
+  short row_seg[2][TILE_M];
+  int n_seg[2];
+  int warp_aligned[2];  // every query of the tile sits inside one warp's 32 rows, starting at its first row
+  float emit[2][2][TILE_M];
+  float xch_m[2][2][TILE_M];  // half 1 -> half 0: per-row running maximum and its column
+  int xch_i[2][2][TILE_M];
+  alignas(16) float col_scale[2][TILE_N];  // read as float4
+  alignas(16) float col_bias[2][TILE_N];
   // fused top-k: state of the candidate list of every query of the resident tiles
-  int seg_cnt[SETS][TILE_M];
-  unsigned seg_thr[SETS][TILE_M];
-  int seg_list[SETS][TILE_M];      // list number (slot * qpg + query within the group)
+  int seg_cnt[2][TILE_M];
+  unsigned seg_thr[2][TILE_M];
+  int seg_list[2][TILE_M];      // list number (slot * qpg + query within the group)
   float plaid_bw[256];          // PLAID kernels: the bucket weights
 };
 
@@ -186,57 +115,24 @@ __device__ __forceinline__ bool wait_bar(unsigned long long* bar, uint32_t parit
 __device__ __forceinline__ bool wait_bar_warp(unsigned long long* bar, uint32_t parity, SharedCtl* ctl, int* status) {
   return __all_sync(0xffffffffu, wait_bar(bar, parity, ctl, status));
 }
-// Bounded wait until the producer has published entry `uc` of a lane's unit ring.  False when the CTA is aborting.
-__device__ __noinline__ bool wait_posted_slow(SharedCtl* ctl, int ln, int uc, int* status) {
+// Bounded wait until the producer has published unit `uc` of this CTA in the unit ring.
+// Returns 1 when the unit is there, 2 when the stream has ended before it, 0 when the CTA is aborting.
+__device__ __noinline__ int wait_posted_slow(SharedCtl* ctl, int uc, int* status) {
   const long long t0 = clock64();
   while (true) {
-    if (ctl->units_posted[ln] > uc) return true;
-    if (ctl->abort_flag) return false;
+    if (ctl->units_posted > uc) return 1;
+    if (ctl->units_total <= uc) return 2;
+    if (ctl->abort_flag) return 0;
     if (clock64() - t0 > ctl->wait_limit) {
       ctl->abort_flag = 1;
       if (status) atomicOr(status, LIK_DEV_WAIT_TIMEOUT);
-      return false;
+      return 0;
     }
   }
 }
-__device__ __forceinline__ bool wait_posted(SharedCtl* ctl, int ln, int uc, int* status) {
-  const bool there = ctl->units_posted[ln] > uc;
-  return __all_sync(0xffffffffu, there || wait_posted_slow(ctl, ln, uc, status));
-}
-// Bounded rendezvous of the warps that share `bar` (initialised with their number); `n` counts this warp's uses of it.
-__device__ __forceinline__ bool warps_sync(unsigned long long* bar, uint32_t& n, int lane, SharedCtl* ctl, int* status) {
-  __syncwarp();
-  if (lane == 0) mbar_arrive(smem_u32(bar));
-  return wait_bar_warp(bar, n++ & 1, ctl, status);
-}
-
-// Query tiles of tile-group g: tiles [g*mt, min((g+1)*mt, n_tiles)).
-struct TileInfo {
-  int qa, qb;        // queries [qa, qb)
-  int chunk;         // chunk index when q_chunks > 1
-  long long row0;    // first matrix row of the tile
-};
-
-__device__ __forceinline__ TileInfo tile_info(const TcParams& P, int tile) {
-  TileInfo t;
-  if (P.tile_q0) {
-    t.qa = P.tile_q0[tile];
-    t.qb = P.tile_q0[tile + 1];
-    t.chunk = 0;
-  } else if (P.q_chunks == 1) {
-    t.qa = tile * P.q_per_tile;
-    t.qb = min(t.qa + P.q_per_tile, P.n_q);
-    t.chunk = 0;
-  } else {
-    t.qa = tile / P.q_chunks;
-    t.qb = t.qa + 1;
-    t.chunk = tile - t.qa * P.q_chunks;
-  }
-  long long r0;
-  int len;
-  seq_bounds(P.q, t.qa, r0, len, nullptr);
-  t.row0 = r0 + (long long)t.chunk * TILE_M;
-  return t;
+__device__ __forceinline__ int wait_posted(SharedCtl* ctl, int uc, int* status) {
+  if (ctl->units_posted > uc) return 1;
+  return wait_posted_slow(ctl, uc, status);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -248,69 +144,103 @@ __device__ __forceinline__ TileInfo tile_info(const TcParams& P, int tile) {
 //   GROUPED: unit = document, group = its query.  LIST: unit = pair, group = its query (from the table).
 // `doc` is the global document index (LIST: the pair).
 // ---------------------------------------------------------------------------------------------
-struct UnitWalk {
+struct UnitIter {
   int sb;               // super-block
-  int doc_lo, n_docs;   // its documents
-  long long u, u_end;   // what is left of this CTA's share of its units
+  int doc_lo, doc_hi;   // its documents
+  int left;             // units of this CTA's share of the super-block still to come, this one included
+  int grp, doc, in_grp;
 };
 
-// moves to the next super-block with units for this CTA, unless there are some left in this one
-__device__ __forceinline__ void walk_settle(const TcParams& P, int n_groups, UnitWalk& w) {
+__device__ __forceinline__ bool iter_enter(const TcParams& P, int n_groups, UnitIter& it) {
   const long long c = blockIdx.x, G = gridDim.x;
-  while (w.u >= w.u_end && w.sb < P.n_sb) {
+  while (it.sb < P.n_sb) {
     long long units;
     if (P.pairing == LIK_PAIR_CROSS) {
-      w.doc_lo = (int)min((long long)w.sb * P.sb_docs, (long long)P.n_d);
-      w.n_docs = (int)min((long long)P.sb_docs, (long long)(P.n_d - w.doc_lo));
-      units = (long long)n_groups * w.n_docs;
+      it.doc_lo = (int)min((long long)it.sb * P.sb_docs, (long long)P.n_d);
+      it.doc_hi = (int)min((long long)it.doc_lo + P.sb_docs, (long long)P.n_d);
+      units = (long long)n_groups * (it.doc_hi - it.doc_lo);
     } else {
-      w.doc_lo = 0;
-      w.n_docs = P.n_d;
+      it.doc_lo = 0;
+      it.doc_hi = P.n_d;
       units = P.n_flat;
     }
+    long long u, u_end;
     if (units < (1ll << 32) / 256) {  // (a 64-bit division is a hundred dependent instructions in front of the first load; grids have at most 256 CTAs)
-      w.u = (unsigned)units * (unsigned)c / (unsigned)G;
-      w.u_end = (unsigned)units * (unsigned)(c + 1) / (unsigned)G;
+      u = (unsigned)units * (unsigned)c / (unsigned)G;
+      u_end = (unsigned)units * (unsigned)(c + 1) / (unsigned)G;
     } else {
-      w.u = units * c / G;
-      w.u_end = units * (c + 1) / G;
+      u = units * c / G;
+      u_end = units * (c + 1) / G;
     }
-    ++w.sb;
+    if (u < u_end) {
+      it.left = (int)(u_end - u);
+      if (P.pairing == LIK_PAIR_CROSS) {
+        const int nd_b = it.doc_hi - it.doc_lo;
+        it.grp = u < (1ll << 32) ? (int)((unsigned)u / (unsigned)nd_b) : (int)(u / nd_b);
+        it.doc = it.doc_lo + (int)(u - (long long)it.grp * nd_b);
+        it.in_grp = 0;
+      } else if (P.pairing == LIK_PAIR_GROUPED) {
+        it.doc = (int)u;
+        it.grp = it.doc / P.group;
+        it.in_grp = it.doc - it.grp * P.group;
+      } else {
+        it.doc = (int)u;
+        it.grp = -1;  // comes from the table
+        it.in_grp = 0;
+      }
+      return true;
+    }
+    ++it.sb;
   }
+  return false;
+}
+__device__ __forceinline__ bool iter_begin(const TcParams& P, int n_groups, UnitIter& it) {
+  it.sb = 0;
+  return iter_enter(P, n_groups, it);
+}
+__device__ __forceinline__ bool iter_next(const TcParams& P, int n_groups, UnitIter& it) {
+  if (--it.left > 0) {
+    ++it.doc;
+    if (P.pairing == LIK_PAIR_CROSS) {
+      if (it.doc == it.doc_hi) {
+        it.doc = it.doc_lo;
+        ++it.grp;
+      }
+    } else if (P.pairing == LIK_PAIR_GROUPED) {
+      if (++it.in_grp == P.group) {
+        it.in_grp = 0;
+        ++it.grp;
+      }
+    }
+    return true;
+  }
+  ++it.sb;
+  return iter_enter(P, n_groups, it);
 }
 
-// A unit as the producer warp fetches it: the length words of 32 units are loaded at once, a lane each, a batch ahead of their use.
+// Length words of a unit's document, loaded one unit ahead of their use.
 struct UnitRaw {
-  int doc, grp, a, b;
+  int a, b, q;
 };
-__device__ __forceinline__ UnitRaw unit_fetch(const TcParams& P, const UnitWalk& w, long long u) {
-  UnitRaw r{0, 0, 0, 0};
-  if (P.pairing == LIK_PAIR_CROSS) {
-    r.grp = u < (1ll << 32) ? (int)((unsigned)u / (unsigned)w.n_docs) : (int)(u / w.n_docs);
-    r.doc = w.doc_lo + (int)(u - (long long)r.grp * w.n_docs);
-  } else {
-    r.doc = (int)u;
-    r.grp = P.pairing == LIK_PAIR_GROUPED ? r.doc / P.group : 0;
-  }
+__device__ __forceinline__ UnitRaw unit_fetch(const TcParams& P, int doc) {
+  UnitRaw r{0, 0, 0};
   if (P.pairing == LIK_PAIR_LIST) {
-    const int4 t = __ldg(P.list_tab + r.doc);
-    r.grp = t.x;
+    const int4 t = __ldg(P.list_tab + doc);
+    r.q = t.x;
     r.a = t.y;
     r.b = t.z;
   } else if (P.d.cu) {
-    r.a = P.d.cu[r.doc];
-    r.b = P.d.cu[r.doc + 1];
+    r.a = P.d.cu[doc];
+    r.b = P.d.cu[doc + 1];
   } else if (P.d.lens) {
-    r.a = P.d.lens[r.doc];
+    r.a = P.d.lens[doc];
   }
   return r;
 }
 // First row and column count of the fetched document; `masked` tells whether its mask has holes.
 // Lengths come from the caller-validated views, clamped to the padded extent.
-// (the tensor-core path takes fewer than 2^31 rows)
-__device__ __forceinline__ void unit_resolve(const TcParams& P, const UnitRaw& r, int& row, int& len, bool& masked) {
+__device__ __forceinline__ void unit_resolve(const TcParams& P, int doc, const UnitRaw& r, long long& row0, int& len, bool& masked) {
   masked = false;
-  long long row0;
   if (P.pairing == LIK_PAIR_LIST) {
     row0 = r.a;
     len = r.b;
@@ -320,7 +250,7 @@ __device__ __forceinline__ void unit_resolve(const TcParams& P, const UnitRaw& r
     len = b > a ? b - a : 0;
     if ((long long)a + len > P.d.n_rows) len = P.d.n_rows > a ? (int)(P.d.n_rows - a) : 0;
   } else {
-    row0 = (long long)r.doc * P.d.seq_stride;
+    row0 = (long long)doc * P.d.seq_stride;
     len = P.d.max_len;
     if (P.d.lens) {
       int l = r.a;
@@ -331,14 +261,13 @@ __device__ __forceinline__ void unit_resolve(const TcParams& P, const UnitRaw& r
       len = l < 0 ? 0 : (l > P.d.max_len ? P.d.max_len : l);
     }
   }
-  row = (int)row0;
 }
 
-// Sum of squares of one row of a stage whose second slab, if any, lies `slab_rows` rows behind the first (lane = row: eight consecutive rows of a swizzled slab lie in different banks).  The
+// Sum of squares of one row of a stage (lane = row: eight consecutive rows of a swizzled slab lie in different banks).  The
 // pieces of 16 bytes are summed and combined in the order of prep_kernel's butterfly, so that the norms of a row are the
 // same number wherever they are taken.
 template <typename T>
-__device__ __forceinline__ float stage_row_sum_sq(const unsigned char* row, int r, int slab_rows) {
+__device__ __forceinline__ float stage_row_sum_sq(const unsigned char* row, int r, bool two_slabs) {
   float half[2];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {  // pieces h, h + 2, h + 4, h + 6, each beside its partner eight further: their loads in flight together
@@ -348,7 +277,7 @@ __device__ __forceinline__ float stage_row_sum_sq(const unsigned char* row, int 
       const unsigned char* a = row + (((2 * i + h) ^ (r & 7)) << 4);
       x[i] = *reinterpret_cast<const uint4*>(a);
       y[i] = make_uint4(0, 0, 0, 0);
-      if (slab_rows) y[i] = *reinterpret_cast<const uint4*>(a + slab_rows * SLAB_BYTES_ROW);
+      if (two_slabs) y[i] = *reinterpret_cast<const uint4*>(a + TILE_N * SLAB_BYTES_ROW);
     }
     float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -364,72 +293,16 @@ __device__ __forceinline__ float stage_row_sum_sq(const unsigned char* row, int 
 }
 
 struct DocMaps {
-  CUtensorMap flat[N_BOXES];  // document boxes of 32, 64, 96 rows, one 128-byte slab wide
-  CUtensorMap deep[N_BOXES];  // the same with all slabs of the rows, slab behind slab (rows that fill their slabs)
+  CUtensorMap m[N_BOXES];  // document boxes of 32, 64, ... rows: one copy per K slab whatever the tile height
 };
 
 // Word the producer leaves beside every ring stage for the MMA issuer.
-constexpr uint32_t STAGE_COLS_MASK = 0x7Fu;    // rows of the stage that are multiplied: a multiple of 32
-constexpr int STAGE_LANE_SHIFT = 16;           // the lane whose accumulator(s) the piece feeds
-constexpr uint32_t STAGE_FIRST = 1u << 18;     // first stage of a query-tile group: take the tiles over first
+constexpr uint32_t STAGE_COLS_MASK = 0x1FFu;   // valid document rows in the stage
+constexpr uint32_t STAGE_ACC0 = 1u << 16;      // feed accumulator 0 / 1
+constexpr uint32_t STAGE_ACC1 = 1u << 17;
+constexpr uint32_t STAGE_FIRST = 1u << 18;     // first stage of a query-tile group: wait for the tiles
+constexpr uint32_t STAGE_LAST = 1u << 19;      // last stage of the group: hand the tiles back afterwards
 constexpr uint32_t STAGE_END = 1u << 20;       // no more work
-constexpr uint32_t STAGE_LONE = 1u << 21;      // the second accumulator has no query tile: it changes hands, nothing is multiplied into it
-constexpr uint32_t STAGE_WIDE = 1u << 22;      // the slabs lie a full stage apart instead of right behind each other
-
-// Monotone map float -> unsigned (larger float, larger key); 0 is below every float.
-__device__ __forceinline__ unsigned ordered_key(float f) {
-  const unsigned u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
-// Cut a full candidate list (TOPK_CAP entries, in arrival = ascending document order) back to its k best
-// and return the k-th best as an ordered key.  One warp; lane l holds entries l, l + 32, ...  The k-th
-// largest key is found by bisection on its bits (32 warp-wide counts); entries above it stay, and of the
-// entries equal to it the earliest ones (lowest document indices), so that exactly k remain, in order.
-__device__ __noinline__ unsigned topk_compact(float* keys, int* idx, int k, int lane) {
-  constexpr int PER = TOPK_CAP / 32;
-  unsigned uk[PER];
-  float fk[PER];
-  int id[PER];
-#pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    fk[j] = keys[j * 32 + lane];
-    id[j] = idx[j * 32 + lane];
-    uk[j] = ordered_key(fk[j]);
-  }
-  unsigned kth = 0;
-  for (int bit = 31; bit >= 0; --bit) {
-    const unsigned cand = kth | (1u << bit);
-    int c = 0;
-#pragma unroll
-    for (int j = 0; j < PER; ++j) c += uk[j] >= cand ? 1 : 0;
-    c = __reduce_add_sync(0xffffffffu, c);
-    if (c >= k) kth = cand;
-  }
-  int n_gt = 0;
-#pragma unroll
-  for (int j = 0; j < PER; ++j) n_gt += uk[j] > kth ? 1 : 0;
-  n_gt = __reduce_add_sync(0xffffffffu, n_gt);
-  const int need = k - n_gt;  // ties to keep (at least one)
-  const unsigned lt = (1u << lane) - 1u;
-  int out = 0, ties = 0;
-#pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    const bool eq = uk[j] == kth;
-    const unsigned m_eq = __ballot_sync(0xffffffffu, eq);
-    const bool keep = uk[j] > kth || (eq && ties + __popc(m_eq & lt) < need);
-    const unsigned m_keep = __ballot_sync(0xffffffffu, keep);
-    if (keep) {
-      const int pos = out + __popc(m_keep & lt);
-      keys[pos] = fk[j];
-      idx[pos] = id[j];
-    }
-    out += __popc(m_keep);
-    ties += __popc(m_eq);
-  }
-  __syncwarp();
-  return kth;
-}
 
 // WINNERS: 0 = scores only, 1 = winners saved, 2 = winners saved and every document takes the lazy winner scan (launched
 // for problems whose documents are long, so that the kernels for short documents carry no third copy of the tile loop)
@@ -437,18 +310,14 @@ template <bool FP8, int WINNERS, bool SCALED, bool PLAID>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ DocMaps d_maps, const TcParams P) {
   constexpr bool ARGMAX = WINNERS != 0;
-  // The last box of a document that is not a multiple of 32 tokens is moved back to end where the document ends: the
-  // columns it shares with the box before hold the same dot products twice, which no maximum minds, and no column has to
-  // be masked.  (Multipliers per column do not move along, and decoded rows have no boxes.)
-  constexpr bool SHIFT = !SCALED && !PLAID;
   extern __shared__ unsigned char smem_raw[];
   // operand tiles need 1024-byte alignment for the 128-byte swizzle
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int q_tile_bytes = P.n_slabs * TILE_M * SLAB_BYTES_ROW;
   const int d_stage_bytes = P.n_slabs * TILE_N * SLAB_BYTES_ROW;
-  unsigned char* q_smem = smem;                              // [mt][n_slabs][128 rows][128 B], on their way to tensor memory
-  unsigned char* d_smem = smem + P.mt * q_tile_bytes;        // [stages][n_slabs][rows][128 B]
-  float* sc_ring = reinterpret_cast<float*>(d_smem + (size_t)P.stages * d_stage_bytes);  // [lanes][sc_per][TILE_N] (kernels with multipliers)
+  unsigned char* q_smem = smem;                              // [2][n_slabs][128 rows][128 B]
+  unsigned char* d_smem = smem + 2 * q_tile_bytes;           // [stages][n_slabs][256 rows][128 B]
+  float* sc_ring = reinterpret_cast<float*>(d_smem + (size_t)P.stages * d_stage_bytes);  // [sc_slots][TILE_N] (kernels with multipliers)
   SharedCtl* ctl = reinterpret_cast<SharedCtl*>(d_smem + (size_t)P.stages * d_stage_bytes + (size_t)P.sc_slots * TILE_N * sizeof(float));
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -457,27 +326,25 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
   const bool topk = !ARGMAX && P.topk.cand_key != nullptr;  // the fused top-k never saves winners
 
   const bool norm_warps = SCALED && !FP8 && !PLAID && P.norm_eps > 0.f;  // (a member of every pipeline barrier then)
-  const int n_issuers = PLAID || norm_warps ? 1 : 2;
   if (tid == 0) {
     mbar_init(smem_u32(&ctl->q_full), 1);
-    mbar_init(smem_u32(&ctl->q_empty), (uint32_t)n_issuers);
-    for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&ctl->a_idle[i]), 1);
+    mbar_init(smem_u32(&ctl->q_empty), 1);
     for (int s = 0; s < P.stages; ++s) {
-      mbar_init(smem_u32(&ctl->d_full[s]), (uint32_t)P.d_full_count);
-      mbar_init(smem_u32(&ctl->d_empty[s]), (uint32_t)(norm_warps ? n_issuers + NORM_WARPS : n_issuers));
+      mbar_init(smem_u32(&ctl->d_full[s]), PLAID ? PLAID_WARPS : 1);  // the decoder warps, or TMA
+      mbar_init(smem_u32(&ctl->d_empty[s]), norm_warps ? 1 + NORM_WARPS : 1);
     }
-    for (int a = 0; a < SETS; ++a) {
+    for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&ctl->acc_full[a]), norm_warps ? 1 + NORM_WARPS : 1);
-      mbar_init(smem_u32(&ctl->acc_empty[a]), SET_WARPS);
-      mbar_init(smem_u32(&ctl->set_sync[a]), SET_WARPS);
+      mbar_init(smem_u32(&ctl->acc_empty[a]), GROUP_WARPS);
     }
     ctl->abort_flag = 0;
     ctl->wait_limit = WAIT_LIMIT_CYCLES;
-    for (int i = 0; i < SETS; ++i) ctl->units_posted[i] = 0;
+    ctl->units_posted = 0;
+    ctl->units_total = 0x7fffffff;
     fence_barrier_init();
     prefetch_tmap(&q_map);
     if (!PLAID)
-      for (int i = 0; i < N_BOXES; ++i) prefetch_tmap(P.d_deep ? &d_maps.deep[i] : &d_maps.flat[i]);
+      for (int i = 0; i < N_BOXES; ++i) prefetch_tmap(&d_maps.m[i]);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(&ctl->tmem_base), 512);
@@ -494,134 +361,102 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
   // greedy-packed query tiles are counted on the device (the count sits in front of the table)
   const int n_tiles = P.tile_q0 ? P.tile_q0[-1] : P.n_tiles;
   const int n_groups = (n_tiles + P.mt - 1) / P.mt;
-  const int lanes = SETS / P.mt;  // documents in flight
 
-  const bool producer_warp = warp == 0 || (PLAID && warp >= 2 + SETS * SET_WARPS);
+  const bool producer_warp = warp == 0 || (PLAID && warp >= 2 + 2 * GROUP_WARPS);
   if (producer_warp) {
     // =========================== producer ===========================
-    // One warp walks the units, loads the query tiles and the document pieces with TMA and leaves the stage words and the
-    // unit rings.  It runs on warp-uniform values and one elected lane issues, as in the issuer below: TMA instructions, too,
-    // take their operands from uniform registers.  In the PLAID kernels three warps walk the units in step; each decodes its
-    // share of every piece's tokens into the swizzled operand layout (generic-proxy stores, fenced for the tensor core's
-    // reads), and arrives on the stage barrier; the elected lane of warp 0 still does everything else.
-    {
-      const int pw = warp == 0 ? 0 : warp - (2 + SETS * SET_WARPS) + 1;  // decoder warp number 0..2
-      const bool elect = warp == 0 && elect_one();
+    // TMA kernels: one thread (warp 0, lane 0) walks the units, loads the query tiles and the document
+    // stages with TMA and leaves the stage words and the unit ring.  PLAID kernels: three whole warps walk
+    // the units in step; each decodes its share of every stage's tokens into the swizzled operand layout
+    // (generic-proxy stores, fenced for the tensor core's reads), and arrives on the stage barrier; the
+    // elected thread of warp 0 still does everything else.
+    const bool elect = warp == 0 && lane == 0;
+    if (PLAID || lane == 0) {
+      const int pw = warp == 0 ? 0 : warp - (2 + 2 * GROUP_WARPS) + 1;  // decoder warp number 0..2
       int cur_grp = -1;
       uint32_t n_qload = 0, st = 0, ph = 0, n_dload = 0;
+      int sc_cnt[2] = {0, 0};  // next slot in either accumulator's multiplier ring
+      long long uc = 0;
       const int x_per_slab = SLAB_BYTES_ROW / P.elt_bytes;
       bool ok = true;
-      uint32_t lone = 0, first = 0;
-      // the documents in flight, one per lane: what is left of each
-      int l_len[SETS], l_c0[SETS], l_uc[SETS], l_sc[SETS], l_row[SETS];
-#pragma unroll
-      for (int l = 0; l < SETS; ++l) {
-        l_len[l] = -1;  // none
-        l_c0[l] = l_uc[l] = l_sc[l] = l_row[l] = 0;
+      int tiles_here = 0;
+      // the iterator stands one unit ahead: that unit's length words are in flight while this one is produced
+      UnitIter it;
+      bool have = iter_begin(P, n_groups, it);
+      int nx_grp = 0, nx_doc = 0;
+      UnitRaw nx_raw{0, 0, 0};
+      if (have) {
+        nx_grp = it.grp;
+        nx_doc = it.doc;
+        nx_raw = unit_fetch(P, nx_doc);
       }
-      int open = 0;  // lanes with a document
-      // 32 units at a time, a lane of the warp each: a batch that is dealt out, and one whose length words are on their way
-      UnitWalk walk{0, 0, 0, 0, 0};
-      walk_settle(P, n_groups, walk);
-      UnitRaw raw{0, 0, 0, 0};
-      int n_raw = 0, n_unit = 0, at_unit = 0;
-      int u_doc = 0, u_grp = 0, u_row = 0, u_len = 0;  // this lane's unit; u_len carries LEN_FLAG_MASKED
-      auto fetch_batch = [&]() {
-        n_raw = (int)min(32ll, walk.u_end - walk.u);
-        if (n_raw > 0) {
-          if (lane < n_raw) raw = unit_fetch(P, walk, walk.u + lane);
-          walk.u += n_raw;
-          walk_settle(P, n_groups, walk);
-        }
-      };
-      bool have;
-      int nx_doc = 0, nx_grp = 0, nx_row = 0, nx_len = 0;
-      auto pull = [&]() {
-        if (at_unit == n_unit) {
-          bool masked = false;
-          u_doc = raw.doc;
-          u_grp = raw.grp;
-          unit_resolve(P, raw, u_row, u_len, masked);
-          u_len = (u_len & UNIT_LEN_MASK) | (masked ? LEN_FLAG_MASKED : 0);
-          n_unit = n_raw > 0 ? n_raw : 0;
-          at_unit = 0;
-          fetch_batch();
-        }
-        have = n_unit > 0;
+      while (have && ok) {
+        const int doc = nx_doc;
+        const int grp = list ? nx_raw.q : nx_grp;
+        long long drow0;
+        int dlen;
+        bool dmasked;
+        unit_resolve(P, doc, nx_raw, drow0, dlen, dmasked);
+        have = iter_next(P, n_groups, it);
+        int next_grp = -1;
         if (have) {
-          nx_doc = __shfl_sync(0xffffffffu, u_doc, at_unit);
-          nx_grp = __shfl_sync(0xffffffffu, u_grp, at_unit);
-          nx_row = __shfl_sync(0xffffffffu, u_row, at_unit);
-          nx_len = __shfl_sync(0xffffffffu, u_len, at_unit);
-          ++at_unit;
+          nx_grp = it.grp;
+          nx_doc = it.doc;
+          nx_raw = unit_fetch(P, nx_doc);
+          next_grp = list ? nx_raw.q : nx_grp;
         }
-      };
-      fetch_batch();
-      pull();
-      while (ok && (have || open)) {
-#pragma unroll
-        for (int l = 0; l < SETS; ++l) {
-          if (l >= lanes || !ok) continue;
-          if (l_len[l] < 0) {
-            // the lane takes the next unit, unless that belongs to another tile group and this one is not finished yet
-            if (!have || (nx_grp != cur_grp && open)) continue;
-            const int doc = nx_doc, grp = nx_grp, drow0 = nx_row, dlen = nx_len & UNIT_LEN_MASK;
-            const int dmasked = nx_len & LEN_FLAG_MASKED;
-            pull();
-            if (grp != cur_grp) {
-              cur_grp = grp;
-              first = STAGE_FIRST;
-              const int t0 = grp * P.mt, t1 = min(t0 + P.mt, n_tiles);
-              lone = P.mt == 2 && t1 - t0 < 2 ? STAGE_LONE : 0u;
-              if (warp == 0) {
-                // wait until the issuers have copied the previous query tiles to tensor memory
-                ok = wait_bar_warp(&ctl->q_empty, (n_qload & 1) ^ 1, ctl, P.status);
-                if (ok && elect) {
-                  mbar_arrive_expect_tx(smem_u32(&ctl->q_full), (uint32_t)((t1 - t0) * q_tile_bytes));
-                  for (int t = t0; t < t1; ++t) {
-                    TileInfo ti = tile_info(P, t);
-                    for (int sl = 0; sl < P.n_slabs; ++sl)
-                      tma_load_2d(smem_u32(q_smem + (t - t0) * q_tile_bytes + sl * TILE_M * SLAB_BYTES_ROW), &q_map, sl * x_per_slab, (int)ti.row0,
-                                  smem_u32(&ctl->q_full));
-                  }
-                }
-                __syncwarp();
-              }
-              ++n_qload;
-              if (!ok) continue;
-            }
-            // publish the unit for the lane's epilogue sets; an empty document still sends one (empty) piece so that every
-            // unit passes through the same hand-shakes
-            if (elect) {
-              ctl->unit_info[l][l_uc[l] & (UNIT_RING - 1)] = make_int4(dlen | (SCALED ? l_sc[l] << UNIT_SLOT_SHIFT : 0) | dmasked, drow0, grp, doc);
-              if (SCALED) {  // (the others learn of it from a full accumulator)
-                __threadfence_block();
-                ctl->units_posted[l] = l_uc[l] + 1;
+        const bool last_unit_of_grp = next_grp != grp;
+        uint32_t first = 0;
+        if (grp != cur_grp) {
+          cur_grp = grp;
+          first = STAGE_FIRST;
+          const int t0 = grp * P.mt, t1 = min(t0 + P.mt, n_tiles);
+          tiles_here = t1 - t0;
+          if (elect) {
+            // wait until the MMAs that read the previous query tiles are done
+            ok = wait_bar(&ctl->q_empty, (n_qload & 1) ^ 1, ctl, P.status);
+            if (ok) {
+              mbar_arrive_expect_tx(smem_u32(&ctl->q_full), (uint32_t)((t1 - t0) * q_tile_bytes));
+              for (int t = t0; t < t1; ++t) {
+                TileInfo ti = tile_info(P, t);
+                for (int sl = 0; sl < P.n_slabs; ++sl)
+                  tma_load_2d(smem_u32(q_smem + (t - t0) * q_tile_bytes + sl * TILE_M * SLAB_BYTES_ROW), &q_map, sl * x_per_slab,
+                              (int)ti.row0, smem_u32(&ctl->q_full));
               }
             }
-            ++l_uc[l];
-            ++open;
-            l_len[l] = dlen;
-            l_c0[l] = 0;
-            l_row[l] = drow0;
           }
-          // the lane's next piece
-          const int c0 = l_c0[l], dlen = l_len[l], drow0 = l_row[l];
-          const int ncols = min(TILE_N, dlen - c0);
-          const bool ends = c0 + TILE_N >= dlen;
-          const int rows = __shfl_sync(0xffffffffu, (ncols + BOX_ROWS - 1) & ~(BOX_ROWS - 1), 0);
-          // A short document that is no multiple of 32 tokens takes two boxes, the second moved back to end where the document
-          // ends; a longer one's last piece is moved back as a whole.
-          const bool split = SHIFT && dlen < rows && dlen > BOX_ROWS;
-          ok = wait_bar_warp(&ctl->d_empty[st], ph ^ 1, ctl, P.status);
-          if (!ok) continue;
+          ++n_qload;
+          if (PLAID && warp == 0) ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+          if (!ok) break;
+        }
+        // which accumulators this unit feeds: both resident tiles, or (one tile) alternating with the unit count
+        const uint32_t acc_bits = P.mt == 2 ? (tiles_here == 2 ? (STAGE_ACC0 | STAGE_ACC1) : STAGE_ACC0)
+                                            : ((uc & 1) ? STAGE_ACC1 : STAGE_ACC0);
+        const int sc_ring_id = (!SCALED || P.mt == 2 || !(uc & 1)) ? 0 : 1;  // the multiplier ring of the accumulator(s) this unit feeds
+        // publish the unit for the epilogue groups, then its stages; an empty document still sends one
+        // (empty) stage so that every unit passes through the same hand-shakes
+        if (elect) {
+          ctl->unit_info[uc & (UNIT_RING - 1)] = make_int4(
+              (dlen & UNIT_LEN_MASK) | (SCALED ? (sc_ring_id * P.sc_per + sc_cnt[sc_ring_id]) << UNIT_SLOT_SHIFT : 0) |
+                  (dmasked ? LEN_FLAG_MASKED : 0),
+              (int)drow0, grp, doc);
+          __threadfence_block();
+          ctl->units_posted = (int)uc + 1;
+        }
+        int c0 = 0;
+        do {
+          const int ncols = max(0, min(TILE_N, dlen - c0));
+          ok = wait_bar(&ctl->d_empty[st], ph ^ 1, ctl, P.status);
+          if (!ok) break;
           const uint32_t full = smem_u32(&ctl->d_full[st]);
-          if (ends) --open;
-          if (elect)
-            ctl->stage_info[st] = (uint32_t)rows | ((uint32_t)l << STAGE_LANE_SHIFT) | first | lone | (split || PLAID ? STAGE_WIDE : 0u);
-          first = 0;
+          if (elect) {
+            uint32_t info = (uint32_t)ncols | acc_bits;
+            if (c0 == 0) info |= first;
+            if (last_unit_of_grp && c0 + TILE_N >= dlen) info |= STAGE_LAST;
+            ctl->stage_info[st] = info;
+          }
           if (PLAID) {
-            // the piece's tokens in six equal runs, one per half-warp of the three decoder warps
+            // the stage's tokens in six equal runs, one per half-warp of the three decoder warps
             const int hl = lane & 15;
             const int hw6 = pw * 2 + (lane >> 4);
             const int per = (ncols + 2 * PLAID_WARPS - 1) / (2 * PLAID_WARPS);
@@ -640,54 +475,43 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
             __syncwarp();
             if (lane == 0) mbar_arrive(full);
           } else {
-            const int row = __shfl_sync(0xffffffffu, drow0 + (SHIFT ? max(min(c0, dlen - rows), 0) : c0), 0);
-            // the piece's multipliers ride on the same barrier: whole groups of four floats, never past the array's end
-            uint32_t sc_bytes = 0;
-            if (SCALED && P.col_src && rows > 0) sc_bytes = (uint32_t)min((long long)((ncols + 3) & ~3), P.d.n_rows - row) * 4u;
-            if (elect) {
-              const uint32_t dst = smem_u32(d_smem) + st * (uint32_t)d_stage_bytes;
-              if (rows > 0) {
-                mbar_arrive_expect_tx(full, (uint32_t)(rows * SLAB_BYTES_ROW * P.n_slabs) + sc_bytes);
-                const int box = rows / BOX_ROWS - 1;
-                if (!split && P.d_deep) {
-                  tma_load_3d(dst, &d_maps.deep[box], 0, row, 0, full);
-                } else {
-                  const uint32_t slab = (uint32_t)((split ? TILE_N : rows) * SLAB_BYTES_ROW);
-                  for (int sl = 0; sl < P.n_slabs; ++sl) {
-                    tma_load_2d(dst + sl * slab, &d_maps.flat[split ? box - 1 : box], sl * x_per_slab, row, full);
-                    if (split) tma_load_2d(dst + sl * slab + box * BOX_ROWS * SLAB_BYTES_ROW, &d_maps.flat[0], sl * x_per_slab, row + dlen - BOX_ROWS, full);
-                  }
-                }
-                if (sc_bytes) bulk_load_1d(smem_u32(sc_ring + (l * P.sc_per + l_sc[l]) * TILE_N), P.col_src + row, sc_bytes, full);
-              } else {
-                mbar_arrive(full);
+            const int boxes = (ncols + BOX_ROWS - 1) / BOX_ROWS;
+            if (boxes > 0) {
+              // the tile's multipliers ride on the same barrier: whole groups of four floats, never past the array's end
+              uint32_t sc_bytes = 0;
+              if (SCALED && P.col_src) {
+                const long long r = drow0 + c0;
+                sc_bytes = (uint32_t)min((long long)((ncols + 3) & ~3), P.d.n_rows - r) * 4u;
               }
+              mbar_arrive_expect_tx(full, (uint32_t)(boxes * BOX_ROWS * SLAB_BYTES_ROW * P.n_slabs) + sc_bytes);
+              const CUtensorMap* map = &d_maps.m[boxes - 1];
+              for (int sl = 0; sl < P.n_slabs; ++sl)
+                tma_load_2d(smem_u32(d_smem + (size_t)st * d_stage_bytes + sl * TILE_N * SLAB_BYTES_ROW), map, sl * x_per_slab,
+                            (int)(drow0 + c0), full);
+              if (sc_bytes)
+                bulk_load_1d(smem_u32(sc_ring + (sc_ring_id * P.sc_per + sc_cnt[sc_ring_id]) * TILE_N), P.col_src + drow0 + c0, sc_bytes, full);
+            } else {
+              mbar_arrive(full);
             }
-            __syncwarp();
           }
           ++n_dload;
           if (++st == (uint32_t)P.stages) { st = 0; ph ^= 1; }
-          if (SCALED && ++l_sc[l] >= P.sc_per) l_sc[l] = 0;
-          l_c0[l] = c0 + TILE_N;
-          if (ends) l_len[l] = -1;
-        }
+          if (SCALED && ++sc_cnt[sc_ring_id] >= P.sc_per) sc_cnt[sc_ring_id] = 0;
+          c0 += TILE_N;
+        } while (c0 < dlen);
+        ++uc;
+      }
+      if (ok && elect) {
+        // tell the epilogue groups how many units there were
+        __threadfence_block();
+        ctl->units_total = (int)uc;
       }
       if (ok) {
-        // tell the epilogue sets and the issuer that the stream has ended
-        ok = wait_bar_warp(&ctl->d_empty[st], ph ^ 1, ctl, P.status);
+        // tell the issuer that the stream has ended
+        ok = wait_bar(&ctl->d_empty[st], ph ^ 1, ctl, P.status);
         if (ok) {
-          if (elect) {
-#pragma unroll
-            for (int l = 0; l < SETS; ++l) {
-              if (l >= lanes) continue;
-              ctl->unit_info[l][l_uc[l] & (UNIT_RING - 1)] = make_int4(UNIT_END, 0, 0, 0);
-              __threadfence_block();
-              ctl->units_posted[l] = l_uc[l] + 1;
-            }
-            ctl->stage_info[st] = STAGE_END;
-          }
-          __syncwarp();
-          if (PLAID ? lane == 0 : elect) mbar_arrive(smem_u32(&ctl->d_full[st]));
+          if (elect) ctl->stage_info[st] = STAGE_END;
+          if (lane == 0) mbar_arrive(smem_u32(&ctl->d_full[st]));
         }
       }
       if (!ok && elect) {
@@ -708,93 +532,59 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
         }
       }
     }
-  } else if (warp == 1 || (warp == 2 + SETS * SET_WARPS && n_issuers == 2)) {
-    // =========================== MMA issuers ===========================
-    // Driven by the stage words alone.  A whole warp runs the loop on warp-uniform values (the stage word is broadcast from
+  } else if (warp == 1) {
+    // =========================== MMA issuer ===========================
+    // Driven by the stage words alone.  The whole warp runs the loop on warp-uniform values (the stage word is broadcast from
     // lane 0, which also tells the compiler that it is uniform) and one elected lane issues: tcgen05.mma takes its
     // descriptors from uniform registers, and with the loop under `lane == 0` every MMA paid about 100 cycles for moving
     // them there, whatever its width.
-    // Two warps share the work where a warp is free for it: one feeds the even accumulators, the other the odd ones.  The
-    // tensor pipe holds about four MMAs ahead, some 250 cycles, and the waits and words of a piece take a warp longer than
-    // that; each of the two has the other's MMAs to hide behind.
-    const uint32_t me = warp == 1 ? 0u : 1u;
-    uint32_t st = 0, ph = 0, n_q = 0, acc_ph = 0;  // acc_ph: one phase bit per accumulator
+    uint32_t st = 0, ph = 0, q_ph = 0, acc_ph = 0;  // acc_ph: one phase bit per accumulator
     bool ok = true;
     const bool issue = elect_one();
     const uint32_t desc_hi = (uint32_t)(smem_desc_sw128(0) >> 32);
     const uint32_t a_desc0 = (uint32_t)smem_desc_sw128(smem_u32(q_smem));
     const uint32_t b_desc0 = (uint32_t)smem_desc_sw128(smem_u32(d_smem));
     const uint32_t stage_desc = (uint32_t)(d_stage_bytes >> 4);
-    const uint32_t q_desc = (uint32_t)(q_tile_bytes >> 4);
+    const uint32_t a_tile1 = P.mt == 2 ? (uint32_t)(q_tile_bytes >> 4) : 0u;  // descriptor offset of the second resident tile
     const uint32_t idesc0 = instr_desc(P.ab_format, 0);
     const int k_steps = P.k_steps;
-    const uint32_t mt = (uint32_t)P.mt;
     constexpr uint32_t A_SLAB = (TILE_M * SLAB_BYTES_ROW) >> 4, B_SLAB = (TILE_N * SLAB_BYTES_ROW) >> 4;
-    // `step` visits this warp's share of the accumulators [a0, a0 + n)
-    const uint32_t step = (uint32_t)n_issuers;
     while (ok) {
       ok = wait_bar_warp(&ctl->d_full[st], ph, ctl, P.status);
       if (!ok) break;
       const uint32_t info = __shfl_sync(0xffffffffu, ctl->stage_info[st], 0);
-      if (info & STAGE_END) {
-        // the accumulators change hands once more, empty: the sets find the end of the stream in their unit ring
-        for (uint32_t a = me; a < SETS; a += step) {
-          if (ok) ok = wait_bar_warp(&ctl->acc_empty[a], ((acc_ph >> a) & 1u) ^ 1u, ctl, P.status);
-          if (ok && issue) tc_commit(smem_u32(&ctl->acc_full[a]));
-          __syncwarp();
-        }
-        break;
-      }
+      if (info & STAGE_END) break;
       if (info & STAGE_FIRST) {
-        // New query tiles: this warp copies the ones it multiplies with to its place(s) in tensor memory, once its MMAs on the
-        // old ones are done.  (A copy and an MMA that follows it run in order.)  With one tile and two issuers either has its own.
-        ok = wait_bar_warp(&ctl->q_full, n_q & 1u, ctl, P.status);
-        if (ok && n_q) {
-          if (issue) tc_commit(smem_u32(&ctl->a_idle[me]));
-          __syncwarp();
-          ok = wait_bar_warp(&ctl->a_idle[me], (n_q - 1) & 1u, ctl, P.status);
-        }
+        ok = wait_bar_warp(&ctl->q_full, q_ph, ctl, P.status);
         if (!ok) break;
-        ++n_q;
-        tc_fence_after();
-        if (issue) {
-          for (uint32_t t = 0; t < mt; ++t) {
-            if (mt == 2 && step == 2 && t != me) continue;
-            const uint32_t to = tmem_base + A_COL0 + (mt == 2 ? t : me) * A_COLS;
-            for (int k = 0; k < k_steps; ++k) tc_copy_128x256b(to + 8 * k, a_desc0 + t * q_desc + (uint32_t)((k & 3) * 2) + (k >> 2) * A_SLAB, desc_hi);
-          }
-          tc_commit(smem_u32(&ctl->q_empty));
-        }
-        __syncwarp();
+        q_ph ^= 1;
       }
-      const uint32_t rows = info & STAGE_COLS_MASK;
-      const uint32_t idesc = idesc0 | (rows << 14);  // N / 8 in bits 17..22
+      const uint32_t ncols = info & STAGE_COLS_MASK;
+      const uint32_t idesc = idesc0 | (((ncols + 15) >> 4) << 18);  // N / 8 in bits 17..22
       const uint32_t b_stage = b_desc0 + st * stage_desc;
-      const uint32_t b_slab = info & STAGE_WIDE ? B_SLAB : rows * (SLAB_BYTES_ROW >> 4);
-      const uint32_t set0 = ((info >> STAGE_LANE_SHIFT) & (SETS - 1)) * mt;
-      uint32_t a = set0;
-      if (step == 2 && ((a ^ me) & 1u)) ++a;
-      bool mine = false;
-      for (; a < set0 + mt; a += step) {
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        if (!ok || !(info & (STAGE_ACC0 << a))) continue;
         ok = wait_bar_warp(&ctl->acc_empty[a], ((acc_ph >> a) & 1u) ^ 1u, ctl, P.status);
-        if (!ok) break;
+        if (!ok) continue;
         acc_ph ^= 1u << a;
-        mine = true;
-        const uint32_t t = a - set0;
         tc_fence_after();
         if (issue) {
-          if (rows && !(t == 1 && (info & STAGE_LONE))) {  // (the accumulator always changes hands, so that both sides keep their phase)
-            const uint32_t d_tmem = tmem_base + a * ACC_COLS;
-            const uint32_t a_tmem = tmem_base + A_COL0 + (mt == 2 ? t : me) * A_COLS;
+          if (ncols) {  // (an empty document: the accumulator still changes hands so that both sides keep their phase)
+            const uint32_t d_tmem = tmem_base + (uint32_t)(a * ACC_COLS);
+            const uint32_t a_desc = a_desc0 + (a ? a_tile1 : 0u);
             // descriptors differ only in the start address, in units of 16 bytes
             if (k_steps == 8) {  // the common width (128 two-byte or 256 one-byte elements): straight-line issue
 #pragma unroll
               for (int k = 0; k < 8; ++k)
-                tc_mma_ts<FP8>(d_tmem, a_tmem + 8 * k, b_stage + (uint32_t)((k & 3) * 2) + (k >> 2) * b_slab, desc_hi, idesc, k ? 1u : 0u);
+                tc_mma<FP8>(d_tmem, a_desc + (uint32_t)((k & 3) * 2) + (k >> 2) * A_SLAB, b_stage + (uint32_t)((k & 3) * 2) + (k >> 2) * B_SLAB, desc_hi,
+                            idesc, k ? 1u : 0u);
             } else {
 #pragma unroll
               for (int k = 0; k < 8; ++k)
-                if (k < k_steps) tc_mma_ts<FP8>(d_tmem, a_tmem + 8 * k, b_stage + (uint32_t)((k & 3) * 2) + (k >> 2) * b_slab, desc_hi, idesc, k ? 1u : 0u);
+                if (k < k_steps)
+                  tc_mma<FP8>(d_tmem, a_desc + (uint32_t)((k & 3) * 2) + (k >> 2) * A_SLAB, b_stage + (uint32_t)((k & 3) * 2) + (k >> 2) * B_SLAB,
+                              desc_hi, idesc, k ? 1u : 0u);
             }
           }
           tc_commit(smem_u32(&ctl->acc_full[a]));
@@ -803,31 +593,30 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
       }
       if (!ok) break;
       if (issue) {
-        if (mine) tc_commit(smem_u32(&ctl->d_empty[st]));  // ring slot reusable once these MMAs retire
-        else mbar_arrive(smem_u32(&ctl->d_empty[st]));
+        tc_commit(smem_u32(&ctl->d_empty[st]));                     // ring slot reusable once these MMAs retire
+        if (info & STAGE_LAST) tc_commit(smem_u32(&ctl->q_empty));  // and so are the query tiles
       }
       __syncwarp();
       if (++st == (uint32_t)P.stages) { st = 0; ph ^= 1; }
     }
-  } else if (warp < 2 + SETS * SET_WARPS) {
-    // =========================== epilogue sets ===========================
-    // Set s (four warps) drains accumulator s: with two resident query tiles, tile s & 1 of lane s >> 1; with one, lane s.
-    // A warp owns 32 rows of a document from its first column to its score.  It waits for its accumulator by itself and gives
-    // it back by itself; the warps of a set meet only where the query tile changes, where columns are staged by all of them
-    // and where a query's rows lie in several warps.  All of these waits are bounded: a warp that gives up leaves the
-    // loop, and the others' waits find the abort flag.
+  } else if (warp < 2 + 2 * GROUP_WARPS) {
+    // =========================== epilogue groups ===========================
+    // Group g (eight warps) drains accumulator g.  Its two halves split the 32-column chunks of a tile
+    // between them (even chunks / odd chunks); half 1 hands its per-row result to half 0, which sums
+    // the rows of every query and writes the score.  (group, document) advance locally; a document's
+    // length and first row come from the producer's unit ring.
     const int e = warp - 2;
-    const int set = e >> 2;
+    const int wg = e >> 3;                   // accumulator / epilogue group
+    const int sub = (e >> 2) & 1;            // half of the group
     const int quad = warp & 3;               // TMEM lane quadrant this warp may read
-    const int wq = e & 3;                    // warp index inside the set
+    const int wq = e & 3;                    // warp index inside the half
     const int row = quad * 32 + lane;        // accumulator row == query token slot in the tile
-    const int et = wq * 32 + lane;           // thread index inside the set (0..127)
-    const int ln = P.mt == 2 ? set >> 1 : set;
-    const int my_tile = P.mt == 2 ? set & 1 : 0;
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(set * ACC_COLS);
-    const uint32_t acc_empty_bar = smem_u32(&ctl->acc_empty[set]);
+    const int et = wq * 32 + lane;           // thread index inside the half (0..127)
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(wg * ACC_COLS);
+    const uint32_t acc_empty_bar = smem_u32(&ctl->acc_empty[wg]);
     int cur_grp = -1;
-    uint32_t n_acc = 0, n_emit = 0, n_sync = 0, n_col = 0;
+    uint32_t n_acc = 0, n_emit = 0, n_doc = 0;
+    int uc = 0;
     bool ok = true;
     // per-row / per-warp state for the resident query tile
     bool have_tile = false, warp_rows = false, in_seg = false, row_ok = false, aligned = false;
@@ -835,15 +624,32 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
     int tile_id = 0;
     long long arg_off = -1;   // ARGMAX: offset of this row's slot for document 0 (-1: row stores nothing)
     long long warp_out = -1;  // aligned tiles: offset of this warp's query score for document 0
-    int my_list = -1;         // top-k: the list whose state thread `et` loaded into shared memory
+    int my_list = -1;         // top-k: the list whose state thread `et` (half 0) loaded into shared memory
     int warp_seg = -1;        // aligned tiles: the query (segment) of this warp's rows
-#define LIK_SET_SYNC() warps_sync(&ctl->set_sync[set], n_sync, lane, ctl, P.status)
-#define LIK_WAIT_ACC() wait_bar_warp(&ctl->acc_full[set], n_acc & 1, ctl, P.status)
+    // Rendezvous of the whole group / of half 0 on hardware named barriers: a waiting warp issues
+    // nothing.  Nobody waits on anything else between two of them, so every warp of the group always
+    // arrives; the only bounded waits of a group (for a unit, for the accumulator) are done by its first warp,
+    // which tells the others whether to go on through the rendezvous itself: a barrier that counts the
+    // threads arriving with a true predicate (0: go on, 1: the wait gave up, 2: the stream has ended).
+    const bool leader = (e & 7) == 0;
+#define LIK_GRP_SYNC_COUNT(pred_, count_out_)                                                                        \
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %3, 0;\n\tbar.red.popc.u32 %0, %1, %2, q;\n\t}"              \
+               : "=r"(count_out_) : "r"(1 + wg), "r"(2 * EPI_THREADS), "r"((int)(pred_)) : "memory")
+#define LIK_GRP_SYNC() asm volatile("bar.sync %0, %1;" ::"r"(1 + wg), "r"(2 * EPI_THREADS) : "memory")
+#define LIK_SUB_SYNC() asm volatile("bar.sync %0, %1;" ::"r"(3 + wg), "r"(EPI_THREADS) : "memory")
+#define LIK_GROUP_WAIT_ACC()                                                         \
+  do {                                                                               \
+    bool gave_up_ = false;                                                           \
+    if (leader) gave_up_ = !wait_bar(&ctl->acc_full[wg], n_acc & 1, ctl, P.status);  \
+    int n_;                                                                          \
+    LIK_GRP_SYNC_COUNT(gave_up_ && lane == 0, n_);                                   \
+    ok = n_ == 0;                                                                    \
+  } while (0)
     // top-k: write the state of the lists this thread loaded back to their headers
 #define LIK_TOPK_STORE_BACK()                                                                          \
   do {                                                                                                 \
-    if (topk && my_list >= 0) {                                                                        \
-      P.topk.hdr[my_list] = make_int2(ctl->seg_cnt[set][et], (int)ctl->seg_thr[set][et]);              \
+    if (topk && sub == 0 && my_list >= 0) {                                                            \
+      P.topk.hdr[my_list] = make_int2(ctl->seg_cnt[wg][et], (int)ctl->seg_thr[wg][et]);                \
       my_list = -1;                                                                                    \
     }                                                                                                  \
   } while (0)
@@ -855,14 +661,14 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
     } else {                                                                                           \
       const float key_ = (P.topk.largest ? (value_) : -(value_)) + 0.f;                                \
       const unsigned ukey_ = ordered_key(key_);                                                        \
-      if (ukey_ > ctl->seg_thr[set][sg_]) {                                                            \
-        int cnt_ = ctl->seg_cnt[set][sg_];                                                             \
-        if ((unsigned)cnt_ >= (unsigned)TOPK_CAP || (unsigned)ctl->seg_list[set][sg_] >= (unsigned)P.topk.n_lists) {  \
+      if (ukey_ > ctl->seg_thr[wg][sg_]) {                                                             \
+        int cnt_ = ctl->seg_cnt[wg][sg_];                                                              \
+        if ((unsigned)cnt_ >= (unsigned)TOPK_CAP || (unsigned)ctl->seg_list[wg][sg_] >= (unsigned)P.topk.n_lists) {  \
           if (lane == 0 && P.status) atomicOr(P.status, LIK_DEV_INTERNAL);                             \
           break;                                                                                       \
         }                                                                                              \
-        float* keys_ = P.topk.cand_key + (long long)ctl->seg_list[set][sg_] * TOPK_CAP;                \
-        int* idx_ = P.topk.cand_idx + (long long)ctl->seg_list[set][sg_] * TOPK_CAP;                   \
+        float* keys_ = P.topk.cand_key + (long long)ctl->seg_list[wg][sg_] * TOPK_CAP;                 \
+        int* idx_ = P.topk.cand_idx + (long long)ctl->seg_list[wg][sg_] * TOPK_CAP;                    \
         if (lane == 0) {                                                                               \
           keys_[cnt_] = key_;                                                                          \
           idx_[cnt_] = doc + P.topk.doc_base;                                                          \
@@ -872,50 +678,66 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
         if (cnt_ == TOPK_CAP) {                                                                        \
           const unsigned thr_ = topk_compact(keys_, idx_, P.topk.k, lane);                             \
           cnt_ = P.topk.k;                                                                             \
-          if (lane == 0) ctl->seg_thr[set][sg_] = thr_;                                                \
+          if (lane == 0) ctl->seg_thr[wg][sg_] = thr_;                                                 \
         }                                                                                              \
-        if (lane == 0) ctl->seg_cnt[set][sg_] = cnt_;                                                  \
+        if (lane == 0) ctl->seg_cnt[wg][sg_] = cnt_;                                                   \
         __syncwarp();                                                                                  \
       }                                                                                                \
     }                                                                                                  \
   } while (0)
 
     const bool cross = P.pairing == LIK_PAIR_CROSS;
-    const bool bulk = SCALED && P.sc_slots != 0;  // the multipliers of a piece arrive with it, or are made from it
-    // multipliers that the set stages itself are fetched while the MMAs run, so the unit has to be known before the accumulator is full
-    const bool early = SCALED && !bulk;
-    for (int uc = 0;; ++uc) {
-      // The unit (tile group, document, length, first row) comes from the lane's ring, where it stands before its first
-      // piece is announced to the issuer, so that a full accumulator says that it is there.
-      ok = early ? wait_posted(ctl, ln, uc, P.status) : LIK_WAIT_ACC();
-      if (!ok) break;
-      const int4 uinfo = ctl->unit_info[ln][uc & (UNIT_RING - 1)];
-      if (uinfo.x < 0) break;  // the end of the stream
+    const bool bulk = SCALED && P.sc_slots != 0;  // the multipliers of a tile arrive with it, or are made from it
+    const bool every_group_full = P.mt == 1 || (n_tiles & 1) == 0;
+    for (;; ++uc) {
+      // with one resident tile the two groups take alternate units
+      if (P.mt == 1 && (uc & 1) != wg) continue;
+      // The unit (tile group, document, length, first row) comes from the producer's ring.  The group's first warp
+      // waits for its publication and - in kernels without per-column multipliers, which have nothing to prepare
+      // while the MMAs run - for the unit's first accumulator, when this group has a tile in the unit's tile group.
+      int st_ = 1;
+      if (leader) {
+        st_ = wait_posted(ctl, uc, P.status);
+        if (st_ == 1 && !SCALED) {
+          // (only the last tile group can lack this group's tile, and only when the tile count is odd)
+          const bool mine_ = every_group_full || ctl->unit_info[uc & (UNIT_RING - 1)].z * P.mt + wg < n_tiles;
+          if (mine_ && !wait_bar(&ctl->acc_full[wg], n_acc & 1, ctl, P.status)) st_ = 0;
+        }
+      }
+      {
+        // the first warp arrives with one true predicate when its wait gave up, with two when the stream has ended
+        int state_;
+        LIK_GRP_SYNC_COUNT((st_ == 0 && lane == 0) || (st_ == 2 && lane < 2), state_);
+        ok = state_ != 1;
+        if (state_ != 0) break;
+      }
+      const int4 uinfo = ctl->unit_info[uc & (UNIT_RING - 1)];
       const int grp = uinfo.z;
       const int doc = uinfo.w;
       // (a group number out of range cannot index anything: its tile number fails the range check below)
       if (grp != cur_grp) {
         cur_grp = grp;
-        // (re)build the segment table of this set's tile
-        tile_id = grp * P.mt + my_tile;
+        // (re)build the segment table of this group's tile `wg` (mt == 2) or tile 0 (mt == 1: both groups)
+        const int m = P.mt == 2 ? wg : 0;
+        tile_id = grp * P.mt + m;
         have_tile = (unsigned)tile_id < (unsigned)n_tiles;
-        ok = LIK_SET_SYNC();  // everyone in the set is done reading the old table
-        if (!ok) break;
+        LIK_GRP_SYNC();  // everyone in the group is done reading the old table
         LIK_TOPK_STORE_BACK();
         TileInfo ti{};
         int nseg = 0;
         if (have_tile) {
           ti = tile_info(P, tile_id);
           nseg = ti.qb - ti.qa;
-          ctl->row_seg[set][et] = -1;
-          if (et == 0) {
-            ctl->n_seg[set] = nseg;
-            ctl->warp_aligned[set] = P.q_chunks == 1 ? 1 : 0;
+          if (sub == 0) {
+            ctl->row_seg[wg][et] = -1;
+            if (et == 0) {
+              ctl->n_seg[wg] = nseg;
+              ctl->warp_aligned[wg] = P.q_chunks == 1 ? 1 : 0;
+            }
           }
         }
-        ok = LIK_SET_SYNC();
-        if (!ok) break;
-        if (have_tile && et < nseg) {
+        LIK_GRP_SYNC();
+        if (have_tile && sub == 0 && et < nseg) {
           long long r0;
           int len;
           seq_bounds(P.q, ti.qa + et, r0, len, P.status);
@@ -933,40 +755,39 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
             if (len > P.q_chunks * TILE_M && P.status) atomicOr(P.status, LIK_DEV_LEN_RANGE);
           }
           // an empty query owns no accumulator row, so only the per-query pass below can write its zero
-          if ((off & 31) != 0 || l > 32 || l == 0) ctl->warp_aligned[set] = 0;
+          if ((off & 31) != 0 || l > 32 || l == 0) ctl->warp_aligned[wg] = 0;
           if (ARGMAX && len > P.argmax_stride && P.status) atomicOr(P.status, LIK_DEV_ARGMAX_STRIDE);
-          ctl->seg_off[set][et] = (short)off;
-          ctl->seg_len[set][et] = (short)l;
-          ctl->seg_q[set][et] = ti.qa + et;
-          for (int i = 0; i < l; ++i) ctl->row_seg[set][off + i] = (short)et;
+          ctl->seg_off[wg][et] = off;
+          ctl->seg_len[wg][et] = l;
+          ctl->seg_q[wg][et] = ti.qa + et;
+          for (int i = 0; i < l; ++i) ctl->row_seg[wg][off + i] = (short)et;
           if (topk) {
-            // the candidate list of (this CTA, this group, this lane, this query)
-            my_list = ((int)blockIdx.x + grp) * P.topk.qpg + set * P.q_per_tile + et;
+            // the candidate list of (this CTA, this group, this query)
+            // (with one resident tile the two epilogue groups take alternate documents: a list each)
+            my_list = ((int)blockIdx.x + grp) * P.topk.qpg + (P.mt == 2 ? m : wg) * P.q_per_tile + et;
             if ((unsigned)my_list >= (unsigned)P.topk.n_lists) {
               if (P.status) atomicOr(P.status, LIK_DEV_INTERNAL);
               my_list = 0;
             }
             const int2 hd = P.topk.hdr[my_list];
-            ctl->seg_list[set][et] = my_list;
-            ctl->seg_cnt[set][et] = hd.x;
-            ctl->seg_thr[set][et] = (unsigned)hd.y;
+            ctl->seg_list[wg][et] = my_list;
+            ctl->seg_cnt[wg][et] = hd.x;
+            ctl->seg_thr[wg][et] = (unsigned)hd.y;
           }
         }
-        ok = LIK_SET_SYNC();
-        if (!ok) break;
+        LIK_GRP_SYNC();
         in_seg = false;
         row_ok = false;
-        warp_rows = false;
         arg_off = -1;
         warp_out = -1;
         warp_seg = -1;
-        aligned = have_tile && ctl->warp_aligned[set] != 0;
+        aligned = have_tile && ctl->warp_aligned[wg] != 0;
         if (have_tile) {
-          const int sg = ctl->row_seg[set][row];
+          const int sg = ctl->row_seg[wg][row];
           if (sg >= 0) {
             in_seg = true;
-            const int my_q = ctl->seg_q[set][sg];
-            const int my_s = row - ctl->seg_off[set][sg] + ti.chunk * TILE_M;
+            const int my_q = ctl->seg_q[wg][sg];
+            const int my_s = row - ctl->seg_off[wg][sg] + ti.chunk * TILE_M;
             const long long qrow = ti.row0 + row;
             row_ok = row_valid(P.q, qrow);
             my_qf = row_factor(P.q, qrow);
@@ -974,15 +795,18 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
               arg_off = (cross ? (long long)my_q * P.n_d : 0ll) * P.argmax_stride + my_s;
           }
           warp_rows = __any_sync(0xffffffffu, in_seg);
-          const int sg0 = ctl->row_seg[set][quad * 32];
+          const int sg0 = ctl->row_seg[wg][quad * 32];
           if (aligned && sg0 >= 0) {
             warp_seg = sg0;
-            warp_out = cross ? (long long)ctl->seg_q[set][sg0] * P.n_d : 0ll;
+            warp_out = cross ? (long long)ctl->seg_q[wg][sg0] * P.n_d : 0ll;
           }
         }
       }
+      // a tile group with an odd tile out: the second epilogue group has nothing in it
+      if (!have_tile) continue;
       const int dlen = uinfo.x & UNIT_LEN_MASK;
-      int sc_slot = SCALED ? (uinfo.x >> UNIT_SLOT_SHIFT) & 15 : 0;  // multiplier slot of the unit's first piece, in its lane's ring
+      int sc_slot = SCALED ? (uinfo.x >> UNIT_SLOT_SHIFT) & 31 : 0;  // multiplier slot of the unit's first tile
+      const int sc_base = SCALED && sc_slot >= P.sc_per ? P.sc_per : 0;  // first slot of its ring
       const long long drow0 = uinfo.y;
       const bool holes = (uinfo.x & LEN_FLAG_MASKED) != 0;  // the document's mask is not a plain prefix
       // where this unit's results go: CROSS / GROUPED index by document, LIST by pair (== unit)
@@ -990,7 +814,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
       float run_m = -INFINITY;
       int run_i = -1;
       int c0 = 0;
-      // The pieces of the document.  The body exists twice in the kernels without per-column multipliers: documents whose
+      // The tiles of the document.  The body exists twice in the kernels without per-column multipliers: documents whose
       // mask is a plain prefix (nearly all) take the copy that has no column arrays in it, the others the general one -
       // the common path's time goes with its code size, so the rare one stays out of it.
       auto document_tiles = [&](auto general_, auto lazy_) {
@@ -999,44 +823,36 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
       constexpr bool use_cols = SCALED || general;          // per-column multiplier / additive mask needed
       do {
         const int ncols = max(0, min(TILE_N, dlen - c0));
-        // SHIFT: the token of the piece's first column; a chunk of 32 columns never reaches behind the document's end
-        const int base = SHIFT ? max(min(c0, dlen - ((ncols + 31) & ~31)), 0) : c0;
-        // Per-column arrays of this piece, staged by the whole set.  There are two of them, so that the one rendezvous
-        // behind the writes also says that everyone is done with the one that the piece after the next will overwrite.
-        float* const col_scale = ctl->col_scale[set][n_col & 1];
-        float* const col_bias = ctl->col_bias[set][n_col & 1];
-        const bool staged = general || (SCALED && !bulk);
-        const float* const sc_arr = SCALED && bulk ? sc_ring + (ln * P.sc_per + sc_slot) * TILE_N : col_scale;
-        auto stage_columns = [&]() {
-          ++n_col;
-          const int c = et;  // a thread per column
-          if (c < ((ncols + 31) & ~31)) {
-            float sc = 1.f, bi = -INFINITY;
-            const int tok = SHIFT && dlen >= BOX_ROWS ? min(base + (c & ~31), dlen - BOX_ROWS) + (c & 31) : base + c;  // the token that column c stands for
-            if (tok < dlen) {
-              const long long drow = drow0 + tok;
-              sc = norm_warps ? sc_arr[c] : row_factor(P.d, drow);
-              bi = row_valid(P.d, drow) ? 0.f : -INFINITY;
-            }
-            col_scale[c] = sc;
-            col_bias[c] = bi;
-          }
-        };
-        if (staged && early) {  // before the accumulator wait: overlaps the MMAs
-          stage_columns();
-          ok = LIK_SET_SYNC();
-          if (!ok) break;
-        }
-        if (early || c0 > 0) {
-          ok = LIK_WAIT_ACC();
+        // per-column arrays of this tile.  They may be written once the previous tile's readers are done with them (a
+        // rendezvous, unless the one at the top of the unit already stands between), and read after one more rendezvous.
+#define LIK_STAGE_COLUMNS(sync_before_)                                                                   \
+  do {                                                                                                    \
+    if (sync_before_) LIK_GRP_SYNC();                                                                     \
+    for (int c = sub * EPI_THREADS + et; c < ((ncols + 31) & ~31); c += 2 * EPI_THREADS) {                \
+      float sc = 1.f, bi = -INFINITY;                                                                     \
+      if (c < ncols) {                                                                                    \
+        const long long drow = drow0 + c0 + c;                                                            \
+        sc = norm_warps ? sc_ring[sc_slot * TILE_N + c] : row_factor(P.d, drow);                          \
+        bi = row_valid(P.d, drow) ? 0.f : -INFINITY;                                                      \
+      }                                                                                                   \
+      ctl->col_scale[wg][c] = sc;                                                                         \
+      ctl->col_bias[wg][c] = bi;                                                                          \
+    }                                                                                                     \
+  } while (0)
+        // before the accumulator wait: overlaps the MMAs; the wait's rendezvous also publishes the columns
+        // (not needed when the multipliers came with the tile and the mask has no holes)
+        const bool staged = SCALED && (general || !bulk) && !norm_warps;
+        if (staged) LIK_STAGE_COLUMNS(c0 > 0);
+        if (SCALED || c0 > 0) {
+          LIK_GROUP_WAIT_ACC();
           if (!ok) break;
         }
         ++n_acc;
-        if (staged && !early) {
-          stage_columns();
-          ok = LIK_SET_SYNC();
-          if (!ok) break;
+        if (general && (!SCALED || norm_warps)) {  // a document whose mask has holes: known only now, or its multipliers are
+          LIK_STAGE_COLUMNS(true);
+          LIK_GRP_SYNC();
         }
+#undef LIK_STAGE_COLUMNS
         tc_fence_after();
         // the accumulator goes back to the issuer as soon as this warp's last columns sit in registers
 #define LIK_RELEASE_ACC()                                          \
@@ -1045,64 +861,68 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
     __syncwarp();                                                  \
     if (lane == 0) mbar_arrive(acc_empty_bar);                     \
   } while (0)
+        // chunks of this half: cc, cc + 64, ...; only the tile's last chunk can be partial
         // (a warp without a query row, as most have under a single short query, only hands the accumulator on)
-        int cc = warp_rows ? 0 : ncols;
+        int cc = warp_rows ? sub * 32 : ncols;
         if (cc >= ncols) LIK_RELEASE_ACC();
         if (use_cols && general) {
           // a mask with holes: every chunk takes multiplier and additive mask
-          for (; cc < ncols; cc += 32) {
+          for (; cc < ncols; cc += 64) {
             float v[32];
             tmem_ld32_issue(lane_addr + (uint32_t)cc, v);
             tmem_ld_wait(v);
-            affine32(v, col_scale + cc, col_bias + cc);  // bias is -inf past ncols and in holes
-            if (cc + 32 >= ncols) LIK_RELEASE_ACC();
-            fold32<ARGMAX, lazy>(v, SHIFT && dlen >= BOX_ROWS ? min(base + cc, dlen - BOX_ROWS) : base + cc, run_m, run_i);
+            if (cc + 64 >= ncols) LIK_RELEASE_ACC();
+            affine32(v, &ctl->col_scale[wg][cc], &ctl->col_bias[wg][cc]);  // bias is -inf past ncols and in holes
+            fold32<ARGMAX, lazy>(v, c0 + cc, run_m, run_i);
           }
         } else if (use_cols) {
           // whole chunks are valid: multiplier only; the partial last chunk also takes the mask (-inf past ncols).
-          // Multipliers that came with the piece sit in a ring slot that is refilled once the accumulator has changed
+          // Multipliers that came with the tile sit in a ring slot that is refilled once the accumulator has changed
           // hands often enough: there the accumulator goes back after the last read of them, not before.
-          for (; cc < ncols; cc += 32) {
-            const bool last = cc + 32 >= ncols;
+          const float* sc_arr = bulk ? sc_ring + sc_slot * TILE_N : ctl->col_scale[wg];
+          for (; cc + 32 <= ncols; cc += 64) {
             float v[32];
             tmem_ld32_issue(lane_addr + (uint32_t)cc, v);
             tmem_ld_wait(v);
-            if (last && !bulk) LIK_RELEASE_ACC();
-            if (cc + 32 <= ncols) scale32(v, sc_arr + cc);
-            else scale32_first(v, sc_arr + cc, ncols - cc);
-            if (last && bulk) LIK_RELEASE_ACC();
+            if (!bulk && cc + 64 >= ncols) LIK_RELEASE_ACC();
+            scale32(v, sc_arr + cc);
+            if (bulk && cc + 64 >= ncols) LIK_RELEASE_ACC();
             fold32<ARGMAX, lazy>(v, c0 + cc, run_m, run_i);
           }
-        } else if (SHIFT) {
-          for (; cc < ncols; cc += 32) {
+          if (cc < ncols) {
             float v[32];
             tmem_ld32_issue(lane_addr + (uint32_t)cc, v);
             tmem_ld_wait(v);
-            if (cc + 32 >= ncols) LIK_RELEASE_ACC();
-            int at = min(base + cc, dlen - BOX_ROWS);
-            if (dlen < BOX_ROWS) {  // a document of fewer than 32 tokens is all that still needs a mask
-#pragma unroll
-              for (int i = 0; i < 32; ++i) v[i] = i < ncols ? v[i] : -INFINITY;
-              at = 0;
+            if (bulk) {
+              scale32_first(v, sc_arr + cc, ncols - cc);
+              LIK_RELEASE_ACC();
+            } else {
+              LIK_RELEASE_ACC();
+              affine32(v, &ctl->col_scale[wg][cc], &ctl->col_bias[wg][cc]);
             }
-            fold32<ARGMAX, lazy>(v, at, run_m, run_i);
+            fold32<ARGMAX, lazy>(v, c0 + cc, run_m, run_i);
           }
         } else {
-          for (; cc < ncols; cc += 32) {
+          for (; cc + 32 <= ncols; cc += 64) {
             float v[32];
             tmem_ld32_issue(lane_addr + (uint32_t)cc, v);
             tmem_ld_wait(v);
-            if (cc + 32 >= ncols) {
-              LIK_RELEASE_ACC();
+            if (cc + 64 >= ncols) LIK_RELEASE_ACC();
+            fold32<ARGMAX, lazy>(v, c0 + cc, run_m, run_i);
+          }
+          if (cc < ncols) {  // the partial last chunk
+            float v[32];
+            tmem_ld32_issue(lane_addr + (uint32_t)cc, v);
+            tmem_ld_wait(v);
+            LIK_RELEASE_ACC();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) v[i] = cc + i < ncols ? v[i] : -INFINITY;
-            }
+            for (int i = 0; i < 32; ++i) v[i] = cc + i < ncols ? v[i] : -INFINITY;
             fold32<ARGMAX, lazy>(v, c0 + cc, run_m, run_i);
           }
         }
 #undef LIK_RELEASE_ACC
         c0 += TILE_N;
-        if (SCALED && ++sc_slot >= P.sc_per) sc_slot = 0;
+        if (SCALED && ++sc_slot >= sc_base + P.sc_per) sc_slot = sc_base;
       } while (c0 < dlen);
       };
       // (long documents, WINNERS == 2: most 32-column chunks past the first few hundred tokens hold no new maximum for any
@@ -1110,90 +930,103 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
       if (holes) document_tiles(std::true_type{}, std::false_type{});
       else document_tiles(std::false_type{}, std::integral_constant<bool, WINNERS == 2>{});
       if (!ok) break;
-      // ---- end of document ----
-      if (!have_tile || (aligned && !warp_rows)) continue;
+      // ---- end of document: half 1 hands over, half 0 merges (lower column wins a tie) ----
+      float* xm = ctl->xch_m[wg][n_doc & 1];
+      int* xi = ctl->xch_i[wg][n_doc & 1];
+      ++n_doc;
+      if (sub == 1) {
+        xm[row] = run_m;
+        if (ARGMAX) xi[row] = run_i;
+      }
+      LIK_GRP_SYNC();
+      if (sub == 1) continue;
+      {
+        const float m1 = xm[row];
+        if (ARGMAX) {
+          const int i1 = xi[row];
+          const bool take = (i1 >= 0) & ((run_i < 0) | (m1 > run_m) | ((m1 == run_m) & (i1 < run_i)));
+          run_m = take ? m1 : run_m;
+          run_i = take ? i1 : run_i;
+        } else {
+          run_m = fmaxf(run_m, m1);
+        }
+      }
       // one value per row, summed per query in a fixed order
       const bool has_winner = ARGMAX ? (run_i >= 0) : (run_m != -INFINITY);
       const float val = (in_seg && row_ok && has_winner) ? run_m * my_qf : 0.f;
       if (ARGMAX && arg_off >= 0) P.argmax[arg_off + out_col * P.argmax_stride] = has_winner ? run_i : -1;
-      if (P.q_chunks > 1) {
-        // a piece of a long query: every warp leaves the sum of its 32 rows
-        const float sum = warp_sum(val);
-        if (lane == 0) P.partial[((long long)tile_id * SET_WARPS + quad) * P.n_d + doc] = sum;
-        continue;
-      }
       if (aligned) {
         // one query per warp: a shuffle tree (fixed order) replaces the shared-memory pass
         const float sum = warp_sum(val);
         if (warp_out >= 0) LIK_EMIT_SCORE(warp_seg, sum, warp_out + out_col);
         continue;
       }
-      float* ebuf = ctl->emit[set][n_emit & 1];
+      float* ebuf = ctl->emit[wg][n_emit & 1];
       ++n_emit;
       ebuf[row] = val;
-      ok = LIK_SET_SYNC();
-      if (!ok) break;
-      const int nseg = ctl->n_seg[set];
-      for (int sg = wq; sg < nseg; sg += SET_WARPS) {
-        const int off = ctl->seg_off[set][sg], len = ctl->seg_len[set][sg];
+      LIK_SUB_SYNC();
+      const int nseg = ctl->n_seg[wg];
+      for (int sg = wq; sg < nseg; sg += 4) {
+        const int off = ctl->seg_off[wg][sg], len = ctl->seg_len[wg][sg];
         float sum = 0.f;
         for (int i = lane; i < len; i += 32) sum += ebuf[off + i];
         sum = warp_sum(sum);
-        const int qq = ctl->seg_q[set][sg];
-        const long long o = cross ? (long long)qq * P.n_d + out_col : out_col;
-        LIK_EMIT_SCORE(sg, sum, o);
+        const int qq = ctl->seg_q[wg][sg];
+        if (P.q_chunks == 1) {
+          const long long o = cross ? (long long)qq * P.n_d + out_col : out_col;
+          LIK_EMIT_SCORE(sg, sum, o);
+        } else if (lane == 0) {
+          P.partial[(long long)tile_id * P.n_d + doc] = sum;
+        }
       }
     }
     // top-k: leave the lists' state where the next launch stage (the merge) finds it
-    if (topk && ok && LIK_SET_SYNC()) LIK_TOPK_STORE_BACK();
+    if (sub == 0) {
+      LIK_SUB_SYNC();
+      LIK_TOPK_STORE_BACK();
+    }
 #undef LIK_EMIT_SCORE
 #undef LIK_TOPK_STORE_BACK
-#undef LIK_WAIT_ACC
-#undef LIK_SET_SYNC
+#undef LIK_GROUP_WAIT_ACC
+#undef LIK_GRP_SYNC
+#undef LIK_GRP_SYNC_COUNT
+#undef LIK_SUB_SYNC
   } else if (SCALED && !FP8 && !PLAID && norm_warps) {
-    // =========================== inverse norms of the pieces ===========================
-    // The multipliers of a piece go into its lane's ring, and the arrival that announces them belongs to the phase of the
-    // accumulator(s) that the piece feeds: the epilogue waits for both with one wait.  An arrival must not fall into the
-    // phase before, hence the wait for that one.
-    const int nw = warp - (2 + SETS * SET_WARPS);
-    uint32_t st = 0, ph = 0, acc_ph = 0, seen = 0;
-    int sc_cnt[SETS] = {0, 0, 0, 0};
+    // =========================== inverse norms of the tiles ===========================
+    // The multipliers of a tile go into its ring slot, and the arrival that announces them belongs to the phase of the
+    // accumulator(s) that the tile feeds: the epilogue waits for both with one wait.  An arrival must not fall into the
+    // phase before, hence the wait for that one; it also says that the epilogue is done with the slots three tiles back.
+    const int nw = warp - (2 + 2 * GROUP_WARPS);
+    uint32_t st = 0, ph = 0, n_acc[2] = {0, 0};
+    int sc_cnt[2] = {0, 0};
     bool ok = true;
     const bool bf16 = P.ab_format == 1, two_slabs = P.n_slabs == 2;
     while (ok) {
       ok = wait_bar_warp(&ctl->d_full[st], ph, ctl, P.status);
       if (!ok) break;
       const uint32_t info = __shfl_sync(0xffffffffu, ctl->stage_info[st], 0);
-      // arrives for accumulator a's current phase, once the one before is complete
-      auto announce = [&](uint32_t a) {
-        if (ok && ((seen >> a) & 1u)) ok = wait_bar_warp(&ctl->acc_full[a], ((acc_ph >> a) & 1u) ^ 1u, ctl, P.status);
-        if (ok && lane == 0) mbar_arrive(smem_u32(&ctl->acc_full[a]));
-        seen |= 1u << a;
-        acc_ph ^= 1u << a;
-      };
-      if (info & STAGE_END) {  // the accumulators' last phase, which brings nothing
-        for (uint32_t a = 0; a < SETS; ++a) announce(a);
-        break;
-      }
-      const int rows = (int)(info & STAGE_COLS_MASK);
-      const uint32_t ln = (info >> STAGE_LANE_SHIFT) & (SETS - 1);
-      int at = 0;
-#pragma unroll
-      for (int l = 0; l < SETS; ++l)
-        if (l == (int)ln) {
-          at = sc_cnt[l];
-          if (++sc_cnt[l] >= P.sc_per) sc_cnt[l] = 0;
-        }
-      float* slot = sc_ring + (ln * P.sc_per + at) * TILE_N;
+      if (info & STAGE_END) break;
+      const int ncols = (int)(info & STAGE_COLS_MASK);
+      const int ring = (info & STAGE_ACC0) ? 0 : 1;
+      float* slot = sc_ring + (ring * P.sc_per + sc_cnt[ring]) * TILE_N;
       const unsigned char* stage = d_smem + (size_t)st * d_stage_bytes;
-      for (int r = nw * 32 + lane; r < rows; r += NORM_WARPS * 32) {
-        const float ss = bf16 ? stage_row_sum_sq<__nv_bfloat16>(stage + r * SLAB_BYTES_ROW, r, two_slabs ? rows : 0)
-                              : stage_row_sum_sq<__half>(stage + r * SLAB_BYTES_ROW, r, two_slabs ? rows : 0);
+      for (int r = nw * 32 + lane; r < ncols; r += NORM_WARPS * 32) {
+        const float ss = bf16 ? stage_row_sum_sq<__nv_bfloat16>(stage + r * SLAB_BYTES_ROW, r, two_slabs)
+                              : stage_row_sum_sq<__half>(stage + r * SLAB_BYTES_ROW, r, two_slabs);
         slot[r] = inv_norm(ss, P.norm_eps);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&ctl->d_empty[st]));
-      for (int t = 0; t < P.mt; ++t) announce(ln * (uint32_t)P.mt + t);
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        if (!ok || !(info & (STAGE_ACC0 << a))) continue;
+        if (n_acc[a]) ok = wait_bar_warp(&ctl->acc_full[a], (n_acc[a] - 1) & 1, ctl, P.status);
+        if (ok && lane == 0) mbar_arrive(smem_u32(&ctl->acc_full[a]));
+        ++n_acc[a];
+      }
+      // the odd tile out of a pair feeds one accumulator only: the other's epilogue must be done with the ring they share
+      if (ok && P.mt == 2 && !(info & STAGE_ACC1) && n_acc[1]) ok = wait_bar_warp(&ctl->acc_empty[1], (n_acc[1] - 1) & 1, ctl, P.status);
+      if (++sc_cnt[ring] >= P.sc_per) sc_cnt[ring] = 0;
       if (++st == (uint32_t)P.stages) { st = 0; ph ^= 1; }
     }
   }
@@ -1289,7 +1122,7 @@ __global__ void __launch_bounds__(256) pack_query_tiles_kernel(const int* __rest
   }
 }
 
-// scores[q, j] = sum over the pieces of 32 rows of query q, in order
+// scores[q, j] = sum over the partial sums of query q, in order
 __global__ void reduce_chunks_kernel(const float* __restrict__ partial, int n_q, int n_d, int pieces, float* __restrict__ scores) {
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)n_q * n_d) return;
@@ -1357,14 +1190,23 @@ static size_t sb_window_bytes() {
   return v;
 }
 
-struct TcPlan {
-  bool pack_tiles;  // ragged queries packed greedily into tiles by pack_query_tiles_kernel
-  int q_per_tile, q_chunks, n_tiles, mt, n_slabs, k_steps, stages;
-  int n_sb, sb_docs, n_groups;
-  long long n_flat, n_units_total;
-  int grid;
-  size_t smem_bytes;
-};
+// Which kernel.  The one with two streams per CTA needs more work per CTA to pay for its longer start (a stage that announces the
+// query tiles, their way through shared memory to tensor memory): STREAMS_UNITS units per CTA, which few problems have that take
+// less than 30 us.  It takes no norms from the tiles and decodes no index; with one resident tile, per-column multipliers
+// that arrive with the tiles are the other kernel's (4 queries x 4096 documents of 256 tokens in e4m3: 43 against 53 us; two tiles
+// and 16 queries 135 against 114).  A fused top-k decides by what the pieces of a corpus have in common, not by their size:
+// the candidate lists are laid out for one kernel.
+constexpr long long STREAMS_UNITS = 12;
+
+// A launch that reads every document up to four times takes the documents' norms from its tiles instead of one pass of
+// prep_kernel in front.  A query of 32 tokens against 1000 documents of up to 300 40 -> 30 us; two groups of query tiles (12 x 32
+// against 8000 of 300) 407 -> 308, (4 x 128 against 8000 of 1030) 1498 -> 953; 128-token queries against 4000 documents of up
+// to 500: three groups 458 -> 394, four 540 -> 484, five 646 -> 611, six 740 -> 724, eight 921 -> 930: the two warps take every
+// norm once per group.
+bool norms_from_tiles(const lik_fwd_args& a, const TcExtra& x, const TcPlan& pl) {
+  if (!(a.normalize & LIK_NORM_D) || x.plaid || (a.dtype != LIK_BF16 && a.dtype != LIK_F16) || a.d.scale || a.d.scale_scalar != 1.0f) return false;
+  return a.pairing == LIK_PAIR_GROUPED || (a.pairing == LIK_PAIR_CROSS && pl.n_groups <= 4);
+}
 
 TcPlan plan_tc(const lik_fwd_args& a, const TcExtra& x) {
   TcPlan pl{};
@@ -1411,13 +1253,21 @@ TcPlan plan_tc(const lik_fwd_args& a, const TcExtra& x) {
       }
     }
   }
+  const bool norms = norms_from_tiles(a, x, pl);
+  const bool multipliers = a.d.scale || ((a.normalize & LIK_NORM_D) && !x.plaid);
+  const bool bulk = multipliers && !a.d.cu && a.d.seq_stride % 4 == 0 && a.d.n_rows % 4 == 0;
+  pl.streams = !x.plaid && !norms && !(multipliers && pl.mt == 1 && (bulk || x.topk_k > 0)) &&
+               (x.topk_k > 0 || pl.n_units_total >= STREAMS_UNITS * sm_count());
   const long long g = pl.n_units_total < sm_count() ? pl.n_units_total : sm_count();
   pl.grid = (int)(g < 0 ? 0 : g);
   // the fused top-k numbers its candidate lists by CTA: the same grid whatever the piece of the corpus
   if (x.topk_k > 0 && pl.grid > 0) pl.grid = sm_count();
-  const size_t q_bytes = (size_t)pl.mt * pl.n_slabs * TILE_M * SLAB_BYTES_ROW;
-  const size_t stage = (size_t)pl.n_slabs * TILE_N * SLAB_BYTES_ROW;
-  const size_t fixed = q_bytes + sizeof(SharedCtl) + 1024;
+  const size_t q_bytes = 2 * (size_t)pl.n_slabs * TILE_M * SLAB_BYTES_ROW;
+  const size_t stage = pl.streams ? fwd_streams_stage_bytes(pl.n_slabs) : (size_t)pl.n_slabs * TILE_N * SLAB_BYTES_ROW;
+  const size_t fixed = pl.streams ? fwd_streams_fixed_smem(pl.n_slabs) : q_bytes + sizeof(SharedCtl) + 1024;
+  pl.stage_bytes = stage;
+  pl.slot_bytes = pl.streams ? fwd_streams_slot_bytes() : TILE_N * sizeof(float);
+  pl.rings = pl.lists = pl.streams ? 4 : 2;
   const size_t budget = 227 * 1024;
   int st = (int)((budget - fixed) / stage);
   pl.stages = st > 8 ? 8 : st;
@@ -1463,12 +1313,12 @@ bool fwd_tc_supported(const lik_fwd_args& a) { return tc_problem_ok(a, false); }
 // Helpers shared with the document-head kernel: a 128-byte-swizzled TMA map over the rows of a matrix whose box is
 // one 128-byte K slab wide and `box_rows` high, and the effective document lengths under a token mask.
 int make_tmap_rows(CUtensorMap* map, const void* data, int dtype, long long inner, long long n_rows, long long row_stride,
-                   int box_rows) {
+                   int box_rows, int slabs) {
   lik_seqs s{};
   s.data = data;
   s.n_rows = n_rows;
   s.row_stride = row_stride;
-  return make_map(map, s, dtype, (int)inner, box_rows);
+  return make_map(map, s, dtype, (int)inner, box_rows, slabs);
 }
 bool tmap_available() { return get_encode_fn() != nullptr; }
 // The fused top-k needs fixed query slots (padded queries of at most 128 tokens) and k within the list size.
@@ -1484,7 +1334,7 @@ bool fwd_tc_plaid_supported(const lik_fwd_args& a, const TcExtra& x) {
   return plaid_row16_ok(*x.plaid);
 }
 
-int topk_merge_parts(int n_ctas, int n_groups, int mt);
+int topk_merge_parts(int n_ctas, int n_groups, int per_slot);
 
 namespace {
 struct TcWs {
@@ -1504,15 +1354,15 @@ TcWs tc_ws_layout(const TcPlan& pl, const lik_fwd_args& a, const TcExtra& x) {
   // when the documents come in pieces
   w.n_lists = 0;
   if (x.topk_k > 0) {
-    w.n_lists = (long long)(pl.grid + pl.n_groups) * SETS * pl.q_per_tile;
+    w.n_lists = (long long)(pl.grid + pl.n_groups) * pl.lists * pl.q_per_tile;
     w.hdr = take((size_t)w.n_lists * sizeof(int2));
     w.keys = take((size_t)w.n_lists * TOPK_CAP * sizeof(float));
     w.idx = take((size_t)w.n_lists * TOPK_CAP * sizeof(int));
     // few tile groups: a query has lists from many CTAs, which are merged in parts by as many CTAs first
-    w.merge_parts = topk_merge_parts(pl.grid, pl.n_groups, pl.mt);
+    w.merge_parts = topk_merge_parts(pl.grid, pl.n_groups, pl.lists / pl.mt);
     w.merge = take(w.merge_parts > 1 ? (size_t)w.merge_parts * a.q.n_seq * x.topk_k * sizeof(long long) : 0);
   }
-  w.partial = take(pl.q_chunks > 1 ? (size_t)pl.n_tiles * SET_WARPS * a.d.n_seq * sizeof(float) : 0);
+  w.partial = take(pl.q_chunks > 1 ? (size_t)pl.n_tiles * (pl.streams ? 4 : 1) * a.d.n_seq * sizeof(float) : 0);  // (the streams kernel: one per 32 rows)
   w.lens = take((a.d.mask && !a.d.cu) ? (size_t)a.d.n_seq * sizeof(int) : 0);
   w.tiles = take(pl.pack_tiles ? (size_t)(a.q.n_seq + 3) * sizeof(int) : 0);
   w.list = take(a.pairing == LIK_PAIR_LIST ? (size_t)a.n_pairs * sizeof(int4) : 0);
@@ -1524,7 +1374,7 @@ TcWs tc_ws_layout(const TcPlan& pl, const lik_fwd_args& a, const TcExtra& x) {
 size_t fwd_tc_workspace(const lik_fwd_args& a, const TcExtra& x) { return tc_ws_layout(plan_tc(a, x), a, x).total; }
 
 int launch_topk_slots(const float* keys, const int* idx, const int2* hdr, long long n_lists, int cap, int n_ctas, int n_groups,
-                      int mt, int qpt, long long n_q, int k, int largest, long long index_offset, float* out_scores,
+                      int mt, int lists, int qpt, long long n_q, int k, int largest, long long index_offset, float* out_scores,
                       long long* out_index, int parts, void* part_buf, cudaStream_t st);
 
 // Raise the kernel's dynamic shared memory limit once per device and size instead of on every launch (a host call
@@ -1541,15 +1391,9 @@ static cudaError_t allow_smem(size_t bytes) {
   return e;
 }
 
-// A launch that reads every document up to four times takes the documents' norms from its tiles instead of one pass of
-// prep_kernel in front.  A query of 32 tokens against 1000 documents of up to 300 40 -> 30 us; two groups of query tiles (12 x 32
-// against 8000 of 300) 407 -> 308, (4 x 128 against 8000 of 1030) 1498 -> 953; 128-token queries against 4000 documents of up
-// to 500: three groups 458 -> 394, four 540 -> 484, five 646 -> 611, six 740 -> 724, eight 921 -> 930: the two warps take every
-// norm once per group.
 bool fwd_tc_norms_in_kernel(const lik_fwd_args& a, const TcExtra& x) {
-  if (!(a.normalize & LIK_NORM_D) || x.plaid || (a.dtype != LIK_BF16 && a.dtype != LIK_F16) || a.d.scale || a.d.scale_scalar != 1.0f) return false;
   const TcPlan pl = plan_tc(a, x);
-  return pl.stages >= 2 && (a.pairing == LIK_PAIR_GROUPED || (a.pairing == LIK_PAIR_CROSS && pl.n_groups <= 4));
+  return pl.stages >= 2 && norms_from_tiles(a, x, pl);
 }
 
 int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float norm_d_eps, PrepJobs prep, void* ws, size_t ws_bytes,
@@ -1569,13 +1413,11 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
   CUtensorMap q_map;
   DocMaps d_maps;
   memset(&d_maps, 0, sizeof(d_maps));
-  int rc = make_map(&q_map, a.q, a.dtype, a.dim, TILE_M);
+  int rc = pl.streams ? LIK_OK : make_map(&q_map, a.q, a.dtype, a.dim, TILE_M);
   if (rc) return rc;
-  const bool deep = a.dim * (int)dtype_size(a.dtype) == pl.n_slabs * SLAB_BYTES_ROW;
-  if (!plaid) {
+  if (!plaid && !pl.streams) {
     for (int i = 0; i < N_BOXES; ++i) {
-      rc = make_map(&d_maps.flat[i], a.d, a.dtype, a.dim, (i + 1) * BOX_ROWS);
-      if (!rc && deep) rc = make_map(&d_maps.deep[i], a.d, a.dtype, a.dim, (i + 1) * BOX_ROWS, pl.n_slabs);
+      rc = make_map(&d_maps.m[i], a.d, a.dtype, a.dim, (i + 1) * BOX_ROWS);
       if (rc) return rc;
     }
   }
@@ -1604,8 +1446,6 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
   P.d_len_flagged = 0;
   P.tile_q0 = nullptr;
   P.list_tab = nullptr;
-  P.d_deep = deep;
-  P.d_full_count = plaid ? PLAID_WARPS : 1;
   // Per-column multipliers that are exactly one fp32 array over the document rows (inverse norms or per-token scales,
   // not both) travel with the tiles when every tile's run of them starts on a 16-byte boundary and whole groups of four
   // stay inside the array: padded documents whose stride and row count are multiples of four.
@@ -1615,9 +1455,9 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
   if (norm_d_eps > 0.f || (!plaid && !a.d.cu && a.d.scale_scalar == 1.0f && ((a.d.scale != nullptr) != (dn != nullptr)))) {
     const float* arr = a.d.scale ? a.d.scale : dn;
     if (norm_d_eps > 0.f || (((uintptr_t)arr & 15) == 0 && a.d.seq_stride % 4 == 0 && a.d.n_rows % 4 == 0)) {
-      const size_t stage = (size_t)pl.n_slabs * TILE_N * SLAB_BYTES_ROW;
+      const size_t stage = pl.stage_bytes;
       const size_t fixed = pl.smem_bytes - (size_t)pl.stages * stage;
-      auto need = [&](int stages) { return fixed + (size_t)stages * stage + (size_t)(SETS / pl.mt) * (stages + 1) * TILE_N * sizeof(float); };
+      auto need = [&](int stages) { return fixed + (size_t)stages * stage + (size_t)pl.rings * (stages + 1) * pl.slot_bytes; };
       int stages = pl.stages;
       while (stages > 1 && need(stages) > (size_t)227 * 1024) --stages;
       if (need(stages) <= (size_t)227 * 1024) {
@@ -1626,7 +1466,7 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
         P.stages = stages;
         P.col_src = arr;
         P.sc_per = stages + 1;
-        P.sc_slots = SETS / pl.mt * P.sc_per;
+        P.sc_slots = pl.rings * P.sc_per;
       }
     }
     if (norm_d_eps > 0.f) P.col_src = nullptr;
@@ -1666,7 +1506,7 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
     P.topk.cand_key = (float*)((char*)ws + w.keys);
     P.topk.cand_idx = (int*)((char*)ws + w.idx);
     P.topk.k = x.topk_k;
-    P.topk.qpg = SETS * pl.q_per_tile;
+    P.topk.qpg = pl.lists * pl.q_per_tile;
     P.topk.largest = x.topk_largest;
     P.topk.doc_base = x.topk_doc_base;
     P.topk.n_lists = (int)w.n_lists;
@@ -1682,22 +1522,6 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
   const bool fp8 = a.dtype == LIK_E4M3;
   const bool argmax = a.argmax != nullptr;
   const bool affine = a.d.scale || dn || norm_d_eps > 0.f;  // a per-column multiplier for every document
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)pl.grid);
-  cfg.blockDim = dim3(NUM_THREADS);
-  cfg.dynamicSmemBytes = pl.smem_bytes;
-  cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-#define LIK_TC_LAUNCH(F, A, X, PL)                                                                                     \
-  do {                                                                                                                 \
-    LIK_CUDA_OK((allow_smem<F, A, X, PL>(pl.smem_bytes)));                                                             \
-    LIK_CUDA_OK(cudaLaunchKernelEx(&cfg, fwd_tc_kernel<F, A, X, PL>, q_map, d_maps, P));                               \
-    ::lik::count_launch();                                                                                             \
-  } while (0)
   // LIK_LONG_DOC_TOKENS overrides the length from which the lazy winner scan is used (a tuning knob)
   static int long_doc_tokens = 0;
   if (!long_doc_tokens) {
@@ -1706,31 +1530,52 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
     long_doc_tokens = v > 0 ? v : LONG_DOC_TOKENS;
   }
   const bool long_docs = argmax && a.d.max_len >= long_doc_tokens;
-  if (plaid) {
-    if (argmax) LIK_TC_LAUNCH(false, 1, false, true);
-    else LIK_TC_LAUNCH(false, 0, false, true);
-  } else if (fp8) {
-    if (argmax && affine) LIK_TC_LAUNCH(true, 1, true, false);
-    else if (argmax) LIK_TC_LAUNCH(true, 1, false, false);
-    else if (affine) LIK_TC_LAUNCH(true, 0, true, false);
-    else LIK_TC_LAUNCH(true, 0, false, false);
+  if (pl.streams) {
+    rc = launch_fwd_streams(a, pl, P, affine, long_docs, st);
+    if (rc) return rc;
   } else {
-    if (long_docs && affine) LIK_TC_LAUNCH(false, 2, true, false);
-    else if (long_docs) LIK_TC_LAUNCH(false, 2, false, false);
-    else if (argmax && affine) LIK_TC_LAUNCH(false, 1, true, false);
-    else if (argmax) LIK_TC_LAUNCH(false, 1, false, false);
-    else if (affine) LIK_TC_LAUNCH(false, 0, true, false);
-    else LIK_TC_LAUNCH(false, 0, false, false);
-  }
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)pl.grid);
+    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.dynamicSmemBytes = pl.smem_bytes;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+#define LIK_TC_LAUNCH(F, A, X, PL)                                                                                     \
+    do {                                                                                                                 \
+      LIK_CUDA_OK((allow_smem<F, A, X, PL>(pl.smem_bytes)));                                                             \
+      LIK_CUDA_OK(cudaLaunchKernelEx(&cfg, fwd_tc_kernel<F, A, X, PL>, q_map, d_maps, P));                               \
+      ::lik::count_launch();                                                                                             \
+    } while (0)
+    if (plaid) {
+      if (argmax) LIK_TC_LAUNCH(false, 1, false, true);
+      else LIK_TC_LAUNCH(false, 0, false, true);
+    } else if (fp8) {
+      if (argmax && affine) LIK_TC_LAUNCH(true, 1, true, false);
+      else if (argmax) LIK_TC_LAUNCH(true, 1, false, false);
+      else if (affine) LIK_TC_LAUNCH(true, 0, true, false);
+      else LIK_TC_LAUNCH(true, 0, false, false);
+    } else {
+      if (long_docs && affine) LIK_TC_LAUNCH(false, 2, true, false);
+      else if (long_docs) LIK_TC_LAUNCH(false, 2, false, false);
+      else if (argmax && affine) LIK_TC_LAUNCH(false, 1, true, false);
+      else if (argmax) LIK_TC_LAUNCH(false, 1, false, false);
+      else if (affine) LIK_TC_LAUNCH(false, 0, true, false);
+      else LIK_TC_LAUNCH(false, 0, false, false);
+    }
 #undef LIK_TC_LAUNCH
+  }
   LIK_CUDA_OK(cudaGetLastError());
   if (pl.q_chunks > 1) {
     const long long n = (long long)a.q.n_seq * a.d.n_seq;
-    reduce_chunks_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(P.partial, a.q.n_seq, a.d.n_seq, SET_WARPS * pl.q_chunks, a.scores), ::lik::count_launch();
+    reduce_chunks_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(P.partial, a.q.n_seq, a.d.n_seq, pl.q_chunks * (pl.streams ? 4 : 1), a.scores), ::lik::count_launch();
     LIK_CUDA_OK(cudaGetLastError());
   }
   if (x.topk_k > 0 && !(x.topk_flags & LIK_TOPK_PARTIAL)) {
-    rc = launch_topk_slots(P.topk.cand_key, P.topk.cand_idx, P.topk.hdr, w.n_lists, TOPK_CAP, pl.grid, pl.n_groups, pl.mt, pl.q_per_tile,
+    rc = launch_topk_slots(P.topk.cand_key, P.topk.cand_idx, P.topk.hdr, w.n_lists, TOPK_CAP, pl.grid, pl.n_groups, pl.mt, pl.lists, pl.q_per_tile,
                            a.q.n_seq, x.topk_k, x.topk_largest, x.topk_index_offset, x.topk_scores, (long long*)x.topk_index,
                            w.merge_parts, w.merge_parts > 1 ? (char*)ws + w.merge : nullptr, st);
     if (rc) return rc;

@@ -11,7 +11,6 @@ namespace lik {
 namespace {
 
 constexpr int TILE_M = 128;                   // accumulator rows (TMEM lanes) of every MMA
-constexpr uint32_t TRY_WAIT_HINT_NS = 20000;  // how long one try_wait may keep the thread suspended
 
 // ---------------------------------------------------------------------------------------------
 // PTX wrappers
@@ -31,10 +30,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(TRY_WAIT_HINT_NS)
+      : "r"(bar), "r"(parity)
       : "memory");
   return ok != 0;
 }

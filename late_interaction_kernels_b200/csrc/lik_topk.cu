@@ -161,10 +161,10 @@ __global__ void __launch_bounds__(NT, MIN_CTAS) topk_kernel(TopkParams P) {
 }
 
 // Merge of the candidate lists the fused scoring kernel leaves (lik_fwd_tc.cu): list slot of (CTA c, tile
-// group g) is c + g, each slot holds 4 * qpt lists of up to 256 entries (unsorted), and CTA c of n_ctas can
+// group g) is c + g, each slot holds `lists` * qpt lists of up to 256 entries (unsorted), and CTA c of n_ctas can
 // only have worked on the groups [n_groups * c / n_ctas, n_groups * (c + 1) / n_ctas] (a superset of the ones
-// it really met; lists it never touched are empty).  A group is `mt` query tiles of `qpt` queries.  The kernel has
-// 4 / mt documents in flight per CTA, each with lists of its own: a query has that many per slot.
+// it really met; lists it never touched are empty).  A group is `mt` query tiles of `qpt` queries.  A kernel has lists of its
+// own for every document it has in flight: a query has lists / mt of them per slot.
 //
 // An entry becomes one 64-bit number, larger = better: the score's ordered key above the complement of the document
 // index, so that ties need no second look.  A CTA holds the entries of up to 32 lists in registers (sixteen per thread),
@@ -183,7 +183,7 @@ struct SlotParams {
   const float* keys;
   const int* idx;
   const int2* hdr;
-  int n_ctas, n_groups, mt, qpt;
+  int n_ctas, n_groups, mt, lists, qpt;
   long long n_q, index_offset, n_lists;
   int k, largest;
   float* out_scores;
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(SLOT_T) topk_slots_kernel(SlotParams P) {
   const long long q = blockIdx.x;
   const int tile = (int)(q / P.qpt), et = (int)(q - (long long)tile * P.qpt);
   const int g = tile / P.mt, m = tile - g * P.mt;
-  const int n_sub = 4 / P.mt;
+  const int n_sub = P.lists / P.mt;
   if (warp == 0) {  // the CTAs that can have met this group
     int n = 0;
     for (int c0 = 0; c0 < P.n_ctas; c0 += 32) {
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(SLOT_T) topk_slots_kernel(SlotParams P) {
     const int li = lo + u * (SLOT_T / 32) + warp;
     if (li < hi) {
       const int sub = li % n_sub;
-      const long long list = (long long)slots[li / n_sub] * (4 * P.qpt) + (sub * P.mt + m) * P.qpt + et;
+      const long long list = (long long)slots[li / n_sub] * (P.lists * P.qpt) + (sub * P.mt + m) * P.qpt + et;
       const int c = list < P.n_lists ? min(P.hdr[list].x, SLOT_CAP) : 0;
 #pragma unroll
       for (int x = 0; x < PER_LIST; ++x) {
@@ -343,20 +343,20 @@ static int launch_topk(TopkParams& P, cudaStream_t st);
 
 // In how many parts the lists of a query are merged first: a CTA holds those of one part.  (The CTAs whose share of the
 // units can touch one tile group are at most n_ctas / n_groups + 2.)
-int topk_merge_parts(int n_ctas, int n_groups, int mt) {
+int topk_merge_parts(int n_ctas, int n_groups, int per_slot) {
   if (n_ctas <= 0 || n_groups <= 0) return 1;
-  return (int)ceil_div((int64_t)(n_ctas / n_groups + 2) * (4 / mt), SLOT_LISTS);
+  return (int)ceil_div((int64_t)(n_ctas / n_groups + 2) * per_slot, SLOT_LISTS);
 }
 
 int launch_topk_slots(const float* keys, const int* idx, const int2* hdr, long long n_lists, int cap, int n_ctas, int n_groups,
-                      int mt, int qpt, long long n_q, int k, int largest, long long index_offset, float* out_scores,
+                      int mt, int lists, int qpt, long long n_q, int k, int largest, long long index_offset, float* out_scores,
                       long long* out_index, int parts, void* part_buf, cudaStream_t st) {
   if (n_q <= 0 || k <= 0) return LIK_OK;
   if (cap != SLOT_CAP || k > SLOT_K || n_ctas > 256 || parts * k > SLOT_PER * SLOT_T || (parts > 1 && !part_buf)) {
     set_error("candidate lists of %d entries from %d CTAs, k = %d: outside what the merge takes", cap, n_ctas, k);
     return LIK_ERR_UNSUPPORTED;
   }
-  SlotParams P{keys, idx, hdr, n_ctas, n_groups, mt, qpt, n_q, index_offset, n_lists, k, largest, out_scores, out_index, parts, (u64*)part_buf};
+  SlotParams P{keys, idx, hdr, n_ctas, n_groups, mt, lists, qpt, n_q, index_offset, n_lists, k, largest, out_scores, out_index, parts, (u64*)part_buf};
   topk_slots_kernel<<<dim3((unsigned)n_q, (unsigned)parts), SLOT_T, 0, st>>>(P), ::lik::count_launch();
   LIK_CUDA_OK(cudaGetLastError());
   if (parts > 1) {
