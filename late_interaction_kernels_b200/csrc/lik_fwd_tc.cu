@@ -97,7 +97,7 @@ struct SharedCtl {
 __device__ __noinline__ bool wait_bar_slow(uint32_t b, uint32_t parity, SharedCtl* ctl, int* status) {
   const long long t0 = clock64();
   while (true) {
-    if (mbar_try_wait(b, parity)) return true;
+    if (mbar_try_wait_long(b, parity)) return true;
     if (ctl->abort_flag) return false;
     if (clock64() - t0 > ctl->wait_limit) {
       ctl->abort_flag = 1;
@@ -108,7 +108,7 @@ __device__ __noinline__ bool wait_bar_slow(uint32_t b, uint32_t parity, SharedCt
 }
 __device__ __forceinline__ bool wait_bar(unsigned long long* bar, uint32_t parity, SharedCtl* ctl, int* status) {
   const uint32_t b = smem_u32(bar);
-  if (mbar_try_wait(b, parity)) return true;
+  if (mbar_try_wait_long(b, parity)) return true;
   return wait_bar_slow(b, parity, ctl, status);
 }
 // The same for all lanes of a warp: they leave together, with one answer.
