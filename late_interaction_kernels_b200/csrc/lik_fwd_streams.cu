@@ -13,7 +13,7 @@
 //   - the query tiles are copied to tensor memory (tcgen05.cp): an MMA with A in shared memory moves 4 KB of it per 16 features
 //     beside the 3 KB of 96 document rows and took 56 cycles instead of 48 for that;
 //   - the last box of a document is moved back to end where the document ends, so that no column needs a mask.
-// In-batch 512 x 512 of 32 x 300 tokens 487 -> 356 us with winners, 355 -> 317 us without; 256 x 256 of 16 x 64 tokens 60 -> 42 us.
+// In-batch 512 x 512 of 32 x 300 tokens 487 -> 354 us with winners, 355 -> 310 us without; 256 x 256 of 16 x 64 tokens 60 -> 42 us.
 // What bounds it now: the search for the winners' columns (54 instructions on the half-rate pipe per 32 columns and warp, half of
 // the pipe's time) and the round trip of an accumulator (MMAs, 3 chunks of TMEM loads and folds, two barriers).
 //
@@ -95,10 +95,8 @@ __device__ __forceinline__ bool wait_bar(unsigned long long* bar, uint32_t parit
   }
   return true;
 }
-// The same for all lanes of a warp: they leave together, with one answer.
-__device__ __forceinline__ bool wait_bar_warp(unsigned long long* bar, uint32_t parity, SharedCtl* ctl, int* status) {
-  return __all_sync(0xffffffffu, wait_bar(bar, parity, ctl, status));
-}
+// (A converged warp probes with one instruction, whose answer all of its lanes get: no vote behind it, which cost 1 % of the
+// kernel.)
 // Bounded wait until the producer has published entry `uc` of a unit ring.  False when the CTA is aborting.
 __device__ __forceinline__ bool wait_posted(SharedCtl* ctl, int ln, int uc, int* status) {
   bool there = ctl->units_posted[ln] > uc;
@@ -119,7 +117,7 @@ __device__ __forceinline__ bool wait_posted(SharedCtl* ctl, int ln, int uc, int*
 __device__ __forceinline__ bool warps_sync(unsigned long long* bar, uint32_t& n, int lane, SharedCtl* ctl, int* status) {
   __syncwarp();
   if (lane == 0) mbar_arrive(smem_u32(bar));
-  return wait_bar_warp(bar, n++ & 1, ctl, status);
+  return wait_bar(bar, n++ & 1, ctl, status);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -311,7 +309,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     bool ok = true;
     // One stage: `rows` of `ncols` document rows from `row` on; split: two boxes, the second at row2
     auto stage = [&](uint32_t info, int ncols, int row, int row2, int slot) {
-      ok = wait_bar_warp(&d_empty[st], ph ^ 1, ctl, P.status);
+      ok = wait_bar(&d_empty[st], ph ^ 1, ctl, P.status);
       if (!ok) return;
       const uint32_t full = smem_u32(&d_full[st]);
       const int rows = (int)(info & STAGE_COLS_MASK);
@@ -375,7 +373,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           for (int t = t0; t < t1; ++t) {
             if (sm == 0) {
               // one tile at a time through the place in shared memory, which is free when its copy to tensor memory is made
-              ok = wait_bar_warp(&ctl->q_empty, (n_qload & 1) ^ 1, ctl, P.status);
+              ok = wait_bar(&ctl->q_empty, (n_qload & 1) ^ 1, ctl, P.status);
               if (!ok) break;
               if (elect) {
                 mbar_arrive_expect_tx(smem_u32(&ctl->q_full), (uint32_t)q_tile_bytes);
@@ -494,13 +492,13 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       }
     };
     while (true) {
-      if (!wait_bar_warp(&d_full[st], ph, ctl, P.status)) break;
+      if (!wait_bar(&d_full[st], ph, ctl, P.status)) break;
       const uint32_t info = __shfl_sync(0xffffffffu, ctl->stage_info[sm][st], 0);
       if (info & (STAGE_FIRST | STAGE_END)) {
         if (info & STAGE_END) {
           // the accumulators change hands once more, empty: the sets find the end of the stream in their unit ring
           for (uint32_t a = 0; a < 2; ++a) {
-            if (!wait_bar_warp(&acc_empty[a], (acc_ph >> a) & 1u, ctl, P.status)) break;
+            if (!wait_bar(&acc_empty[a], (acc_ph >> a) & 1u, ctl, P.status)) break;
             if (issue) tc_commit(smem_u32(&acc_full[a]));
             __syncwarp();
           }
@@ -512,10 +510,10 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         __syncwarp();
         bool ok = true;
         if (sm == 0) {
-          ok = wait_bar_warp(&ctl->a_idle, n_grp & 1u, ctl, P.status);
+          ok = wait_bar(&ctl->a_idle, n_grp & 1u, ctl, P.status);
           const uint32_t n_new = two && !(info & STAGE_LONE) ? 2u : 1u;
           for (uint32_t t = 0; ok && t < n_new; ++t, ++n_q) {
-            ok = wait_bar_warp(&ctl->q_full, n_q & 1u, ctl, P.status);
+            ok = wait_bar(&ctl->q_full, n_q & 1u, ctl, P.status);
             if (!ok) break;
             tc_fence_after();
             if (issue) {
@@ -527,7 +525,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
             __syncwarp();
           }
         }
-        ok = ok && wait_bar_warp(&ctl->a_ready, n_grp & 1u, ctl, P.status);
+        ok = ok && wait_bar(&ctl->a_ready, n_grp & 1u, ctl, P.status);
         if (!ok) break;
         ++n_grp;
       }
@@ -539,14 +537,14 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         if (issue) mbar_arrive(smem_u32(&d_empty[st]));
       } else if (two) {
         // (the accumulators always change hands, so that both sides keep their phase)
-        if (!wait_bar_warp(&acc_empty[0], acc_ph & 1u, ctl, P.status)) break;
+        if (!wait_bar(&acc_empty[0], acc_ph & 1u, ctl, P.status)) break;
         tc_fence_after();
         if (issue) {
           if (rows) multiply(0, 0, rows, b_stage, b_slab);
           tc_commit(smem_u32(&acc_full[0]));
         }
         __syncwarp();
-        if (!wait_bar_warp(&acc_empty[1], (acc_ph >> 1) & 1u, ctl, P.status)) break;
+        if (!wait_bar(&acc_empty[1], (acc_ph >> 1) & 1u, ctl, P.status)) break;
         acc_ph ^= 3u;
         tc_fence_after();
         if (issue) {
@@ -556,7 +554,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         }
       } else {
         const uint32_t a = info & STAGE_ACC1 ? 1u : 0u;
-        if (!wait_bar_warp(&acc_empty[a], (acc_ph >> a) & 1u, ctl, P.status)) break;
+        if (!wait_bar(&acc_empty[a], (acc_ph >> a) & 1u, ctl, P.status)) break;
         acc_ph ^= 1u << a;
         tc_fence_after();
         if (issue) {

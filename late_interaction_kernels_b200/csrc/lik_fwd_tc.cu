@@ -1196,7 +1196,9 @@ static size_t sb_window_bytes() {
 // that arrive with the tiles are the other kernel's (4 queries x 4096 documents of 256 tokens in e4m3: 43 against 53 us; two tiles
 // and 16 queries 135 against 114).  A fused top-k decides by what the pieces of a corpus have in common, not by their size:
 // the candidate lists are laid out for one kernel.
-constexpr long long STREAMS_UNITS = 12;
+// A pair list changes its query tile with every query: where documents take more than two pieces of 96 tokens it needs more units
+// (3001 pairs of 61 queries and 300-token documents 36.6 us there, 35.5 here; 10 000 pairs 88 to 97; 3001 of 64 tokens 18 to 23).
+constexpr long long STREAMS_UNITS = 12, STREAMS_PAIRS = 32;
 
 // A launch that reads every document up to four times takes the documents' norms from its tiles instead of one pass of
 // prep_kernel in front.  A query of 32 tokens against 1000 documents of up to 300 40 -> 30 us; two groups of query tiles (12 x 32
@@ -1257,7 +1259,7 @@ TcPlan plan_tc(const lik_fwd_args& a, const TcExtra& x) {
   const bool multipliers = a.d.scale || ((a.normalize & LIK_NORM_D) && !x.plaid);
   const bool bulk = multipliers && !a.d.cu && a.d.seq_stride % 4 == 0 && a.d.n_rows % 4 == 0;
   pl.streams = !x.plaid && !norms && !(multipliers && pl.mt == 1 && (bulk || x.topk_k > 0)) &&
-               (x.topk_k > 0 || pl.n_units_total >= STREAMS_UNITS * sm_count());
+               (x.topk_k > 0 || pl.n_units_total >= (a.pairing == LIK_PAIR_LIST && a.d.max_len > 192 ? STREAMS_PAIRS : STREAMS_UNITS) * sm_count());
   const long long g = pl.n_units_total < sm_count() ? pl.n_units_total : sm_count();
   pl.grid = (int)(g < 0 ? 0 : g);
   // the fused top-k numbers its candidate lists by CTA: the same grid whatever the piece of the corpus

@@ -1,0 +1,129 @@
+"""The scoring kernel of two streams per CTA, which takes problems of at least twelve units per SM, at the sizes where its pieces
+(96 tokens), boxes (32) and query tiles (128 rows, two at a time) change.
+
+Integer-valued inputs make every sum exact in fp32, so scores and winners are compared with ``==`` against plain torch."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+LENGTHS = [0, 1, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 159, 191, 192, 193, 223, 287, 288, 289, 300]
+
+
+def ints(gen, *shape, scale=1.0):
+    return torch.randint(-2, 3, shape, generator=gen, device="cuda").float() * scale
+
+
+def lengths(n, ld, gen):
+    pool = torch.tensor([x for x in LENGTHS if x <= ld] + [ld], device="cuda")
+    return pool[torch.randint(0, len(pool), (n,), generator=gen, device="cuda")]
+
+
+def reference(Q, D, mask):
+    """Row maxima [Nq, Nd, Lq] and their first positions (-1: none), a slice of documents at a time."""
+    vals, pos = [], []
+    for j in range(0, D.shape[0], 64):
+        s = torch.einsum("isd,jtd->ijst", Q, D[j:j + 64])
+        s = s.masked_fill(~mask[None, j:j + 64, None, :], float("-inf"))
+        m = s.amax(-1)
+        t = torch.arange(s.shape[-1], device="cuda").expand_as(s)
+        p = torch.where(s == m[..., None], t, s.shape[-1]).amin(-1)
+        none = torch.isinf(m)
+        vals.append(torch.where(none, torch.zeros_like(m), m))
+        pos.append(torch.where(none, torch.full_like(p, -1), p))
+    return torch.cat(vals, 1), torch.cat(pos, 1)
+
+
+# units = ceil(query tiles / 2) * documents; tiles: 128 // lq queries each, or 128-row pieces of one query
+@pytest.mark.parametrize("Nq,Nd,Lq,Ld,d,dtype", [
+    (4, 1800, 32, 300, 128, torch.bfloat16),   # one tile: the streams' accumulators take turns
+    (1, 1777, 5, 65, 64, torch.float16),       # one query of five tokens, rows of one slab
+    (8, 1800, 32, 129, 128, torch.float16),    # two tiles
+    (9, 900, 32, 193, 96, torch.bfloat16),     # three tiles, the last group's second place empty; rows that do not fill two slabs
+    (11, 900, 24, 97, 128, torch.bfloat16),    # queries that lie across warps
+    (30, 450, 128, 33, 32, torch.float16),     # full tiles, documents of one or two boxes
+    (5, 450, 300, 289, 64, torch.bfloat16),    # queries of three pieces, the last short
+    (7, 1800, 16, 31, 128, torch.bfloat16),    # documents shorter than a box
+])
+@pytest.mark.parametrize("holes", [False, True])
+def test_scores_and_winners(Nq, Nd, Lq, Ld, d, dtype, holes):
+    import late_interaction_kernels_b200 as lik
+    from late_interaction_kernels_b200.forward import maxsim_forward
+
+    gen = torch.Generator(device="cuda").manual_seed(Nq * 1009 + Ld)
+    Q, D = ints(gen, Nq, Lq, d), ints(gen, Nd, Ld, d)
+    mask = torch.arange(Ld, device="cuda")[None] < lengths(Nd, Ld, gen)[:, None]
+    if holes:
+        mask &= torch.rand(Nd, Ld, generator=gen, device="cuda") < 0.7
+    val, pos = reference(Q, D, mask)
+    tq, td = Q.to(dtype), D.to(dtype)
+    scores, am = maxsim_forward(tq, td, None, mask, save_argmax=True)
+    assert torch.equal(scores.view(Nq, Nd), val.sum(-1))
+    assert torch.equal(am.view(Nq, Nd, Lq).long(), pos)
+    assert torch.equal(lik.maxsim(tq, td, d_mask=mask), val.sum(-1))
+    if Lq <= 128:
+        k = 37
+        ts, ti = lik.retrieve(tq, td, k, d_mask=mask, normalize=False)
+        order = torch.sort(val.sum(-1), dim=1, descending=True, stable=True)
+        assert torch.equal(ts, order.values[:, :k]) and torch.equal(ti, order.indices[:, :k])
+    lik.check_device_status(scores.device)
+
+
+def test_scores_beyond_two_to_the_64():
+    from late_interaction_kernels_b200.forward import maxsim_forward
+
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    Q, D = ints(gen, 4, 32, 64, scale=2.0**31), ints(gen, 1800, 100, 64, scale=2.0**31)
+    mask = torch.ones(1800, 100, dtype=torch.bool, device="cuda")
+    val, pos = reference(Q, D, mask)
+    scores, am = maxsim_forward(Q.bfloat16(), D.bfloat16(), None, mask, save_argmax=True)
+    assert torch.equal(scores.view(4, 1800), val.sum(-1)) and torch.equal(am.view(4, 1800, 32).long(), pos)
+
+
+# candidate lists and pair lists: the query tile changes with every query
+@pytest.mark.parametrize("Nq,K,Lq,Ld", [(64, 30, 32, 300), (300, 7, 30, 97)])
+def test_lists(Nq, K, Lq, Ld):
+    import late_interaction_kernels_b200 as lik
+    from late_interaction_kernels_b200.score_pairs import score_pairs_packed
+
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    Q, D = ints(gen, Nq, Lq, 128), ints(gen, Nq * K, Ld, 128)
+    lens = lengths(Nq * K, Ld, gen)
+    mask = torch.arange(Ld, device="cuda")[None] < lens[:, None]
+    want = torch.cat([reference(Q[i:i + 1], D[i * K:(i + 1) * K], mask[i * K:(i + 1) * K])[0].sum(-1) for i in range(Nq)])
+    got = lik.maxsim(Q.bfloat16(), D.view(Nq, K, Ld, 128).bfloat16(), d_mask=mask.view(Nq, K, Ld))
+    assert torch.equal(got, want)
+    # the same pairs as a list over packed documents, often enough for 32 units per SM
+    rep = -(-32 * 160 // (Nq * K))
+    cu_q = torch.arange(Nq + 1, device="cuda", dtype=torch.int32) * Lq
+    cu_d = torch.nn.functional.pad(lens.cumsum(0), (1, 0)).int()
+    pq = torch.arange(Nq, device="cuda", dtype=torch.int32).repeat_interleave(K).repeat(rep)
+    pd = torch.arange(Nq * K, device="cuda", dtype=torch.int32).repeat(rep)
+    s = score_pairs_packed(Q.view(-1, 128).bfloat16(), D[mask].bfloat16(), cu_q, cu_d, pq, pd, max_seqlen_q=Lq, max_seqlen_d=Ld)
+    assert torch.equal(s.view(rep, Nq, K), want.expand(rep, Nq, K))
+    lik.check_device_status(s.device)
+
+
+# multipliers per document token: inverse norms that ride with the tiles (row counts that are multiples of four) or are staged by
+# the epilogue, per-token scales of e4m3; 1e-5 as for all fp32 sums of exact products
+@pytest.mark.parametrize("Ld", [96, 97, 128, 300])
+@pytest.mark.parametrize("holes", [False, True])
+def test_multipliers(Ld, holes):
+    import late_interaction_kernels_b200 as lik
+    from late_interaction_kernels_b200.fp8 import maxsim_inference_fp8, quantize_fp8_per_token
+
+    gen = torch.Generator(device="cuda").manual_seed(Ld)
+    Nq, Nd, Lq = 40, 400, 32
+    Q, D = torch.randn(Nq, Lq, 128, generator=gen, device="cuda").bfloat16(), torch.randn(Nd, Ld, 128, generator=gen, device="cuda").bfloat16()
+    mask = torch.arange(Ld, device="cuda")[None] < lengths(Nd, Ld, gen)[:, None]
+    if holes:
+        mask &= torch.rand(Nd, Ld, generator=gen, device="cuda") < 0.7
+    unit = [x.double() / x.double().norm(dim=-1, keepdim=True) for x in (Q, D)]
+    want = reference(*unit, mask)[0].sum(-1)
+    got = lik.maxsim(Q, D, d_mask=mask, normalize=True).double()
+    assert (got - want).abs().max() <= 1e-5 * want.abs().max()
+    (q8, sq), (d8, sd) = quantize_fp8_per_token(Q), quantize_fp8_per_token(D)
+    want = reference(q8.double() * sq.double()[..., None], d8.double() * sd.double()[..., None], mask)[0].sum(-1)
+    got = maxsim_inference_fp8(q8, d8, scale_Q=sq, scale_D=sd, d_mask=mask).double()
+    assert (got - want).abs().max() <= 1e-5 * want.abs().max()
