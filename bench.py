@@ -442,7 +442,7 @@ def retrieve_bench(n_docs, world, rank, dev, verify):
            "ms_per_batch_min": ms_min, "repetitions": 3, "n_docs": n_docs, "queries": 1024, "top_k": 100, "scaling": "strong",
            "tflops_valid": flops / (ms_med * 1e-3) / 1e12, "launches_per_batch_per_rank": int(launches),
            "clocks": clk.summary(),
-           "roofline": roofline("tensor", flops / world, ms_med * 1e-3, kernel="fwd_tc_kernel (bf16, fused top-k)", sustained=True,
+           "roofline": roofline("tensor", flops / world, ms_med * 1e-3, kernel="fwd_streams_kernel (bf16, fused top-k)", sustained=True,
                                 traffic=scaled_traffic("fwd_tc_kernel_topk_per_document", n_docs / world),
                                 note="per GPU: valid FLOPs of the shard over the batch time; one kernel runs for the whole "
                                      "batch, so the power cap sets the clock and the sustained cuBLAS figure is the peak")}
@@ -475,7 +475,7 @@ def retrieve_bench(n_docs, world, rank, dev, verify):
         run(q=Q8)
         ms_min, ms_med, _ = _timed(lambda: run(q=Q8), dev, 3, world)
         out["eight_queries"] = {"ms_per_batch": ms_med, "queries_per_s": 8 / (ms_med * 1e-3),
-                                "roofline": roofline("hbm", n_tok * DIM * 2, ms_med * 1e-3, kernel="fwd_tc_kernel (bf16, fused top-k)",
+                                "roofline": roofline("hbm", n_tok * DIM * 2, ms_med * 1e-3, kernel="fwd_streams_kernel (bf16, fused top-k)",
                                                      note="valid document bytes read once; 256 rows of queries make it tensor work "
                                                           "at the same time (256 FLOP per byte)")}
     if verify and world == 1:
@@ -528,7 +528,7 @@ def plaid_retrieve_bench(n_docs, world, rank, dev, verify):
     out = {"metric": "PLAID retrieve queries/s", "value": 1024 / (ms_med * 1e-3), "unit": "queries/s", "ms_per_batch": ms_med,
            "ms_per_batch_min": ms_min, "repetitions": 3, "n_docs": n_docs, "queries": 1024, "top_k": 100, "nbits": 2, "scaling": "strong",
            "tflops_valid": flops / (ms_med * 1e-3) / 1e12,
-           "roofline": roofline("tensor", flops / world, ms_med * 1e-3, kernel="plaid_decompress16_kernel + fwd_tc_kernel (fused top-k)",
+           "roofline": roofline("tensor", flops / world, ms_med * 1e-3, kernel="plaid_decompress16_kernel + fwd_streams_kernel (fused top-k)",
                                 sustained=True,
                                 note="per GPU; 128 query-tile groups share every decoded token, so the tensor pipe bounds it")}
     if verify and world == 1:
@@ -637,7 +637,7 @@ def other_configs(dev):
     qb, db = Q.bfloat16(), D.bfloat16()
     t = _time_us(lambda: lik.maxsim(qb, db, d_mask=dm), dev, graph=True)
     out["kd_bf16_fwd"] = {"us": t, "shape": "Q[64,32,128] x D[64,32,300,128]",
-                          "roofline": roofline("hbm", valid * 256 + qb.numel() * 2, t * 1e-6, kernel="fwd_tc_kernel (grouped)",
+                          "roofline": roofline("hbm", valid * 256 + qb.numel() * 2, t * 1e-6, kernel="fwd_streams_kernel (grouped)",
                                                note="valid document rows + queries, read once")}
     q8, sq = fp8.quantize_fp8_per_token(Q)
     d8, sd = fp8.quantize_fp8_per_token(D)
@@ -655,7 +655,7 @@ def other_configs(dev):
     fl = 2.0 * 128 * float(ql.sum()) * float(dl.sum())
     t = _time_us(lambda: lik.maxsim_varlen(Qp, Dp, cq, cd, 32, 1030), dev, graph=True)
     out["varlen_fwd"] = {"us": t, "shape": "128 q U[16,32] x 128 docs U[900,1030]",
-                         "roofline": roofline("tensor", fl, t * 1e-6, kernel="fwd_tc_kernel (packed)")}
+                         "roofline": roofline("tensor", fl, t * 1e-6, kernel="fwd_streams_kernel (packed)")}
     Qr, Dr = Qp.clone().requires_grad_(), Dp.clone().requires_grad_()
     go = torch.randn((128, 128), generator=g, device=dev)
 
@@ -667,7 +667,7 @@ def other_configs(dev):
     t = _time_us(fb, dev, graph=True)
     flb = fl + 4.0 * 128 * float(ql.sum()) * 128
     out["varlen_fwd_bwd"] = {"us": t, "timed": "CUDA-graph replay of forward + backward",
-                             "roofline": roofline("tensor", flb, t * 1e-6, kernel="fwd_tc_kernel + bwd_dq16 + bwd_dd_sort4 + bwd_dd_reduce16",
+                             "roofline": roofline("tensor", flb, t * 1e-6, kernel="fwd_streams_kernel + bwd_dq16 + bwd_dd_sort4 + bwd_dd_reduce16",
                                                   note="the 60 % target is quoted on this shape")}
     # PLAID candidate score: 65536 centroids, 8192 candidate documents of up to 300 codes
     qcs = torch.randn((65536, 32), generator=g, device=dev)
@@ -695,7 +695,7 @@ def other_configs(dev):
             t = _time_us(lambda: plaid.retrieve_residual_varlen(Qq, pc, pr, pcu, cent, bw, 2, 10), dev, iters=5)
             out[f"plaid_top10_{nq}q_{nd // 1000}k_docs"] = {
                 "us": t, "tokens": T,
-                "roofline": roofline("hbm", T * 36.0, t * 1e-6, kernel="plaid_decompress16_kernel + fwd_tc_kernel (fused top-k) + topk_slots_kernel",
+                "roofline": roofline("hbm", T * 36.0, t * 1e-6, kernel="plaid_decompress16_kernel + fwd_streams_kernel (fused top-k) + topk_slots_kernel",
                                      note="compressed bytes (36 B per token) read once; the decoded rows (256 B per token) are written and "
                                           "read back, and with 256 query rows the scoring is tensor work: HBM on compressed bytes is a loose bound")}
     # document head: 1 query x 1024 documents of 2048 hidden states (768 -> 128), the largest shape of the reference's
@@ -784,7 +784,7 @@ def other_configs(dev):
         out[f"cached_contrastive_bs256_ld{ld_cc}"] = {
             "us": t, "per_tile_calls_us": _time_us(tile_step, dev, iters=2, warm=1), "shape": f"bs 256, Lq 128, Ld {ld_cc}, d 128, 64 tiles of 32 x 32",
             "roofline": roofline("tensor", fl_cc + 4.0 * 128 * (256 * 128) * 256, t * 1e-6, sustained=ld_cc >= 8192,
-                                 kernel="fwd_tc_kernel + bwd_dq16 + bwd_dd_sort4 + bwd_dd_reduce16 (+ the cat of the chunks and its backward)",
+                                 kernel="fwd_streams_kernel + bwd_dq16 + bwd_dd_sort4 + bwd_dd_reduce16 (+ the cat of the chunks and its backward)",
                                  note="forward + backward of the whole grid in one call (loss_heads.maxsim_tiles)")}
         del qc, dc
         torch.cuda.empty_cache()
@@ -1025,8 +1025,8 @@ def main():
     rows_valid = float(lens.sum())
     fwd_bytes = dQ.numel() * 2 + rows_valid * DIM * 2 + dM.numel() + NQ * ND * 4 + NQ * ND * LQ * 4
     bwd_bytes = dQ.numel() * 2 + rows_valid * DIM * 2 + NQ * ND * LQ * 4 + NQ * ND * 4 + dQ.numel() * 2 + dD.numel() * 2
-    main_roof = roofline("tensor", fwd_flops, fwd_ms * 1e-3, kernel="fwd_tc_kernel (bf16, argmax, masked)",
-                         traffic=profiled_traffic("fwd_tc_kernel_argmax_inbatch"))
+    main_roof = roofline("tensor", fwd_flops, fwd_ms * 1e-3, kernel="fwd_streams_kernel (bf16, argmax, masked)",
+                         traffic=profiled_traffic("fwd_streams_kernel_argmax_inbatch"))
     main_roof["traffic_unit"] = "bytes per launch (ncu dram__bytes_read.sum + dram__bytes_write.sum; null when no capture is committed)"
     main_roof["algorithmic_bytes"] = fwd_bytes
 
@@ -1045,7 +1045,7 @@ def main():
         "clocks": clocks.summary(),
         "extra": {
             "step_kernels": {
-                "forward_no_argmax": roofline("tensor", fwd_flops, infer_ms * 1e-3, kernel="fwd_tc_kernel (bf16, masked)"),
+                "forward_no_argmax": roofline("tensor", fwd_flops, infer_ms * 1e-3, kernel="fwd_streams_kernel (bf16, masked)"),
                 "backward": roofline("hbm", bwd_bytes, bwd_ms * 1e-3, kernel="bwd_dq16 + bwd_dd_sort4 + bwd_dd_reduce16",
                                      traffic=profiled_traffic("bwd_three_kernels_inbatch"),
                                      note="algorithmic bytes: Q, valid D rows, winners, upstream gradient in; both gradients out.  "

@@ -1258,7 +1258,7 @@ TcPlan plan_tc(const lik_fwd_args& a, const TcExtra& x) {
   const bool norms = norms_from_tiles(a, x, pl);
   const bool multipliers = a.d.scale || ((a.normalize & LIK_NORM_D) && !x.plaid);
   const bool bulk = multipliers && !a.d.cu && a.d.seq_stride % 4 == 0 && a.d.n_rows % 4 == 0;
-  pl.streams = !x.plaid && !norms && !(multipliers && pl.mt == 1 && (bulk || x.topk_k > 0)) &&
+  pl.streams = !x.small_ws && !x.plaid && !norms && !(multipliers && pl.mt == 1 && (bulk || x.topk_k > 0)) &&
                (x.topk_k > 0 || pl.n_units_total >= (a.pairing == LIK_PAIR_LIST && a.d.max_len > 192 ? STREAMS_PAIRS : STREAMS_UNITS) * sm_count());
   const long long g = pl.n_units_total < sm_count() ? pl.n_units_total : sm_count();
   pl.grid = (int)(g < 0 ? 0 : g);

@@ -127,3 +127,27 @@ def test_multipliers(Ld, holes):
     want = reference(q8.double() * sq.double()[..., None], d8.double() * sd.double()[..., None], mask)[0].sum(-1)
     got = maxsim_inference_fp8(q8, d8, scale_Q=sq, scale_D=sd, d_mask=mask).double()
     assert (got - want).abs().max() <= 1e-5 * want.abs().max()
+
+
+def test_a_workspace_of_a_fixed_size_is_enough_without_the_streams():
+    """Queries of more than 128 tokens leave four partial sums per tile and document here, one in the kernel of smaller
+    problems: a buffer that holds those alone (the static scratch, 16 MiB) still takes the problem."""
+    import ctypes as C
+
+    from late_interaction_kernels_b200 import _lib, _ops
+
+    lib = _lib.load()
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    Nq, Lq, Nd, Ld, d = 64, 130, 9000, 4, 16  # 128 tiles x 9000 documents
+    Q, D = ints(gen, Nq, Lq, d).bfloat16(), ints(gen, Nd, Ld, d).bfloat16()
+    q, dd = _ops.padded_spec(Q), _ops.padded_spec(D)
+    out = torch.full((Nq, Nd), float("nan"), device="cuda")
+    a = _lib.FwdArgs(
+        q=q.c_struct(), d=dd.c_struct(), dtype=_lib.lik_dtype(Q.dtype), dim=d, pairing=_lib.PAIR_CROSS, group=0, pair_q=None, pair_d=None,
+        n_pairs=0, normalize=_lib.NORM_NONE, engine=0, scores=out.data_ptr(), argmax=None, argmax_stride=Lq, reserved=0, workspace=None,
+        workspace_bytes=0, status=_ops.status_word(Q.device).data_ptr(),
+    )
+    assert lib.lik_maxsim_fwd_workspace(C.byref(a)) > _lib.STATIC_SCRATCH_BYTES
+    _lib.check(lib.lik_maxsim_fwd_static(C.byref(a), torch.cuda.current_stream().cuda_stream), "lik_maxsim_fwd_static")
+    want = reference(Q.float(), D.float(), torch.ones(Nd, Ld, dtype=torch.bool, device="cuda"))[0].sum(-1)
+    assert torch.equal(out, want)
