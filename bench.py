@@ -443,7 +443,7 @@ def retrieve_bench(n_docs, world, rank, dev, verify):
            "tflops_valid": flops / (ms_med * 1e-3) / 1e12, "launches_per_batch_per_rank": int(launches),
            "clocks": clk.summary(),
            "roofline": roofline("tensor", flops / world, ms_med * 1e-3, kernel="fwd_streams_kernel (bf16, fused top-k)", sustained=True,
-                                traffic=scaled_traffic("fwd_tc_kernel_topk_per_document", n_docs / world),
+                                traffic=scaled_traffic("fwd_streams_kernel_topk_per_document", n_docs / world),
                                 note="per GPU: valid FLOPs of the shard over the batch time; one kernel runs for the whole "
                                      "batch, so the power cap sets the clock and the sustained cuBLAS figure is the peak")}
     # the default of retrieve(): fused L2 normalisation of both sides
