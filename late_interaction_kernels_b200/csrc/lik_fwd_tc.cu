@@ -93,8 +93,10 @@ struct SharedCtl {
 
 // Bounded wait.  Returns false when the CTA is aborting.  The first probe lets the hardware suspend
 // the thread until the phase completes (or the hint expires), so the common case costs two
-// instructions; everything else lives in one out-of-line function.
-__device__ __noinline__ bool wait_bar_slow(uint32_t b, uint32_t parity, SharedCtl* ctl, int* status) {
+// instructions; everything else is out of line or, with INLINE, behind it.  A call has registers around it saved to
+// local memory.  Only the kernels for e4m3 operands gain from doing without it: 4 x 4096 documents of 256 tokens
+// 43.9 -> 41.9 us; with all of them inlined the others lose (1 x 1000 normalised fp16 28.6 -> 31.1 us, 3001 pairs 37.0 -> 37.6).
+__device__ __forceinline__ bool wait_bar_loop(uint32_t b, uint32_t parity, SharedCtl* ctl, int* status) {
   const long long t0 = clock64();
   while (true) {
     if (mbar_try_wait_long(b, parity)) return true;
@@ -106,14 +108,19 @@ __device__ __noinline__ bool wait_bar_slow(uint32_t b, uint32_t parity, SharedCt
     }
   }
 }
+__device__ __noinline__ bool wait_bar_slow(uint32_t b, uint32_t parity, SharedCtl* ctl, int* status) {
+  return wait_bar_loop(b, parity, ctl, status);
+}
+template <bool INLINE>
 __device__ __forceinline__ bool wait_bar(unsigned long long* bar, uint32_t parity, SharedCtl* ctl, int* status) {
   const uint32_t b = smem_u32(bar);
   if (mbar_try_wait_long(b, parity)) return true;
-  return wait_bar_slow(b, parity, ctl, status);
+  return INLINE ? wait_bar_loop(b, parity, ctl, status) : wait_bar_slow(b, parity, ctl, status);
 }
 // The same for all lanes of a warp: they leave together, with one answer.
+template <bool INLINE>
 __device__ __forceinline__ bool wait_bar_warp(unsigned long long* bar, uint32_t parity, SharedCtl* ctl, int* status) {
-  return __all_sync(0xffffffffu, wait_bar(bar, parity, ctl, status));
+  return __all_sync(0xffffffffu, wait_bar<INLINE>(bar, parity, ctl, status));
 }
 // Bounded wait until the producer has published unit `uc` of this CTA in the unit ring.
 // Returns 1 when the unit is there, 2 when the stream has ended before it, 0 when the CTA is aborting.
@@ -414,7 +421,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
           tiles_here = t1 - t0;
           if (elect) {
             // wait until the MMAs that read the previous query tiles are done
-            ok = wait_bar(&ctl->q_empty, (n_qload & 1) ^ 1, ctl, P.status);
+            ok = wait_bar<FP8>(&ctl->q_empty, (n_qload & 1) ^ 1, ctl, P.status);
             if (ok) {
               mbar_arrive_expect_tx(smem_u32(&ctl->q_full), (uint32_t)((t1 - t0) * q_tile_bytes));
               for (int t = t0; t < t1; ++t) {
@@ -446,7 +453,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
         int c0 = 0;
         do {
           const int ncols = max(0, min(TILE_N, dlen - c0));
-          ok = wait_bar(&ctl->d_empty[st], ph ^ 1, ctl, P.status);
+          ok = wait_bar<FP8>(&ctl->d_empty[st], ph ^ 1, ctl, P.status);
           if (!ok) break;
           const uint32_t full = smem_u32(&ctl->d_full[st]);
           if (elect) {
@@ -508,7 +515,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
       }
       if (ok) {
         // tell the issuer that the stream has ended
-        ok = wait_bar(&ctl->d_empty[st], ph ^ 1, ctl, P.status);
+        ok = wait_bar<FP8>(&ctl->d_empty[st], ph ^ 1, ctl, P.status);
         if (ok) {
           if (elect) ctl->stage_info[st] = STAGE_END;
           if (lane == 0) mbar_arrive(smem_u32(&ctl->d_full[st]));
@@ -550,12 +557,12 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
     const int k_steps = P.k_steps;
     constexpr uint32_t A_SLAB = (TILE_M * SLAB_BYTES_ROW) >> 4, B_SLAB = (TILE_N * SLAB_BYTES_ROW) >> 4;
     while (ok) {
-      ok = wait_bar_warp(&ctl->d_full[st], ph, ctl, P.status);
+      ok = wait_bar_warp<FP8>(&ctl->d_full[st], ph, ctl, P.status);
       if (!ok) break;
       const uint32_t info = __shfl_sync(0xffffffffu, ctl->stage_info[st], 0);
       if (info & STAGE_END) break;
       if (info & STAGE_FIRST) {
-        ok = wait_bar_warp(&ctl->q_full, q_ph, ctl, P.status);
+        ok = wait_bar_warp<FP8>(&ctl->q_full, q_ph, ctl, P.status);
         if (!ok) break;
         q_ph ^= 1;
       }
@@ -565,7 +572,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
 #pragma unroll
       for (int a = 0; a < 2; ++a) {
         if (!ok || !(info & (STAGE_ACC0 << a))) continue;
-        ok = wait_bar_warp(&ctl->acc_empty[a], ((acc_ph >> a) & 1u) ^ 1u, ctl, P.status);
+        ok = wait_bar_warp<FP8>(&ctl->acc_empty[a], ((acc_ph >> a) & 1u) ^ 1u, ctl, P.status);
         if (!ok) continue;
         acc_ph ^= 1u << a;
         tc_fence_after();
@@ -640,7 +647,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
 #define LIK_GROUP_WAIT_ACC()                                                         \
   do {                                                                               \
     bool gave_up_ = false;                                                           \
-    if (leader) gave_up_ = !wait_bar(&ctl->acc_full[wg], n_acc & 1, ctl, P.status);  \
+    if (leader) gave_up_ = !wait_bar<FP8>(&ctl->acc_full[wg], n_acc & 1, ctl, P.status);  \
     int n_;                                                                          \
     LIK_GRP_SYNC_COUNT(gave_up_ && lane == 0, n_);                                   \
     ok = n_ == 0;                                                                    \
@@ -701,7 +708,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
         if (st_ == 1 && !SCALED) {
           // (only the last tile group can lack this group's tile, and only when the tile count is odd)
           const bool mine_ = every_group_full || ctl->unit_info[uc & (UNIT_RING - 1)].z * P.mt + wg < n_tiles;
-          if (mine_ && !wait_bar(&ctl->acc_full[wg], n_acc & 1, ctl, P.status)) st_ = 0;
+          if (mine_ && !wait_bar<FP8>(&ctl->acc_full[wg], n_acc & 1, ctl, P.status)) st_ = 0;
         }
       }
       {
@@ -1002,7 +1009,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
     bool ok = true;
     const bool bf16 = P.ab_format == 1, two_slabs = P.n_slabs == 2;
     while (ok) {
-      ok = wait_bar_warp(&ctl->d_full[st], ph, ctl, P.status);
+      ok = wait_bar_warp<FP8>(&ctl->d_full[st], ph, ctl, P.status);
       if (!ok) break;
       const uint32_t info = __shfl_sync(0xffffffffu, ctl->stage_info[st], 0);
       if (info & STAGE_END) break;
@@ -1020,12 +1027,12 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
 #pragma unroll
       for (int a = 0; a < 2; ++a) {
         if (!ok || !(info & (STAGE_ACC0 << a))) continue;
-        if (n_acc[a]) ok = wait_bar_warp(&ctl->acc_full[a], (n_acc[a] - 1) & 1, ctl, P.status);
+        if (n_acc[a]) ok = wait_bar_warp<FP8>(&ctl->acc_full[a], (n_acc[a] - 1) & 1, ctl, P.status);
         if (ok && lane == 0) mbar_arrive(smem_u32(&ctl->acc_full[a]));
         ++n_acc[a];
       }
       // the odd tile out of a pair feeds one accumulator only: the other's epilogue must be done with the ring they share
-      if (ok && P.mt == 2 && !(info & STAGE_ACC1) && n_acc[1]) ok = wait_bar_warp(&ctl->acc_empty[1], (n_acc[1] - 1) & 1, ctl, P.status);
+      if (ok && P.mt == 2 && !(info & STAGE_ACC1) && n_acc[1]) ok = wait_bar_warp<FP8>(&ctl->acc_empty[1], (n_acc[1] - 1) & 1, ctl, P.status);
       if (++sc_cnt[ring] >= P.sc_per) sc_cnt[ring] = 0;
       if (++st == (uint32_t)P.stages) { st = 0; ph ^= 1; }
     }
@@ -1056,7 +1063,7 @@ __global__ void wait_probe_kernel(long long limit, int* status, int* result) {
   __syncthreads();
   if (threadIdx.x == 0) {
     const long long t0 = clock64();
-    const bool got = wait_bar(&ctl.q_full, 0, &ctl, status);
+    const bool got = wait_bar<false>(&ctl.q_full, 0, &ctl, status);
     const long long dt = clock64() - t0;
     result[0] = got ? 1 : 0;
     result[1] = ctl.abort_flag;
