@@ -367,6 +367,11 @@ int lik_row_inv_norm(const void* data, int32_t dtype, int64_t n_rows, int32_t di
  * second) as its limit.  result (device, int32[3]) = {what the wait returned (0 = gave up), the CTA's abort flag,
  * cycles spent}.  Nothing faults, traps or hangs.  (No counterpart in the reference, whose length checks trap.) */
 int lik_selftest_wait_timeout(int64_t limit_cycles, int32_t* status, int32_t* result, lik_stream_t stream);
+/* The same for the other forms of the wait: with its loop inlined (e4m3 operands), and the three of the kernel for larger
+ * problems, which a whole warp runs together (on a barrier, on the unit ring, on the other warps of an epilogue set).
+ * result (device, int32[12]): three numbers each as above; for the warps' waits the first one counts the lanes that were
+ * told to go on. */
+int lik_selftest_other_waits(int64_t limit_cycles, int32_t* status, int32_t* result, lik_stream_t stream);
 const char* lik_last_error(void);
 /* kernels this library has launched in this process so far (all threads, all devices) */
 uint64_t lik_launch_count(void);

@@ -77,41 +77,33 @@ struct SharedCtl {
   int seg_list[SETS][TILE_M];      // list number (slot * qpg + query within the group)
 };
 
-// Bounded wait.  Returns false when the CTA is aborting.  A probe lets the hardware suspend the thread until the phase
-// completes (or some thousands of cycles have passed), so the common case costs two instructions.  The loop behind it is
-// inlined: a call would have the registers around it saved to local memory, and next to 220 KB of shared memory there is no
-// L1 left to keep that.
-__device__ __forceinline__ bool wait_bar(unsigned long long* bar, uint32_t parity, SharedCtl* ctl, int* status) {
-  const uint32_t b = smem_u32(bar);
-  if (mbar_try_wait(b, parity)) return true;
+// Bounded waits of a whole warp.  They return false when the CTA is aborting.  A probe lets the hardware suspend the threads
+// until the phase completes (or some thousands of cycles have passed), so the common case costs a probe and a vote.
+// The lanes leave together, with one answer: TMEM loads, shuffles and rendezvous of the full warp follow, and nothing promises
+// that two lanes that probe a barrier get the same answer, or read the clock in the same cycle.  What every warp waits for
+// cannot pass by unseen: the phase after it needs this warp's arrival first, so an answer "complete" stays true.
+// The loop behind the first probe is inlined: a call would have the registers around it saved to local memory, and next to the
+// 204 KB of shared memory there is little L1 left to keep that.
+template <class Done>
+__device__ __forceinline__ bool wait_warp(Done done, SharedCtl* ctl, int* status) {
+  if (__all_sync(0xffffffffu, done())) return true;
   const long long t0 = clock64();
-  while (!mbar_try_wait(b, parity)) {
-    if (ctl->abort_flag) return false;
+  while (!__all_sync(0xffffffffu, done())) {
     if (clock64() - t0 > ctl->wait_limit) {
       ctl->abort_flag = 1;
       if (status) atomicOr(status, LIK_DEV_WAIT_TIMEOUT);
-      return false;
     }
+    if (__any_sync(0xffffffffu, ctl->abort_flag != 0)) return false;
   }
   return true;
 }
-// (A converged warp probes with one instruction, whose answer all of its lanes get: no vote behind it, which cost 1 % of the
-// kernel.)
-// Bounded wait until the producer has published entry `uc` of a unit ring.  False when the CTA is aborting.
+__device__ __forceinline__ bool wait_bar(unsigned long long* bar, uint32_t parity, SharedCtl* ctl, int* status) {
+  const uint32_t b = smem_u32(bar);
+  return wait_warp([&] { return mbar_try_wait(b, parity); }, ctl, status);
+}
+// until the producer has published entry `uc` of a unit ring
 __device__ __forceinline__ bool wait_posted(SharedCtl* ctl, int ln, int uc, int* status) {
-  bool there = ctl->units_posted[ln] > uc;
-  if (!there) {
-    const long long t0 = clock64();
-    while (!(there = ctl->units_posted[ln] > uc)) {
-      if (ctl->abort_flag) break;
-      if (clock64() - t0 > ctl->wait_limit) {
-        ctl->abort_flag = 1;
-        if (status) atomicOr(status, LIK_DEV_WAIT_TIMEOUT);
-        break;
-      }
-    }
-  }
-  return __all_sync(0xffffffffu, there);
+  return wait_warp([&] { return ctl->units_posted[ln] > uc; }, ctl, status);
 }
 // Bounded rendezvous of the warps that share `bar` (initialised with their number); `n` counts this warp's uses of it.
 __device__ __forceinline__ bool warps_sync(unsigned long long* bar, uint32_t& n, int lane, SharedCtl* ctl, int* status) {
@@ -442,8 +434,8 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       __syncwarp();
       stage(STAGE_END, 0, 0, 0, 0);
     }
-    if (!ok && elect) {
-      // aborting: let the copies already issued land before the CTA goes away
+    if (elect) {
+      // let the copies already issued land before the CTA goes away: an issuer that gives up takes no more of them
       for (uint32_t i = 1; i <= (uint32_t)stages && i <= n_dload; ++i) {
         const bool wrapped = i > st;  // that use lies before the last wrap of the ring
         const uint32_t at = wrapped ? st + (uint32_t)stages - i : st - i;
@@ -910,6 +902,38 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
 }
 
 
+// The bounded waits of the kernel above, alone (see wait_probe_kernel in lik_fwd_tc.cu): a warp waits on a barrier that nothing
+// arrives at, then for a unit that nobody posts, then for a second warp that never comes.
+// result[3 * w + ...] = lanes that were told to go on (0: all gave up), the abort flag, cycles spent by the slowest lane.
+__global__ void streams_wait_probe_kernel(long long limit, int* status, int* result) {
+  __shared__ SharedCtl ctl;
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&ctl.q_full), 1);
+    mbar_init(smem_u32(&ctl.set_sync[0]), 2);
+    ctl.units_posted[0] = 0;
+    ctl.wait_limit = limit;
+    fence_barrier_init();
+  }
+  for (int w = 0; w < 3; ++w) {
+    if (threadIdx.x == 0) ctl.abort_flag = 0;
+    __syncwarp();
+    uint32_t n = 0;
+    const long long t0 = clock64();
+    const bool got = w == 0   ? wait_bar(&ctl.q_full, 0, &ctl, status)
+                     : w == 1 ? wait_posted(&ctl, 0, 0, status)
+                              : warps_sync(&ctl.set_sync[0], n, (int)threadIdx.x, &ctl, status);
+    const long long dt = clock64() - t0;
+    const int lanes = __popc(__ballot_sync(0xffffffffu, got));
+    const unsigned cycles = __reduce_max_sync(0xffffffffu, dt > 0x7fffffffll ? 0x7fffffffu : (unsigned)dt);
+    if (threadIdx.x == 0) {
+      result[3 * w] = lanes;
+      result[3 * w + 1] = ctl.abort_flag;
+      result[3 * w + 2] = (int)cycles;
+    }
+    __syncwarp();
+  }
+}
+
 template <bool F, int A, bool X>
 cudaError_t launch_one(const cudaLaunchConfig_t& cfg, const CUtensorMap& q_map, const DocMaps& d_maps, const TcParams& P) {
   // the limit is raised once per device and size: a host call of a microsecond or two that small problems feel
@@ -932,6 +956,12 @@ cudaError_t launch_one(const cudaLaunchConfig_t& cfg, const CUtensorMap& q_map, 
 size_t fwd_streams_fixed_smem(int n_slabs) { return (size_t)n_slabs * TILE_M * SLAB_BYTES_ROW + sizeof(SharedCtl) + 1024; }
 size_t fwd_streams_stage_bytes(int n_slabs) { return 2 * (size_t)n_slabs * TILE_N * SLAB_BYTES_ROW; }
 size_t fwd_streams_slot_bytes() { return TILE_N * sizeof(float); }
+
+int launch_streams_wait_probe(long long limit, int* status, int* result, cudaStream_t st) {
+  streams_wait_probe_kernel<<<1, 32, 0, st>>>(limit, status, result), count_launch();
+  LIK_CUDA_OK(cudaGetLastError());
+  return LIK_OK;
+}
 
 int launch_fwd_streams(const lik_fwd_args& a, const TcPlan& pl, const TcParams& P0, bool affine, bool long_docs, cudaStream_t st) {
   TcParams P = P0;

@@ -521,8 +521,8 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
           if (lane == 0) mbar_arrive(smem_u32(&ctl->d_full[st]));
         }
       }
-      if (!ok && elect) {
-        // aborting: let the copies already issued land before the CTA goes away
+      if (elect) {
+        // let the copies already issued land before the CTA goes away: an issuer that gives up takes no more of them
         if (!PLAID) {
           for (uint32_t i = 1; i <= (uint32_t)P.stages && i <= n_dload; ++i) {
             const bool wrapped = i > st;  // that use lies before the last wrap of the ring
@@ -1052,6 +1052,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
 // limit the caller chooses.  It must give up after that many cycles, raise LIK_DEV_WAIT_TIMEOUT in the status word,
 // set the abort flag and return - the path every role of the scoring kernel takes when a hand-shake never comes.
 // result[0] = what the wait returned (0 = gave up), result[1] = the abort flag, result[2] = cycles spent.
+template <bool INLINE>
 __global__ void wait_probe_kernel(long long limit, int* status, int* result) {
   __shared__ SharedCtl ctl;
   if (threadIdx.x == 0) {
@@ -1063,7 +1064,7 @@ __global__ void wait_probe_kernel(long long limit, int* status, int* result) {
   __syncthreads();
   if (threadIdx.x == 0) {
     const long long t0 = clock64();
-    const bool got = wait_bar<false>(&ctl.q_full, 0, &ctl, status);
+    const bool got = wait_bar<INLINE>(&ctl.q_full, 0, &ctl, status);
     const long long dt = clock64() - t0;
     result[0] = got ? 1 : 0;
     result[1] = ctl.abort_flag;
@@ -1598,7 +1599,16 @@ extern "C" int lik_selftest_wait_timeout(int64_t limit_cycles, int32_t* status, 
   using namespace lik;
   LIK_REQUIRE(result != nullptr, "result is NULL");
   LIK_REQUIRE(limit_cycles > 0 && limit_cycles <= 200000000ll, "limit_cycles outside (0, 2e8]");
-  wait_probe_kernel<<<1, 32, 0, (cudaStream_t)stream>>>((long long)limit_cycles, status, result), ::lik::count_launch();
+  wait_probe_kernel<false><<<1, 32, 0, (cudaStream_t)stream>>>((long long)limit_cycles, status, result), ::lik::count_launch();
   LIK_CUDA_OK(cudaGetLastError());
   return LIK_OK;
+}
+
+extern "C" int lik_selftest_other_waits(int64_t limit_cycles, int32_t* status, int32_t* result, lik_stream_t stream) {
+  using namespace lik;
+  LIK_REQUIRE(result != nullptr, "result is NULL");
+  LIK_REQUIRE(limit_cycles > 0 && limit_cycles <= 200000000ll, "limit_cycles outside (0, 2e8]");
+  wait_probe_kernel<true><<<1, 32, 0, (cudaStream_t)stream>>>((long long)limit_cycles, status, result), ::lik::count_launch();
+  LIK_CUDA_OK(cudaGetLastError());
+  return launch_streams_wait_probe((long long)limit_cycles, status, result + 3, (cudaStream_t)stream);
 }

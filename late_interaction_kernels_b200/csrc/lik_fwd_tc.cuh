@@ -188,5 +188,6 @@ size_t fwd_streams_fixed_smem(int n_slabs);   // shared memory beside its rings
 size_t fwd_streams_stage_bytes(int n_slabs);  // a stage of both streams
 size_t fwd_streams_slot_bytes();
 int launch_fwd_streams(const lik_fwd_args& a, const TcPlan& pl, const TcParams& P, bool affine, bool long_docs, cudaStream_t st);
+int launch_streams_wait_probe(long long limit, int* status, int* result, cudaStream_t st);
 
 }  // namespace lik

@@ -287,3 +287,24 @@ def test_a_bounded_wait_that_runs_out_reports_and_returns():
     lik.check_device_status()  # the word was reset; the context is healthy
     assert float(lik.maxsim(torch.ones(1, 2, 16, device="cuda").bfloat16(), torch.ones(1, 3, 16, device="cuda").bfloat16())) == 32.0
     assert lib.lik_selftest_wait_timeout(10**10, None, res.data_ptr(), None) == -1
+
+
+def test_every_form_of_the_bounded_wait_gives_up_with_all_its_lanes():
+    """The wait with its loop inlined, and the three waits of the kernel for larger problems: on expiry the whole warp is told
+    the same, reports and returns (TMEM loads and shuffles of the full warp stand behind these waits)."""
+    import late_interaction_kernels_b200 as lik
+    from late_interaction_kernels_b200 import _lib, _ops
+
+    lib = _lib.load()
+    status = _ops.status_word("cuda")
+    lik.check_device_status()
+    res = torch.full((4, 3), -1, dtype=torch.int32, device="cuda")
+    limit = 2_000_000
+    _lib.check(lib.lik_selftest_other_waits(limit, status.data_ptr(), res.data_ptr(), _lib.stream_ptr(res.device)), "selftest")
+    torch.cuda.synchronize()
+    for got, aborted, cycles in res.tolist():
+        assert got == 0 and aborted == 1
+        assert limit <= cycles < 50 * limit
+    with pytest.raises(RuntimeError, match="bounded wait expired"):
+        lik.check_device_status()
+    lik.check_device_status()
