@@ -524,7 +524,8 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
       if (elect) {
         // let the copies already issued land before the CTA goes away: an issuer that gives up takes no more of them
         if (!PLAID) {
-          for (uint32_t i = 1; i <= (uint32_t)P.stages && i <= n_dload; ++i) {
+          // (the end of the stream has completed a phase of slot `st` without a copy: its copy before that has been taken)
+          for (uint32_t i = 1; i <= (uint32_t)P.stages - (ok ? 1u : 0u) && i <= n_dload; ++i) {
             const bool wrapped = i > st;  // that use lies before the last wrap of the ring
             const uint32_t slot = wrapped ? st + (uint32_t)P.stages - i : st - i;
             const uint32_t bar = smem_u32(&ctl->d_full[slot]);
