@@ -164,12 +164,7 @@ int fwd_entry(const lik_fwd_args* a, lik_stream_t stream) {
   LIK_REQUIRE(a != nullptr, "args is NULL");
   int rc = validate_fwd(*a);
   if (rc) return rc;
-  TcExtra x;
-  FwdPlan pl = plan_fwd(*a, x);
-  if (pl.need > a->workspace_bytes) {  // (a buffer of a fixed size: queries of more than 128 tokens need a quarter as much without the streams)
-    x.small_ws = true;
-    pl = plan_fwd(*a, x);
-  }
+  FwdPlan pl = plan_fwd(*a);
   if (a->engine == 2 && !pl.use_tc) {
     set_error("tcgen05 engine requested but this problem is outside what it takes");
     return LIK_ERR_UNSUPPORTED;
@@ -178,7 +173,7 @@ int fwd_entry(const lik_fwd_args* a, lik_stream_t stream) {
     set_error("workspace too small: need %zu bytes, got %zu", pl.total, a->workspace_bytes);
     return LIK_ERR_WORKSPACE;
   }
-  return run_fwd(*a, pl, (cudaStream_t)stream, x);
+  return run_fwd(*a, pl, (cudaStream_t)stream);
 }
 }  // namespace
 }  // namespace lik
@@ -320,12 +315,7 @@ extern "C" int lik_maxsim_fwd_static(const lik_fwd_args* a, lik_stream_t stream)
   LIK_REQUIRE(a != nullptr, "args is NULL");
   int rc = validate_fwd(*a);
   if (rc) return rc;
-  size_t need = plan_fwd(*a).need;
-  if (need > (size_t)LIK_STATIC_SCRATCH_BYTES) {
-    TcExtra x;
-    x.small_ws = true;
-    need = plan_fwd(*a, x).need;
-  }
+  const size_t need = plan_fwd(*a).need;
   if (need > (size_t)LIK_STATIC_SCRATCH_BYTES) {
     set_error("lik_maxsim_fwd_static: this problem needs %zu bytes of scratch, the built-in buffer holds %zu; "
               "use lik_maxsim_fwd with a caller workspace", need, (size_t)LIK_STATIC_SCRATCH_BYTES);

@@ -855,12 +855,6 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       const bool has_winner = ARGMAX ? (run_i >= 0) : (run_m != -INFINITY);
       const float val = (in_seg && row_ok && has_winner) ? run_m * my_qf : 0.f;
       if (ARGMAX && arg_off >= 0) P.argmax[arg_off + out_col * P.argmax_stride] = has_winner ? run_i : -1;
-      if (P.q_chunks > 1) {
-        // a piece of a long query: every warp leaves the sum of its 32 rows
-        const float sum = warp_sum(val);
-        if (lane == 0) P.partial[((long long)tile_id * SET_WARPS + quad) * P.n_d + doc] = sum;
-        continue;
-      }
       if (aligned) {
         // one query per warp: a shuffle tree (fixed order) replaces the shared-memory pass
         const float sum = warp_sum(val);
@@ -879,8 +873,12 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         for (int i = lane; i < len; i += 32) sum += ebuf[off + i];
         sum = warp_sum(sum);
         const int qq = ctl->seg_q[set][sg];
-        const long long o = cross ? (long long)qq * P.n_d + out_col : out_col;
-        LIK_EMIT_SCORE(sg, sum, o);
+        if (P.q_chunks == 1) {
+          const long long o = cross ? (long long)qq * P.n_d + out_col : out_col;
+          LIK_EMIT_SCORE(sg, sum, o);
+        } else if (lane == 0) {
+          P.partial[(long long)tile_id * P.n_d + doc] = sum;  // a piece of a long query
+        }
       }
     }
     // top-k: leave the lists' state where the next launch stage (the merge) finds it

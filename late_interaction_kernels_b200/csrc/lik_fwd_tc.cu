@@ -1131,13 +1131,13 @@ __global__ void __launch_bounds__(256) pack_query_tiles_kernel(const int* __rest
   }
 }
 
-// scores[q, j] = sum over the partial sums of query q, in order
-__global__ void reduce_chunks_kernel(const float* __restrict__ partial, int n_q, int n_d, int pieces, float* __restrict__ scores) {
+// scores[q, j] = sum over the chunks of query q, in chunk order
+__global__ void reduce_chunks_kernel(const float* __restrict__ partial, int n_q, int n_d, int q_chunks, float* __restrict__ scores) {
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)n_q * n_d) return;
   const int q = (int)(idx / n_d), j = (int)(idx - (long long)q * n_d);
   float s = 0.f;
-  for (int c = 0; c < pieces; ++c) s += partial[((long long)q * pieces + c) * n_d + j];
+  for (int c = 0; c < q_chunks; ++c) s += partial[((long long)q * q_chunks + c) * n_d + j];
   scores[idx] = s;
 }
 
@@ -1267,7 +1267,7 @@ TcPlan plan_tc(const lik_fwd_args& a, const TcExtra& x) {
   const bool norms = norms_from_tiles(a, x, pl);
   const bool multipliers = a.d.scale || ((a.normalize & LIK_NORM_D) && !x.plaid);
   const bool bulk = multipliers && !a.d.cu && a.d.seq_stride % 4 == 0 && a.d.n_rows % 4 == 0;
-  pl.streams = !x.small_ws && !x.plaid && !norms && !(multipliers && pl.mt == 1 && (bulk || x.topk_k > 0)) &&
+  pl.streams = !x.plaid && !norms && !(multipliers && pl.mt == 1 && (bulk || x.topk_k > 0)) &&
                (x.topk_k > 0 || pl.n_units_total >= (a.pairing == LIK_PAIR_LIST && a.d.max_len > 192 ? STREAMS_PAIRS : STREAMS_UNITS) * sm_count());
   const long long g = pl.n_units_total < sm_count() ? pl.n_units_total : sm_count();
   pl.grid = (int)(g < 0 ? 0 : g);
@@ -1373,7 +1373,7 @@ TcWs tc_ws_layout(const TcPlan& pl, const lik_fwd_args& a, const TcExtra& x) {
     w.merge_parts = topk_merge_parts(pl.grid, pl.n_groups, pl.lists / pl.mt);
     w.merge = take(w.merge_parts > 1 ? (size_t)w.merge_parts * a.q.n_seq * x.topk_k * sizeof(long long) : 0);
   }
-  w.partial = take(pl.q_chunks > 1 ? (size_t)pl.n_tiles * (pl.streams ? 4 : 1) * a.d.n_seq * sizeof(float) : 0);  // (the streams kernel: one per 32 rows)
+  w.partial = take(pl.q_chunks > 1 ? (size_t)pl.n_tiles * a.d.n_seq * sizeof(float) : 0);
   w.lens = take((a.d.mask && !a.d.cu) ? (size_t)a.d.n_seq * sizeof(int) : 0);
   w.tiles = take(pl.pack_tiles ? (size_t)(a.q.n_seq + 3) * sizeof(int) : 0);
   w.list = take(a.pairing == LIK_PAIR_LIST ? (size_t)a.n_pairs * sizeof(int4) : 0);
@@ -1582,7 +1582,7 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
   LIK_CUDA_OK(cudaGetLastError());
   if (pl.q_chunks > 1) {
     const long long n = (long long)a.q.n_seq * a.d.n_seq;
-    reduce_chunks_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(P.partial, a.q.n_seq, a.d.n_seq, pl.q_chunks * (pl.streams ? 4 : 1), a.scores), ::lik::count_launch();
+    reduce_chunks_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(P.partial, a.q.n_seq, a.d.n_seq, pl.q_chunks, a.scores), ::lik::count_launch();
     LIK_CUDA_OK(cudaGetLastError());
   }
   if (x.topk_k > 0 && !(x.topk_flags & LIK_TOPK_PARTIAL)) {

@@ -76,7 +76,7 @@ struct TcParams {
   long long n_flat;  // GROUPED / LIST: number of units
   const int4* list_tab;  // LIST: one row per pair
   float* scores;
-  float* partial;    // [n_tiles * 4, n_d] when q_chunks > 1: sums of 32 rows
+  float* partial;    // [n_tiles, n_d] when q_chunks > 1
   int* argmax;
   int argmax_stride;
   int* status;

@@ -20,7 +20,6 @@ struct TcExtra {
   int topk_flags = 0;     // LIK_TOPK_CONTINUE / LIK_TOPK_PARTIAL
   int topk_doc_base = 0;  // index of this call's first document in the corpus
   const PlaidSrc* plaid = nullptr;
-  bool small_ws = false;  // the caller's workspace holds what the kernel of smaller problems needs, but not the streams kernel's partial sums
 };
 
 bool fwd_tc_supported(const lik_fwd_args& a);

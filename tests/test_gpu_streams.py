@@ -129,9 +129,9 @@ def test_multipliers(Ld, holes):
     assert (got - want).abs().max() <= 1e-5 * want.abs().max()
 
 
-def test_a_workspace_of_a_fixed_size_is_enough_without_the_streams():
-    """Queries of more than 128 tokens leave four partial sums per tile and document here, one in the kernel of smaller
-    problems: a buffer that holds those alone (the static scratch, 16 MiB) still takes the problem."""
+def test_long_queries_need_one_partial_sum_per_tile_and_document():
+    """Queries of more than 128 tokens leave one partial sum per 128-row tile and document in either kernel: the static scratch
+    (16 MiB) holds those of 128 tiles x 9000 documents with room to spare."""
     import ctypes as C
 
     from late_interaction_kernels_b200 import _lib, _ops
@@ -147,7 +147,19 @@ def test_a_workspace_of_a_fixed_size_is_enough_without_the_streams():
         n_pairs=0, normalize=_lib.NORM_NONE, engine=0, scores=out.data_ptr(), argmax=None, argmax_stride=Lq, reserved=0, workspace=None,
         workspace_bytes=0, status=_ops.status_word(Q.device).data_ptr(),
     )
-    assert lib.lik_maxsim_fwd_workspace(C.byref(a)) > _lib.STATIC_SCRATCH_BYTES
+    assert 128 * Nd * 4 <= lib.lik_maxsim_fwd_workspace(C.byref(a)) <= 128 * Nd * 4 + 4096
     _lib.check(lib.lik_maxsim_fwd_static(C.byref(a), torch.cuda.current_stream().cuda_stream), "lik_maxsim_fwd_static")
     want = reference(Q.float(), D.float(), torch.ones(Nd, Ld, dtype=torch.bool, device="cuda"))[0].sum(-1)
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("Nq,Lq,Ld,d", [(5, 300, 289, 64), (16, 24, 97, 128), (40, 32, 300, 96)])
+def test_few_documents_and_many_give_the_same_bits(Nq, Lq, Ld, d):
+    """The first documents alone go to the kernel of smaller problems: same products, same order of every sum."""
+    import late_interaction_kernels_b200 as lik
+
+    gen = torch.Generator(device="cuda").manual_seed(Lq)
+    Q, D = torch.randn(Nq, Lq, d, generator=gen, device="cuda").bfloat16(), torch.randn(1800, Ld, d, generator=gen, device="cuda").bfloat16()
+    mask = torch.arange(Ld, device="cuda")[None] < lengths(1800, Ld, gen)[:, None]
+    with torch.no_grad():
+        assert torch.equal(lik.maxsim(Q, D, d_mask=mask)[:, :20], lik.maxsim(Q, D[:20], d_mask=mask[:20]))
