@@ -123,6 +123,10 @@ typedef struct lik_fwd_args {
 } lik_fwd_args;
 
 size_t lik_maxsim_fwd_workspace(const lik_fwd_args* args);
+/* Which kernel this forward (topk == NULL) or fused top-k (its flags and outputs are not looked at) goes to by itself, given the
+ * workspace it asks for: 0 = portable, 1 = tensor cores, 2 = tensor cores, the kernel for larger problems; negative: refused. */
+struct lik_topk_spec;
+int lik_maxsim_fwd_kernel(const lik_fwd_args* args, const struct lik_topk_spec* topk);
 int lik_maxsim_fwd(const lik_fwd_args* args, lik_stream_t stream);
 
 /*
@@ -264,7 +268,11 @@ int lik_plaid_bwd_dq(const lik_plaid_index* index, int32_t max_ld, int64_t n_doc
 /* every call but the first sets LIK_TOPK_CONTINUE (keep the candidate lists of the earlier pieces),     */
 /* every call but the last sets LIK_TOPK_PARTIAL (no merge, nothing written to out_*); doc_base is the   */
 /* index of the piece's first document (pieces in ascending order, same queries, same k).                */
-enum lik_topk_flags { LIK_TOPK_CONTINUE = 1, LIK_TOPK_PARTIAL = 2 };
+/* LIK_TOPK_LARGE on ALL calls of a corpus (and on the calls that ask for their workspace size) lets it  */
+/* run in the kernel for larger problems, whose candidate lists take twice the bytes.  Worth it where    */
+/* lik_maxsim_fwd_kernel() names that kernel for the first piece.  A call that is no piece of a corpus   */
+/* needs no such flag; where its workspace holds the smaller lists only, it runs in the other kernel.    */
+enum lik_topk_flags { LIK_TOPK_CONTINUE = 1, LIK_TOPK_PARTIAL = 2, LIK_TOPK_LARGE = 4 };
 typedef struct lik_topk_spec {
   int32_t k;
   int32_t largest;      /* 0: the k smallest scores */

@@ -20,7 +20,7 @@ PAIR_CROSS, PAIR_GROUPED, PAIR_LIST = 0, 1, 2
 NORM_NONE, NORM_Q, NORM_D, NORM_BOTH = 0, 1, 2, 3
 NORM_ROUNDED = 4  # search paths: normalised operands rounded to the input dtype (workspace copies), see lik_b200.h
 TOPK_MAX = 8192
-TOPK_CONTINUE, TOPK_PARTIAL = 1, 2
+TOPK_CONTINUE, TOPK_PARTIAL, TOPK_LARGE = 1, 2, 4
 TOPK_FUSED_MAX = 128  # largest k of the fused scoring + top-k kernel
 STATIC_SCRATCH_BYTES = 16 << 20
 
@@ -114,6 +114,8 @@ def _declare(lib):
     lib.lik_maxsim_bwd_workspace.restype = sz
     lib.lik_maxsim_bwd.argtypes = [C.POINTER(BwdArgs), vp]
     lib.lik_maxsim_bwd.restype = i32
+    lib.lik_maxsim_fwd_kernel.argtypes = [C.POINTER(FwdArgs), C.POINTER(TopkSpec)]
+    lib.lik_maxsim_fwd_kernel.restype = i32
     lib.lik_maxsim_fwd_topk_supported.argtypes = [C.POINTER(FwdArgs), C.POINTER(TopkSpec)]
     lib.lik_maxsim_fwd_topk_supported.restype = i32
     lib.lik_maxsim_fwd_topk_workspace.argtypes = [C.POINTER(FwdArgs), C.POINTER(TopkSpec)]
@@ -162,7 +164,7 @@ def _declare(lib):
 
 EXPORTED_SYMBOLS = (
     "lik_maxsim_fwd_workspace", "lik_maxsim_fwd", "lik_maxsim_fwd_static", "lik_maxsim_bwd_workspace", "lik_maxsim_bwd", "lik_topk_rows",
-    "lik_maxsim_fwd_topk_supported", "lik_maxsim_fwd_topk_workspace", "lik_maxsim_fwd_topk",
+    "lik_maxsim_fwd_kernel", "lik_maxsim_fwd_topk_supported", "lik_maxsim_fwd_topk_workspace", "lik_maxsim_fwd_topk",
     "lik_maxsim_hidden_fwd_supported", "lik_maxsim_hidden_fwd_workspace", "lik_maxsim_hidden_fwd",
     "lik_hidden_winners", "lik_hidden_scatter_rows",
     "lik_plaid_fwd_supported", "lik_plaid_fwd_workspace", "lik_plaid_fwd", "lik_launch_count", "lik_selftest_wait_timeout",

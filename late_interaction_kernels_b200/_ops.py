@@ -172,6 +172,7 @@ class TopkState:
     def __init__(self):
         self.ws = None
         self.started = False
+        self.large = False  # all pieces run in the kernel for larger problems (decided by the first)
 
 
 @_no_trace
@@ -211,6 +212,10 @@ def forward_fused(q: SeqSpec, d, *, normalize=0, plaid: PlaidIndex | None = None
     )
     tkp = C.byref(tk) if tk is not None else None
     with torch.cuda.device(dev):
+        if state is not None and tk is not None and flags and plaid is None:
+            if not state.started:
+                state.large = lib.lik_maxsim_fwd_kernel(C.byref(a), tkp) == 2
+            tk.flags = flags | (_lib.TOPK_LARGE if state.large else 0)
         if plaid is not None:
             if not lib.lik_plaid_fwd_supported(C.byref(a), C.byref(plaid), tkp):
                 return None

@@ -17,6 +17,7 @@ struct FwdPlan {
   size_t qn_off, dn_off, qcopy_off, dcopy_off, tc_off, lens_off;
   size_t need, total;  // without and with the trimmed lengths of the portable kernel, which it can do without
   bool use_tc;
+  bool streams;  // of the two tensor-core kernels, the one for larger problems
   bool copies;  // fused normalisation through normalised operand copies instead of per-row multipliers
 };
 
@@ -86,6 +87,7 @@ FwdPlan plan_fwd(const lik_fwd_args& a, const TcExtra& x = TcExtra()) {
   // the kernel's own workspace comes first: its leading part (the candidate lists of a fused top-k) then sits at
   // the same place for every piece of a corpus that is scored piece by piece into one workspace
   if (pl.use_tc) pl.tc_off = take(fwd_tc_workspace(b, x));
+  pl.streams = pl.use_tc && fwd_tc_streams(b, x);
   if (a.normalize & LIK_NORM_Q) {
     if (pl.copies) pl.qcopy_off = take((size_t)a.q.n_rows * a.dim * eb);
     else pl.qn_off = take((size_t)a.q.n_rows * 4);
@@ -229,6 +231,10 @@ int fused_entry(const lik_fwd_args* a, const lik_plaid_index* ix, const lik_topk
   rc = fill_extra(*a, ix, tk, x, src);
   if (rc) return rc;
   FwdPlan pl = plan_fwd(*a, x);
+  if (tk && pl.total > a->workspace_bytes && !(tk->flags & (LIK_TOPK_CONTINUE | LIK_TOPK_PARTIAL))) {
+    x.small_lists = true;  // (a buffer of a fixed size: the kernel of smaller problems has half as many candidate lists)
+    pl = plan_fwd(*a, x);
+  }
   if (!pl.use_tc) {
     set_error("this problem is outside what the fused tensor-core path takes");
     return LIK_ERR_UNSUPPORTED;
@@ -257,6 +263,20 @@ extern "C" int lik_maxsim_fwd_topk_supported(const lik_fwd_args* a, const lik_to
   int ok = 0;
   if (tk) lik::fused_workspace(a, nullptr, tk, &ok);
   return ok;
+}
+extern "C" int lik_maxsim_fwd_kernel(const lik_fwd_args* a, const lik_topk_spec* tk) {
+  using namespace lik;
+  LIK_REQUIRE(a != nullptr, "args is NULL");
+  int rc = validate_fwd(*a, false, tk != nullptr);
+  if (rc) return rc;
+  TcExtra x;
+  if (tk) {
+    LIK_REQUIRE(tk->k > 0, "k must be positive");
+    x.topk_k = tk->k;
+    x.topk_largest = tk->largest != 0;
+  }
+  const FwdPlan pl = plan_fwd(*a, x);
+  return !pl.use_tc ? 0 : pl.streams ? 2 : 1;
 }
 extern "C" size_t lik_maxsim_fwd_topk_workspace(const lik_fwd_args* a, const lik_topk_spec* tk) {
   return tk ? lik::fused_workspace(a, nullptr, tk, nullptr) : 0;

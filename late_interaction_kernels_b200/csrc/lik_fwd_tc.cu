@@ -1203,8 +1203,8 @@ static size_t sb_window_bytes() {
 // query tiles, their way through shared memory to tensor memory): STREAMS_UNITS units per CTA, which few problems have that take
 // less than 30 us.  It takes no norms from the tiles and decodes no index; with one resident tile, per-column multipliers
 // that arrive with the tiles are the other kernel's (4 queries x 4096 documents of 256 tokens in e4m3: 43 against 53 us; two tiles
-// and 16 queries 135 against 114).  A fused top-k decides by what the pieces of a corpus have in common, not by their size:
-// the candidate lists are laid out for one kernel.
+// and 16 queries 135 against 114).  The candidate lists of a fused
+// top-k are laid out for one kernel: the pieces of a corpus go where LIK_TOPK_LARGE says, never by a piece's own size.
 // A pair list changes its query tile with every query: where documents take more than two pieces of 96 tokens it needs more units
 // (3001 pairs of 61 queries and 300-token documents 36.6 us there, 35.5 here; 10 000 pairs 88 to 97; 3001 of 64 tokens 18 to 23).
 constexpr long long STREAMS_UNITS = 12, STREAMS_PAIRS = 32;
@@ -1218,6 +1218,14 @@ bool norms_from_tiles(const lik_fwd_args& a, const TcExtra& x, const TcPlan& pl)
   if (!(a.normalize & LIK_NORM_D) || x.plaid || (a.dtype != LIK_BF16 && a.dtype != LIK_F16) || a.d.scale || a.d.scale_scalar != 1.0f) return false;
   return a.pairing == LIK_PAIR_GROUPED || (a.pairing == LIK_PAIR_CROSS && pl.n_groups <= 4);
 }
+
+// Candidate lists of a fused top-k: a slot per CTA and tile group (see TopkOut).
+size_t topk_list_bytes(int n_groups, int per_slot) {
+  return (size_t)(sm_count() + n_groups) * per_slot * (TOPK_CAP * (sizeof(float) + sizeof(int)) + sizeof(int2));
+}
+// The streams kernel keeps twice as many of them, which is a matter of megabytes for the batches that wait for an answer (256
+// queries of 32 tokens: 6 MB).  Beyond this the other kernel runs: 100 000 queries would take 414 MB instead of 207.
+constexpr size_t STREAMS_LISTS_BYTES = 128u << 20;
 
 TcPlan plan_tc(const lik_fwd_args& a, const TcExtra& x) {
   TcPlan pl{};
@@ -1267,8 +1275,10 @@ TcPlan plan_tc(const lik_fwd_args& a, const TcExtra& x) {
   const bool norms = norms_from_tiles(a, x, pl);
   const bool multipliers = a.d.scale || ((a.normalize & LIK_NORM_D) && !x.plaid);
   const bool bulk = multipliers && !a.d.cu && a.d.seq_stride % 4 == 0 && a.d.n_rows % 4 == 0;
-  pl.streams = !x.plaid && !norms && !(multipliers && pl.mt == 1 && (bulk || x.topk_k > 0)) &&
-               (x.topk_k > 0 || pl.n_units_total >= (a.pairing == LIK_PAIR_LIST && a.d.max_len > 192 ? STREAMS_PAIRS : STREAMS_UNITS) * sm_count());
+  const bool pieces = x.topk_flags & (LIK_TOPK_CONTINUE | LIK_TOPK_PARTIAL);
+  pl.streams = !x.small_lists && !x.plaid && !norms && !(multipliers && pl.mt == 1 && (bulk || x.topk_k > 0)) &&
+               (x.topk_k > 0 ? (!pieces || (x.topk_flags & LIK_TOPK_LARGE)) && topk_list_bytes(pl.n_groups, 4 * pl.q_per_tile) <= STREAMS_LISTS_BYTES
+                             : pl.n_units_total >= (a.pairing == LIK_PAIR_LIST && a.d.max_len > 192 ? STREAMS_PAIRS : STREAMS_UNITS) * sm_count());
   const long long g = pl.n_units_total < sm_count() ? pl.n_units_total : sm_count();
   pl.grid = (int)(g < 0 ? 0 : g);
   // the fused top-k numbers its candidate lists by CTA: the same grid whatever the piece of the corpus
@@ -1382,6 +1392,7 @@ TcWs tc_ws_layout(const TcPlan& pl, const lik_fwd_args& a, const TcExtra& x) {
 }
 }  // namespace
 
+bool fwd_tc_streams(const lik_fwd_args& a, const TcExtra& x) { return plan_tc(a, x).streams; }
 size_t fwd_tc_workspace(const lik_fwd_args& a, const TcExtra& x) { return tc_ws_layout(plan_tc(a, x), a, x).total; }
 
 int launch_topk_slots(const float* keys, const int* idx, const int2* hdr, long long n_lists, int cap, int n_ctas, int n_groups,

@@ -49,7 +49,7 @@ struct TopkOut {
   int* cand_idx;    // same shape: document index
   int2* hdr;        // [n_slots * qpg]: x = entries in the list, y = threshold as an ordered key (0: none yet)
   int k;
-  int qpg;          // lists per slot: two query tiles' worth
+  int qpg;          // lists per slot: two query tiles' worth, of every document that the kernel has in flight for them
   int largest;
   int doc_base;     // added to the document index stored with a candidate
   int n_lists;      // lists allocated (the kernel checks every list number against it)

@@ -17,7 +17,8 @@ struct TcExtra {
   long long topk_index_offset = 0;
   float* topk_scores = nullptr;
   int64_t* topk_index = nullptr;
-  int topk_flags = 0;     // LIK_TOPK_CONTINUE / LIK_TOPK_PARTIAL
+  int topk_flags = 0;     // lik_topk_flags
+  bool small_lists = false;  // the caller's workspace holds the candidate lists of the kernel for smaller problems, but not the streams kernel's
   int topk_doc_base = 0;  // index of this call's first document in the corpus
   const PlaidSrc* plaid = nullptr;
 };
@@ -26,6 +27,7 @@ bool fwd_tc_supported(const lik_fwd_args& a);
 bool fwd_tc_topk_supported(const lik_fwd_args& a, const TcExtra& x);
 bool fwd_tc_plaid_supported(const lik_fwd_args& a, const TcExtra& x);
 size_t fwd_tc_workspace(const lik_fwd_args& a, const TcExtra& x);
+bool fwd_tc_streams(const lik_fwd_args& a, const TcExtra& x);  // whether the kernel for larger problems takes it
 // `prep`: what still has to be written before the kernel runs; the launch adds its own jobs and sends them in one go
 // `norm_d_eps` > 0 (where fwd_tc_norms_in_kernel says so, dn == nullptr): the kernel takes the documents' norms itself
 bool fwd_tc_norms_in_kernel(const lik_fwd_args& a, const TcExtra& x);

@@ -163,3 +163,90 @@ def test_few_documents_and_many_give_the_same_bits(Nq, Lq, Ld, d):
     mask = torch.arange(Ld, device="cuda")[None] < lengths(1800, Ld, gen)[:, None]
     with torch.no_grad():
         assert torch.equal(lik.maxsim(Q, D, d_mask=mask)[:, :20], lik.maxsim(Q, D[:20], d_mask=mask[:20]))
+
+
+def topk_args(Q, D, mask, k, out_s=None, out_i=None, flags=0, doc_base=0):
+    from late_interaction_kernels_b200 import _lib, _ops
+
+    q, d = _ops.padded_spec(Q), _ops.padded_spec(D, mask)
+    a = _lib.FwdArgs(
+        q=q.c_struct(), d=d.c_struct(), dtype=_lib.lik_dtype(Q.dtype), dim=Q.shape[-1], pairing=_lib.PAIR_CROSS,
+        group=0, pair_q=None, pair_d=None, n_pairs=0, normalize=_lib.NORM_NONE, engine=0, scores=None, argmax=None, argmax_stride=Q.shape[1],
+        reserved=0, workspace=None, workspace_bytes=0, status=_ops.status_word(Q.device).data_ptr(),
+    )
+    a.keep = q, d
+    return a, _lib.TopkSpec(k=k, largest=1, index_offset=0, out_scores=_lib.ptr(out_s), out_index=_lib.ptr(out_i), flags=flags, doc_base=doc_base)
+
+
+@pytest.mark.parametrize("Nq", [3, 40])
+def test_topk_in_a_workspace_that_holds_the_lists_of_the_smaller_kernel(Nq):
+    """A call of its own falls back to the kernel whose lists take half the bytes when the buffer holds no more."""
+    import ctypes as C
+
+    from late_interaction_kernels_b200 import _lib
+
+    lib = _lib.load()
+    gen = torch.Generator(device="cuda").manual_seed(Nq)
+    k, Nd = 17, 32 * torch.cuda.get_device_properties(0).multi_processor_count * (2 if Nq < 5 else 1)
+    Q, D = ints(gen, Nq, 32, 64).bfloat16(), ints(gen, Nd, 40, 64).bfloat16()
+    mask = torch.arange(40, device="cuda")[None] < lengths(Nd, 40, gen)[:, None]
+    s, i = torch.empty(Nq, k, device="cuda"), torch.empty(Nq, k, dtype=torch.long, device="cuda")
+    a, t = topk_args(Q, D, mask, k, s, i)
+    assert lib.lik_maxsim_fwd_kernel(C.byref(a), C.byref(t)) == 2
+    whole = lib.lik_maxsim_fwd_topk_workspace(C.byref(a), C.byref(t))
+    t.flags = _lib.TOPK_PARTIAL  # the size that a piece without LIK_TOPK_LARGE needs
+    small = lib.lik_maxsim_fwd_topk_workspace(C.byref(a), C.byref(t))
+    t.flags |= _lib.TOPK_LARGE
+    assert lib.lik_maxsim_fwd_topk_workspace(C.byref(a), C.byref(t)) == whole and small < 0.6 * whole
+    t.flags = 0
+    want = torch.sort(reference(Q.float(), D.float(), mask)[0].sum(-1), dim=1, descending=True, stable=True)
+    for size in (whole, small):
+        s.fill_(float("nan"))
+        ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+        a.workspace, a.workspace_bytes = ws.data_ptr(), size
+        _lib.check(lib.lik_maxsim_fwd_topk(C.byref(a), C.byref(t), _lib.stream_ptr(ws.device)), "lik_maxsim_fwd_topk")
+        assert torch.equal(s, want.values[:, :k]) and torch.equal(i, want.indices[:, :k])
+    a.workspace_bytes = small - 256
+    assert lib.lik_maxsim_fwd_topk(C.byref(a), C.byref(t), _lib.stream_ptr(ws.device)) == -4
+
+
+def test_topk_lists_of_many_queries_take_no_more_than_before():
+    """The second set of lists is for batches whose lists are small."""
+    import ctypes as C
+
+    from late_interaction_kernels_b200 import _lib
+
+    lib = _lib.load()
+    Q, D = torch.zeros(1, 32, 128, device="cuda").bfloat16(), torch.zeros(4000, 4, 128, device="cuda").bfloat16()
+    a, t = topk_args(Q, D, None, 100, torch.empty(1, device="cuda"), torch.empty(1, dtype=torch.long, device="cuda"))
+    a.q.n_seq, a.q.n_rows = 100_000, 3_200_000  # (only the size is asked for)
+    assert lib.lik_maxsim_fwd_topk_workspace(C.byref(a), C.byref(t)) < 215e6
+
+
+@pytest.mark.parametrize("large", [False, True])
+@pytest.mark.parametrize("Nq", [2, 9, 40])
+def test_topk_in_pieces_of_different_sizes(Nq, large):
+    """Pieces of one document up to several super-blocks (their window is 48 MB) share one workspace and one kernel."""
+    import ctypes as C
+
+    from late_interaction_kernels_b200 import _lib
+
+    lib = _lib.load()
+    gen = torch.Generator(device="cuda").manual_seed(Nq)
+    k, sizes = 29, [1500, 1, 700, 40]
+    Nd, Ld = sum(sizes), 420  # 1500 x 420 x 256 bytes = 161 MB
+    Q, D = ints(gen, Nq, 32, 128).bfloat16(), ints(gen, Nd, Ld, 128).bfloat16()
+    mask = torch.arange(Ld, device="cuda")[None] < lengths(Nd, Ld, gen)[:, None]
+    s, i = torch.empty(Nq, k, device="cuda"), torch.empty(Nq, k, dtype=torch.long, device="cuda")
+    ws, base = None, 0
+    for n, size in enumerate(sizes):
+        flags = (_lib.TOPK_CONTINUE if n else 0) | (_lib.TOPK_PARTIAL if n + 1 < len(sizes) else 0) | (_lib.TOPK_LARGE if large else 0)
+        m = mask[base:base + size].contiguous()
+        a, t = topk_args(Q, D[base:base + size], m, k, s, i, flags, base)
+        if ws is None:
+            ws = torch.empty(lib.lik_maxsim_fwd_topk_workspace(C.byref(a), C.byref(t)), dtype=torch.uint8, device="cuda")
+        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+        _lib.check(lib.lik_maxsim_fwd_topk(C.byref(a), C.byref(t), _lib.stream_ptr(ws.device)), "lik_maxsim_fwd_topk")
+        base += size
+    want = torch.sort(reference(Q.float(), D.float(), mask)[0].sum(-1), dim=1, descending=True, stable=True)
+    assert torch.equal(s, want.values[:, :k]) and torch.equal(i, want.indices[:, :k])
