@@ -82,8 +82,6 @@ struct SharedCtl {
 // The lanes leave together, with one answer: TMEM loads, shuffles and rendezvous of the full warp follow, and nothing promises
 // that two lanes that probe a barrier get the same answer, or read the clock in the same cycle.  What every warp waits for
 // cannot pass by unseen: the phase after it needs this warp's arrival first, so an answer "complete" stays true.
-// The loop behind the first probe is inlined: a call would have the registers around it saved to local memory, and next to the
-// 204 KB of shared memory there is little L1 left to keep that.
 template <class Done>
 __device__ __forceinline__ bool wait_warp(Done done, SharedCtl* ctl, int* status) {
   if (__all_sync(0xffffffffu, done())) return true;
@@ -97,19 +95,27 @@ __device__ __forceinline__ bool wait_warp(Done done, SharedCtl* ctl, int* status
   }
   return true;
 }
+__device__ __noinline__ bool wait_bar_slow(uint32_t b, uint32_t parity, SharedCtl* ctl, int* status) {
+  return wait_warp([&] { return mbar_try_wait(b, parity); }, ctl, status);
+}
+// The loop behind the first probe is out of line, except (INLINE) in the epilogue that looks for winners: there a call would have
+// the registers around it saved to local memory, next to 204 KB of shared memory that leave little L1.
+template <bool INLINE = false>
 __device__ __forceinline__ bool wait_bar(unsigned long long* bar, uint32_t parity, SharedCtl* ctl, int* status) {
   const uint32_t b = smem_u32(bar);
-  return wait_warp([&] { return mbar_try_wait(b, parity); }, ctl, status);
+  if (INLINE) return wait_warp([&] { return mbar_try_wait(b, parity); }, ctl, status);
+  return __all_sync(0xffffffffu, mbar_try_wait(b, parity)) || wait_bar_slow(b, parity, ctl, status);
 }
 // until the producer has published entry `uc` of a unit ring
 __device__ __forceinline__ bool wait_posted(SharedCtl* ctl, int ln, int uc, int* status) {
   return wait_warp([&] { return ctl->units_posted[ln] > uc; }, ctl, status);
 }
 // Bounded rendezvous of the warps that share `bar` (initialised with their number); `n` counts this warp's uses of it.
+template <bool INLINE = false>
 __device__ __forceinline__ bool warps_sync(unsigned long long* bar, uint32_t& n, int lane, SharedCtl* ctl, int* status) {
   __syncwarp();
   if (lane == 0) mbar_arrive(smem_u32(bar));
-  return wait_bar(bar, n++ & 1, ctl, status);
+  return wait_bar<INLINE>(bar, n++ & 1, ctl, status);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -588,8 +594,8 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     long long warp_out = -1;  // aligned tiles: offset of this warp's query score for document 0
     int my_list = -1;         // top-k: the list whose state thread `et` loaded into shared memory
     int warp_seg = -1;        // aligned tiles: the query (segment) of this warp's rows
-#define LIK_SET_SYNC() warps_sync(&ctl->set_sync[set], n_sync, lane, ctl, P.status)
-#define LIK_WAIT_ACC() wait_bar(&ctl->acc_full[set], n_acc & 1, ctl, P.status)
+#define LIK_SET_SYNC() warps_sync<ARGMAX && !SCALED>(&ctl->set_sync[set], n_sync, lane, ctl, P.status)
+#define LIK_WAIT_ACC() wait_bar<ARGMAX && !SCALED>(&ctl->acc_full[set], n_acc & 1, ctl, P.status)
     // top-k: write the state of the lists this thread loaded back to their headers
 #define LIK_TOPK_STORE_BACK()                                                                          \
   do {                                                                                                 \
@@ -917,7 +923,7 @@ __global__ void streams_wait_probe_kernel(long long limit, int* status, int* res
     __syncwarp();
     uint32_t n = 0;
     const long long t0 = clock64();
-    const bool got = w == 0   ? wait_bar(&ctl.q_full, 0, &ctl, status)
+    const bool got = w == 0   ? wait_bar<true>(&ctl.q_full, 0, &ctl, status)
                      : w == 1 ? wait_posted(&ctl, 0, 0, status)
                               : warps_sync(&ctl.set_sync[0], n, (int)threadIdx.x, &ctl, status);
     const long long dt = clock64() - t0;
