@@ -214,8 +214,7 @@ __device__ __forceinline__ void unit_resolve(const TcParams& P, const UnitRaw& r
 }
 
 struct DocMaps {
-  CUtensorMap flat[N_BOXES];  // document boxes of 32, 64, 96 rows, one 128-byte slab wide
-  CUtensorMap deep[N_BOXES];  // the same with all slabs of the rows, slab behind slab (rows that fill their slabs)
+  CUtensorMap m[N_BOXES];  // document boxes of 32, 64, 96 rows, one 128-byte slab wide
 };
 
 // Word the producer leaves beside every ring stage for the MMA issuer.
@@ -224,7 +223,7 @@ constexpr uint32_t STAGE_ACC1 = 1u << 16;      // one resident tile: the piece g
 constexpr uint32_t STAGE_FIRST = 1u << 18;     // no piece: the query tiles change
 constexpr uint32_t STAGE_END = 1u << 20;       // no more work
 constexpr uint32_t STAGE_LONE = 1u << 21;      // the second accumulator has no query tile: it changes hands, nothing is multiplied into it
-constexpr uint32_t STAGE_WIDE = 1u << 22;      // the slabs lie a full stage apart instead of right behind each other
+constexpr uint32_t STAGE_SPLIT = 1u << 22;     // the last box of the stage does not follow the others: it ends where the document ends
 
 // WINNERS: 0 = scores only, 1 = winners saved, 2 = winners saved and every document takes the lazy winner scan (launched
 // for problems whose documents are long, so that the kernels for short documents carry no third copy of the tile loop)
@@ -271,7 +270,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     for (int i = 0; i < SETS; ++i) ctl->units_posted[i] = 0;
     fence_barrier_init();
     prefetch_tmap(&q_map);
-    for (int i = 0; i < N_BOXES; ++i) prefetch_tmap(P.d_deep ? &d_maps.deep[i] : &d_maps.flat[i]);
+    for (int i = 0; i < N_BOXES; ++i) prefetch_tmap(&d_maps.m[i]);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(&ctl->tmem_base), 512);
@@ -320,15 +319,11 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
             const uint32_t sc_bytes = SCALED && P.col_src ? (uint32_t)min((long long)((ncols + 3) & ~3), P.d.n_rows - row) * 4u : 0u;
             mbar_arrive_expect_tx(full, (uint32_t)(rows * SLAB_BYTES_ROW * n_slabs) + sc_bytes);
             const int box = rows / BOX_ROWS - 1;
-            if (!(info & STAGE_WIDE) && P.d_deep) {
-              tma_load_3d(dst, &d_maps.deep[box], 0, row, 0, full);
-            } else {
-              const bool split = info & STAGE_WIDE;
-              const uint32_t slab = (uint32_t)((split ? TILE_N : rows) * SLAB_BYTES_ROW);
-              for (int sl = 0; sl < n_slabs; ++sl) {
-                tma_load_2d(dst + sl * slab, &d_maps.flat[split ? box - 1 : box], sl * x_per_slab, row, full);
-                if (split) tma_load_2d(dst + sl * slab + box * BOX_ROWS * SLAB_BYTES_ROW, &d_maps.flat[0], sl * x_per_slab, row2, full);
-              }
+            const bool split = info & STAGE_SPLIT;
+            for (int sl = 0; sl < n_slabs; ++sl) {
+              const uint32_t at = dst + sl * TILE_N * SLAB_BYTES_ROW;
+              tma_load_2d(at, &d_maps.m[split ? box - 1 : box], sl * x_per_slab, row, full);
+              if (split) tma_load_2d(at + box * BOX_ROWS * SLAB_BYTES_ROW, &d_maps.m[0], sl * x_per_slab, row2, full);
             }
             if (sc_bytes) bulk_load_1d(smem_u32(sc_ring + slot * TILE_N), P.col_src + row, sc_bytes, full);
           } else {
@@ -415,7 +410,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           // A short document that is no multiple of 32 tokens takes two boxes, the second moved back to end where the document
           // ends; a longer one's last piece is moved back as a whole.
           const bool split = SHIFT && dlen < rows && dlen > BOX_ROWS;
-          stage((uint32_t)rows | lone | (j ? STAGE_ACC1 : 0u) | (split ? STAGE_WIDE : 0u), ncols,
+          stage((uint32_t)rows | lone | (j ? STAGE_ACC1 : 0u) | (split ? STAGE_SPLIT : 0u), ncols,
                 __shfl_sync(0xffffffffu, drow0 + (SHIFT ? max(min(c0, dlen - rows), 0) : c0), 0), __shfl_sync(0xffffffffu, drow0 + dlen - BOX_ROWS, 0),
                 SCALED ? ln * P.sc_per + slot : 0);
           if (SCALED && ++slot >= P.sc_per) slot = 0;
@@ -475,18 +470,18 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     const int k_steps = P.k_steps;
     constexpr uint32_t A_SLAB = (TILE_M * SLAB_BYTES_ROW) >> 4, B_SLAB = (TILE_N * SLAB_BYTES_ROW) >> 4;
     // the MMAs of one tile on one stage
-    auto multiply = [&](uint32_t acc, uint32_t tile, uint32_t rows, uint32_t b_stage, uint32_t b_slab) {
+    auto multiply = [&](uint32_t acc, uint32_t tile, uint32_t rows, uint32_t b_stage) {
       const uint32_t idesc = idesc0 | (rows << 14);  // N / 8 in bits 17..22
       const uint32_t d_tmem = d_tmem0 + acc * ACC_COLS, a_tmem = a_tmem0 + tile * A_COLS;
       // descriptors differ only in the start address, in units of 16 bytes
       if (k_steps == 8) {  // the common width (128 two-byte or 256 one-byte elements): straight-line issue
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          tc_mma_ts<FP8>(d_tmem, a_tmem + 8 * k, b_stage + (uint32_t)((k & 3) * 2) + (k >> 2) * b_slab, desc_hi, idesc, k ? 1u : 0u);
+          tc_mma_ts<FP8>(d_tmem, a_tmem + 8 * k, b_stage + (uint32_t)((k & 3) * 2) + (k >> 2) * B_SLAB, desc_hi, idesc, k ? 1u : 0u);
       } else {
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          if (k < k_steps) tc_mma_ts<FP8>(d_tmem, a_tmem + 8 * k, b_stage + (uint32_t)((k & 3) * 2) + (k >> 2) * b_slab, desc_hi, idesc, k ? 1u : 0u);
+          if (k < k_steps) tc_mma_ts<FP8>(d_tmem, a_tmem + 8 * k, b_stage + (uint32_t)((k & 3) * 2) + (k >> 2) * B_SLAB, desc_hi, idesc, k ? 1u : 0u);
       }
     };
     while (true) {
@@ -529,7 +524,6 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
       }
       const uint32_t rows = info & STAGE_COLS_MASK;
       const uint32_t b_stage = b_desc0 + st * stage_desc;
-      const uint32_t b_slab = info & STAGE_WIDE ? B_SLAB : rows * (SLAB_BYTES_ROW >> 4);
       if (info & STAGE_FIRST) {
         // (a stage that only announced them: nobody else gives it back)
         if (issue) mbar_arrive(smem_u32(&d_empty[st]));
@@ -538,7 +532,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         if (!wait_bar(&acc_empty[0], acc_ph & 1u, ctl, P.status)) break;
         tc_fence_after();
         if (issue) {
-          if (rows) multiply(0, 0, rows, b_stage, b_slab);
+          if (rows) multiply(0, 0, rows, b_stage);
           tc_commit(smem_u32(&acc_full[0]));
         }
         __syncwarp();
@@ -546,7 +540,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         acc_ph ^= 3u;
         tc_fence_after();
         if (issue) {
-          if (rows && !(info & STAGE_LONE)) multiply(1, 1, rows, b_stage, b_slab);
+          if (rows && !(info & STAGE_LONE)) multiply(1, 1, rows, b_stage);
           tc_commit(smem_u32(&acc_full[1]));
           tc_commit(smem_u32(&d_empty[st]));  // ring slot reusable once these MMAs retire
         }
@@ -556,7 +550,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         acc_ph ^= 1u << a;
         tc_fence_after();
         if (issue) {
-          if (rows) multiply(a, 0, rows, b_stage, b_slab);
+          if (rows) multiply(a, 0, rows, b_stage);
           tc_commit(smem_u32(&acc_full[a]));
           tc_commit(smem_u32(&d_empty[st]));
         }
@@ -967,17 +961,13 @@ int launch_streams_wait_probe(long long limit, int* status, int* result, cudaStr
   return LIK_OK;
 }
 
-int launch_fwd_streams(const lik_fwd_args& a, const TcPlan& pl, const TcParams& P0, bool affine, bool long_docs, cudaStream_t st) {
-  TcParams P = P0;
-  P.d_deep = a.dim * (int)dtype_size(a.dtype) == pl.n_slabs * SLAB_BYTES_ROW;
+int launch_fwd_streams(const lik_fwd_args& a, const TcPlan& pl, const TcParams& P, bool affine, bool long_docs, cudaStream_t st) {
   CUtensorMap q_map;
   DocMaps d_maps;
   memset(&d_maps, 0, sizeof(d_maps));
   int rc = make_tmap_rows(&q_map, a.q.data, a.dtype, a.dim, a.q.n_rows, a.q.row_stride, TILE_M);
-  for (int i = 0; i < N_BOXES && !rc; ++i) {
-    rc = make_tmap_rows(&d_maps.flat[i], a.d.data, a.dtype, a.dim, a.d.n_rows, a.d.row_stride, (i + 1) * BOX_ROWS);
-    if (!rc && P.d_deep) rc = make_tmap_rows(&d_maps.deep[i], a.d.data, a.dtype, a.dim, a.d.n_rows, a.d.row_stride, (i + 1) * BOX_ROWS, pl.n_slabs);
-  }
+  for (int i = 0; i < N_BOXES && !rc; ++i)
+    rc = make_tmap_rows(&d_maps.m[i], a.d.data, a.dtype, a.dim, a.d.n_rows, a.d.row_stride, (i + 1) * BOX_ROWS);
   if (rc) return rc;
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -1162,8 +1162,7 @@ EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// `slabs` 0: a map over the rows, one slab wide; otherwise rows x slabs, whose boxes hold all slabs of their rows
-int make_map(CUtensorMap* map, const lik_seqs& s, int dtype, int dim, int box_rows, int slabs = 0) {
+int make_map(CUtensorMap* map, const lik_seqs& s, int dtype, int dim, int box_rows) {
   EncodeTiledFn enc = get_encode_fn();
   if (!enc) {
     set_error("cuTensorMapEncodeTiled is not available from this driver");
@@ -1173,12 +1172,11 @@ int make_map(CUtensorMap* map, const lik_seqs& s, int dtype, int dim, int box_ro
   CUtensorMapDataType dt = dtype == LIK_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                            : dtype == LIK_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                               : CU_TENSOR_MAP_DATA_TYPE_UINT8;
-  const cuuint32_t slab_elems = (cuuint32_t)(SLAB_BYTES_ROW / eb);
-  cuuint64_t gdim[3] = {slabs ? (cuuint64_t)slab_elems : (cuuint64_t)dim, (cuuint64_t)(s.n_rows > 0 ? s.n_rows : 1), (cuuint64_t)slabs};
-  cuuint64_t gstride[2] = {(cuuint64_t)s.row_stride * eb, (cuuint64_t)SLAB_BYTES_ROW};
-  cuuint32_t box[3] = {slab_elems, (cuuint32_t)box_rows, (cuuint32_t)slabs};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(map, dt, slabs ? 3 : 2, const_cast<void*>(s.data), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  cuuint64_t gdim[2] = {(cuuint64_t)dim, (cuuint64_t)(s.n_rows > 0 ? s.n_rows : 1)};
+  cuuint64_t gstride[1] = {(cuuint64_t)s.row_stride * eb};
+  cuuint32_t box[2] = {(cuuint32_t)(SLAB_BYTES_ROW / eb), (cuuint32_t)box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = enc(map, dt, 2, const_cast<void*>(s.data), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     set_error("cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
@@ -1334,12 +1332,12 @@ bool fwd_tc_supported(const lik_fwd_args& a) { return tc_problem_ok(a, false); }
 // Helpers shared with the document-head kernel: a 128-byte-swizzled TMA map over the rows of a matrix whose box is
 // one 128-byte K slab wide and `box_rows` high, and the effective document lengths under a token mask.
 int make_tmap_rows(CUtensorMap* map, const void* data, int dtype, long long inner, long long n_rows, long long row_stride,
-                   int box_rows, int slabs) {
+                   int box_rows) {
   lik_seqs s{};
   s.data = data;
   s.n_rows = n_rows;
   s.row_stride = row_stride;
-  return make_map(map, s, dtype, (int)inner, box_rows, slabs);
+  return make_map(map, s, dtype, (int)inner, box_rows);
 }
 bool tmap_available() { return get_encode_fn() != nullptr; }
 // The fused top-k needs fixed query slots (padded queries of at most 128 tokens) and k within the list size.

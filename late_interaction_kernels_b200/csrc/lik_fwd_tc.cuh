@@ -88,7 +88,6 @@ struct TcParams {
   const float* col_src;  // nullptr: the epilogue stages the multipliers itself
   int sc_per, sc_slots;  // slots per ring, and of all rings (0: the epilogue stages the multipliers)
   float norm_eps;     // > 0: the kernel takes the documents' inverse norms from the tiles themselves
-  int d_deep;         // the documents' rows fill their slabs: one copy brings all slabs of a piece
   TopkOut topk;       // cand_key == nullptr: scores are written instead
   PlaidSrc plaid;     // PLAID kernels: the compressed documents
   int plaid_f16;      // PLAID kernels: operand type fp16 instead of bf16

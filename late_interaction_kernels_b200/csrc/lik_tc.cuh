@@ -38,7 +38,7 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
 // Shared with the document-head kernel (lik_head.cu).
 constexpr int LEN_FLAG_MASKED = 1 << 30;  // effective length of a document whose mask is not a plain prefix
 int make_tmap_rows(CUtensorMap* map, const void* data, int dtype, long long inner, long long n_rows, long long row_stride,
-                   int box_rows, int slabs = 0);
+                   int box_rows);
 bool tmap_available();
 
 }  // namespace lik
