@@ -47,7 +47,8 @@ constexpr int EPI_WARP0 = 2;        // 16 epilogue warps; 0 and 1 load and issue
 constexpr int UNIT_RING = 16;       // slots of a producer -> epilogue unit ring: more than ring stages + 2
 constexpr int UNIT_END = 1 << 31;   // unit_info.x, the sign bit: the entry behind the last unit
 
-// Rings of multiplier slots: sc_per = stages + 1 slots per accumulator (per stream, where both accumulators take every piece).
+// Rings of multiplier slots: sc_per = stages + 1 slots per stream (they arrive with the pieces only where both of its accumulators
+// take every piece).
 // The slot of piece n is refilled for piece n + sc_per: by then the MMAs of piece n + 1 have completed (the producer is at most
 // `stages` pieces ahead of the tensor pipe), which needed the accumulator(s) back from piece n - and an epilogue gives an
 // accumulator back only after its last read of the multipliers.
@@ -242,7 +243,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
   const int d_stage_bytes = P.n_slabs * TILE_N * SLAB_BYTES_ROW;
   unsigned char* q_smem = smem;                              // [n_slabs][128 rows][128 B], a tile on its way to tensor memory
   unsigned char* d_smem = smem + q_tile_bytes;               // [2 streams][stages][n_slabs][rows][128 B]
-  float* sc_ring = reinterpret_cast<float*>(d_smem + (size_t)2 * P.stages * d_stage_bytes);  // [SETS][sc_per][TILE_N] (kernels with multipliers)
+  float* sc_ring = reinterpret_cast<float*>(d_smem + (size_t)2 * P.stages * d_stage_bytes);  // [2 streams][sc_per][TILE_N] (kernels with multipliers)
   SharedCtl* ctl = reinterpret_cast<SharedCtl*>(d_smem + (size_t)2 * P.stages * d_stage_bytes + (size_t)P.sc_slots * TILE_N * sizeof(float));
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -302,7 +303,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     unsigned long long *const d_full = ctl->d_full[sm], *const d_empty = ctl->d_empty[sm];
     int cur_grp = -1;
     uint32_t n_qload = 0, st = 0, ph = 0, n_dload = 0, lone = 0;
-    int n_unit[2] = {0, 0}, n_slot[2] = {0, 0}, turn = 0;  // by accumulator (one resident tile) or the first alone (two)
+    int n_unit[2] = {0, 0}, n_slot = 0, turn = 0;  // units by accumulator (one resident tile) or the first alone (two)
     bool ok = true;
     // One stage: `rows` of `ncols` document rows from `row` on; split: two boxes, the second at row2
     auto stage = [&](uint32_t info, int ncols, int row, int row2, int slot) {
@@ -393,7 +394,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         turn ^= 1;
         // publish the unit for the epilogue; an empty document still sends one (empty) piece so that every unit passes through
         // the same hand-shakes
-        int slot = SCALED ? (j ? n_slot[1] : n_slot[0]) : 0;
+        int slot = n_slot;
         if (elect) {
           const int at = j ? n_unit[1] : n_unit[0];
           ctl->unit_info[ln][at & (UNIT_RING - 1)] = make_int4(dlen | slot << UNIT_SLOT_SHIFT | (len & LEN_FLAG_MASKED), drow0, grp, doc);
@@ -412,12 +413,11 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
           const bool split = SHIFT && dlen < rows && dlen > BOX_ROWS;
           stage((uint32_t)rows | lone | (j ? STAGE_ACC1 : 0u) | (split ? STAGE_SPLIT : 0u), ncols,
                 __shfl_sync(0xffffffffu, drow0 + (SHIFT ? max(min(c0, dlen - rows), 0) : c0), 0), __shfl_sync(0xffffffffu, drow0 + dlen - BOX_ROWS, 0),
-                SCALED ? ln * P.sc_per + slot : 0);
+                SCALED ? sm * P.sc_per + slot : 0);
           if (SCALED && ++slot >= P.sc_per) slot = 0;
           c0 += TILE_N;
         } while (ok && c0 < dlen);
-        if (j) n_slot[1] = slot;
-        else n_slot[0] = slot;
+        n_slot = slot;
       }
     }
     if (ok) {
@@ -573,7 +573,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     const int row = quad * 32 + lane;        // accumulator row == query token slot in the tile
     const int et = wq * 32 + lane;           // thread index inside the set (0..127)
     const int sm = set >> 1;                 // stream
-    const int ln = P.mt == 2 ? set & 2 : set;  // whose unit ring and multiplier slots
+    const int ln = P.mt == 2 ? set & 2 : set;  // whose unit ring
     const int my_tile = P.mt == 2 ? set & 1 : 0;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(set * ACC_COLS);
     const uint32_t acc_empty_bar = smem_u32(&ctl->acc_empty[set]);
@@ -757,7 +757,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
         float* const col_scale = ctl->col_scale[set][n_col & 1];
         float* const col_bias = ctl->col_bias[set][n_col & 1];
         const bool staged = general || (SCALED && !bulk);
-        const float* const sc_arr = SCALED && bulk ? sc_ring + (ln * P.sc_per + sc_slot) * TILE_N : col_scale;
+        const float* const sc_arr = SCALED && bulk ? sc_ring + (sm * P.sc_per + sc_slot) * TILE_N : col_scale;
         auto stage_columns = [&]() {
           ++n_col;
           const int c = et;  // a thread per column

@@ -1286,7 +1286,7 @@ TcPlan plan_tc(const lik_fwd_args& a, const TcExtra& x) {
   const size_t fixed = pl.streams ? fwd_streams_fixed_smem(pl.n_slabs) : q_bytes + sizeof(SharedCtl) + 1024;
   pl.stage_bytes = stage;
   pl.slot_bytes = pl.streams ? fwd_streams_slot_bytes() : TILE_N * sizeof(float);
-  pl.rings = pl.lists = pl.streams ? 4 : 2;
+  pl.lists = pl.streams ? 4 : 2;
   const size_t budget = 227 * 1024;
   int st = (int)((budget - fixed) / stage);
   pl.stages = st > 8 ? 8 : st;
@@ -1474,10 +1474,11 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
   P.norm_eps = norm_d_eps;
   if (norm_d_eps > 0.f || (!plaid && !a.d.cu && a.d.scale_scalar == 1.0f && ((a.d.scale != nullptr) != (dn != nullptr)))) {
     const float* arr = a.d.scale ? a.d.scale : dn;
-    if (norm_d_eps > 0.f || (((uintptr_t)arr & 15) == 0 && a.d.seq_stride % 4 == 0 && a.d.n_rows % 4 == 0)) {
+    // (the streams kernel has a ring per stream, which goes with both accumulators of a stream taking every piece)
+    if (norm_d_eps > 0.f || (!(pl.streams && pl.mt == 1) && ((uintptr_t)arr & 15) == 0 && a.d.seq_stride % 4 == 0 && a.d.n_rows % 4 == 0)) {
       const size_t stage = pl.stage_bytes;
       const size_t fixed = pl.smem_bytes - (size_t)pl.stages * stage;
-      auto need = [&](int stages) { return fixed + (size_t)stages * stage + (size_t)pl.rings * (stages + 1) * pl.slot_bytes; };
+      auto need = [&](int stages) { return fixed + (size_t)stages * stage + (size_t)2 * (stages + 1) * pl.slot_bytes; };
       int stages = pl.stages;
       while (stages > 1 && need(stages) > (size_t)227 * 1024) --stages;
       if (need(stages) <= (size_t)227 * 1024) {
@@ -1486,7 +1487,7 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
         P.stages = stages;
         P.col_src = arr;
         P.sc_per = stages + 1;
-        P.sc_slots = pl.rings * P.sc_per;
+        P.sc_slots = 2 * P.sc_per;
       }
     }
     if (norm_d_eps > 0.f) P.col_src = nullptr;

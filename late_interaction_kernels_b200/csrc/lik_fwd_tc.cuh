@@ -17,7 +17,6 @@ struct TcPlan {
   int grid;
   size_t smem_bytes;
   int lists;        // candidate lists of a query's place per list slot (fused top-k)
-  int rings;        // rings of multiplier slots
   size_t stage_bytes, slot_bytes;  // shared memory per ring stage / per multiplier slot
 };
 
@@ -86,7 +85,7 @@ struct TcParams {
   // allows it travel with the tile: the producer copies the tile's run of them into a slot of a small ring in shared
   // memory (bulk copy on the stage's barrier) instead of the epilogue fetching them from device memory per tile.
   const float* col_src;  // nullptr: the epilogue stages the multipliers itself
-  int sc_per, sc_slots;  // slots per ring, and of all rings (0: the epilogue stages the multipliers)
+  int sc_per, sc_slots;  // slots per ring, and of both rings (0: the epilogue stages the multipliers)
   float norm_eps;     // > 0: the kernel takes the documents' inverse norms from the tiles themselves
   TopkOut topk;       // cand_key == nullptr: scores are written instead
   PlaidSrc plaid;     // PLAID kernels: the compressed documents
