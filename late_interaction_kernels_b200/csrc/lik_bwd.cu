@@ -2046,7 +2046,7 @@ int run_bwd(const lik_bwd_args& a, BwdParams& P, const BwdPlan& pl, cudaStream_t
       O.tok_cnt = (int*)(ws + pl.cnt_off);
       O.clear_rest = pl.sort_clears;
       auto kernel = winners_in_quads(a) ? bwd_dd_sort4_kernel : bwd_dd_sort_kernel;
-      if (pl.sort_smem > 48 * 1024) LIK_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.sort_smem));
+      if (pl.sort_smem > 48 * 1024) LIK_CUDA_OK(winners_in_quads(a) ? allow_smem<bwd_dd_sort4_kernel>() : allow_smem<bwd_dd_sort_kernel>());
       cudaLaunchAttribute attr{};
       attr.id = cudaLaunchAttributeClusterDimension;
       attr.val.clusterDim.x = (unsigned)pl.sort_cluster;

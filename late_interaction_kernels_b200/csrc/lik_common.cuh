@@ -6,6 +6,7 @@
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -35,6 +36,25 @@ const char* get_error();
       return LIK_ERR_INVALID;         \
     }                                 \
   } while (0)
+
+// Raise a kernel's limit of dynamic shared memory to the most that a block can have, once per device: a host call of a microsecond
+// or two that small problems feel.  Host threads that come here at the same time set the same value, so none can lower the
+// limit between another's look and its launch (with a limit per size they could).
+template <auto KERNEL>
+cudaError_t allow_smem() {
+  constexpr int BLOCK_SMEM = 227 * 1024;
+  static std::atomic<uint64_t> devices{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = dev >= 0 && dev < 64 ? 1ull << dev : 0;
+  if (devices.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  cudaFuncAttributes fa;
+  e = cudaFuncGetAttributes(&fa, KERNEL);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, BLOCK_SMEM - (int)fa.sharedSizeBytes);
+  if (e == cudaSuccess) devices.fetch_or(bit, std::memory_order_release);
+  return e;
+}
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }

@@ -934,16 +934,8 @@ __global__ void streams_wait_probe_kernel(long long limit, int* status, int* res
 
 template <bool F, int A, bool X>
 cudaError_t launch_one(const cudaLaunchConfig_t& cfg, const CUtensorMap& q_map, const DocMaps& d_maps, const TcParams& P) {
-  // the limit is raised once per device and size: a host call of a microsecond or two that small problems feel
-  static size_t allowed[64] = {0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  cudaError_t e = allow_smem<fwd_streams_kernel<F, A, X>>();
   if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64 || allowed[dev] < cfg.dynamicSmemBytes) {
-    e = cudaFuncSetAttribute(fwd_streams_kernel<F, A, X>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64) allowed[dev] = cfg.dynamicSmemBytes;
-  }
   e = cudaLaunchKernelEx(&cfg, fwd_streams_kernel<F, A, X>, q_map, d_maps, P);
   count_launch();
   return e;

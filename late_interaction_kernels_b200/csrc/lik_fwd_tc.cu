@@ -1397,20 +1397,6 @@ int launch_topk_slots(const float* keys, const int* idx, const int2* hdr, long l
                       int mt, int lists, int qpt, long long n_q, int k, int largest, long long index_offset, float* out_scores,
                       long long* out_index, int parts, void* part_buf, cudaStream_t st);
 
-// Raise the kernel's dynamic shared memory limit once per device and size instead of on every launch (a host call
-// of a microsecond or two that small problems feel).
-template <bool F, int A, bool X, bool PL>
-static cudaError_t allow_smem(size_t bytes) {
-  static size_t allowed[64] = {0};  // by device ordinal
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev >= 0 && dev < 64 && allowed[dev] >= bytes) return cudaSuccess;
-  e = cudaFuncSetAttribute(fwd_tc_kernel<F, A, X, PL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess && dev >= 0 && dev < 64) allowed[dev] = bytes;
-  return e;
-}
-
 bool fwd_tc_norms_in_kernel(const lik_fwd_args& a, const TcExtra& x) {
   const TcPlan pl = plan_tc(a, x);
   return pl.stages >= 2 && norms_from_tiles(a, x, pl);
@@ -1567,7 +1553,7 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
     cfg.numAttrs = 1;
 #define LIK_TC_LAUNCH(F, A, X, PL)                                                                                     \
     do {                                                                                                                 \
-      LIK_CUDA_OK((allow_smem<F, A, X, PL>(pl.smem_bytes)));                                                             \
+      LIK_CUDA_OK((allow_smem<fwd_tc_kernel<F, A, X, PL>>()));                                                           \
       LIK_CUDA_OK(cudaLaunchKernelEx(&cfg, fwd_tc_kernel<F, A, X, PL>, q_map, d_maps, P));                               \
       ::lik::count_launch();                                                                                             \
     } while (0)

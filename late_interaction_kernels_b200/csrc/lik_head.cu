@@ -743,16 +743,8 @@ extern "C" int lik_maxsim_hidden_fwd(const lik_hidden_fwd_args* args, lik_stream
   // positions of the saved winners that no accumulator row covers
   if (a.argmax && a.argmax_stride > a.q.max_len)
     LIK_CUDA_OK(cudaMemsetAsync(a.argmax, 0xFF, (size_t)a.q.n_seq * a.h.n_seq * a.argmax_stride * sizeof(int), st));
-  static size_t allowed[2][64] = {{0}};
-  int dev = 0;
-  LIK_CUDA_OK(cudaGetDevice(&dev));
-  const int v = a.argmax ? 1 : 0;
-  if (dev < 0 || dev >= 64 || allowed[v][dev] < pl.smem_bytes) {
-    if (v) LIK_CUDA_OK(cudaFuncSetAttribute(head_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem_bytes));
-    else LIK_CUDA_OK(cudaFuncSetAttribute(head_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem_bytes));
-    if (dev >= 0 && dev < 64) allowed[v][dev] = pl.smem_bytes;
-  }
-  if (v) head_tc_kernel<true><<<pl.grid, HD_THREADS, pl.smem_bytes, st>>>(q_map, h_map, w_map, P), ::lik::count_launch();
+  LIK_CUDA_OK(a.argmax ? allow_smem<head_tc_kernel<true>>() : allow_smem<head_tc_kernel<false>>());
+  if (a.argmax) head_tc_kernel<true><<<pl.grid, HD_THREADS, pl.smem_bytes, st>>>(q_map, h_map, w_map, P), ::lik::count_launch();
   else head_tc_kernel<false><<<pl.grid, HD_THREADS, pl.smem_bytes, st>>>(q_map, h_map, w_map, P), ::lik::count_launch();
   LIK_CUDA_OK(cudaGetLastError());
   return LIK_OK;
