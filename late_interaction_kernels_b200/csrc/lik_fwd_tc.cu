@@ -529,13 +529,13 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
             const bool wrapped = i > st;  // that use lies before the last wrap of the ring
             const uint32_t slot = wrapped ? st + (uint32_t)P.stages - i : st - i;
             const uint32_t bar = smem_u32(&ctl->d_full[slot]);
-            for (int spin = 0; spin < (1 << 16) && !mbar_try_wait(bar, wrapped ? ph ^ 1 : ph); ++spin) {
+            for (int spin = 0; spin < (1 << 16) && !mbar_try_wait_long(bar, wrapped ? ph ^ 1 : ph); ++spin) {
             }
           }
         }
         if (n_qload) {
           const uint32_t bar = smem_u32(&ctl->q_full);
-          for (int spin = 0; spin < (1 << 16) && !mbar_try_wait(bar, (n_qload - 1) & 1); ++spin) {
+          for (int spin = 0; spin < (1 << 16) && !mbar_try_wait_long(bar, (n_qload - 1) & 1); ++spin) {
           }
         }
       }

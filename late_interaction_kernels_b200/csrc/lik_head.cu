@@ -101,7 +101,7 @@ struct HeadCtl {
 __device__ __noinline__ bool hd_wait_slow(uint32_t b, uint32_t parity, HeadCtl* ctl, int* status) {
   const long long t0 = clock64();
   while (true) {
-    if (mbar_try_wait(b, parity)) return true;
+    if (mbar_try_wait_long(b, parity)) return true;
     if (ctl->abort_flag) return false;
     if (clock64() - t0 > ctl->wait_limit) {
       ctl->abort_flag = 1;
@@ -112,7 +112,7 @@ __device__ __noinline__ bool hd_wait_slow(uint32_t b, uint32_t parity, HeadCtl* 
 }
 __device__ __forceinline__ bool hd_wait(unsigned long long* bar, uint32_t parity, HeadCtl* ctl, int* status) {
   const uint32_t b = smem_u32(bar);
-  if (mbar_try_wait(b, parity)) return true;
+  if (mbar_try_wait_long(b, parity)) return true;
   return hd_wait_slow(b, parity, ctl, status);
 }
 
@@ -308,11 +308,11 @@ head_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
           const bool wrapped = i > st;
           const uint32_t slot = wrapped ? st + (uint32_t)P.stages - i : st - i;
           const uint32_t bar = smem_u32(&ctl->ring_full[slot]);
-          for (int spin = 0; spin < (1 << 16) && !mbar_try_wait(bar, wrapped ? ph ^ 1 : ph); ++spin) {
+          for (int spin = 0; spin < (1 << 16) && !mbar_try_wait_long(bar, wrapped ? ph ^ 1 : ph); ++spin) {
           }
         }
         const uint32_t qbar = smem_u32(&ctl->q_full);
-        for (int spin = 0; spin < (1 << 16) && !mbar_try_wait(qbar, 0); ++spin) {
+        for (int spin = 0; spin < (1 << 16) && !mbar_try_wait_long(qbar, 0); ++spin) {
         }
       }
     }
