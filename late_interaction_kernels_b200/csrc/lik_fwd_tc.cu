@@ -38,6 +38,8 @@
 
 namespace lik {
 
+int topk_merge_parts(int n_ctas, int n_groups, int per_slot);
+
 namespace {
 
 #ifndef LIK_TILE_N
@@ -1197,16 +1199,6 @@ static size_t sb_window_bytes() {
   return v;
 }
 
-// Which kernel.  The one with two streams per CTA needs more work per CTA to pay for its longer start (a stage that announces the
-// query tiles, their way through shared memory to tensor memory): STREAMS_UNITS units per CTA, which few problems have that take
-// less than 30 us.  It takes no norms from the tiles and decodes no index; with one resident tile, per-column multipliers
-// that arrive with the tiles are the other kernel's (4 queries x 4096 documents of 256 tokens in e4m3: 43 against 53 us; two tiles
-// and 16 queries 135 against 114).  The candidate lists of a fused
-// top-k are laid out for one kernel: the pieces of a corpus go where LIK_TOPK_LARGE says, never by a piece's own size.
-// A pair list changes its query tile with every query: where documents take more than two pieces of 96 tokens it needs more units
-// (3001 pairs of 61 queries and 300-token documents 36.6 us there, 35.5 here; 10 000 pairs 88 to 97; 3001 of 64 tokens 18 to 23).
-constexpr long long STREAMS_UNITS = 12, STREAMS_PAIRS = 32;
-
 // A launch that reads every document up to four times takes the documents' norms from its tiles instead of one pass of
 // prep_kernel in front.  A query of 32 tokens against 1000 documents of up to 300 40 -> 30 us; two groups of query tiles (12 x 32
 // against 8000 of 300) 407 -> 308, (4 x 128 against 8000 of 1030) 1498 -> 953; 128-token queries against 4000 documents of up
@@ -1224,6 +1216,40 @@ size_t topk_list_bytes(int n_groups, int per_slot) {
 // The streams kernel keeps twice as many of them, which is a matter of megabytes for the batches that wait for an answer (256
 // queries of 32 tokens: 6 MB).  Beyond this the other kernel runs: 100 000 queries would take 414 MB instead of 207.
 constexpr size_t STREAMS_LISTS_BYTES = 128u << 20;
+
+// Which kernel takes a problem that both can: true for the one with two streams per CTA.  Times in us, the other kernel / streams,
+// bf16, 128 features, queries of 32 tokens, document lengths spread from a fifth of the longest to the longest unless said otherwise;
+// "units" are per SM.  What the streams kernel loses by: a longer start (query tiles on their way through shared to tensor memory),
+// the same way again with both streams idle whenever the query tiles change, and documents of more than 100 up to 256
+// tokens, which are two or three pieces there and one tile in the other kernel.
+bool streams_pay(const lik_fwd_args& a, const TcExtra& x, const TcPlan& pl, bool multipliers) {
+  const long long sms = sm_count(), len = a.d.max_len;
+  const bool two = pl.mt == 2, list = a.pairing == LIK_PAIR_LIST;
+  const bool brief = len <= 100, middle = !brief && len <= 256;
+  // Plain scores of documents that are all of one length and fill their last tile of 256: 64 queries x 445 documents of 256 tokens
+  // 53.7 / 55.2, of 512 84.6 / 87.6 (of 300: 76.2 / 62.5; of 700 even).
+  if (!a.argmax && !multipliers && !a.d.cu && !a.d.lens && !a.d.mask && (len - 1) % 256 + 1 > 192) return false;
+  // Units.  One query x documents of 64 tokens: 6 units 13.8 / 13.0, 12 17.2 / 14.0; of 192: 12 units 18.5 / 19.2, 24 32.6 / 27.3; of
+  // 256: 16 units 26.2 / 26.5, 24 36.8 / 34.9; of 300: 12 1.03 to 1.17.  Two tiles, 64 queries x documents of 256: 8 units 23.4 /
+  // 23.9, 12 29.5 / 29.3, with winners 34.4 / 32.2.  A pair list reads its table besides: 256 queries, documents of 300 tokens: 16 units
+  // 31.6 / 32.8, 32 47.5 / 46.9, 48 65.2 / 60.8; of 200 tokens 48 units 0.99, 96 1.09; of 256 0.89 and 0.95.
+  long long units = middle && !two ? 24 : 12;
+  if (list && !brief) units = middle ? 96 : 32;
+  // Units per change of the query tiles.  One tile, candidate lists with winners, 12 units, of 300 tokens: 1 per query 49.6 / 56.4, 2 (one for
+  // either stream) 40.8 / 40.6 (of 512 1.10), 3 0.93, 4 35.1 / 36.5 (of 512 1.03), 6 1.04, 8 35.6 / 32.8; of 192 tokens, 24 units: 1 62.9 /
+  // 77.4, 4 44.0 / 50.5, 8 39.0 / 40.9, 12 37.6 / 38.2, 16 37.6 / 36.4.  Two tiles, 12 units: documents of 64 tokens: 1 42.6 / 48.6, 2 35.7 / 29.8, 3
+  // 0.94 to 1.09, 4 29.7 / 25.6; of 300: 2 0.88 to 0.98, 4 0.95 to 1.01, 6 39.9 / 37.7, 8 42.2 / 39.6.
+  const long long have = a.pairing == LIK_PAIR_CROSS ? a.d.n_seq : list ? a.n_pairs / a.q.n_seq : a.group;
+  const long long run = two ? (brief ? 4 : 8) : brief ? 1 : middle ? 12 : 6;
+  if (have < run && !(have == 2 && (two ? brief : !middle))) return false;
+  // Twice the candidate lists may need one more pass to merge (about 15 us): 40 queries over 500 documents of 180 tokens (17 units)
+  // 51.5 / 59.1, 1000 (34) 77.4 / 79.5, 2000 (68) 126.3 / 108.9; of 1030 tokens 0.91 to 0.98 at any size.
+  if (x.topk_k > 0 && topk_merge_parts((int)sms, pl.n_groups, 2 / pl.mt) == 1 && topk_merge_parts((int)sms, pl.n_groups, 4 / pl.mt) > 1) {
+    if (len > 512) return false;
+    units = 40;
+  }
+  return pl.n_units_total >= units * sms;
+}
 
 TcPlan plan_tc(const lik_fwd_args& a, const TcExtra& x) {
   TcPlan pl{};
@@ -1273,10 +1299,13 @@ TcPlan plan_tc(const lik_fwd_args& a, const TcExtra& x) {
   const bool norms = norms_from_tiles(a, x, pl);
   const bool multipliers = a.d.scale || ((a.normalize & LIK_NORM_D) && !x.plaid);
   const bool bulk = multipliers && !a.d.cu && a.d.seq_stride % 4 == 0 && a.d.n_rows % 4 == 0;
+  // It takes no norms from the tiles and decodes no index; with one resident tile, per-column multipliers that arrive with the tiles
+  // are the other kernel's (4 queries x 4096 documents of 256 tokens in e4m3: 43 against 53 us).  The candidate lists of a fused
+  // top-k are laid out for one kernel: the pieces of a corpus go where LIK_TOPK_LARGE says, never by a piece's own size.
   const bool pieces = x.topk_flags & (LIK_TOPK_CONTINUE | LIK_TOPK_PARTIAL);
   pl.streams = !x.small_lists && !x.plaid && !norms && !(multipliers && pl.mt == 1 && (bulk || x.topk_k > 0)) &&
-               (x.topk_k > 0 ? (!pieces || (x.topk_flags & LIK_TOPK_LARGE)) && topk_list_bytes(pl.n_groups, 4 * pl.q_per_tile) <= STREAMS_LISTS_BYTES
-                             : pl.n_units_total >= (a.pairing == LIK_PAIR_LIST && a.d.max_len > 192 ? STREAMS_PAIRS : STREAMS_UNITS) * sm_count());
+               (x.topk_k == 0 || topk_list_bytes(pl.n_groups, 4 * pl.q_per_tile) <= STREAMS_LISTS_BYTES) &&
+               (pieces ? (x.topk_flags & LIK_TOPK_LARGE) != 0 : streams_pay(a, x, pl, multipliers));
   const long long g = pl.n_units_total < sm_count() ? pl.n_units_total : sm_count();
   pl.grid = (int)(g < 0 ? 0 : g);
   // the fused top-k numbers its candidate lists by CTA: the same grid whatever the piece of the corpus
@@ -1352,8 +1381,6 @@ bool fwd_tc_plaid_supported(const lik_fwd_args& a, const TcExtra& x) {
   if (x.plaid->dim != a.dim || a.dim % 16 != 0 || a.dim > 128 || a.d.mask || a.d.scale) return false;
   return plaid_row16_ok(*x.plaid);
 }
-
-int topk_merge_parts(int n_ctas, int n_groups, int per_slot);
 
 namespace {
 struct TcWs {

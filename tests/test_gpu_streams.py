@@ -250,3 +250,80 @@ def test_topk_in_pieces_of_different_sizes(Nq, large):
         base += size
     want = torch.sort(reference(Q.float(), D.float(), mask)[0].sum(-1), dim=1, descending=True, stable=True)
     assert torch.equal(s, want.values[:, :k]) and torch.equal(i, want.indices[:, :k])
+
+
+def route(Nq, Nd, Lq, Ld, *, masked=True, winners=False, k=0, group=0, n_pairs=0, queries=0, normalize=0, dtype=torch.bfloat16, scaled=False):
+    """The kernel that a call goes to by itself (only its sizes are looked at)."""
+    import ctypes as C
+
+    from late_interaction_kernels_b200 import _lib
+
+    lib = _lib.load()
+    x = torch.zeros(16, device="cuda")
+
+    def side(n, length):
+        return _lib.Seqs(data=x.data_ptr(), row_stride=128, n_rows=n * length, n_seq=n, max_len=length, seq_stride=length, cu=None, lens=None, mask=None,
+                         scale=x.data_ptr() if scaled else None, scale_scalar=1.0, reserved=0)
+
+    q, d = side(Nq, Lq), side(Nd, Ld)
+    if masked:
+        d.lens = x.data_ptr()
+    a = _lib.FwdArgs(
+        q=q, d=d, dtype=_lib.lik_dtype(dtype), dim=128, pairing=_lib.PAIR_GROUPED if group else _lib.PAIR_LIST if n_pairs else _lib.PAIR_CROSS, group=group,
+        pair_q=x.data_ptr(), pair_d=x.data_ptr(), n_pairs=n_pairs, normalize=normalize, engine=0, scores=x.data_ptr(),
+        argmax=x.data_ptr() if winners else None, argmax_stride=Lq, reserved=0, workspace=None, workspace_bytes=0, status=None,
+    )
+    t = _lib.TopkSpec(k=k, largest=1, index_offset=0, out_scores=None, out_index=None, flags=0, doc_base=0)
+    return lib.lik_maxsim_fwd_kernel(C.byref(a), C.byref(t) if k else None)
+
+
+def test_which_kernel_takes_a_call():
+    """Both sides of every line of the rule: units per SM, units per query tile, document lengths, full documents, merges."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert route(4, 12 * sms, 32, 64) == 2 and route(4, 12 * sms - 1, 32, 64) == 1
+    assert route(4, 12 * sms, 32, 300) == 2 and route(4, 12 * sms - 1, 32, 300) == 1
+    # more than 100 and up to 256 tokens: twice as much with one query tile
+    assert route(1, 12 * sms, 32, 100) == 2 and route(1, 12 * sms, 32, 101) == 1 and route(1, 12 * sms, 32, 256) == 1
+    assert route(1, 12 * sms, 32, 257) == 2 and route(1, 24 * sms, 32, 180) == 2 and route(8, 12 * sms, 32, 180) == 2
+    # query tiles that change with every few documents
+    many = 8 * 12 * sms
+    assert route(many, 1, 32, 64) == 1 and route(many // 2, 2, 32, 64) == 2 and route(many // 3 + 8, 3, 32, 64) == 1 and route(many // 4, 4, 32, 64) == 2
+    assert route(many, 1, 32, 300) == 1 and route(many // 7 + 8, 7, 32, 300) == 1 and route(many // 8, 8, 32, 300) == 2
+    for group, at_64, at_180, at_300 in ((1, 2, 1, 1), (2, 2, 1, 2), (3, 2, 1, 1), (5, 2, 1, 1), (6, 2, 1, 2), (11, 2, 1, 2), (12, 2, 2, 2)):
+        n = 24 * sms // group + 1
+        assert [route(n, n * group, 32, ld, group=group, winners=True) for ld in (64, 180, 300)] == [at_64, at_180, at_300]
+    assert route(64, 1000, 32, 300, n_pairs=32 * sms) == 2 and route(64, 1000, 32, 300, n_pairs=32 * sms - 1) == 1
+    assert route(64, 1000, 32, 180, n_pairs=95 * sms) == 1 and route(64, 1000, 32, 180, n_pairs=96 * sms) == 2
+    assert route(8 * sms, 1000, 32, 300, n_pairs=32 * sms) == 1  # four pairs per query
+    # documents known to fill their last tile of 256
+    assert route(64, 3 * sms, 32, 256, masked=False) == 1 and route(64, 3 * sms, 32, 256, masked=False, winners=True) == 2
+    assert route(64, 3 * sms, 32, 256) == 2 and route(64, 3 * sms, 32, 300, masked=False) == 2
+    # norms from the tiles, multipliers that arrive with the tiles
+    assert route(4, 40 * sms, 32, 300, normalize=3) == 1 and route(72, 2 * sms, 32, 300, normalize=3) == 2
+    assert route(4, 40 * sms, 32, 64, scaled=True, dtype=torch.float8_e4m3fn) == 1
+    assert route(4, 40 * sms + 1, 32, 65, scaled=True, dtype=torch.float8_e4m3fn) == 2  # (the set stages them)
+    # fused top-k: as everything else, and more where the lists need one more pass
+    assert route(1, 12 * sms, 32, 300, k=10) == 2 and route(1, 12 * sms - 1, 32, 300, k=10) == 1
+    assert route(40, 8 * sms, 32, 300, k=10) == 2 and route(40, 8 * sms - 1, 32, 300, k=10) == 1 and route(40, 100 * sms, 32, 1030, k=10) == 1
+    assert route(80, 2 * sms, 32, 300, k=10) == 2 and route(100_000, 2 * sms, 32, 300, k=10) == 1
+
+
+# documents of more than one piece and fewer than three, in the amounts from which they go to this kernel
+@pytest.mark.parametrize("Nq,units,Lq,Ld,dtype,norm", [
+    (1, 24, 32, 101, torch.bfloat16, False), (3, 24, 40, 192, torch.float16, False), (4, 25, 32, 256, torch.bfloat16, False), (8, 13, 31, 129, torch.float16, False),
+])
+def test_middling_documents(Nq, units, Lq, Ld, dtype, norm):
+    import late_interaction_kernels_b200 as lik
+    from late_interaction_kernels_b200.forward import maxsim_forward
+
+    Nd = units * torch.cuda.get_device_properties(0).multi_processor_count
+    assert route(Nq, Nd, Lq, Ld, winners=True, dtype=dtype) == 2 and route(Nq, Nd, Lq, Ld, k=9, dtype=dtype) == 2
+    gen = torch.Generator(device="cuda").manual_seed(Ld)
+    Q, D = ints(gen, Nq, Lq, 128), ints(gen, Nd, Ld, 128)
+    mask = torch.arange(Ld, device="cuda")[None] < lengths(Nd, Ld, gen)[:, None]
+    val, pos = reference(Q, D, mask)
+    scores, am = maxsim_forward(Q.to(dtype), D.to(dtype), None, mask, save_argmax=True)
+    assert torch.equal(scores.view(Nq, Nd), val.sum(-1)) and torch.equal(am.view(Nq, Nd, Lq).long(), pos)
+    ts, ti = lik.retrieve(Q.to(dtype), D.to(dtype), 9, d_mask=mask, normalize=False)
+    order = torch.sort(val.sum(-1), dim=1, descending=True, stable=True)
+    assert torch.equal(ts, order.values[:, :9]) and torch.equal(ti, order.indices[:, :9])
