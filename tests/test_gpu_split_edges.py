@@ -367,3 +367,19 @@ def test_workspaces_and_winners_off_a_16_byte_boundary(shift):
     _lib.check(lib.lik_maxsim_bwd(C.byref(b), st), "lik_maxsim_bwd")
     assert torch.equal(gq, want_q) and torch.equal(gd, want_d)
     lik.check_device_status()
+
+
+@pytest.mark.parametrize("Nq,Nd", [(4, 256), (4, 257), (1, 256), (9, 255), (3, 1)])
+def test_fp32_documents_in_the_order_of_their_lengths(Nq, Nd):
+    """Up to 256 documents with given lengths are dealt longest first (equal lengths in their own order), more as they come.
+    Small integers: every sum is exact."""
+    import late_interaction_kernels_b200 as lik
+
+    gen = torch.Generator(device="cuda").manual_seed(Nd)
+    Lq, Ld, d = 20, 70, 40
+    Q, D = (torch.randint(-2, 3, s, generator=gen, device="cuda").float() for s in ((Nq, Lq, d), (Nd, Ld, d)))
+    lens = torch.tensor([0, 1, 33, 64, Ld, Ld], device="cuda")[torch.randint(0, 6, (Nd,), generator=gen, device="cuda")]
+    mask = torch.arange(Ld, device="cuda")[None] < lens[:, None]
+    s = torch.einsum("isd,jtd->ijst", Q, D).masked_fill(~mask[None, :, None, :], float("-inf")).amax(-1)
+    want = torch.where(torch.isinf(s), torch.zeros_like(s), s).sum(-1)
+    assert torch.equal(lik.maxsim(Q, D, d_mask=mask), want)

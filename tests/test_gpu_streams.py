@@ -327,3 +327,71 @@ def test_middling_documents(Nq, units, Lq, Ld, dtype, norm):
     ts, ti = lik.retrieve(Q.to(dtype), D.to(dtype), 9, d_mask=mask, normalize=False)
     order = torch.sort(val.sum(-1), dim=1, descending=True, stable=True)
     assert torch.equal(ts, order.values[:, :9]) and torch.equal(ti, order.indices[:, :9])
+
+
+@pytest.mark.parametrize("holes", [False, True])
+def test_multipliers_staged_with_one_query_tile(holes):
+    """Per-token scales whose rows do not start on 16 bytes: the epilogue sets stage them, and a stream's two accumulators take
+    turns.  1e-5 as for all fp32 sums of exact products."""
+    from late_interaction_kernels_b200.fp8 import maxsim_inference_fp8, quantize_fp8_per_token
+
+    Nq, Lq, Ld = 4, 32, 97
+    Nd = 12 * torch.cuda.get_device_properties(0).multi_processor_count + 25
+    assert route(Nq, Nd, Lq, Ld, scaled=True, dtype=torch.float8_e4m3fn) == 2
+    gen = torch.Generator(device="cuda").manual_seed(97)
+    Q, D = torch.randn(Nq, Lq, 128, generator=gen, device="cuda"), torch.randn(Nd, Ld, 128, generator=gen, device="cuda")
+    mask = torch.arange(Ld, device="cuda")[None] < lengths(Nd, Ld, gen)[:, None]
+    if holes:
+        mask &= torch.rand(Nd, Ld, generator=gen, device="cuda") < 0.7
+    (q8, sq), (d8, sd) = quantize_fp8_per_token(Q), quantize_fp8_per_token(D)
+    want = reference(q8.double() * sq.double()[..., None], d8.double() * sd.double()[..., None], mask)[0].sum(-1)
+    got = maxsim_inference_fp8(q8, d8, scale_Q=sq, scale_D=sd, d_mask=mask).double()
+    assert (got - want).abs().max() <= 1e-5 * want.abs().max()
+
+
+def test_infinities_and_nan_rows_as_in_the_other_kernel():
+    """Rows of infinities and NaN in documents and queries: the first documents alone, which the other kernel takes, agree bit for
+    bit (NaN with NaN), winners included."""
+    from late_interaction_kernels_b200.forward import maxsim_forward
+
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    Nq, Lq, Ld, few = 9, 32, 120, 40
+    Nd = 12 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert route(Nq, Nd, Lq, Ld, winners=True, masked=False) == 2 and route(Nq, few, Lq, Ld, winners=True, masked=False) == 1
+    Q, D = torch.randn(Nq, Lq, 128, generator=gen, device="cuda"), torch.randn(Nd, Ld, 128, generator=gen, device="cuda")
+    for x, values in ((Q, (float("inf"), float("nan"))), (D, (float("inf"), float("-inf"), float("nan")))):
+        hit = torch.rand(x.shape[:2], generator=gen, device="cuda")
+        for n, v in enumerate(values):
+            x[(hit > 0.02 * n) & (hit < 0.02 * n + 0.015)] = v
+    D[3] = float("nan")
+    D[5] = float("-inf")
+    Q, D = Q.bfloat16(), D.bfloat16()
+    s, am = maxsim_forward(Q, D, save_argmax=True)
+    s1, am1 = maxsim_forward(Q, D[:few], save_argmax=True)
+    assert torch.equal(s[:, :few].nan_to_num(7.0), s1.nan_to_num(7.0)) and torch.equal(s[:, :few].isnan(), s1.isnan())
+    assert torch.equal(am.view(Nq, Nd, Lq)[:, :few], am1.view(Nq, few, Lq))
+
+
+def test_rows_with_a_stride_wider_than_the_row():
+    import ctypes as C
+
+    from late_interaction_kernels_b200 import _lib, _ops
+
+    lib = _lib.load()
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    Nq, Lq, Ld, d, wide = 8, 32, 50, 128, 136
+    Nd = 12 * torch.cuda.get_device_properties(0).multi_processor_count
+    Q, big = ints(gen, Nq, Lq, d).bfloat16(), ints(gen, Nd * Ld, wide).bfloat16()
+    out = torch.empty(Nq, Nd, device="cuda")
+    q = _ops.padded_spec(Q).c_struct()
+    dd = _lib.Seqs(data=big.data_ptr(), row_stride=wide, n_rows=Nd * Ld, n_seq=Nd, max_len=Ld, seq_stride=Ld, cu=None, lens=None, mask=None, scale=None,
+                   scale_scalar=1.0, reserved=0)
+    a = _lib.FwdArgs(
+        q=q, d=dd, dtype=_lib.lik_dtype(Q.dtype), dim=d, pairing=_lib.PAIR_CROSS, group=0, pair_q=None, pair_d=None, n_pairs=0, normalize=_lib.NORM_NONE,
+        engine=0, scores=out.data_ptr(), argmax=None, argmax_stride=Lq, reserved=0, workspace=None, workspace_bytes=0, status=None,
+    )
+    assert lib.lik_maxsim_fwd_kernel(C.byref(a), None) == 2
+    _lib.check(lib.lik_maxsim_fwd_static(C.byref(a), _lib.stream_ptr(out.device)), "lik_maxsim_fwd_static")
+    D = big[:, :d].float().view(Nd, Ld, d)
+    want = reference(Q.float(), D, torch.ones(Nd, Ld, dtype=torch.bool, device="cuda"))[0].sum(-1)
+    assert torch.equal(out, want)
