@@ -86,8 +86,7 @@ FwdPlan plan_fwd(const lik_fwd_args& a, const TcExtra& x = TcExtra()) {
     pl.use_tc = a.engine != 1 && fwd_tc_supported(b);
   // the kernel's own workspace comes first: its leading part (the candidate lists of a fused top-k) then sits at
   // the same place for every piece of a corpus that is scored piece by piece into one workspace
-  if (pl.use_tc) pl.tc_off = take(fwd_tc_workspace(b, x));
-  pl.streams = pl.use_tc && fwd_tc_streams(b, x);
+  if (pl.use_tc) pl.tc_off = take(fwd_tc_workspace(b, x, &pl.streams));
   if (a.normalize & LIK_NORM_Q) {
     if (pl.copies) pl.qcopy_off = take((size_t)a.q.n_rows * a.dim * eb);
     else pl.qn_off = take((size_t)a.q.n_rows * 4);

@@ -13,7 +13,8 @@
 //   - the query tiles are copied to tensor memory (tcgen05.cp): an MMA with A in shared memory moves 4 KB of it per 16 features
 //     beside the 3 KB of 96 document rows and took 56 cycles instead of 48 for that;
 //   - the last box of a document is moved back to end where the document ends, so that no column needs a mask.
-// In-batch 512 x 512 of 32 x 300 tokens 487 -> 354 us with winners, 355 -> 310 us without; 256 x 256 of 16 x 64 tokens 60 -> 42 us.
+// In-batch 512 x 512 of 32 x 300 tokens 477 -> 326 us with winners, 334 -> 284 us without; 256 x 256 of 16 x 64 tokens 61 -> 41 and
+// 57 -> 39 us.
 // What bounds it now: the search for the winners' columns (54 instructions on the half-rate pipe per 32 columns and warp, half of
 // the pipe's time) and the round trip of an accumulator (MMAs, 3 chunks of TMEM loads and folds, two barriers).
 //
@@ -294,8 +295,7 @@ fwd_streams_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_const
     // the time of two pieces.  A CTA's units go to the streams in turn; both pass through the same tile groups.
     // The warp walks the units (32 are looked up at a time, a thread each), cuts them into pieces, loads these with TMA and
     // publishes units and pieces.  It runs on warp-uniform values and one elected lane issues, as in the issuers below: TMA
-    // instructions, too, take their operands from uniform registers.  In the PLAID kernels it decodes the tokens into the
-    // swizzled operand layout instead (generic-proxy stores, fenced for the tensor core's reads).
+    // instructions, too, take their operands from uniform registers.
     const int sm = warp == 0 ? 0 : 1;
     const bool elect = elect_one();
     const int x_per_slab = SLAB_BYTES_ROW / P.elt_bytes, n_slabs = P.n_slabs, stages = P.stages, mt = P.mt;

@@ -1,6 +1,6 @@
 // Blackwell tensor-core MaxSim forward (sm_100a: TMA + tcgen05.mma + TMEM): the kernel for smaller problems, for norms taken
 // from the document tiles and for documents decoded from a PLAID index, and the host side of both tensor-core kernels.
-// Larger problems run in lik_fwd_streams.cu (plan_tc has the rule).
+// Larger problems run in lik_fwd_streams.cu (streams_pay has the rule).
 //
 // GEMM view: rows = query tokens (A operand, K-major, 128 per tile), columns = document tokens (B
 // operand, K-major, up to 256 per tile), K = embedding width.  A CTA is persistent: it keeps one or
@@ -1417,8 +1417,11 @@ TcWs tc_ws_layout(const TcPlan& pl, const lik_fwd_args& a, const TcExtra& x) {
 }
 }  // namespace
 
-bool fwd_tc_streams(const lik_fwd_args& a, const TcExtra& x) { return plan_tc(a, x).streams; }
-size_t fwd_tc_workspace(const lik_fwd_args& a, const TcExtra& x) { return tc_ws_layout(plan_tc(a, x), a, x).total; }
+size_t fwd_tc_workspace(const lik_fwd_args& a, const TcExtra& x, bool* streams) {
+  const TcPlan pl = plan_tc(a, x);
+  if (streams) *streams = pl.streams;
+  return tc_ws_layout(pl, a, x).total;
+}
 
 int launch_topk_slots(const float* keys, const int* idx, const int2* hdr, long long n_lists, int cap, int n_ctas, int n_groups,
                       int mt, int lists, int qpt, long long n_q, int k, int largest, long long index_offset, float* out_scores,

@@ -54,8 +54,6 @@ struct TopkOut {
   int n_lists;      // lists allocated (the kernel checks every list number against it)
 };
 
-// One row of the pair-list table (LIK_PAIR_LIST): written by list_units_kernel, read by the producer.
-//   x = query (0 for a pair that is out of range), y = first document row, z = document length, w = unused
 struct TcParams {
   SeqView q, d;
   int pairing;       // CROSS, GROUPED or LIST
@@ -73,7 +71,7 @@ struct TcParams {
   int n_sb;          // CROSS: the documents are walked in n_sb super-blocks of sb_docs documents (L2-sized)
   int sb_docs;
   long long n_flat;  // GROUPED / LIST: number of units
-  const int4* list_tab;  // LIST: one row per pair
+  const int4* list_tab;  // LIST: one row per pair, by list_units_kernel: x = query (0: out of range), y = first document row, z = document length
   float* scores;
   float* partial;    // [n_tiles, n_d] when q_chunks > 1
   int* argmax;

@@ -26,8 +26,7 @@ struct TcExtra {
 bool fwd_tc_supported(const lik_fwd_args& a);
 bool fwd_tc_topk_supported(const lik_fwd_args& a, const TcExtra& x);
 bool fwd_tc_plaid_supported(const lik_fwd_args& a, const TcExtra& x);
-size_t fwd_tc_workspace(const lik_fwd_args& a, const TcExtra& x);
-bool fwd_tc_streams(const lik_fwd_args& a, const TcExtra& x);  // whether the kernel for larger problems takes it
+size_t fwd_tc_workspace(const lik_fwd_args& a, const TcExtra& x, bool* streams = nullptr);  // streams: whether the kernel for larger problems takes it
 // `prep`: what still has to be written before the kernel runs; the launch adds its own jobs and sends them in one go
 // `norm_d_eps` > 0 (where fwd_tc_norms_in_kernel says so, dn == nullptr): the kernel takes the documents' norms itself
 bool fwd_tc_norms_in_kernel(const lik_fwd_args& a, const TcExtra& x);

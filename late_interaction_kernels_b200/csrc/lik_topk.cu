@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(NT, MIN_CTAS) topk_kernel(TopkParams P) {
   }
 }
 
-// Merge of the candidate lists the fused scoring kernel leaves (lik_fwd_tc.cu): list slot of (CTA c, tile
+// Merge of the candidate lists the fused scoring kernels leave (lik_fwd_tc.cuh): list slot of (CTA c, tile
 // group g) is c + g, each slot holds `lists` * qpt lists of up to 256 entries (unsorted), and CTA c of n_ctas can
 // only have worked on the groups [n_groups * c / n_ctas, n_groups * (c + 1) / n_ctas] (a superset of the ones
 // it really met; lists it never touched are empty).  A group is `mt` query tiles of `qpt` queries.  A kernel has lists of its
