@@ -395,3 +395,34 @@ def test_rows_with_a_stride_wider_than_the_row():
     D = big[:, :d].float().view(Nd, Ld, d)
     want = reference(Q.float(), D, torch.ones(Nd, Ld, dtype=torch.bool, device="cuda"))[0].sum(-1)
     assert torch.equal(out, want)
+
+
+def test_host_threads_with_different_shared_memory_sizes():
+    """The limit of a kernel's shared memory is one per process: launches of other widths in other threads leave it alone."""
+    import threading
+
+    from late_interaction_kernels_b200.forward import maxsim_forward
+
+    Nd = 12 * torch.cuda.get_device_properties(0).multi_processor_count
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    sets, errors = [], []
+    for d in (16, 32, 64, 80, 96, 128):  # one slab or two, deeper and shallower rings
+        Q, D = ints(gen, 8, 32, d).bfloat16(), ints(gen, Nd, 40, d).bfloat16()
+        sets.append((Q, D, maxsim_forward(Q, D)[0], maxsim_forward(Q, D[:20])[0]))
+
+    def work(n):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for i in range(60):
+                    Q, D, many, few = sets[(n + i) % len(sets)]
+                    assert torch.equal(maxsim_forward(Q, D)[0], many) and torch.equal(maxsim_forward(Q, D[:20])[0], few)
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(n,)) for n in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
