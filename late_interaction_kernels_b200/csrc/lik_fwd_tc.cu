@@ -1316,6 +1316,15 @@ TcPlan plan_tc(const lik_fwd_args& a, const TcExtra& x) {
   pl.stage_bytes = stage;
   pl.slot_bytes = pl.streams ? fwd_streams_slot_bytes() : TILE_N * sizeof(float);
   pl.lists = pl.streams ? 4 : 2;
+  // Scores or a top-k of one query tile from a compressed index
+  pl.decode = x.plaid && a.pairing == LIK_PAIR_CROSS && !a.argmax && !a.q.cu && a.q.max_len <= TILE_M && pl.n_tiles == 1;
+  if (pl.decode) {
+    pl.lists = 1;
+    pl.grid = fwd_plaid_ctas_per_sm() * sm_count();
+    pl.smem_bytes = fwd_plaid_smem(pl.n_slabs);
+    pl.stages = 1;
+    return pl;
+  }
   const size_t budget = 227 * 1024;
   int st = (int)((budget - fixed) / stage);
   pl.stages = st > 8 ? 8 : st;
@@ -1449,7 +1458,7 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
   CUtensorMap q_map;
   DocMaps d_maps;
   memset(&d_maps, 0, sizeof(d_maps));
-  int rc = pl.streams ? LIK_OK : make_map(&q_map, a.q, a.dtype, a.dim, TILE_M);
+  int rc = pl.streams || pl.decode ? LIK_OK : make_map(&q_map, a.q, a.dtype, a.dim, TILE_M);
   if (rc) return rc;
   if (!plaid && !pl.streams) {
     for (int i = 0; i < N_BOXES; ++i) {
@@ -1569,6 +1578,9 @@ int launch_fwd_tc(const lik_fwd_args& a, const float* qn, const float* dn, float
   const bool long_docs = argmax && a.d.max_len >= long_doc_tokens;
   if (pl.streams) {
     rc = launch_fwd_streams(a, pl, P, affine, long_docs, st);
+    if (rc) return rc;
+  } else if (pl.decode) {
+    rc = launch_fwd_plaid(a, pl, P, st);
     if (rc) return rc;
   } else {
     cudaLaunchAttribute attr{};

@@ -10,6 +10,7 @@ namespace lik {
 
 struct TcPlan {
   bool streams;     // the kernel with two streams (lik_fwd_streams.cu)
+  bool decode;      // the kernel that decodes a compressed index for one query tile (lik_fwd_plaid.cu)
   bool pack_tiles;  // ragged queries packed greedily into tiles by pack_query_tiles_kernel
   int q_per_tile, q_chunks, n_tiles, mt, n_slabs, k_steps, stages;
   int n_sb, sb_docs, n_groups;
@@ -132,7 +133,9 @@ __device__ __forceinline__ unsigned ordered_key(float f) {
 // and return the k-th best as an ordered key.  One warp; lane l holds entries l, l + 32, ...  The k-th
 // largest key is found by bisection on its bits (32 warp-wide counts); entries above it stay, and of the
 // entries equal to it the earliest ones (lowest document indices), so that exactly k remain, in order.
-__device__ __noinline__ unsigned topk_compact(float* keys, int* idx, int k, int lane) {
+// PARTIAL: the list holds n entries, k at least.
+template <bool PARTIAL = false>
+__device__ __noinline__ unsigned topk_compact(float* keys, int* idx, int k, int lane, int n = TOPK_CAP) {
   constexpr int PER = TOPK_CAP / 32;
   unsigned uk[PER];
   float fk[PER];
@@ -141,7 +144,7 @@ __device__ __noinline__ unsigned topk_compact(float* keys, int* idx, int k, int 
   for (int j = 0; j < PER; ++j) {
     fk[j] = keys[j * 32 + lane];
     id[j] = idx[j * 32 + lane];
-    uk[j] = ordered_key(fk[j]);
+    uk[j] = !PARTIAL || j * 32 + lane < n ? ordered_key(fk[j]) : 0u;
   }
   unsigned kth = 0;
   for (int bit = 31; bit >= 0; --bit) {
@@ -184,6 +187,10 @@ size_t fwd_streams_fixed_smem(int n_slabs);   // shared memory beside its rings
 size_t fwd_streams_stage_bytes(int n_slabs);  // a stage of both streams
 size_t fwd_streams_slot_bytes();
 int launch_fwd_streams(const lik_fwd_args& a, const TcPlan& pl, const TcParams& P, bool affine, bool long_docs, cudaStream_t st);
+// the kernel that decodes a compressed index
+size_t fwd_plaid_smem(int n_slabs);
+int fwd_plaid_ctas_per_sm();
+int launch_fwd_plaid(const lik_fwd_args& a, const TcPlan& pl, const TcParams& P, cudaStream_t st);
 int launch_streams_wait_probe(long long limit, int* status, int* result, cudaStream_t st);
 
 }  // namespace lik

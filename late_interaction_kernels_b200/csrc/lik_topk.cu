@@ -178,6 +178,7 @@ constexpr int SLOT_LISTS = 32;    // lists per CTA
 constexpr int SLOT_T = 512;
 constexpr int SLOT_PER = SLOT_LISTS * SLOT_CAP / SLOT_T;
 constexpr int SLOT_K = 128;       // largest k of the fused path
+constexpr int SLOT_CTAS = 512;    // largest grid whose lists it takes
 
 struct SlotParams {
   const float* keys;
@@ -269,7 +270,7 @@ __device__ __forceinline__ void slot_write(const SlotParams& P, long long q, con
 __global__ void __launch_bounds__(SLOT_T) topk_slots_kernel(SlotParams P) {
   __shared__ u64 top[SLOT_K];
   __shared__ int cnt[2 * SLOT_T / 32 + 1];
-  __shared__ int slots[256];  // list slots of this query, in CTA order
+  __shared__ int slots[SLOT_CTAS];  // list slots of this query, in CTA order
   __shared__ int n_slots_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long q = blockIdx.x;
@@ -283,10 +284,10 @@ __global__ void __launch_bounds__(SLOT_T) topk_slots_kernel(SlotParams P) {
       const bool hit = c < P.n_ctas && g >= (long long)P.n_groups * c / P.n_ctas && g <= (long long)P.n_groups * (c + 1) / P.n_ctas;
       const unsigned mask = __ballot_sync(0xffffffffu, hit);
       const int pos = n + __popc(mask & ((1u << lane) - 1u));
-      if (hit && pos < 256) slots[pos] = c + g;
+      if (hit && pos < SLOT_CTAS) slots[pos] = c + g;
       n += __popc(mask);
     }
-    if (lane == 0) n_slots_s = n < 256 ? n : 256;
+    if (lane == 0) n_slots_s = n < SLOT_CTAS ? n : SLOT_CTAS;
   }
   __syncthreads();
   const int n_lists = n_slots_s * n_sub;
@@ -352,7 +353,7 @@ int launch_topk_slots(const float* keys, const int* idx, const int2* hdr, long l
                       int mt, int lists, int qpt, long long n_q, int k, int largest, long long index_offset, float* out_scores,
                       long long* out_index, int parts, void* part_buf, cudaStream_t st) {
   if (n_q <= 0 || k <= 0) return LIK_OK;
-  if (cap != SLOT_CAP || k > SLOT_K || n_ctas > 256 || parts * k > SLOT_PER * SLOT_T || (parts > 1 && !part_buf)) {
+  if (cap != SLOT_CAP || k > SLOT_K || n_ctas > SLOT_CTAS || parts * k > SLOT_PER * SLOT_T || (parts > 1 && !part_buf)) {
     set_error("candidate lists of %d entries from %d CTAs, k = %d: outside what the merge takes", cap, n_ctas, k);
     return LIK_ERR_UNSUPPORTED;
   }

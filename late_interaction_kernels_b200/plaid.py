@@ -15,14 +15,20 @@ from . import _lib, _ops
 
 # decompressed tokens held at once (rows of `dim` operand-dtype values)
 _DECOMPRESS_TOKENS = 1 << 22
-# The index can also be decoded INSIDE the scoring kernel (``lik_plaid_fwd``: the kernel's producer warps gather,
-# unpack, normalise and write the operand tiles, so no operand row ever exists in memory).  Every query-tile group
-# (256 query-token rows = eight 32-token queries) then decodes the tokens it scores, with three decoder warps per SM.
-# Measured on B200 that is slower than decoding once per call with the whole machine (``lik_plaid_decompress``, about
-# half the HBM copy rate) and scoring the rows, even for a single query (4.0 ms against 0.64 ms for 25 000 documents),
-# so by default no problem takes it: this is the largest number of tile groups for which it is used.  Both ways
-# produce the same bits.
+# The index can also be decoded INSIDE the scoring kernel (``lik_plaid_fwd``), so that no operand row ever exists in
+# memory.  The kernel for that takes the query tokens that fit one tile of 128 rows (four 32-token queries) and decodes
+# every token once.  More queries, and calls that save the winners, would go to an older form that decodes every token
+# once per group of two tiles with three warps per SM, slower than decoding once with the whole machine: this is the
+# largest number of such groups for which it is used.  All ways produce the same bits.
 _FUSED_DECODE_MAX_GROUPS = 0
+
+
+def _decode_in_kernel(Nq: int, Lq: int, winners: bool = False) -> bool:
+    if Nq <= 0 or Lq <= 0:
+        return False
+    if not winners and Lq <= 128 and Nq <= 128 // Lq:
+        return True
+    return _tile_groups(Nq, Lq) <= _FUSED_DECODE_MAX_GROUPS
 
 
 def _tile_groups(Nq: int, Lq: int) -> int:
@@ -86,7 +92,7 @@ def _residual_scores(Q, ix, cu_or_lens, max_ld, padded, normalize, save_argmax):
     Qo = Q.to(odt)
     q = _ops.padded_spec(Qo)
     norm = _lib.NORM_Q if normalize else _lib.NORM_NONE
-    if Nq > 0 and _tile_groups(Nq, Lq) <= _FUSED_DECODE_MAX_GROUPS and ix.n_tokens > 0:
+    if _decode_in_kernel(Nq, Lq, save_argmax) and ix.n_tokens > 0:
         if padded:
             nd = cu_or_lens.numel()
             lay = _ops.layout_spec(nd * max_ld, nd, max_ld, lens=cu_or_lens, seq_stride=max_ld)
@@ -291,7 +297,7 @@ def retrieve_residual_varlen(Q, codes_flat, residuals_flat, cu_seqlens_d, centro
     norm = _lib.NORM_Q if normalize else _lib.NORM_NONE
     out = None
     with torch.no_grad():
-        if k <= _lib.TOPK_FUSED_MAX and _tile_groups(Nq, Lq) <= _FUSED_DECODE_MAX_GROUPS:
+        if k <= _lib.TOPK_FUSED_MAX and _decode_in_kernel(Nq, Lq):
             # few queries: one kernel decodes, scores and keeps the candidates; nothing is read on the host
             lay = _ops.layout_spec(ix.n_tokens, Nd, 0, cu=cu)
             out = _ops.forward_fused(q, lay, normalize=(_lib.NORM_BOTH if normalize else _lib.NORM_NONE), plaid=ix, topk=k,
