@@ -9,6 +9,8 @@ namespace lik {
 int launch_row_normalize(const void* data, int dtype, long long n_rows, int dim, long long stride, float eps, void* out,
                          cudaStream_t st);
 int launch_fwd_generic(const lik_fwd_args& a, const float* qn, const float* dn, cudaStream_t st);
+bool fwd_split_supported(const lik_fwd_args& a);
+int launch_fwd_split(const lik_fwd_args& a, float eps, cudaStream_t st);
 
 namespace {
 constexpr float kFwdNormEps = 1e-12f;
@@ -18,6 +20,7 @@ struct FwdPlan {
   size_t need, total;  // without and with the trimmed lengths of the portable kernel, which it can do without
   bool use_tc;
   bool streams;  // of the two tensor-core kernels, the one for larger problems
+  bool split;    // fp32 rows cut into parts for the tensor cores; takes the norms itself
   bool copies;  // fused normalisation through normalised operand copies instead of per-row multipliers
 };
 
@@ -84,6 +87,7 @@ FwdPlan plan_fwd(const lik_fwd_args& a, const TcExtra& x = TcExtra()) {
     pl.use_tc = fwd_tc_topk_supported(b, x);
   else
     pl.use_tc = a.engine != 1 && fwd_tc_supported(b);
+  pl.split = !pl.use_tc && !x.plaid && x.topk_k == 0 && fwd_split_supported(b);
   // the kernel's own workspace comes first: its leading part (the candidate lists of a fused top-k) then sits at
   // the same place for every piece of a corpus that is scored piece by piece into one workspace
   if (pl.use_tc) pl.tc_off = take(fwd_tc_workspace(b, x, &pl.streams));
@@ -118,7 +122,7 @@ int run_fwd(const lik_fwd_args& a, const FwdPlan& pl, cudaStream_t st, const TcE
       b.q.row_stride = a.dim;
     } else {
       float* w = (float*)(ws + pl.qn_off);
-      prep.norm[0] = norm_job(a.q, a.dtype, a.dim, kFwdNormEps, w, false);
+      if (!pl.split) prep.norm[0] = norm_job(a.q, a.dtype, a.dim, kFwdNormEps, w, false);
       qn = w;
     }
   }
@@ -132,7 +136,7 @@ int run_fwd(const lik_fwd_args& a, const FwdPlan& pl, cudaStream_t st, const TcE
       norm_d_eps = kFwdNormEps;
     } else {
       float* w = (float*)(ws + pl.dn_off);
-      prep.norm[1] = norm_job(a.d, a.dtype, a.dim, kFwdNormEps, w, false);
+      if (!pl.split) prep.norm[1] = norm_job(a.d, a.dtype, a.dim, kFwdNormEps, w, false);
       dn = w;
     }
   }
@@ -149,6 +153,7 @@ int run_fwd(const lik_fwd_args& a, const FwdPlan& pl, cudaStream_t st, const TcE
   }
   rc = launch_prep(prep, st);
   if (rc) return rc;
+  if (pl.split) return launch_fwd_split(b, kFwdNormEps, st);
   return launch_fwd_generic(b, qn, dn, st);
 }
 }  // namespace

@@ -1,0 +1,133 @@
+"""fp32 scores on the tensor cores (rows cut into three parts) against the fused multiply-add kernel (``engine=1``) and against
+64 bits, at the edges of pieces and tiles, on rows that the cut does not fit, and on integers, where both must be exact.
+
+Bound used on real data: a dot product is two roundings of a result and what the cut loses, 2^-25 of the largest magnitudes of
+either row per feature: |error| <= (2^-23 + 2 * 128 * 2^-25 * f) |q| |d| with f = max / norm of a row, below 1e-5 |q| |d| for
+any row; a score sums up to 128 of them."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(Q, D, engine, normalize=0, qm=None, dm=None, lens=None, cu=None, max_d=None):
+    from late_interaction_kernels_b200 import _ops, check_device_status
+
+    q = _ops.padded_spec(Q, mask=qm)
+    d = _ops.packed_spec(D, cu, max_d) if cu is not None else _ops.padded_spec(D, mask=dm, lens=lens)
+    s = _ops.forward(q, d, normalize=normalize, engine=engine)[0].view(Q.shape[0], -1)
+    check_device_status()
+    return s
+
+
+def _exact(Q, D, normalize, qm, dm):
+    Q, D = Q.double(), D.double()
+    if normalize:
+        Q, D = torch.nn.functional.normalize(Q, dim=-1), torch.nn.functional.normalize(D, dim=-1)
+    x = torch.einsum("isd,jtd->ijst", Q, D).masked_fill(~dm[None, :, None, :], -torch.inf).amax(-1)
+    return x.masked_fill(x == -torch.inf, 0.0).masked_fill(~qm[:, None, :], 0.0).sum(-1)
+
+
+def _masks(nq, lq, nd, ld, g):
+    dl = torch.tensor(([0, 1, 15, 16, 17, 63, 64, 65, 127, 128, 129, ld] * nd)[:nd]).clamp(max=ld)
+    dm = torch.arange(ld) < dl[:, None]
+    holes = torch.rand((nd, ld), generator=g) > 0.2
+    dm[nd // 2 :] &= holes[nd // 2 :]
+    qm = torch.arange(lq) < torch.randint(0, lq + 1, (nq, 1), generator=g)
+    return qm.cuda(), dm.cuda()
+
+
+@pytest.mark.parametrize("nq,lq,nd,ld,d", [(1, 1, 1, 1, 4), (1, 128, 24, 200, 128), (9, 32, 24, 130, 128), (13, 24, 300, 70, 96), (5, 33, 24, 129, 100),
+                                           (40, 5, 24, 65, 20), (3, 100, 24, 200, 12), (130, 1, 24, 64, 128)])
+@pytest.mark.parametrize("normalize", [0, 3])
+def test_scores_against_64_bits_and_the_chain(nq, lq, nd, ld, d, normalize):
+    g = torch.Generator().manual_seed(nq * 7 + d)
+    Q, D = torch.randn((nq, lq, d), generator=g).cuda(), (torch.randn((nd, ld, d), generator=g) * torch.rand((nd, ld, 1), generator=g)).cuda()
+    qm, dm = _masks(nq, lq, nd, ld, g)
+    a, b = _run(Q, D, 0, normalize, qm, dm), _run(Q, D, 1, normalize, qm, dm)
+    e = _exact(Q, D, normalize, qm, dm)
+    scale = e.abs().max().clamp(min=1e-30)
+    err = ((a.double() - e).norm() / e.norm().clamp(min=1e-30)).item()
+    assert ((a.double() - e).abs().max() / scale).item() < 2e-6 and ((b.double() - e).abs().max() / scale).item() < 2e-6
+    assert err < 1e-6
+
+
+@pytest.mark.parametrize("nq,lq,nd,ld,d", [(8, 4, 40, 180, 128), (17, 3, 20, 64, 64)])
+def test_integers_are_exact(nq, lq, nd, ld, d):
+    """Whole numbers of up to 16 bits: any product of parts that went missing shows.  A dot product is below 3 * 30000 * 128 and a
+    score of four of them, for rows in random directions a third of that at most, below 2^24."""
+    g = torch.Generator().manual_seed(5)
+    Q = torch.randint(-3, 4, (nq, lq, d), generator=g).float().cuda()
+    D = torch.randint(-30000, 30001, (nd, ld, d), generator=g).float().cuda()
+    qm, dm = _masks(nq, lq, nd, ld, g)
+    want = _exact(Q, D, 0, qm, dm)
+    assert torch.equal(_run(Q, D, 0, 0, qm, dm).double(), want)
+    assert torch.equal(_run(D[:nq, :lq].contiguous(), Q[:, :, :], 0).double(),
+                       _exact(D[:nq, :lq], Q, 0, torch.ones(nq, min(lq, ld), dtype=torch.bool, device="cuda"), torch.ones(nq, lq, dtype=torch.bool, device="cuda")))
+
+
+@pytest.mark.parametrize("nq,lq,nd,ld,d", [(5, 32, 40, 200, 128), (7, 20, 40, 130, 64), (2, 128, 40, 300, 32), (130, 1, 20, 65, 16)])
+@pytest.mark.parametrize("extra", [0, 3])
+def test_winners(nq, lq, nd, ld, d, extra):
+    """Small whole numbers tie often: the first token wins, in the order of the two sets' pieces too; scores have the same bits with
+    and without winners; places behind a query hold -1."""
+    from late_interaction_kernels_b200 import _ops
+
+    g = torch.Generator().manual_seed(11)
+    Q, D = torch.randint(-1, 2, (nq, lq, d), generator=g).float().cuda(), torch.randint(-1, 2, (nd, ld, d), generator=g).float().cuda()
+    qm, dm = _masks(nq, lq, nd, ld, g)
+    got = [_ops.forward(_ops.padded_spec(Q, mask=qm), _ops.padded_spec(D, mask=dm), save_argmax=True, argmax_stride=lq + extra, engine=e) for e in (0, 1)]
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert torch.equal(got[0][0].view(nq, nd), _run(Q, D, 0, 0, qm, dm))
+    Q, D = torch.randn((nq, lq, d), generator=g).cuda(), torch.randn((nd, ld, d), generator=g).cuda()
+    for n in (0, 3):
+        a, _ = _ops.forward(_ops.padded_spec(Q, mask=qm), _ops.padded_spec(D, mask=dm), normalize=n, save_argmax=True, argmax_stride=lq + extra)
+        assert torch.equal(a.view(nq, nd), _run(Q, D, 0, n, qm, dm))
+
+
+def test_layouts():
+    """Packed documents, lengths, row strides and offsets, and what stays with the other kernel (unaligned rows)."""
+    g = torch.Generator().manual_seed(1)
+    Q = torch.randn((6, 20, 64), generator=g).cuda()
+    lens = torch.tensor([0, 64, 1, 200, 65, 0, 33, 128, 5, 0])
+    cu = torch.cat([torch.zeros(1, dtype=torch.int64), lens.cumsum(0)]).to(torch.int32).cuda()
+    Dp = torch.randn((int(lens.sum()), 64), generator=g).cuda()
+    a, b = _run(Q, Dp, 0, 3, cu=cu, max_d=200), _run(Q, Dp, 1, 3, cu=cu, max_d=200)
+    assert torch.allclose(a, b, rtol=1e-5, atol=1e-5) and (a[:, lens == 0] == 0).all()
+    D = torch.zeros((10, 200, 64), device="cuda")
+    for j, n in enumerate(lens):
+        D[j, :n] = Dp[cu[j] : cu[j + 1]]
+    assert torch.equal(_run(Q, D, 0, 3, lens=lens.cuda()), a)
+    from late_interaction_kernels_b200 import _ops
+
+    wide = torch.randn((10 * 200, 80), device="cuda")
+    wide[:, 4:68] = D.view(-1, 64)
+    for lo in (4, 3):  # rows sixteen bytes apart from a boundary of sixteen bytes, and not
+        wide[:, lo : lo + 64] = D.view(-1, 64).clone()
+        spec = _ops.padded_spec(D, lens=lens.cuda())
+        spec.data = wide[:, lo : lo + 64]
+        s = _ops.forward(_ops.padded_spec(Q), spec, normalize=3)[0].view(6, 10)
+        assert torch.allclose(s, a, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("where", ["document", "query", "both"])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 1e30, 3e38, 1e-30, 1e-42])
+@pytest.mark.parametrize("normalize", [0, 3])
+def test_rows_that_do_not_fit(where, value, normalize):
+    """A piece or tile with such a row takes the chain: the same numbers as that kernel's, also infinities, NaN and subnormals."""
+    g = torch.Generator().manual_seed(2)
+    Q, D = torch.randn((5, 32, 128), generator=g).cuda(), torch.randn((12, 150, 128), generator=g).cuda()
+    if where != "query":
+        D[3, 70] = value if abs(value) < 1e-20 else D[3, 70]
+        D[3, 70, 5] = value
+        D[7, :] *= value if abs(value) < 1e20 else 1.0
+    if where != "document":
+        Q[1, 4] = value if abs(value) < 1e-20 else Q[1, 4]
+        Q[1, 4, 9] = value
+    a, b = _run(Q, D, 0, normalize), _run(Q, D, 1, normalize)
+    assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+    ok = a.isfinite()
+    assert torch.allclose(a[ok], b[ok], rtol=2e-6, atol=0 if normalize or abs(value) > 1e20 else 1e-5)
+    if where != "document":  # the whole first tile (four queries) is taken by the chain
+        assert torch.equal(a[:4].nan_to_num(1.5), b[:4].nan_to_num(1.5)) or torch.allclose(a[:4], b[:4], rtol=1e-6, equal_nan=True)
