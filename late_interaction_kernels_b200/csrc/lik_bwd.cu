@@ -698,7 +698,10 @@ __device__ __forceinline__ void dq16_finish_row(const BwdParams& P, float (&acc)
 }
 
 // One block of 16 * TOK threads: query tokens [s0, s0 + TOK) of query i, document range z.
-template <typename T, typename G, int CH, int TOK>
+// AHEAD: winners and weights of a batch of documents are fetched while the rows of the batch before are gathered.  For launches whose
+// blocks have few others beside them (packed 128 x 128 step, backward 71 -> 66 us); with many, the loads only stand in the way of the
+// gathers' (512 x 512 step 843 -> 860 us).
+template <typename T, typename G, int CH, int TOK, bool AHEAD = false>
 __device__ __forceinline__ void dq16_block(const BwdParams& P, int i, int s0, int z, int2 (*s_e)[TOK]) {
   constexpr int N = Vec16<T>::N;
   constexpr int U = 8 / CH;  // rows in flight per half-warp
@@ -734,31 +737,73 @@ __device__ __forceinline__ void dq16_block(const BwdParams& P, int i, int s0, in
     jb_lo = min(count, z * chunk);
     jb_hi = min(count, jb_lo + chunk);
   }
-  for (int jb = jb_lo; jb < jb_hi; jb += DQ_JC) {
-    __syncthreads();
+  // entry (jj, r) of a batch: winner of document jb + jj for query token s0 + r
+  constexpr int PER = AHEAD ? DQ_JC / 16 : 1;  // entries per thread
+  int win[PER];
+  float wgt[PER];
+  auto fetch = [&](int jb) {
 #pragma unroll
-    for (int x = tid; x < DQ_JC * TOK; x += 16 * TOK) {
-      // entry (jj, r): winner of document jb + jj for query token s0 + r
-      const int jj = x / TOK, r = x % TOK;
-      int2 e = make_int2(-1, 0);
+    for (int y = 0; y < PER; ++y) {
+      const int x = tid + y * 16 * TOK, jj = x / TOK, r = x % TOK;
+      win[y] = -1;
+      wgt[y] = 0.f;
       if (jb + jj < jb_hi && s0 + r < lq) {
         long long slot;
         int j;
         nth_score(P, p0, j0, jb + jj, slot, j);
-        const int t = P.argmax[slot * lq + s0 + r];
+        win[y] = P.argmax[slot * lq + s0 + r];
+        wgt[y] = P.g[slot];
+      }
+    }
+  };
+  if (AHEAD) fetch(jb_lo);
+  for (int jb = jb_lo; jb < jb_hi; jb += DQ_JC) {
+    __syncthreads();
+    if constexpr (AHEAD) {
+#pragma unroll
+      for (int y = 0; y < PER; ++y) {
+        const int x = tid + y * 16 * TOK, jj = x / TOK, r = x % TOK, t = win[y];
+        int2 e = make_int2(-1, 0);
         if (t >= 0) {
-          long long r0;
-          int dl;
+          long long slot, r0;
+          int j, dl;
+          nth_score(P, p0, j0, jb + jj, slot, j);
           seq_bounds(P.d, j, r0, dl, nullptr);
           const long long drow = r0 + t;
           if (t < dl && drow < P.d.n_rows) {  // a saved winner outside its document contributes nothing
-            float f = P.g[slot];
+            float f = wgt[y];
             if (d_factor) f *= row_factor(P.d, drow);
             e = make_int2((int)drow, __float_as_int(f));
           }
         }
+        s_e[jj][r] = e;
       }
-      s_e[jj][r] = e;
+      if (jb + DQ_JC < jb_hi) fetch(jb + DQ_JC);
+    } else {
+#pragma unroll
+      for (int x = tid; x < DQ_JC * TOK; x += 16 * TOK) {
+        // entry (jj, r): winner of document jb + jj for query token s0 + r
+        const int jj = x / TOK, r = x % TOK;
+        int2 e = make_int2(-1, 0);
+        if (jb + jj < jb_hi && s0 + r < lq) {
+          long long slot;
+          int j;
+          nth_score(P, p0, j0, jb + jj, slot, j);
+          const int t = P.argmax[slot * lq + s0 + r];
+          if (t >= 0) {
+            long long r0;
+            int dl;
+            seq_bounds(P.d, j, r0, dl, nullptr);
+            const long long drow = r0 + t;
+            if (t < dl && drow < P.d.n_rows) {  // a saved winner outside its document contributes nothing
+              float f = P.g[slot];
+              if (d_factor) f *= row_factor(P.d, drow);
+              e = make_int2((int)drow, __float_as_int(f));
+            }
+          }
+        }
+        s_e[jj][r] = e;
+      }
     }
     __syncthreads();
     if (active) {
@@ -1285,7 +1330,8 @@ __global__ void __launch_bounds__(DDS_WARPS * 32) bwd_dd_sort4_kernel(BwdParams 
 
 // grad_d reduce with 16-byte gathers: one half-warp per document token, 16 tokens per CTA.
 // GLOBAL: the list is in device memory (read-only loads), not in shared memory
-template <typename T, typename G, int CH, bool GLOBAL>
+// LONE: lists of one or two entries, nearly all of them: one by one
+template <typename T, typename G, int CH, bool GLOBAL, bool LONE = false>
 __device__ __forceinline__ void dd_reduce16_list(const BwdParams& P, const int2* __restrict__ list, int cnt, long long drow, int hl) {
   constexpr int N = Vec16<T>::N;
   constexpr int U = 8 / CH;
@@ -1304,32 +1350,47 @@ __device__ __forceinline__ void dd_reduce16_list(const BwdParams& P, const int2*
     bool lane_on[CH];
 #pragma unroll
     for (int c = 0; c < CH; ++c) lane_on[c] = elt16<T>(c, hl) < P.dim;
-    int k = 0;
-    for (; k + U <= cnt; k += U) {
-      int2 e[U];
+    // `n` entries from k on, their rows in flight together (n < W: the others are left out)
+    auto batch = [&](auto w_, int k, int n) {
+      constexpr int W = decltype(w_)::value;
+      int2 e[W];
 #pragma unroll
-      for (int u = 0; u < U; ++u) e[u] = entry(k + u);
-      uint4 v[U][CH];
+      for (int u = 0; u < W; ++u) e[u] = entry(k + min(u, n - 1));
+      uint4 v[W][CH];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
+      for (int u = 0; u < W; ++u) {
         const T* src = Qlane + e[u].x * pitch;
 #pragma unroll
-        for (int c = 0; c < CH; ++c) v[u][c] = lane_on[c] ? load16_raw<T>(src + c * 16 * N) : make_uint4(0, 0, 0, 0);
+        for (int c = 0; c < CH; ++c) v[u][c] = u < n && lane_on[c] ? load16_raw<T>(src + c * 16 * N) : make_uint4(0, 0, 0, 0);
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
+      for (int u = 0; u < W; ++u) {
         const float w = __int_as_float(e[u].y);
+        if (u < n) {
 #pragma unroll
-        for (int c = 0; c < CH; ++c) fma16_raw<T>(acc[c], w, v[u][c]);
+          for (int c = 0; c < CH; ++c) fma16_raw<T>(acc[c], w, v[u][c]);
+        }
       }
-    }
-    for (; k < cnt; ++k) {
-      const int2 e = entry(k);
-      const float w = __int_as_float(e.y);
-      const T* src = Qlane + e.x * pitch;
+    };
+    int k = 0;
+    for (; k + U <= cnt; k += U) batch(std::integral_constant<int, U>{}, k, U);
+    if constexpr (LONE) {
+      for (; k < cnt; ++k) {
+        const int2 e = entry(k);
+        const float w = __int_as_float(e.y);
+        const T* src = Qlane + e.x * pitch;
 #pragma unroll
-      for (int c = 0; c < CH; ++c)
-        if (lane_on[c]) fma16_raw<T>(acc[c], w, load16_raw<T>(src + c * 16 * N));
+        for (int c = 0; c < CH; ++c)
+          if (lane_on[c]) fma16_raw<T>(acc[c], w, load16_raw<T>(src + c * 16 * N));
+      }
+    } else {
+      // The rest in one or two trips to L2 instead of one per entry: a token of a small batch has three or four entries in all.
+      // (Packed 128 x 128 step, grad_D alone 50 -> 41 us.)
+      if (U > 4 && k + 4 <= cnt) {
+        batch(std::integral_constant<int, 4>{}, k, 4);
+        k += 4;
+      }
+      if (k < cnt) batch(std::integral_constant<int, 3>{}, k, cnt - k);
     }
   }
   if (P.normalize & LIK_NORM_D) {
@@ -1412,7 +1473,7 @@ __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape
   const int first_doc = F.dq_blocks * F.dq_split;
   if ((int)blockIdx.x < first_doc) {
     const int z = blockIdx.x / F.dq_blocks, b = blockIdx.x - z * F.dq_blocks, i = b / F.dq_per_query;
-    dq16_block<T, G, CH, TOK>(P, i, (b - i * F.dq_per_query) * TOK, z, reinterpret_cast<int2(*)[TOK]>(fused_raw));
+    dq16_block<T, G, CH, TOK, (NT > 256)>(P, i, (b - i * F.dq_per_query) * TOK, z, reinterpret_cast<int2(*)[TOK]>(fused_raw));
     return;
   }
   const int j = (blockIdx.x - first_doc) / F.parts, part = (blockIdx.x - first_doc) - j * F.parts;
@@ -1493,7 +1554,7 @@ __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape
       else if ((set_b >> lane) & 1u) mine[32 + __popc(set_b & below)] = make_int2(qrow, __float_as_int(w));
       __syncwarp();
       const unsigned set = lane < 16 ? set_a : set_b;
-      if (set) dd_reduce16_list<T, G, CH, false>(P, mine + (lane & 16) * 2, __popc(set), drow0 + tok, hl);
+      if (set) dd_reduce16_list<T, G, CH, false, true>(P, mine + (lane & 16) * 2, __popc(set), drow0 + tok, hl);
       first &= first - 1;
       second &= second - 1;
     }
@@ -1545,21 +1606,43 @@ __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape
         t_r[k] = __ldg(P.argmax + doc_slot(P, ds, j, ii) * lq + s);
       }
     }
+    // the query of a round's entry: its first row and length, and the weight of its score; the four words of a load share theirs, which
+    // are fetched while the winners are on their way (per entry and twice before: grad_D alone 54 -> 50 us)
+    struct Owner {
+      int row0, len, s;  // s: the entry's token of the query (of a load's first word)
+      float g;
+    };
+    auto owner_of = [&](int k, bool weight) {
+      Owner o{0, 0, 0, 0.f};
+      const int e = entry_of(k);
+      if (k < F.rounds && e < n_ent) {
+        const int ii = e / lq;
+        o.s = e - ii * lq;
+        long long r0;
+        seq_bounds(P.q, ds.i_begin + ii, r0, o.len, nullptr);
+        o.row0 = (int)r0;
+        if (weight) o.g = P.g[doc_slot(P, ds, j, ii)];
+      }
+      return o;
+    };
+    constexpr int FOURS = ROUNDS >= 4 ? ROUNDS / 4 : 1;
+    Owner owner[FOURS];
+    if (by_four) {
+#pragma unroll
+      for (int f = 0; f < FOURS; ++f) owner[f] = owner_of(4 * f, true);
+    }
     if (prefill)
       for (int t = part * TOK + hw; t < d_rows; t += TOK * F.parts) store_row16<T, G, CH>((G*)P.grad_d + (drow0 + t) * P.dim, zero, P.dim, hl);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < ROUNDS; ++k) {
       if (k >= F.rounds) break;
-      const int e = entry_of(k);
       int t = t_r[k];
       if (t >= dlen) t = -1;
       if (t >= 0) {
-        const int ii = e / lq, s = e - ii * lq;
-        long long qrow0;
-        int qlen;
-        seq_bounds(P.q, ds.i_begin + ii, qrow0, qlen, nullptr);
-        if (s >= qlen || !row_valid(P.q, qrow0 + s)) t = -1;
+        const Owner o = by_four ? owner[k / 4 < FOURS ? k / 4 : 0] : owner_of(k, false);
+        const int s = o.s + (by_four ? k & 3 : 0);
+        if (s >= o.len || !row_valid(P.q, (long long)o.row0 + s)) t = -1;
       }
       t_r[k] = t;
       if (t >= 0) atomicAdd(&hist[warp * F.ld_pad + t], 1);
@@ -1605,13 +1688,9 @@ __global__ void __launch_bounds__(NT) bwd_fused16_kernel(BwdParams P, FusedShape
       const int t = t_r[k];
       const unsigned peers = warp_peers(t, t_bits);
       if (t >= 0) {
-        const int e = entry_of(k), ii = e / lq, s = e - ii * lq;
-        const int i = ds.i_begin + ii;
-        long long qrow0;
-        int qlen;
-        seq_bounds(P.q, i, qrow0, qlen, nullptr);
-        const long long qrow = qrow0 + s;
-        const float w = P.g[doc_slot(P, ds, j, ii)] * row_factor(P.q, qrow);
+        const Owner o = by_four ? owner[k / 4 < FOURS ? k / 4 : 0] : owner_of(k, true);
+        const long long qrow = (long long)o.row0 + o.s + (by_four ? k & 3 : 0);
+        const float w = o.g * row_factor(P.q, qrow);
         list[hist[warp * F.ld_pad + t] + __popc(peers & ((1u << lane) - 1u))] = make_int2((int)qrow, __float_as_int(w));
       }
       __syncwarp();
