@@ -627,7 +627,7 @@ def other_configs(dev):
     flf = 2.0 * 128 * float(qlf.sum()) * float(dlf.sum())
     out["inbatch_fp32_fwd_32x32"] = {"us": t, "shape": "fp32 Q[32,32,128] x D[32,180,128], normalize, q U[8,32], d U[32,180]",
                                      "tflops_valid": flf / (t * 1e-6) / 1e12,
-                                     "note": "exact fp32-FMA kernel (fwd_generic_kernel); a launch-latency-sized problem"}
+                                     "note": "fp32 rows in three bf16 parts on the tensor cores (fwd_split_kernel); a launch-latency-sized problem"}
     # KD: Q[64,32,128] x D[64,32,300,128], lengths U[64,300] per candidate
     Q = F.normalize(torch.randn((64, 32, 128), generator=g, device=dev), dim=-1)
     D = F.normalize(torch.randn((64, 32, 300, 128), generator=g, device=dev), dim=-1)

@@ -1,7 +1,7 @@
 // Portable fp32-accumulate MaxSim forward: any element type, any embedding
-// width, every layout and pairing.  It is the exact path (fp32 FMA in a fixed
-// order, so fp32 inputs keep fp32 accuracy) and the home of shapes the tcgen05
-// kernel does not take (odd widths, pair lists).
+// width, every layout and pairing, fp32 FMA in a fixed order.  It is the home of
+// the shapes that the tcgen05 kernels do not take (odd widths; of fp32 inputs also
+// pair lists, candidate lists, packed queries and long ones).
 #include <atomic>
 
 #include "lik_common.cuh"

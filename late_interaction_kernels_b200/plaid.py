@@ -3,8 +3,9 @@
 ``plaid_approx_score`` is the IVF-prune step.  ``maxsim_residual`` / ``maxsim_residual_varlen``
 score queries against a compressed index (centroid codes + bit-packed residuals).  The reference
 decompresses every document token once per (query, document) program; here every token is
-decompressed once per call (``lik_plaid_decompress``) into the operand dtype and then scored by the
-regular MaxSim forward, in document chunks so the decompressed rows stay small.
+decompressed once per call: inside the scoring kernel (``lik_plaid_fwd``) for a few queries, else
+(``lik_plaid_decompress``) into the operand dtype, to be scored by the regular MaxSim forward in
+document chunks so the decompressed rows stay small.
 """
 
 from __future__ import annotations
@@ -298,7 +299,7 @@ def retrieve_residual_varlen(Q, codes_flat, residuals_flat, cu_seqlens_d, centro
     out = None
     with torch.no_grad():
         if k <= _lib.TOPK_FUSED_MAX and _decode_in_kernel(Nq, Lq):
-            # few queries: one kernel decodes, scores and keeps the candidates; nothing is read on the host
+            # few queries: one kernel decodes, scores and keeps the candidates; nothing is read on the host, no piece is placed
             lay = _ops.layout_spec(ix.n_tokens, Nd, 0, cu=cu)
             out = _ops.forward_fused(q, lay, normalize=(_lib.NORM_BOTH if normalize else _lib.NORM_NONE), plaid=ix, topk=k,
                                      largest=largest)
