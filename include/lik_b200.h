@@ -124,7 +124,8 @@ typedef struct lik_fwd_args {
 
 size_t lik_maxsim_fwd_workspace(const lik_fwd_args* args);
 /* Which kernel this forward (topk == NULL) or fused top-k (its flags and outputs are not looked at) goes to by itself, given the
- * workspace it asks for: 0 = portable, 1 = tensor cores, 2 = tensor cores, the kernel for larger problems; negative: refused. */
+ * workspace it asks for: 0 = portable (or, of fp32 rows, their parts on the tensor cores), 1 = tensor cores, 2 = tensor cores, the kernel for
+ * larger problems; negative: refused. */
 struct lik_topk_spec;
 int lik_maxsim_fwd_kernel(const lik_fwd_args* args, const struct lik_topk_spec* topk);
 int lik_maxsim_fwd(const lik_fwd_args* args, lik_stream_t stream);

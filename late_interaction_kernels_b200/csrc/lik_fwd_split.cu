@@ -21,7 +21,7 @@
 // 32 x 32 documents of 180 tokens 52 -> 25 us, 1 x 256 of 512 58 -> 40, 64 x 64 of 300 (48-token queries, 96 features) 397 -> 110,
 // 64 x 256 of 512 2926 -> 558 (one set of epilogue warps: 781); calls of 8 to 16 documents wait for the host either way (21 us).
 // Error of the scores against 64 bits, 2-norm over these shapes: 2.6e-8 to 5.2e-8, the other kernel's 4.1e-8 to 6.4e-8.
-// What bounds it: hand-shakes and the epilogue's chain per piece; the MMAs of a piece are 1500 cycles of about 3600.
+// What bounds it: instruction issue (68 % active; the tensor pipe 39 %): every document is cut again for each query tile.
 // Every wait is bounded: on expiry the CTA raises LIK_DEV_WAIT_TIMEOUT in the status word, sets a shared abort flag, frees TMEM and
 // returns.
 #include "lik_common.cuh"
@@ -474,14 +474,18 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
           const int row = hw * 4 + i, slot = row / P.q.max_len, s = row - slot * P.q.max_len;
           Row8 r;
           r.a = r.b = make_float4(0.f, 0.f, 0.f, 0.f);
+          bool used = false;
           if (slot < nq) {
             long long r0;
             int ql;
             seq_bounds(P.q, q0 + slot, r0, ql, nullptr);
-            if (s < ql) r = load_row8(static_cast<const float*>(P.q.data) + (r0 + s) * P.q.row_stride + (on0 ? hl * 8 : 0), on0, on1);
+            if (s < ql) {
+              r = load_row8(static_cast<const float*>(P.q.data) + (r0 + s) * P.q.row_stride + (on0 ? hl * 8 : 0), on0, on1);
+              used = row_valid(P.q, r0 + s);  // (what padding holds must not send the tile to the chain)
+            }
           }
           float ss = 0.f;
-          fits = cut_row(r, place(a_smem, row, A_SLAB), A_PART, P.norm_q, ss) && fits;
+          fits = (cut_row(r, place(a_smem, row, A_SLAB), A_PART, P.norm_q, ss) || !used) && fits;
           if (hl == 0) ctl->q_inv[ts][row] = P.norm_q ? inv_norm(ss, P.eps) : 1.f;
         }
         const bool all = __all_sync(0xffffffffu, fits);
@@ -517,7 +521,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
           ctl->col_mul[slot][r_lo + hl] = P.norm_d ? mul * inv_norm(hl ? ss1 : ss0, P.eps) : mul;
           ctl->col_add[slot][r_lo + hl] = hl ? add1 : add0;
         }
-        const bool all = __all_sync(0xffffffffu, fits0 && fits1);
+        const bool all = __all_sync(0xffffffffu, (fits0 || add0 != 0.f) && (fits1 || add1 != 0.f));  // (tokens that do not count may hold anything)
         if (lane == 0) ctl->piece_odd[slot][cw] = all ? 0 : 1;
         fence_proxy_async();
         __syncwarp();

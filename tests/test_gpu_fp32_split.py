@@ -131,3 +131,18 @@ def test_rows_that_do_not_fit(where, value, normalize):
     assert torch.allclose(a[ok], b[ok], rtol=2e-6, atol=0 if normalize or abs(value) > 1e20 else 1e-5)
     if where != "document":  # the whole first tile (four queries) is taken by the chain
         assert torch.equal(a[:4].nan_to_num(1.5), b[:4].nan_to_num(1.5)) or torch.allclose(a[:4], b[:4], rtol=1e-6, equal_nan=True)
+
+
+def test_what_masked_rows_hold_does_not_matter():
+    """Padding of either side holds infinities and NaN: the scores are those with zeros there, bit for bit, with and without winners."""
+    from late_interaction_kernels_b200 import _ops
+
+    g = torch.Generator().manual_seed(8)
+    Q, D = torch.randn((9, 32, 128), generator=g).cuda(), torch.randn((20, 100, 128), generator=g).cuda()
+    qm, dm = _masks(9, 32, 20, 100, g)
+    want = _run(Q * qm[..., None], D * dm[..., None], 0, 3, qm, dm)
+    bad = torch.tensor([float("nan"), float("inf"), -float("inf"), 3e38], device="cuda").repeat(32)
+    Qn, Dn = torch.where(qm[..., None], Q, bad), torch.where(dm[..., None], D, bad)
+    assert torch.equal(_run(Qn, Dn, 0, 3, qm, dm), want)
+    s, am = _ops.forward(_ops.padded_spec(Qn, mask=qm), _ops.padded_spec(Dn, mask=dm), normalize=3, save_argmax=True, argmax_stride=32)
+    assert torch.equal(s.view(9, 20), want) and int(am.max()) < 100 and int(am.min()) >= -1
