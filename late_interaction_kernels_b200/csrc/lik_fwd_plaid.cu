@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(NUM_THREADS, CTAS_PER_SM) fwd_plaid_kernel(con
         // the values of eight tokens; the next eight's rows are on their way while these are finished
         float e[4][8];
 #pragma unroll
-        for (int p = 0; p < 4; ++p) plaid_values<CF32, CBF16, NBITS>(nx[p], tab, e[p]);
+        for (int p = 0; p < 4; ++p) plaid_values_near<CF32, CBF16, NBITS>(nx[p], tab, e[p]);
         if (grp + 1 < GROUPS) {
           load_rows(t, grp + 1);
         } else {

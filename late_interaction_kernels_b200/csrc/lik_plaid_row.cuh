@@ -99,7 +99,7 @@ __device__ __forceinline__ void plaid_features(const PlaidSrc& S, const PlaidRaw
 // (lanes whose features lie beyond the width pass zeros).  1.0f when the index is scored un-normalised.
 __device__ __forceinline__ float plaid_inv_norm(const PlaidSrc& S, const float (&e)[8]) {
   if (!S.normalize) return 1.f;
-  float even = 0.f, odd = 0.f;  // two sums of four squares, as the two-wide form below takes them
+  float even = 0.f, odd = 0.f;  // two chains of four
 #pragma unroll
   for (int i = 0; i < 8; i += 2) {
     even = fmaf(e[i], e[i], even);
@@ -194,107 +194,46 @@ __device__ __forceinline__ PlaidPiece<CF32, NBITS> plaid_piece(const char* cen, 
   return r;
 }
 
-// w's two 16-bit values plus a and b: the conversion and the addition in one instruction each, rounded once
-template <bool BF16>
-__device__ __forceinline__ void add_16(unsigned w, float& a, float& b) {
-  if (BF16)
-    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.bf16 %0, l, %0;\n\tadd.rn.f32.bf16 %1, h, %1;\n\t}" : "+f"(a), "+f"(b) : "r"(w));
-  else
-    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.f16 %0, l, %0;\n\tadd.rn.f32.f16 %1, h, %1;\n\t}" : "+f"(a), "+f"(b) : "r"(w));
+// two-wide forms of the same IEEE operations
+__device__ __forceinline__ void plaid_add2(float& a, float& b, float x, float y) {
+  asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%0, %1};\n\tmov.b64 q, {%2, %3};\n\tadd.rn.f32x2 p, p, q;\n\tmov.b64 {%0, %1}, p;\n\t}" : "+f"(a), "+f"(b) : "f"(x), "f"(y));
+}
+__device__ __forceinline__ void plaid_mul2(float& a, float& b, float m) {
+  asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%0, %1};\n\tmov.b64 q, {%2, %2};\n\tmul.rn.f32x2 p, p, q;\n\tmov.b64 {%0, %1}, p;\n\t}" : "+f"(a), "+f"(b) : "f"(m));
 }
 
-// the lane's eight values; tab: the table, an array in shared memory as such (its address then is part of the loads)
 template <bool CF32, bool CBF16, int NBITS>
 __device__ __forceinline__ void plaid_values(const PlaidPiece<CF32, NBITS>& r, const float* tab, float (&e)[8]) {
-  const char* t = reinterpret_cast<const char*>(tab);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    if constexpr (NBITS == 2) {
-      const float2 v = *reinterpret_cast<const float2*>(t + (i == 0 ? (r.w0 << 3) & 0x78u : (r.w0 >> (4 * i - 3)) & 0x78u));  // eight bytes per entry
-      e[2 * i] = v.x;
-      e[2 * i + 1] = v.y;
-    } else {
-      const unsigned w = NBITS == 4 ? r.w0 : (i < 2 ? r.w0 : r.w1);
-      auto at = [&](int k) {  // four times code k of the word
-        const int sh = NBITS * k - 2;
-        return (sh < 0 ? w << 2 : w >> sh) & (NBITS == 4 ? 0x3cu : 0x3fcu);
-      };
-      const int k = NBITS == 4 ? 2 * i : 2 * (i & 1);
-      e[2 * i] = *reinterpret_cast<const float*>(t + at(k));
-      e[2 * i + 1] = *reinterpret_cast<const float*>(t + at(k + 1));
-    }
-  }
   if constexpr (CF32) {
-    const unsigned w[8] = {r.c0.x, r.c0.y, r.c0.z, r.c0.w, r.c1.x, r.c1.y, r.c1.z, r.c1.w};
-#pragma unroll
-    for (int i = 0; i < 8; ++i) e[i] += __uint_as_float(w[i]);
+    e[0] = __uint_as_float(r.c0.x); e[1] = __uint_as_float(r.c0.y); e[2] = __uint_as_float(r.c0.z); e[3] = __uint_as_float(r.c0.w);
+    e[4] = __uint_as_float(r.c1.x); e[5] = __uint_as_float(r.c1.y); e[6] = __uint_as_float(r.c1.z); e[7] = __uint_as_float(r.c1.w);
   } else {
-    add_16<CBF16>(r.c0.x, e[0], e[1]);
-    add_16<CBF16>(r.c0.y, e[2], e[3]);
-    add_16<CBF16>(r.c0.z, e[4], e[5]);
-    add_16<CBF16>(r.c0.w, e[6], e[7]);
-  }
-}
-
-// The last step of four tokens of a half-warp: divided by their norms, where that is asked for.
-__device__ __forceinline__ void plaid_finish4(bool normalize, float (&e)[4][8], int lane, bool lane_on) {
-  if (!normalize) return;
-  const int hl = lane & 15;
-  float ss[4];
+    const unsigned w[4] = {r.c0.x, r.c0.y, r.c0.z, r.c0.w};
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    float even = 0.f, odd = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; i += 2) {
-      even = fmaf(e[u][i], e[u][i], even);
-      odd = fmaf(e[u][i + 1], e[u][i + 1], odd);
+    for (int i = 0; i < 4; ++i) {
+      if constexpr (CBF16) {
+        e[2 * i] = __uint_as_float(w[i] << 16);
+        e[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+      } else {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+        e[2 * i] = v.x;
+        e[2 * i + 1] = v.y;
+      }
     }
-    ss[u] = lane_on ? even + odd : 0.f;
   }
-  // (the sums pair lanes 8, 4, 2 and 1 apart, in that order, as the one-token reduction does)
-  const bool h8 = hl & 8, h4 = hl & 4;
-  const float a0 = (h8 ? ss[2] : ss[0]) + __shfl_xor_sync(0xffffffffu, h8 ? ss[0] : ss[2], 8);
-  const float a1 = (h8 ? ss[3] : ss[1]) + __shfl_xor_sync(0xffffffffu, h8 ? ss[1] : ss[3], 8);
-  float t = (h4 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, h4 ? a0 : a1, 4);
-  t += __shfl_xor_sync(0xffffffffu, t, 2);
-  t += __shfl_xor_sync(0xffffffffu, t, 1);
-  const float mine = inv_norm(t, 1e-12f);  // of token 2 * (bit 3) + (bit 2)
+  if constexpr (NBITS == 2) {
+    const char* t = reinterpret_cast<const char*>(tab);
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const float inv = __shfl_sync(0xffffffffu, mine, (lane & 16) | ((u >> 1) << 3) | ((u & 1) << 2));
-#pragma unroll
-    for (int i = 0; i < 8; ++i) e[u][i] *= inv;
-  }
-}
-
-// The same for two tokens of a quarter-warp, whose lane l has the features from 8 l and from 64 + 8 l on (e[2 u], e[2 u + 1] of token u):
-// the sums are the same numbers.
-__device__ __forceinline__ void plaid_finish2(bool normalize, float (&e)[4][8], int lane, bool on0, bool on1) {
-  if (!normalize) return;
-  float ss[4];
-#pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    float even = 0.f, odd = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; i += 2) {
-      even = fmaf(e[p][i], e[p][i], even);
-      odd = fmaf(e[p][i + 1], e[p][i + 1], odd);
+    for (int i = 0; i < 4; ++i) {
+      const unsigned at = i == 0 ? (r.w0 << 3) & 0x78u : (r.w0 >> (4 * i - 3)) & 0x78u;  // eight bytes per entry
+      const float2 v = *reinterpret_cast<const float2*>(t + at);
+      plaid_add2(e[2 * i], e[2 * i + 1], v.x, v.y);
     }
-    ss[p] = (p & 1 ? on1 : on0) ? even + odd : 0.f;
-  }
-  const float s0 = ss[0] + ss[1], s1 = ss[2] + ss[3];
-  const bool h4 = lane & 4;
-  float t = (h4 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, h4 ? s0 : s1, 4);
-  t += __shfl_xor_sync(0xffffffffu, t, 2);
-  t += __shfl_xor_sync(0xffffffffu, t, 1);
-  const float mine = inv_norm(t, 1e-12f);  // of token (bit 2)
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const float inv = __shfl_sync(0xffffffffu, mine, (lane & 24) | (u << 2));
+  } else {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      e[2 * u][i] *= inv;
-      e[2 * u + 1][i] *= inv;
+      const unsigned c = NBITS == 4 ? (r.w0 >> (4 * i)) & 15u : ((i < 4 ? r.w0 : r.w1) >> (8 * (i & 3))) & 255u;
+      e[i] += tab[c];
     }
   }
 }
@@ -330,14 +269,115 @@ __device__ __forceinline__ void plaid_decode_run(const PlaidSrc& S, const float*
         const int code = b + U < 16 ? __shfl_sync(0xffffffffu, code_cur, (lane & 16) | ((b + U + u) & 15)) : __shfl_sync(0xffffffffu, code_next, (lane & 16) | u);
         nx[u] = plaid_piece<CF32, NBITS>(cen, cen_pitch, code, res, res_pitch, min(c0 + b + U + u, t_max));
       }
-      float e[U][8];
-#pragma unroll
-      for (int u = 0; u < U; ++u) plaid_values<CF32, CBF16, NBITS>(cur[u], tab, e[u]);
-      plaid_finish4(S.normalize != 0, e, lane, lane_on);
+      float e[U][8], ss[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
+        plaid_values<CF32, CBF16, NBITS>(cur[u], tab, e[u]);
+        float even = 0.f, odd = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+          even = fmaf(e[u][i], e[u][i], even);
+          odd = fmaf(e[u][i + 1], e[u][i + 1], odd);
+        }
+        ss[u] = lane_on ? even + odd : 0.f;
+      }
+      float inv[U];
+      if (S.normalize) {
+        // (the sums pair lanes 8, 4, 2 and 1 apart, in that order, as the one-token reduction does)
+        const bool h8 = hl & 8, h4 = hl & 4;
+        const float a0 = (h8 ? ss[2] : ss[0]) + __shfl_xor_sync(0xffffffffu, h8 ? ss[0] : ss[2], 8);
+        const float a1 = (h8 ? ss[3] : ss[1]) + __shfl_xor_sync(0xffffffffu, h8 ? ss[1] : ss[3], 8);
+        float t = (h4 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, h4 ? a0 : a1, 4);
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        t += __shfl_xor_sync(0xffffffffu, t, 1);
+        const float mine = inv_norm(t, 1e-12f);  // of token 2 * (bit 3) + (bit 2)
+#pragma unroll
+        for (int u = 0; u < U; ++u) inv[u] = __shfl_sync(0xffffffffu, mine, (lane & 16) | ((u >> 1) << 3) | ((u & 1) << 2));
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (S.normalize) {
+#pragma unroll
+          for (int i = 0; i < 8; i += 2) plaid_mul2(e[u][i], e[u][i + 1], inv[u]);
+        }
         if (c0 + b + u < n && lane_on) sink(c0 + b + u, e[u]);
       }
+    }
+  }
+}
+
+// w's two 16-bit values plus a and b: the conversion and the addition in one instruction each, rounded once
+template <bool BF16>
+__device__ __forceinline__ void add_16(unsigned w, float& a, float& b) {
+  if (BF16)
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.bf16 %0, l, %0;\n\tadd.rn.f32.bf16 %1, h, %1;\n\t}" : "+f"(a), "+f"(b) : "r"(w));
+  else
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.f16 %0, l, %0;\n\tadd.rn.f32.f16 %1, h, %1;\n\t}" : "+f"(a), "+f"(b) : "r"(w));
+}
+
+// The same values for the scoring kernel that decodes (lik_fwd_plaid.cu), whose decoders are bound by issue: conversion and addition in one
+// instruction.  tab: an array in shared memory as such, so that its address is part of the loads.  (The stand-alone kernel above is slower with
+// this form: 25 000 documents decoded and scored for eight queries 618 -> 650 us.)
+template <bool CF32, bool CBF16, int NBITS>
+__device__ __forceinline__ void plaid_values_near(const PlaidPiece<CF32, NBITS>& r, const float* tab, float (&e)[8]) {
+  const char* t = reinterpret_cast<const char*>(tab);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if constexpr (NBITS == 2) {
+      const float2 v = *reinterpret_cast<const float2*>(t + (i == 0 ? (r.w0 << 3) & 0x78u : (r.w0 >> (4 * i - 3)) & 0x78u));  // eight bytes per entry
+      e[2 * i] = v.x;
+      e[2 * i + 1] = v.y;
+    } else {
+      const unsigned w = NBITS == 4 ? r.w0 : (i < 2 ? r.w0 : r.w1);
+      auto at = [&](int k) {  // four times code k of the word
+        const int sh = NBITS * k - 2;
+        return (sh < 0 ? w << 2 : w >> sh) & (NBITS == 4 ? 0x3cu : 0x3fcu);
+      };
+      const int k = NBITS == 4 ? 2 * i : 2 * (i & 1);
+      e[2 * i] = *reinterpret_cast<const float*>(t + at(k));
+      e[2 * i + 1] = *reinterpret_cast<const float*>(t + at(k + 1));
+    }
+  }
+  if constexpr (CF32) {
+    const unsigned w[8] = {r.c0.x, r.c0.y, r.c0.z, r.c0.w, r.c1.x, r.c1.y, r.c1.z, r.c1.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) e[i] += __uint_as_float(w[i]);
+  } else {
+    add_16<CBF16>(r.c0.x, e[0], e[1]);
+    add_16<CBF16>(r.c0.y, e[2], e[3]);
+    add_16<CBF16>(r.c0.z, e[4], e[5]);
+    add_16<CBF16>(r.c0.w, e[6], e[7]);
+  }
+}
+
+// Two tokens of a quarter-warp, whose lane l has the features from 8 l and from 64 + 8 l on (e[2 u], e[2 u + 1] of token u), divided by
+// their norms, where that is asked for: the sums are the same numbers as above.
+__device__ __forceinline__ void plaid_finish2(bool normalize, float (&e)[4][8], int lane, bool on0, bool on1) {
+  if (!normalize) return;
+  float ss[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    float even = 0.f, odd = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+      even = fmaf(e[p][i], e[p][i], even);
+      odd = fmaf(e[p][i + 1], e[p][i + 1], odd);
+    }
+    ss[p] = (p & 1 ? on1 : on0) ? even + odd : 0.f;
+  }
+  const float s0 = ss[0] + ss[1], s1 = ss[2] + ss[3];
+  const bool h4 = lane & 4;
+  float t = (h4 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, h4 ? s0 : s1, 4);
+  t += __shfl_xor_sync(0xffffffffu, t, 2);
+  t += __shfl_xor_sync(0xffffffffu, t, 1);
+  const float mine = inv_norm(t, 1e-12f);  // of token (bit 2)
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const float inv = __shfl_sync(0xffffffffu, mine, (lane & 24) | (u << 2));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      e[2 * u][i] *= inv;
+      e[2 * u + 1][i] *= inv;
     }
   }
 }
