@@ -1,29 +1,43 @@
-// Exact fp32 scores on the tensor cores (sm_100a: tcgen05.mma + TMEM): every fp32 row is cut into three bf16 parts on its way into
-// shared memory, and six products of parts make a dot product.
+// fp32 scores on the tensor cores (sm_100a: tcgen05.mma + TMEM): rows cut into three bf16 parts, eight products of parts to a dot product,
+// a bound for what that is off, and dot products in fp32 where the bound says so.
 //
-// The cut.  Let 2^e be the power of two at or below the largest magnitude of a row.  a0 = the row rounded to multiples of 2^(e-7),
-// a1 = the rest rounded to multiples of 2^(e-15), a2 = what is left, rounded to bf16: at most 2^(e-25) is lost, a quarter of an ulp of the
-// largest element.  The tensor core adds into fp32 but cuts off below (measured: -0.3 ulp on average per 16 products of full bf16
-// values, -1.8 over 128), which would shift every score.  Here it has nothing to cut: products a0 b0 are whole multiples of one
-// unit, at most 2^16 of it, and 128 of them stay below 2^24; so do those of a0 b1 + a1 b0 of theirs; each has an accumulator
-// of its own.  The third, a0 b2 + a1 b1 + a2 b0, is 2^-16 of the first and may be cut.  The three are added in fp32, so a dot product
-// is rounded twice where a chain of fused multiply-adds rounds 128 times.
-// Rows that this does not fit (infinities, NaN, magnitudes beyond 2^50 or all below 2^-50, whose parts or products could leave fp32's range) are marked, and the epilogue takes
-// the dot products of a marked piece or query tile with such a chain itself: rare, slow, and what fwd_generic_kernel gives.
+// The cut.  Let 2^e be the power of two at or below the largest magnitude of a row a (its size).  a0 = the row rounded to multiples of 2^(e-7),
+// a1 = the rest rounded to multiples of 2^(e-15), a2 = what is left, rounded to bf16.  a0 b0 has an accumulator of its own, a0 b1 + a1 b0
+// another, the third a0 b2 + a1 b1 + a2 b0 + a1 b2 + a2 b1.  The tensor core adds into fp32 but cuts off below (measured: -0.3 ulp on average per 16
+// products of full bf16 values, -1.8 over 128, which would shift every score); in the first two it has nothing to cut, since their terms are
+// whole multiples of one unit and their sums stay below 2^24 of it.
+// The bound.  A product p~ of rows of sizes 2^e and 2^f and width n can be away from the true p by
+//   the cuts       2^(e-25) per feature of a, 2^(f-25) of b                                     2^-25 (2^e |b|_1 + 2^f |a|_1)
+//   third sum      40 MMAs, each off by 17 ulp of the sum at most: a1 b1, below n 2^(e+f-16)    n 2^(e+f-29.5)
+//                  a0 b2 + a2 b0, |a0| <= 2 |a|, below 2^-15 (2^e |b|_1 + 2^f |a|_1)            a twelfth of the first line
+//   left out       a2 b2                                                                        n 2^(e+f-32)
+//   sum of three   the second and third, below 2^-7 (2^e |b|_1 + 2^f |a|_1), rounded            2^-6 of the first line
+// in all below 1.25 times the first line + n 2^(e+f-29), and two roundings of p~ itself (the last sum, the column's multiplier).  It goes with the rows' sizes, not with p: on rows of even features p~
+// is off by two or three roundings, where one feature is 2^16 times the others it may be worth nothing.  Sizes and sums of magnitudes are
+// taken with the cut, the largest of them per piece, and the epilogue keeps, per query token, the largest p~ of a document and the columns
+// that could be the largest in truth: those within both bounds of it, in up to two groups of sixteen.
+// The answer.  One candidate whose bound is below max(4, n / 4) 2^-24 |p~|, a quarter of what a chain of n fused multiply-adds is bound by:
+// p~.  (Rows of independent Gaussian features, 128 wide, against the best of thirty: half of that.)  Else the candidates' dot products are
+// taken in fp32, eight features per lane, and the largest counts; where more than two groups could hold it, all tokens of the document are
+// taken that way, and so they are for rows that the cut does not fit (infinities, NaN, sizes beyond 2^50 or below 2^-40).
 //
 // A CTA per SM takes an equal run of (query tile, document) units, tile by tile, and walks a document in pieces of 64 tokens.
 // Warp roles (800 threads):
 //   warps 0..7   epilogue, a thread per query token: two sets of four warps take the pieces in turn; where a document ends, the set
-//                of its last piece gets the other's maxima through shared memory
-//   warp 8       issues the MMAs of a piece: six products x one per 16 features
+//                of its last piece gets the other's candidates through shared memory
+//   warp 8       issues the MMAs of a piece, a part of the query times up to three of the piece at once: five per 16 features
 //   warps 9..24  cut the rows of the pieces and, where it changes, of the query tile: a half-warp per row; they take the norms too
-// Against fwd_generic_kernel, whose fp32 FMAs bound it (queries of up to 32 tokens, documents a fifth to the whole of the length given):
-// 32 x 32 documents of 180 tokens 52 -> 25 us, 1 x 256 of 512 58 -> 40, 64 x 64 of 300 (48-token queries, 96 features) 397 -> 110,
-// 64 x 256 of 512 2926 -> 558 (one set of epilogue warps: 781); calls of 8 to 16 documents wait for the host either way (21 us).
-// Error of the scores against 64 bits, 2-norm over these shapes: 2.6e-8 to 5.2e-8, the other kernel's 4.1e-8 to 6.4e-8.
-// What bounds it: instruction issue (68 % active; the tensor pipe 39 %): every document is cut again for each query tile.
+// Against fwd_generic_kernel, whose fp32 FMAs bound it (queries of up to 32 tokens, documents a fifth to the whole of the length given, normalised):
+// 32 x 32 documents of 180 tokens 52 -> 29 us, 1 x 256 of 512 68 -> 51, 64 x 64 of 300 (48-token queries, 96 features) 418 -> 140, 64 x 256 of
+// 512 (48 tokens) 3010 -> 790; that last with a feature of the documents 100 or 1000 times the others, every product in fp32, 1150; with infinities in a query
+// of every tile 4800, in every sixteenth document 3600; with two features 2^16 times the others, each where the other side has zeros, so that everything
+// is gone through, 28 ms.  (Products for all rows instead of the bound: 32 x 32 35 us, 64 x 256 of 512 and 32 tokens 454 instead of 400; six parts' products
+// instead of eight are not enough for the bound.)
+// Error of the scores against 64 bits, 2-norm over 24 problems of Gaussian rows: 3.3e-8 to 4.7e-8, the other kernel's 5.1e-8 to 6.4e-8.
 // Every wait is bounded: on expiry the CTA raises LIK_DEV_WAIT_TIMEOUT in the status word, sets a shared abort flag, frees TMEM and
-// returns.
+// returns.  A warp that goes through a document counts its steps, and who waits for it begins anew while they go on.
+#include <cfloat>
+
 #include "lik_common.cuh"
 #include "lik_tc_ptx.cuh"
 
@@ -39,9 +53,11 @@ constexpr int STAGES = 2, ACCS = 2;
 constexpr int ACC_COLS = 256;                 // three accumulators of 64 columns, and a gap
 constexpr int RING = 4;                       // column arrays and query arrays: see `columns`
 constexpr int ROW_BYTES = 128;                // one swizzle span: 64 bf16
-constexpr int B_SLAB = PIECE * ROW_BYTES, B_PART = 2 * B_SLAB, B_STAGE = PARTS * B_PART;
+constexpr int B_PART = PIECE * ROW_BYTES, B_SLAB = PARTS * B_PART, B_STAGE = 2 * B_SLAB;  // (the parts of B are one matrix of 192 rows)
 constexpr int A_SLAB = TILE_M * ROW_BYTES, A_PART = 2 * A_SLAB;
 constexpr long long WAIT_LIMIT = 4000000000ll;
+// Candidates of a query token: columns at + i for bit i of `bits`, at2 + i for bit 16 + i
+constexpr int NO_MORE = -1, WHOLE_DOC = -2;  // instead of at2: no second group; all tokens
 static_assert(PIECE == 4 * CUT_WARPS && TILE_M == 8 * CUT_WARPS, "a half-warp cuts two rows of a piece and four of a query tile");
 
 struct SplitParams {
@@ -61,32 +77,41 @@ struct SharedCtl {
   unsigned long long b_full[STAGES], b_empty[STAGES];
   unsigned long long acc_full[ACCS], acc_empty[ACCS];
   unsigned long long epi_sync[2];
-  // maxima of the set without a document's last piece, on their way to the other.  It can be three pieces ahead, so two exchanges.
+  // candidates of the set without a document's last piece, on their way to the other.  It can be three pieces ahead, so two exchanges.
   unsigned long long x_full[4][4];  // by exchange and quadrant of rows
   uint32_t tmem_base;
   volatile int abort_flag;
+  SplitParams params;     // for `products`
+  volatile int progress;  // counts up while a scan of a document goes on: who waits for its warp starts again
   // A slot is written again four pieces (query tiles) later.  By then the MMAs of the piece two behind it have completed, for the
   // cutters waited for its stage; they had taken the accumulator that the epilogue of this piece gave back after its last look here.
   alignas(16) float col_mul[RING][PIECE], col_add[RING][PIECE];  // 0 or, for columns that are no valid token, -inf
-  alignas(16) unsigned char piece_odd[RING][CUT_WARPS];            // the rows that a warp cut do not fit
+  // of the counted rows that a warp cut, with their multipliers: the largest size (infinity: one does not fit) and the largest sum of magnitudes
+  alignas(16) float2 piece_size[RING][CUT_WARPS];
   float q_inv[RING][TILE_M];
-  alignas(16) unsigned char tile_odd[RING][CUT_WARPS];
+  float2 q_size[RING][TILE_M];
+  float2 x_size[4][4];
+  int4 x_row[4][TILE_M];          // largest p~, at, at2, bits
   float emit[2][2][TILE_M];
-  float x_max[4][TILE_M];
-  int x_idx[4][TILE_M];
 };
 
 __device__ __forceinline__ bool wait_bar(unsigned long long* bar, uint32_t parity, SharedCtl* ctl, int* status) {
   const uint32_t b = smem_u32(bar);
   if (__all_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
-  const long long t0 = clock64();
+  long long t0 = clock64();
+  int seen = ctl->progress;
   while (true) {
 #pragma unroll 1
     for (int i = 0; i < 16; ++i)
       if (__all_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
     if (clock64() - t0 > WAIT_LIMIT) {
-      ctl->abort_flag = 1;
-      if (status) atomicOr(status, LIK_DEV_WAIT_TIMEOUT);
+      const int now = ctl->progress;
+      if (now == seen) {
+        ctl->abort_flag = 1;
+        if (status) atomicOr(status, LIK_DEV_WAIT_TIMEOUT);
+      }
+      seen = now;
+      t0 = clock64();
     }
     if (__any_sync(0xffffffffu, ctl->abort_flag != 0)) return false;
   }
@@ -94,18 +119,16 @@ __device__ __forceinline__ bool wait_bar(unsigned long long* bar, uint32_t parit
 
 // The units of a CTA: unit = tile * n_d + document.
 struct Units {
-  long long u, end;
-  int tile, doc;
+  int left, tile, doc;  // (a CTA's share of the scores fits an int)
   __device__ __forceinline__ Units(const SplitParams& P) {
-    const long long n = (long long)P.n_tiles * P.n_d;
-    u = n * blockIdx.x / gridDim.x;
-    end = n * (blockIdx.x + 1) / gridDim.x;
+    const long long n = (long long)P.n_tiles * P.n_d, u = n * blockIdx.x / gridDim.x;
+    left = (int)(n * (blockIdx.x + 1) / gridDim.x - u);
     tile = (int)(u / P.n_d);
     doc = (int)(u - (long long)tile * P.n_d);
   }
-  __device__ __forceinline__ bool more() const { return u < end; }
+  __device__ __forceinline__ bool more() const { return left > 0; }
   __device__ __forceinline__ void next(const SplitParams& P) {
-    ++u;
+    --left;
     if (++doc == P.n_d) {
       doc = 0;
       ++tile;
@@ -132,9 +155,9 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&h);
 }
-// Cuts a row that a half-warp holds and stores its three parts at `dst` (+ 1, 2 strides).  Returns whether the row fits; ss: sum of
-// squares of the whole row, where wanted.
-__device__ __forceinline__ bool cut_row(const Row8& r, unsigned char* dst, int part_stride, bool want_ss, float& ss) {
+// Cuts a row that a half-warp holds and stores its three parts at `dst` (+ 1, 2 strides).  Returns the row's size 2^e: 0 for a row of zeros,
+// infinity for one that does not fit.
+__device__ __forceinline__ float cut_row(const Row8& r, unsigned char* dst, int part_stride) {
   const float x[8] = {r.a.x, r.a.y, r.a.z, r.a.w, r.b.x, r.b.y, r.b.z, r.b.w};
   // (as bit patterns of magnitudes: NaN lies above infinity)
   unsigned top = 0;
@@ -142,19 +165,8 @@ __device__ __forceinline__ bool cut_row(const Row8& r, unsigned char* dst, int p
   for (int i = 0; i < 8; ++i) top = max(top, __float_as_uint(x[i]) & 0x7fffffffu);
 #pragma unroll
   for (int o = 8; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
-  if (want_ss) {
-    float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; i += 2) {
-      s0 = fmaf(x[i], x[i], s0);
-      s1 = fmaf(x[i + 1], x[i + 1], s1);
-    }
-    ss = s0 + s1;
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  }
   const unsigned ex = top >> 23;  // biased exponent of the largest magnitude
-  const bool fits = top == 0 || (ex >= 77 && ex <= 177);
+  const bool fits = top == 0 || (ex >= 87 && ex <= 177);
   // adding and taking away 1.5 * 2^(e + 16) rounds to multiples of 2^(e - 7)
   const float m0 = __uint_as_float(((fits ? ex : 127u) + 16u) << 23 | 0x400000u), m1 = m0 * 0x1p-8f;
   uint32_t w[3][4];
@@ -175,22 +187,211 @@ __device__ __forceinline__ bool cut_row(const Row8& r, unsigned char* dst, int p
   }
 #pragma unroll
   for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(dst + p * part_stride) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
-  return fits;
+  return top == 0 ? 0.f : fits ? __uint_as_float(ex << 23) : INFINITY;
 }
 
-// The dot product as fwd_generic_kernel takes it.
-__device__ __noinline__ float chain_dot(const float* q, const float* d, int dim) {
-  float acc = 0.f;
-  for (int k = 0; k < dim; ++k) acc = fmaf(__ldg(q + k), __ldg(d + k), acc);
-  return acc;
+__device__ __forceinline__ float dot8(const Row8& x, const Row8& y) {
+  float s = x.a.x * y.a.x, t = x.a.y * y.a.y;
+  s = fmaf(x.a.z, y.a.z, s);
+  t = fmaf(x.a.w, y.a.w, t);
+  s = fmaf(x.b.x, y.b.x, s);
+  t = fmaf(x.b.y, y.b.y, t);
+  s = fmaf(x.b.z, y.b.z, s);
+  return s + fmaf(x.b.w, y.b.w, t);
+}
+__device__ __forceinline__ float squares8(const Row8& x) {
+  const float s = fmaf(x.b.z, x.b.z, fmaf(x.b.x, x.b.x, fmaf(x.a.z, x.a.z, x.a.x * x.a.x)));
+  return s + fmaf(x.b.w, x.b.w, fmaf(x.b.y, x.b.y, fmaf(x.a.w, x.a.w, x.a.y * x.a.y)));
+}
+__device__ __forceinline__ float magnitudes8(const Row8& x) {
+  return ((fabsf(x.a.x) + fabsf(x.a.y)) + (fabsf(x.a.z) + fabsf(x.a.w))) + ((fabsf(x.b.x) + fabsf(x.b.y)) + (fabsf(x.b.z) + fabsf(x.b.w)));
+}
+// Sums of four values over a half-warp, with the order of a sum over lanes 8, 4, 2 and 1 apart: lane hl gets that of value 2 (hl >> 3) + (hl >> 2 & 1).
+__device__ __forceinline__ float half_sums4(float a, float b, float c, float d, int lane) {
+  const bool h8 = lane & 8, h4 = lane & 4;
+  const float x0 = (h8 ? c : a) + __shfl_xor_sync(0xffffffffu, h8 ? a : c, 8);
+  const float x1 = (h8 ? d : b) + __shfl_xor_sync(0xffffffffu, h8 ? b : d, 8);
+  float t = (h4 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, h4 ? x0 : x1, 4);
+  t += __shfl_xor_sync(0xffffffffu, t, 2);
+  t += __shfl_xor_sync(0xffffffffu, t, 1);
+  return t;
+}
+
+__device__ __forceinline__ void better(float p, int i, float& best, int& who) {
+  if (i >= 0 && (p > best || (p == best && i < who))) {
+    best = p;
+    who = i;
+  }
+}
+// A document in memory, and what its tokens' products are multiplied by: NaN where a token does not count.
+struct Document {
+  const float* rows;
+  const unsigned char* mask;
+  const float* scale;
+  long long pitch;
+  float scalar, eps;  // eps < 0: no norms
+  int dim;
+  __device__ __forceinline__ Document(const SplitParams& P, long long row0)
+      : rows(static_cast<const float*>(P.d.data) + row0 * P.d.row_stride), mask(P.d.mask ? P.d.mask + row0 : nullptr), scale(P.d.scale ? P.d.scale + row0 : nullptr),
+        pitch(P.d.row_stride), scalar(P.d.scale_scalar), eps(P.norm_d ? P.eps : -1.f), dim(P.dim) {}
+  __device__ __forceinline__ float scaled(int t) const {
+    const float f = scale ? scalar * scale[t] : scalar;
+    return mask && !mask[t] ? __int_as_float(0x7fffffff) : f;
+  }
+  __device__ __forceinline__ float normed(float f, float ss) const { return eps >= 0.f ? f * inv_norm(ss, eps) : f; }
+};
+
+// The best of all tokens of a document, in fp32, for the rows of a warp that are set in `rows`: four rows at a time, held in registers, against four
+// tokens per step, a half-warp per token.  A lane gets its row's largest product and whose it is, < 0: no token counts, or every product is a NaN
+// or -inf.  The sums are those of `products`.
+__device__ __noinline__ int2 whole_document(const Document& doc, unsigned rows, const float* q_tile, long long q_off, int len, int* progress) {
+  const int lane = threadIdx.x & 31, hl = lane & 15, half = lane >> 4;
+  const Document D = doc;
+  const bool on0 = hl * 8 < D.dim, on1 = hl * 8 + 4 < D.dim;
+  const float* d_lane = D.rows + (on0 ? hl * 8 : 0);
+  q_tile += on0 ? hl * 8 : 0;
+  int2 mine = make_int2(0, 0);
+  while (rows) {
+    const unsigned first = rows;  // the four rows: its lowest bits (fewer: the last again)
+    Row8 q[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      q[r] = load_row8(q_tile + __shfl_sync(0xffffffffu, q_off, __ffs(rows) - 1), on0, on1);
+      if (r == 3 || (rows & (rows - 1))) rows &= rows - 1;
+    }
+    float best = -INFINITY;  // of row hl >> 2 and this lane's tokens
+    int who = -1;
+#pragma unroll 1
+    for (int t = 0; t < len; t += 4) {
+      const int tok = t + 2 * half + (hl >> 1 & 1);
+      const Row8 x = load_row8(d_lane + min(t + 2 * half, len - 1) * D.pitch, on0, on1), y = load_row8(d_lane + min(t + 2 * half + 1, len - 1) * D.pitch, on0, on1);
+      const float f = D.scaled(min(tok, len - 1));
+      float v[8];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        v[2 * r] = dot8(q[r], x);
+        v[2 * r + 1] = dot8(q[r], y);
+      }
+      const float sx = squares8(x), sy = squares8(y);
+#pragma unroll
+      for (int o = 8; o >= 2; o >>= 1) {  // lane hl ends with the sum of value hl >> 1
+        const bool up = lane & o;
+#pragma unroll
+        for (int k = 0; k < o / 2; ++k) v[k] = (up ? v[k + o / 2] : v[k]) + __shfl_xor_sync(0xffffffffu, up ? v[k] : v[k + o / 2], o);
+      }
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+      const float ss = __shfl_sync(0xffffffffu, half_sums4(sx, sy, sx, sy, lane), (lane & 16) | (lane & 2) << 1);
+      if (tok < len) better(v[0] * D.normed(f, ss), tok, best, who);
+      if ((t & 255) == 0 && lane == 0) atomicAdd(progress, 1);
+    }
+#pragma unroll
+    for (int o = 2; o <= 16; o <<= 3) better(__shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, who, o), best, who);
+    unsigned left = first;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float b = __shfl_sync(0xffffffffu, best, r * 4);
+      const int i = __shfl_sync(0xffffffffu, who, r * 4);
+      if (left && lane == __ffs(left) - 1) mine = make_int2(__float_as_int(b), i);
+      left &= left - 1;
+    }
+  }
+  return mine;
+}
+
+// Products in fp32 for the rows of a warp that need them (`what`): a lane gives its row's candidates and gets their largest and who it is.
+// (Not inlined: its registers would cost the epilogue's loop over the columns its own.)
+enum Need { NOTHING, ONE, MANY, ALL };
+__device__ __noinline__ int2 products(SharedCtl* ctl, int what, int tile, long long drow0, int len, int at, int at2, unsigned bits, int row) {
+  const SplitParams& P = ctl->params;
+  const Document D(P, drow0);
+  const int lane = row & 31, hl = lane & 15, ml = P.q.max_len;
+  const bool on0 = hl * 8 < D.dim, on1 = hl * 8 + 4 < D.dim;
+  const long long pitch = D.pitch, q_stride = P.q.row_stride;
+  const float* d_lane = D.rows + (on0 ? hl * 8 : 0);
+  const float* q_tile = static_cast<const float*>(P.q.data) + (long long)tile * P.q_per_tile * P.q.seq_stride * q_stride;
+  const long long q_off = ((row / ml) * P.q.seq_stride + row % ml) * q_stride;  // of the lane's row in the tile
+  const float* q_lane = q_tile + (on0 ? hl * 8 : 0);
+  const int tok = at + __ffs(bits) - 1;
+  float r = -INFINITY;
+  int ri = -1;
+  // one candidate: a row per half-warp, two at a time
+  const unsigned ones = __ballot_sync(0xffffffffu, what == ONE);
+  float dot = 0.f, ss = 0.f;
+#pragma unroll 1
+  for (unsigned both = (ones | ones >> 16) & 0xffffu; both;) {
+    int i[2];
+    i[0] = __ffs(both) - 1;
+    both &= both - 1;
+    i[1] = both ? __ffs(both) - 1 : i[0];
+    both &= both - 1;
+    Row8 q[2], d[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int from = (lane & 16) | i[k];
+      const bool on = ones >> from & 1;
+      q[k] = load_row8(q_lane + __shfl_sync(0xffffffffu, q_off, from), on && on0, on && on1);
+      d[k] = load_row8(d_lane + __shfl_sync(0xffffffffu, tok, from) * pitch, on && on0, on && on1);
+    }
+    const float s = half_sums4(dot8(q[0], d[0]), squares8(d[0]), dot8(q[1], d[1]), squares8(d[1]), lane);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float x = __shfl_sync(0xffffffffu, s, (lane & 16) | k * 8), y = __shfl_sync(0xffffffffu, s, (lane & 16) | k * 8 | 4);
+      if (hl == i[k]) {
+        dot = x;
+        ss = y;
+      }
+    }
+  }
+  if (what == ONE) {
+    r = dot * D.normed(D.scaled(tok), ss);
+    ri = tok;
+  }
+  // several: row by row, four candidates at a time
+  for (unsigned rows = __ballot_sync(0xffffffffu, what == MANY); rows; rows &= rows - 1) {
+    const int from = __ffs(rows) - 1, a0 = __shfl_sync(0xffffffffu, at, from), a1 = __shfl_sync(0xffffffffu, at2, from) - 16;
+    const Row8 q = load_row8(q_lane + __shfl_sync(0xffffffffu, q_off, from), on0, on1);
+    float best = -INFINITY;
+    int who = -1;
+#pragma unroll 1
+    for (unsigned left = __shfl_sync(0xffffffffu, bits, from); left;) {
+      int t[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int b = __ffs(left) - 1;
+        t[k] = b < 0 ? t[0] : b + (b < 16 ? a0 : a1);
+        left &= left - 1;
+      }
+      const int ta = lane & 16 ? t[2] : t[0], tb = lane & 16 ? t[3] : t[1], mine = lane & 8 ? tb : ta;
+      const float f = D.scaled(mine);
+      const Row8 x = load_row8(d_lane + ta * pitch, on0, on1), y = load_row8(d_lane + tb * pitch, on0, on1);
+      const float s = half_sums4(dot8(q, x), squares8(x), dot8(q, y), squares8(y), lane);
+      const float p = __shfl_sync(0xffffffffu, s, lane & 24), y2 = __shfl_sync(0xffffffffu, s, (lane & 24) | 4);
+      better(p * D.normed(f, y2), mine, best, who);
+    }
+#pragma unroll
+    for (int o = 8; o <= 16; o <<= 1) better(__shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, who, o), best, who);
+    if (lane == from) {
+      r = best;
+      ri = who;
+    }
+  }
+  const unsigned alls = __ballot_sync(0xffffffffu, what == ALL);
+  if (alls) {
+    const int2 x = whole_document(D, alls, q_tile, q_off, len, const_cast<int*>(&ctl->progress));
+    if (what == ALL) {
+      r = __int_as_float(x.x);
+      ri = x.y;
+    }
+  }
+  return make_int2(__float_as_int(r), ri);
 }
 
 template <bool WINNERS>
-__global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitParams P) {
+__global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const __grid_constant__ SplitParams P) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
   unsigned char* a_smem = smem;                           // [3 parts][2 slabs][128 rows][128 B]
-  unsigned char* b_smem = smem + PARTS * A_PART;          // [stages][3 parts][2 slabs][64 rows][128 B]
+  unsigned char* b_smem = smem + PARTS * A_PART;          // [stages][2 slabs][3 parts][64 rows][128 B]
   SharedCtl* ctl = reinterpret_cast<SharedCtl*>(b_smem + STAGES * B_STAGE);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
@@ -207,6 +408,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
     for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&ctl->epi_sync[i]), 4);
     for (int i = 0; i < 16; ++i) mbar_init(smem_u32(&ctl->x_full[i >> 2][i & 3]), 1);
     ctl->abort_flag = 0;
+    ctl->progress = 0;
+    ctl->params = P;
     fence_barrier_init();
   }
   if (warp == ISSUE_WARP) {
@@ -237,29 +440,28 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
         cur = w.tile;
         ok = wait_bar(&ctl->a_full, n_tile++ & 1, ctl, P.status);
       }
-      const bool tile_ends = w.u + 1 == w.end || w.doc + 1 == P.n_d;
+      const bool tile_ends = w.left == 1 || w.doc + 1 == P.n_d;
       for (int c0 = 0; ok && (c0 == 0 || c0 < len); c0 += PIECE, ++n) {
         const uint32_t st = n % STAGES, acc = n % ACCS;
         ok = wait_bar(&ctl->acc_empty[acc], ((n / ACCS) & 1) ^ 1, ctl, P.status) && wait_bar(&ctl->b_full[st], (n / STAGES) & 1, ctl, P.status);
         if (!ok) break;
         tc_fence_after();
         if (issue) {
-          const int cols = max(16, (min(PIECE, len - c0) + 15) & ~15);
-          const uint32_t idesc = instr_desc(1, cols), d = tmem_base + acc * ACC_COLS, b = b0 + st * (B_STAGE >> 4);
-          // product of part i of A and part j of B into accumulator i + j
-          auto product = [&](int i, int j, bool first) {
+          const uint32_t d = tmem_base + acc * ACC_COLS, b = b0 + st * (B_STAGE >> 4);
+          // part i of A times parts j .. j + n - 1 of B, into accumulators `to` and on
+          auto product = [&](int i, int j, int n, int to, bool first) {
+            const uint32_t idesc = instr_desc(1, n * PIECE);
 #pragma unroll
             for (int k = 0; k < 8; ++k)
               if (k < k_steps)
-                tc_mma<false>(d + (i + j) * PIECE, a0 + i * (A_PART >> 4) + (k & 3) * 2 + (k >> 2) * (A_SLAB >> 4),
+                tc_mma<false>(d + to * PIECE, a0 + i * (A_PART >> 4) + (k & 3) * 2 + (k >> 2) * (A_SLAB >> 4),
                               b + j * (B_PART >> 4) + (k & 3) * 2 + (k >> 2) * (B_SLAB >> 4), desc_hi, idesc, first && k == 0 ? 0u : 1u);
           };
-          product(0, 0, true);
-          product(0, 1, true);
-          product(1, 0, false);
-          product(0, 2, true);
-          product(1, 1, false);
-          product(2, 0, false);
+          product(0, 0, 3, 0, true);
+          product(1, 0, 2, 1, false);
+          product(1, 2, 1, 2, false);
+          product(2, 0, 1, 2, false);
+          product(2, 1, 1, 2, false);
           tc_commit(smem_u32(&ctl->b_empty[st]));
           tc_commit(smem_u32(&ctl->acc_full[acc]));
           if (tile_ends && c0 + PIECE >= len) tc_commit(smem_u32(&ctl->a_empty));
@@ -274,11 +476,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
     uint32_t n = 0, n_tile = 0, n_sync = 0, n_emit = 0, n_x = 0;
     int cur = -1;
     const int ml = P.q.max_len;
-    const bool lone = ml == 32;  // a query per warp
     const int my_slot = row / ml, my_s = row - my_slot * ml;
     bool have = false, counts = false;
     float qf = 0.f;
-    const float* q_row = nullptr;
+    const float c_sums = 0x1.4p-24f, c_sizes = (float)P.dim * 0x1p-28f;  // both bounds of a comparison
+    const bool lone = ml == 32;  // a query per warp
+    const float enough = fmaxf(4.f, (float)P.dim * 0.25f) * 0x1p-23f;  // what both bounds may be of a product
     for (; ok && w.more(); w.next(P)) {
       long long drow0;
       const int len = doc_length(P, w.doc, drow0, tid == 0 ? P.status : nullptr);
@@ -298,7 +501,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
           }
           have = my_s < ql;
           if (have) {
-            q_row = static_cast<const float*>(P.q.data) + (r0 + my_s) * P.q.row_stride;
             counts = row_valid(P.q, r0 + my_s);
             qf = row_factor(P.q, r0 + my_s);
           }
@@ -306,8 +508,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
       }
       const uint32_t ts = (n_tile - 1) % RING;
       const bool any = __any_sync(0xffffffffu, have);
-      float r = -INFINITY, f = 0.f;
-      int ri = -1;
+      float r = -FLT_MAX, f = 0.f;  // the largest p~
+      float2 q_size = make_float2(0.f, 0.f), d_size = make_float2(0.f, 0.f);
+      int at = 0, at2 = NO_MORE;
+      unsigned bits = 0;
+      // twice the bound for this row and the document so far
+      auto bounds = [&]() { return fmaf(q_size.x, fmaf(c_sums, d_size.y, c_sizes * d_size.x), q_size.y * (c_sums * d_size.x)); };
       const int pieces = max(1, (len + PIECE - 1) / PIECE);
       const bool mine = ((n + pieces - 1) & 1) == set;  // the document's last piece
       for (int p = 0; p < pieces; ++p, ++n) {
@@ -318,13 +524,18 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
         if (!ok) break;
         tc_fence_after();
         const int cols = min(PIECE, len - c0);
-        // (sixteen bytes each: any of the pieces' or the tile's rows that do not fit)
-        const uint4 po = *reinterpret_cast<const uint4*>(ctl->piece_odd[slot]), to = *reinterpret_cast<const uint4*>(ctl->tile_odd[ts]);
-        const bool odd = (po.x | po.y | po.z | po.w | to.x | to.y | to.z | to.w) != 0;
-        if (any && !odd) {
+#pragma unroll
+        for (int i = 0; i < CUT_WARPS; i += 2) {
+          const float4 x = *reinterpret_cast<const float4*>(&ctl->piece_size[slot][i]);
+          d_size.x = max3(d_size.x, x.x, x.z);
+          d_size.y = max3(d_size.y, x.y, x.w);
+        }
+        if (any) {
+          q_size = ctl->q_size[ts][row];
+          const float both = bounds();
 #pragma unroll 1
           for (int c = 0; c < cols; c += 16) {
-            float v[16], p1[16], p2[16];
+            float v[16], p[16];
             const uint32_t t = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * ACC_COLS + c;
             auto ld16 = [](uint32_t addr, float (&x)[16]) {
               asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
@@ -337,43 +548,44 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
               asm volatile("" : "+f"(x[0]), "+f"(x[1]), "+f"(x[2]), "+f"(x[3]), "+f"(x[4]), "+f"(x[5]), "+f"(x[6]), "+f"(x[7]), "+f"(x[8]), "+f"(x[9]),
                                 "+f"(x[10]), "+f"(x[11]), "+f"(x[12]), "+f"(x[13]), "+f"(x[14]), "+f"(x[15]));
             };
-            ld16(t, v);
-            ld16(t + PIECE, p1);
-            ld16(t + 2 * PIECE, p2);
+            ld16(t + PIECE, v);
+            ld16(t + 2 * PIECE, p);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             held16(v);
-            held16(p1);
-            held16(p2);
+            held16(p);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) p[i] += v[i];
+            ld16(t, v);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            held16(v);
 #pragma unroll
             for (int i = 0; i < 16; i += 4) {
               const float4 mul = *reinterpret_cast<const float4*>(&ctl->col_mul[slot][c + i]), add = *reinterpret_cast<const float4*>(&ctl->col_add[slot][c + i]);
               // (a NaN beats nothing; columns that are no valid token end as -inf or NaN)
-              v[i] = fmaf(v[i] + (p1[i] + p2[i]), mul.x, add.x);
-              v[i + 1] = fmaf(v[i + 1] + (p1[i + 1] + p2[i + 1]), mul.y, add.y);
-              v[i + 2] = fmaf(v[i + 2] + (p1[i + 2] + p2[i + 2]), mul.z, add.z);
-              v[i + 3] = fmaf(v[i + 3] + (p1[i + 3] + p2[i + 3]), mul.w, add.w);
+              v[i] = fmaf(v[i] + p[i], mul.x, add.x);
+              v[i + 1] = fmaf(v[i + 1] + p[i + 1], mul.y, add.y);
+              v[i + 2] = fmaf(v[i + 2] + p[i + 2], mul.z, add.z);
+              v[i + 3] = fmaf(v[i + 3] + p[i + 3], mul.w, add.w);
             }
             const float m = fmaxf(max3(max3(v[0], v[1], v[2]), max3(v[3], v[4], v[5]), max3(v[6], v[7], v[8])),
                                   max3(max3(v[9], v[10], v[11]), max3(v[12], v[13], v[14]), v[15]));
-            if (WINNERS) {
-              const bool better = m > r;
-              if (__any_sync(0xffffffffu, better)) {  // the first column that has it
-                int at = 0;
+            const float gap = fmaf(fabsf(m) + fabsf(r), 0x1p-22f, both);
+            const bool candidate = m > r - gap;
+            if (__any_sync(0xffffffffu, candidate)) {
+              const float least = m - fmaf(fabsf(m), 0x1p-21f, both);
+              unsigned near = 0;
 #pragma unroll
-                for (int i = 15; i >= 0; --i) at = v[i] == m ? i : at;
-                ri = better ? c0 + c + at : ri;
+              for (int i = 0; i < 16; ++i) near |= v[i] >= least ? 1u << i : 0u;
+              if (m > r + gap) {
+                at = c0 + c;
+                at2 = NO_MORE;
+                bits = near;
+              } else if (candidate) {
+                at2 = at2 == NO_MORE ? c0 + c : WHOLE_DOC;
+                bits |= near << 16;
               }
             }
             r = fmaxf(r, m);
-          }
-        } else if (odd && have) {
-          for (int c = 0; c < cols; ++c) {
-            if (ctl->col_add[slot][c] != 0.f) continue;
-            const float x = chain_dot(q_row, static_cast<const float*>(P.d.data) + (drow0 + c0 + c) * P.d.row_stride, P.dim) * ctl->col_mul[slot][c];
-            if (x > r) {
-              r = x;
-              ri = c0 + c;
-            }
           }
         }
         // (what the tile's slot holds is looked at before the accumulator goes back)
@@ -386,23 +598,52 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
       if (pieces > 1) {
         const uint32_t x = n_x % 4;
         if (!mine) {
-          ctl->x_max[x][row] = r;
-          if (WINNERS) ctl->x_idx[x][row] = ri;
+          ctl->x_row[x][row] = make_int4(__float_as_int(r), at, at2, (int)bits);
+          if (lane == 0) ctl->x_size[x][quad] = d_size;
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&ctl->x_full[x][quad]));
         } else {
           ok = wait_bar(&ctl->x_full[x][quad], (n_x / 4) & 1, ctl, P.status);
           if (!ok) break;
-          const float xr = ctl->x_max[x][row];
-          if (WINNERS) {
-            const int xi = ctl->x_idx[x][row];
-            if (xr > r || (xr == r && (unsigned)xi < (unsigned)ri)) ri = xi;
+          const int4 o = ctl->x_row[x][row];
+          const float2 o_size = ctl->x_size[x][quad];
+          d_size = make_float2(fmaxf(d_size.x, o_size.x), fmaxf(d_size.y, o_size.y));
+          if (o.w) {
+            const float xr = __int_as_float(o.x), gap = fmaf(fabsf(xr) + fabsf(r), 0x1p-22f, bounds());
+            if (!bits || xr > r + gap || (xr == r && gap == 0.f && o.y < at)) {
+              r = xr;
+              at = o.y;
+              at2 = o.z;
+              bits = (unsigned)o.w;
+            } else if (xr > r - gap) {
+              at2 = at2 == NO_MORE && o.z == NO_MORE ? o.y : WHOLE_DOC;
+              bits |= (unsigned)o.w << 16;
+              r = fmaxf(r, xr);
+            }
           }
-          r = fmaxf(r, xr);
         }
         ++n_x;
       }
       if (!mine) continue;
+      int ri = -1;
+      {
+        const float both = bounds();  // 0: a row of zeros on either side; infinity, NaN: there is no bound
+        if (bits) ri = at + __ffs(bits) - 1;
+        const bool will_do = bits && both < INFINITY && both <= fabsf(r) * enough;  // r is the score as it is
+        const bool live = WINNERS ? have : counts && !will_do;
+        if (!bits) r = -INFINITY;
+        int what = NOTHING;
+        if (live && (at2 == WHOLE_DOC || !(both < INFINITY))) what = ALL;
+        else if (live && both != 0.f && (bits & (bits - 1))) what = MANY;
+        else if (counts && !will_do && both != 0.f && bits) what = ONE;
+        if (__any_sync(0xffffffffu, what != NOTHING)) {
+          const int2 x = products(ctl, what, w.tile, drow0, len, at, at2, bits, row);
+          if (what != NOTHING) {
+            if (!will_do) r = __int_as_float(x.x);
+            ri = x.y;
+          }
+        }
+      }
       const float val = counts && r != -INFINITY ? r * f : 0.f;
       if (WINNERS && my_slot < nq) {
         int* out = P.argmax + ((long long)(q0 + my_slot) * P.n_d + w.doc) * P.argmax_stride;
@@ -438,21 +679,17 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
     bool ok = true;
     const int r_lo = hw * 2;  // this half-warp's rows of a piece: r_lo, r_lo + 1
     Row8 nx[2];
-    float nx_mul[2], nx_add[2];
+    float nx_mul = 0.f;  // multiplier of row r_lo + (hl >> 3); NaN: the token does not count
     auto load_piece = [&](long long row0, int len, int c0) {
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int c = c0 + r_lo + i;
         const bool on = c < len;
-        const long long dr = row0 + (on ? c : 0);
-        nx[i] = load_row8(dbase + dr * P.d.row_stride, on && on0, on && on1);
-        nx_mul[i] = 1.f;
-        nx_add[i] = -INFINITY;
-        if (on && row_valid(P.d, dr)) {
-          nx_mul[i] = row_factor(P.d, dr);
-          nx_add[i] = 0.f;
-        }
+        nx[i] = load_row8(dbase + (row0 + (on ? c : 0)) * P.d.row_stride, on && on0, on && on1);
       }
+      const int c = c0 + r_lo + (hl >> 3);
+      nx_mul = __int_as_float(0x7fffffff);
+      if (c < len && row_valid(P.d, row0 + c)) nx_mul = row_factor(P.d, row0 + c);
     };
     long long row0 = 0;
     int len = 0;
@@ -468,7 +705,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
         if (!ok) break;
         ++n_tile;
         const int q0 = w.tile * P.q_per_tile, nq = min(P.q_per_tile, P.n_q - q0);
-        bool fits = true;
 #pragma unroll 1
         for (int i = 0; i < 4; ++i) {
           const int row = hw * 4 + i, slot = row / P.q.max_len, s = row - slot * P.q.max_len;
@@ -481,15 +717,17 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
             seq_bounds(P.q, q0 + slot, r0, ql, nullptr);
             if (s < ql) {
               r = load_row8(static_cast<const float*>(P.q.data) + (r0 + s) * P.q.row_stride + (on0 ? hl * 8 : 0), on0, on1);
-              used = row_valid(P.q, r0 + s);  // (what padding holds must not send the tile to the chain)
+              used = row_valid(P.q, r0 + s);
             }
           }
-          float ss = 0.f;
-          fits = (cut_row(r, place(a_smem, row, A_SLAB), A_PART, P.norm_q, ss) || !used) && fits;
-          if (hl == 0) ctl->q_inv[ts][row] = P.norm_q ? inv_norm(ss, P.eps) : 1.f;
+          const float size = cut_row(r, place(a_smem, row, A_SLAB), A_PART);
+          const float sums = half_sums4(P.norm_q ? squares8(r) : 0.f, magnitudes8(r), 0.f, 0.f, lane), sum = __shfl_xor_sync(0xffffffffu, sums, 4);
+          if (hl == 0) {
+            ctl->q_inv[ts][row] = P.norm_q ? inv_norm(sums, P.eps) : 1.f;
+            // (what padding holds must send nobody through the document)
+            ctl->q_size[ts][row] = used || size < INFINITY ? make_float2(size, sum) : make_float2(0.f, 0.f);
+          }
         }
-        const bool all = __all_sync(0xffffffffu, fits);
-        if (lane == 0) ctl->tile_odd[ts][cw] = all ? 0 : 1;
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&ctl->a_full));
@@ -497,7 +735,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
       for (int c0 = 0; ok && (c0 == 0 || c0 < len); ++n) {
         const uint32_t st = n % STAGES, slot = n % RING;
         const Row8 x0 = nx[0], x1 = nx[1];
-        const float mul0 = nx_mul[0], mul1 = nx_mul[1], add0 = nx_add[0], add1 = nx_add[1];
+        float mul = nx_mul;
         // the next piece's rows are on their way while these are cut
         c0 += PIECE;
         const bool doc_done = c0 >= len;
@@ -513,16 +751,25 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const SplitPa
         ok = wait_bar(&ctl->b_empty[st], ((n / STAGES) & 1) ^ 1, ctl, P.status);
         if (!ok) break;
         unsigned char* stage = b_smem + st * B_STAGE;
-        float ss0 = 0.f, ss1 = 0.f;
-        const bool fits0 = cut_row(x0, place(stage, r_lo, B_SLAB), B_PART, P.norm_d, ss0);
-        const bool fits1 = cut_row(x1, place(stage, r_lo + 1, B_SLAB), B_PART, P.norm_d, ss1);
-        if (hl < 2) {
-          const float mul = hl ? mul1 : mul0;
-          ctl->col_mul[slot][r_lo + hl] = P.norm_d ? mul * inv_norm(hl ? ss1 : ss0, P.eps) : mul;
-          ctl->col_add[slot][r_lo + hl] = hl ? add1 : add0;
+        const float size0 = cut_row(x0, place(stage, r_lo, B_SLAB), B_PART), size1 = cut_row(x1, place(stage, r_lo + 1, B_SLAB), B_PART);
+        const float sums = half_sums4(P.norm_d ? squares8(x0) : 0.f, magnitudes8(x0), P.norm_d ? squares8(x1) : 0.f, magnitudes8(x1), lane);
+        const float sum = __shfl_xor_sync(0xffffffffu, sums, 4);
+        unsigned size = 0, most = 0;
+        if ((hl & 7) == 0) {  // a lane per row
+          const bool counts = mul == mul;
+          if (!counts) mul = 1.f;
+          if (P.norm_d) mul *= inv_norm(sums, P.eps);
+          ctl->col_mul[slot][r_lo + (hl >> 3)] = mul;
+          ctl->col_add[slot][r_lo + (hl >> 3)] = counts ? 0.f : -INFINITY;
+          if (counts) {  // (tokens that do not count may hold anything)
+            const float x = (hl ? size1 : size0) * fabsf(mul), y = sum * fabsf(mul);
+            size = __float_as_uint(x < 0x1p60f ? (x > 0.f ? fmaxf(x, 0x1p-70f) : 0.f) : INFINITY);
+            most = __float_as_uint(y < 0x1p60f ? (y > 0.f ? fmaxf(y, 0x1p-70f) : 0.f) : INFINITY);
+          }
         }
-        const bool all = __all_sync(0xffffffffu, (fits0 || add0 != 0.f) && (fits1 || add1 != 0.f));  // (tokens that do not count may hold anything)
-        if (lane == 0) ctl->piece_odd[slot][cw] = all ? 0 : 1;
+        size = __reduce_max_sync(0xffffffffu, size);
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (lane == 0) ctl->piece_size[slot][cw] = make_float2(__uint_as_float(size), __uint_as_float(most));
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&ctl->b_full[st]));
@@ -549,9 +796,9 @@ static_assert(SMEM_BYTES <= 227 * 1024, "a block's shared memory");
 
 }  // namespace
 
-// fp32 cross products whose queries fit a tile and whose rows can be read sixteen bytes at a time; no size is too small (8 documents: even).
+// fp32 cross products whose queries fit a tile and whose rows can be read sixteen bytes at a time.
 bool fwd_split_supported(const lik_fwd_args& a) {
-  if (a.dtype != LIK_F32 || a.engine != 0 || a.pairing != LIK_PAIR_CROSS) return false;
+  if (a.dtype != LIK_F32 || (a.engine != 0 && a.engine != 3) || a.pairing != LIK_PAIR_CROSS) return false;
   if (a.dim % 4 != 0 || a.dim > 128 || a.q.cu || a.q.max_len < 1 || a.q.max_len > TILE_M) return false;
   if (a.q.n_seq <= 0 || a.d.n_seq <= 0 || a.q.n_rows <= 0 || a.d.n_rows <= 0) return false;
   if (a.q.row_stride % 4 != 0 || a.d.row_stride % 4 != 0 || ((uintptr_t)a.q.data & 15) || ((uintptr_t)a.d.data & 15)) return false;

@@ -1,14 +1,15 @@
-"""fp32 scores on the tensor cores (rows cut into three parts) against the fused multiply-add kernel (``engine=1``) and against
-64 bits, at the edges of pieces and tiles, on rows that the cut does not fit, and on integers, where both must be exact.
+"""fp32 scores on the tensor cores (rows cut into three parts, a bound per product, dot products in fp32 where the bound is too wide) against
+the fused multiply-add kernel (``engine=1``) and against 64 bits: at the edges of pieces and tiles, on rows whose features differ much in size, on
+rows that the cut does not fit, where products tie, and on integers, where both kernels must be exact.
 
-Bound used on real data: a dot product is two roundings of a result and what the cut loses, 2^-25 of the largest magnitudes of
-either row per feature: |error| <= (2^-23 + 2 * 128 * 2^-25 * f) |q| |d| with f = max / norm of a row, below 1e-5 |q| |d| for
-any row; a score sums up to 128 of them."""
+Bounds used: a product that is taken from the tensor cores is within max(4, d / 4) 2^-24 of itself, one taken in fp32 within 9 roundings of
+sum |q_k d_k|; a score sums up to 128 of them.  For Gaussian rows that is below 2^-19 of a score, and what is seen is about 2^-24."""
 
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
+PARTS = 3  # the kernel under test
 
 
 def _run(Q, D, engine, normalize=0, qm=None, dm=None, lens=None, cu=None, max_d=None):
@@ -16,7 +17,7 @@ def _run(Q, D, engine, normalize=0, qm=None, dm=None, lens=None, cu=None, max_d=
 
     q = _ops.padded_spec(Q, mask=qm)
     d = _ops.packed_spec(D, cu, max_d) if cu is not None else _ops.padded_spec(D, mask=dm, lens=lens)
-    s = _ops.forward(q, d, normalize=normalize, engine=engine)[0].view(Q.shape[0], -1)
+    s = _ops.forward(q, d, normalize=normalize, engine=engine or PARTS)[0].view(Q.shape[0], -1)
     check_device_status()
     return s
 
@@ -77,12 +78,12 @@ def test_winners(nq, lq, nd, ld, d, extra):
     g = torch.Generator().manual_seed(11)
     Q, D = torch.randint(-1, 2, (nq, lq, d), generator=g).float().cuda(), torch.randint(-1, 2, (nd, ld, d), generator=g).float().cuda()
     qm, dm = _masks(nq, lq, nd, ld, g)
-    got = [_ops.forward(_ops.padded_spec(Q, mask=qm), _ops.padded_spec(D, mask=dm), save_argmax=True, argmax_stride=lq + extra, engine=e) for e in (0, 1)]
+    got = [_ops.forward(_ops.padded_spec(Q, mask=qm), _ops.padded_spec(D, mask=dm), save_argmax=True, argmax_stride=lq + extra, engine=e) for e in (PARTS, 1)]
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
     assert torch.equal(got[0][0].view(nq, nd), _run(Q, D, 0, 0, qm, dm))
     Q, D = torch.randn((nq, lq, d), generator=g).cuda(), torch.randn((nd, ld, d), generator=g).cuda()
     for n in (0, 3):
-        a, _ = _ops.forward(_ops.padded_spec(Q, mask=qm), _ops.padded_spec(D, mask=dm), normalize=n, save_argmax=True, argmax_stride=lq + extra)
+        a, _ = _ops.forward(_ops.padded_spec(Q, mask=qm), _ops.padded_spec(D, mask=dm), normalize=n, save_argmax=True, argmax_stride=lq + extra, engine=PARTS)
         assert torch.equal(a.view(nq, nd), _run(Q, D, 0, n, qm, dm))
 
 
@@ -107,7 +108,7 @@ def test_layouts():
         wide[:, lo : lo + 64] = D.view(-1, 64).clone()
         spec = _ops.padded_spec(D, lens=lens.cuda())
         spec.data = wide[:, lo : lo + 64]
-        s = _ops.forward(_ops.padded_spec(Q), spec, normalize=3)[0].view(6, 10)
+        s = _ops.forward(_ops.padded_spec(Q), spec, normalize=3, engine=PARTS)[0].view(6, 10)
         assert torch.allclose(s, a, rtol=1e-5, atol=1e-5)
 
 
@@ -144,5 +145,130 @@ def test_what_masked_rows_hold_does_not_matter():
     bad = torch.tensor([float("nan"), float("inf"), -float("inf"), 3e38], device="cuda").repeat(32)
     Qn, Dn = torch.where(qm[..., None], Q, bad), torch.where(dm[..., None], D, bad)
     assert torch.equal(_run(Qn, Dn, 0, 3, qm, dm), want)
-    s, am = _ops.forward(_ops.padded_spec(Qn, mask=qm), _ops.padded_spec(Dn, mask=dm), normalize=3, save_argmax=True, argmax_stride=32)
+    s, am = _ops.forward(_ops.padded_spec(Qn, mask=qm), _ops.padded_spec(Dn, mask=dm), normalize=3, save_argmax=True, argmax_stride=32, engine=PARTS)
     assert torch.equal(s.view(9, 20), want) and int(am.max()) < 100 and int(am.min()) >= -1
+
+
+# Rows whose features differ much in size: bounds relative to the products' own magnitudes, sum |q_k d_k|.  A dot product of 128 features is at
+# most 9 roundings deep, its two norms 10 each (halved by the root), the multipliers 6: 2^-24 * 25 with normalisation, below it without.
+UNEVEN = 25 * 2.0**-24
+
+
+def _uneven(nq, lq, nd, ld, d, ratio, form, g):
+    """``form``: which side has features `ratio` times the others', where the other side's counterparts lie."""
+    Q, D = torch.randn((nq, lq, d), generator=g), torch.randn((nd, ld, d), generator=g)
+    if form == "documents, query 0 there":
+        D[..., 3] *= ratio
+        Q[..., 3] = 0
+    elif form == "eight features of the queries":
+        Q[..., 8:16] *= ratio
+    elif form == "both, same feature":
+        Q[..., 7] *= ratio
+        D[..., 7] *= ratio
+    elif form == "both, other features":
+        Q[..., 7] *= ratio
+        D[..., 70 % d] *= ratio
+    elif form == "both, other side 0 there":
+        Q[..., 7], D[..., 7] = Q[..., 7] * ratio, 0
+        D[..., 70 % d], Q[..., 70 % d] = D[..., 70 % d] * ratio, 0
+    elif form == "one feature counts":  # a query of one feature against a small one of the document
+        Q[:] = 0
+        Q[..., 1] = 1.0
+        D[..., 0] *= ratio
+    return Q.cuda(), D.cuda()
+
+
+FORMS = ["documents, query 0 there", "eight features of the queries", "both, same feature", "both, other features", "both, other side 0 there", "one feature counts"]
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("log_ratio", [2, 4, 7, 10, 13, 16, 20])
+@pytest.mark.parametrize("normalize", [0, 3])
+def test_uneven_features_keep_every_product(form, log_ratio, normalize):
+    g = torch.Generator().manual_seed(log_ratio)
+    Q, D = _uneven(150, 1, 160, 1, 128, 2.0**log_ratio, form, g)
+    q, d = Q.double()[:, 0], D.double()[:, 0]
+    if normalize:
+        q, d = torch.nn.functional.normalize(q, dim=-1), torch.nn.functional.normalize(d, dim=-1)
+    want, size = q @ d.T, q.abs() @ d.abs().T
+    err = [((_run(Q, D, e, normalize).double() - want).abs() / size) for e in (0, 1)]
+    assert err[0].max().item() < UNEVEN
+    assert err[0].norm().item() <= 2 * err[1].norm().item()
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("log_ratio", [4, 10, 16])
+@pytest.mark.parametrize("nq,lq,nd,ld,d", [(5, 32, 24, 300, 128), (3, 100, 24, 130, 96), (9, 24, 24, 64, 128)])
+@pytest.mark.parametrize("normalize", [0, 3])
+def test_uneven_features_scores_and_winners(form, log_ratio, nq, lq, nd, ld, d, normalize):
+    from late_interaction_kernels_b200 import _ops
+
+    g = torch.Generator().manual_seed(log_ratio + nq)
+    Q, D = _uneven(nq, lq, nd, ld, d, 2.0**log_ratio, form, g)
+    qm, dm = _masks(nq, lq, nd, ld, g)
+    s, am = _ops.forward(_ops.padded_spec(Q, mask=qm), _ops.padded_spec(D, mask=dm), normalize=normalize, save_argmax=True, argmax_stride=lq, engine=PARTS)
+    s, am = s.view(nq, nd), am.view(nq, nd, lq).long()
+    assert torch.equal(s, _run(Q, D, 0, normalize, qm, dm))
+    q, x = Q.double(), D.double()
+    if normalize:
+        q, x = torch.nn.functional.normalize(q, dim=-1), torch.nn.functional.normalize(x, dim=-1)
+    p = torch.einsum("isd,jtd->ijst", q, x).masked_fill(~dm[None, :, None, :], -torch.inf)
+    size = torch.einsum("isd,jtd->ijst", q.abs(), x.abs()).masked_fill(~dm[None, :, None, :], 0)
+    full = dm.any(-1)[None, :, None].expand_as(am)
+    assert (am[full] >= 0).all() and (am[~full] == -1).all()
+    # the winner's own product is the largest but for what either may be off
+    won, won_size = p.gather(3, am.clamp(min=0)[..., None])[..., 0], size.gather(3, am.clamp(min=0)[..., None])[..., 0]
+    assert (p <= (won + UNEVEN * won_size)[..., None] + UNEVEN * size)[full].all()
+    live = full & qm[:, None, :]
+    want, bound = torch.where(live, won, 0).sum(-1), torch.where(live, won_size, 0).sum(-1) * (UNEVEN + 8 * 2.0**-24)  # (a sum of up to 128 on top)
+    assert ((s.double() - want).abs() <= bound).all()
+    e = [((t.double() - _exact(Q, D, normalize, qm, dm)) / (bound + 1e-300)).norm().item() for t in (s, _run(Q, D, 1, normalize, qm, dm))]
+    assert e[0] <= 2 * e[1]
+
+
+@pytest.mark.parametrize("what", ["repeated tokens", "signs", "zero queries", "zero documents", "scales"])
+@pytest.mark.parametrize("normalize", [0, 3])
+def test_products_that_tie(what, normalize):
+    """More than one token may be the best, in one group of sixteen columns, in both sets' pieces, in the whole document: the products are whole numbers (or
+    equal for equal rows), so the first of them wins, as in the other kernel."""
+    from late_interaction_kernels_b200 import _ops
+
+    g = torch.Generator().manual_seed(3)
+    nq, lq, nd, ld, d = 6, 24, 24, 200, 64
+    Q, D = torch.randint(-3, 4, (nq, lq, d), generator=g).float(), torch.randint(-3, 4, (nd, ld, d), generator=g).float()
+    scale = None
+    if what == "repeated tokens":
+        D[:, 100:] = D[:, :100]
+        D[:, 40:60] = D[:, 20:40]
+        D[:8] = D[:8, :1]
+    elif what == "signs":
+        Q, D = torch.where(Q >= 0, 1.0, -1.0), torch.where(D >= 0, 1.0, -1.0)
+    elif what == "zero queries":
+        Q[:, ::3] = 0
+    elif what == "zero documents":
+        D[::2] = 0
+        D[1::2, 5:150] = 0
+    else:
+        scale = torch.tensor([2.0, -1.0, 0.0, 0.5], dtype=torch.float32).repeat(nd * ld // 4).cuda()
+    qm, dm = _masks(nq, lq, nd, ld, g)
+    got = [_ops.forward(_ops.padded_spec(Q.cuda(), mask=qm), _ops.padded_spec(D.cuda(), mask=dm, scale=scale), normalize=normalize, save_argmax=True, argmax_stride=lq, engine=e)
+           for e in (PARTS, 1)]
+    if not normalize:
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    else:
+        assert torch.allclose(got[0][0], got[1][0], rtol=1e-6, atol=1e-6)
+        if what in ("zero queries", "repeated tokens"):  # equal rows have equal products; the first of them
+            first = got[0][1].view(nq, nd, lq)
+            assert (first[..., ::3][dm.any(-1)[None, :].expand(nq, nd)] == dm.float().argmax(-1)[None, :, None].expand(nq, nd, lq)[..., ::3][dm.any(-1)[None, :].expand(nq, nd)]).all() if what == "zero queries" else True
+
+
+def test_a_row_that_does_not_fit_changes_nobody_else():
+    """Infinities in one query, in one document: the scores of the others keep their bits."""
+    g = torch.Generator().manual_seed(12)
+    Q, D = torch.randn((9, 32, 128), generator=g).cuda(), torch.randn((20, 200, 128), generator=g).cuda()
+    want = _run(Q, D, 0, 3)
+    Q[1, 3, 5], D[7, 70, 9], D[8, 3] = float("inf"), float("nan"), 1e30
+    s = _run(Q, D, 0, 3)
+    others = torch.ones_like(s, dtype=torch.bool)
+    others[1], others[:, 7], others[:, 8] = False, False, False
+    assert torch.equal(s[others], want[others])
