@@ -112,7 +112,8 @@ typedef struct lik_fwd_args {
   const int32_t* pair_d;
   int64_t n_pairs; /* LIK_PAIR_LIST */
   int32_t normalize;
-  int32_t engine; /* 0 = automatic, 1 = force the portable fp32 kernel, 2 = force the tcgen05 kernel, 3 = as 0 */
+  int32_t engine; /* 0 = automatic, 1 = force the portable fp32 kernel, 2 = force the tcgen05 kernel; 3 = automatic, but of fp32 rows
+                   * their parts go to the tensor cores wherever they can, not only where that is faster */
   float* scores;
   int32_t* argmax;
   int32_t argmax_stride;

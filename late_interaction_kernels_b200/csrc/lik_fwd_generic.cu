@@ -403,13 +403,14 @@ __global__ void __launch_bounds__(128, 3) fwd_generic_kernel(GenericFwdParams P)
   }
 }
 
+// Two queries of a cross product share a staged document where that still leaves every SM two blocks; fewer pairs spread better one by one
+// (8 x 32 documents of up to 300 tokens 57.6 -> 47.3 us, 4 x 100 of 512 96.7 -> 74.2; at 32 x 32 sharing is ahead, 64.1 to 67.3)
+bool fwd_generic_shares(long long n_q, long long n_d) { return n_q > 1 && (n_q + 1) / 2 * n_d >= 2 * sm_count(); }
+
 template <typename T>
 static int launch_generic(GenericFwdParams P, cudaStream_t st) {
-  // Two queries share a staged document where that still leaves every SM two blocks; fewer pairs spread better one by one
-  // (8 x 32 documents of up to 300 tokens 57.6 -> 47.3 us, 4 x 100 of 512 96.7 -> 74.2; at 32 x 32 sharing is ahead, 64.1 to 67.3)
-  const long long shared = (long long)((P.pm.n_q + 1) / 2) * P.pm.n_d;
-  const bool cross = P.pm.pairing == LIK_PAIR_CROSS && P.pm.n_q > 1 && shared >= 2 * sm_count();
-  const long long blocks = cross ? shared : P.pm.n_scores;
+  const bool cross = P.pm.pairing == LIK_PAIR_CROSS && fwd_generic_shares(P.pm.n_q, P.pm.n_d);
+  const long long blocks = cross ? (long long)((P.pm.n_q + 1) / 2) * P.pm.n_d : P.pm.n_scores;
   P.by_length = P.pm.pairing == LIK_PAIR_CROSS && P.pm.n_d <= G_RANKED && (P.d.lens || P.d.cu) && blocks <= 8 * sm_count();
   constexpr long long kMaxGrid = 1ll << 30;
   const size_t smem = (size_t)((cross ? 2 : 1) * G_QC + G_DC) * G_PITCH * sizeof(float);

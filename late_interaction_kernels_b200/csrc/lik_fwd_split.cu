@@ -37,6 +37,7 @@
 // Every wait is bounded: on expiry the CTA raises LIK_DEV_WAIT_TIMEOUT in the status word, sets a shared abort flag, frees TMEM and
 // returns.  A warp that goes through a document counts its steps, and who waits for it begins anew while they go on.
 #include <cfloat>
+#include <cmath>
 
 #include "lik_common.cuh"
 #include "lik_tc_ptx.cuh"
@@ -796,13 +797,31 @@ static_assert(SMEM_BYTES <= 227 * 1024, "a block's shared memory");
 
 }  // namespace
 
-// fp32 cross products whose queries fit a tile and whose rows can be read sixteen bytes at a time.
+bool fwd_generic_shares(long long n_q, long long n_d);
+
+// Whether this kernel is the faster one, by what either takes in us: a launch, and a CTA's units of so many tokens here; a launch, and an SM's
+// blocks of 32 query tokens (of one query or of two) there.  Measured at 1, 4 and 16 queries of 8 to 128 tokens x 1 to 1000 documents of
+// up to 16 to 512, 128 and 32 features wide, by graph replay (here / there): 32 tokens x 100 documents of up to 64 15.5 / 13.4, of 180 19.5 / 23.4, of
+// 512 31 / 47; x 1000 of 16 41 / 25; 128 tokens x 8 of 16 19 / 24; 16 x 1000 of 512 426 / 1520; 32 wide: 32 x 1000 of 512 109 / 60, 16 x 256 of 512 101 / 149,
+// 16 x 100 of 64 27 / 23.  In 350 calls measured the choice is on average 1 % behind the faster one.
+static bool split_pays(const lik_fwd_args& a) {
+  const float len = a.d.cu ? (float)a.d.n_rows / a.d.n_seq : (float)a.d.max_len, d = (float)a.dim, sms = (float)sm_count();
+  const int per_tile = TILE_M / a.q.max_len;
+  const float units = (float)ceil_div(a.q.n_seq, per_tile) * a.d.n_seq / sms;
+  const float here = 12.f + fmaxf(1.f, units) * ((len <= 32.f ? 4.f : 3.f) + 0.043f * len);  // (short documents: more products in fp32)
+  const bool two = fwd_generic_shares(a.q.n_seq, a.d.n_seq);
+  const float blocks = (two ? (float)((a.q.n_seq + 1) / 2) : (float)a.q.n_seq) * a.d.n_seq / sms;
+  const float block = two ? 1.2f + 0.019f * d + (0.0063f + 0.0005f * d) * len : 0.4f + 0.006f * d + (0.0036f + 0.00054f * d) * len;
+  return here < 7.f + (float)ceil_div(a.q.max_len, 32) * fmaxf(1.f, blocks) * block;
+}
+
+// fp32 cross products whose queries fit a tile and whose rows can be read sixteen bytes at a time, where it pays (engine 3: wherever it can).
 bool fwd_split_supported(const lik_fwd_args& a) {
   if (a.dtype != LIK_F32 || (a.engine != 0 && a.engine != 3) || a.pairing != LIK_PAIR_CROSS) return false;
   if (a.dim % 4 != 0 || a.dim > 128 || a.q.cu || a.q.max_len < 1 || a.q.max_len > TILE_M) return false;
   if (a.q.n_seq <= 0 || a.d.n_seq <= 0 || a.q.n_rows <= 0 || a.d.n_rows <= 0) return false;
   if (a.q.row_stride % 4 != 0 || a.d.row_stride % 4 != 0 || ((uintptr_t)a.q.data & 15) || ((uintptr_t)a.d.data & 15)) return false;
-  return lik_device_supported() != 0;
+  return (a.engine == 3 || split_pays(a)) && lik_device_supported() != 0;
 }
 
 int launch_fwd_split(const lik_fwd_args& a, float eps, cudaStream_t st) {

@@ -9,7 +9,7 @@ import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
-PARTS = 3  # the kernel under test
+PARTS = 3  # the kernel under test, also at sizes where the other one is faster
 
 
 def _run(Q, D, engine, normalize=0, qm=None, dm=None, lens=None, cu=None, max_d=None):
@@ -272,3 +272,16 @@ def test_a_row_that_does_not_fit_changes_nobody_else():
     others = torch.ones_like(s, dtype=torch.bool)
     others[1], others[:, 7], others[:, 8] = False, False, False
     assert torch.equal(s[others], want[others])
+
+
+@pytest.mark.parametrize("nq,lq,nd,ld,d,parts", [(1, 32, 8, 16, 128, False), (1, 32, 1000, 512, 32, False), (16, 32, 100, 64, 32, False),
+                                                 (1, 32, 1000, 512, 128, True), (1, 128, 8, 64, 128, True), (32, 32, 32, 180, 128, True)])
+def test_the_faster_kernel_takes_a_call(nq, lq, nd, ld, d, parts):
+    """The two kernels add in different orders: a call's bits say which one it went to."""
+    from late_interaction_kernels_b200 import _ops
+
+    g = torch.Generator().manual_seed(nq + d)
+    Q, D = torch.randn((nq, lq, d), generator=g).cuda(), torch.randn((nd, ld, d), generator=g).cuda()
+    auto = _ops.forward(_ops.padded_spec(Q), _ops.padded_spec(D), normalize=3)[0].view(nq, nd)
+    fma, split = _run(Q, D, 1, 3), _run(Q, D, PARTS, 3)
+    assert not torch.equal(fma, split) and torch.equal(auto, split if parts else fma)
