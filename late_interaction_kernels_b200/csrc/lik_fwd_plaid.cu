@@ -15,7 +15,7 @@
 //   warps 6..13  decode: sixteen columns of every tile each, a quarter-warp per token, the next tokens' rows on their way while these
 //                are finished
 // 25 000 documents of 60..300 tokens, 2 bits, top-10: one query of 32 tokens 574 -> 387 us, four 581 -> 411 (against decoding the
-// rows to memory and scoring them from there); 4 bits 575 -> 408, 8 bits 652 -> 601; 1000 documents of up to 64 tokens 132 -> 65.
+// rows to memory and scoring them from there); 4 bits 575 -> 408, 8 bits (scores) 698 -> 457; 1000 documents of up to 64 tokens 132 -> 65.
 // What bounds it: the decoders (361 us without an epilogue): shared-memory wavefronts (the table look-ups) 74 % of the pipe,
 // instruction issue 58 %, and their waits for centroid rows out of L2.  Two CTAs per SM, because every role is a chain of dependent
 // steps at some ten cycles each: one CTA with sixteen decoder warps took 642 us, its single epilogue warp 4200 cycles per tile.
@@ -37,7 +37,7 @@ constexpr int NUM_THREADS = (DEC_WARP0 + DEC_WARPS) * 32;
 constexpr int CTAS_PER_SM = 2;
 static_assert(DEC_COLS % 8 == 0, "a decoder warp decodes eight tokens at a time");
 constexpr int TABLES = 8;                     // ring of tile tables
-constexpr int MAX_SEGS = 64;                  // document segments per tile; a tile with more (empty documents) ends early
+constexpr int MAX_SEGS = 48;                  // document segments per tile; a tile with more (empty documents) ends early
 constexpr int ACCS = 2;                       // accumulators of 128 columns: half of the tensor memory
 constexpr int STAGES = 2;
 constexpr int GRANULE = 8;                    // a document starts at a multiple of this many columns; its last token fills the gap behind it
@@ -131,6 +131,10 @@ __device__ __forceinline__ void tidy_list(const TcParams& P, SharedCtl* ctl, int
   __syncwarp();
 }
 static_assert(TOPK_CAP - MAX_SEGS >= TOPK_CAP / 2, "a list that was cut back has room for a tile");
+
+constexpr size_t dynamic_smem(int n_slabs) { return (size_t)n_slabs * (TILE_M + STAGES * TILE_T) * SLAB_BYTES_ROW + sizeof(SharedCtl) + 1024; }
+// (an SM has 228 KB and takes 1 KB of them per CTA; 512 bytes more and eight-bit indexes, with the largest table, had one CTA per SM)
+static_assert(CTAS_PER_SM * (dynamic_smem(2) + PlaidTable<8>::WORDS * sizeof(float) + 1024) <= 228 * 1024, "two CTAs per SM for every index");
 
 // FULL: 128 features
 template <bool CF32, bool CBF16, int NBITS, bool FULL>
@@ -512,9 +516,7 @@ __global__ void __launch_bounds__(NUM_THREADS, CTAS_PER_SM) fwd_plaid_kernel(con
 
 }  // namespace
 
-size_t fwd_plaid_smem(int n_slabs) {
-  return (size_t)n_slabs * (TILE_M + STAGES * TILE_T) * SLAB_BYTES_ROW + sizeof(SharedCtl) + 1024;
-}
+size_t fwd_plaid_smem(int n_slabs) { return dynamic_smem(n_slabs); }
 int fwd_plaid_ctas_per_sm() { return CTAS_PER_SM; }
 
 int launch_fwd_plaid(const lik_fwd_args& a, const TcPlan& pl, const TcParams& P, cudaStream_t st) {
