@@ -18,18 +18,18 @@ from . import _lib, _ops
 _DECOMPRESS_TOKENS = 1 << 22
 # The index can also be decoded INSIDE the scoring kernel (``lik_plaid_fwd``), so that no operand row ever exists in
 # memory.  The kernel for that takes the query tokens that fit one tile of 128 rows (four 32-token queries) and decodes
-# every token once.  More queries, and calls that save the winners, would go to an older form that decodes every token
-# once per group of two tiles with three warps per SM, slower than decoding once with the whole machine: this is the
-# largest number of such groups for which it is used.  All ways produce the same bits.
-_FUSED_DECODE_MAX_GROUPS = 0
+# every token once.  More queries, and calls that save the winners, have an older form that decodes every token once per
+# group of two tiles with three warps per SM, slower than decoding once with the whole machine.  All ways produce the same
+# bits.  None: the faster way; a number: calls of at most that many groups are decoded in the kernel, others are not.
+_FUSED_DECODE_MAX_GROUPS = None
 
 
 def _decode_in_kernel(Nq: int, Lq: int, winners: bool = False) -> bool:
     if Nq <= 0 or Lq <= 0:
         return False
-    if not winners and Lq <= 128 and Nq <= 128 // Lq:
-        return True
-    return _tile_groups(Nq, Lq) <= _FUSED_DECODE_MAX_GROUPS
+    if _FUSED_DECODE_MAX_GROUPS is not None:
+        return _tile_groups(Nq, Lq) <= _FUSED_DECODE_MAX_GROUPS
+    return not winners and Lq <= 128 and Nq <= 128 // Lq
 
 
 def _tile_groups(Nq: int, Lq: int) -> int:

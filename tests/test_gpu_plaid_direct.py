@@ -105,3 +105,20 @@ def test_codes_out_of_range_are_reported():
         check_device_status()
     codes[100], codes[700] = 0, 0
     assert torch.equal(s, plaid.maxsim_residual_varlen(Q, codes, res, cu, cent, bw, 2))
+
+
+def test_the_knob_says_which_way_a_call_goes(monkeypatch):
+    """Decoding to memory is a launch of its own, so a call's launches tell; both ways give the same bits."""
+    from late_interaction_kernels_b200 import _lib, plaid
+
+    lib, ix = _lib.load(), _index([100, 30, 64] * 40, 128, 2, torch.float16)
+    Q = torch.randn((2, 32, 128)).cuda().to(torch.float16)
+    seen = {}
+    for knob in (None, 1 << 30, 0):
+        monkeypatch.setattr(plaid, "_FUSED_DECODE_MAX_GROUPS", knob)
+        n0 = lib.lik_launch_count()
+        s = plaid.maxsim_residual_varlen(Q, *ix, 2)
+        t = plaid.retrieve_residual_varlen(Q, *ix, 2, 5)
+        seen[knob] = (lib.lik_launch_count() - n0, s, *t)
+    assert seen[None][0] == seen[1 << 30][0] < seen[0][0]
+    assert all(torch.equal(a, b) for k in (None, 1 << 30) for a, b in zip(seen[k][1:], seen[0][1:]))
