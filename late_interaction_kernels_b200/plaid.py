@@ -24,12 +24,31 @@ _DECOMPRESS_TOKENS = 1 << 22
 _FUSED_DECODE_MAX_GROUPS = None
 
 
-def _decode_in_kernel(Nq: int, Lq: int, winners: bool = False) -> bool:
+def _decode_in_kernel(Nq: int, Lq: int, winners: bool, Nd: int, tokens: int, longest: int, nbits: int, host: float = 50.0) -> bool:
+    """Which way a call goes.  ``host``: us that the host needs for decoding first (in the kernel: 50); infinite where it would read offsets.  In the kernel a document is one CTA's, of 296, from end to end, and unless every query has a
+    warp of its own the epilogue warps meet for each document; decoding to memory is two more launches, a write and a
+    read of every row, with the whole machine.  us, in the kernel / first: one 32-token query, 2 bits, 1000 documents of
+    60..300 tokens 29 / 41, 25 000 of them 343 / 580, 8 of 64 10 / 23, 44 of 2380 62 / 36, 8 of up to 4096 56 / 38,
+    1184 of them 262 / 348; 8 bits, 78 of up to 3449, four of 20 tokens 99 / 55; 25 000 of 60..300, 64 queries of 2 tokens 872 / 832.  By
+    graph replay of 467 calls these estimates choose 0.6 % behind the faster way on average, 11 % at most."""
     if Nq <= 0 or Lq <= 0:
         return False
     if _FUSED_DECODE_MAX_GROUPS is not None:
         return _tile_groups(Nq, Lq) <= _FUSED_DECODE_MAX_GROUPS
-    return not winners and Lq <= 128 and Nq <= 128 // Lq
+    if winners or Lq > 128 or Nq > 128 // Lq:
+        return False
+    ctas = 2 * 148
+    docs = 0.0 if (Nq == 1 and Lq <= 32) or (Lq == 32 and Nq <= 4) else max(Nd / ctas, 1.0)  # per CTA, where warps meet
+    wide = 1.25 if nbits == 8 else 1.0
+    most = max(longest, tokens / ctas + 0.75 * longest if Nd > ctas else 0.0)  # tokens of the fullest CTA
+    inside = 9.0 + 0.017 * wide * most + docs * (0.35 + 0.09 * Nq)
+    first = 25.0 + 0.003 * longest + 8e-5 * wide * tokens + docs * 0.05 * Nq
+    return max(inside, 50.0) <= max(first, host)
+
+
+def _longest(n_docs: int, tokens: int, known: int) -> int:
+    # (offsets lie on the device and are not read for this: twice the mean where nobody says)
+    return known if known > 0 else min(tokens, 2 * tokens // max(n_docs, 1))
 
 
 def _tile_groups(Nq: int, Lq: int) -> int:
@@ -93,7 +112,9 @@ def _residual_scores(Q, ix, cu_or_lens, max_ld, padded, normalize, save_argmax):
     Qo = Q.to(odt)
     q = _ops.padded_spec(Qo)
     norm = _lib.NORM_Q if normalize else _lib.NORM_NONE
-    if _decode_in_kernel(Nq, Lq, save_argmax) and ix.n_tokens > 0:
+    n_docs = cu_or_lens.numel() - (0 if padded else 1)
+    host = 75.0 if padded else 50.0 if ix.n_tokens <= _DECOMPRESS_TOKENS else float("inf")
+    if _decode_in_kernel(Nq, Lq, save_argmax, n_docs, ix.n_tokens, _longest(n_docs, ix.n_tokens, max_ld), ix.nbits, host) and ix.n_tokens > 0:
         if padded:
             nd = cu_or_lens.numel()
             lay = _ops.layout_spec(nd * max_ld, nd, max_ld, lens=cu_or_lens, seq_stride=max_ld)
@@ -259,12 +280,13 @@ def maxsim_residual_varlen(Q, codes_flat, residuals_flat, cu_seqlens_d, centroid
 def retrieve_residual_varlen(Q, codes_flat, residuals_flat, cu_seqlens_d, centroids, bucket_weights, nbits, top_k, *,
                              normalize=True, chunk=4096, largest=True, doc_lengths_host=None):
     """Top-``top_k`` documents per query straight from a ragged PLAID index, never materialising
-    ``[Nq, Nd]``: documents are decompressed ``chunk`` at a time into operand rows, scored, and merged
-    into a running ``[Nq, k]`` list (score desc, index asc).  This is the fused form of "call
+    ``[Nq, Nd]``.  Few queries are scored by one kernel that decodes the index itself; else documents are
+    decompressed, at least ``chunk`` at a time, into operand rows, scored, and merged into a running
+    ``[Nq, k]`` list (score desc, index asc).  This is the fused form of "call
     ``maxsim_residual_varlen`` then ``torch.topk``" (docs/benchmarks.md:191-206 of the reference).
 
-    ``cu_seqlens_d`` is read on the host once to place chunk boundaries (pass ``doc_lengths_host``, a CPU
-    int64 tensor of per-document lengths, to skip that device->host copy).  Returns
+    Where documents go in chunks, ``cu_seqlens_d`` is read on the host once to place their boundaries (pass
+    ``doc_lengths_host``, a CPU int64 tensor of per-document lengths, to skip that device->host copy).  Returns
     ``(scores fp32 [Nq, k], indices int64 [Nq, k])`` with ``k = min(top_k, Nd)``; 2-D ``Q`` squeezes."""
     if nbits not in (2, 4, 8):
         raise ValueError(f"nbits must be 2, 4, or 8; got {nbits}")
@@ -298,7 +320,11 @@ def retrieve_residual_varlen(Q, codes_flat, residuals_flat, cu_seqlens_d, centro
     norm = _lib.NORM_Q if normalize else _lib.NORM_NONE
     out = None
     with torch.no_grad():
-        if k <= _lib.TOPK_FUSED_MAX and _decode_in_kernel(Nq, Lq):
+        longest = 0
+        if isinstance(doc_lengths_host, torch.Tensor) and doc_lengths_host.device.type == "cpu" and 0 < doc_lengths_host.numel() <= 4096:
+            longest = int(doc_lengths_host.max())
+        host = 125.0 if doc_lengths_host is not None else float("inf")
+        if k <= _lib.TOPK_FUSED_MAX and _decode_in_kernel(Nq, Lq, False, Nd, ix.n_tokens, _longest(Nd, ix.n_tokens, longest), nbits, host):
             # few queries: one kernel decodes, scores and keeps the candidates; nothing is read on the host, no piece is placed
             lay = _ops.layout_spec(ix.n_tokens, Nd, 0, cu=cu)
             out = _ops.forward_fused(q, lay, normalize=(_lib.NORM_BOTH if normalize else _lib.NORM_NONE), plaid=ix, topk=k,

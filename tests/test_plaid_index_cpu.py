@@ -74,3 +74,26 @@ def test_inverted_file_matches_the_oracle():
     for c in range(23):
         want = [j for j in range(60) if (codes[cu[j]:cu[j + 1]] == c).any()]
         assert docs[off[c]:off[c + 1]].tolist() == want
+
+
+def test_which_way_a_compressed_index_is_scored():
+    """Both sides of the rule's lines, at sizes where the two ways are far apart; the knob overrides it."""
+    from late_interaction_kernels_b200 import plaid
+
+    def way(nq, lq, nd, longest, tokens=None, winners=False, nbits=2, **kw):
+        return plaid._decode_in_kernel(nq, lq, winners, nd, longest * nd if tokens is None else tokens, longest, nbits, **kw)
+
+    assert way(1, 32, 25000, 300, 4_500_000) and way(4, 32, 25000, 300, 4_500_000) and way(1, 32, 8, 64) and way(1, 128, 1000, 300, 180_000)
+    assert way(1, 32, 1184, 4096, 2_900_000) and way(16, 8, 25000, 300, 4_500_000)
+    assert not way(1, 32, 8, 4096) and not way(4, 20, 78, 3449, 161_205, nbits=8)  # few long documents
+    assert not way(128, 1, 2925, 71, 35_242, nbits=8) and not way(64, 2, 10000, 8, 45_000)  # many queries, short documents
+    assert way(1, 32, 8, 4096, host=125.0) and way(128, 1, 2925, 71, 35_242, host=float("inf"))  # where the host is what takes the time
+    assert not way(5, 32, 25000, 300) and not way(1, 129, 8, 64) and not way(1, 32, 8, 64, winners=True) and not way(0, 32, 8, 64) and not way(1, 0, 8, 64)
+    assert plaid._longest(10, 1000, 0) == 200 and plaid._longest(10, 1000, 150) == 150 and plaid._longest(0, 0, 0) == 0 and plaid._longest(1, 1000, 0) == 1000
+    try:
+        plaid._FUSED_DECODE_MAX_GROUPS = 0
+        assert not way(1, 32, 25000, 300)
+        plaid._FUSED_DECODE_MAX_GROUPS = 3
+        assert way(1, 32, 8, 4096) and way(24, 32, 8, 64, winners=True) and not way(32, 32, 8, 64)
+    finally:
+        plaid._FUSED_DECODE_MAX_GROUPS = None
