@@ -382,6 +382,9 @@ int lik_selftest_wait_timeout(int64_t limit_cycles, int32_t* status, int32_t* re
  * result (device, int32[12]): three numbers each as above; for the warps' waits the first one counts the lanes that were
  * told to go on. */
 int lik_selftest_other_waits(int64_t limit_cycles, int32_t* status, int32_t* result, lik_stream_t stream);
+/* The same for the wait that the compressed-index kernel and the kernel for fp32 rows share, which a whole warp runs together: alone, and
+ * beside a warp that reports progress for three limits, which the wait must outlast.  result (device, int32[6]). */
+int lik_selftest_all_lanes_wait(int64_t limit_cycles, int32_t* status, int32_t* result, lik_stream_t stream);
 const char* lik_last_error(void);
 /* kernels this library has launched in this process so far (all threads, all devices) */
 uint64_t lik_launch_count(void);

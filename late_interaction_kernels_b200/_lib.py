@@ -142,6 +142,8 @@ def _declare(lib):
     lib.lik_selftest_wait_timeout.restype = i32
     lib.lik_selftest_other_waits.argtypes = [i64, vp, vp, vp]
     lib.lik_selftest_other_waits.restype = i32
+    lib.lik_selftest_all_lanes_wait.argtypes = [i64, vp, vp, vp]
+    lib.lik_selftest_all_lanes_wait.restype = i32
     lib.lik_launch_count.argtypes = []
     lib.lik_launch_count.restype = C.c_uint64
     lib.lik_topk_rows.argtypes = [vp, i64, i64, i64, i32, i32, i64, i32, vp, vp, vp]
@@ -168,7 +170,7 @@ EXPORTED_SYMBOLS = (
     "lik_maxsim_hidden_fwd_supported", "lik_maxsim_hidden_fwd_workspace", "lik_maxsim_hidden_fwd",
     "lik_hidden_winners", "lik_hidden_scatter_rows",
     "lik_plaid_fwd_supported", "lik_plaid_fwd_workspace", "lik_plaid_fwd", "lik_launch_count", "lik_selftest_wait_timeout",
-    "lik_selftest_other_waits",
+    "lik_selftest_other_waits", "lik_selftest_all_lanes_wait",
     "lik_topk_merge", "lik_plaid_decompress", "lik_plaid_approx", "lik_plaid_bwd_dq", "lik_row_inv_norm",
     "lik_last_error", "lik_version", "lik_device_supported",
 )

@@ -50,8 +50,7 @@ struct SharedCtl {
   unsigned long long acc_full[ACCS], acc_empty[ACCS];
   unsigned long long epi_sync;
   uint32_t tmem_base;
-  volatile int abort_flag;
-  long long wait_limit;
+  WaitCtl wait;
   alignas(16) int2 col[TABLES][TILE_T];       // per column: token, centroid
   int2 seg[TABLES][MAX_SEGS];                 // x = document, y = first granule behind the segment | SEG_ENDS
   int n_seg[TABLES];                          // -1: the stream has ended before this tile
@@ -62,23 +61,8 @@ struct SharedCtl {
   int seg_list[TILE_M];
 };
 
-// Bounded wait of a whole warp; the lanes leave together, with one answer.  False: the CTA is aborting.  (No suspension hint: a warp
-// that it puts to sleep comes back late, 642 us against 587.)
-// The flag and the clock are looked at after every sixteenth question: what a waiting warp issues, others cannot.
 __device__ __forceinline__ bool wait_bar(unsigned long long* bar, uint32_t parity, SharedCtl* ctl, int* status) {
-  const uint32_t b = smem_u32(bar);
-  if (__all_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
-  const long long t0 = clock64();
-  while (true) {
-#pragma unroll 1
-    for (int i = 0; i < 16; ++i)
-      if (__all_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
-    if (clock64() - t0 > ctl->wait_limit) {
-      ctl->abort_flag = 1;
-      if (status) atomicOr(status, LIK_DEV_WAIT_TIMEOUT);
-    }
-    if (__any_sync(0xffffffffu, ctl->abort_flag != 0)) return false;
-  }
+  return wait_bar_all(bar, parity, &ctl->wait, status);
 }
 
 // First index in [0, n) whose offset is not below x (n: none), 32 places per step.  For ascending x the results ascend, whatever the
@@ -169,8 +153,7 @@ __global__ void __launch_bounds__(NUM_THREADS, CTAS_PER_SM) fwd_plaid_kernel(con
       mbar_init(smem_u32(&ctl->acc_empty[i]), epi_warps);
     }
     mbar_init(smem_u32(&ctl->epi_sync), 4);
-    ctl->abort_flag = 0;
-    ctl->wait_limit = WAIT_LIMIT_CYCLES;
+    ctl->wait.init();
     fence_barrier_init();
     prefetch_tmap(&q_map);
   }

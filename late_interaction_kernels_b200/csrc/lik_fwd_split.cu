@@ -56,7 +56,6 @@ constexpr int RING = 4;                       // column arrays and query arrays:
 constexpr int ROW_BYTES = 128;                // one swizzle span: 64 bf16
 constexpr int B_PART = PIECE * ROW_BYTES, B_SLAB = PARTS * B_PART, B_STAGE = 2 * B_SLAB;  // (the parts of B are one matrix of 192 rows)
 constexpr int A_SLAB = TILE_M * ROW_BYTES, A_PART = 2 * A_SLAB;
-constexpr long long WAIT_LIMIT = 4000000000ll;
 // Candidates of a query token: columns at + i for bit i of `bits`, at2 + i for bit 16 + i
 constexpr int NO_MORE = -1, WHOLE_DOC = -2;  // instead of at2: no second group; all tokens
 static_assert(PIECE == 4 * CUT_WARPS && TILE_M == 8 * CUT_WARPS, "a half-warp cuts two rows of a piece and four of a query tile");
@@ -81,9 +80,8 @@ struct SharedCtl {
   // candidates of the set without a document's last piece, on their way to the other.  It can be three pieces ahead, so two exchanges.
   unsigned long long x_full[4][4];  // by exchange and quadrant of rows
   uint32_t tmem_base;
-  volatile int abort_flag;
+  WaitCtl wait;           // (its progress: a scan of a document goes on)
   SplitParams params;     // for `products`
-  volatile int progress;  // counts up while a scan of a document goes on: who waits for its warp starts again
   // A slot is written again four pieces (query tiles) later.  By then the MMAs of the piece two behind it have completed, for the
   // cutters waited for its stage; they had taken the accumulator that the epilogue of this piece gave back after its last look here.
   alignas(16) float col_mul[RING][PIECE], col_add[RING][PIECE];  // 0 or, for columns that are no valid token, -inf
@@ -97,25 +95,7 @@ struct SharedCtl {
 };
 
 __device__ __forceinline__ bool wait_bar(unsigned long long* bar, uint32_t parity, SharedCtl* ctl, int* status) {
-  const uint32_t b = smem_u32(bar);
-  if (__all_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
-  long long t0 = clock64();
-  int seen = ctl->progress;
-  while (true) {
-#pragma unroll 1
-    for (int i = 0; i < 16; ++i)
-      if (__all_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
-    if (clock64() - t0 > WAIT_LIMIT) {
-      const int now = ctl->progress;
-      if (now == seen) {
-        ctl->abort_flag = 1;
-        if (status) atomicOr(status, LIK_DEV_WAIT_TIMEOUT);
-      }
-      seen = now;
-      t0 = clock64();
-    }
-    if (__any_sync(0xffffffffu, ctl->abort_flag != 0)) return false;
-  }
+  return wait_bar_all(bar, parity, &ctl->wait, status);
 }
 
 // The units of a CTA: unit = tile * n_d + document.
@@ -378,7 +358,7 @@ __device__ __noinline__ int2 products(SharedCtl* ctl, int what, int tile, long l
   }
   const unsigned alls = __ballot_sync(0xffffffffu, what == ALL);
   if (alls) {
-    const int2 x = whole_document(D, alls, q_tile, q_off, len, const_cast<int*>(&ctl->progress));
+    const int2 x = whole_document(D, alls, q_tile, q_off, len, const_cast<int*>(&ctl->wait.progress));
     if (what == ALL) {
       r = __int_as_float(x.x);
       ri = x.y;
@@ -408,8 +388,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const __grid_
     }
     for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&ctl->epi_sync[i]), 4);
     for (int i = 0; i < 16; ++i) mbar_init(smem_u32(&ctl->x_full[i >> 2][i & 3]), 1);
-    ctl->abort_flag = 0;
-    ctl->progress = 0;
+    ctl->wait.init();
     ctl->params = P;
     fence_barrier_init();
   }
@@ -795,6 +774,37 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const __grid_
 constexpr size_t SMEM_BYTES = (size_t)PARTS * A_PART + STAGES * B_STAGE + sizeof(SharedCtl) + 1024;
 static_assert(SMEM_BYTES <= 227 * 1024, "a block's shared memory");
 
+// The wait of this kernel and of the compressed-index kernel, alone: a warp waits on a barrier that nothing arrives at, first with nobody
+// busy, then beside a warp that counts its progress for three limits and stops.
+// result[3 * w + ...] = lanes that were told to go on (0: all gave up), the abort flag, cycles spent by the slowest lane.
+__global__ void all_lanes_wait_probe_kernel(long long limit, int* status, int* result) {
+  __shared__ unsigned long long bar;
+  __shared__ WaitCtl ctl;
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&bar), 1);
+    fence_barrier_init();
+  }
+  for (int w = 0; w < 2; ++w) {
+    if (threadIdx.x == 0) ctl.init(limit);
+    __syncthreads();
+    const long long t0 = clock64();
+    if (threadIdx.x < 32) {
+      const bool got = wait_bar_all(&bar, 0, &ctl, status);
+      const long long dt = clock64() - t0;
+      const int lanes = __popc(__ballot_sync(0xffffffffu, got));
+      const unsigned cycles = __reduce_max_sync(0xffffffffu, dt > 0x7fffffffll ? 0x7fffffffu : (unsigned)dt);
+      if (threadIdx.x == 0) {
+        result[3 * w] = lanes;
+        result[3 * w + 1] = ctl.abort_flag;
+        result[3 * w + 2] = (int)cycles;
+      }
+    } else if (w == 1 && threadIdx.x == 32) {
+      while (clock64() - t0 < 3 * limit) atomicAdd(const_cast<int*>(&ctl.progress), 1);
+    }
+    __syncthreads();
+  }
+}
+
 }  // namespace
 
 bool fwd_generic_shares(long long n_q, long long n_d);
@@ -863,3 +873,12 @@ int launch_fwd_split(const lik_fwd_args& a, float eps, cudaStream_t st) {
 }
 
 }  // namespace lik
+
+extern "C" int lik_selftest_all_lanes_wait(int64_t limit_cycles, int32_t* status, int32_t* result, lik_stream_t stream) {
+  using namespace lik;
+  LIK_REQUIRE(result != nullptr, "result is NULL");
+  LIK_REQUIRE(limit_cycles > 0 && limit_cycles <= 200000000ll, "limit_cycles outside (0, 2e8]");
+  all_lanes_wait_probe_kernel<<<1, 64, 0, (cudaStream_t)stream>>>((long long)limit_cycles, status, result), ::lik::count_launch();
+  LIK_CUDA_OK(cudaGetLastError());
+  return LIK_OK;
+}

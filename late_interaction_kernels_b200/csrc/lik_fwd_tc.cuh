@@ -26,7 +26,6 @@ namespace {
 constexpr int SLAB_BYTES_ROW = 128; // one swizzle span: 64 two-byte or 128 one-byte elements
 constexpr int MAX_SLABS = 2;
 constexpr int BOX_ROWS = 32;        // granule of the document TMA boxes (64 read a sixth more rows than ragged documents have)
-constexpr long long WAIT_LIMIT_CYCLES = 4000000000ll;  // default limit of a wait: about 2 s at 2 GHz
 constexpr int UNIT_LEN_MASK = 0xFFFFFF;       // unit_info.x: document length in the low 24 bits,
 constexpr int UNIT_SLOT_SHIFT = 24;           // the multiplier slot of its first tile in bits 24..28, LEN_FLAG_MASKED above
 

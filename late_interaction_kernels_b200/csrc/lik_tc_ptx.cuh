@@ -49,6 +49,42 @@ __device__ __forceinline__ bool mbar_try_wait_long(uint32_t bar, uint32_t parity
       : "memory");
   return ok != 0;
 }
+constexpr long long WAIT_LIMIT_CYCLES = 4000000000ll;  // default limit of a wait: about 2 s at 2 GHz
+
+// What the bounded waits of a CTA share, in shared memory.
+struct WaitCtl {
+  volatile int abort_flag;
+  volatile int progress;  // counted up by a warp that is busy for longer than a wait's limit may be: who waits for it begins anew
+  long long limit;
+  __device__ __forceinline__ void init(long long cycles = WAIT_LIMIT_CYCLES) {
+    abort_flag = progress = 0;
+    limit = cycles;
+  }
+};
+// Bounded wait of a whole warp; the lanes leave together, with one answer.  False: the CTA is aborting.  (No suspension hint: a warp
+// that it puts to sleep comes back late, 642 us against 587 in the compressed-index kernel.)
+// The flag and the clock are looked at after every sixteenth question: what a waiting warp issues, others cannot.
+__device__ __forceinline__ bool wait_bar_all(unsigned long long* bar, uint32_t parity, WaitCtl* ctl, int* status) {
+  const uint32_t b = smem_u32(bar);
+  if (__all_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
+  long long t0 = clock64();
+  int seen = 0;
+  while (true) {
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i)
+      if (__all_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
+    if (clock64() - t0 > ctl->limit) {
+      const int now = ctl->progress;
+      if (now == seen) {
+        ctl->abort_flag = 1;
+        if (status) atomicOr(status, LIK_DEV_WAIT_TIMEOUT);
+      }
+      seen = now;
+      t0 = clock64();
+    }
+    if (__any_sync(0xffffffffu, ctl->abort_flag != 0)) return false;
+  }
+}
 // generic-proxy writes to shared memory become visible to the async proxy (the tensor core's operand reads)
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }

@@ -289,6 +289,28 @@ def test_a_bounded_wait_that_runs_out_reports_and_returns():
     assert lib.lik_selftest_wait_timeout(10**10, None, res.data_ptr(), None) == -1
 
 
+def test_the_wait_of_whole_warps_gives_up_and_outlasts_a_busy_warp():
+    """The wait of the compressed-index kernel and of the kernel for fp32 rows: alone it gives up after its limit; while another warp counts its
+    progress it goes on, and gives up when that has stopped."""
+    import late_interaction_kernels_b200 as lik
+    from late_interaction_kernels_b200 import _lib, _ops
+
+    lib = _lib.load()
+    status = _ops.status_word("cuda")
+    lik.check_device_status()
+    res = torch.full((2, 3), -1, dtype=torch.int32, device="cuda")
+    limit = 2_000_000
+    _lib.check(lib.lik_selftest_all_lanes_wait(limit, status.data_ptr(), res.data_ptr(), _lib.stream_ptr(res.device)), "selftest")
+    torch.cuda.synchronize()
+    for (got, aborted, cycles), least in zip(res.tolist(), (limit, 3 * limit)):
+        assert got == 0 and aborted == 1
+        assert least <= cycles < 50 * limit
+    with pytest.raises(RuntimeError, match="bounded wait expired"):
+        lik.check_device_status()
+    lik.check_device_status()
+    assert lib.lik_selftest_all_lanes_wait(10**10, None, res.data_ptr(), None) == -1
+
+
 def test_every_form_of_the_bounded_wait_gives_up_with_all_its_lanes():
     """The wait with its loop inlined, and the three waits of the kernel for larger problems: on expiry the whole warp is told
     the same, reports and returns (TMEM loads and shuffles of the full warp stand behind these waits)."""
