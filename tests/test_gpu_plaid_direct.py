@@ -123,3 +123,48 @@ def test_the_knob_says_which_way_a_call_goes(monkeypatch):
         seen[knob] = (lib.lik_launch_count() - n0, s, *t)
     assert seen[None][0] == seen[1 << 30][0] < seen[0][0]
     assert all(torch.equal(a, b) for k in (None, 1 << 30) for a, b in zip(seen[k][1:], seen[0][1:]))
+
+
+@pytest.mark.parametrize("nbits", [2, 4, 8])
+@pytest.mark.parametrize("cdtype", [torch.float16, torch.bfloat16, torch.float32])
+def test_infinities_and_nan_in_the_index(nbits, cdtype, monkeypatch):
+    """Centroids and weights that are no numbers: what they do to a token stays with its document, and both ways agree bit for bit."""
+    from late_interaction_kernels_b200 import plaid
+
+    codes, res, cu, cent, bw = _index([30, 1, 0, 129, 64, 7] * 30, 128, nbits, cdtype, seed=nbits)
+    Q = torch.randn((3, 32, 128), generator=torch.Generator().manual_seed(1)).cuda().to(torch.float16)
+    for normalize in (True, False):
+        for what in ("centroids", "weight"):
+            c, w = cent.clone(), bw.clone()
+            if what == "centroids":
+                c[3, 5], c[9], c[20, ::2] = float("inf"), float("nan"), -float("inf")
+            else:
+                w[1] = float("inf")
+            got, want = _both(monkeypatch, lambda: plaid.maxsim_residual_varlen(Q, codes, res, cu, c, w, nbits, normalize=normalize))
+            assert torch.equal(got.nan_to_num(1.5, 2.5, 3.5), want.nan_to_num(1.5, 2.5, 3.5))
+            got, want = _both(monkeypatch, lambda: plaid.retrieve_residual_varlen(Q, codes, res, cu, c, w, nbits, 20, normalize=normalize))
+            assert torch.equal(got[0].nan_to_num(1.5, 2.5, 3.5), want[0].nan_to_num(1.5, 2.5, 3.5)) and torch.equal(got[1], want[1])
+
+
+def test_two_streams_at_once(monkeypatch):
+    """Calls of this kernel, of the one for fp32 rows and of the others beside each other: each allocates tensor memory on the same SMs."""
+    import late_interaction_kernels_b200 as lik
+    from late_interaction_kernels_b200 import plaid
+
+    monkeypatch.setattr(plaid, "_decode_in_kernel", lambda *a: True)
+    g = torch.Generator().manual_seed(4)
+    ix = _index([60, 200, 300] * 300, 128, 2, torch.float16)
+    Q = torch.randn((2, 32, 128), generator=g).cuda().to(torch.float16)
+    Qf, Df = torch.randn((32, 32, 128), generator=g).cuda(), torch.randn((40, 180, 128), generator=g).cuda()
+    Qh, Dh = Qf.half(), Df.half()
+    calls = [lambda: plaid.maxsim_residual_varlen(Q, *ix, 2), lambda: lik.maxsim(Qf, Df), lambda: lik.maxsim(Qh, Dh), lambda: plaid.retrieve_residual_varlen(Q, *ix, 2, 10)[0]]
+    want = [f() for f in calls]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    out = []
+    for r in range(12):
+        for n, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                out.append(((r + n) % 4, calls[(r + n) % 4]()))
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, want[k]) for k, x in out)
