@@ -91,13 +91,15 @@ FwdPlan plan_fwd(const lik_fwd_args& a, const TcExtra& x = TcExtra()) {
   // the kernel's own workspace comes first: its leading part (the candidate lists of a fused top-k) then sits at
   // the same place for every piece of a corpus that is scored piece by piece into one workspace
   if (pl.use_tc) pl.tc_off = take(fwd_tc_workspace(b, x, &pl.streams));
+  // (Room for the norms is asked for also where the scoring kernel takes them itself, of either side with fp32 rows: what a call needs must not
+  // depend on how its rows are aligned, which a caller who asks ahead may not know.)
   if (a.normalize & LIK_NORM_Q) {
     if (pl.copies) pl.qcopy_off = take((size_t)a.q.n_rows * a.dim * eb);
     else pl.qn_off = take((size_t)a.q.n_rows * 4);
   }
   if (norm_d) {
     if (pl.copies) pl.dcopy_off = take((size_t)a.d.n_rows * a.dim * eb);
-    else pl.dn_off = take((size_t)a.d.n_rows * 4);  // (also where the kernel takes the norms itself: a caller's buffer fits by size alone)
+    else pl.dn_off = take((size_t)a.d.n_rows * 4);
   }
   pl.need = off;
   // the portable kernel trims masked documents too, where the workspace has room for the lengths: calls that never had to
