@@ -282,8 +282,10 @@ __device__ __noinline__ int2 whole_document(const Document& doc, unsigned rows, 
 // Products in fp32 for the rows of a warp that need them (`what`): a lane gives its row's candidates and gets their largest and who it is.
 // (Not inlined: its registers would cost the epilogue's loop over the columns its own.)
 enum Need { NOTHING, ONE, MANY, ALL };
-__device__ __noinline__ int2 products(SharedCtl* ctl, int what, int tile, long long drow0, int len, int at, int at2, unsigned bits, int row) {
+__device__ __noinline__ int2 products(SharedCtl* ctl, int what, int tile, int doc, int len, int at, int at2, unsigned bits, int row) {
   const SplitParams& P = ctl->params;
+  long long drow0;
+  doc_length(P, doc, drow0, nullptr);
   const Document D(P, drow0);
   const int lane = row & 31, hl = lane & 15, ml = P.q.max_len;
   const bool on0 = hl * 8 < D.dim, on1 = hl * 8 + 4 < D.dim;
@@ -453,20 +455,17 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const __grid_
     // =========================== epilogue ===========================
     const int set = warp >> 2, quad = warp & 3, row = quad * 32 + lane;
     bool ok = true;
-    uint32_t n = 0, n_tile = 0, n_sync = 0, n_emit = 0, n_x = 0;
+    uint32_t n = 0, n_tile = 0, n_sync = 0, n_x = 0;
     int cur = -1;
     const int ml = P.q.max_len;
     const int my_slot = row / ml, my_s = row - my_slot * ml;
     bool have = false, counts = false;
     float qf = 0.f;
-    const float c_sums = 0x1.4p-24f, c_sizes = (float)P.dim * 0x1p-28f;  // both bounds of a comparison
-    const bool lone = ml == 32;  // a query per warp
-    const float enough = fmaxf(4.f, (float)P.dim * 0.25f) * 0x1p-23f;  // what both bounds may be of a product
     for (; ok && w.more(); w.next(P)) {
       long long drow0;
       const int len = doc_length(P, w.doc, drow0, tid == 0 ? P.status : nullptr);
-      const int q0 = w.tile * P.q_per_tile, nq = min(P.q_per_tile, P.n_q - q0);
       if (w.tile != cur) {
+        const int q0 = w.tile * P.q_per_tile, nq = min(P.q_per_tile, P.n_q - q0);
         cur = w.tile;
         ++n_tile;
         have = my_slot < nq;
@@ -493,7 +492,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const __grid_
       int at = 0, at2 = NO_MORE;
       unsigned bits = 0;
       // twice the bound for this row and the document so far
-      auto bounds = [&]() { return fmaf(q_size.x, fmaf(c_sums, d_size.y, c_sizes * d_size.x), q_size.y * (c_sums * d_size.x)); };
+      auto bounds = [&]() { return fmaf(q_size.x, fmaf(0x1.4p-24f, d_size.y, (float)P.dim * 0x1p-28f * d_size.x), q_size.y * (0x1.4p-24f * d_size.x)); };
       const int pieces = max(1, (len + PIECE - 1) / PIECE);
       const bool mine = ((n + pieces - 1) & 1) == set;  // the document's last piece
       for (int p = 0; p < pieces; ++p, ++n) {
@@ -609,7 +608,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const __grid_
       {
         const float both = bounds();  // 0: a row of zeros on either side; infinity, NaN: there is no bound
         if (bits) ri = at + __ffs(bits) - 1;
-        const bool will_do = bits && both < INFINITY && both <= fabsf(r) * enough;  // r is the score as it is
+        const bool will_do = bits && both < INFINITY && both <= fabsf(r) * (fmaxf(4.f, (float)P.dim * 0.25f) * 0x1p-23f);  // r is the product as it is
         const bool live = WINNERS ? have : counts && !will_do;
         if (!bits) r = -INFINITY;
         int what = NOTHING;
@@ -617,7 +616,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const __grid_
         else if (live && both != 0.f && (bits & (bits - 1))) what = MANY;
         else if (counts && !will_do && both != 0.f && bits) what = ONE;
         if (__any_sync(0xffffffffu, what != NOTHING)) {
-          const int2 x = products(ctl, what, w.tile, drow0, len, at, at2, bits, row);
+          const int2 x = products(ctl, what, w.tile, w.doc, len, at, at2, bits, row);
           if (what != NOTHING) {
             if (!will_do) r = __int_as_float(x.x);
             ri = x.y;
@@ -625,15 +624,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) fwd_split_kernel(const __grid_
         }
       }
       const float val = counts && r != -INFINITY ? r * f : 0.f;
+      const int q0 = w.tile * P.q_per_tile, nq = min(P.q_per_tile, P.n_q - q0);
       if (WINNERS && my_slot < nq) {
         int* out = P.argmax + ((long long)(q0 + my_slot) * P.n_d + w.doc) * P.argmax_stride;
         for (int i = my_s; i < P.argmax_stride; i += ml) out[i] = have && i == my_s ? ri : -1;
       }
-      if (lone) {
+      if (ml == 32) {  // a query per warp
         const float sum = warp_sum(val);
         if (lane == 0 && quad < nq) P.scores[(long long)(q0 + quad) * P.n_d + w.doc] = sum;
       } else {
-        float* e = ctl->emit[set][n_emit++ & 1];
+        float* e = ctl->emit[set][n_sync & 1];
         e[row] = val;
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&ctl->epi_sync[set]));
