@@ -28,12 +28,13 @@
 //   warp 8       issues the MMAs of a piece, a part of the query times up to three of the piece at once: five per 16 features
 //   warps 9..24  cut the rows of the pieces and, where it changes, of the query tile: a half-warp per row; they take the norms too
 // Against fwd_generic_kernel, whose fp32 FMAs bound it (queries of up to 32 tokens, documents a fifth to the whole of the length given, normalised):
-// 32 x 32 documents of 180 tokens 52 -> 29 us, 1 x 256 of 512 68 -> 51, 64 x 64 of 300 (48-token queries, 96 features) 418 -> 140, 64 x 256 of
-// 512 (48 tokens) 3010 -> 790; that last with a feature of the documents 100 or 1000 times the others, every product in fp32, 1150; with infinities in a query
-// of every tile 4800, in every sixteenth document 3600; with two features 2^16 times the others, each where the other side has zeros, so that everything
-// is gone through, 28 ms.  (Products for all rows instead of the bound: 32 x 32 35 us, 64 x 256 of 512 and 32 tokens 454 instead of 400; six parts' products
-// instead of eight are not enough for the bound.)
-// Error of the scores against 64 bits, 2-norm over 24 problems of Gaussian rows: 3.3e-8 to 4.7e-8, the other kernel's 5.1e-8 to 6.4e-8.
+// 32 x 32 documents of 180 tokens 52 -> 28 us, 1 x 256 of 512 68 -> 50, 64 x 64 of 300 (48-token queries, 96 features) 421 -> 136, 64 x 256 of
+// 512 (48 tokens) 3010 -> 750; that last with a feature of the documents 100 or 1000 times the others, every product in fp32, 1120; with infinities in a query
+// of every tile 4700, in every sixteenth document 3500; with two features 2^16 times the others, each where the other side has zeros, so that everything
+// is gone through by four warps at a time, 28 ms.  (Products for all rows instead of the bound: 32 x 32 35 us, 64 x 256 of 512 and 32 tokens 454 against 375;
+// the same by three warps of their own 54 and 620.  Without a1 b2 + a2 b1 the bound is four times as wide, too much for Gaussian rows.)
+// What bounds it: issue (59 % active) and the round trips between its roles; the tensor pipe is busy for 45 %.
+// Error of the scores against 64 bits, 2-norm over 24 problems of Gaussian rows: 3.3e-8 to 5.3e-8, the other kernel's 5.0e-8 to 6.4e-8.
 // Every wait is bounded: on expiry the CTA raises LIK_DEV_WAIT_TIMEOUT in the status word, sets a shared abort flag, frees TMEM and
 // returns.  A warp that goes through a document counts its steps, and who waits for it begins anew while they go on.
 #include <cfloat>
