@@ -38,7 +38,7 @@ def ensure_contiguous_last(x: torch.Tensor) -> torch.Tensor:
 def common_dtype(Q: torch.Tensor, D: torch.Tensor) -> torch.dtype:
     """Element type both operands are brought to before the kernel runs.
 
-    Same dtype -> kept (fp32 stays fp32 and is scored by the exact fp32 kernel).  Mixed
+    Same dtype -> kept (fp32 stays fp32 and is scored as such).  Mixed
     inputs follow the reference's rule (_utils.py:137-148): bf16 if either side is bf16,
     otherwise fp16."""
     if Q.dtype == D.dtype:
